@@ -15,15 +15,12 @@
 namespace sa2 {
 namespace tc {
 
+constexpr int SM_COUNT = 148;     // B200
+
 inline int tiles_per_query_tile(int w1) { return (w1 + TJ - 1 + TJ - 1) / TJ; }   // ceil((w1 + 127) / 128)
 
-// The tensor-core forward handles bf16 with head dim 64 and first-key windows whose
-// tiles fit in shared memory (w1 <= 513), or head dim 128 with any window (the
-// window is walked in passes).
-inline bool fwd_supported(const sa2_shape &s) {
-    if (s.dtype != SA2_BF16) return false;
-    return s.d == 128 || (s.d == 64 && tiles_per_query_tile(s.w1) <= MAX_NT);
-}
+// The tensor-core forward handles bf16 at every head dim and any window.
+inline bool fwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 // The tensor-core backward handles bf16 and head dim 64 or 128, any window.
 inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16 && (s.d == 64 || s.d == 128); }
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -93,27 +90,37 @@ inline int fwd128(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
-inline int fwd(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
-    if (!fwd_addressable(kp)) return SA2_ERR_INVALID;
-    if (s.d == 128) return fwd128(kp, s, st);
+template <int D>
+inline int fwd_launch(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
     FwdParams P;
     P.kp = kp;
-    P.nt = tiles_per_query_tile(s.w1);
+    P.ri_log2 = fwd_ri_log2(s, SM_COUNT);
+    P.win_boxes = fwd_win_boxes(s.w2, P.ri_log2);
+    P.nslots = fwd_slots(s.w1, P.ri_log2, P.win_boxes);
     P.c = s.scale * 1.4426950408889634f;
     P.status = status_word();
     if (!P.status) return SA2_ERR_CUDA;
-    CUtensorMap mapK, mapV;
-    if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, 64, kp.k1.sb, kp.k1.sn, kp.k1.sh, TJ) ||
-        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, 64, kp.v1.sb, kp.v1.sn, kp.v1.sh, TJ))
+    CUtensorMap mapK, mapV, mapK2, mapV2;       // 64-row boxes of K1 / V1, 32-row boxes of the second keys / values
+    if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, FWD_UNIT) ||
+        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, FWD_UNIT) ||
+        !tmap::make_rows_map(&mapK2, kp.k2.p, kp.b, kp.nk2, kp.hk, D, kp.k2.sb, kp.k2.sn, kp.k2.sh, 32) ||
+        !tmap::make_rows_map(&mapV2, kp.v2.p, kp.b, kp.nk2, kp.hk, D, kp.v2.sb, kp.v2.sn, kp.v2.sh, 32))
         return SA2_ERR_CUDA;
-    CUtensorMap mapK2;      // second keys, 32-row boxes
-    if (!tmap::make_rows_map(&mapK2, kp.k2.p, kp.b, kp.nk2, kp.hk, 64, kp.k2.sb, kp.k2.sn, kp.k2.sh, 32)) return SA2_ERR_CUDA;
-    const size_t smem = fwd_smem_bytes(P.nt);
-    if (cudaFuncSetAttribute(fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    const size_t smem = fwd_smem_bytes(P.nslots, P.win_boxes);
+    if (cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SA2_ERR_CUDA;
-    dim3 grid((kp.n + TQ - 1) / TQ, kp.hq, kp.b);
-    fwd_kernel<<<grid, FWD_THREADS, smem, st>>>(mapK, mapV, mapK2, P);
+    const int ri = 1 << P.ri_log2;
+    fwd_kernel<D><<<dim3((kp.n + ri - 1) / ri, kp.hq, kp.b), FWD_THREADS, smem, st>>>(mapK, mapV, mapK2, mapV2, P);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
+}
+
+inline int fwd(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
+    if (!fwd_addressable(kp)) return SA2_ERR_INVALID;
+    switch (s.d) {
+        case 32: return fwd_launch<32>(kp, s, st);
+        case 64: return fwd_launch<64>(kp, s, st);
+        default: return fwd128(kp, s, st);
+    }
 }
 
 inline bool bwd_addressable(const KernelParams &kp) {

@@ -31,7 +31,7 @@
 // columns so that the next S^T/dP^T of a half can be issued as soon as the compute
 // group has read the current one.
 #pragma once
-#include "sa2_tc_fwd.cuh"
+#include "sa2_tc_common.cuh"
 
 namespace sa2 {
 namespace tc {

@@ -1,0 +1,91 @@
+// What the tcgen05 kernels share: tile sizes, fast math and packing helpers, the warp-wide bounded wait.
+#pragma once
+#include "sa2_common.cuh"
+#include "sa2_sm100.cuh"
+#include <cuda.h>
+#include <math_constants.h>
+
+namespace sa2 {
+namespace tc {
+
+using namespace sa2::sm100;
+
+constexpr int TQ = 128;          // rows of a tile of query-side operands (TMEM lanes)
+constexpr int TJ = 128;          // first-key rows per tile
+constexpr uint32_t TILE_BYTES = TJ * 64 * 2;
+
+// error bits reported through the device status word
+enum { ERR_FWD_PRODUCER = 1, ERR_FWD_MMA = 2, ERR_FWD_SOFTMAX = 4, ERR_FWD_OUTPUT = 8 };
+
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float lg2(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t *>(&v);
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162 *>(&a), *reinterpret_cast<__nv_bfloat162 *>(&b));
+    return *reinterpret_cast<uint32_t *>(&r);
+}
+
+#ifndef SA2_WARP_WAIT_SLEEP
+#define SA2_WARP_WAIT_SLEEP 64
+#endif
+// every lane of the warp waits; the result is uniform so that the .sync.aligned
+// tcgen05 instructions that follow are never reached by a partial warp
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int prof = -1) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, SA2_WARP_WAIT_SLEEP, prof));
+}
+
+// per-row hand-over between a softmax thread and the output thread of its row:
+// [group][sweep parity][128] final reference of the sweep, then [group][128] denominator and
+// [group][128] the reference it is expressed against
+constexpr int FWD_STATS_FLOATS = 2 * 2 * 128 + 2 * 128 + 2 * 128;
+
+// exp2(c * s - ref) for 32 logits of one row -> 16 packed bf16 pairs; returns their sum.
+// Columns outside (lo, hi] are masked (window / causality / sequence start).
+__device__ __forceinline__ float fwd_probs32(const uint32_t (&s)[32], uint32_t (&pk)[16], float c, float ref,
+                                             bool full, int col0, int lo, int hi) {
+    if (full) {
+        const uint64_t c2 = f2_pack(c, c), nref2 = f2_pack(-ref, -ref);
+        float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+        for (int x = 0; x < 32; x += 2) {
+            float a0, a1;
+            f2_unpack(f2_fma(f2_pack(s[x], s[x + 1]), c2, nref2), a0, a1);
+            const float p0 = ex2(a0), p1 = ex2(a1);
+            sum0 += p0; sum1 += p1;
+            pk[x >> 1] = pack_bf16(p0, p1);
+        }
+        return sum0 + sum1;
+    } else {
+        // Valid columns are the integers in (lo, hi]: |col - mid| <= half, and an invalid column is at least
+        // half + 1 away, so saturate(half + 1 - |col - mid|) is exactly 1 or 0: two FADDs and an FMUL on the
+        // FMA pipe instead of two compares and a select on the (half as wide) ALU pipe.  The exponent is
+        // clamped so that a masked-out logit far above the reference cannot produce inf * 0; a clamped
+        // valid logit still trips the slow path.
+        const float mid = 0.5f * (float)(lo + 1 + hi), hwp = 0.5f * (float)(hi - lo - 1) + 1.f;
+        float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+        for (int x = 0; x < 32; x += 2) {
+            const float v0 = __saturatef(hwp - fabsf((float)(col0 + x) - mid));
+            const float v1 = __saturatef(hwp - fabsf((float)(col0 + x + 1) - mid));
+            const float p0 = ex2(fminf(fmaf(__uint_as_float(s[x]), c, -ref), 100.f)) * v0;
+            const float p1 = ex2(fminf(fmaf(__uint_as_float(s[x + 1]), c, -ref), 100.f)) * v1;
+            sum0 += p0; sum1 += p1;
+            pk[x >> 1] = pack_bf16(p0, p1);
+        }
+        return sum0 + sum1;
+    }
+}
+
+}  // namespace tc
+}  // namespace sa2

@@ -1,319 +1,307 @@
 // Forward kernel on the 5th-generation tensor cores (tcgen05 + TMEM + TMA),
-// bf16 operands, fp32 accumulation, head dim 64.
+// bf16 operands, fp32 accumulation, head dims 32 and 64.
 //
-// One CTA owns 128 query rows of one (batch, query head).  For every offset
-// e = i - k of the second key ("sweep") it forms A_e[i,:] = q_i * k2_{i-e}
-// (bf16, CUDA cores, 128-byte-swizzled shared memory), multiplies it against
-// the TMA-staged K1 tiles of the window (S = A_e K1^T, 128x128x64 per tile,
-// accumulator in TMEM), turns S into P = exp2(c*S - ref) in registers, writes
-// P to TMEM as bf16 and feeds it as the A operand of W_e += P V1 (128x64x128,
-// V1 tile as an MN-major B operand).  At the end of a sweep the row owner adds
-// v2_{i-e} * W_e to its output registers.  The softmax is joint over all
-// (j, e): one denominator per row.
+// A tile is 128 (query row, second-key offset) pairs of one (batch, query head): RI query rows times
+// RE = 128 / RI offsets e = i - k, row r = s * RI + (i - i0) holding e = RE * t + s in "sweep" t.  Per sweep
+// the kernel forms A[r,:] = q_i * k2_{i-e} (bf16, written straight to TMEM), multiplies it against the
+// TMA-staged K1 window of the RI rows (S = A K1^T, 64 keys a unit), turns S into P = exp2(c*S - ref) in
+// registers, writes P to TMEM as bf16 and feeds it as the A operand of W += P V1 (V1 unit as an MN-major B
+// operand).  At the end of a sweep the row owner adds v2_{i-e} * W to its output registers; at the end of
+// the tile the RE partial outputs of a query row are merged through shared memory.  The softmax is joint
+// over all (j, e).
+//
+// Why pairs: the window of RI rows is w1 + RI - 1 keys, so a small RI wastes fewer masked columns (w1 = 512:
+// 576 columns at RI = 64, 640 at RI = 128), a short sequence is spread over more CTAs of fewer sweeps each,
+// and a single new token (generation) still fills the rows of its tile.  fwd_rows_per_tile() picks RI.
 //
 // Warp roles (512 threads, four aligned warpgroups):
-//   warp 0        TMA producer: the K1/V1 window and the 127 + 32 second-key rows
-//                 the tile can pair with, loaded once and resident in shared memory;
-//                 then issues the tcgen05.mma stream of group 1 (one lane)
-//   warp 1        owns the TMEM allocation, issues the tcgen05.mma stream of group 0
-//   warps 2-3     idle (they fill the issuers' warpgroup)
-//   warps 4-7     output group, one thread per query row: builds the A tile of each
-//                 group's next sweep as soon as the last S product of its current sweep
-//                 has completed, and at the end of a sweep adds v2_{i-e} * W_e to the
-//                 row's output registers (one accumulator per softmax group)
-//   warps 8-11    softmax group 0: even sweeps, one thread per query row
-//   warps 12-15   softmax group 1: odd sweeps, one thread per query row
-// An even and an odd sweep are in flight together, so while one group runs the
-// exponentials of its tile the tensor cores work for the other and each SM
-// sub-partition has two softmax warps to hide latencies.  A softmax thread keeps
-// only (reference, denominator) per row; the output thread keeps the two groups'
-// accumulators, each against the reference its group last reported, and merges
-// them at the end.  Registers move between the warpgroups with setmaxnreg.
+//   warp 0, 1     lane 0 issues the tcgen05.mma stream of group 0 / group 1 (warp 1 owns the TMEM allocation)
+//   warp 2, 3     lane 0 of each is a TMA producer: second keys of the tile and K1 units, second values and V1
+//                 units (units are resident if the window fits, else a ring walked once per pair of sweeps)
+//   warps 4-7     output group, one thread per row: builds the A row of each group's next sweep as soon as the
+//                 last S product of its current sweep has completed, and folds v2 * W of the finished sweep
+//   warps 8-11    softmax group 0: even sweeps, one thread per row
+//   warps 12-15   softmax group 1: odd sweeps, one thread per row
+// An even and an odd sweep are in flight together, so while one group runs the exponentials of its unit the
+// tensor cores work for the other and each SM sub-partition has two softmax warps to hide latencies.
 //
-// The unit of the pipeline is half a key tile (64 keys): S = A_e K1[64 rows]^T is
-// 128x64, and every group has two S and two P buffers, so its next unit is
-// ready in TMEM while it works on the current one.
+// A unit is 64 keys.  TMEM columns of group g, from 256 g: S 2 x 64, P (bf16) 2 x 32, W 64.
 //
-// TMEM columns, group g, buffer s: S [128g + 64s, +64), P (bf16) [384 + 64g + 32s, +32);
-// W of group g [256 + 64g, +64).
+// Bound: not the exponentials (512 MUFU cycles per scheduler and unit) but the chain of a group, P stored ->
+// P V1 -> S of the unit after the next -> its exponentials: without any arithmetic in the softmax groups a unit
+// still takes 950 cycles, with it 1000.  So a softmax warp has one barrier wait and one arrival per unit - the
+// issuing thread of a group alternates P V1 of unit u and S of unit u + 2, whose completion therefore also says
+// that the P columns are free - and which 32-column chunks need no mask, or are seen by nobody, is decided from
+// warp-uniform bounds without votes.  (Separate issuing threads for S and P V1, A in TMEM, 128-key units and a
+// second chunk in flight per warp were measured: 1.15 to 1.6 ms where this form takes 1.12.)
+// Measured: b4 n4096 h8 d64 w512/32 1.26 -> 1.12 ms (459 TFLOP/s), b2 n1024 0.178 -> 0.168 ms; what ran on the fp32
+// kernels before: b1 n3001 h8 d64 w1024/16 4.16 -> 0.23 ms, b4 n2048 h8 d32 w512/32 3.9 -> 0.48 ms; one new row
+// of b1 h8 behind a full window 0.19 -> 0.01 ms.
 //
 // Reference handling: probabilities are computed against a per-row reference
 // that only moves when it must, so the W accumulator in TMEM normally never
 // needs a rescale; bf16 has fp32's exponent range, so P may exceed 1 by many
-// orders of magnitude without loss.  When the probabilities of a tile sum to
-// more than 2^64 (always true for a row's very first tile, whose reference is
-// -inf) the warp takes a slow path: exact tile maximum, rescale of the row's
+// orders of magnitude without loss.  When the probabilities of a unit sum to
+// more than 2^64 (always true for a row's very first unit, whose reference is
+// -inf) the warp takes a slow path: exact unit maximum, rescale of the row's
 // partial sums (including W in TMEM), recomputation of P.
 #pragma once
-#include "sa2_common.cuh"
-#include "sa2_sm100.cuh"
-#include <cuda.h>
-#include <math_constants.h>
+#include "sa2_tc_common.cuh"
 
 namespace sa2 {
 namespace tc {
 
-using namespace sa2::sm100;
-
-constexpr int TQ = 128;          // query rows per CTA
-constexpr int TJ = 128;          // first-key rows per tile
 constexpr int FWD_THREADS = 512;
-// Register hand-over between warpgroups (launch: 128 per thread; the budgets must add up to 4 * 128, or
+// Register hand-over between warpgroups (launch: 128 per thread; the budgets must add up to at most 4 * 128, or
 // the growing group never returns from its setmaxnreg).
-constexpr int FWD_REGS_LAUNCH = 128, FWD_REGS_ISSUE = 56, FWD_REGS_SOFTMAX = 112, FWD_REGS_OUT = 232;
-static_assert(FWD_REGS_ISSUE + 2 * FWD_REGS_SOFTMAX + FWD_REGS_OUT == 4 * FWD_REGS_LAUNCH, "register pool must balance");
+constexpr int FWD_REGS_LAUNCH = 128, FWD_REGS_ISSUE = 48, FWD_REGS_SOFTMAX = 120, FWD_REGS_OUT = 216;
+static_assert(FWD_REGS_ISSUE + 2 * FWD_REGS_SOFTMAX + FWD_REGS_OUT <= 4 * FWD_REGS_LAUNCH, "register pool must balance");
 static_assert(FWD_REGS_SOFTMAX < FWD_REGS_LAUNCH, "the softmax groups release registers");
-constexpr int MAX_NT = 5;        // K1/V1 tiles resident in shared memory (head dim 64)
-constexpr uint32_t TILE_BYTES = TJ * 64 * 2;
-constexpr int K2_ROWS = 160;     // second-key rows kept in shared memory: positions i0 - 32 ... i0 + 127
+constexpr int FWD_UNIT = 64;                                  // first-key rows of a unit
+constexpr uint32_t FWD_UNIT_BYTES = FWD_UNIT * 128;           // its K1 (or V1) rows, 128 bytes each
+constexpr int FWD_MAX_SLOTS = 12;
+constexpr int FWD_WIN_ROWS = 128;                             // most second-key rows staged in shared memory
 
 enum FwdBar {
-    BAR_KV_FULL = 0,                     // [MAX_NT]
-    BAR_A_FULL = BAR_KV_FULL + MAX_NT,   // [2] per group
-    BAR_K2_FULL = BAR_A_FULL + 2,
-    BAR_W_FULL = BAR_K2_FULL + 2,        // [2] per group
-    BAR_W_EMPTY = BAR_W_FULL + 2,        // [2] per group
-    BAR_S_FULL = BAR_W_EMPTY + 2,        // [4] group * 2 + buffer
-    BAR_P_FULL = BAR_S_FULL + 4,         // [4]
-    BAR_PV_DONE = BAR_P_FULL + 4,        // [4]
-    BAR_A_FREE = BAR_PV_DONE + 4,        // [2] per group: every S product of the sweep has completed
-    BAR_REF_FULL = BAR_A_FREE + 2,       // [2] per group: the sweep's final reference is in shared memory
+    BAR_KV_FULL = 0,                              // [FWD_MAX_SLOTS] K1 and V1 rows of the unit have landed
+    BAR_KV_FREE = BAR_KV_FULL + FWD_MAX_SLOTS,    // [FWD_MAX_SLOTS] both groups' products on the unit are done
+    BAR_WIN_FULL = BAR_KV_FREE + FWD_MAX_SLOTS,   // second-key and second-value rows have landed
+    BAR_A_FULL = BAR_WIN_FULL + 1,                // [2] per group
+    BAR_A_FREE = BAR_A_FULL + 2,                  // [2] every S product of the sweep has completed
+    BAR_S_FULL = BAR_A_FREE + 2,                  // [4] group * 2 + buffer
+    BAR_P_FULL = BAR_S_FULL + 4,                  // [4] P of the unit is in TMEM and its S has been read (one per
+                                                  // buffer: a warp may be a unit ahead of another)
+    BAR_PV_DONE = BAR_P_FULL + 4,                 // [2] W += P V1 of the unit has completed
+    BAR_W_FULL = BAR_PV_DONE + 2,                 // [2]
+    BAR_W_EMPTY = BAR_W_FULL + 2,                 // [2]
+    BAR_REF_FULL = BAR_W_EMPTY + 2,               // [2] the sweep's final reference is in shared memory
     BAR_COUNT = BAR_REF_FULL + 2
 };
 
-// error bits reported through the device status word
-enum { ERR_FWD_PRODUCER = 1, ERR_FWD_MMA = 2, ERR_FWD_SOFTMAX = 4, ERR_FWD_OUTPUT = 8 };
-
 struct FwdParams {
     KernelParams kp;
-    int nt;          // tiles per query tile: ceil((w1 + 127) / 128), <= MAX_NT
+    int ri_log2;     // query rows per tile
+    int nslots;      // K1/V1 units in shared memory
+    int win_boxes;   // 32-row boxes of staged k2 (and v2) rows; 0: read from global memory
     float c;         // scale * log2(e)
     int *status;     // device status word
 };
 
-// per-row hand-over between a softmax thread and the output thread of its row:
-// [group][sweep parity][128] final reference of the sweep, then [group][128] denominator and
-// [group][128] the reference it is expressed against
-constexpr int FWD_STATS_FLOATS = 2 * 2 * 128 + 2 * 128 + 2 * 128;
-// at least 120 KB: one CTA per SM, so the 512-column TMEM allocation never waits for a co-resident CTA
-inline size_t fwd_smem_bytes(int nt) {
-    const size_t need = 1024 + (size_t)nt * 2 * TILE_BYTES + 2 * TILE_BYTES + K2_ROWS * 128 + FWD_STATS_FLOATS * 4 + 256 + 1024;
+// at least 120 KB: one CTA per SM, so the 512-column TMEM allocation never waits for a co-resident CTA; at least
+// three slots: the merge of the row partials (128 rows of D + 4 floats) reuses them
+inline size_t fwd_smem_bytes(int nslots, int win_boxes) {
+    const size_t need = 1024 + (size_t)(nslots > 3 ? nslots : 3) * 2 * FWD_UNIT_BYTES + (size_t)win_boxes * 2 * 4096 + 2 * TILE_BYTES +
+                        FWD_STATS_FLOATS * 4 + BAR_COUNT * 8 + 64;
     return need > 120 * 1024 ? need : 120 * 1024;
 }
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float lg2(float x) {
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t *>(&v);
-}
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-    __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162 *>(&a), *reinterpret_cast<__nv_bfloat162 *>(&b));
-    return *reinterpret_cast<uint32_t *>(&r);
-}
-
-#ifndef SA2_WARP_WAIT_SLEEP
-#define SA2_WARP_WAIT_SLEEP 64
-#endif
-// every lane of the warp waits; the result is uniform so that the .sync.aligned
-// tcgen05 instructions that follow are never reached by a partial warp
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int prof = -1) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, SA2_WARP_WAIT_SLEEP, prof));
-}
-
 struct FwdGeom {
-    int i0, i_last, jbase, t_first, ntiles, nsweeps;
-    int upe;          // units (half tiles) per sweep
-    int units[2];     // units each group processes: its sweeps x upe
+    int i0, i_last, ri, ri_log2, re;
+    int jbase;        // unit x of a sweep covers rows jbase + 64 x ... + 63
+    int upe;          // units per sweep
+    int nsw[2];       // sweeps of each group
+    int win0;         // position of the first staged second-key row
+    bool resident;    // every unit of the window has its own slot
 };
 
 __device__ __forceinline__ FwdGeom fwd_geom(const FwdParams &P) {
     FwdGeom g;
-    g.i0 = blockIdx.x * TQ;
-    g.i_last = min(g.i0 + TQ - 1, P.kp.n - 1);
-    g.jbase = g.i0 + P.kp.off1 + TJ - TJ * P.nt;      // tile t covers rows jbase + 128 t ... + 127
-    g.t_first = g.jbase >= 0 ? 0 : min(P.nt - 1, (-g.jbase) / TJ);
-    g.ntiles = P.nt - g.t_first;
-    g.nsweeps = min(P.kp.w2, g.i_last + P.kp.off2 + 1);
-    g.upe = 2 * g.ntiles;
-    g.units[0] = ((g.nsweeps + 1) / 2) * g.upe;
-    g.units[1] = (g.nsweeps / 2) * g.upe;
+    const KernelParams &kp = P.kp;
+    g.ri_log2 = P.ri_log2;
+    g.ri = 1 << P.ri_log2;
+    g.re = TQ >> P.ri_log2;
+    g.i0 = blockIdx.x << P.ri_log2;
+    g.i_last = min(g.i0 + g.ri - 1, kp.n - 1);
+    const int jend = g.i_last + kp.off1 + 1, jlow = max(0, g.i0 + kp.off1 - kp.w1 + 1);
+    g.upe = (jend - jlow + FWD_UNIT - 1) / FWD_UNIT;
+    g.jbase = jend - FWD_UNIT * g.upe;                 // may be negative: TMA reads zeros there
+    const int ne = min(kp.w2, g.i_last + kp.off2 + 1);
+    const int nsweeps = (ne + g.re - 1) >> (7 - P.ri_log2);
+    g.nsw[0] = (nsweeps + 1) / 2;
+    g.nsw[1] = nsweeps / 2;
+    g.win0 = g.i0 + kp.off2 - (kp.w2 - 1);
+    g.resident = g.upe <= P.nslots;
     return g;
 }
 
-// ------------------------------------------------------------------ warp 0 (one lane)
-__device__ __forceinline__ void fwd_producer(const FwdParams &P, const FwdGeom &g, const CUtensorMap *mapK, const CUtensorMap *mapV,
-                                             const CUtensorMap *mapK2, uint8_t *sK, uint8_t *sV, uint8_t *sK2, uint64_t *bars) {
-    const KernelParams &kp = P.kp;
-    const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
-    prefetch_tmap(mapK);
-    prefetch_tmap(mapV);
-    prefetch_tmap(mapK2);
-    if (kp.w2 <= 32) {
-        mbar_arrive_expect_tx(&bars[BAR_K2_FULL], K2_ROWS * 128);
-        for (int bx = 0; bx < K2_ROWS / 32; ++bx)
-            tma_load_4d(sK2 + bx * 4096, mapK2, &bars[BAR_K2_FULL], 0, hk, g.i0 + kp.off2 - 32 + 32 * bx, b);
-    } else {
-        mbar_arrive(&bars[BAR_K2_FULL]);
+// Where the units of a walk live: in a resident window unit w has slot w and is loaded once; a ring gives the x-th
+// unit of the walk (x counts units over pairs of sweeps) slot x % nslots.
+struct FwdSlot {
+    int slot = 0, use = 0;       // `use`: how often the slot has been used before (ring)
+    __device__ __forceinline__ void next(const FwdParams &P, const FwdGeom &g, int w) {
+        if (g.resident) slot = w + 1 == g.upe ? 0 : w + 1;
+        else if (++slot == P.nslots) { slot = 0; ++use; }
     }
-    for (int t = P.nt - 1; t >= g.t_first; --t) {      // the diagonal tile first
-        mbar_arrive_expect_tx(&bars[BAR_KV_FULL + t], 2 * TILE_BYTES);
-        tma_load_4d(sK + (size_t)t * TILE_BYTES, mapK, &bars[BAR_KV_FULL + t], 0, hk, g.jbase + TJ * t, b);
-        tma_load_4d(sV + (size_t)t * TILE_BYTES, mapV, &bars[BAR_KV_FULL + t], 0, hk, g.jbase + TJ * t, b);
+};
+
+// ------------------------------------------------------------------ TMA producers (warps 2 and 3, one lane each)
+__device__ __forceinline__ int fwd_producer(const FwdParams &P, const FwdGeom &g, const CUtensorMap *map, const CUtensorMap *map2,
+                                            uint8_t *dst, uint8_t *win, uint64_t *bars, volatile int *abort_flag) {
+    const int b = blockIdx.z, hk = blockIdx.y / P.kp.g;
+    const int items = g.resident ? g.upe : g.nsw[0] * g.upe;
+    FwdSlot s;
+    int w = 0;
+    auto load = [&]() -> bool {
+        if (s.use >= 1 && !mbar_wait(&bars[BAR_KV_FREE + s.slot], (s.use - 1) & 1, abort_flag, 32, 1)) return false;
+        mbar_arrive_expect_tx(&bars[BAR_KV_FULL + s.slot], FWD_UNIT_BYTES);
+        tma_load_4d(dst + s.slot * FWD_UNIT_BYTES, map, &bars[BAR_KV_FULL + s.slot], 0, hk, g.jbase + FWD_UNIT * w, b);
+        s.next(P, g, w);
+        if (++w == g.upe) w = 0;
+        return true;
+    };
+    if (P.win_boxes > 0) {
+        mbar_arrive_expect_tx(&bars[BAR_WIN_FULL], P.win_boxes * 4096);
+        for (int bx = 0; bx < P.win_boxes; ++bx) tma_load_4d(win + bx * 4096, map2, &bars[BAR_WIN_FULL], 0, hk, g.win0 + 32 * bx, b);
     }
+    for (int x = 0; x < items; ++x)
+        if (!load()) return ERR_FWD_PRODUCER;
+    // every load must have landed before the CTA may exit, even if the consumers gave up
+    if (P.win_boxes > 0 && !mbar_wait(&bars[BAR_WIN_FULL], 0, abort_flag, 32)) return ERR_FWD_PRODUCER;
+    for (int x = max(0, items - P.nslots); x < items; ++x)
+        if (!mbar_wait(&bars[BAR_KV_FULL + x % P.nslots], (x / P.nslots) & 1, abort_flag, 32)) return ERR_FWD_PRODUCER;
+    return 0;
 }
 
 // ------------------------------------------------------------------ MMA issuers (one lane each)
-// Lane 0 of warp 1 issues for group 0 and lane 0 of warp 0 for group 1: the two groups touch disjoint
-// TMEM columns and only read shared memory, so their MMA streams need no ordering between them, and
-// two issuing threads double the rate at which instructions reach the tensor cores.
-// Group g's stream: unit r is half tile r % upe of the group's (r / upe)-th sweep, e = 2 (r / upe) + g.
-__device__ __forceinline__ int fwd_mma(const FwdGeom &g, int grp, uint32_t tmem, uint8_t *sK, uint8_t *sV, uint8_t *sA,
+// Lane 0 of warp g issues for group g: the two groups touch disjoint TMEM columns and only read shared memory,
+// so their MMA streams need no ordering between them.  P V1 of unit u goes before S of unit u + 2, whose
+// completion therefore covers it (and the sweep after the next needs its A rows by then, whose builder waits for
+// the W that P V1 completes).
+template <int D>
+__device__ __forceinline__ int fwd_mma(const FwdParams &P, const FwdGeom &g, int grp, uint32_t tmem, uint8_t *sK, uint8_t *sV, uint8_t *sA,
                                        uint64_t *bars, volatile int *abort_flag) {
-    constexpr uint32_t IDESC_S = idesc_bf16(128, 64, false, false);
-    constexpr uint32_t IDESC_PV = idesc_bf16(128, 64, false, true);
-    // descriptors differ only in their start-address field (units of 16 bytes): build them once
+    constexpr uint32_t IDESC_S = idesc_bf16(128, FWD_UNIT, false, false);
+    constexpr uint32_t IDESC_PV = idesc_bf16(128, 64, false, true);    // (head dim 32: the upper 32 channels are zeros)
+    const uint64_t dK = smem_desc_sw128(smem_u32(sK)), dV = smem_desc_sw128(smem_u32(sV));
     const uint64_t dA = smem_desc_sw128(smem_u32(sA) + grp * TILE_BYTES);
-    const uint64_t dK = smem_desc_sw128(smem_u32(sK));
-    const uint64_t dV = smem_desc_sw128(smem_u32(sV));
-    const uint32_t tS = tmem + grp * 128, tW = tmem + 256 + grp * 64, tP = tmem + 384 + grp * 64;
-    const int n = g.units[grp];
+    const uint32_t tS = tmem + grp * 256, tP = tS + 128, tW = tS + 192;
+    const int upe = g.upe, n = g.nsw[grp] * upe;
+    FwdSlot ss, ps;
+    int s_k = 0, s_w = 0, p_k = 0, p_w = 0;             // sweep and unit of the next S and of the next P V1
 
-    // running position of the unit whose S is issued next (s_*) and whose PV is issued next (p_*)
-    int s_k = 0, s_w = 0, p_k = 0, p_w = 0;
-
-    auto issue_s = [&](int r) -> bool {
-        const int tile = g.t_first + (s_w >> 1), half = s_w & 1, sb = r & 1;
+    auto issue_s = [&](int u) -> bool {
         if (s_w == 0 && !mbar_wait(&bars[BAR_A_FULL + grp], s_k & 1, abort_flag, 0, 1)) return false;
-        if (s_k == 0 && half == 0 && !mbar_wait(&bars[BAR_KV_FULL + tile], 0, abort_flag)) return false;
+        if ((s_k == 0 || !g.resident) && !mbar_wait(&bars[BAR_KV_FULL + ss.slot], ss.use & 1, abort_flag, 0, 4)) return false;
         tc_fence_after();
-        const uint64_t kt = dK + (uint64_t)((tile * TILE_BYTES + half * 8192) >> 4);
-        const uint32_t d = tS + sb * 64;
-        mma_ss(d, dA, kt, IDESC_S, 0u);
-        mma_ss(d, dA + 2, kt + 2, IDESC_S, 1u);
-        mma_ss(d, dA + 4, kt + 4, IDESC_S, 1u);
-        mma_ss(d, dA + 6, kt + 6, IDESC_S, 1u);
-        tc_commit(&bars[BAR_S_FULL + grp * 2 + sb]);
-        if (s_w == g.upe - 1) tc_commit(&bars[BAR_A_FREE + grp]);      // the A stage may be rebuilt
-        if (++s_w == g.upe) { s_w = 0; ++s_k; }
+        const uint64_t kt = dK + (uint64_t)((ss.slot * FWD_UNIT_BYTES) >> 4);
+        const uint32_t d = tS + (u & 1) * 64;
+#pragma unroll
+        for (int st = 0; st < D / 16; ++st) mma_ss(d, dA + st * 2, kt + st * 2, IDESC_S, st > 0 ? 1u : 0u);
+        tc_commit(&bars[BAR_S_FULL + grp * 2 + (u & 1)]);
+        if (s_w == upe - 1) tc_commit(&bars[BAR_A_FREE + grp]);          // the A rows may be rebuilt
+        ss.next(P, g, s_w);
+        if (++s_w == upe) { s_w = 0; ++s_k; }
         return true;
     };
-    auto issue_pv = [&](int r) -> bool {
-        const int tile = g.t_first + (p_w >> 1), half = p_w & 1, sb = r & 1;
-        if (!mbar_wait(&bars[BAR_P_FULL + grp * 2 + sb], (r >> 1) & 1, abort_flag, 0, 2)) return false;
-        if (p_w == 0 && p_k >= 1 && !mbar_wait(&bars[BAR_W_EMPTY + grp], (p_k - 1) & 1, abort_flag, 0, 3)) return false;
+    for (int u = 0; u < 2 && u < n; ++u)
+        if (!issue_s(u)) return ERR_FWD_MMA;
+    for (int u = 0; u < n; ++u) {
+        if (p_w == 0 && p_k >= 1 && !mbar_wait(&bars[BAR_W_EMPTY + grp], (p_k - 1) & 1, abort_flag, 0, 3)) return ERR_FWD_MMA;
+        if (!mbar_wait(&bars[BAR_P_FULL + grp * 2 + (u & 1)], (u >> 1) & 1, abort_flag, 0, 2)) return ERR_FWD_MMA;
         tc_fence_after();
-        const uint64_t vt = dV + (uint64_t)((tile * TILE_BYTES + half * 8192) >> 4);
-        const uint32_t a = tP + sb * 32;
-        mma_ts(tW, a, vt, IDESC_PV, p_w > 0 ? 1u : 0u);
-        mma_ts(tW, a + 8, vt + 128, IDESC_PV, 1u);
-        mma_ts(tW, a + 16, vt + 256, IDESC_PV, 1u);
-        mma_ts(tW, a + 24, vt + 384, IDESC_PV, 1u);
-        tc_commit(&bars[BAR_PV_DONE + grp * 2 + sb]);
-        if (p_w == g.upe - 1) tc_commit(&bars[BAR_W_FULL + grp]);
-        if (++p_w == g.upe) { p_w = 0; ++p_k; }
-        return true;
-    };
-
-    for (int r = 0; r < 2 && r < n; ++r)
-        if (!issue_s(r)) return ERR_FWD_MMA;
-    for (int r = 0; r < n; ++r) {
-        if (!issue_pv(r)) return ERR_FWD_MMA;
-        if (r + 2 < n && !issue_s(r + 2)) return ERR_FWD_MMA;
+        const uint64_t vt = dV + (uint64_t)((ps.slot * FWD_UNIT_BYTES) >> 4);
+        const uint32_t a = tP + (u & 1) * 32;
+#pragma unroll
+        for (int st = 0; st < 4; ++st) mma_ts(tW, a + st * 8, vt + st * 128, IDESC_PV, (p_w > 0 || st > 0) ? 1u : 0u);
+        tc_commit(&bars[BAR_PV_DONE + grp]);
+        if (!g.resident) tc_commit(&bars[BAR_KV_FREE + ps.slot]);
+        if (p_w == upe - 1) tc_commit(&bars[BAR_W_FULL + grp]);
+        ps.next(P, g, p_w);
+        if (++p_w == upe) { p_w = 0; ++p_k; }
+        if (u + 2 < n && !issue_s(u + 2)) return ERR_FWD_MMA;
+    }
+    // The ring follows group 0's walk.  With an odd number of sweeps group 1 has one sweep less: it lets the
+    // units of that last sweep pass, so that every slot still collects two releases.
+    if (!g.resident) {
+        for (int x = n; x < g.nsw[0] * upe; ++x, ps.next(P, g, 0)) {
+            if (!mbar_wait(&bars[BAR_KV_FULL + ps.slot], ps.use & 1, abort_flag, 32)) return ERR_FWD_MMA;
+            mbar_arrive(&bars[BAR_KV_FREE + ps.slot]);
+        }
     }
     return 0;
 }
 
 // ------------------------------------------------------------------ softmax groups (warps 8-11, 12-15)
-// exp2(c * s - ref) for 32 logits of one row -> 16 packed bf16 pairs; returns their sum.
-// Columns outside (lo, hi] are masked (window / causality / sequence start).
-__device__ __forceinline__ float fwd_probs32(const uint32_t (&s)[32], uint32_t (&pk)[16], float c, float ref,
-                                             bool full, int col0, int lo, int hi) {
-    float sum0 = 0.f, sum1 = 0.f;
-    if (full) {
-#pragma unroll
-        for (int x = 0; x < 32; x += 2) {
-            const float p0 = ex2(fmaf(__uint_as_float(s[x]), c, -ref));
-            const float p1 = ex2(fmaf(__uint_as_float(s[x + 1]), c, -ref));
-            sum0 += p0; sum1 += p1;
-            pk[x >> 1] = pack_bf16(p0, p1);
-        }
-    } else {
-        // Valid columns are the integers in (lo, hi]: |col - mid| <= half, and an invalid column is at least
-        // half + 1 away, so saturate(half + 1 - |col - mid|) is exactly 1 or 0: two FADDs and an FMUL on the
-        // FMA pipe instead of two compares and a select on the (half as wide) ALU pipe.  The exponent is
-        // clamped so that a masked-out logit far above the reference cannot produce inf * 0; a clamped
-        // valid logit still trips the slow path.
-        const float mid = 0.5f * (float)(lo + 1 + hi), hwp = 0.5f * (float)(hi - lo - 1) + 1.f;
-#pragma unroll
-        for (int x = 0; x < 32; x += 2) {
-            const float v0 = __saturatef(hwp - fabsf((float)(col0 + x) - mid));
-            const float v1 = __saturatef(hwp - fabsf((float)(col0 + x + 1) - mid));
-            const float p0 = ex2(fminf(fmaf(__uint_as_float(s[x]), c, -ref), 100.f)) * v0;
-            const float p1 = ex2(fminf(fmaf(__uint_as_float(s[x + 1]), c, -ref), 100.f)) * v1;
-            sum0 += p0; sum1 += p1;
-            pk[x >> 1] = pack_bf16(p0, p1);
-        }
-    }
-    return sum0 + sum1;
+// Which rows the 32 rows of a warp are, in terms that are the same for all its lanes.
+struct FwdWarpRows {
+    int imin, imax;     // query rows (imax may lie past the end of the sequence)
+    int emin, emax;     // offsets of the rows in sweep 0
+    int some0, some1;   // 32-key chunks (counted from jbase) that some row sees: some0 <= x <= some1
+    int full0, full1;   // chunks that every row sees whole
+};
+__device__ __forceinline__ FwdWarpRows fwd_warp_rows(const KernelParams &kp, const FwdGeom &g) {
+    const int first = __shfl_sync(0xffffffffu, ((int)threadIdx.x >> 5) & 3, 0) * 32;      // warp-uniform
+    FwdWarpRows w;
+    const int span = min(32, g.ri);
+    w.imin = g.i0 + (first & (g.ri - 1));
+    w.imax = w.imin + span - 1;
+    w.emin = first >> g.ri_log2;
+    w.emax = (first + 31) >> g.ri_log2;
+    const int jlo = max(0, w.imin + kp.off1 - kp.w1 + 1), jlo_all = max(0, w.imax + kp.off1 - kp.w1 + 1);    // any / every row from
+    w.some0 = max(0, jlo - g.jbase) >> 5;
+    w.some1 = (w.imax + kp.off1 - g.jbase) >> 5;
+    w.full0 = (max(0, jlo_all - g.jbase) + 31) >> 5;
+    w.full1 = ((w.imin + kp.off1 - g.jbase + 1) >> 5) - 1;
+    return w;
 }
 
-__device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g, int grp, uint32_t tmem, float *stats,
+__device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g, int grp, uint32_t tmem, int d_w, float *stats,
                                            uint64_t *bars, volatile int *abort_flag) {
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = (warp & 3) * 32 + lane;            // query row within the tile = TMEM lane
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t s_addr = lane_addr + grp * 128, p_addr = lane_addr + 384 + grp * 64, w_addr = lane_addr + 256 + grp * 64;
-    const int i = g.i0 + r;
-    const bool row_ok = i < kp.n;
+    const int r = (warp & 3) * 32 + lane;            // row of the tile = TMEM lane
+    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + grp * 256;
+    const int i = g.i0 + (r & (g.ri - 1)), e0 = r >> g.ri_log2;
+    const FwdWarpRows wr = fwd_warp_rows(kp, g);
     const float c = P.c;
-    const int nsw = grp == 0 ? (g.nsweeps + 1) / 2 : g.nsweeps / 2;
+    const int upe = g.upe, nsw = g.nsw[grp];
     float *ref_slot = stats + grp * 256 + r;          // + 128 * (sweep parity)
 
+    const uint32_t w_addr = lane_addr + 192;
+
     float ref = -CUDART_INF_F, l = 0.f;
-
+    int u = 0;
     for (int k = 0; k < nsw; ++k) {
-        const int e = 2 * k + grp;
-        const bool sweep_ok = row_ok && (i + kp.off2 - e >= 0);
+        const int eb = g.re * (2 * k + grp);
+        // every row of the warp pairs with a second key in this sweep / no row does
+        const bool all_ok = wr.imax < kp.n && eb + wr.emax < kp.w2 && wr.imin + kp.off2 - eb - wr.emax >= 0;
+        const bool none_ok = wr.imin >= kp.n || eb + wr.emin >= kp.w2 || wr.imax + kp.off2 - eb - wr.emin < 0;
+        const bool row_ok = i < kp.n && eb + e0 < kp.w2 && i + kp.off2 - eb - e0 >= 0;
+        const int full0 = all_ok ? wr.full0 : 1 << 30, some1 = none_ok ? -1 : wr.some1;
 #pragma unroll 1
-        for (int w = 0; w < g.upe; ++w) {
-            const int u = k * g.upe + w, sb = u & 1;
-            const int j0 = g.jbase + TJ * (g.t_first + (w >> 1)) + 64 * (w & 1);
-            // valid columns of this row: lo < col <= hi
-            const int d1 = i + kp.off1 - j0;
-            const int hi = sweep_ok ? min(d1, 63) : -1;
-            const int lo = max(d1 - kp.w1, -j0 - 1);
-            if (!warp_wait(&bars[BAR_S_FULL + grp * 2 + sb], (u >> 1) & 1, abort_flag, 1)) return ERR_FWD_SOFTMAX;
+        for (int w = 0; w < upe; ++w, ++u) {
+            const int j0 = g.jbase + FWD_UNIT * w, buf = u & 1;
+            const uint32_t s_addr = lane_addr + buf * 64, p_addr = lane_addr + 128 + buf * 32;
+            if (!warp_wait(&bars[BAR_S_FULL + grp * 2 + buf], (u >> 1) & 1, abort_flag, 1)) return ERR_FWD_SOFTMAX;
             tc_fence_after();
-            const bool full = __all_sync(0xffffffffu, lo < 0 && hi >= 63);
-
-            float tile_sum = 0.f;
+            // valid columns of this row: lo < col <= hi
+            const int d1 = i + kp.off1 - j0, hi = row_ok ? d1 : -1, lo = max(d1 - kp.w1, -j0 - 1);
+            float sum = 0.f;
 #pragma unroll
             for (int ch = 0; ch < 2; ++ch) {
                 uint32_t s[32], pk[16];
-                tmem_ld32(s_addr + sb * 64 + ch * 32, s);
-                tmem_wait_ld();
-                tile_sum += fwd_probs32(s, pk, c, ref, full, ch * 32, lo, hi);
-                tmem_st16(p_addr + sb * 32 + ch * 16, pk);
+                tmem_ld32(s_addr + ch * 32, s);
+                const int x = 2 * w + ch;            // 32-key chunk of the window
+                tmem_wait_ld(s);
+                if (x >= full0 && x <= wr.full1) {
+                    sum += fwd_probs32(s, pk, c, ref, true, 0, 0, 0);
+                } else if (x >= wr.some0 && x <= some1) {
+                    sum += fwd_probs32(s, pk, c, ref, false, ch * 32, lo, hi);
+                } else {
+#pragma unroll
+                    for (int z = 0; z < 16; ++z) pk[z] = 0u;
+                }
+                tmem_st16(p_addr + ch * 16, pk);
             }
-            const bool exceed = !(tile_sum <= 1.8446744e19f);       // above 2^64, inf or NaN
+            const bool exceed = !(sum <= 1.8446744e19f);       // above 2^64, inf or NaN
             if (__any_sync(0xffffffffu, exceed)) {
                 // ---- slow path (whole warp): exact maximum of this unit, rescale, recompute
                 float mx = -CUDART_INF_F;
 #pragma unroll 1
                 for (int ch = 0; ch < 2; ++ch) {
                     uint32_t s[32];
-                    tmem_ld32(s_addr + sb * 64 + ch * 32, s);
-                    tmem_wait_ld();
+                    tmem_ld32(s_addr + ch * 32, s);
+                    tmem_wait_ld(s);
 #pragma unroll
                     for (int x = 0; x < 32; ++x) {
                         const int col = ch * 32 + x;
@@ -329,42 +317,40 @@ __device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g,
                 }
                 if (w > 0) {
                     // W of this sweep already holds partial sums against the old reference
-                    const int up = u - 1;
-                    if (!warp_wait(&bars[BAR_PV_DONE + grp * 2 + (up & 1)], (up >> 1) & 1, abort_flag)) return ERR_FWD_SOFTMAX;
+                    if (!warp_wait(&bars[BAR_PV_DONE + grp], (u - 1) & 1, abort_flag)) return ERR_FWD_SOFTMAX;
                     tc_fence_after();
 #pragma unroll 1
-                    for (int half = 0; half < 2; ++half) {
+                    for (int ch = 0; ch < d_w; ch += 32) {
                         uint32_t wv[32];
-                        tmem_ld32(w_addr + half * 32, wv);
-                        tmem_wait_ld();
+                        tmem_ld32(w_addr + ch, wv);
+                        tmem_wait_ld(wv);
 #pragma unroll
                         for (int x = 0; x < 32; ++x) wv[x] = __float_as_uint(__uint_as_float(wv[x]) * f);
-                        tmem_st32(w_addr + half * 32, wv);
+                        tmem_st32(w_addr + ch, wv);
                     }
                 }
-                tile_sum = 0.f;
+                tmem_wait_st();
+                sum = 0.f;
 #pragma unroll 1
                 for (int ch = 0; ch < 2; ++ch) {
                     uint32_t s[32], pk[16];
-                    tmem_ld32(s_addr + sb * 64 + ch * 32, s);
-                    tmem_wait_ld();
-                    tile_sum += fwd_probs32(s, pk, c, ref, false, ch * 32, lo, hi);
-                    tmem_st16(p_addr + sb * 32 + ch * 16, pk);
+                    tmem_ld32(s_addr + ch * 32, s);
+                    tmem_wait_ld(s);
+                    sum += fwd_probs32(s, pk, c, ref, false, ch * 32, lo, hi);
+                    tmem_st16(p_addr + ch * 16, pk);
                 }
             }
-            l += tile_sum;
+            l += sum;
             tmem_wait_st();
-            if (w == g.upe - 1) {
-                // W_e is expressed against the reference the row has now.  The output thread has read the
-                // slot of sweep k - 2 before it released that sweep's W; waiting for the release of sweep
-                // k - 1 also keeps this barrier from running two phases ahead of its reader.
-                if (k >= 1 && !warp_wait(&bars[BAR_W_EMPTY + grp], (k - 1) & 1, abort_flag)) return ERR_FWD_SOFTMAX;
-                ref_slot[(k & 1) * 128] = ref;
-                mbar_arrive(&bars[BAR_REF_FULL + grp]);
-            }
             tc_fence_before();
-            mbar_arrive(&bars[BAR_P_FULL + grp * 2 + sb]);
+            mbar_arrive(&bars[BAR_P_FULL + grp * 2 + buf]);
         }
+        // W of the sweep is expressed against the reference the row has now.  The output thread has read the
+        // slot of sweep k - 2 before it released that sweep's W; waiting for the release of sweep
+        // k - 1 also keeps this barrier from running two phases ahead of its reader.
+        if (k >= 1 && !warp_wait(&bars[BAR_W_EMPTY + grp], (k - 1) & 1, abort_flag, 3)) return ERR_FWD_SOFTMAX;
+        ref_slot[(k & 1) * 128] = ref;
+        mbar_arrive(&bars[BAR_REF_FULL + grp]);
     }
     stats[512 + grp * 128 + r] = l;
     stats[768 + grp * 128 + r] = ref;
@@ -372,130 +358,200 @@ __device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g,
 }
 
 // ------------------------------------------------------------------ output group (warps 4-7)
-// Thread r owns query row r: it builds row r of every A tile and accumulates the row's output, one
-// accumulator per softmax group, each against the reference that group reported with its last sweep.
-__device__ __forceinline__ int fwd_output(const FwdParams &P, const FwdGeom &g, uint32_t tmem, float (&o0)[64], float (&o1)[64],
-                                          float &ref0, float &ref1, uint8_t *sA, const uint8_t *sK2, const float *stats,
-                                          uint64_t *bars, volatile int *abort_flag) {
+// Thread r owns row r of the tile: it builds the row of every A and accumulates the row's output against the
+// larger of the references the two groups have reported (`ref_o`).
+template <int D>
+__device__ __forceinline__ int fwd_output(const FwdParams &P, const FwdGeom &g, uint32_t tmem, uint64_t (&o)[D / 2], float &ref_o,
+                                          const uint8_t *sWin, uint8_t *sA, const float *stats, uint64_t *bars, volatile int *abort_flag) {
+    constexpr int NC = D / 8;                          // 16-byte chunks of a row
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
-    const int i = g.i0 + r;
+    const int i = g.i0 + (r & (g.ri - 1)), e0 = r >> g.ri_log2;
     const bool row_ok = i < kp.n;
     const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p);
     const __nv_bfloat16 *v2 = reinterpret_cast<const __nv_bfloat16 *>(kp.v2.p);
-    const bool k2_in_smem = kp.w2 <= 32;
-    const int nsw0 = (g.nsweeps + 1) / 2, nsw1 = g.nsweeps / 2;
+    const bool staged = P.win_boxes > 0;
+    const uint8_t *sWinV = sWin + P.win_boxes * 4096;
 
-    uint4 qv[8];
+    uint4 qv[NC];
+    const __nv_bfloat16 *qrow = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, row_ok ? i : 0, h);
 #pragma unroll
-    for (int cc = 0; cc < 8; ++cc) qv[cc] = make_uint4(0u, 0u, 0u, 0u);
-    if (row_ok) {
-        const __nv_bfloat16 *qrow = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, i, h);
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc) qv[cc] = __ldg(reinterpret_cast<const uint4 *>(qrow + cc * 8));
-    }
+    for (int cc = 0; cc < NC; ++cc) qv[cc] = row_ok ? __ldg(reinterpret_cast<const uint4 *>(qrow + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
 
-    // row r of A_e = q_i * k2_{i-e} for sweep e = 2 k + grp, into the group's A stage
-    auto build_a = [&](int grp, int k) {
-        const int e = 2 * k + grp;
-        uint8_t *dst = sA + (size_t)grp * TILE_BYTES;
-        const int kk = i + kp.off2 - e;
-        const bool ok = row_ok && kk >= 0;
+    // this thread's row of A = q_i * k2_{i-e} for the group's sweep k; the products are formed before the wait for
+    // the stage (`bar`, unless null)
+    auto build_a = [&](int grp, int k, uint64_t *bar, uint32_t parity) -> bool {
+        const int e = g.re * (2 * k + grp) + e0, kk = i + kp.off2 - e;
+        const bool ok = row_ok && e < kp.w2 && kk >= 0;
+        const int wr = kk - g.win0;
         const __nv_bfloat16 *krow = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-        // all eight loads first, then the products and stores
-        uint4 kv[8];
+        uint8_t *dst = sA + (size_t)grp * TILE_BYTES;
+        uint4 a[NC];
 #pragma unroll
-        for (int cc = 0; cc < 8; ++cc)
-            kv[cc] = !ok ? make_uint4(0u, 0u, 0u, 0u)
-                         : k2_in_smem ? *reinterpret_cast<const uint4 *>(sK2 + sw128_offset(r + 32 - e, cc))
-                                      : __ldg(reinterpret_cast<const uint4 *>(krow + cc * 8));
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc) {
-            uint4 v;
-            v.x = mul_bf16x2(qv[cc].x, kv[cc].x); v.y = mul_bf16x2(qv[cc].y, kv[cc].y);
-            v.z = mul_bf16x2(qv[cc].z, kv[cc].z); v.w = mul_bf16x2(qv[cc].w, kv[cc].w);
-            *reinterpret_cast<uint4 *>(dst + sw128_offset(r, cc)) = v;
+        for (int cc = 0; cc < NC; ++cc) {
+            uint4 kv = make_uint4(0u, 0u, 0u, 0u);
+            if (ok) kv = staged ? *reinterpret_cast<const uint4 *>(sWin + sw128_offset(wr, cc)) : __ldg(reinterpret_cast<const uint4 *>(krow + cc * 8));
+            a[cc].x = mul_bf16x2(qv[cc].x, kv.x); a[cc].y = mul_bf16x2(qv[cc].y, kv.y);
+            a[cc].z = mul_bf16x2(qv[cc].z, kv.z); a[cc].w = mul_bf16x2(qv[cc].w, kv.w);
         }
+        if (bar && !warp_wait(bar, parity, abort_flag, 1)) return false;
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) *reinterpret_cast<uint4 *>(dst + sw128_offset(r, cc)) = a[cc];
         fence_proxy_async_smem();
         mbar_arrive(&bars[BAR_A_FULL + grp]);
+        return true;
     };
 
-    // o += v2_{i-e} * W_e (TMEM), after moving o to the reference W_e was built against
-    auto drain = [&](int grp, int k, float (&o)[64], float &ref_o) -> bool {
+    // o += v2_{i-e} * W (TMEM), with o held against the larger reference seen so far
+    auto drain = [&](int grp, int k) -> bool {
+        const int e = g.re * (2 * k + grp) + e0, kk = i + kp.off2 - e;
+        const bool row = row_ok && e < kp.w2 && kk >= 0;
+        const int wr = kk - g.win0;
+        const __nv_bfloat16 *vrow = v2 + elem_off(kp.v2, b, row ? kk : 0, hk);
         if (!warp_wait(&bars[BAR_REF_FULL + grp], k & 1, abort_flag, 2)) return false;
         const float ref_w = stats[grp * 256 + (k & 1) * 128 + r];
         if (!warp_wait(&bars[BAR_W_FULL + grp], k & 1, abort_flag, 3)) return false;
         tc_fence_after();
-        const int kk = i + kp.off2 - (2 * k + grp);
-        const bool ok = row_ok && kk >= 0 && ref_w > -CUDART_INF_F;
-        if (ok && ref_w > ref_o) {
-            const float f = ex2(ref_o - ref_w);              // 0 while the accumulator is still empty
+        const bool ok = row && ref_w > -CUDART_INF_F;
+        float fw = 1.f;
+        if (ok) {
+            if (ref_w > ref_o) {
+                const float f = ex2(ref_o - ref_w);              // 0 while the accumulator is still empty
+                const uint64_t f2 = f2_pack(f, f);
 #pragma unroll
-            for (int x = 0; x < 64; ++x) o[x] *= f;
-            ref_o = ref_w;
+                for (int x = 0; x < D / 2; ++x) o[x] = f2_mul(o[x], f2);
+                ref_o = ref_w;
+            } else {
+                fw = ex2(ref_w - ref_o);
+            }
         }
+        const uint64_t fw2 = f2_pack(fw, fw);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (int half = 0; half < D / 32; ++half) {
             uint32_t w[32];
-            tmem_ld32(lane_addr + 256 + grp * 64 + half * 32, w);
-            tmem_wait_ld();
-            if (ok) {
-                const __nv_bfloat16 *vp = v2 + elem_off(kp.v2, b, kk, hk) + half * 32;
-                uint4 raw[4];
+            tmem_ld32(lane_addr + grp * 256 + 192 + half * 32, w);
+            uint4 raw[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) raw[u] = __ldg(reinterpret_cast<const uint4 *>(vp + u * 8));
+            for (int u = 0; u < 4; ++u) {
+                raw[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (ok) raw[u] = staged ? *reinterpret_cast<const uint4 *>(sWinV + sw128_offset(wr, half * 4 + u))
+                                        : __ldg(reinterpret_cast<const uint4 *>(vrow + half * 32 + u * 8));
+            }
+            tmem_wait_ld(w);
+            if (half == D / 32 - 1) {           // W of the sweep is in registers: the tensor cores may overwrite it
+                tc_fence_before();
+                mbar_arrive(&bars[BAR_W_EMPTY + grp]);
+            }
+            if (ok) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const uint32_t rr[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
 #pragma unroll
                     for (int z = 0; z < 4; ++z) {
-                        const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162 *>(&rr[z]);
-                        const int x = half * 32 + u * 8 + z * 2;
-                        o[x] = fmaf(__uint_as_float(w[u * 8 + z * 2]), __low2float(vv), o[x]);
-                        o[x + 1] = fmaf(__uint_as_float(w[u * 8 + z * 2 + 1]), __high2float(vv), o[x + 1]);
+                        const int x = u * 8 + z * 2;
+                        uint64_t &acc = o[half * 16 + (x >> 1)];
+                        acc = f2_fma(f2_pack(w[x], w[x + 1]), f2_mul(f2_from_bf16x2(rr[z]), fw2), acc);
                     }
                 }
             }
         }
-        tc_fence_before();
-        mbar_arrive(&bars[BAR_W_EMPTY + grp]);
         return true;
     };
 
-    if (!warp_wait(&bars[BAR_K2_FULL], 0, abort_flag)) return ERR_FWD_OUTPUT;
-    if (nsw0 > 0) build_a(0, 0);
-    if (nsw1 > 0) build_a(1, 0);
-    for (int k = 0; k < nsw0; ++k) {
-        // the A stages first: the tensor cores wait for them, the W accumulators have a unit's slack
-        if (k + 1 < nsw0) {
-            if (!warp_wait(&bars[BAR_A_FREE + 0], k & 1, abort_flag, 1)) return ERR_FWD_OUTPUT;
-            build_a(0, k + 1);
-        }
-        if (k + 1 < nsw1) {
-            if (!warp_wait(&bars[BAR_A_FREE + 1], k & 1, abort_flag, 1)) return ERR_FWD_OUTPUT;
-            build_a(1, k + 1);
-        }
-        if (!drain(0, k, o0, ref0)) return ERR_FWD_OUTPUT;
-        if (k < nsw1 && !drain(1, k, o1, ref1)) return ERR_FWD_OUTPUT;
+    if (staged && !warp_wait(&bars[BAR_WIN_FULL], 0, abort_flag)) return ERR_FWD_OUTPUT;
+    if (g.nsw[0] > 0) build_a(0, 0, nullptr, 0);
+    if (g.nsw[1] > 0) build_a(1, 0, nullptr, 0);
+    for (int k = 0; k < g.nsw[0]; ++k) {
+        // the A rows first: the tensor cores wait for them, the W accumulators have a unit's slack
+        if (k + 1 < g.nsw[0] && !build_a(0, k + 1, &bars[BAR_A_FREE + 0], k & 1)) return ERR_FWD_OUTPUT;
+        if (k + 1 < g.nsw[1] && !build_a(1, k + 1, &bars[BAR_A_FREE + 1], k & 1)) return ERR_FWD_OUTPUT;
+        if (!drain(0, k)) return ERR_FWD_OUTPUT;
+        if (k < g.nsw[1] && !drain(1, k)) return ERR_FWD_OUTPUT;
     }
     return 0;
 }
 
 __device__ __forceinline__ void fwd_rows_sync() { asm volatile("bar.sync 2, 384;" ::: "memory"); }
+__device__ __forceinline__ void fwd_out_sync() { asm volatile("bar.sync 3, 128;" ::: "memory"); }
 
+// Merge of the RE partial results of every query row and the store of out and lse.  `buf`: 128 rows of D + 4
+// floats, then two rows of 128 statistics (the K1/V1 rows, which nothing reads any more).
+template <int D, int RE>
+__device__ __forceinline__ void fwd_store(const FwdParams &P, const FwdGeom &g, const float *buf) {
+    constexpr int LD = D + 4, RI = TQ / RE, PER = D / RE, VEC = PER < 4 ? PER : 4;      // PER channels of a row per thread
+    const KernelParams &kp = P.kp;
+    const int r = threadIdx.x & 127, ii = r & (RI - 1), c0 = (r / RI) * PER, i = g.i0 + ii;
+    if (i >= kp.n) return;
+    __nv_bfloat16 *op = reinterpret_cast<__nv_bfloat16 *>(kp.out.p) + elem_off(kp.out, blockIdx.z, i, blockIdx.y) + c0;
+#pragma unroll
+    for (int c = 0; c < PER; c += VEC) {
+        float x[VEC];
+#pragma unroll
+        for (int z = 0; z < VEC; ++z) x[z] = 0.f;
+#pragma unroll
+        for (int s = 0; s < RE; ++s) {
+            float v[VEC];
+            load_vec<VEC>(buf, (s * RI + ii) * LD + c0 + c, false, v);
+#pragma unroll
+            for (int z = 0; z < VEC; ++z) x[z] += v[z];
+        }
+        store_vec<VEC>(op, c, true, x);
+    }
+}
+
+template <int D>
+__device__ __forceinline__ void fwd_merge(const FwdParams &P, const FwdGeom &g, const uint64_t (&o)[D / 2], float ref_o,
+                                          const float *stats, float *buf, bool bad) {
+    constexpr int LD = D + 4;
+    const KernelParams &kp = P.kp;
+    const int r = threadIdx.x & 127, ii = r & (g.ri - 1), i = g.i0 + ii;
+    float *sM = buf + 128 * LD, *sL = sM + 128;
+    // the row's two denominators are expressed against their groups' last references, o against ref_o
+    const float m0 = stats[768 + r], m1 = stats[896 + r], m = fmaxf(m0, m1);
+    const float f0 = m0 > -CUDART_INF_F ? ex2(m0 - m) : 0.f, f1 = m1 > -CUDART_INF_F ? ex2(m1 - m) : 0.f;
+    sM[r] = m;
+    sL[r] = stats[512 + r] * f0 + stats[640 + r] * f1;
+    fwd_out_sync();
+    float M = -CUDART_INF_F, L = 0.f;
+    for (int s = 0; s < g.re; ++s) M = fmaxf(M, sM[s * g.ri + ii]);
+    for (int s = 0; s < g.re; ++s) {
+        const float ms = sM[s * g.ri + ii];
+        L += ms > -CUDART_INF_F ? sL[s * g.ri + ii] * ex2(ms - M) : 0.f;
+    }
+    // a CTA in which any wait ran out reports NaN
+    const float sc = bad ? CUDART_NAN_F : ref_o > -CUDART_INF_F ? ex2(ref_o - M) / L : 0.f;
+#pragma unroll
+    for (int x = 0; x < D / 4; ++x) {
+        float4 v;
+        f2_unpack(o[2 * x], v.x, v.y);
+        f2_unpack(o[2 * x + 1], v.z, v.w);
+        *reinterpret_cast<float4 *>(buf + r * LD + 4 * x) = make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
+    }
+    if (r < g.ri && i < kp.n)
+        kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = bad ? CUDART_NAN_F : (M + lg2(L)) * 0.6931471805599453f;
+    fwd_out_sync();
+    switch (g.re) {
+        case 2: fwd_store<D, 2>(P, g, buf); break;
+        case 4: fwd_store<D, 4>(P, g, buf); break;
+        case 8: fwd_store<D, 8>(P, g, buf); break;
+        default: fwd_store<D, 16>(P, g, buf); break;
+    }
+}
+
+template <int D>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
-           const __grid_constant__ CUtensorMap mapK2, const FwdParams P) {
+           const __grid_constant__ CUtensorMap mapK2, const __grid_constant__ CUtensorMap mapV2, const FwdParams P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *sK = smem;
-    uint8_t *sV = sK + (size_t)P.nt * TILE_BYTES;
-    uint8_t *sA = sV + (size_t)P.nt * TILE_BYTES;
-    uint8_t *sK2 = sA + 2 * TILE_BYTES;
-    float *stats = reinterpret_cast<float *>(sK2 + K2_ROWS * 128);
+    uint8_t *sV = sK + (size_t)max(P.nslots, 3) * FWD_UNIT_BYTES;
+    uint8_t *sA = sV + (size_t)max(P.nslots, 3) * FWD_UNIT_BYTES;         // [2] one tile per group
+    uint8_t *sWin = sA + 2 * TILE_BYTES;
+    float *stats = reinterpret_cast<float *>(sWin + (size_t)P.win_boxes * 2 * 4096);
     uint64_t *bars = reinterpret_cast<uint64_t *>(stats + FWD_STATS_FLOATS);
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + BAR_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
@@ -505,7 +561,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
         for (int x = 0; x < BAR_COUNT; ++x) {
             const bool many = (x >= BAR_P_FULL && x < BAR_P_FULL + 4) || (x >= BAR_W_EMPTY && x < BAR_W_EMPTY + 2) ||
                               (x >= BAR_A_FULL && x < BAR_A_FULL + 2) || (x >= BAR_REF_FULL && x < BAR_REF_FULL + 2);
-            mbar_init(&bars[x], many ? 128u : 1u);
+            const bool two = x <= BAR_WIN_FULL;          // FULL: the two producers; FREE: one commit from each group
+            mbar_init(&bars[x], many ? 128u : two ? 2u : 1u);
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -528,57 +585,26 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
     if (warp < 4) {
         reg_dealloc<FWD_REGS_ISSUE>();                // one instruction for the whole warpgroup
         if ((threadIdx.x & 31) == 0) {
-            if (warp == 0) {
-                fwd_producer(P, g, &mapK, &mapV, &mapK2, sK, sV, sK2, bars);
-                err = fwd_mma(g, 1, tmem, sK, sV, sA, bars, abort_flag);
-            } else if (warp == 1) {
-                err = fwd_mma(g, 0, tmem, sK, sV, sA, bars, abort_flag);
-            }
+            if (warp < 2) err = fwd_mma<D>(P, g, warp, tmem, sK, sV, sA, bars, abort_flag);
+            else if (warp == 2) err = fwd_producer(P, g, &mapK, &mapK2, sK, sWin, bars, abort_flag);
+            else err = fwd_producer(P, g, &mapV, &mapV2, sV, sWin + (size_t)P.win_boxes * 4096, bars, abort_flag);
         }
         __syncwarp();
     } else if (warp >= 8) {
         reg_dealloc<FWD_REGS_SOFTMAX>();
-        err = fwd_softmax(P, g, (warp - 8) >> 2, tmem, stats, bars, abort_flag);
+        err = fwd_softmax(P, g, (warp - 8) >> 2, tmem, D, stats, bars, abort_flag);
         // the barrier sits outside fwd_softmax so that a group that gave up still reaches it
         fwd_rows_sync();
     } else {
         reg_alloc<FWD_REGS_OUT>();
-        float o0[64], o1[64];
+        uint64_t o[D / 2];
 #pragma unroll
-        for (int x = 0; x < 64; ++x) { o0[x] = 0.f; o1[x] = 0.f; }
-        float ref0 = -CUDART_INF_F, ref1 = -CUDART_INF_F;
-        err = fwd_output(P, g, tmem, o0, o1, ref0, ref1, sA, sK2, stats, bars, abort_flag);
+        for (int x = 0; x < D / 2; ++x) o[x] = 0ull;
+        float ref_o = -CUDART_INF_F;
+        err = fwd_output<D>(P, g, tmem, o, ref_o, sWin, sA, stats, bars, abort_flag);
         fwd_rows_sync();                              // both groups' denominators are in shared memory
-
-        // merge the two groups' states: each accumulator is expressed against its group's last reference
-        const KernelParams &kp = P.kp;
-        const int r = ((warp & 3) * 32) + (threadIdx.x & 31);
-        const int i = g.i0 + r;
-        const float l0 = stats[512 + r], l1 = stats[640 + r];
-        const float lref0 = stats[768 + r], lref1 = stats[896 + r];
-        const float rmax = fmaxf(lref0, lref1);
-        const float f0 = lref0 > -CUDART_INF_F ? ex2(lref0 - rmax) : 0.f;
-        const float f1 = lref1 > -CUDART_INF_F ? ex2(lref1 - rmax) : 0.f;
-        const float l = l0 * f0 + l1 * f1;
-        if (i < kp.n) {
-            // a CTA in which any wait ran out reports NaN instead of leaving its rows unwritten
-            const bool bad = err != 0 || *abort_flag != 0;
-            // an accumulator that last saw an older reference than its group's final one is moved to it
-            const float inv = bad ? CUDART_NAN_F : 1.f / l;
-            const float s0 = ref0 > -CUDART_INF_F ? ex2(ref0 - rmax) * inv : (bad ? inv : 0.f);
-            const float s1 = ref1 > -CUDART_INF_F ? ex2(ref1 - rmax) * inv : (bad ? inv : 0.f);
-            __nv_bfloat16 *op = reinterpret_cast<__nv_bfloat16 *>(kp.out.p) + elem_off(kp.out, blockIdx.z, i, blockIdx.y);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                uint4 v;
-                v.x = pack_bf16(o0[u * 8 + 0] * s0 + o1[u * 8 + 0] * s1, o0[u * 8 + 1] * s0 + o1[u * 8 + 1] * s1);
-                v.y = pack_bf16(o0[u * 8 + 2] * s0 + o1[u * 8 + 2] * s1, o0[u * 8 + 3] * s0 + o1[u * 8 + 3] * s1);
-                v.z = pack_bf16(o0[u * 8 + 4] * s0 + o1[u * 8 + 4] * s1, o0[u * 8 + 5] * s0 + o1[u * 8 + 5] * s1);
-                v.w = pack_bf16(o0[u * 8 + 6] * s0 + o1[u * 8 + 6] * s1, o0[u * 8 + 7] * s0 + o1[u * 8 + 7] * s1);
-                *reinterpret_cast<uint4 *>(op + u * 8) = v;
-            }
-            kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = bad ? CUDART_NAN_F : (rmax + lg2(l)) * 0.6931471805599453f;
-        }
+        if (err) *abort_flag = 1;
+        fwd_merge<D>(P, g, o, ref_o, stats, reinterpret_cast<float *>(sK), err != 0 || *abort_flag != 0);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
@@ -590,6 +616,44 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
         tc_fence_after();
         tmem_dealloc(tmem, 512);
     }
+}
+
+// ------------------------------------------------------------------ host side
+// Query rows per tile.  Measured on a B200: a tile costs ~5500 cycles of set-up, first loads and merge, a 64-key
+// unit ~650 cycles while both softmax groups have sweeps and ~1100 when one works alone.  Fewer rows per tile
+// mean more tiles with fewer sweeps each (a short or thin problem then fills the chip), more set-up and, below 64
+// rows, no fewer units per sweep; the choice is the smallest total over one tile per SM at a time.  The result of
+// a batch element must not depend on the others that ride in the call (to the last bit: callers cut batches into
+// chunks), so the rule assumes four of them: at one element a tile may be twice as long as it could be, at
+// sixteen there may be twice as many tiles as needed.
+inline int fwd_ri_log2(const sa2_shape &s, int sms) {
+    int best = 6;
+    double best_cost = 0.;
+    for (int l = 6; l >= 3; --l) {
+        const int ri = 1 << l, re = TQ >> l;
+        const double tiles = (double)((s.n + ri - 1) / ri) * s.hq * 4.;
+        const int rows = ri < s.n ? ri : s.n;
+        const int keys = s.w1 + rows - 1 < s.n + s.off1 ? s.w1 + rows - 1 : s.n + s.off1;
+        const int units = (keys + FWD_UNIT - 1) / FWD_UNIT;
+        const int w2 = s.w2 < s.n + s.off2 ? s.w2 : s.n + s.off2;
+        const int sweeps = (w2 + re - 1) / re;
+        const double both = sweeps * units * 650., one = ((sweeps + 1) / 2) * units * 1100.;
+        const double waves = tiles > sms ? tiles / sms : 1.;
+        const double cost = waves * (5500. + (both > one ? both : one));
+        if (l == 6 || cost < 0.98 * best_cost) { best = l; best_cost = cost; }
+    }
+    return best;
+}
+inline int fwd_win_boxes(int w2, int ri_log2) {
+    const int rows = w2 + (1 << ri_log2) - 1;
+    return rows <= FWD_WIN_ROWS ? (rows + 31) / 32 : 0;
+}
+// slots for the widest window of a tile, or as many as fit beside everything else
+inline int fwd_slots(int w1, int ri_log2, int win_boxes) {
+    const int units = (w1 + (1 << ri_log2) - 1 + FWD_UNIT - 1) / FWD_UNIT;
+    const size_t fixed = 1024 + (size_t)win_boxes * 8192 + 2 * TILE_BYTES + FWD_STATS_FLOATS * 4 + BAR_COUNT * 8 + 64;
+    const int room = (int)((232448 - fixed) / (2 * FWD_UNIT_BYTES)), most = room < FWD_MAX_SLOTS ? room : FWD_MAX_SLOTS;
+    return units < most ? units : most;
 }
 
 }  // namespace tc

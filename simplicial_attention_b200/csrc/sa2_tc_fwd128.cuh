@@ -40,7 +40,7 @@
 //   12-15  softmax group 0 (even sweeps), 16-19 softmax group 1 (odd sweeps)
 //   20, 21 lane 0 is the TMA producer of the K1 ring / of the V1 ring; 22-23 idle
 #pragma once
-#include "sa2_tc_fwd.cuh"
+#include "sa2_tc_common.cuh"
 
 namespace sa2 {
 namespace tc {
