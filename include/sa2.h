@@ -234,6 +234,47 @@ int sa2_headnorm_fwd(const sa2_headnorm_args *args);
 int sa2_headnorm_bwd(const sa2_headnorm_args *args);
 size_t sa2_headnorm_partial_bytes(int64_t rows, int32_t channels);
 
+/*
+ * The same norm with the module's own five gain vectors (simplicial_mha.py:69-73) instead of one gain per
+ * channel: channels = d * (hq + 4 * hk), laid out as the fused projection is - hq query heads, then per key/value
+ * head its two keys, then per key/value head its two values.  gain[0..4] = q, k, k', v, v', d entries each
+ * (16-byte aligned); the backward writes their gradients, summed over rows and heads, to dgain[0..4] in gain_dtype.
+ * `partial` as for sa2_headnorm_bwd with that many channels.  d must be 32, 64 or 128.
+ */
+typedef struct sa2_qkvnorm_args {
+    const void *x, *dy;
+    void *y;               /* forward: y; backward: dx */
+    float *rstd;           /* [rows][hq + 4 hk] */
+    const void *gain[5];
+    void *dgain[5];        /* backward only */
+    void *partial;         /* backward only */
+    size_t partial_bytes;
+    int64_t rows, x_stride, y_stride, dy_stride;
+    int32_t hq, hk, d;
+    int32_t x_dtype, y_dtype, gain_dtype;
+    float eps;
+    void *stream;
+} sa2_qkvnorm_args;
+
+int sa2_qkvnorm_fwd(const sa2_qkvnorm_args *args);
+int sa2_qkvnorm_bwd(const sa2_qkvnorm_args *args);
+
+/*
+ * Generation: normalises the projection of n new rows of b sequences (args: x, y, gain, rows = b * n; y receives
+ * q as [b][n][hq][d]) and puts it behind the cached rows: set s (k, k', v, v') becomes dst [b][keep + n][hk][d], its
+ * first `keep` rows copied from cache [b][keep][hk][d] (element strides, multiples of 16 bytes).  Stands in for the
+ * norms and the four concatenations of the cached forward; the reference re-runs the whole prefix instead
+ * (train.py:92-111).  x_dtype == y_dtype.
+ */
+typedef struct sa2_append_set {
+    const void *cache;
+    sa2_strides strides;
+    void *dst;
+    int32_t keep;
+} sa2_append_set;
+
+int sa2_qkv_append(const sa2_qkvnorm_args *args, const sa2_append_set sets[4], int32_t b, int32_t n);
+
 #ifdef __cplusplus
 }
 #endif

@@ -20,7 +20,8 @@ BWD_ROWSUM, BWD_K1, BWD_Q = 1, 2, 4     # sa2_bwd_phase
 EXPORTS = ("sa2_fwd", "sa2_bwd", "sa2_bwd_workspace_bytes", "sa2_strerror", "sa2_version",
            "sa2_kernel_launches", "sa2_device_status", "sa2_check_device", "sa2_selftest_wait",
            "sa2_bwd_static_scratch",
-           "sa2_headnorm_fwd", "sa2_headnorm_bwd", "sa2_headnorm_partial_bytes")
+           "sa2_headnorm_fwd", "sa2_headnorm_bwd", "sa2_headnorm_partial_bytes",
+           "sa2_qkvnorm_fwd", "sa2_qkvnorm_bwd", "sa2_qkv_append")
 STATIC_SCRATCH_ROWS = 262144   # SA2_STATIC_SCRATCH_ROWS in include/sa2.h
 SELFTEST_WAIT_BIT = 0x10000    # SA2_SELFTEST_WAIT_BIT
 SA2_ERR_DEVICE = 5
@@ -123,6 +124,32 @@ def lib() -> C.CDLL:
         handle.sa2_version.restype = C.c_int
         _lib = handle
     return _lib
+
+
+_ext = None
+
+
+def ext():
+    """The native host path (``csrc/sa2_torch.cpp``), bound to the loaded library's entry points."""
+    global _ext
+    if _ext is not None:
+        return _ext
+    handle = lib()
+    with _lock:
+        if _ext is not None:
+            return _ext
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries must be loaded first)
+
+        from . import build
+        path = build.build_ext()
+        spec = importlib.util.spec_from_file_location("_sa2_torch", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in EXPORTS})
+        _ext = module
+    return _ext
 
 
 class Sa2Error(RuntimeError):

@@ -173,6 +173,17 @@ class SlidingTwoSimplicialAttention(Function):
     extend it; with ``return_lse`` the result is ``(out, lse)``."""
 
     @staticmethod
+    def apply(q, k1, k2, v1, v2, w1=512, w2=32, causal=True, scale=None, kernel="auto", return_lse=False):
+        """Runs the node of the native host path, which does what ``forward`` and ``backward`` below do in Python
+        (a forward + backward pair cost the host 280 us there, more than the kernels of a short sequence)."""
+        assert causal, "only the causal sliding-window form is implemented (the reference's module always passes causal=True)"
+        res = _lib.ext().attn(q, k1, k2, v1, v2, int(w1), int(w2), None if scale is None else float(scale), _lib.KERNELS[kernel], bool(return_lse))
+        if res is None:
+            _check_inputs(q, k1, k2, v1, v2)
+            raise ValueError("unsupported inputs")
+        return res
+
+    @staticmethod
     def forward(ctx, q, k1, k2, v1, v2, w1=512, w2=32, causal=True, scale=None, kernel="auto", return_lse=False):
         assert causal, "only the causal sliding-window form is implemented (the reference's module always passes causal=True)"
         out, lse = sa2_forward(q, k1, k2, v1, v2, w1, w2, scale, kernel)

@@ -1,8 +1,9 @@
-"""Build the CUDA library in-tree with nvcc for sm_100a.
+"""Build the CUDA library in-tree with nvcc for sm_100a, and the native host path beside it.
 
     python -m simplicial_attention_b200.build [--force] [--verbose]
 
-Produces ``simplicial_attention_b200/libsa2.so`` (C ABI in ``include/sa2.h``).
+Produces ``simplicial_attention_b200/libsa2.so`` (C ABI in ``include/sa2.h``) and ``_sa2_torch.so`` (the argument
+blocks, allocations and autograd nodes of the Python entry points in C++, against torch's headers).
 nvcc cross-compiles without a GPU, so this also serves as the build check.
 """
 from __future__ import annotations
@@ -16,6 +17,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libsa2.so")
+EXT = os.path.join(PKG, "_sa2_torch.so")
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -32,7 +34,7 @@ def sources() -> list[str]:
 
 
 def _inputs() -> list[str]:
-    files = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    files = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith(".cpp")]
     files.append(os.path.join(ROOT, "include", "sa2.h"))
     files.append(os.path.abspath(__file__))
     return files
@@ -43,6 +45,39 @@ def is_stale() -> bool:
         return True
     t = os.path.getmtime(LIB)
     return any(os.path.getmtime(f) > t for f in _inputs())
+
+
+def ext_is_stale() -> bool:
+    if not os.path.exists(EXT):
+        return True
+    t = os.path.getmtime(EXT)
+    return any(os.path.getmtime(f) > t for f in (os.path.join(CSRC, "sa2_torch.cpp"), os.path.join(ROOT, "include", "sa2.h"),
+                                                 os.path.abspath(__file__)))
+
+
+def build_ext(force: bool = False) -> str:
+    """Compile _sa2_torch.so if it is missing or older than its sources (host code only, so g++)."""
+    if not force and not ext_is_stale():
+        return EXT
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    includes = [os.path.join(ROOT, "include"), *cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    tmp = EXT + f".{os.getpid()}.tmp"
+    cmd = [
+        shutil.which("g++") or "g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-DTORCH_EXTENSION_NAME=_sa2_torch", "-DTORCH_API_INCLUDE_EXTENSION_H",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[x for d in includes for x in ("-isystem", d)],
+        os.path.join(CSRC, "sa2_torch.cpp"), "-o", tmp,
+        "-L" + lib_dir, "-Wl,-rpath," + lib_dir, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python",
+    ]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
+    os.replace(tmp, EXT)
+    return EXT
 
 
 def build(force: bool = False, verbose: bool = False, out: str = LIB, defines: tuple[str, ...] = ()) -> str:
@@ -70,3 +105,4 @@ def build(force: bool = False, verbose: bool = False, out: str = LIB, defines: t
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_ext(force="--force" in sys.argv))

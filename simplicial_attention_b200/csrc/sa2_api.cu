@@ -343,53 +343,118 @@ int headnorm_check(const sa2_headnorm_args *a, bool backward) {
     return SA2_OK;
 }
 
-template <typename TX, typename TY>
-int headnorm_launch(const sa2_headnorm_args *a, const sa2::headnorm::Params &P, bool backward) {
+using sa2::headnorm::Gains;
+using sa2::headnorm::GainGrads;
+
+inline int rows_aligned(const void *p, int64_t stride, int dtype) {
+    return aligned16(p) && stride % (dtype == SA2_BF16 ? 8 : 4) == 0;
+}
+
+template <typename TX, typename TY, int D>
+int headnorm_run(const sa2::headnorm::Params &P, bool backward, float *dtable, const GainGrads &grads, cudaStream_t st) {
     using namespace sa2::headnorm;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
+    const int segs = (P.channels + Seg<D>::CH - 1) / Seg<D>::CH;
     if (!backward) {
-        const int64_t pairs = a->rows * (a->channels / a->d);
-        const int grid = (int)((pairs + WARPS - 1) / WARPS < 148 * 16 ? (pairs + WARPS - 1) / WARPS : 148 * 16);
-        if (a->d == 32) fwd_kernel<TX, TY, 1><<<grid, WARPS * 32, 0, st>>>(P);
-        else if (a->d == 64) fwd_kernel<TX, TY, 2><<<grid, WARPS * 32, 0, st>>>(P);
-        else if (a->d == 128) fwd_kernel<TX, TY, 4><<<grid, WARPS * 32, 0, st>>>(P);
-        else if (a->d == 256) fwd_kernel<TX, TY, 8><<<grid, WARPS * 32, 0, st>>>(P);
-        else fwd_kernel<TX, TY, 16><<<grid, WARPS * 32, 0, st>>>(P);
-    } else {
-        const int grid = headnorm_grid(a->rows);
-        const size_t smem = (size_t)WARPS * a->channels * sizeof(float);
-        auto run = [&](auto kern) -> int {
-            if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SA2_ERR_CUDA;
-            kern<<<grid, WARPS * 32, smem, st>>>(P);
-            return SA2_OK;
-        };
-        int rc;
-        if (a->d == 32) rc = run(bwd_kernel<TX, TY, 1>);
-        else if (a->d == 64) rc = run(bwd_kernel<TX, TY, 2>);
-        else if (a->d == 128) rc = run(bwd_kernel<TX, TY, 4>);
-        else if (a->d == 256) rc = run(bwd_kernel<TX, TY, 8>);
-        else rc = run(bwd_kernel<TX, TY, 16>);
-        if (rc != SA2_OK) return rc;
-        dweight_reduce_kernel<<<(a->channels + 31) / 32, 256, 0, st>>>(P.partial, a->dweight, grid, a->channels);
+        const int64_t blocks = (P.rows * segs + 7) / 8;
+        fwd_kernel<TX, TY, D><<<(unsigned)(blocks < 148 * 64 ? blocks : 148 * 64), 256, 0, st>>>(P);
+        return launch_status();
     }
-    return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
+    const int grid = headnorm_grid(P.rows);
+    const int rpc = segs >= 8 ? 1 : 8 / segs;
+    const size_t smem = (size_t)(rpc - 1) * P.channels * sizeof(float);
+    bwd_kernel<TX, TY, D><<<grid, 32 * segs * rpc, smem, st>>>(P);        // at most 7/8 * 8 warps * 2 KB of shared memory
+    if (int e = launch_status()) return e;
+    const dim3 rgrid = dtable ? dim3((P.channels + 31) / 32) : dim3(D / 32, 5);
+    dgain_reduce_kernel<<<rgrid, 1024, 0, st>>>(P.partial, dtable, grads, P.gains, grid, P.channels, D);
+    return launch_status();
+}
+
+template <typename TX, typename TY>
+int headnorm_launch(const sa2::headnorm::Params &P, int d, bool backward, float *dtable, const GainGrads &grads, cudaStream_t st) {
+    switch (d) {
+        case 32: return headnorm_run<TX, TY, 32>(P, backward, dtable, grads, st);
+        case 64: return headnorm_run<TX, TY, 64>(P, backward, dtable, grads, st);
+        case 128: return headnorm_run<TX, TY, 128>(P, backward, dtable, grads, st);
+        case 256: return headnorm_run<TX, TY, 256>(P, backward, dtable, grads, st);
+        default: return headnorm_run<TX, TY, 512>(P, backward, dtable, grads, st);
+    }
+}
+
+int headnorm_types(const sa2::headnorm::Params &P, int d, int x_dtype, int y_dtype, bool backward, float *dtable,
+                   const GainGrads &grads, cudaStream_t st) {
+    // a CTA of the backward spans a row: 32 warps of 256 channels
+    if (backward && P.channels > 6400) return SA2_ERR_UNSUPPORTED;
+    const bool xb = x_dtype == SA2_BF16, yb = y_dtype == SA2_BF16;
+    if (xb && yb) return headnorm_launch<__nv_bfloat16, __nv_bfloat16>(P, d, backward, dtable, grads, st);
+    if (xb) return headnorm_launch<__nv_bfloat16, float>(P, d, backward, dtable, grads, st);
+    if (yb) return headnorm_launch<float, __nv_bfloat16>(P, d, backward, dtable, grads, st);
+    return headnorm_launch<float, float>(P, d, backward, dtable, grads, st);
 }
 
 int headnorm_dispatch(const sa2_headnorm_args *a, bool backward) {
     const int rc = headnorm_check(a, backward);
     if (rc != SA2_OK) return rc;
-    // only the backward keeps per-warp partial rows of the gain gradient in shared memory
-    if (backward && (size_t)sa2::headnorm::WARPS * a->channels * sizeof(float) > 200 * 1024) return SA2_ERR_UNSUPPORTED;
-    sa2::headnorm::Params P;
-    P.x = a->x; P.dy = a->dy; P.weight = a->weight; P.y = a->y; P.rstd = a->rstd;
+    sa2::headnorm::Params P{};
+    P.x = a->x; P.dy = a->dy; P.y = a->y; P.rstd = a->rstd;
+    P.gains.table = a->weight;
+    P.gains.al = aligned16(a->weight);
     P.partial = reinterpret_cast<float *>(a->partial);
     P.rows = a->rows; P.x_stride = a->x_stride; P.y_stride = a->y_stride; P.dy_stride = a->dy_stride;
-    P.channels = a->channels; P.d = a->d; P.eps = a->eps;
-    const bool xb = a->x_dtype == SA2_BF16, yb = a->y_dtype == SA2_BF16;
-    if (xb && yb) return headnorm_launch<__nv_bfloat16, __nv_bfloat16>(a, P, backward);
-    if (xb) return headnorm_launch<__nv_bfloat16, float>(a, P, backward);
-    if (yb) return headnorm_launch<float, __nv_bfloat16>(a, P, backward);
-    return headnorm_launch<float, float>(a, P, backward);
+    P.channels = a->channels; P.eps = a->eps;
+    P.x_al = rows_aligned(a->x, a->x_stride, a->x_dtype);
+    P.y_al = rows_aligned(a->y, a->y_stride, backward ? a->x_dtype : a->y_dtype);
+    P.dy_al = backward && rows_aligned(a->dy, a->dy_stride, a->y_dtype);
+    return headnorm_types(P, a->d, a->x_dtype, a->y_dtype, backward, a->dweight, GainGrads{}, reinterpret_cast<cudaStream_t>(a->stream));
+}
+
+int qkvnorm_fill(const sa2_qkvnorm_args *a, bool backward, sa2::headnorm::Params &P, GainGrads &grads) {
+    if (!a || !a->x || !a->y || a->rows <= 0 || a->hq <= 0 || a->hk <= 0) return SA2_ERR_INVALID;
+    if (a->d != 32 && a->d != 64 && a->d != 128) return SA2_ERR_UNSUPPORTED;
+    for (int dt : {a->x_dtype, a->y_dtype, a->gain_dtype})
+        if (dt != SA2_F32 && dt != SA2_BF16) return SA2_ERR_UNSUPPORTED;
+    const int64_t channels = (int64_t)a->d * (a->hq + 4LL * a->hk);
+    if (channels > 1 << 20 || a->x_stride < channels) return SA2_ERR_INVALID;
+    P = sa2::headnorm::Params{};
+    grads = GainGrads{};
+    for (int v = 0; v < 5; ++v) {
+        if (!a->gain[v] || !aligned16(a->gain[v])) return SA2_ERR_INVALID;
+        P.gains.p[v] = a->gain[v];
+        grads.p[v] = a->dgain[v];
+        if (backward && !a->dgain[v]) return SA2_ERR_INVALID;
+    }
+    P.gains.bf16 = grads.bf16 = a->gain_dtype == SA2_BF16;
+    P.gains.hq = a->hq; P.gains.hk = a->hk;
+    P.x = a->x; P.dy = a->dy; P.y = a->y; P.rstd = a->rstd;
+    P.partial = reinterpret_cast<float *>(a->partial);
+    P.rows = a->rows; P.x_stride = a->x_stride; P.y_stride = a->y_stride; P.dy_stride = a->dy_stride;
+    P.channels = (int)channels; P.eps = a->eps;
+    P.x_al = rows_aligned(a->x, a->x_stride, a->x_dtype);
+    P.y_al = rows_aligned(a->y, a->y_stride, backward ? a->x_dtype : a->y_dtype);
+    P.dy_al = backward && rows_aligned(a->dy, a->dy_stride, a->y_dtype);
+    return SA2_OK;
+}
+
+int qkvnorm_dispatch(const sa2_qkvnorm_args *a, bool backward) {
+    sa2::headnorm::Params P;
+    GainGrads grads;
+    if (int e = qkvnorm_fill(a, backward, P, grads)) return e;
+    if (!a->rstd || a->y_stride < P.channels) return SA2_ERR_INVALID;
+    if (backward) {
+        if (!a->dy || a->dy_stride < P.channels) return SA2_ERR_INVALID;
+        if (!a->partial || a->partial_bytes < sa2_headnorm_partial_bytes(a->rows, P.channels)) return SA2_ERR_WORKSPACE;
+    }
+    return headnorm_types(P, a->d, a->x_dtype, a->y_dtype, backward, nullptr, grads, reinterpret_cast<cudaStream_t>(a->stream));
+}
+
+template <typename T>
+int append_launch(const sa2::headnorm::AppendParams &A, int d, cudaStream_t st) {
+    using namespace sa2::headnorm;
+    const int64_t want = (A.copy_items + 1023) / 1024;           // four pieces per thread
+    const unsigned grid = (unsigned)((A.norm_items + 7) / 8 + (want < 148 * 8 ? want : 148 * 8));
+    if (d == 32) append_kernel<T, 32><<<grid, 256, 0, st>>>(A);
+    else if (d == 64) append_kernel<T, 64><<<grid, 256, 0, st>>>(A);
+    else append_kernel<T, 128><<<grid, 256, 0, st>>>(A);
+    return launch_status();
 }
 
 }  // namespace
@@ -407,6 +472,37 @@ int sa2_headnorm_fwd(const sa2_headnorm_args *a) {
 int sa2_headnorm_bwd(const sa2_headnorm_args *a) {
     sa2::nvtx::Range range("sa2_headnorm_bwd");
     return headnorm_dispatch(a, true);
+}
+
+int sa2_qkvnorm_fwd(const sa2_qkvnorm_args *a) {
+    sa2::nvtx::Range range("sa2_qkvnorm_fwd");
+    return qkvnorm_dispatch(a, false);
+}
+int sa2_qkvnorm_bwd(const sa2_qkvnorm_args *a) {
+    sa2::nvtx::Range range("sa2_qkvnorm_bwd");
+    return qkvnorm_dispatch(a, true);
+}
+int sa2_qkv_append(const sa2_qkvnorm_args *a, const sa2_append_set *sets, int32_t b, int32_t n) {
+    sa2::nvtx::Range range("sa2_qkv_append");
+    sa2::headnorm::AppendParams A{};
+    GainGrads grads;
+    if (int e = qkvnorm_fill(a, false, A.norm, grads)) return e;
+    if (!sets || b <= 0 || n <= 0 || a->rows != (int64_t)b * n || a->x_dtype != a->y_dtype || !aligned16(a->y)) return SA2_ERR_INVALID;
+    const int piece = a->x_dtype == SA2_BF16 ? 8 : 4;
+    const int64_t segs = (A.norm.channels + 255) / 256, items = a->rows * segs;
+    if (items > 1 << 28) return SA2_ERR_UNSUPPORTED;
+    A.b = b; A.n = n; A.hq = a->hq; A.hk = a->hk;
+    A.norm_items = (int)items;
+    for (int s = 0; s < 4; ++s) {
+        const sa2_append_set &t = sets[s];
+        if (t.keep < 0 || !t.dst || !aligned16(t.dst)) return SA2_ERR_INVALID;
+        if (t.keep > 0 && (!t.cache || !aligned16(t.cache) || t.strides.batch % piece || t.strides.seq % piece || t.strides.head % piece))
+            return SA2_ERR_INVALID;
+        A.set[s] = sa2::headnorm::AppendSet{t.cache, t.strides.batch, t.strides.seq, t.strides.head, t.dst, t.keep};
+        A.copy_items += (int64_t)b * t.keep * a->hk * (a->d / piece);
+    }
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
+    return a->x_dtype == SA2_BF16 ? append_launch<__nv_bfloat16>(A, a->d, st) : append_launch<float>(A, a->d, st);
 }
 
 }  // extern "C"

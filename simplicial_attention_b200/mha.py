@@ -18,6 +18,7 @@ from typing import Callable
 import torch
 from torch.nn import Identity, Linear, Module, ModuleList, RMSNorm
 
+from . import _lib
 from .attention import divisible_by, exists, sliding_two_simplicial_attn
 from .headnorm import RMSNorm as RowRMSNorm
 
@@ -99,8 +100,6 @@ class HigherOrderAttention(Module):
     def _fused_norm(self, proj):
         """Per-head RMSNorm of the packed projection with the gains of q_norm / k_norms / v_norms tiled to
         one entry per channel; same arithmetic as the modules, applied before the split."""
-        import torch
-
         from .headnorm import head_rmsnorm
         kw = torch.cat([n.weight for n in self.k_norms]).repeat(self.key_value_heads)
         vw = torch.cat([n.weight for n in self.v_norms]).repeat(self.key_value_heads)
@@ -114,8 +113,9 @@ class HigherOrderAttention(Module):
 
     def _project(self, tokens):
         """tokens -> (queries, keys, values) after the head split and the per-head norms."""
-        tokens = self.prenorm(tokens)
-        proj = self.to_qkv(tokens)
+        return self._split_heads(self.to_qkv(self.prenorm(tokens)))
+
+    def _split_heads(self, proj):
         fused = (self.fused_head_norm and self.qk_rmsnorm and proj.is_cuda and not self.head_first_dim
                  and self.dim_head_values == self.dim_head and self.dim_head in (32, 64, 128)
                  and proj.shape[-1] <= self.fused_head_norm_max_channels
@@ -166,13 +166,56 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
         super().__init__(*args, number_key_value_sets=2, head_first_dim=False, attend=attend, **kwargs)
         self.w1, self.w2 = w1, w2
 
+    def _fused_call(self, proj):
+        """Arguments of the native calls that take the packed projection as a whole - norm and attention forward and
+        backward without splitting or concatenating it - or None where the general path is needed."""
+        at = self.attend
+        if not (self.fused_head_norm and self.qk_rmsnorm and proj.is_cuda and isinstance(at, partial)
+                and at.func is sliding_two_simplicial_attn and not at.args
+                and at.keywords.keys() <= {"w1", "w2", "causal", "kernel"} and at.keywords.get("causal", True)):
+            return None
+        autocast = torch.is_autocast_enabled()
+        norms = (self.q_norm, *self.k_norms, *self.v_norms)
+        eps = self.q_norm.eps
+        if any(n.eps != eps for n in norms):
+            return None
+        # the modules leave eps unset: the machine epsilon of the dtype they compute in (fp32 under autocast)
+        if eps is None:
+            eps = torch.finfo(torch.float32 if autocast else proj.dtype).eps
+        dtype = torch.get_autocast_dtype("cuda") if autocast else proj.dtype
+        return ([n.weight for n in norms], (self.heads, self.key_value_heads, self.dim_head, eps), dtype,
+                (at.keywords.get("w1", 512), at.keywords.get("w2", 32), _lib.KERNELS[at.keywords.get("kernel", "auto")]))
+
+    def _attend_packed(self, tokens):
+        """The attention output before the heads are combined, or the projection when the general path has to run."""
+        proj = self.to_qkv(self.prenorm(tokens))
+        call = self._fused_call(proj)
+        if call is None:
+            return proj, None
+        gains, heads, dtype, windows = call
+        return proj, _lib.ext().qkv_attn(proj, gains, *heads, dtype, *windows)
+
     def forward(self, tokens, cache=None, return_cache=False):
         """``cache`` (from an earlier call with ``return_cache=True``) holds the last ``w1 - 1`` rows of the
         first key/value set and the last ``w2 - 1`` rows of the second: all a later token can still see.
         With a cache, ``tokens`` are only the new positions; the cached rows ride in front of the new keys
         as the halo the kernels already understand, so decoding a token costs one window, not the prefix
         (the reference's sampling loop re-runs the whole prefix for every token, train.py:103-104)."""
-        queries, keys, values = self._project(tokens)
+        if cache is None and not return_cache:
+            proj, out = self._attend_packed(tokens)
+            if out is not None:
+                return self._merge(out)
+            queries, keys, values = self._split_heads(proj)
+            return self._merge(self.attend(queries, keys, values))
+        proj = self.to_qkv(self.prenorm(tokens))
+        if cache is not None and return_cache and not torch.is_grad_enabled():
+            call = self._fused_call(proj)
+            if call is not None and call[2] == proj.dtype and call[3][:2] == (self.w1, self.w2):
+                gains, heads, _, windows = call
+                res = _lib.ext().qkv_attn_cached(proj, gains, [*cache[0], *cache[1]], *heads, *windows)
+                if res is not None:
+                    return self._merge(res[0]), ((res[1], res[2]), (res[3], res[4]))
+        queries, keys, values = self._split_heads(proj)
         if cache is not None:
             keys = tuple(torch.cat((c, t), dim=1) for c, t in zip(cache[0], keys))
             values = tuple(torch.cat((c, t), dim=1) for c, t in zip(cache[1], values))
