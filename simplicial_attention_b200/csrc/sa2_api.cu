@@ -49,51 +49,19 @@ void fill_common(KernelParams &p, const sa2_shape &s) {
     p.scale = s.scale;
 }
 
-template <typename K>
-int set_smem(K kernel, size_t bytes) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess
-               ? SA2_OK : SA2_ERR_CUDA;
-}
-
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA; }
 
 template <int D>
 int simt_fwd(const KernelParams &p, cudaStream_t st) {
-    using namespace sa2::simt;
-    auto k = row_kernel<D, MODE_FWD>;
-    if (int e = set_smem(k, Cfg<D>::smem_fwd)) return e;
-    dim3 grid((p.n + TILE - 1) / TILE, p.hq, p.b);
-    k<<<grid, NTHREADS, Cfg<D>::smem_fwd, st>>>(p);
-    return launch_status();
+    return sa2::simt::launch_fwd<D>(p, sa2::tc::SM_COUNT, st) ? SA2_OK : SA2_ERR_CUDA;
 }
 
 template <int D>
 int simt_bwd(const KernelParams &p, cudaStream_t st, int phases = 0) {
-    using namespace sa2::simt;
     if (phases == 0) phases = SA2_BWD_ROWSUM | SA2_BWD_K1 | SA2_BWD_Q;
-    if (phases & SA2_BWD_ROWSUM) {
-        const int64_t rows = (int64_t)p.b * p.n * p.hq;
-        delta_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>(p, D);
-        if (int e = launch_status()) return e;
-    }
-
-    auto kq = row_kernel<D, MODE_BWD_Q>;
-    auto kk2 = row_kernel<D, MODE_BWD_K2>;
-    auto kk1 = k1_kernel<D>;
-    if (int e = set_smem(kq, Cfg<D>::smem_bwd)) return e;
-    if (int e = set_smem(kk2, Cfg<D>::smem_bwd)) return e;
-    if (int e = set_smem(kk1, Cfg<D>::smem_bwd)) return e;
-
-    if (phases & SA2_BWD_Q) {
-        kq<<<dim3((p.n + TILE - 1) / TILE, p.hq, p.b), NTHREADS, Cfg<D>::smem_bwd, st>>>(p);
-        if (int e = launch_status()) return e;
-        kk2<<<dim3((p.nk2 + TILE - 1) / TILE, p.hk, p.b), NTHREADS, Cfg<D>::smem_bwd, st>>>(p);
-        if (int e = launch_status()) return e;
-    }
-    if (phases & SA2_BWD_K1) {
-        kk1<<<dim3((p.nk1 + TILE - 1) / TILE, p.hk, p.b), NTHREADS, Cfg<D>::smem_bwd, st>>>(p);
-        return launch_status();
-    }
+    if ((phases & SA2_BWD_ROWSUM) && !sa2::simt::launch_delta<D>(p, st)) return SA2_ERR_CUDA;
+    const bool q = phases & SA2_BWD_Q, k1 = phases & SA2_BWD_K1;
+    if ((q || k1) && !sa2::simt::launch_bwd<D>(p, q, q, k1, sa2::tc::SM_COUNT, st)) return SA2_ERR_CUDA;
     return SA2_OK;
 }
 
@@ -200,7 +168,7 @@ int sa2_kernel_launches(const sa2_shape *s, int backward) {
     const bool tc_ok = backward ? sa2::tc::bwd_supported(*s) : sa2::tc::fwd_supported(*s);
     if (s->kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
     if (tc_ok && s->kernel != SA2_KERNEL_SIMT) return sa2::tc::launches(*s, backward != 0);
-    return backward ? 4 : 1;   // SIMT: delta + dQ + dK2/dV2 + dK1/dV1
+    return backward ? 2 : 1;   // SIMT: row sums + all gradients
 }
 
 size_t sa2_bwd_workspace_bytes(const sa2_shape *s) {

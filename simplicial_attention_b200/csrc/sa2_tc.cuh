@@ -41,8 +41,8 @@ inline size_t bwd_extra_workspace_bytes(const sa2_shape &s) {
     return align256(bq_part_dq_bytes(s, ns)) + align256(bq_part_k2_bytes(s, ns));
 }
 // forward: 1 kernel; backward: D = rowsum(O*dO), dK1/dV1, dQ/dK2/dV2 partials, their reduction
-// (or, when w2 is too large for the shared accumulators, two fp32 kernels for dQ and dK2/dV2)
-inline int launches(const sa2_shape &, bool backward) { return backward ? 4 : 1; }
+// (or, when w2 is too large for the shared accumulators, one fp32 launch for dQ and dK2/dV2)
+inline int launches(const sa2_shape &s, bool backward) { return !backward ? 1 : bq_supported(s) ? 4 : 3; }
 
 inline bool tma_addressable(const TensorRef &t) {
     return (reinterpret_cast<uintptr_t>(t.p) & 15u) == 0 && t.sb % 8 == 0 && t.sn % 8 == 0 && t.sh % 8 == 0;
@@ -157,19 +157,10 @@ inline int bwd_q_launch(const KernelParams &kp, const sa2_shape &s, const CUtens
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
+// dQ and dK2/dV2 in fp32 (second-key windows too long for the shared accumulators)
 template <int D>
 inline int bwd_q_simt(const KernelParams &kp, cudaStream_t st) {
-    // dQ and dK2/dV2: fp32 SIMT kernels (second-key windows too long for the shared accumulators)
-    using namespace sa2::simt;
-    auto kq = row_kernel<D, MODE_BWD_Q>;
-    auto kk2 = row_kernel<D, MODE_BWD_K2>;
-    if (cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<D>::smem_bwd) != cudaSuccess ||
-        cudaFuncSetAttribute(kk2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<D>::smem_bwd) != cudaSuccess)
-        return SA2_ERR_CUDA;
-    kq<<<dim3((kp.n + TILE - 1) / TILE, kp.hq, kp.b), NTHREADS, Cfg<D>::smem_bwd, st>>>(kp);
-    if (cudaGetLastError() != cudaSuccess) return SA2_ERR_CUDA;
-    kk2<<<dim3((kp.nk2 + TILE - 1) / TILE, kp.hk, kp.b), NTHREADS, Cfg<D>::smem_bwd, st>>>(kp);
-    return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
+    return simt::launch_bwd<D>(kp, true, true, false, SM_COUNT, st) ? SA2_OK : SA2_ERR_CUDA;
 }
 
 inline int bwd(const KernelParams &kp, const sa2_shape &s, void *extra, cudaStream_t st, int phases = 0) {
@@ -181,9 +172,7 @@ inline int bwd(const KernelParams &kp, const sa2_shape &s, void *extra, cudaStre
 
     // D_i = sum_c O_ic dO_ic
     if (phases & SA2_BWD_ROWSUM) {
-        const int64_t rows = (int64_t)kp.b * kp.n * kp.hq;
-        simt::delta_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>(kp, s.d);
-        if (cudaGetLastError() != cudaSuccess) return SA2_ERR_CUDA;
+        if (!(s.d == 128 ? simt::launch_delta<128>(kp, st) : simt::launch_delta<64>(kp, st))) return SA2_ERR_CUDA;
     }
 
     // 128-row, 64-channel boxes of K1 / V1 (a head-dim-128 tile is two boxes)
