@@ -18,6 +18,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The dynamic shared memory from its first 1024-byte boundary on, as an offset from the array: an address rounded up
+// as an integer would make every access behind it a generic one (64-bit address, address-space test).
+__device__ __forceinline__ uint8_t *align_smem(uint8_t *raw) { return raw + ((0u - smem_u32(raw)) & 1023u); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -102,6 +106,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     }
     SA2_PROF_ADD(prof, clock64() - t0);
     return true;
+}
+
+// One lane of a converged warp.  The roles that issue tcgen05 and TMA instructions run as whole warps and elect the
+// issuing lane per batch: the compiler then knows that the operands (descriptors, TMEM and barrier addresses) are the
+// same for the warp and keeps them in uniform registers.  Under a per-lane branch (lane == 0) every instruction is
+// preceded by moves of its operands into uniform registers: 62 cycles per tcgen05.mma of N = 64 instead of 42 to 52
+// (one issuing thread, M = 128).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+    return pred != 0;
+}
+// The wait of such a role: every lane waits, and the result is the same for all.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag, unsigned sleep_ns = 0, int prof = -1) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, sleep_ns, prof));
 }
 
 // make generic-proxy writes to shared memory visible to the async proxy (TMA, tcgen05.mma)

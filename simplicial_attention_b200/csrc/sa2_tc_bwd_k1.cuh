@@ -219,7 +219,7 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
     const uint64_t dT = smem_desc_sw128(smem_u32(sKV));
     const uint64_t dAB = smem_desc_sw128(smem_u32(sAB + which * TILE_BYTES));
     const uint64_t dSt = smem_desc_sw128(smem_u32(sStat)), dOnes = smem_desc_sw128(smem_u32(sOnes));
-    if (!mbar_wait(&bars[BK1_KV_FULL], 0, abort_flag)) return ERR_BK1_MMA;
+    if (!mbar_wait_warp(&bars[BK1_KV_FULL], 0, abort_flag)) return ERR_BK1_MMA;
     int s = 0, tile_counter = 0;
     for (int hh = 0; hh < kp.g; ++hh) {
         for (int t = 0; t < g.n_it; ++t, ++tile_counter) {
@@ -228,21 +228,23 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
             const uint64_t stL0 = dSt + (uint64_t)((((tile_counter >> 1) & 1) * TILE_BYTES) >> 4) + (uint64_t)((tile_counter & 1) * 4);
             for (int e = 0; e < ne; ++e, ++s) {
                 const int stage = s % BK1_STAGES;
-                if (!mbar_wait(&bars[BK1_AB_FULL + stage], (s / BK1_STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
+                if (!mbar_wait_warp(&bars[BK1_AB_FULL + stage], (s / BK1_STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     // the compute group must have read the previous step's S^T / dP^T of this half
-                    if (s >= 1 && !mbar_wait(&bars[BK1_P_FULL + half], (s - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
+                    if (s >= 1 && !mbar_wait_warp(&bars[BK1_P_FULL + half], (s - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
                     tc_fence_after();
                     const uint64_t a = dAB + (uint64_t)((stage * 2 * TILE_BYTES + half * 8192) >> 4);
                     const uint64_t st = stL0 + (uint64_t)((half * 8192) >> 4) + (uint64_t)(which * 2);
                     const uint32_t d = tmem + half * 128 + which * 64;
+                    if (elect_one()) {
                     mma_ss(d, dT, a, IDESC_F, 0u);
                     mma_ss(d, dT + 2, a + 2, IDESC_F, 1u);
                     mma_ss(d, dT + 4, a + 4, IDESC_F, 1u);
                     mma_ss(d, dT + 6, a + 6, IDESC_F, 1u);
                     mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
                     tc_commit(&bars[BK1_S_FULL + half]);
+                    }
                 }
             }
         }
@@ -258,11 +260,12 @@ __device__ __forceinline__ int bk1_mma_second(const Bk1Geom &g, uint32_t tmem, u
         const int stage = s % BK1_STAGES;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            if (!mbar_wait(&bars[BK1_P_FULL + half], s & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
+            if (!mbar_wait_warp(&bars[BK1_P_FULL + half], s & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
             tc_fence_after();
             const uint64_t a = dAB + (uint64_t)((stage * 2 * TILE_BYTES + half * 8192) >> 4), bq = a + (TILE_BYTES >> 4);
             const uint32_t t = tmem + 256 + half * 64;
             const uint32_t first = (s > 0 || half > 0) ? 1u : 0u;
+            if (elect_one()) {
             mma_ts(tmem + 448, t, bq, IDESC_G, first);
             mma_ts(tmem + 448, t + 8, bq + 128, IDESC_G, 1u);
             mma_ts(tmem + 448, t + 16, bq + 256, IDESC_G, 1u);
@@ -272,10 +275,11 @@ __device__ __forceinline__ int bk1_mma_second(const Bk1Geom &g, uint32_t tmem, u
             mma_ts(tmem + 384, t + 48, a + 256, IDESC_G, 1u);
             mma_ts(tmem + 384, t + 56, a + 384, IDESC_G, 1u);
             tc_commit(&bars[BK1_G_DONE + half]);
+            if (half == 1) tc_commit(&bars[BK1_AB_EMPTY + stage]);
+            }
         }
-        tc_commit(&bars[BK1_AB_EMPTY + stage]);
     }
-    tc_commit(&bars[BK1_DONE]);
+    if (elect_one()) tc_commit(&bars[BK1_DONE]);
     return 0;
 }
 
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(BK1_THREADS, 1)
 bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
               const __grid_constant__ CUtensorMap mapK2, const __grid_constant__ CUtensorMap mapV2, const BwdParams P) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;
     uint8_t *sV = sK + TILE_BYTES;
     uint8_t *sAB = sV + TILE_BYTES;                       // BK1_STAGES x (A tile, B tile)
@@ -392,7 +396,7 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + BK1_BAR_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);       // warp-uniform, and known to be
     if (threadIdx.x == 0) {
         for (int x = 0; x < BK1_BAR_COUNT; ++x) {
             const bool many = (x >= BK1_AB_FULL && x < BK1_AB_FULL + BK1_STAGES) || (x >= BK1_P_FULL && x < BK1_P_FULL + 2) ||
@@ -419,25 +423,24 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
     sa2::sm100::prof_begin();
 #endif
     if (warp == 0) {
-        if (lane == 0) {
-            if (g.total > 0) {
+        if (g.total > 0) {
+            if (elect_one()) {
                 prefetch_tmap(&mapK);
                 prefetch_tmap(&mapV);
                 mbar_arrive_expect_tx(&bars[BK1_KV_FULL], 2 * TILE_BYTES);
                 tma_load_4d(sK, &mapK, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
                 tma_load_4d(sV, &mapV, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
-                err = bk1_mma_second(g, tmem, sAB, bars, abort_flag);
-                // the tile must have landed before the CTA may exit, even if every other role gave up
-                if (!mbar_wait(&bars[BK1_KV_FULL], 0, abort_flag)) err |= ERR_BK1_PRODUCER;
-            } else {
-                tc_commit(&bars[BK1_DONE]);
             }
+            err = bk1_mma_second(g, tmem, sAB, bars, abort_flag);
+            // the tile must have landed before the CTA may exit, even if every other role gave up
+            if (!mbar_wait_warp(&bars[BK1_KV_FULL], 0, abort_flag)) err |= ERR_BK1_PRODUCER;
+        } else if (elect_one()) {
+            tc_commit(&bars[BK1_DONE]);
         }
-        __syncwarp();
-    } else if (warp == 1 || warp == 14) {
-        if (lane == 0 && g.total > 0)
-            err = bk1_mma_first(P.kp, g, warp == 1 ? 0 : 1, tmem, warp == 1 ? sK : sV, sAB, sStat, sOnes, bars, abort_flag);
-        __syncwarp();
+    } else if (warp == 1) {
+        if (g.total > 0) err = bk1_mma_first(P.kp, g, 0, tmem, sK, sAB, sStat, sOnes, bars, abort_flag);
+    } else if (warp == 14) {
+        if (g.total > 0) err = bk1_mma_first(P.kp, g, 1, tmem, sV, sAB, sStat, sOnes, bars, abort_flag);
     } else if (warp < 10) {
         err = bk1_compute(P, g, (warp - 2) >> 2, tmem, bars, abort_flag);
     } else {

@@ -227,7 +227,7 @@ __device__ __forceinline__ int mma_first(const KernelParams &kp, const Geom &g, 
     const uint64_t dT = smem_desc_sw128(smem_u32(sKV));
     const uint64_t dAB = smem_desc_sw128(smem_u32(sAB + which * AB_BYTES));
     const uint64_t dOnes = smem_desc_sw128(smem_u32(sConst));
-    if (!mbar_wait(&bars[B_KV_FULL], 0, abort_flag)) return ERR_BK1_MMA;
+    if (!mbar_wait_warp(&bars[B_KV_FULL], 0, abort_flag)) return ERR_BK1_MMA;
     int s = 0, blk = 0;
     for (int hh = 0; hh < kp.g; ++hh) {
         for (int ib = 0; ib < g.n_ib; ++ib, ++blk) {
@@ -236,12 +236,13 @@ __device__ __forceinline__ int mma_first(const KernelParams &kp, const Geom &g, 
             const uint64_t st = dOnes + (uint64_t)((stat_row(blk % 3, which, 0) * 128) >> 4) + (uint64_t)stat_chunk(blk % 3, which);
             for (int e = 0; e < ne; ++e, ++s) {
                 const int stage = s % STAGES, half = s & 1;
-                if (!mbar_wait(&bars[B_AB_FULL + stage], (s / STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
+                if (!mbar_wait_warp(&bars[B_AB_FULL + stage], (s / STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
                 // P^T / G^T of the step that used this half last lie over these columns until its second products are done
-                if (s >= 2 && !mbar_wait(&bars[B_G_DONE + half], ((s >> 1) - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
+                if (s >= 2 && !mbar_wait_warp(&bars[B_G_DONE + half], ((s >> 1) - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
                 tc_fence_after();
                 const uint64_t a = dAB + (uint64_t)((stage * STAGE_BYTES) >> 4);
                 const uint32_t d = tmem + half * 128 + which * 64;
+                if (elect_one()) {
 #pragma unroll
                 for (int k8 = 0; k8 < 8; ++k8) {
                     const uint64_t kin = (uint64_t)((k8 & 3) * 2);
@@ -250,6 +251,7 @@ __device__ __forceinline__ int mma_first(const KernelParams &kp, const Geom &g, 
                 }
                 mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
                 tc_commit(&bars[B_S_FULL + half]);
+                }
             }
         }
     }
@@ -264,11 +266,12 @@ __device__ __forceinline__ int mma_second(const Params &P, const Geom &g, uint32
     const uint64_t dAB = smem_desc_sw128(smem_u32(sAB), 1024, QBLK_BYTES);   // channel blocks 8 KB apart
     for (int s = 0; s < g.total; ++s) {
         const int stage = s % STAGES, half = s & 1;
-        if (!mbar_wait(&bars[B_P_FULL + half], (s >> 1) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
+        if (!mbar_wait_warp(&bars[B_P_FULL + half], (s >> 1) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
         tc_fence_after();
         const uint64_t a = dAB + (uint64_t)((stage * STAGE_BYTES) >> 4), bq = a + (AB_BYTES >> 4);
         const uint32_t tp = tmem + half * 128, tg = tp + 64;
         const uint32_t first = s > 0 ? 1u : 0u;
+        if (elect_one()) {
         if (!P.n_split) {
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4) mma_ts(tmem + 384, tp + k4 * 8, bq + k4 * 128, IDESC_G, (first || k4 > 0) ? 1u : 0u);
@@ -288,8 +291,9 @@ __device__ __forceinline__ int mma_second(const Params &P, const Geom &g, uint32
         }
         tc_commit(&bars[B_G_DONE + half]);
         tc_commit(&bars[B_AB_EMPTY + stage]);
+        }
     }
-    tc_commit(&bars[B_DONE]);
+    if (elect_one()) tc_commit(&bars[B_DONE]);
     return 0;
 }
 
@@ -394,7 +398,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 bwd_k1_128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
                   const __grid_constant__ CUtensorMap mapK2, const __grid_constant__ CUtensorMap mapV2, const Params P) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;
     uint8_t *sV = sK + T_BYTES;
     uint8_t *sAB = sV + T_BYTES;                          // STAGES x (A_e, B_e)
@@ -404,7 +408,7 @@ bwd_k1_128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constan
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + B_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);       // warp-uniform, and known to be
     if (threadIdx.x == 0) {
         for (int x = 0; x < B_COUNT; ++x) {
             uint32_t count = 1;
@@ -434,8 +438,8 @@ bwd_k1_128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constan
     if (warp < 4) {
         reg_dealloc<REGS_ISSUE>();
         if (warp == 0) {
-            if (lane == 0) {
-                if (g.total > 0) {
+            if (g.total > 0) {
+                if (elect_one()) {
                     prefetch_tmap(&mapK);
                     prefetch_tmap(&mapV);
                     mbar_arrive_expect_tx(&bars[B_KV_FULL], 2 * T_BYTES);
@@ -443,18 +447,17 @@ bwd_k1_128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constan
                     tma_load_4d(sK + BLK_BYTES, &mapK, &bars[B_KV_FULL], 64, blockIdx.y, g.j0, blockIdx.z);
                     tma_load_4d(sV, &mapV, &bars[B_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
                     tma_load_4d(sV + BLK_BYTES, &mapV, &bars[B_KV_FULL], 64, blockIdx.y, g.j0, blockIdx.z);
-                    err = mma_second(P, g, tmem, sAB, bars, abort_flag);
-                    // the tile must have landed before the CTA may exit, even if every other role gave up
-                    if (!mbar_wait(&bars[B_KV_FULL], 0, abort_flag)) err |= ERR_BK1_PRODUCER;
-                } else {
-                    tc_commit(&bars[B_DONE]);
                 }
+                err = mma_second(P, g, tmem, sAB, bars, abort_flag);
+                // the tile must have landed before the CTA may exit, even if every other role gave up
+                if (!mbar_wait_warp(&bars[B_KV_FULL], 0, abort_flag)) err |= ERR_BK1_PRODUCER;
+            } else if (elect_one()) {
+                tc_commit(&bars[B_DONE]);
             }
-            __syncwarp();
-        } else if (warp == 1 || warp == 2) {
-            if (lane == 0 && g.total > 0)
-                err = mma_first(P.kp, g, warp - 1, tmem, warp == 1 ? sK : sV, sAB, sConst, bars, abort_flag);
-            __syncwarp();
+        } else if (warp == 1) {
+            if (g.total > 0) err = mma_first(P.kp, g, 0, tmem, sK, sAB, sConst, bars, abort_flag);
+        } else if (warp == 2) {
+            if (g.total > 0) err = mma_first(P.kp, g, 1, tmem, sV, sAB, sConst, bars, abort_flag);
         }
     } else if (warp < 12) {
         reg_alloc<REGS_COMPUTE>();

@@ -232,20 +232,21 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
     constexpr uint32_t IDESC_F = idesc_bf16(128, 64, false, false);
     const uint64_t dT = smem_desc_sw128(smem_u32(sKV)), dA = smem_desc_sw128(smem_u32(sAB));
     if constexpr (D == 64) {
-        if (!mbar_wait(&bars[BQ_KV_FULL], 0, abort_flag)) return ERR_BQ_MMA;
+        if (!mbar_wait_warp(&bars[BQ_KV_FULL], 0, abort_flag)) return ERR_BQ_MMA;
     }
     int u = 0, buf = 0, use = 0;                         // use = u / NBUF: how often the buffer has been used before
     int slot = 0, suse = 0;                              // head dim 128: ring slot u % NSLOT and u / NSLOT
     for (int e = 0; e < g.nsweeps; ++e) {
-        if (!mbar_wait(&bars[BQ_AB_FULL], e & 1, abort_flag, 0, 1)) return ERR_BQ_MMA;
+        if (!mbar_wait_warp(&bars[BQ_AB_FULL], e & 1, abort_flag, 0, 1)) return ERR_BQ_MMA;
         for (int w = 0; w < g.nunits; ++w, ++u) {
             // the buffer holds P / G of its previous unit until the U / W products of that unit are done
-            if (use >= 1 && !mbar_wait(&bars[BQ_G_DONE + buf], (use - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
+            if (use >= 1 && !mbar_wait_warp(&bars[BQ_G_DONE + buf], (use - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
             if constexpr (D == 128) {
-                if (!mbar_wait(&bars[BQ_KV_SLOT + slot], suse & 1, abort_flag, 0, 3)) return ERR_BQ_MMA;
+                if (!mbar_wait_warp(&bars[BQ_KV_SLOT + slot], suse & 1, abort_flag, 0, 3)) return ERR_BQ_MMA;
             }
             tc_fence_after();
             SA2_PROF_MARK(seg);
+            if (elect_one()) {
             const uint32_t d = tmem + buf * 128 + which * 64;
             if constexpr (D == 64) {
                 const uint64_t t = dT + (uint64_t)((w * 8192) >> 4);       // unit w: rows [64 w, +64) of the resident tiles
@@ -261,10 +262,11 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
             SA2_PROF_LAP(4, seg);                         // issue of the products
             tc_commit(&bars[BQ_S_FULL + buf]);
             SA2_PROF_LAP(5, seg);                         // the commit
+            }
             if (++buf == C::NBUF) { buf = 0; ++use; }
             if (++slot == C::NSLOT) { slot = 0; ++suse; }
         }
-        tc_commit(&bars[BQ_AB_EMPTY]);
+        if (elect_one()) tc_commit(&bars[BQ_AB_EMPTY]);
     }
     return 0;
 }
@@ -280,20 +282,22 @@ __device__ __forceinline__ int bq_ring_producer(const BqParams &P, const BqGeom 
     int w = 0, slot = 0, suse = 0;
     for (int u = 0; u < g.total; ++u) {
         // the slot is free when the U / W products of the unit it held are done
-        if (suse >= 1 && !mbar_wait(&bars[BQ_KV_FREE + slot], (suse - 1) & 1, abort_flag, 32, 1)) return ERR_BQ_PRODUCER;
+        if (suse >= 1 && !mbar_wait_warp(&bars[BQ_KV_FREE + slot], (suse - 1) & 1, abort_flag, 32, 1)) return ERR_BQ_PRODUCER;
         const int row = g.ubase + 64 * w;
+        if (elect_one()) {
         mbar_arrive_expect_tx(&bars[BQ_KV_SLOT + slot], 4 * C::UBLK);
 #pragma unroll
         for (int cb = 0; cb < 2; ++cb) {
             tma_load_4d(sK + slot * 2 * C::UBLK + cb * C::UBLK, mapK, &bars[BQ_KV_SLOT + slot], cb * 64, hk, row, blockIdx.z);
             tma_load_4d(sV + slot * 2 * C::UBLK + cb * C::UBLK, mapV, &bars[BQ_KV_SLOT + slot], cb * 64, hk, row, blockIdx.z);
         }
+        }
         if (++w == g.nunits) w = 0;
         if (++slot == C::NSLOT) { slot = 0; ++suse; }
     }
     // every load must have landed before the CTA may exit, even if the consumers gave up
     for (int u = max(0, g.total - C::NSLOT); u < g.total; ++u)
-        if (!mbar_wait(&bars[BQ_KV_SLOT + u % C::NSLOT], (u / C::NSLOT) & 1, abort_flag, 32)) return ERR_BQ_PRODUCER;
+        if (!mbar_wait_warp(&bars[BQ_KV_SLOT + u % C::NSLOT], (u / C::NSLOT) & 1, abort_flag, 32)) return ERR_BQ_PRODUCER;
     return 0;
 }
 
@@ -311,14 +315,16 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
             prefetch_tmap(mapK);
             prefetch_tmap(mapV);
             const int nt = g.nunits / 2;
+            if (elect_one()) {
             mbar_arrive_expect_tx(&bars[BQ_KV_FULL], 2 * C::BLK * nt);
             for (int t = 0; t < nt; ++t) {
                 const int row = g.ubase + TJ * t;
                 tma_load_4d(sK + (size_t)t * C::BLK, mapK, &bars[BQ_KV_FULL], 0, hk, row, blockIdx.z);
                 tma_load_4d(sV + (size_t)t * C::BLK, mapV, &bars[BQ_KV_FULL], 0, hk, row, blockIdx.z);
             }
+            }
         }
-        if (!mbar_wait(&bars[BQ_KV_FULL], 0, abort_flag)) return ERR_BQ_PRODUCER;
+        if (!mbar_wait_warp(&bars[BQ_KV_FULL], 0, abort_flag)) return ERR_BQ_PRODUCER;
     }
     // head dim 128: U / W take the CTA's 64-channel block of the unit as an MN-major B operand
     const uint64_t dK = smem_desc_sw128(smem_u32(sK) + (D == 64 ? 0 : g.chh * C::UBLK));
@@ -328,14 +334,15 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
         const int wb = e % C::UWBUF, wuse = e / C::UWBUF;
         const uint32_t tu = tmem + C::UW0 + wb * 128, tw = tu + 64;
         for (int w = 0; w < g.nunits; ++w, ++u) {
-            if (!mbar_wait(&bars[BQ_P_FULL + buf], use & 1, abort_flag, 0, 1)) return ERR_BQ_MMA;
+            if (!mbar_wait_warp(&bars[BQ_P_FULL + buf], use & 1, abort_flag, 0, 1)) return ERR_BQ_MMA;
             // the fold group must have read the accumulators of the sweep that used them last
-            if (w == 0 && wuse >= 1 && !mbar_wait(&bars[BQ_W_EMPTY + wb], (wuse - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
+            if (w == 0 && wuse >= 1 && !mbar_wait_warp(&bars[BQ_W_EMPTY + wb], (wuse - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
             tc_fence_after();
             const uint64_t off = (uint64_t)((D == 64 ? w * 8192 : slot * 2 * C::UBLK) >> 4);
             const uint64_t kt = dK + off, vt = dV + off;
             const uint32_t a = tmem + buf * 128;
             const uint32_t acc = w > 0 ? 1u : 0u;
+            if (elect_one()) {
             if (part != 1) {
                 // keys [32 x, +32) of G are 16 columns at 64 + 32 x, those of P at 32 x
                 mma_ts(tu, a + 64, kt, IDESC_G, acc);               // U += G K1
@@ -351,10 +358,11 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
             }
             tc_commit(&bars[BQ_G_DONE + buf]);
             if constexpr (D == 128) tc_commit(&bars[BQ_KV_FREE + slot]);
+            }
             if (++buf == C::NBUF) { buf = 0; ++use; }
             if (++slot == C::NSLOT) slot = 0;
         }
-        tc_commit(&bars[BQ_W_FULL + wb]);
+        if (elect_one()) tc_commit(&bars[BQ_W_FULL + wb]);
     }
     return 0;
 }
@@ -837,7 +845,7 @@ __global__ void __launch_bounds__(BQ_THREADS, 1)
 bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const BqParams P) {
     using C = BqCfg<D>;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;
     uint8_t *sV = sK + C::KV_BYTES;
     uint8_t *sA = sV + C::KV_BYTES;
@@ -849,7 +857,7 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + BQ_BAR_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);       // warp-uniform, and known to be
     if (threadIdx.x == 0) {
         for (int x = 0; x < BQ_BAR_COUNT; ++x) {
             const bool pfull = x >= BQ_P_FULL && x < BQ_P_FULL + 3;          // every compute thread
@@ -881,17 +889,12 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
 #endif
     if (warp < 4) {
         reg_dealloc<BQ_REGS_ISSUE>();                 // one instruction for the whole warpgroup
-        if (warp == 0 || (D == 64 && warp == 3)) {
-            if (lane == 0 && g.total > 0)
-                err = bq_mma_second<D>(P, g, D == 64 ? (warp == 0 ? 0 : 1) : 2, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
-            __syncwarp();
-        } else if (warp == 1 || warp == 2) {
-            if (lane == 0 && g.total > 0)
-                err = bq_mma_first<D>(g, warp - 1, tmem, warp == 1 ? sK : sV, warp == 1 ? sA : sB, bars, abort_flag);
-            __syncwarp();
-        } else if constexpr (D == 128) {
-            if (lane == 0 && g.total > 0) err = bq_ring_producer<D>(P, g, &mapK, &mapV, sK, sV, bars, abort_flag);
-            __syncwarp();
+        if (g.total > 0) {
+            if (warp == 0) err = bq_mma_second<D>(P, g, D == 64 ? 0 : 2, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
+            else if (warp == 1) err = bq_mma_first<D>(g, 0, tmem, sK, sA, bars, abort_flag);
+            else if (warp == 2) err = bq_mma_first<D>(g, 1, tmem, sV, sB, bars, abort_flag);
+            else if constexpr (D == 64) err = bq_mma_second<D>(P, g, 1, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
+            else err = bq_ring_producer<D>(P, g, &mapK, &mapV, sK, sV, bars, abort_flag);
         }
     } else if (warp < 4 + 4 * C::NCG) {
         // one call site for both compute groups: they run the same instructions, which the instruction caches

@@ -15,8 +15,8 @@
 // and a single new token (generation) still fills the rows of its tile.  fwd_rows_per_tile() picks RI.
 //
 // Warp roles (512 threads, four aligned warpgroups):
-//   warp 0, 1     lane 0 issues the tcgen05.mma stream of group 0 / group 1 (warp 1 owns the TMEM allocation)
-//   warp 2, 3     lane 0 of each is a TMA producer: second keys of the tile and K1 units, second values and V1
+//   warp 0, 1     issue the tcgen05.mma stream of group 0 / group 1 (warp 1 owns the TMEM allocation)
+//   warp 2, 3     TMA producers: second keys of the tile and K1 units, second values and V1
 //                 units (units are resident if the window fits, else a ring walked once per pair of sweeps)
 //   warps 4-7     output group, one thread per row: builds the A row of each group's next sweep as soon as the
 //                 last S product of its current sweep has completed, and folds v2 * W of the finished sweep
@@ -54,7 +54,7 @@ namespace tc {
 constexpr int FWD_THREADS = 512;
 // Register hand-over between warpgroups (launch: 128 per thread; the budgets must add up to at most 4 * 128, or
 // the growing group never returns from its setmaxnreg).
-constexpr int FWD_REGS_LAUNCH = 128, FWD_REGS_ISSUE = 48, FWD_REGS_SOFTMAX = 120, FWD_REGS_OUT = 216;
+constexpr int FWD_REGS_LAUNCH = 128, FWD_REGS_ISSUE = 56, FWD_REGS_SOFTMAX = 120, FWD_REGS_OUT = 216;
 static_assert(FWD_REGS_ISSUE + 2 * FWD_REGS_SOFTMAX + FWD_REGS_OUT <= 4 * FWD_REGS_LAUNCH, "register pool must balance");
 static_assert(FWD_REGS_SOFTMAX < FWD_REGS_LAUNCH, "the softmax groups release registers");
 constexpr int FWD_UNIT = 64;                                  // first-key rows of a unit
@@ -134,7 +134,7 @@ struct FwdSlot {
     }
 };
 
-// ------------------------------------------------------------------ TMA producers (warps 2 and 3, one lane each)
+// ------------------------------------------------------------------ TMA producers (warps 2 and 3)
 __device__ __forceinline__ int fwd_producer(const FwdParams &P, const FwdGeom &g, const CUtensorMap *map, const CUtensorMap *map2,
                                             uint8_t *dst, uint8_t *win, uint64_t *bars, volatile int *abort_flag) {
     const int b = blockIdx.z, hk = blockIdx.y / P.kp.g;
@@ -142,28 +142,30 @@ __device__ __forceinline__ int fwd_producer(const FwdParams &P, const FwdGeom &g
     FwdSlot s;
     int w = 0;
     auto load = [&]() -> bool {
-        if (s.use >= 1 && !mbar_wait(&bars[BAR_KV_FREE + s.slot], (s.use - 1) & 1, abort_flag, 32, 1)) return false;
-        mbar_arrive_expect_tx(&bars[BAR_KV_FULL + s.slot], FWD_UNIT_BYTES);
-        tma_load_4d(dst + s.slot * FWD_UNIT_BYTES, map, &bars[BAR_KV_FULL + s.slot], 0, hk, g.jbase + FWD_UNIT * w, b);
+        if (s.use >= 1 && !mbar_wait_warp(&bars[BAR_KV_FREE + s.slot], (s.use - 1) & 1, abort_flag, 32, 1)) return false;
+        if (elect_one()) {
+            mbar_arrive_expect_tx(&bars[BAR_KV_FULL + s.slot], FWD_UNIT_BYTES);
+            tma_load_4d(dst + s.slot * FWD_UNIT_BYTES, map, &bars[BAR_KV_FULL + s.slot], 0, hk, g.jbase + FWD_UNIT * w, b);
+        }
         s.next(P, g, w);
         if (++w == g.upe) w = 0;
         return true;
     };
-    if (P.win_boxes > 0) {
+    if (P.win_boxes > 0 && elect_one()) {
         mbar_arrive_expect_tx(&bars[BAR_WIN_FULL], P.win_boxes * 4096);
         for (int bx = 0; bx < P.win_boxes; ++bx) tma_load_4d(win + bx * 4096, map2, &bars[BAR_WIN_FULL], 0, hk, g.win0 + 32 * bx, b);
     }
     for (int x = 0; x < items; ++x)
         if (!load()) return ERR_FWD_PRODUCER;
     // every load must have landed before the CTA may exit, even if the consumers gave up
-    if (P.win_boxes > 0 && !mbar_wait(&bars[BAR_WIN_FULL], 0, abort_flag, 32)) return ERR_FWD_PRODUCER;
+    if (P.win_boxes > 0 && !mbar_wait_warp(&bars[BAR_WIN_FULL], 0, abort_flag, 32)) return ERR_FWD_PRODUCER;
     for (int x = max(0, items - P.nslots); x < items; ++x)
-        if (!mbar_wait(&bars[BAR_KV_FULL + x % P.nslots], (x / P.nslots) & 1, abort_flag, 32)) return ERR_FWD_PRODUCER;
+        if (!mbar_wait_warp(&bars[BAR_KV_FULL + x % P.nslots], (x / P.nslots) & 1, abort_flag, 32)) return ERR_FWD_PRODUCER;
     return 0;
 }
 
-// ------------------------------------------------------------------ MMA issuers (one lane each)
-// Lane 0 of warp g issues for group g: the two groups touch disjoint TMEM columns and only read shared memory,
+// ------------------------------------------------------------------ MMA issuers (warps 0 and 1)
+// Warp g issues for group g: the two groups touch disjoint TMEM columns and only read shared memory,
 // so their MMA streams need no ordering between them.  P V1 of unit u goes before S of unit u + 2, whose
 // completion therefore covers it (and the sweep after the next needs its A rows by then, whose builder waits for
 // the W that P V1 completes).
@@ -180,15 +182,17 @@ __device__ __forceinline__ int fwd_mma(const FwdParams &P, const FwdGeom &g, int
     int s_k = 0, s_w = 0, p_k = 0, p_w = 0;             // sweep and unit of the next S and of the next P V1
 
     auto issue_s = [&](int u) -> bool {
-        if (s_w == 0 && !mbar_wait(&bars[BAR_A_FULL + grp], s_k & 1, abort_flag, 0, 1)) return false;
-        if ((s_k == 0 || !g.resident) && !mbar_wait(&bars[BAR_KV_FULL + ss.slot], ss.use & 1, abort_flag, 0, 4)) return false;
+        if (s_w == 0 && !mbar_wait_warp(&bars[BAR_A_FULL + grp], s_k & 1, abort_flag, 0, 1)) return false;
+        if ((s_k == 0 || !g.resident) && !mbar_wait_warp(&bars[BAR_KV_FULL + ss.slot], ss.use & 1, abort_flag, 0, 4)) return false;
         tc_fence_after();
         const uint64_t kt = dK + (uint64_t)((ss.slot * FWD_UNIT_BYTES) >> 4);
         const uint32_t d = tS + (u & 1) * 64;
+        if (elect_one()) {
 #pragma unroll
-        for (int st = 0; st < D / 16; ++st) mma_ss(d, dA + st * 2, kt + st * 2, IDESC_S, st > 0 ? 1u : 0u);
-        tc_commit(&bars[BAR_S_FULL + grp * 2 + (u & 1)]);
-        if (s_w == upe - 1) tc_commit(&bars[BAR_A_FREE + grp]);          // the A rows may be rebuilt
+            for (int st = 0; st < D / 16; ++st) mma_ss(d, dA + st * 2, kt + st * 2, IDESC_S, st > 0 ? 1u : 0u);
+            tc_commit(&bars[BAR_S_FULL + grp * 2 + (u & 1)]);
+            if (s_w == upe - 1) tc_commit(&bars[BAR_A_FREE + grp]);      // the A rows may be rebuilt
+        }
         ss.next(P, g, s_w);
         if (++s_w == upe) { s_w = 0; ++s_k; }
         return true;
@@ -196,16 +200,18 @@ __device__ __forceinline__ int fwd_mma(const FwdParams &P, const FwdGeom &g, int
     for (int u = 0; u < 2 && u < n; ++u)
         if (!issue_s(u)) return ERR_FWD_MMA;
     for (int u = 0; u < n; ++u) {
-        if (p_w == 0 && p_k >= 1 && !mbar_wait(&bars[BAR_W_EMPTY + grp], (p_k - 1) & 1, abort_flag, 0, 3)) return ERR_FWD_MMA;
-        if (!mbar_wait(&bars[BAR_P_FULL + grp * 2 + (u & 1)], (u >> 1) & 1, abort_flag, 0, 2)) return ERR_FWD_MMA;
+        if (p_w == 0 && p_k >= 1 && !mbar_wait_warp(&bars[BAR_W_EMPTY + grp], (p_k - 1) & 1, abort_flag, 0, 3)) return ERR_FWD_MMA;
+        if (!mbar_wait_warp(&bars[BAR_P_FULL + grp * 2 + (u & 1)], (u >> 1) & 1, abort_flag, 0, 2)) return ERR_FWD_MMA;
         tc_fence_after();
         const uint64_t vt = dV + (uint64_t)((ps.slot * FWD_UNIT_BYTES) >> 4);
         const uint32_t a = tP + (u & 1) * 32;
+        if (elect_one()) {
 #pragma unroll
-        for (int st = 0; st < 4; ++st) mma_ts(tW, a + st * 8, vt + st * 128, IDESC_PV, (p_w > 0 || st > 0) ? 1u : 0u);
-        tc_commit(&bars[BAR_PV_DONE + grp]);
-        if (!g.resident) tc_commit(&bars[BAR_KV_FREE + ps.slot]);
-        if (p_w == upe - 1) tc_commit(&bars[BAR_W_FULL + grp]);
+            for (int st = 0; st < 4; ++st) mma_ts(tW, a + st * 8, vt + st * 128, IDESC_PV, (p_w > 0 || st > 0) ? 1u : 0u);
+            tc_commit(&bars[BAR_PV_DONE + grp]);
+            if (!g.resident) tc_commit(&bars[BAR_KV_FREE + ps.slot]);
+            if (p_w == upe - 1) tc_commit(&bars[BAR_W_FULL + grp]);
+        }
         ps.next(P, g, p_w);
         if (++p_w == upe) { p_w = 0; ++p_k; }
         if (u + 2 < n && !issue_s(u + 2)) return ERR_FWD_MMA;
@@ -214,8 +220,8 @@ __device__ __forceinline__ int fwd_mma(const FwdParams &P, const FwdGeom &g, int
     // units of that last sweep pass, so that every slot still collects two releases.
     if (!g.resident) {
         for (int x = n; x < g.nsw[0] * upe; ++x, ps.next(P, g, 0)) {
-            if (!mbar_wait(&bars[BAR_KV_FULL + ps.slot], ps.use & 1, abort_flag, 32)) return ERR_FWD_MMA;
-            mbar_arrive(&bars[BAR_KV_FREE + ps.slot]);
+            if (!mbar_wait_warp(&bars[BAR_KV_FULL + ps.slot], ps.use & 1, abort_flag, 32)) return ERR_FWD_MMA;
+            if (elect_one()) mbar_arrive(&bars[BAR_KV_FREE + ps.slot]);
         }
     }
     return 0;
@@ -546,7 +552,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
            const __grid_constant__ CUtensorMap mapK2, const __grid_constant__ CUtensorMap mapV2, const FwdParams P) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;
     uint8_t *sV = sK + (size_t)max(P.nslots, 3) * FWD_UNIT_BYTES;
     uint8_t *sA = sV + (size_t)max(P.nslots, 3) * FWD_UNIT_BYTES;         // [2] one tile per group
@@ -556,7 +562,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + BAR_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);        // warp-uniform, and known to be
     if (threadIdx.x == 0) {
         for (int x = 0; x < BAR_COUNT; ++x) {
             const bool many = (x >= BAR_P_FULL && x < BAR_P_FULL + 4) || (x >= BAR_W_EMPTY && x < BAR_W_EMPTY + 2) ||
@@ -584,12 +590,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
 #endif
     if (warp < 4) {
         reg_dealloc<FWD_REGS_ISSUE>();                // one instruction for the whole warpgroup
-        if ((threadIdx.x & 31) == 0) {
-            if (warp < 2) err = fwd_mma<D>(P, g, warp, tmem, sK, sV, sA, bars, abort_flag);
-            else if (warp == 2) err = fwd_producer(P, g, &mapK, &mapK2, sK, sWin, bars, abort_flag);
-            else err = fwd_producer(P, g, &mapV, &mapV2, sV, sWin + (size_t)P.win_boxes * 4096, bars, abort_flag);
-        }
-        __syncwarp();
+        if (warp == 0) err = fwd_mma<D>(P, g, 0, tmem, sK, sV, sA, bars, abort_flag);
+        else if (warp == 1) err = fwd_mma<D>(P, g, 1, tmem, sK, sV, sA, bars, abort_flag);
+        else if (warp == 2) err = fwd_producer(P, g, &mapK, &mapK2, sK, sWin, bars, abort_flag);
+        else err = fwd_producer(P, g, &mapV, &mapV2, sV, sWin + (size_t)P.win_boxes * 4096, bars, abort_flag);
     } else if (warp >= 8) {
         reg_dealloc<FWD_REGS_SOFTMAX>();
         err = fwd_softmax(P, g, (warp - 8) >> 2, tmem, D, stats, bars, abort_flag);

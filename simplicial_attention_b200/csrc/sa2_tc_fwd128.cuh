@@ -118,16 +118,18 @@ __device__ __forceinline__ int producer(const Params &P, const Geom &g, const CU
     int w = 0;
     for (int x = 0; x < items; ++x) {
         const int slot = x % SLOTS;
-        if (x >= SLOTS && !mbar_wait(&bars[empty0 + slot], (x / SLOTS - 1) & 1, abort_flag, 32, 1)) return ERR_FWD_PRODUCER;
+        if (x >= SLOTS && !mbar_wait_warp(&bars[empty0 + slot], (x / SLOTS - 1) & 1, abort_flag, 32, 1)) return ERR_FWD_PRODUCER;
         const int row = g.hbase + UNIT * (g.h_first + w);
+        if (elect_one()) {
         mbar_arrive_expect_tx(&bars[full0 + slot], UNIT_BYTES);
         tma_load_4d(ring + slot * UNIT_BYTES, map, &bars[full0 + slot], 0, hk, row, b);
         tma_load_4d(ring + slot * UNIT_BYTES + BLK_BYTES, map, &bars[full0 + slot], 64, hk, row, b);
+        }
         if (++w == g.nunits) w = 0;
     }
     // every load must have landed before the CTA may exit, even if the consumers gave up
     for (int x = max(0, items - SLOTS); x < items; ++x)
-        if (!mbar_wait(&bars[full0 + x % SLOTS], (x / SLOTS) & 1, abort_flag, 32)) return ERR_FWD_PRODUCER;
+        if (!mbar_wait_warp(&bars[full0 + x % SLOTS], (x / SLOTS) & 1, abort_flag, 32)) return ERR_FWD_PRODUCER;
     return 0;
 }
 
@@ -146,13 +148,14 @@ __device__ __forceinline__ int issue_s(const Params &P, const Geom &g, int grp, 
     int w = 0, ks = 0;
     for (int u = 0; u < n; ++u) {
         const int sb = u & 1, slot = u % SLOTS;
-        if (w == 0 && !mbar_wait(&bars[B_A_FULL + grp], ks & 1, abort_flag, 0, 1)) return ERR_FWD_MMA;
-        if (!mbar_wait(&bars[B_K_FULL + slot], (u / SLOTS) & 1, abort_flag, 0, 2)) return ERR_FWD_MMA;
+        if (w == 0 && !mbar_wait_warp(&bars[B_A_FULL + grp], ks & 1, abort_flag, 0, 1)) return ERR_FWD_MMA;
+        if (!mbar_wait_warp(&bars[B_K_FULL + slot], (u / SLOTS) & 1, abort_flag, 0, 2)) return ERR_FWD_MMA;
         // P of the unit that used this buffer last must have been consumed: S overwrites it
-        if (u >= 2 && !mbar_wait(&bars[B_PV_DONE + grp * 2 + sb], ((u - 2) >> 1) & 1, abort_flag, 0, 3)) return ERR_FWD_MMA;
+        if (u >= 2 && !mbar_wait_warp(&bars[B_PV_DONE + grp * 2 + sb], ((u - 2) >> 1) & 1, abort_flag, 0, 3)) return ERR_FWD_MMA;
         tc_fence_after();
         const uint64_t kt = dK + (uint64_t)((slot * UNIT_BYTES) >> 4);
         const uint32_t d = tS + sb * 64;
+        if (elect_one()) {
 #pragma unroll
         for (int st = 0; st < 8; ++st) {
             const uint64_t a = dA + (uint64_t)(((st >> 2) * ABLK_BYTES) >> 4) + (uint64_t)((st & 3) * 2);
@@ -162,14 +165,15 @@ __device__ __forceinline__ int issue_s(const Params &P, const Geom &g, int grp, 
         tc_commit(&bars[B_S_FULL + grp * 2 + sb]);
         tc_commit(&bars[B_K_EMPTY + slot]);
         if (w == nu - 1) tc_commit(&bars[B_A_FREE + grp]);      // the A stage may be rebuilt
+        }
         if (++w == nu) { w = 0; ++ks; }
     }
     // The rings follow group 0's walk.  With an odd number of sweeps group 1 has one sweep less: it lets the
     // units of that last sweep pass, so that every slot still collects two releases.
     for (int x = n; x < g.nsw[0] * nu; ++x) {
         const int slot = x % SLOTS;
-        if (!mbar_wait(&bars[B_K_FULL + slot], (x / SLOTS) & 1, abort_flag, 32)) return ERR_FWD_MMA;
-        mbar_arrive(&bars[B_K_EMPTY + slot]);
+        if (!mbar_wait_warp(&bars[B_K_FULL + slot], (x / SLOTS) & 1, abort_flag, 32)) return ERR_FWD_MMA;
+        if (elect_one()) mbar_arrive(&bars[B_K_EMPTY + slot]);
     }
     return 0;
 }
@@ -185,12 +189,13 @@ __device__ __forceinline__ int issue_pv(const Params &P, const Geom &g, int grp,
     int w = 0, ks = 0;
     for (int u = 0; u < n; ++u) {
         const int sb = u & 1, slot = u % SLOTS;
-        if (!mbar_wait(&bars[B_V_FULL + slot], (u / SLOTS) & 1, abort_flag, 0, 4)) return ERR_FWD_MMA;
-        if (!mbar_wait(&bars[B_P_FULL + grp * 2 + sb], (u >> 1) & 1, abort_flag, 0, 5)) return ERR_FWD_MMA;
-        if (w == 0 && ks >= 1 && !mbar_wait(&bars[B_W_EMPTY + grp], (ks - 1) & 1, abort_flag, 0, 6)) return ERR_FWD_MMA;
+        if (!mbar_wait_warp(&bars[B_V_FULL + slot], (u / SLOTS) & 1, abort_flag, 0, 4)) return ERR_FWD_MMA;
+        if (!mbar_wait_warp(&bars[B_P_FULL + grp * 2 + sb], (u >> 1) & 1, abort_flag, 0, 5)) return ERR_FWD_MMA;
+        if (w == 0 && ks >= 1 && !mbar_wait_warp(&bars[B_W_EMPTY + grp], (ks - 1) & 1, abort_flag, 0, 6)) return ERR_FWD_MMA;
         tc_fence_after();
         const uint32_t a = tS + sb * 64;                 // P lies over the first 32 columns of its S
         const uint64_t vt = dV + (uint64_t)((slot * UNIT_BYTES) >> 4);
+        if (elect_one()) {
         if (!P.pv_split) {
 #pragma unroll
             for (int st = 0; st < 4; ++st) mma_ts(tW, a + st * 8, vt + st * 128, IDESC_PV, (w > 0 || st > 0) ? 1u : 0u);
@@ -204,12 +209,13 @@ __device__ __forceinline__ int issue_pv(const Params &P, const Geom &g, int grp,
         tc_commit(&bars[B_PV_DONE + grp * 2 + sb]);
         tc_commit(&bars[B_V_EMPTY + slot]);
         if (w == nu - 1) tc_commit(&bars[B_W_FULL + grp]);
+        }
         if (++w == nu) { w = 0; ++ks; }
     }
     for (int x = n; x < g.nsw[0] * nu; ++x) {
         const int slot = x % SLOTS;
-        if (!mbar_wait(&bars[B_V_FULL + slot], (x / SLOTS) & 1, abort_flag, 32)) return ERR_FWD_MMA;
-        mbar_arrive(&bars[B_V_EMPTY + slot]);
+        if (!mbar_wait_warp(&bars[B_V_FULL + slot], (x / SLOTS) & 1, abort_flag, 32)) return ERR_FWD_MMA;
+        if (elect_one()) mbar_arrive(&bars[B_V_EMPTY + slot]);
     }
     return 0;
 }
@@ -455,7 +461,7 @@ __device__ __forceinline__ void rows_sync() { asm volatile("bar.sync 2, 512;" ::
 __global__ void __launch_bounds__(THREADS, 1)
 fwd128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const Params P) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;                               // K1 ring
     uint8_t *sV = sK + SLOTS * UNIT_BYTES;            // V1 ring
     uint8_t *sA = sV + SLOTS * UNIT_BYTES;
@@ -464,7 +470,7 @@ fwd128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + B_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);       // warp-uniform, and known to be
     const Geom g = geom(P);
     if (threadIdx.x == 0) {
         for (int x = 0; x < B_COUNT; ++x) {
@@ -495,18 +501,14 @@ fwd128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
 #endif
     if (warp < 4) {
         reg_dealloc<REGS_ISSUE>();                    // one instruction for the whole warpgroup
-        if ((threadIdx.x & 31) == 0) {
-            if (warp < 2) err = issue_s(P, g, warp, tmem, sK, sA, bars, abort_flag);
-            else err = issue_pv(P, g, warp - 2, tmem, sV, bars, abort_flag);
-        }
-        __syncwarp();
+        if (warp == 0) err = issue_s(P, g, 0, tmem, sK, sA, bars, abort_flag);
+        else if (warp == 1) err = issue_s(P, g, 1, tmem, sK, sA, bars, abort_flag);
+        else if (warp == 2) err = issue_pv(P, g, 0, tmem, sV, bars, abort_flag);
+        else err = issue_pv(P, g, 1, tmem, sV, bars, abort_flag);
     } else if (warp >= 20) {
         reg_dealloc<REGS_PRODUCE>();
-        if ((threadIdx.x & 31) == 0) {
-            if (warp == 20) err = producer(P, g, &mapK, sK, B_K_FULL, B_K_EMPTY, bars, abort_flag);
-            else if (warp == 21) err = producer(P, g, &mapV, sV, B_V_FULL, B_V_EMPTY, bars, abort_flag);
-        }
-        __syncwarp();
+        if (warp == 20) err = producer(P, g, &mapK, sK, B_K_FULL, B_K_EMPTY, bars, abort_flag);
+        else if (warp == 21) err = producer(P, g, &mapV, sV, B_V_FULL, B_V_EMPTY, bars, abort_flag);
     } else if (warp >= 12) {
         reg_dealloc<REGS_SOFTMAX>();
         err = softmax(P, g, (warp - 12) >> 2, tmem, stats, bars, abort_flag);
