@@ -21,28 +21,52 @@ inline int tiles_per_query_tile(int w1) { return (w1 + TJ - 1 + TJ - 1) / TJ; } 
 
 // The tensor-core forward handles bf16 at every head dim and any window.
 inline bool fwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
-// The tensor-core backward handles bf16 and head dim 64 or 128, any window.
-inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16 && (s.d == 64 || s.d == 128); }
+// So does the tensor-core backward.
+inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-// CTAs sharing one query tile in the dQ/dK2/dV2 kernel (head dim 128 walks the whole window in one CTA)
-inline int bq_splits(int w1, int d) { return d == 128 ? 1 : (tiles_per_query_tile(w1) + BQ_MAX_TILES - 1) / BQ_MAX_TILES; }
+// CTAs sharing one query tile in the dQ/dK2/dV2 kernel: splits of the window (head dim 128 walks it in one CTA) times
+// splits of the offsets.  A CTA costs ~12000 cycles of set-up, loads, slab and its share of the reduction, a 64-key unit
+// of a sweep ~1600 (3000 at head dim 128); at most as many offsets per CTA as its accumulators hold.
+struct BqSplit { int tsplit, esplit, epc; };
+inline BqSplit bq_split(const sa2_shape &s, int sms) {
+    BqSplit r;
+    r.tsplit = s.d == 128 ? 1 : (tiles_per_query_tile(s.w1) + BQ_MAX_TILES - 1) / BQ_MAX_TILES;
+    const int nt = tiles_per_query_tile(s.w1), have = (s.n + s.off1 + TJ - 1) / TJ;
+    const int tiles = (nt < have ? nt : have), per = (tiles + r.tsplit - 1) / r.tsplit;
+    const int64_t ctas = (int64_t)((s.n + TQ - 1) / TQ) * s.hq * r.tsplit * (s.d == 128 ? 2 : 1);
+    const int w2 = s.w2 < s.n + s.off2 ? s.w2 : s.n + s.off2;
+    const int least = (w2 + BQ_MAX_EPC - 1) / BQ_MAX_EPC;
+    double best_cost = 0.;
+    r.esplit = least;
+    for (int es = least; es <= w2 && (es <= 16 || es == least); ++es) {
+        const double cost = split_cost(ctas * es, 12000. + (w2 + es - 1) / es * (per * 2. * (s.d == 128 ? 3000. : 1600.)), sms);
+        if (best_cost == 0. || cost < 0.94 * best_cost) { r.esplit = es; best_cost = cost; }
+    }
+    r.epc = (w2 + r.esplit - 1) / r.esplit;
+    r.esplit = (w2 + r.epc - 1) / r.epc;
+    return r;
+}
 // Diagnostic switch: SA2_MMA_N64=1 issues every head-dim-128 product over the channels as two N = 64
 // instructions instead of one N = 128 instruction.
 inline int n64_products() {
     static const int v = [] { const char *e = std::getenv("SA2_MMA_N64"); return (e && e[0] == '1') ? 1 : 0; }();
     return v;
 }
-// dQ/dK2/dV2 run on the tensor cores when their shared accumulators (127 + w2 rows) fit
-inline bool bq_supported(const sa2_shape &s) { return bwd_supported(s) && s.w2 <= BQ_MAX_W2; }
-// scratch after the D vector: per-split partial dQ, then the per-CTA dK2/dV2 slabs
+// scratch after the D vector: per-split partial dQ, the per-CTA dK2/dV2 slabs, partial dK1/dV1
+struct BwdScratch { size_t dq, k2, k1; };
+inline BwdScratch bwd_scratch(const sa2_shape &s) {
+    const BqSplit sp = bq_split(s, SM_COUNT);
+    const K1Split k1 = k1_split(s, SM_COUNT);
+    const int ns = sp.tsplit * sp.esplit;
+    return BwdScratch{align256(bq_part_dq_bytes(s, ns)), align256(bq_part_k2_bytes(s, ns, sp.epc)), align256(k1_part_bytes(s, k1.si * k1.se))};
+}
 inline size_t bwd_extra_workspace_bytes(const sa2_shape &s) {
-    if (!bq_supported(s)) return 0;
-    const int ns = bq_splits(s.w1, s.d);
-    return align256(bq_part_dq_bytes(s, ns)) + align256(bq_part_k2_bytes(s, ns));
+    if (!bwd_supported(s)) return 0;
+    const BwdScratch b = bwd_scratch(s);
+    return b.dq + b.k2 + b.k1;
 }
 // forward: 1 kernel; backward: D = rowsum(O*dO), dK1/dV1, dQ/dK2/dV2 partials, their reduction
-// (or, when w2 is too large for the shared accumulators, one fp32 launch for dQ and dK2/dV2)
-inline int launches(const sa2_shape &s, bool backward) { return !backward ? 1 : bq_supported(s) ? 4 : 3; }
+inline int launches(const sa2_shape &, bool backward) { return backward ? 4 : 1; }
 
 inline bool tma_addressable(const TensorRef &t) {
     return (reinterpret_cast<uintptr_t>(t.p) & 15u) == 0 && t.sb % 8 == 0 && t.sn % 8 == 0 && t.sh % 8 == 0;
@@ -127,21 +151,10 @@ inline bool bwd_addressable(const KernelParams &kp) {
     return fwd_addressable(kp) && tma_addressable(kp.dout);
 }
 
+// dQ, dK2, dV2: query-tile-owned tcgen05 kernel
 template <int D>
-inline int bwd_q_launch(const KernelParams &kp, const sa2_shape &s, const CUtensorMap &mapK, const CUtensorMap &mapV,
-                        float c, int *status, void *extra, cudaStream_t st) {
-    // dQ, dK2, dV2: query-tile-owned tcgen05 kernel + deterministic reduction of its partials
-    BqParams Q;
-    Q.kp = kp;
-    Q.c = c;
-    Q.nt = tiles_per_query_tile(s.w1);
-    Q.nsplit = bq_splits(s.w1, D);
-    Q.tiles_per_split = (Q.nt + Q.nsplit - 1) / Q.nsplit;
-    Q.nqt = (kp.n + TQ - 1) / TQ;
-    Q.part_dq = reinterpret_cast<float *>(extra);
-    Q.part_k2 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + align256(bq_part_dq_bytes(s, Q.nsplit)));
-    Q.status = status;
-    const size_t smem = bq_smem_bytes<D>(s.w2);
+inline int bwd_q_launch(const BqParams &Q, const KernelParams &kp, const CUtensorMap &mapK, const CUtensorMap &mapV, cudaStream_t st) {
+    const size_t smem = bq_smem_bytes<D>(Q.epc);
     if (cudaFuncSetAttribute(bwd_q_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SA2_ERR_CUDA;
     CUtensorMap ringK = mapK, ringV = mapV;
@@ -151,69 +164,92 @@ inline int bwd_q_launch(const KernelParams &kp, const sa2_shape &s, const CUtens
             return SA2_ERR_CUDA;
     }
     bwd_q_kernel<D><<<dim3(Q.nqt * Q.nsplit * BqCfg<D>::CH, kp.hq, kp.b), BQ_THREADS, smem, st>>>(ringK, ringV, Q);
-    if (cudaGetLastError() != cudaSuccess) return SA2_ERR_CUDA;
-    const int64_t work = ((Q.nsplit == 1 ? 0 : (int64_t)kp.b * kp.n * kp.hq) + (int64_t)kp.b * kp.nk2 * kp.hk) * (D / 4);
-    bwd_q_reduce_kernel<D><<<(unsigned)((work + 255) / 256), 256, 0, st>>>(Q);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
-// dQ and dK2/dV2 in fp32 (second-key windows too long for the shared accumulators)
+// deterministic reduction of the partials
 template <int D>
-inline int bwd_q_simt(const KernelParams &kp, cudaStream_t st) {
-    return simt::launch_bwd<D>(kp, true, true, false, SM_COUNT, st) ? SA2_OK : SA2_ERR_CUDA;
+inline int bwd_reduce_launch(const BqParams &Q, cudaStream_t st) {
+    const KernelParams &kp = Q.kp;
+    const int64_t rows = (Q.reduce_q ? (Q.nsplit == 1 ? 0 : (int64_t)kp.b * kp.n * kp.hq) + (int64_t)kp.b * kp.nk2 * kp.hk : 0) +
+                         (Q.reduce_k1 ? (int64_t)kp.b * kp.nk1 * kp.hk : 0);
+    if (rows == 0) return SA2_OK;
+    bwd_q_reduce_kernel<D><<<(unsigned)((rows * (D / 4) + 255) / 256), 256, 0, st>>>(Q);
+    return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
-inline int bwd(const KernelParams &kp, const sa2_shape &s, void *extra, cudaStream_t st, int phases = 0) {
-    if (!bwd_addressable(kp)) return SA2_ERR_INVALID;
+template <int D>
+inline int bwd_k1_launch(const KernelParams &kp, const sa2_shape &s, const CUtensorMap &mapK, const CUtensorMap &mapV, float c, int *status,
+                         const K1Split &sp, float *part, cudaStream_t st) {
+    CUtensorMap mapK2, mapV2;      // second keys / values, 32-row boxes of 64 channels
+    if (!tmap::make_rows_map(&mapK2, kp.k2.p, kp.b, kp.nk2, kp.hk, D, kp.k2.sb, kp.k2.sn, kp.k2.sh, 32) ||
+        !tmap::make_rows_map(&mapV2, kp.v2.p, kp.b, kp.nk2, kp.hk, D, kp.v2.sb, kp.v2.sn, kp.v2.sh, 32))
+        return SA2_ERR_CUDA;
+    const int ce = sp.si * sp.se;
+    const dim3 grid((kp.nk1 + TJ - 1) / TJ * ce, kp.hk, kp.b);
+    if constexpr (D == 128) {
+        k128::Params P;
+        P.kp = kp; P.c = c; P.ce = ce; P.si = sp.si; P.epc = sp.epc; P.part = part; P.n_split = n64_products(); P.status = status;
+        if (cudaFuncSetAttribute(k128::bwd_k1_128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k128::smem_bytes()) != cudaSuccess)
+            return SA2_ERR_CUDA;
+        k128::bwd_k1_128_kernel<<<grid, k128::THREADS, k128::smem_bytes(), st>>>(mapK, mapV, mapK2, mapV2, P);
+    } else {
+        BwdParams P;
+        P.kp = kp; P.c = c; P.ce = ce; P.si = sp.si; P.epc = sp.epc; P.part = part; P.status = status;
+        if (cudaFuncSetAttribute(bwd_k1_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bk1_smem_bytes()) != cudaSuccess)
+            return SA2_ERR_CUDA;
+        bwd_k1_kernel<D><<<grid, BK1_THREADS, bk1_smem_bytes(), st>>>(mapK, mapV, mapK2, mapV2, P);
+    }
+    return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
+}
+
+template <int D>
+inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, void *extra, cudaStream_t st, int phases) {
     const float c = s.scale * 1.4426950408889634f;
     int *status = status_word();
     if (!status) return SA2_ERR_CUDA;
     if (phases == 0) phases = SA2_BWD_ROWSUM | SA2_BWD_K1 | SA2_BWD_Q;
-
     // D_i = sum_c O_ic dO_ic
-    if (phases & SA2_BWD_ROWSUM) {
-        if (!(s.d == 128 ? simt::launch_delta<128>(kp, st) : simt::launch_delta<64>(kp, st))) return SA2_ERR_CUDA;
-    }
-
+    if ((phases & SA2_BWD_ROWSUM) && !simt::launch_delta<D>(kp, st)) return SA2_ERR_CUDA;
     // 128-row, 64-channel boxes of K1 / V1 (a head-dim-128 tile is two boxes)
     CUtensorMap mapK, mapV;
-    if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, s.d, kp.k1.sb, kp.k1.sn, kp.k1.sh, TJ) ||
-        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, s.d, kp.v1.sb, kp.v1.sn, kp.v1.sh, TJ))
+    if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, TJ) ||
+        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, TJ))
         return SA2_ERR_CUDA;
+    const BwdScratch room = bwd_scratch(s);
+    const BqSplit sp = bq_split(s, SM_COUNT);
+    BqParams Q;
+    Q.kp = kp;
+    Q.c = c;
+    Q.nt = tiles_per_query_tile(s.w1);
+    Q.tsplit = sp.tsplit;
+    Q.nsplit = sp.tsplit * sp.esplit;
+    Q.epc = sp.epc;
+    Q.tiles_per_split = (Q.nt + Q.tsplit - 1) / Q.tsplit;
+    Q.nqt = (kp.n + TQ - 1) / TQ;
+    Q.part_dq = reinterpret_cast<float *>(extra);
+    Q.part_k2 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + room.dq);
+    float *part_k1 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + room.dq + room.k2);
+    Q.part_k1 = part_k1;
+    Q.status = status;
+    const K1Split k1 = k1_split(s, SM_COUNT);
+    Q.ce = k1.si * k1.se;
+    Q.reduce_q = (phases & SA2_BWD_Q) != 0;
+    Q.reduce_k1 = (phases & SA2_BWD_K1) && Q.ce > 1;
+    if (phases & SA2_BWD_K1)
+        if (int e = bwd_k1_launch<D>(kp, s, mapK, mapV, c, status, k1, part_k1, st)) return e;
+    if (phases & SA2_BWD_Q)
+        if (int e = bwd_q_launch<D>(Q, kp, mapK, mapV, st)) return e;
+    return bwd_reduce_launch<D>(Q, st);
+}
 
-    // dK1, dV1: key-tile-owned tcgen05 kernel
-    if (phases & SA2_BWD_K1) {
-        CUtensorMap mapK2, mapV2;      // second keys / values, 32-row boxes of 64 channels
-        if (!tmap::make_rows_map(&mapK2, kp.k2.p, kp.b, kp.nk2, kp.hk, s.d, kp.k2.sb, kp.k2.sn, kp.k2.sh, 32) ||
-            !tmap::make_rows_map(&mapV2, kp.v2.p, kp.b, kp.nk2, kp.hk, s.d, kp.v2.sb, kp.v2.sn, kp.v2.sh, 32))
-            return SA2_ERR_CUDA;
-        const dim3 grid((kp.nk1 + TJ - 1) / TJ, kp.hk, kp.b);
-        if (s.d == 128) {
-            k128::Params P;
-            P.kp = kp;
-            P.c = c;
-            P.n_split = n64_products();
-            P.status = status;
-            if (cudaFuncSetAttribute(k128::bwd_k1_128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k128::smem_bytes()) != cudaSuccess)
-                return SA2_ERR_CUDA;
-            k128::bwd_k1_128_kernel<<<grid, k128::THREADS, k128::smem_bytes(), st>>>(mapK, mapV, mapK2, mapV2, P);
-        } else {
-            BwdParams P;
-            P.kp = kp;
-            P.c = c;
-            P.status = status;
-            if (cudaFuncSetAttribute(bwd_k1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bk1_smem_bytes()) != cudaSuccess)
-                return SA2_ERR_CUDA;
-            bwd_k1_kernel<<<grid, BK1_THREADS, bk1_smem_bytes(), st>>>(mapK, mapV, mapK2, mapV2, P);
-        }
-        if (cudaGetLastError() != cudaSuccess) return SA2_ERR_CUDA;
+inline int bwd(const KernelParams &kp, const sa2_shape &s, void *extra, cudaStream_t st, int phases = 0) {
+    if (!bwd_addressable(kp)) return SA2_ERR_INVALID;
+    switch (s.d) {
+        case 32: return bwd_launch<32>(kp, s, extra, st, phases);
+        case 64: return bwd_launch<64>(kp, s, extra, st, phases);
+        default: return bwd_launch<128>(kp, s, extra, st, phases);
     }
-
-    if (!(phases & SA2_BWD_Q)) return SA2_OK;
-    if (bq_supported(s))
-        return s.d == 128 ? bwd_q_launch<128>(kp, s, mapK, mapV, c, status, extra, st)
-                          : bwd_q_launch<64>(kp, s, mapK, mapV, c, status, extra, st);
-    return s.d == 128 ? bwd_q_simt<128>(kp, st) : bwd_q_simt<64>(kp, st);
 }
 
 }  // namespace tc

@@ -1,5 +1,5 @@
 // Backward kernel for dK1 / dV1 on tcgen05 tensor cores (bf16 operands, fp32
-// accumulation in TMEM, head dim 64).
+// accumulation in TMEM, head dims 32 and 64).
 //
 // One CTA owns 128 rows j of K1/V1 of one (batch, kv head); the tile stays in
 // shared memory and dK1/dV1 for those rows accumulate in TMEM for the whole
@@ -30,6 +30,12 @@
 // G^T (bf16) [288+64h, +32); dK1 [384,448); dV1 [448,512).  P^T/G^T have their own
 // columns so that the next S^T/dP^T of a half can be issued as soon as the compute
 // group has read the current one.
+//
+// The offsets may be split over several CTAs per key tile (consecutive ranges): a short sequence has few key tiles, and
+// with grouped-query heads each walks over every head of its group.  The splits write fp32 partials, which the
+// reduction of the dQ/dK2/dV2 kernel adds in order.  k1_split() picks the number.  (Splits as the CTAs of a cluster,
+// added through distributed shared memory, cost 20 to 35 % at large grids: a cluster waits for its SMs to be free
+// together.)  Measured: b1 n3001 h8/2 d64 w1024/16 0.78 -> SPLIT_LW ms, b2 n128 h4 d64 w64/32 58 -> SPLIT_ST us.
 #pragma once
 #include "sa2_tc_common.cuh"
 
@@ -61,6 +67,10 @@ enum { ERR_BK1_PRODUCER = 16, ERR_BK1_MMA = 32, ERR_BK1_COMPUTE = 64, ERR_BK1_BU
 struct BwdParams {
     KernelParams kp;
     float c;        // scale * log2(e)
+    int ce;         // CTAs that share a key tile: si x (splits of the offsets)
+    int si;         // splits of the (query head, query tile) pairs
+    int epc;        // second-key offsets of a CTA
+    float *part;    // ce > 1: partial dK1, dV1 [ce][b][nk1][hk][2][d]
     int *status;
 };
 
@@ -72,22 +82,31 @@ inline size_t bk1_smem_bytes() {
 
 struct Bk1Geom {
     int j0, i_lo, i_hi, n_it, total;
+    int e0, e1;     // offsets of this CTA
+    int x0, x1;     // its pairs: x = (query head of the group) * n_it + query tile
 };
 
 __device__ __forceinline__ int bk1_sweeps(const KernelParams &kp, const Bk1Geom &g, int t) {
     const int last = min(g.i_lo + TQ * t + TQ - 1, g.i_hi);
-    return min(kp.w2, last + kp.off2 + 1);
+    return min(g.e1, last + kp.off2 + 1) - g.e0;
 }
 
-__device__ __forceinline__ Bk1Geom bk1_geom(const KernelParams &kp) {
+__device__ __forceinline__ Bk1Geom bk1_geom(const BwdParams &P) {
+    const KernelParams &kp = P.kp;
     Bk1Geom g;
-    g.j0 = blockIdx.x * TJ;
-    g.i_lo = max(0, g.j0 - kp.off1);
+    g.j0 = (int)(blockIdx.x / P.ce) * TJ;
+    const int split = (int)(blockIdx.x % P.ce), is = split % P.si;
+    g.e0 = split / P.si * P.epc;
+    g.e1 = min(kp.w2, g.e0 + P.epc);
+    // (rows before offset e0's first second key have no work here, so every tile has at least one sweep)
+    g.i_lo = max(max(0, g.j0 - kp.off1), g.e0 - kp.off2);
     g.i_hi = min(kp.n - 1, min(g.j0 + TJ - 1, kp.nk1 - 1) + kp.w1 - 1 - kp.off1);
     g.n_it = g.i_hi >= g.i_lo ? (g.i_hi - g.i_lo) / TQ + 1 : 0;
-    int per_head = 0;
-    for (int t = 0; t < g.n_it; ++t) per_head += bk1_sweeps(kp, g, t);
-    g.total = per_head * kp.g;
+    if (g.e0 >= g.e1) g.n_it = 0;
+    g.x0 = g.n_it * kp.g * is / P.si;
+    g.x1 = g.n_it * kp.g * (is + 1) / P.si;
+    g.total = 0;
+    for (int x = g.x0; x < g.x1; ++x) g.total += bk1_sweeps(kp, g, x % g.n_it);
     return g;
 }
 
@@ -104,9 +123,11 @@ __device__ __forceinline__ uint4 split3_bf16(float x) {
     return v;
 }
 
+template <int D>
 __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g, const CUtensorMap *mapK2, const CUtensorMap *mapV2,
                                            uint8_t *sAB, uint8_t *sStat, uint8_t *sOnes, uint8_t *sWin,
                                            uint64_t *bars, volatile int *abort_flag) {
+    constexpr int NC = D / 8;              // 16-byte chunks of a row
     const KernelParams &kp = P.kp;
     const int r = threadIdx.x - 320;       // row of the query tile
     const int hk = blockIdx.y, b = blockIdx.z;
@@ -123,85 +144,83 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
     }
     const float inv_c = 1.f / P.c;
     int s = 0, tile_counter = 0;
-    for (int hh = 0; hh < kp.g; ++hh) {
-        const int h = hk * kp.g + hh;
-        for (int t = 0; t < g.n_it; ++t, ++tile_counter) {
-            const int i = g.i_lo + TQ * t + r;
-            const bool iv = i <= g.i_hi;
-            const int ne = bk1_sweeps(kp, g, t);
-            // The k2 / v2 rows this query tile pairs with over all sweeps (positions it0 - 32 .. it0 + 127)
-            // are staged once per tile by TMA; every step then reads its rows from shared memory.
-            const bool win = kp.w2 <= 32;
-            if (win) {
-                if (tile_counter > 0) mbar_arrive(&bars[BK1_WIN_FREE]);
-                if (r == 0) {
-                    if (tile_counter > 0 && !mbar_wait(&bars[BK1_WIN_FREE], (tile_counter - 1) & 1, abort_flag)) return ERR_BK1_BUILDER;
-                    mbar_arrive_expect_tx(&bars[BK1_WIN_FULL], 2 * BK1_WIN_ROWS * 128);
-                    const int row0 = g.i_lo + TQ * t + kp.off2 - 32;
-                    for (int bx = 0; bx < BK1_WIN_ROWS / 32; ++bx) {
-                        tma_load_4d(sWin + bx * 4096, mapK2, &bars[BK1_WIN_FULL], 0, hk, row0 + 32 * bx, b);
-                        tma_load_4d(sWin + BK1_WIN_ROWS * 128 + bx * 4096, mapV2, &bars[BK1_WIN_FULL], 0, hk, row0 + 32 * bx, b);
-                    }
+    for (int x = g.x0; x < g.x1; ++x, ++tile_counter) {
+        const int t = x % g.n_it, h = hk * kp.g + x / g.n_it;
+        const int i = g.i_lo + TQ * t + r;
+        const bool iv = i <= g.i_hi;
+        const int ne = bk1_sweeps(kp, g, t);
+        // The k2 / v2 rows this query tile pairs with over all sweeps (positions it0 - e0 - 32 .. it0 - e0 + 127)
+        // are staged once per tile by TMA; every step then reads its rows from shared memory.
+        const bool win = P.epc <= 32;
+        if (win) {
+            if (tile_counter > 0) mbar_arrive(&bars[BK1_WIN_FREE]);
+            if (r == 0) {
+                if (tile_counter > 0 && !mbar_wait(&bars[BK1_WIN_FREE], (tile_counter - 1) & 1, abort_flag)) return ERR_BK1_BUILDER;
+                mbar_arrive_expect_tx(&bars[BK1_WIN_FULL], 2 * BK1_WIN_ROWS * 128);
+                const int row0 = g.i_lo + TQ * t + kp.off2 - g.e0 - 32;
+                for (int bx = 0; bx < BK1_WIN_ROWS / 32; ++bx) {
+                    tma_load_4d(sWin + bx * 4096, mapK2, &bars[BK1_WIN_FULL], 0, hk, row0 + 32 * bx, b);
+                    tma_load_4d(sWin + BK1_WIN_ROWS * 128 + bx * 4096, mapV2, &bars[BK1_WIN_FULL], 0, hk, row0 + 32 * bx, b);
                 }
-                if (!mbar_wait(&bars[BK1_WIN_FULL], tile_counter & 1, abort_flag, 64, 1)) return ERR_BK1_BUILDER;
             }
-            uint4 qv[8], dv[8];
+            if (!mbar_wait(&bars[BK1_WIN_FULL], tile_counter & 1, abort_flag, 64, 1)) return ERR_BK1_BUILDER;
+        }
+        uint4 qv[NC], dv[NC];
 #pragma unroll
-            for (int cc = 0; cc < 8; ++cc) { qv[cc] = make_uint4(0, 0, 0, 0); dv[cc] = make_uint4(0, 0, 0, 0); }
-            float lse2 = 0.f, dl = 0.f;
-            if (iv) {
-                const __nv_bfloat16 *qp = q + elem_off(kp.q, b, i, h);
-                const __nv_bfloat16 *dp = dout + elem_off(kp.dout, b, i, h);
+        for (int cc = 0; cc < NC; ++cc) { qv[cc] = make_uint4(0, 0, 0, 0); dv[cc] = make_uint4(0, 0, 0, 0); }
+        float lse2 = 0.f, dl = 0.f;
+        if (iv) {
+            const __nv_bfloat16 *qp = q + elem_off(kp.q, b, i, h);
+            const __nv_bfloat16 *dp = dout + elem_off(kp.dout, b, i, h);
 #pragma unroll
-                for (int cc = 0; cc < 8; ++cc) {
-                    qv[cc] = *reinterpret_cast<const uint4 *>(qp + cc * 8);
-                    dv[cc] = *reinterpret_cast<const uint4 *>(dp + cc * 8);
-                }
-                const int64_t o = ((int64_t)b * kp.hq + h) * kp.n + i;
-                lse2 = kp.lse[o] * 1.4426950408889634f;
-                dl = kp.delta[o];
+            for (int cc = 0; cc < NC; ++cc) {
+                qv[cc] = *reinterpret_cast<const uint4 *>(qp + cc * 8);
+                dv[cc] = *reinterpret_cast<const uint4 *>(dp + cc * 8);
             }
-            for (int e = 0; e < ne; ++e, ++s) {
-                const int stage = s % BK1_STAGES;
-                if (s >= BK1_STAGES && !warp_wait(&bars[BK1_AB_EMPTY + stage], (s / BK1_STAGES - 1) & 1, abort_flag, 2)) return ERR_BK1_BUILDER;
-                if (e == 0) {
-                    // Statistics of this query tile: two K = 16 slabs (-lse2/c, -D) of a four-slab tile; two
-                    // such tiles hold the last four query tiles.  Step s - 3 has completed, and every tile has
-                    // at least one step, so the slabs of four tiles ago are no longer read.
-                    uint8_t *st = sStat + (size_t)((tile_counter >> 1) & 1) * TILE_BYTES;
-                    const int c0 = (tile_counter & 1) * 4;
-                    *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0)) = split3_bf16(-lse2 * inv_c);
-                    *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 1)) = make_uint4(0u, 0u, 0u, 0u);
-                    *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 2)) = split3_bf16(-dl);
-                    *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 3)) = make_uint4(0u, 0u, 0u, 0u);
-                }
-                uint8_t *dA = sAB + (size_t)stage * 2 * TILE_BYTES;
-                uint8_t *dB = dA + TILE_BYTES;
-                const int kk = i + kp.off2 - e;
-                const bool ok = iv && kk >= 0;
-                const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-                const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk);
-                const int wr = r + 32 - e;                       // row of the staged window
-                const uint8_t *wk = sWin + wr * 128, *wv = wk + BK1_WIN_ROWS * 128;
-#pragma unroll
-                for (int cc = 0; cc < 8; ++cc) {
-                    uint4 a = make_uint4(0, 0, 0, 0), bb = make_uint4(0, 0, 0, 0);
-                    if (ok) {
-                        const uint4 kv = win ? *reinterpret_cast<const uint4 *>(wk + ((cc ^ (wr & 7)) << 4))
-                                             : *reinterpret_cast<const uint4 *>(kp2 + cc * 8);
-                        const uint4 vv = win ? *reinterpret_cast<const uint4 *>(wv + ((cc ^ (wr & 7)) << 4))
-                                             : *reinterpret_cast<const uint4 *>(vp2 + cc * 8);
-                        a.x = mul_bf16x2(qv[cc].x, kv.x); a.y = mul_bf16x2(qv[cc].y, kv.y);
-                        a.z = mul_bf16x2(qv[cc].z, kv.z); a.w = mul_bf16x2(qv[cc].w, kv.w);
-                        bb.x = mul_bf16x2(dv[cc].x, vv.x); bb.y = mul_bf16x2(dv[cc].y, vv.y);
-                        bb.z = mul_bf16x2(dv[cc].z, vv.z); bb.w = mul_bf16x2(dv[cc].w, vv.w);
-                    }
-                    *reinterpret_cast<uint4 *>(dA + sw128_offset(r, cc)) = a;
-                    *reinterpret_cast<uint4 *>(dB + sw128_offset(r, cc)) = bb;
-                }
-                fence_proxy_async_smem();
-                mbar_arrive(&bars[BK1_AB_FULL + stage]);
+            const int64_t o = ((int64_t)b * kp.hq + h) * kp.n + i;
+            lse2 = kp.lse[o] * 1.4426950408889634f;
+            dl = kp.delta[o];
+        }
+        for (int e = 0; e < ne; ++e, ++s) {
+            const int stage = s % BK1_STAGES;
+            if (s >= BK1_STAGES && !warp_wait(&bars[BK1_AB_EMPTY + stage], (s / BK1_STAGES - 1) & 1, abort_flag, 2)) return ERR_BK1_BUILDER;
+            if (e == 0) {
+                // Statistics of this query tile: two K = 16 slabs (-lse2/c, -D) of a four-slab tile; two
+                // such tiles hold the last four query tiles.  Step s - 3 has completed, and every tile has
+                // at least one step, so the slabs of four tiles ago are no longer read.
+                uint8_t *st = sStat + (size_t)((tile_counter >> 1) & 1) * TILE_BYTES;
+                const int c0 = (tile_counter & 1) * 4;
+                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0)) = split3_bf16(-lse2 * inv_c);
+                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 1)) = make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 2)) = split3_bf16(-dl);
+                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 3)) = make_uint4(0u, 0u, 0u, 0u);
             }
+            uint8_t *dA = sAB + (size_t)stage * 2 * TILE_BYTES;
+            uint8_t *dB = dA + TILE_BYTES;
+            const int kk = i + kp.off2 - g.e0 - e;
+            const bool ok = iv && kk >= 0;
+            const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
+            const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk);
+            const int wr = r + 32 - e;                       // row of the staged window
+            const uint8_t *wk = sWin + wr * 128, *wv = wk + BK1_WIN_ROWS * 128;
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc) {
+                uint4 a = make_uint4(0, 0, 0, 0), bb = make_uint4(0, 0, 0, 0);
+                if (ok) {
+                    const uint4 kv = win ? *reinterpret_cast<const uint4 *>(wk + ((cc ^ (wr & 7)) << 4))
+                                         : *reinterpret_cast<const uint4 *>(kp2 + cc * 8);
+                    const uint4 vv = win ? *reinterpret_cast<const uint4 *>(wv + ((cc ^ (wr & 7)) << 4))
+                                         : *reinterpret_cast<const uint4 *>(vp2 + cc * 8);
+                    a.x = mul_bf16x2(qv[cc].x, kv.x); a.y = mul_bf16x2(qv[cc].y, kv.y);
+                    a.z = mul_bf16x2(qv[cc].z, kv.z); a.w = mul_bf16x2(qv[cc].w, kv.w);
+                    bb.x = mul_bf16x2(dv[cc].x, vv.x); bb.y = mul_bf16x2(dv[cc].y, vv.y);
+                    bb.z = mul_bf16x2(dv[cc].z, vv.z); bb.w = mul_bf16x2(dv[cc].w, vv.w);
+                }
+                *reinterpret_cast<uint4 *>(dA + sw128_offset(r, cc)) = a;
+                *reinterpret_cast<uint4 *>(dB + sw128_offset(r, cc)) = bb;
+            }
+            fence_proxy_async_smem();
+            mbar_arrive(&bars[BK1_AB_FULL + stage]);
         }
     }
     return 0;
@@ -213,6 +232,7 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
 // The two products have an issuing thread each: the time from "the compute group has read the buffer" to
 // "the next S^T / dP^T are complete" is on the critical chain of every step, and one thread issues only
 // one tcgen05.mma per 60-100 cycles.
+template <int D>
 __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Geom &g, int which, uint32_t tmem, uint8_t *sKV,
                                              uint8_t *sAB, uint8_t *sStat, uint8_t *sOnes, uint64_t *bars, volatile int *abort_flag) {
     constexpr uint32_t IDESC_F = idesc_bf16(128, 64, false, false);
@@ -221,30 +241,27 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
     const uint64_t dSt = smem_desc_sw128(smem_u32(sStat)), dOnes = smem_desc_sw128(smem_u32(sOnes));
     if (!mbar_wait_warp(&bars[BK1_KV_FULL], 0, abort_flag)) return ERR_BK1_MMA;
     int s = 0, tile_counter = 0;
-    for (int hh = 0; hh < kp.g; ++hh) {
-        for (int t = 0; t < g.n_it; ++t, ++tile_counter) {
-            const int ne = bk1_sweeps(kp, g, t);
-            // slab (16 channels = 32 bytes = 2 descriptor units) of the statistics tile that holds this query tile
-            const uint64_t stL0 = dSt + (uint64_t)((((tile_counter >> 1) & 1) * TILE_BYTES) >> 4) + (uint64_t)((tile_counter & 1) * 4);
-            for (int e = 0; e < ne; ++e, ++s) {
-                const int stage = s % BK1_STAGES;
-                if (!mbar_wait_warp(&bars[BK1_AB_FULL + stage], (s / BK1_STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
+    for (int x = g.x0; x < g.x1; ++x, ++tile_counter) {
+        const int t = x % g.n_it;
+        const int ne = bk1_sweeps(kp, g, t);
+        // slab (16 channels = 32 bytes = 2 descriptor units) of the statistics tile that holds this query tile
+        const uint64_t stL0 = dSt + (uint64_t)((((tile_counter >> 1) & 1) * TILE_BYTES) >> 4) + (uint64_t)((tile_counter & 1) * 4);
+        for (int e = 0; e < ne; ++e, ++s) {
+            const int stage = s % BK1_STAGES;
+            if (!mbar_wait_warp(&bars[BK1_AB_FULL + stage], (s / BK1_STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    // the compute group must have read the previous step's S^T / dP^T of this half
-                    if (s >= 1 && !mbar_wait_warp(&bars[BK1_P_FULL + half], (s - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
-                    tc_fence_after();
-                    const uint64_t a = dAB + (uint64_t)((stage * 2 * TILE_BYTES + half * 8192) >> 4);
-                    const uint64_t st = stL0 + (uint64_t)((half * 8192) >> 4) + (uint64_t)(which * 2);
-                    const uint32_t d = tmem + half * 128 + which * 64;
-                    if (elect_one()) {
-                    mma_ss(d, dT, a, IDESC_F, 0u);
-                    mma_ss(d, dT + 2, a + 2, IDESC_F, 1u);
-                    mma_ss(d, dT + 4, a + 4, IDESC_F, 1u);
-                    mma_ss(d, dT + 6, a + 6, IDESC_F, 1u);
-                    mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
-                    tc_commit(&bars[BK1_S_FULL + half]);
-                    }
+            for (int half = 0; half < 2; ++half) {
+                // the compute group must have read the previous step's S^T / dP^T of this half
+                if (s >= 1 && !mbar_wait_warp(&bars[BK1_P_FULL + half], (s - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
+                tc_fence_after();
+                const uint64_t a = dAB + (uint64_t)((stage * 2 * TILE_BYTES + half * 8192) >> 4);
+                const uint64_t st = stL0 + (uint64_t)((half * 8192) >> 4) + (uint64_t)(which * 2);
+                const uint32_t d = tmem + half * 128 + which * 64;
+                if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < D / 16; ++k) mma_ss(d, dT + 2 * k, a + 2 * k, IDESC_F, k > 0 ? 1u : 0u);
+                mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
+                tc_commit(&bars[BK1_S_FULL + half]);
                 }
             }
         }
@@ -253,8 +270,9 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
 }
 
 // ---------------------------------------------------------------- issuer of dV1, dK1 (warp 0, one lane)
+template <int D>
 __device__ __forceinline__ int bk1_mma_second(const Bk1Geom &g, uint32_t tmem, uint8_t *sAB, uint64_t *bars, volatile int *abort_flag) {
-    constexpr uint32_t IDESC_G = idesc_bf16(128, 64, false, true);    // B operand MN-major
+    constexpr uint32_t IDESC_G = idesc_bf16(128, D, false, true);    // B operand MN-major
     const uint64_t dAB = smem_desc_sw128(smem_u32(sAB));
     for (int s = 0; s < g.total; ++s) {
         const int stage = s % BK1_STAGES;
@@ -284,6 +302,7 @@ __device__ __forceinline__ int bk1_mma_second(const Bk1Geom &g, uint32_t tmem, u
 }
 
 // ---------------------------------------------------------------- compute (group h = half h: warps 2-5, 6-9)
+template <int D>
 __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g, int half, uint32_t tmem,
                                            uint64_t *bars, volatile int *abort_flag) {
     const KernelParams &kp = P.kp;
@@ -298,58 +317,57 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
 
     // the walk over the steps; a wait that runs out ends it early, the rows are then reported as NaN below
     auto walk = [&]() -> int {
-        int s = 0, tile_counter = 0;
-        for (int hh = 0; hh < kp.g; ++hh) {
-            for (int t = 0; t < g.n_it; ++t, ++tile_counter) {
-                const int it0 = g.i_lo + TQ * t;
-                const int ne = bk1_sweeps(kp, g, t);
-                const int base = j - kp.off1 - it0;                       // column of the diagonal i + off1 == j
-                const int hi = (jv ? min(min(TQ - 1, base + kp.w1 - 1), g.i_hi - it0) : -1) - half * 64;
-                for (int e = 0; e < ne; ++e, ++s) {
-                    const int lo = max(max(0, base), e - kp.off2 - it0) - half * 64;     // valid columns: lo <= col <= hi
-                    if (!warp_wait(&bars[BK1_S_FULL + half], s & 1, abort_flag, 1)) return ERR_BK1_COMPUTE;
-                    tc_fence_after();
-                    const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 63);
-                    // P^T / G^T of the previous step must have been consumed before they are overwritten
-                    if (s >= 1 && !warp_wait(&bars[BK1_G_DONE + half], (s - 1) & 1, abort_flag, 2)) return ERR_BK1_COMPUTE;
+        int s = 0;
+        for (int xt = g.x0; xt < g.x1; ++xt) {
+            const int t = xt % g.n_it;
+            const int it0 = g.i_lo + TQ * t;
+            const int ne = bk1_sweeps(kp, g, t);
+            const int base = j - kp.off1 - it0;                       // column of the diagonal i + off1 == j
+            const int hi = (jv ? min(min(TQ - 1, base + kp.w1 - 1), g.i_hi - it0) : -1) - half * 64;
+            for (int e = 0; e < ne; ++e, ++s) {
+                const int lo = max(max(0, base), g.e0 + e - kp.off2 - it0) - half * 64;     // valid columns: lo <= col <= hi
+                if (!warp_wait(&bars[BK1_S_FULL + half], s & 1, abort_flag, 1)) return ERR_BK1_COMPUTE;
+                tc_fence_after();
+                const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 63);
+                // P^T / G^T of the previous step must have been consumed before they are overwritten
+                if (s >= 1 && !warp_wait(&bars[BK1_G_DONE + half], (s - 1) & 1, abort_flag, 2)) return ERR_BK1_COMPUTE;
 #pragma unroll
-                    for (int ch = 0; ch < 2; ++ch) {
-                        uint32_t sv[32], dv[32], pk[16], gk[16];
-                        tmem_ld32(buf + ch * 32, sv);
-                        tmem_ld32(buf + 64 + ch * 32, dv);
-                        tmem_wait_ld();
-                        // the accumulators already hold S^T - lse2 / c and dP^T - D
-                        if (full) {
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t sv[32], dv[32], pk[16], gk[16];
+                    tmem_ld32(buf + ch * 32, sv);
+                    tmem_ld32(buf + 64 + ch * 32, dv);
+                    tmem_wait_ld();
+                    // the accumulators already hold S^T - lse2 / c and dP^T - D
+                    if (full) {
 #pragma unroll
-                            for (int x = 0; x < 32; x += 2) {
-                                const float p0 = ex2(__uint_as_float(sv[x]) * c);
-                                const float p1 = ex2(__uint_as_float(sv[x + 1]) * c);
-                                pk[x >> 1] = pack_bf16(p0, p1);
-                                gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
-                            }
-                        } else {
-                            // valid columns are the integers in [lo, hi]: saturate(half + 1 - |col - mid|) is
-                            // exactly 1 inside and 0 outside (FMA pipe instead of compares and selects on the
-                            // ALU pipe); the exponent is clamped so that a masked-out cell cannot give inf * 0
-                            const float mid = 0.5f * (float)(lo + hi), hwp = 0.5f * (float)(hi - lo) + 1.f;
-#pragma unroll
-                            for (int x = 0; x < 32; x += 2) {
-                                const int col = ch * 32 + x;
-                                const float v0 = __saturatef(hwp - fabsf((float)col - mid));
-                                const float v1 = __saturatef(hwp - fabsf((float)(col + 1) - mid));
-                                const float p0 = ex2(fminf(__uint_as_float(sv[x]) * c, 100.f)) * v0;
-                                const float p1 = ex2(fminf(__uint_as_float(sv[x + 1]) * c, 100.f)) * v1;
-                                pk[x >> 1] = pack_bf16(p0, p1);
-                                gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
-                            }
+                        for (int x = 0; x < 32; x += 2) {
+                            const float p0 = ex2(__uint_as_float(sv[x]) * c);
+                            const float p1 = ex2(__uint_as_float(sv[x + 1]) * c);
+                            pk[x >> 1] = pack_bf16(p0, p1);
+                            gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
                         }
-                        tmem_st16(pg + ch * 16, pk);
-                        tmem_st16(pg + 32 + ch * 16, gk);
+                    } else {
+                        // valid columns are the integers in [lo, hi]: saturate(half + 1 - |col - mid|) is
+                        // exactly 1 inside and 0 outside (FMA pipe instead of compares and selects on the
+                        // ALU pipe); the exponent is clamped so that a masked-out cell cannot give inf * 0
+                        const float mid = 0.5f * (float)(lo + hi), hwp = 0.5f * (float)(hi - lo) + 1.f;
+#pragma unroll
+                        for (int x = 0; x < 32; x += 2) {
+                            const int col = ch * 32 + x;
+                            const float v0 = __saturatef(hwp - fabsf((float)col - mid));
+                            const float v1 = __saturatef(hwp - fabsf((float)(col + 1) - mid));
+                            const float p0 = ex2(fminf(__uint_as_float(sv[x]) * c, 100.f)) * v0;
+                            const float p1 = ex2(fminf(__uint_as_float(sv[x + 1]) * c, 100.f)) * v1;
+                            pk[x >> 1] = pack_bf16(p0, p1);
+                            gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
+                        }
                     }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    mbar_arrive(&bars[BK1_P_FULL + half]);
+                    tmem_st16(pg + ch * 16, pk);
+                    tmem_st16(pg + 32 + ch * 16, gk);
                 }
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive(&bars[BK1_P_FULL + half]);
             }
         }
         return 0;
@@ -363,11 +381,22 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
     const TensorRef &dst = half == 0 ? kp.dk1 : kp.dv1;
     const float mul = half == 0 ? kp.scale : 1.f;
 #pragma unroll 1
-    for (int hf = 0; hf < 2; ++hf) {
+    for (int hf = 0; hf < D / 32; ++hf) {
         uint32_t w[32];
         tmem_ld32(lane_addr + 384 + half * 64 + hf * 32, w);
         tmem_wait_ld();
-        if (jv) {
+        if (P.ce > 1 && jv) {
+            float *row = P.part + (((((size_t)(blockIdx.x % P.ce) * kp.b + b) * kp.nk1 + j) * kp.hk + hk) * 2 + half) * D + hf * 32;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                float4 x;
+                x.x = __uint_as_float(w[u * 4]); x.y = __uint_as_float(w[u * 4 + 1]);
+                x.z = __uint_as_float(w[u * 4 + 2]); x.w = __uint_as_float(w[u * 4 + 3]);
+                if (g.total == 0) x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (bad) x = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F);
+                *reinterpret_cast<float4 *>(row + u * 4) = x;
+            }
+        } else if (jv) {
             const int64_t off = elem_off(dst, b, j, hk) + hf * 32;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -381,6 +410,7 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
     return err;
 }
 
+template <int D>
 __global__ void __launch_bounds__(BK1_THREADS, 1)
 bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
               const __grid_constant__ CUtensorMap mapK2, const __grid_constant__ CUtensorMap mapV2, const BwdParams P) {
@@ -415,7 +445,7 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_holder;
-    const Bk1Geom g = bk1_geom(P.kp);
+    const Bk1Geom g = bk1_geom(P);
 
     int err = 0;
 #ifdef SA2_PROF
@@ -431,20 +461,20 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
                 tma_load_4d(sK, &mapK, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
                 tma_load_4d(sV, &mapV, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
             }
-            err = bk1_mma_second(g, tmem, sAB, bars, abort_flag);
+            err = bk1_mma_second<D>(g, tmem, sAB, bars, abort_flag);
             // the tile must have landed before the CTA may exit, even if every other role gave up
             if (!mbar_wait_warp(&bars[BK1_KV_FULL], 0, abort_flag)) err |= ERR_BK1_PRODUCER;
         } else if (elect_one()) {
             tc_commit(&bars[BK1_DONE]);
         }
     } else if (warp == 1) {
-        if (g.total > 0) err = bk1_mma_first(P.kp, g, 0, tmem, sK, sAB, sStat, sOnes, bars, abort_flag);
+        if (g.total > 0) err = bk1_mma_first<D>(P.kp, g, 0, tmem, sK, sAB, sStat, sOnes, bars, abort_flag);
     } else if (warp == 14) {
-        if (g.total > 0) err = bk1_mma_first(P.kp, g, 1, tmem, sV, sAB, sStat, sOnes, bars, abort_flag);
+        if (g.total > 0) err = bk1_mma_first<D>(P.kp, g, 1, tmem, sV, sAB, sStat, sOnes, bars, abort_flag);
     } else if (warp < 10) {
-        err = bk1_compute(P, g, (warp - 2) >> 2, tmem, bars, abort_flag);
+        err = bk1_compute<D>(P, g, (warp - 2) >> 2, tmem, bars, abort_flag);
     } else {
-        err = bk1_builder(P, g, &mapK2, &mapV2, sAB, sStat, sOnes, sWin, bars, abort_flag);
+        err = bk1_builder<D>(P, g, &mapK2, &mapV2, sAB, sStat, sOnes, sWin, bars, abort_flag);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
@@ -456,6 +486,36 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
         tc_fence_after();
         tmem_dealloc(tmem, 512);
     }
+}
+
+// ------------------------------------------------------------------ host side
+// The weight of splitting work into `ctas` CTAs per batch element of `one` cycles each: whole waves of one CTA per SM.  A
+// result must not depend, to the last bit, on what else rides in the call, so the rules weigh one batch element (where
+// splitting fills the chip) and eight (where it costs set-up).
+inline double split_cost(int64_t ctas, double one, int sms) {
+    return (double)((ctas + sms - 1) / sms) * one * ((double)((ctas * 8 + sms - 1) / sms) * one);
+}
+// CTAs per key tile: splits of the (query head, query tile) pairs first, then of the offsets.  A CTA costs ~8000 cycles
+// of set-up, loads and store, a pair ~4000 (its rows and second-key window), a step of 128 query rows and one offset
+// ~2600 (twice that at head dim 128), measured on a B200.
+struct K1Split { int si, se, epc; };
+inline K1Split k1_split(const sa2_shape &s, int sms) {
+    const int nk1 = s.n + s.off1, rows = s.w1 + TJ - 1 < s.n ? s.w1 + TJ - 1 : s.n;
+    const int64_t tiles = (int64_t)((nk1 + TJ - 1) / TJ) * s.hk;
+    const int pairs = (s.hq / s.hk) * ((rows + TQ - 1) / TQ), w2 = s.w2 < s.n + s.off2 ? s.w2 : s.n + s.off2;
+    const double step = s.d == 128 ? 5200. : 2600.;
+    K1Split best{1, 1, w2};
+    double best_cost = 0.;
+    for (int se = 1; se <= 16 && se <= w2; ++se)
+        for (int si = 1; si * se <= 16 && si <= pairs; ++si) {
+            const int epc = (w2 + se - 1) / se;
+            const double cost = split_cost(tiles * si * se, 8000. + (pairs + si - 1) / si * (4000. + epc * step), sms);
+            if (best_cost == 0. || cost < 0.94 * best_cost) { best = K1Split{si, (w2 + epc - 1) / epc, epc}; best_cost = cost; }
+        }
+    return best;
+}
+inline size_t k1_part_bytes(const sa2_shape &s, int ce) {
+    return ce == 1 ? 0 : (size_t)ce * s.b * (s.n + s.off1) * s.hk * 2 * s.d * sizeof(float);
 }
 
 }  // namespace tc

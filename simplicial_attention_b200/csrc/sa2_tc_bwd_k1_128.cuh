@@ -84,6 +84,10 @@ __device__ __forceinline__ int stat_chunk(int slot, int which) { return slot < 2
 struct Params {
     KernelParams kp;
     float c;        // scale * log2(e)
+    int ce;         // CTAs that share a key tile: si x (splits of the offsets)
+    int si;         // splits of the (query head, query block) pairs
+    int epc;        // second-key offsets of a CTA
+    float *part;    // ce > 1: partial dK1, dV1 [ce][b][nk1][hk][2][d]
     int n_split;    // diagnostic: issue the second products as two N = 64 products instead of one N = 128
     int *status;
 };
@@ -94,23 +98,32 @@ inline size_t smem_bytes() {
 
 struct Geom {
     int j0, i_lo, i_hi, n_ib, total;
+    int e0, e1;     // offsets of this CTA
+    int x0, x1;     // its pairs: x = (query head of the group) * n_ib + query block
 };
 
 // sweeps of query block ib (rows i_lo + 64 ib ...)
 __device__ __forceinline__ int block_sweeps(const KernelParams &kp, const Geom &g, int ib) {
     const int last = min(g.i_lo + QB * ib + QB - 1, g.i_hi);
-    return min(kp.w2, last + kp.off2 + 1);
+    return min(g.e1, last + kp.off2 + 1) - g.e0;
 }
 
-__device__ __forceinline__ Geom geom(const KernelParams &kp) {
+__device__ __forceinline__ Geom geom(const Params &P) {
+    const KernelParams &kp = P.kp;
     Geom g;
-    g.j0 = blockIdx.x * TJ;
-    g.i_lo = max(0, g.j0 - kp.off1);
+    g.j0 = (int)(blockIdx.x / P.ce) * TJ;
+    const int split = (int)(blockIdx.x % P.ce), is = split % P.si;
+    g.e0 = split / P.si * P.epc;
+    g.e1 = min(kp.w2, g.e0 + P.epc);
+    // (rows before offset e0's first second key have no work here, so every block has at least one sweep)
+    g.i_lo = max(max(0, g.j0 - kp.off1), g.e0 - kp.off2);
     g.i_hi = min(kp.n - 1, min(g.j0 + TJ - 1, kp.nk1 - 1) + kp.w1 - 1 - kp.off1);
     g.n_ib = g.i_hi >= g.i_lo ? (g.i_hi - g.i_lo) / QB + 1 : 0;
-    int per_head = 0;
-    for (int ib = 0; ib < g.n_ib; ++ib) per_head += block_sweeps(kp, g, ib);
-    g.total = per_head * kp.g;
+    if (g.e0 >= g.e1) g.n_ib = 0;
+    g.x0 = g.n_ib * kp.g * is / P.si;
+    g.x1 = g.n_ib * kp.g * (is + 1) / P.si;
+    g.total = 0;
+    for (int x = g.x0; x < g.x1; ++x) g.total += block_sweeps(kp, g, x % g.n_ib);
     return g;
 }
 
@@ -134,86 +147,84 @@ __device__ __forceinline__ int builder(const Params &P, const Geom &g, const CUt
         *reinterpret_cast<uint4 *>(sConst + sw128_offset(bt, 1)) = make_uint4(0u, 0u, 0u, 0u);
     }
     const float inv_c = 1.f / P.c;
-    const bool win = kp.w2 <= 32;
+    const bool win = P.epc <= 32;
     int s = 0, blk = 0;
-    for (int hh = 0; hh < kp.g; ++hh) {
-        const int h = hk * kp.g + hh;
-        for (int ib = 0; ib < g.n_ib; ++ib, ++blk) {
-            const int it0 = g.i_lo + QB * ib;
-            const int i = it0 + r;
-            const bool iv = i <= g.i_hi;
-            const int ne = block_sweeps(kp, g, ib);
-            if (win) {
-                // The k2 / v2 rows this query block pairs with over all sweeps (positions it0 - 32 .. it0 + 63)
-                // are staged once per block by TMA; every step then reads its rows from shared memory.
-                if (blk > 0) mbar_arrive(&bars[B_WIN_FREE]);
-                if (bt == 0) {
-                    if (blk > 0 && !mbar_wait(&bars[B_WIN_FREE], (blk - 1) & 1, abort_flag)) return ERR_BK1_BUILDER;
-                    mbar_arrive_expect_tx(&bars[B_WIN_FULL], 2 * WIN_BYTES);
-                    const int row0 = it0 + kp.off2 - 32;
-                    for (int bx = 0; bx < WIN_ROWS / 32; ++bx)
-                        for (int c2 = 0; c2 < 2; ++c2) {
-                            tma_load_4d(sWin + c2 * WBLK_BYTES + bx * 4096, mapK2, &bars[B_WIN_FULL], c2 * 64, hk, row0 + 32 * bx, b);
-                            tma_load_4d(sWin + WIN_BYTES + c2 * WBLK_BYTES + bx * 4096, mapV2, &bars[B_WIN_FULL], c2 * 64, hk, row0 + 32 * bx, b);
-                        }
-                }
-            }
-            uint4 qv[4], dv[4];
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) { qv[cc] = make_uint4(0, 0, 0, 0); dv[cc] = make_uint4(0, 0, 0, 0); }
-            float stat = 0.f;       // part 0: -lse2 / c, part 1: -D
-            if (iv) {
-                const __nv_bfloat16 *qp = q + elem_off(kp.q, b, i, h) + part * 32;
-                const __nv_bfloat16 *dp = dout + elem_off(kp.dout, b, i, h) + part * 32;
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    qv[cc] = __ldg(reinterpret_cast<const uint4 *>(qp + cc * 8));
-                    dv[cc] = __ldg(reinterpret_cast<const uint4 *>(dp + cc * 8));
-                }
-                const int64_t o = ((int64_t)b * kp.hq + h) * kp.n + i;
-                if (part == 0) stat = -kp.lse[o] * 1.4426950408889634f * inv_c;
-                else if (part == 1) stat = -kp.delta[o];
-            }
-            if (win && !mbar_wait(&bars[B_WIN_FULL], blk & 1, abort_flag, 64, 1)) return ERR_BK1_BUILDER;
-            for (int e = 0; e < ne; ++e, ++s) {
-                const int stage = s % STAGES;
-                // the stage is free once the second products of three steps ago have completed
-                if (s >= STAGES && !warp_wait(&bars[B_AB_EMPTY + stage], (s / STAGES - 1) & 1, abort_flag, 2)) return ERR_BK1_BUILDER;
-                if (e == 0 && part < 2) {
-                    // Statistics of this query block (K = 16 slabs of -lse2/c and of -D) in slot blk % 3.  Step
-                    // s - 3 has completed and every block has at least one step, so the slabs of three blocks ago
-                    // are no longer read.
-                    const int row = stat_row(blk % 3, part, r), ch = stat_chunk(blk % 3, part);
-                    *reinterpret_cast<uint4 *>(sConst + sw128_offset(row, ch)) = split3_bf16(stat);
-                    *reinterpret_cast<uint4 *>(sConst + sw128_offset(row, ch + 1)) = make_uint4(0u, 0u, 0u, 0u);
-                }
-                uint8_t *dA = sAB + (size_t)stage * STAGE_BYTES + (size_t)cb * QBLK_BYTES;
-                uint8_t *dB = dA + AB_BYTES;
-                const int kk = i + kp.off2 - e;
-                const bool ok = iv && kk >= 0;
-                const int wr = r + 32 - e;                       // row of the staged window
-                const uint8_t *wk = sWin + cb * WBLK_BYTES + wr * 128, *wv = wk + WIN_BYTES;
-                const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk) + part * 32;
-                const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk) + part * 32;
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    uint4 a = make_uint4(0, 0, 0, 0), bb = make_uint4(0, 0, 0, 0);
-                    if (ok) {
-                        const uint4 kv = win ? *reinterpret_cast<const uint4 *>(wk + (((ch0 + cc) ^ (wr & 7)) << 4))
-                                             : __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8));
-                        const uint4 vv = win ? *reinterpret_cast<const uint4 *>(wv + (((ch0 + cc) ^ (wr & 7)) << 4))
-                                             : __ldg(reinterpret_cast<const uint4 *>(vp2 + cc * 8));
-                        a.x = mul_bf16x2(qv[cc].x, kv.x); a.y = mul_bf16x2(qv[cc].y, kv.y);
-                        a.z = mul_bf16x2(qv[cc].z, kv.z); a.w = mul_bf16x2(qv[cc].w, kv.w);
-                        bb.x = mul_bf16x2(dv[cc].x, vv.x); bb.y = mul_bf16x2(dv[cc].y, vv.y);
-                        bb.z = mul_bf16x2(dv[cc].z, vv.z); bb.w = mul_bf16x2(dv[cc].w, vv.w);
+    for (int x = g.x0; x < g.x1; ++x, ++blk) {
+        const int ib = x % g.n_ib, h = hk * kp.g + x / g.n_ib;
+        const int it0 = g.i_lo + QB * ib;
+        const int i = it0 + r;
+        const bool iv = i <= g.i_hi;
+        const int ne = block_sweeps(kp, g, ib);
+        if (win) {
+            // The k2 / v2 rows this query block pairs with over all sweeps (positions it0 - e0 - 32 .. it0 - e0 + 63)
+            // are staged once per block by TMA; every step then reads its rows from shared memory.
+            if (blk > 0) mbar_arrive(&bars[B_WIN_FREE]);
+            if (bt == 0) {
+                if (blk > 0 && !mbar_wait(&bars[B_WIN_FREE], (blk - 1) & 1, abort_flag)) return ERR_BK1_BUILDER;
+                mbar_arrive_expect_tx(&bars[B_WIN_FULL], 2 * WIN_BYTES);
+                const int row0 = it0 + kp.off2 - g.e0 - 32;
+                for (int bx = 0; bx < WIN_ROWS / 32; ++bx)
+                    for (int c2 = 0; c2 < 2; ++c2) {
+                        tma_load_4d(sWin + c2 * WBLK_BYTES + bx * 4096, mapK2, &bars[B_WIN_FULL], c2 * 64, hk, row0 + 32 * bx, b);
+                        tma_load_4d(sWin + WIN_BYTES + c2 * WBLK_BYTES + bx * 4096, mapV2, &bars[B_WIN_FULL], c2 * 64, hk, row0 + 32 * bx, b);
                     }
-                    *reinterpret_cast<uint4 *>(dA + sw128_offset(r, ch0 + cc)) = a;
-                    *reinterpret_cast<uint4 *>(dB + sw128_offset(r, ch0 + cc)) = bb;
-                }
-                fence_proxy_async_smem();
-                mbar_arrive(&bars[B_AB_FULL + stage]);
             }
+        }
+        uint4 qv[4], dv[4];
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) { qv[cc] = make_uint4(0, 0, 0, 0); dv[cc] = make_uint4(0, 0, 0, 0); }
+        float stat = 0.f;       // part 0: -lse2 / c, part 1: -D
+        if (iv) {
+            const __nv_bfloat16 *qp = q + elem_off(kp.q, b, i, h) + part * 32;
+            const __nv_bfloat16 *dp = dout + elem_off(kp.dout, b, i, h) + part * 32;
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) {
+                qv[cc] = __ldg(reinterpret_cast<const uint4 *>(qp + cc * 8));
+                dv[cc] = __ldg(reinterpret_cast<const uint4 *>(dp + cc * 8));
+            }
+            const int64_t o = ((int64_t)b * kp.hq + h) * kp.n + i;
+            if (part == 0) stat = -kp.lse[o] * 1.4426950408889634f * inv_c;
+            else if (part == 1) stat = -kp.delta[o];
+        }
+        if (win && !mbar_wait(&bars[B_WIN_FULL], blk & 1, abort_flag, 64, 1)) return ERR_BK1_BUILDER;
+        for (int e = 0; e < ne; ++e, ++s) {
+            const int stage = s % STAGES;
+            // the stage is free once the second products of three steps ago have completed
+            if (s >= STAGES && !warp_wait(&bars[B_AB_EMPTY + stage], (s / STAGES - 1) & 1, abort_flag, 2)) return ERR_BK1_BUILDER;
+            if (e == 0 && part < 2) {
+                // Statistics of this query block (K = 16 slabs of -lse2/c and of -D) in slot blk % 3.  Step
+                // s - 3 has completed and every block has at least one step, so the slabs of three blocks ago
+                // are no longer read.
+                const int row = stat_row(blk % 3, part, r), ch = stat_chunk(blk % 3, part);
+                *reinterpret_cast<uint4 *>(sConst + sw128_offset(row, ch)) = split3_bf16(stat);
+                *reinterpret_cast<uint4 *>(sConst + sw128_offset(row, ch + 1)) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            uint8_t *dA = sAB + (size_t)stage * STAGE_BYTES + (size_t)cb * QBLK_BYTES;
+            uint8_t *dB = dA + AB_BYTES;
+            const int kk = i + kp.off2 - g.e0 - e;
+            const bool ok = iv && kk >= 0;
+            const int wr = r + 32 - e;                       // row of the staged window
+            const uint8_t *wk = sWin + cb * WBLK_BYTES + wr * 128, *wv = wk + WIN_BYTES;
+            const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk) + part * 32;
+            const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk) + part * 32;
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) {
+                uint4 a = make_uint4(0, 0, 0, 0), bb = make_uint4(0, 0, 0, 0);
+                if (ok) {
+                    const uint4 kv = win ? *reinterpret_cast<const uint4 *>(wk + (((ch0 + cc) ^ (wr & 7)) << 4))
+                                         : __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8));
+                    const uint4 vv = win ? *reinterpret_cast<const uint4 *>(wv + (((ch0 + cc) ^ (wr & 7)) << 4))
+                                         : __ldg(reinterpret_cast<const uint4 *>(vp2 + cc * 8));
+                    a.x = mul_bf16x2(qv[cc].x, kv.x); a.y = mul_bf16x2(qv[cc].y, kv.y);
+                    a.z = mul_bf16x2(qv[cc].z, kv.z); a.w = mul_bf16x2(qv[cc].w, kv.w);
+                    bb.x = mul_bf16x2(dv[cc].x, vv.x); bb.y = mul_bf16x2(dv[cc].y, vv.y);
+                    bb.z = mul_bf16x2(dv[cc].z, vv.z); bb.w = mul_bf16x2(dv[cc].w, vv.w);
+                }
+                *reinterpret_cast<uint4 *>(dA + sw128_offset(r, ch0 + cc)) = a;
+                *reinterpret_cast<uint4 *>(dB + sw128_offset(r, ch0 + cc)) = bb;
+            }
+            fence_proxy_async_smem();
+            mbar_arrive(&bars[B_AB_FULL + stage]);
         }
     }
     return 0;
@@ -229,29 +240,28 @@ __device__ __forceinline__ int mma_first(const KernelParams &kp, const Geom &g, 
     const uint64_t dOnes = smem_desc_sw128(smem_u32(sConst));
     if (!mbar_wait_warp(&bars[B_KV_FULL], 0, abort_flag)) return ERR_BK1_MMA;
     int s = 0, blk = 0;
-    for (int hh = 0; hh < kp.g; ++hh) {
-        for (int ib = 0; ib < g.n_ib; ++ib, ++blk) {
-            const int ne = block_sweeps(kp, g, ib);
-            // this block's slab of the constant tile (rows are multiples of 64: whole 8-row swizzle groups)
-            const uint64_t st = dOnes + (uint64_t)((stat_row(blk % 3, which, 0) * 128) >> 4) + (uint64_t)stat_chunk(blk % 3, which);
-            for (int e = 0; e < ne; ++e, ++s) {
-                const int stage = s % STAGES, half = s & 1;
-                if (!mbar_wait_warp(&bars[B_AB_FULL + stage], (s / STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
-                // P^T / G^T of the step that used this half last lie over these columns until its second products are done
-                if (s >= 2 && !mbar_wait_warp(&bars[B_G_DONE + half], ((s >> 1) - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
-                tc_fence_after();
-                const uint64_t a = dAB + (uint64_t)((stage * STAGE_BYTES) >> 4);
-                const uint32_t d = tmem + half * 128 + which * 64;
-                if (elect_one()) {
+    for (int x = g.x0; x < g.x1; ++x, ++blk) {
+        const int ib = x % g.n_ib;
+        const int ne = block_sweeps(kp, g, ib);
+        // this block's slab of the constant tile (rows are multiples of 64: whole 8-row swizzle groups)
+        const uint64_t st = dOnes + (uint64_t)((stat_row(blk % 3, which, 0) * 128) >> 4) + (uint64_t)stat_chunk(blk % 3, which);
+        for (int e = 0; e < ne; ++e, ++s) {
+            const int stage = s % STAGES, half = s & 1;
+            if (!mbar_wait_warp(&bars[B_AB_FULL + stage], (s / STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
+            // P^T / G^T of the step that used this half last lie over these columns until its second products are done
+            if (s >= 2 && !mbar_wait_warp(&bars[B_G_DONE + half], ((s >> 1) - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
+            tc_fence_after();
+            const uint64_t a = dAB + (uint64_t)((stage * STAGE_BYTES) >> 4);
+            const uint32_t d = tmem + half * 128 + which * 64;
+            if (elect_one()) {
 #pragma unroll
-                for (int k8 = 0; k8 < 8; ++k8) {
-                    const uint64_t kin = (uint64_t)((k8 & 3) * 2);
-                    mma_ss(d, dT + (uint64_t)(((k8 >> 2) * BLK_BYTES) >> 4) + kin, a + (uint64_t)(((k8 >> 2) * QBLK_BYTES) >> 4) + kin,
-                           IDESC_F, k8 > 0 ? 1u : 0u);
-                }
-                mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
-                tc_commit(&bars[B_S_FULL + half]);
-                }
+            for (int k8 = 0; k8 < 8; ++k8) {
+                const uint64_t kin = (uint64_t)((k8 & 3) * 2);
+                mma_ss(d, dT + (uint64_t)(((k8 >> 2) * BLK_BYTES) >> 4) + kin, a + (uint64_t)(((k8 >> 2) * QBLK_BYTES) >> 4) + kin,
+                       IDESC_F, k8 > 0 ? 1u : 0u);
+            }
+            mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
+            tc_commit(&bars[B_S_FULL + half]);
             }
         }
     }
@@ -313,56 +323,55 @@ __device__ __forceinline__ int compute(const Params &P, const Geom &g, int half,
     // the walk over the steps; a wait that runs out ends it early, the rows are then reported as NaN below
     auto walk = [&]() -> int {
         int s = 0;
-        for (int hh = 0; hh < kp.g; ++hh) {
-            for (int ib = 0; ib < g.n_ib; ++ib) {
-                const int it0 = g.i_lo + QB * ib;
-                const int ne = block_sweeps(kp, g, ib);
-                const int base = j - kp.off1 - it0;                       // column of the diagonal i + off1 == j
-                const int hi = jv ? min(min(QB - 1, base + kp.w1 - 1), g.i_hi - it0) : -1;
-                for (int e = 0; e < ne; ++e, ++s) {
-                    if ((s & 1) != half) continue;
-                    const int lo = max(max(0, base), e - kp.off2 - it0);      // valid columns: lo <= col <= hi
-                    if (!warp_wait(&bars[B_S_FULL + half], (s >> 1) & 1, abort_flag, 1)) return ERR_BK1_COMPUTE;
-                    tc_fence_after();
-                    const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 63);
+        for (int xb = g.x0; xb < g.x1; ++xb) {
+            const int ib = xb % g.n_ib;
+            const int it0 = g.i_lo + QB * ib;
+            const int ne = block_sweeps(kp, g, ib);
+            const int base = j - kp.off1 - it0;                       // column of the diagonal i + off1 == j
+            const int hi = jv ? min(min(QB - 1, base + kp.w1 - 1), g.i_hi - it0) : -1;
+            for (int e = 0; e < ne; ++e, ++s) {
+                if ((s & 1) != half) continue;
+                const int lo = max(max(0, base), g.e0 + e - kp.off2 - it0);      // valid columns: lo <= col <= hi
+                if (!warp_wait(&bars[B_S_FULL + half], (s >> 1) & 1, abort_flag, 1)) return ERR_BK1_COMPUTE;
+                tc_fence_after();
+                const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 63);
 #pragma unroll
-                    for (int ch = 0; ch < 2; ++ch) {
-                        uint32_t sv[32], dv[32], pk[16], gk[16];
-                        tmem_ld32(buf + ch * 32, sv);
-                        tmem_ld32(buf + 64 + ch * 32, dv);
-                        tmem_wait_ld();
-                        // the accumulators already hold S^T - lse2 / c and dP^T - D
-                        if (full) {
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t sv[32], dv[32], pk[16], gk[16];
+                    tmem_ld32(buf + ch * 32, sv);
+                    tmem_ld32(buf + 64 + ch * 32, dv);
+                    tmem_wait_ld();
+                    // the accumulators already hold S^T - lse2 / c and dP^T - D
+                    if (full) {
 #pragma unroll
-                            for (int x = 0; x < 32; x += 2) {
-                                const float p0 = ex2(__uint_as_float(sv[x]) * c);
-                                const float p1 = ex2(__uint_as_float(sv[x + 1]) * c);
-                                pk[x >> 1] = pack_bf16(p0, p1);
-                                gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
-                            }
-                        } else {
-                            // valid columns are the integers in [lo, hi]: saturate(half + 1 - |col - mid|) is exactly
-                            // 1 inside and 0 outside; the exponent is clamped so that a masked-out cell cannot give inf * 0
-                            const float mid = 0.5f * (float)(lo + hi), hwp = 0.5f * (float)(hi - lo) + 1.f;
-#pragma unroll
-                            for (int x = 0; x < 32; x += 2) {
-                                const int col = ch * 32 + x;
-                                const float v0 = __saturatef(hwp - fabsf((float)col - mid));
-                                const float v1 = __saturatef(hwp - fabsf((float)(col + 1) - mid));
-                                const float p0 = ex2(fminf(__uint_as_float(sv[x]) * c, 100.f)) * v0;
-                                const float p1 = ex2(fminf(__uint_as_float(sv[x + 1]) * c, 100.f)) * v1;
-                                pk[x >> 1] = pack_bf16(p0, p1);
-                                gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
-                            }
+                        for (int x = 0; x < 32; x += 2) {
+                            const float p0 = ex2(__uint_as_float(sv[x]) * c);
+                            const float p1 = ex2(__uint_as_float(sv[x + 1]) * c);
+                            pk[x >> 1] = pack_bf16(p0, p1);
+                            gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
                         }
-                        // over columns of S^T / dP^T that this thread has already read
-                        tmem_st16(buf + ch * 16, pk);
-                        tmem_st16(buf + 64 + ch * 16, gk);
+                    } else {
+                        // valid columns are the integers in [lo, hi]: saturate(half + 1 - |col - mid|) is exactly
+                        // 1 inside and 0 outside; the exponent is clamped so that a masked-out cell cannot give inf * 0
+                        const float mid = 0.5f * (float)(lo + hi), hwp = 0.5f * (float)(hi - lo) + 1.f;
+#pragma unroll
+                        for (int x = 0; x < 32; x += 2) {
+                            const int col = ch * 32 + x;
+                            const float v0 = __saturatef(hwp - fabsf((float)col - mid));
+                            const float v1 = __saturatef(hwp - fabsf((float)(col + 1) - mid));
+                            const float p0 = ex2(fminf(__uint_as_float(sv[x]) * c, 100.f)) * v0;
+                            const float p1 = ex2(fminf(__uint_as_float(sv[x + 1]) * c, 100.f)) * v1;
+                            pk[x >> 1] = pack_bf16(p0, p1);
+                            gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
+                        }
                     }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    mbar_arrive(&bars[B_P_FULL + half]);
+                    // over columns of S^T / dP^T that this thread has already read
+                    tmem_st16(buf + ch * 16, pk);
+                    tmem_st16(buf + 64 + ch * 16, gk);
                 }
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive(&bars[B_P_FULL + half]);
             }
         }
         return 0;
@@ -380,7 +389,18 @@ __device__ __forceinline__ int compute(const Params &P, const Geom &g, int half,
         uint32_t w[32];
         tmem_ld32(lane_addr + 256 + half * 128 + q4 * 32, w);
         tmem_wait_ld();
-        if (jv) {
+        if (P.ce > 1 && jv) {
+            float *row = P.part + (((((size_t)(blockIdx.x % P.ce) * kp.b + b) * kp.nk1 + j) * kp.hk + hk) * 2 + half) * 128 + q4 * 32;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                float4 x;
+                x.x = __uint_as_float(w[u * 4]); x.y = __uint_as_float(w[u * 4 + 1]);
+                x.z = __uint_as_float(w[u * 4 + 2]); x.w = __uint_as_float(w[u * 4 + 3]);
+                if (g.total == 0) x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (bad) x = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F);
+                *reinterpret_cast<float4 *>(row + u * 4) = x;
+            }
+        } else if (jv) {
             const int64_t off = elem_off(dst, b, j, hk) + q4 * 32;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -428,7 +448,7 @@ bwd_k1_128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_holder;
-    const Geom g = geom(P.kp);
+    const Geom g = geom(P);
 
     int err = 0;
 #ifdef SA2_PROF

@@ -58,17 +58,18 @@ constexpr int BQ_REGS_LAUNCH = 128, BQ_REGS_ISSUE = 40, BQ_REGS_COMPUTE = 120;
 // sweep or a k2 row and chunks of U and W.  (With one compute group at head dim 128 - NCG = 1 - warps 8-11 form
 // A_e with 144 registers and the fold group keeps 208.)
 template <int D> struct BqCfg {
-    static constexpr int CH = D / 64;                            // channel halves = CTAs per (query tile, split)
+    static constexpr int CH = D == 128 ? 2 : 1;                  // channel halves = CTAs per (query tile, split)
+    static constexpr int CC = D < 64 ? D : 64;                   // channels this CTA produces
     static constexpr int KSTEPS = D / 16;                        // K = 16 steps of S and dP
     static constexpr uint32_t BLK = TJ * 128;                    // A_e / B_e: one [128 rows][64 channels] swizzled block
-    static constexpr uint32_t TILE = (D / 64) * BLK;             // A_e or B_e
+    static constexpr uint32_t TILE = CH * BLK;                   // A_e or B_e
     // K1 / V1 in shared memory: head dim 64 keeps three 128-row tiles of 16 KB resident; head dim 128 has a
     // ring of three 64-row units, each two [64 rows][64 channels] blocks of 8 KB
     static constexpr int NSLOT = 3;
-    static constexpr uint32_t KV_BYTES = D == 64 ? 3 * BLK : NSLOT * 16384;
+    static constexpr uint32_t KV_BYTES = D <= 64 ? 3 * BLK : NSLOT * 16384;
     static constexpr uint32_t UBLK = 8192;                       // one channel block of a 64-row unit (head dim 128)
-    static constexpr int NBUF = D == 64 ? 3 : 2;                 // S / dP (P / G) buffers in TMEM
-    static constexpr int UWBUF = D == 64 ? 1 : 2;                // U / W accumulator pairs in TMEM
+    static constexpr int NBUF = D <= 64 ? 3 : 2;                 // S / dP (P / G) buffers in TMEM
+    static constexpr int UWBUF = D <= 64 ? 1 : 2;                // U / W accumulator pairs in TMEM
     static constexpr int NCG = 2;                                // compute groups (1 is still supported at head dim 128)
     static constexpr uint32_t UW0 = NBUF * 128;                  // first TMEM column of U / W
 };
@@ -79,9 +80,9 @@ template <int D> struct BqRegs {
 static_assert(BQ_REGS_ISSUE + BQ_REGS_COMPUTE + BqRegs<64>::FOLD + BqRegs<64>::BUILD == 4 * BQ_REGS_LAUNCH, "register pool must balance");
 static_assert(BQ_REGS_ISSUE + BQ_REGS_COMPUTE + BqRegs<128>::FOLD + BqRegs<128>::BUILD == 4 * BQ_REGS_LAUNCH, "register pool must balance");
 constexpr int BQ_MAX_TILES = 3;          // K1/V1 tiles of one split (head dim 64)
-// Shared accumulators of dK2 / dV2: in sweep e thread r adds to slab row r + w2 - 1 - e, so 128 consecutive rows
+// Shared accumulators of dK2 / dV2: in sweep e thread r adds to slab row r + epc - 1 - e (epc offsets per CTA), so 128 consecutive rows
 // are live at a time.
-// Head dim 64 keeps all 127 + w2 rows, 68 floats apart (64 + 4: the row-per-thread accesses of a warp spread over
+// Head dims 32 and 64 keep all 127 + epc rows, 68 floats apart (64 + 4: the row-per-thread accesses of a warp spread over
 // all banks, and the offsets inside a row are compile-time constants).
 // Head dim 128 needs the space for its K1 / V1 ring and keeps a ring of 128 rows (slab row modulo 128): the top
 // row of a sweep is complete when thread 127 has added to it; one warp copies it to the slab in global memory at
@@ -89,10 +90,10 @@ constexpr int BQ_MAX_TILES = 3;          // K1/V1 tiles of one split (head dim 6
 // floats; its sixteen 16-byte chunks are XOR-ed with the row number instead of padding.
 constexpr int BQ_ACC_RING = 128;
 constexpr int BQ_ACC_STRIDE = 68;
-constexpr int BQ_MAX_W2 = 56;            // head dim 64: 127 + w2 accumulator rows must fit; also the tested range
+constexpr int BQ_MAX_EPC = 56;           // offsets of a CTA: 127 + epc accumulator rows must fit (head dim 64)
 template <int D> struct BqAcc {
     static constexpr bool RING = D == 128;
-    __host__ __device__ static int rows(int w2) { return RING ? BQ_ACC_RING : 127 + w2; }
+    __host__ __device__ static int rows(int epc) { return RING ? BQ_ACC_RING : 127 + epc; }
     __host__ __device__ static int row_floats() { return RING ? 64 : BQ_ACC_STRIDE; }
     // float index of (slab row, channel col) inside one accumulator array, col % 4 == 0
     __device__ static int off(int slab_row, int col) {
@@ -126,29 +127,34 @@ struct BqParams {
     KernelParams kp;
     float c;            // scale * log2(e)
     int nt;             // K1/V1 tiles per query tile
-    int nsplit;         // CTAs sharing one query tile
+    int nsplit;         // CTAs sharing one query tile: tsplit x (offset splits)
+    int tsplit;         // splits of the K1/V1 window
     int tiles_per_split;
+    int epc;            // second-key offsets of a CTA: split s takes [epc * (s / tsplit), +epc)
     int nqt;            // query tiles
     float *part_dq;     // [nsplit][b][n][hq][d]
-    float *part_k2;     // [b][hq][nqt][nsplit][2][acc_rows][d]   (dK2 slab, then dV2 slab)
+    float *part_k2;     // [b][hq][nqt][nsplit][2][127 + epc][d]   (dK2 slab, then dV2 slab)
     int *status;
+    // what the reduction adds up: dQ and dK2/dV2, and the dK1/dV1 partials of ce CTAs per key tile
+    const float *part_k1;
+    int ce, reduce_q, reduce_k1;
 };
 
-inline int bq_acc_rows(int w2) { return 127 + w2; }
-template <int D> inline size_t bq_smem_bytes(int w2) {
+template <int D> inline size_t bq_smem_bytes(int epc) {
     return 1024 + (size_t)2 * BqCfg<D>::KV_BYTES + 2 * BqCfg<D>::TILE +
-           (size_t)2 * BqAcc<D>::rows(w2) * BqAcc<D>::row_floats() * sizeof(float) + 256;
+           (size_t)2 * BqAcc<D>::rows(epc) * BqAcc<D>::row_floats() * sizeof(float) + 256;
 }
 // (a query tile with one split writes dQ itself and needs no partials)
 inline size_t bq_part_dq_bytes(const sa2_shape &s, int nsplit) { return nsplit == 1 ? 0 : (size_t)nsplit * s.b * s.n * s.hq * s.d * sizeof(float); }
-inline size_t bq_part_k2_bytes(const sa2_shape &s, int nsplit) {
+inline size_t bq_part_k2_bytes(const sa2_shape &s, int nsplit, int epc) {
     const size_t nqt = (s.n + TQ - 1) / TQ;
-    return (size_t)s.b * s.hq * nqt * nsplit * 2 * bq_acc_rows(s.w2) * s.d * sizeof(float);
+    return (size_t)s.b * s.hq * nqt * nsplit * 2 * (127 + epc) * s.d * sizeof(float);
 }
 
 struct BqGeom {
     int qt, split, chh;          // query tile, split, channel half of this CTA
     int i0, i_last, nsweeps;
+    int e0;                      // first offset of the CTA: sweep e is offset e0 + e
     int ubase;                   // first-key row of the CTA's unit 0; unit x covers rows ubase + 64 x ... + 63
     int nunits;                  // 64-key units the CTA visits in every sweep
     int total;                   // nunits * nsweeps
@@ -164,12 +170,14 @@ __device__ __forceinline__ BqGeom bq_geom(const BqParams &P) {
     g.split = qs % P.nsplit;
     g.i0 = g.qt * TQ;
     g.i_last = min(g.i0 + TQ - 1, kp.n - 1);
-    g.nsweeps = min(kp.w2, g.i_last + kp.off2 + 1);
-    if constexpr (D == 64) {
+    g.e0 = (g.split / P.tsplit) * P.epc;
+    g.nsweeps = max(0, min(min(kp.w2, g.e0 + P.epc), g.i_last + kp.off2 + 1) - g.e0);
+    const int ts = g.split % P.tsplit;
+    if constexpr (D <= 64) {
         const int jbase = g.i0 + kp.off1 + TJ - TJ * P.nt;        // tile t covers rows jbase + 128 t ...
         const int t_first = jbase >= 0 ? 0 : min(P.nt - 1, (-jbase) / TJ);
-        const int t_begin = max(t_first, g.split * P.tiles_per_split);
-        const int t_end = min(P.nt, (g.split + 1) * P.tiles_per_split);
+        const int t_begin = max(t_first, ts * P.tiles_per_split);
+        const int t_end = min(P.nt, (ts + 1) * P.tiles_per_split);
         g.ubase = jbase + TJ * t_begin;
         g.nunits = 2 * max(0, t_end - t_begin);
     } else {
@@ -197,7 +205,7 @@ __device__ __forceinline__ int bq_builder(const BqParams &P, const BqGeom &g, ui
     const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p);
     const __nv_bfloat16 *qp = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, iv ? i : 0, h);
     for (int e = 0; e < g.nsweeps; ++e) {
-        const int kk = i + kp.off2 - e;
+        const int kk = i + kp.off2 - g.e0 - e;
         const bool ok = iv && kk >= 0;
         const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
         uint4 qv[D / 8], kv[D / 8];
@@ -231,7 +239,7 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
     using C = BqCfg<D>;
     constexpr uint32_t IDESC_F = idesc_bf16(128, 64, false, false);
     const uint64_t dT = smem_desc_sw128(smem_u32(sKV)), dA = smem_desc_sw128(smem_u32(sAB));
-    if constexpr (D == 64) {
+    if constexpr (D <= 64) {
         if (!mbar_wait_warp(&bars[BQ_KV_FULL], 0, abort_flag)) return ERR_BQ_MMA;
     }
     int u = 0, buf = 0, use = 0;                         // use = u / NBUF: how often the buffer has been used before
@@ -248,10 +256,10 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
             SA2_PROF_MARK(seg);
             if (elect_one()) {
             const uint32_t d = tmem + buf * 128 + which * 64;
-            if constexpr (D == 64) {
+            if constexpr (D <= 64) {
                 const uint64_t t = dT + (uint64_t)((w * 8192) >> 4);       // unit w: rows [64 w, +64) of the resident tiles
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_ss(d, dA + 2 * k, t + 2 * k, IDESC_F, k > 0 ? 1u : 0u);
+                for (int k = 0; k < C::KSTEPS; ++k) mma_ss(d, dA + 2 * k, t + 2 * k, IDESC_F, k > 0 ? 1u : 0u);
             } else {
                 const uint64_t t = dT + (uint64_t)((slot * 2 * C::UBLK) >> 4);
 #pragma unroll
@@ -308,8 +316,8 @@ template <int D>
 __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g, int part, const CUtensorMap *mapK, const CUtensorMap *mapV,
                                              uint32_t tmem, uint8_t *sK, uint8_t *sV, uint64_t *bars, volatile int *abort_flag) {
     using C = BqCfg<D>;
-    constexpr uint32_t IDESC_G = idesc_bf16(128, 64, false, true);
-    if constexpr (D == 64) {
+    constexpr uint32_t IDESC_G = idesc_bf16(128, C::CC, false, true);
+    if constexpr (D <= 64) {
         if (part == 0) {
             const int hk = blockIdx.y / P.kp.g;
             prefetch_tmap(mapK);
@@ -327,8 +335,8 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
         if (!mbar_wait_warp(&bars[BQ_KV_FULL], 0, abort_flag)) return ERR_BQ_PRODUCER;
     }
     // head dim 128: U / W take the CTA's 64-channel block of the unit as an MN-major B operand
-    const uint64_t dK = smem_desc_sw128(smem_u32(sK) + (D == 64 ? 0 : g.chh * C::UBLK));
-    const uint64_t dV = smem_desc_sw128(smem_u32(sV) + (D == 64 ? 0 : g.chh * C::UBLK));
+    const uint64_t dK = smem_desc_sw128(smem_u32(sK) + (D <= 64 ? 0 : g.chh * C::UBLK));
+    const uint64_t dV = smem_desc_sw128(smem_u32(sV) + (D <= 64 ? 0 : g.chh * C::UBLK));
     int u = 0, buf = 0, use = 0, slot = 0;
     for (int e = 0; e < g.nsweeps; ++e) {
         const int wb = e % C::UWBUF, wuse = e / C::UWBUF;
@@ -338,7 +346,7 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
             // the fold group must have read the accumulators of the sweep that used them last
             if (w == 0 && wuse >= 1 && !mbar_wait_warp(&bars[BQ_W_EMPTY + wb], (wuse - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
             tc_fence_after();
-            const uint64_t off = (uint64_t)((D == 64 ? w * 8192 : slot * 2 * C::UBLK) >> 4);
+            const uint64_t off = (uint64_t)((D <= 64 ? w * 8192 : slot * 2 * C::UBLK) >> 4);
             const uint64_t kt = dK + off, vt = dV + off;
             const uint32_t a = tmem + buf * 128;
             const uint32_t acc = w > 0 ? 1u : 0u;
@@ -394,7 +402,7 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
         int e = 0, w = 0;
         for (int u = 0; u < g.total; ++u, ++w) {
             if (w == g.nunits) { w = 0; ++e; }
-            const bool sweep_ok = row_ok && (i + kp.off2 - e >= 0);
+            const bool sweep_ok = row_ok && (i + kp.off2 - g.e0 - e >= 0);
             {
                 const int buf = u % C::NBUF, use = u / C::NBUF;
                 const int j0 = g.ubase + 64 * w;
@@ -486,7 +494,7 @@ __device__ __forceinline__ bool bq_build_b(const BqParams &P, const BqGeom &g, i
     const KernelParams &kp = P.kp;
     const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
     const int i = g.i0 + r;
-    const int kk = i + kp.off2 - e;
+    const int kk = i + kp.off2 - g.e0 - e;
     const bool ok = i < kp.n && kk >= 0;
     const __nv_bfloat16 *dp = reinterpret_cast<const __nv_bfloat16 *>(kp.dout.p) + elem_off(kp.dout, b, ok ? i : 0, h);
     const __nv_bfloat16 *vp = reinterpret_cast<const __nv_bfloat16 *>(kp.v2.p) + elem_off(kp.v2, b, ok ? kk : 0, hk);
@@ -521,9 +529,10 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     const int c0 = g.chh * 64;                        // first channel this CTA produces
     const int i = g.i0 + r;
     const bool row_ok = i < kp.n;
-    float dq[64];
+    constexpr int NC = C::CC / 8;                     // 16-byte chunks of the CTA's channels
+    float dq[C::CC];
 #pragma unroll
-    for (int x = 0; x < 64; ++x) dq[x] = 0.f;
+    for (int x = 0; x < C::CC; ++x) dq[x] = 0.f;
     const __nv_bfloat16 *qrow = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, row_ok ? i : 0, h) + c0;
     const __nv_bfloat16 *dorow = reinterpret_cast<const __nv_bfloat16 *>(kp.dout.p) + elem_off(kp.dout, b, row_ok ? i : 0, h) + c0;
     const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p) + c0;
@@ -533,10 +542,10 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     long long seg_build = 0, seg_drain = 0;           // cycles after the waits of a build and of a fold
 #endif
     // head dim 64: the q and dO rows serve every A_e / B_e and every fold of this thread
-    uint4 qv[8], dv[8];
-    if constexpr (D == 64) {
+    uint4 qv[NC], dv[NC];
+    if constexpr (D <= 64) {
 #pragma unroll
-        for (int cc = 0; cc < 8; ++cc) {
+        for (int cc = 0; cc < NC; ++cc) {
             qv[cc] = row_ok ? __ldg(reinterpret_cast<const uint4 *>(qrow + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
             dv[cc] = row_ok ? __ldg(reinterpret_cast<const uint4 *>(dorow + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
         }
@@ -544,20 +553,20 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
 
     // row r of A_e and B_e for sweep e (head dim 64): the second-key rows are fetched before the wait for the stage
     auto build = [&](int e) -> bool {
-        if constexpr (D == 64) {
-            const int kk = i + kp.off2 - e;
+        if constexpr (D <= 64) {
+            const int kk = i + kp.off2 - g.e0 - e;
             const bool ok = row_ok && kk >= 0;
             const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
             const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk);
-            uint4 kv[8], vv[8];
+            uint4 kv[NC], vv[NC];
 #pragma unroll
-            for (int cc = 0; cc < 8; ++cc) {
+            for (int cc = 0; cc < NC; ++cc) {
                 kv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
                 vv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(vp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
             }
             // the products too are formed before the wait: only the stores follow it
 #pragma unroll
-            for (int cc = 0; cc < 8; ++cc) {
+            for (int cc = 0; cc < NC; ++cc) {
                 uint4 a = make_uint4(0u, 0u, 0u, 0u), bb = make_uint4(0u, 0u, 0u, 0u);
                 if (ok) {
                     a.x = mul_bf16x2(qv[cc].x, kv[cc].x); a.y = mul_bf16x2(qv[cc].y, kv[cc].y);
@@ -573,7 +582,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
             const long long seg_t0 = clock64();
 #endif
 #pragma unroll
-            for (int cc = 0; cc < 8; ++cc) {
+            for (int cc = 0; cc < NC; ++cc) {
                 *reinterpret_cast<uint4 *>(sA + sw128_offset(r, cc)) = kv[cc];
                 *reinterpret_cast<uint4 *>(sB + sw128_offset(r, cc)) = vv[cc];
             }
@@ -586,7 +595,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         } else if constexpr (C::NCG == 2) {
             // head dim 128 with two compute groups: this group forms A_e and B_e.  All four rows are fetched and
             // multiplied before the wait (A_e, then B_e in two halves, to stay within the register budget).
-            const int kk = i + kp.off2 - e;
+            const int kk = i + kp.off2 - g.e0 - e;
             const bool ok = row_ok && kk >= 0;
             const __nv_bfloat16 *qf = qrow - c0, *df = dorow - c0;
             const __nv_bfloat16 *kp2 = k2 - c0 + elem_off(kp.k2, b, ok ? kk : 0, hk);
@@ -636,7 +645,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
 
     auto drain = [&](int v) -> bool {
         const int wb = v % C::UWBUF, e = v;
-        const int kk = i + kp.off2 - e;
+        const int kk = i + kp.off2 - g.e0 - e;
         const bool ok = row_ok && kk >= 0;
         // the first half of the k2 row is fetched before the wait, so that its latency overlaps the end of the
         // sweep; the second half with U
@@ -652,13 +661,13 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
 #ifdef SA2_PROF
         const long long seg_t0 = clock64();
 #endif
-        const int arow = r + kp.w2 - 1 - e;           // slab row of this thread in this sweep
+        const int arow = r + P.epc - 1 - e;           // slab row of this thread in this sweep
         const bool fresh = BqAcc<D>::RING && (e == 0 || r == 0);      // ring: nothing has been added to the row yet
         if (BqAcc<D>::RING && v >= 1 && warp == 12) {
             // the top row of the last sweep is complete: it goes to the slab before thread 0 reuses its place
-            const int trow = TQ - 1 + kp.w2 - e, arr = lane >> 4, c4 = (lane & 15) * 4;
+            const int trow = TQ - 1 + P.epc - e, arr = lane >> 4, c4 = (lane & 15) * 4;
             const float4 t = *reinterpret_cast<const float4 *>((arr ? acc_v : acc_k) + BqAcc<D>::off(trow, c4));
-            *reinterpret_cast<float4 *>(slab + ((size_t)arr * (127 + kp.w2) + trow) * D + c4) = t;
+            *reinterpret_cast<float4 *>(slab + ((size_t)arr * (127 + P.epc) + trow) * D + c4) = t;
             __syncwarp();
         }
         const bool add = ok || BqAcc<D>::RING;       // (a ring row is written even when this thread has nothing to add)
@@ -687,14 +696,14 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         // W first, then U, 32 channels at a time: only 32 registers of U / W are live at once, which keeps this
         // group within its budget without spills (the accumulator pair is released after the last read).
         {
-            uint4 dr[8];
+            uint4 dr[NC];
 #pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) {
-                if constexpr (D == 64) dr[c8] = dv[c8];
+            for (int c8 = 0; c8 < NC; ++c8) {
+                if constexpr (D <= 64) dr[c8] = dv[c8];
                 else dr[c8] = __ldg(reinterpret_cast<const uint4 *>(dorow + c8 * 8));
             }
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
+            for (int hf = 0; hf < C::CC / 32; ++hf) {
                 uint32_t w[32];
                 tmem_ld32(lane_addr + C::UW0 + wb * 128 + 64 + hf * 32, w);
                 tmem_wait_ld();
@@ -717,14 +726,14 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
             }
         }
         {
-            uint4 qr[8];
+            uint4 qr[NC];
 #pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) {
-                if constexpr (D == 64) qr[c8] = qv[c8];
+            for (int c8 = 0; c8 < NC; ++c8) {
+                if constexpr (D <= 64) qr[c8] = qv[c8];
                 else qr[c8] = __ldg(reinterpret_cast<const uint4 *>(qrow + c8 * 8));
             }
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
+            for (int hf = 0; hf < C::CC / 32; ++hf) {
                 uint32_t u[32];
                 tmem_ld32(lane_addr + C::UW0 + wb * 128 + hf * 32, u);
                 if (hf == 1) {
@@ -733,7 +742,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
                         k2r[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(kr + 32 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
                 }
                 tmem_wait_ld();
-                if (hf == 1) {
+                if (hf == C::CC / 32 - 1) {
                     // U and W of the sweep are in registers (or already used): the tensor cores may overwrite them
                     tc_fence_before();
                     mbar_arrive(&bars[BQ_W_EMPTY + wb]);
@@ -788,7 +797,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
             const bool gbf16 = kp.grad_bf16 != 0;
             const int64_t o = elem_off(kp.dq, b, i, h) + c0;
 #pragma unroll
-            for (int x = 0; x < 64; x += 4) {
+            for (int x = 0; x < C::CC; x += 4) {
                 float v[4];
 #pragma unroll
                 for (int z = 0; z < 4; ++z) v[z] = bad ? CUDART_NAN_F : dq[x + z] * kp.scale;
@@ -797,7 +806,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         } else {
             float *dst = P.part_dq + ((((size_t)g.split * kp.b + b) * kp.n + i) * kp.hq + h) * D + c0;
 #pragma unroll
-            for (int x = 0; x < 64; x += 4)
+            for (int x = 0; x < C::CC; x += 4)
                 *reinterpret_cast<float4 *>(dst + x) = bad ? make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F)
                                                            : make_float4(dq[x], dq[x + 1], dq[x + 2], dq[x + 3]);
         }
@@ -811,7 +820,7 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
     const KernelParams &kp = P.kp;
     const int ft = threadIdx.x - 384;                 // 0..127 among the fold threads
     const int h = blockIdx.y, b = blockIdx.z;
-    const int slab_rows = 127 + kp.w2;
+    const int slab_rows = 127 + P.epc;
     // this CTA's 64 channels of its slab (dK2 rows, then dV2 rows)
     float *slab = P.part_k2 + ((((size_t)b * kp.hq + h) * P.nqt + g.qt) * P.nsplit + g.split) * (size_t)(2 * slab_rows * D) + g.chh * 64;
     if constexpr (!BqAcc<D>::RING) {
@@ -825,13 +834,14 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
     // Ring: rows above the live ones went to the slab when they were completed; the live rows follow now, and
     // the rows below them (second keys before the sequence start, when fewer than w2 sweeps ran) are zero.
     const int nv = g.total > 0 ? g.nsweeps : 0;
-    const int live0 = BqAcc<D>::RING ? kp.w2 - nv : 0;                 // first slab row held in shared memory
+    const int live0 = BqAcc<D>::RING ? P.epc - nv : 0;                 // first slab row held in shared memory
     const int rows = BqAcc<D>::RING && nv > 0 ? live0 + BQ_ACC_RING : slab_rows;
     const bool held = !BqAcc<D>::RING || nv > 0;
     const bool bad = err != 0 || *abort_flag != 0;     // a CTA in which a wait ran out reports NaN
-    for (int x = ft; x < 2 * rows * 16; x += 128) {
-        const int arr = x / (rows * 16), y = x - arr * rows * 16;
-        const int row = y >> 4, c4 = (y & 15) * 4;
+    constexpr int C4 = BqCfg<D>::CC / 4;
+    for (int x = ft; x < 2 * rows * C4; x += 128) {
+        const int arr = x / (rows * C4), y = x - arr * rows * C4;
+        const int row = y / C4, c4 = (y % C4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (held && row >= live0) v = *reinterpret_cast<const float4 *>((arr ? acc_v : acc_k) + BqAcc<D>::off(row, c4));
         if (bad) v = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F);
@@ -851,7 +861,7 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     uint8_t *sA = sV + C::KV_BYTES;
     uint8_t *sB = sA + C::TILE;
     float *acc_k = reinterpret_cast<float *>(sB + C::TILE);
-    const int acc_floats = BqAcc<D>::rows(P.kp.w2) * BqAcc<D>::row_floats();
+    const int acc_floats = BqAcc<D>::rows(P.epc) * BqAcc<D>::row_floats();
     float *acc_v = acc_k + acc_floats;
     uint64_t *bars = reinterpret_cast<uint64_t *>(acc_v + acc_floats);
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + BQ_BAR_COUNT);
@@ -865,7 +875,7 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
             // S_FULL and AB_EMPTY collect one commit from each of the two first-product issuers; head dim 64:
             // G_DONE and W_FULL one from each of the two second-product issuers
             const bool two = (x >= BQ_S_FULL && x < BQ_S_FULL + 3) || x == BQ_AB_EMPTY ||
-                             (D == 64 && ((x >= BQ_G_DONE && x < BQ_G_DONE + 3) || (x >= BQ_W_FULL && x < BQ_W_FULL + 2)));
+                             (D <= 64 && ((x >= BQ_G_DONE && x < BQ_G_DONE + 3) || (x >= BQ_W_FULL && x < BQ_W_FULL + 2)));
             // head dim 64: the fold group forms A_e and B_e; head dim 128: the builders A_e, the fold group B_e
             mbar_init(&bars[x], x == BQ_AB_FULL ? (BqRegs<D>::BUILDERS ? 256u : 128u) : pfull ? 128u * C::NCG : many ? 128u : two ? 2u : 1u);
         }
@@ -890,10 +900,10 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     if (warp < 4) {
         reg_dealloc<BQ_REGS_ISSUE>();                 // one instruction for the whole warpgroup
         if (g.total > 0) {
-            if (warp == 0) err = bq_mma_second<D>(P, g, D == 64 ? 0 : 2, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
+            if (warp == 0) err = bq_mma_second<D>(P, g, D <= 64 ? 0 : 2, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
             else if (warp == 1) err = bq_mma_first<D>(g, 0, tmem, sK, sA, bars, abort_flag);
             else if (warp == 2) err = bq_mma_first<D>(g, 1, tmem, sV, sB, bars, abort_flag);
-            else if constexpr (D == 64) err = bq_mma_second<D>(P, g, 1, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
+            else if constexpr (D <= 64) err = bq_mma_second<D>(P, g, 1, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
             else err = bq_ring_producer<D>(P, g, &mapK, &mapV, sK, sV, bars, abort_flag);
         }
     } else if (warp < 4 + 4 * C::NCG) {
@@ -929,17 +939,19 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
 //   dq[b,i,h]   = scale * sum_split part_dq[split][b][i][h]        (two or more splits only)
 //   dk2[b,k,hk] = scale * sum_{h in group} sum_{tiles touching k} sum_split slab_k[...]
 //   dv2[b,k,hk] =         same over slab_v
+//   dk1[b,j,hk] = scale * sum_{split of the key tile} part_k1[...], dv1 the same (two or more splits only)
 // Row k (position k - off2 in query coordinates) lies in the slab of query tile
-// T at slab row k - off2 - 128 T + (w2 - 1), for the one or two tiles where
-// that index falls inside [0, 127 + w2).
+// T and the split of offsets [e0, e0 + epc) at slab row k - off2 - 128 T + e0 + epc - 1, for the
+// one or two tiles where that index falls inside [0, 127 + epc).
 // ---------------------------------------------------------------------------
 template <int D>
 __global__ void bwd_q_reduce_kernel(const BqParams P) {
     constexpr int TPR = D / 4;                          // threads per row
     const KernelParams &kp = P.kp;
-    const int acc_rows = 127 + kp.w2;
-    const int64_t nq = P.nsplit == 1 ? 0 : (int64_t)kp.b * kp.n * kp.hq * TPR;      // one split: dQ is already in place
-    const int64_t nk = (int64_t)kp.b * kp.nk2 * kp.hk * TPR;
+    const int acc_rows = 127 + P.epc;
+    const int64_t nq = !P.reduce_q || P.nsplit == 1 ? 0 : (int64_t)kp.b * kp.n * kp.hq * TPR;      // one split: dQ is already in place
+    const int64_t nk = !P.reduce_q ? 0 : (int64_t)kp.b * kp.nk2 * kp.hk * TPR;
+    const int64_t nk1 = !P.reduce_k1 ? 0 : (int64_t)kp.b * kp.nk1 * kp.hk * TPR;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool gbf16 = kp.grad_bf16 != 0;
     if (idx < nq) {
@@ -967,12 +979,13 @@ __global__ void bwd_q_reduce_kernel(const BqParams P) {
         const int pos = k - kp.off2;                    // in query coordinates (may be negative for halo rows)
         for (int hh = 0; hh < kp.g; ++hh) {
             const int h = hk * kp.g + hh;
-            // tiles T with 0 <= pos - 128 T + w2 - 1 < acc_rows
-            const int t_hi = min(P.nqt - 1, (pos + kp.w2 - 1) >= 0 ? (pos + kp.w2 - 1) / TQ : -1);
-            for (int T = max(0, t_hi - 1); T <= t_hi; ++T) {
-                const int row = pos - TQ * T + kp.w2 - 1;
-                if (row < 0 || row >= acc_rows) continue;
-                for (int s = 0; s < P.nsplit; ++s) {
+            for (int s = 0; s < P.nsplit; ++s) {
+                // tiles T with 0 <= pos - 128 T + top < acc_rows
+                const int top = (s / P.tsplit) * P.epc + P.epc - 1;
+                const int t_hi = min(P.nqt - 1, pos + top >= 0 ? (pos + top) / TQ : -1);
+                for (int T = max(0, t_hi - 1); T <= t_hi; ++T) {
+                    const int row = pos - TQ * T + top;
+                    if (row < 0 || row >= acc_rows) continue;
                     const float *slab = P.part_k2 + ((((size_t)b * kp.hq + h) * P.nqt + T) * P.nsplit + s) * (size_t)(2 * acc_rows * D);
                     const float4 vk = *reinterpret_cast<const float4 *>(slab + (size_t)row * D + c4);
                     const float4 vv = *reinterpret_cast<const float4 *>(slab + (size_t)(acc_rows + row) * D + c4);
@@ -985,6 +998,21 @@ __global__ void bwd_q_reduce_kernel(const BqParams P) {
         for (int z = 0; z < 4; ++z) ak[z] *= kp.scale;
         store_vec<4>(kp.dk2.p, elem_off(kp.dk2, b, k, hk) + c4, gbf16, ak);
         store_vec<4>(kp.dv2.p, elem_off(kp.dv2, b, k, hk) + c4, gbf16, av);
+    } else if (idx < nq + nk + nk1) {
+        const int64_t id3 = idx - nq - nk, row = id3 / TPR, rows = (int64_t)kp.b * kp.nk1 * kp.hk;
+        const int c4 = (int)(id3 % TPR) * 4;
+        const int hk = (int)(row % kp.hk), j = (int)(row / kp.hk % kp.nk1), b = (int)(row / ((int64_t)kp.hk * kp.nk1));
+        float ak[4] = {0.f, 0.f, 0.f, 0.f}, av[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s = 0; s < P.ce; ++s) {
+            const float *src = P.part_k1 + ((size_t)s * rows + row) * (2 * D) + c4;
+            const float4 vk = *reinterpret_cast<const float4 *>(src), vv = *reinterpret_cast<const float4 *>(src + D);
+            ak[0] += vk.x; ak[1] += vk.y; ak[2] += vk.z; ak[3] += vk.w;
+            av[0] += vv.x; av[1] += vv.y; av[2] += vv.z; av[3] += vv.w;
+        }
+#pragma unroll
+        for (int z = 0; z < 4; ++z) ak[z] *= kp.scale;
+        store_vec<4>(kp.dk1.p, elem_off(kp.dk1, b, j, hk) + c4, gbf16, ak);
+        store_vec<4>(kp.dv1.p, elem_off(kp.dv1, b, j, hk) + c4, gbf16, av);
     }
 }
 
