@@ -97,20 +97,23 @@ inline bool fwd_addressable(const KernelParams &kp) {
 inline int fwd128(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
     f128::Params P;
     P.kp = kp;
-    P.nh = (s.w1 + TQ - 1 + f128::UNIT - 1) / f128::UNIT;       // ceil((w1 + 127) / 64)
+    P.ri_log2 = fwd_ri_log2(s, SM_COUNT);
+    P.nslots = f128::SLOTS;
+    P.win_boxes = f128::win_boxes(s.w2, P.ri_log2);
     P.c = s.scale * 1.4426950408889634f;
     P.pv_split = n64_products();
     P.status = status_word();
     if (!P.status) return SA2_ERR_CUDA;
-    CUtensorMap mapK, mapV;     // 64-row, 64-channel boxes
+    CUtensorMap mapK, mapV, mapV2;     // 64-row, 64-channel boxes; 32-row boxes of the second values
     if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, 128, kp.k1.sb, kp.k1.sn, kp.k1.sh, f128::UNIT) ||
-        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, 128, kp.v1.sb, kp.v1.sn, kp.v1.sh, f128::UNIT))
+        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, 128, kp.v1.sb, kp.v1.sn, kp.v1.sh, f128::UNIT) ||
+        !tmap::make_rows_map(&mapV2, kp.v2.p, kp.b, kp.nk2, kp.hk, 128, kp.v2.sb, kp.v2.sn, kp.v2.sh, 32))
         return SA2_ERR_CUDA;
     const size_t smem = f128::smem_bytes();
     if (cudaFuncSetAttribute(f128::fwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SA2_ERR_CUDA;
-    dim3 grid((kp.n + TQ - 1) / TQ, kp.hq, kp.b);
-    f128::fwd128_kernel<<<grid, f128::THREADS, smem, st>>>(mapK, mapV, P);
+    const int ri = 1 << P.ri_log2;
+    f128::fwd128_kernel<<<dim3((kp.n + ri - 1) / ri, kp.hq, kp.b), f128::THREADS, smem, st>>>(mapK, mapV, mapV2, P);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 

@@ -54,9 +54,8 @@ constexpr int BQ_THREADS = 512;
 // thread; a group can only grow by what another has released, or its setmaxnreg never returns, so the
 // four budgets must add up to 4 * 128.
 constexpr int BQ_REGS_LAUNCH = 128, BQ_REGS_ISSUE = 40, BQ_REGS_COMPUTE = 120;
-// The fold group (232) holds dQ and, at head dim 64, the q and dO rows, plus either the operand rows of the next
-// sweep or a k2 row and chunks of U and W.  (With one compute group at head dim 128 - NCG = 1 - warps 8-11 form
-// A_e with 144 registers and the fold group keeps 208.)
+// The fold group (232) holds dQ and, up to head dim 64, the q and dO rows, plus either the operands of the next sweep or
+// a k2 row and chunks of U and W.
 template <int D> struct BqCfg {
     static constexpr int CH = D == 128 ? 2 : 1;                  // channel halves = CTAs per (query tile, split)
     static constexpr int CC = D < 64 ? D : 64;                   // channels this CTA produces
@@ -70,15 +69,10 @@ template <int D> struct BqCfg {
     static constexpr uint32_t UBLK = 8192;                       // one channel block of a 64-row unit (head dim 128)
     static constexpr int NBUF = D <= 64 ? 3 : 2;                 // S / dP (P / G) buffers in TMEM
     static constexpr int UWBUF = D <= 64 ? 1 : 2;                // U / W accumulator pairs in TMEM
-    static constexpr int NCG = 2;                                // compute groups (1 is still supported at head dim 128)
     static constexpr uint32_t UW0 = NBUF * 128;                  // first TMEM column of U / W
 };
-template <int D> struct BqRegs {
-    static constexpr bool BUILDERS = D == 128 && BqCfg<D>::NCG == 1;          // warps 8-11 form A_e instead of computing
-    static constexpr int FOLD = BUILDERS ? 208 : 232, BUILD = BUILDERS ? 144 : BQ_REGS_COMPUTE;
-};
-static_assert(BQ_REGS_ISSUE + BQ_REGS_COMPUTE + BqRegs<64>::FOLD + BqRegs<64>::BUILD == 4 * BQ_REGS_LAUNCH, "register pool must balance");
-static_assert(BQ_REGS_ISSUE + BQ_REGS_COMPUTE + BqRegs<128>::FOLD + BqRegs<128>::BUILD == 4 * BQ_REGS_LAUNCH, "register pool must balance");
+constexpr int BQ_REGS_FOLD = 232;
+static_assert(BQ_REGS_ISSUE + 2 * BQ_REGS_COMPUTE + BQ_REGS_FOLD == 4 * BQ_REGS_LAUNCH, "register pool must balance");
 constexpr int BQ_MAX_TILES = 3;          // K1/V1 tiles of one split (head dim 64)
 // Shared accumulators of dK2 / dV2: in sweep e thread r adds to slab row r + epc - 1 - e (epc offsets per CTA), so 128 consecutive rows
 // are live at a time.
@@ -189,43 +183,6 @@ __device__ __forceinline__ BqGeom bq_geom(const BqParams &P) {
     }
     g.total = g.nunits * g.nsweeps;
     return g;
-}
-
-// ---------------------------------------------------------------- head dim 128: builders of A_e (warps 8-11)
-// One thread per query row forms row r of A_e = q_i * k2_{i-e} for every sweep (the fold group forms B_e, see
-// bq_build_b); the whole row is fetched before the wait, so that the stage is rebuilt as soon as the tensor
-// cores release it.
-template <int D>
-__device__ __forceinline__ int bq_builder(const BqParams &P, const BqGeom &g, uint8_t *sA, uint64_t *bars, volatile int *abort_flag) {
-    const KernelParams &kp = P.kp;
-    const int r = threadIdx.x - 256;
-    const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
-    const int i = g.i0 + r;
-    const bool iv = i < kp.n;
-    const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p);
-    const __nv_bfloat16 *qp = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, iv ? i : 0, h);
-    for (int e = 0; e < g.nsweeps; ++e) {
-        const int kk = i + kp.off2 - g.e0 - e;
-        const bool ok = iv && kk >= 0;
-        const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-        uint4 qv[D / 8], kv[D / 8];
-#pragma unroll
-        for (int cc = 0; cc < D / 8; ++cc) {
-            qv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(qp + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-            kv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-        }
-        if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 1)) return ERR_BQ_BUILDER;
-#pragma unroll
-        for (int cc = 0; cc < D / 8; ++cc) {
-            uint4 a;
-            a.x = mul_bf16x2(qv[cc].x, kv[cc].x); a.y = mul_bf16x2(qv[cc].y, kv[cc].y);
-            a.z = mul_bf16x2(qv[cc].z, kv[cc].z); a.w = mul_bf16x2(qv[cc].w, kv[cc].w);
-            *reinterpret_cast<uint4 *>(sA + (cc >> 3) * BqCfg<D>::BLK + sw128_offset(r, cc & 7)) = a;
-        }
-        fence_proxy_async_smem();
-        mbar_arrive(&bars[BQ_AB_FULL]);
-    }
-    return 0;
 }
 
 // ---------------------------------------------------------------- issuers of S (warp 1) and dP (warp 2), one lane each
@@ -380,7 +337,6 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
 template <int D>
 __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, int cg, uint32_t tmem, uint64_t *bars, volatile int *abort_flag) {
     using C = BqCfg<D>;
-    if (cg >= C::NCG) return 0;
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = (warp & 3) * 32 + lane;             // query row within the tile = TMEM lane
@@ -412,18 +368,14 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                 if (!warp_wait(&bars[BQ_S_FULL + buf], use & 1, abort_flag, 1)) return ERR_BQ_COMPUTE;
                 tc_fence_after();
                 const bool full = __all_sync(0xffffffffu, lo < 0 && hi >= 63);
-                const int ch_end = C::NCG == 2 ? cg + 1 : 2;
-#pragma unroll 1
-                for (int ch = C::NCG == 2 ? cg : 0; ch < ch_end; ++ch) {
+                {
+                    const int ch = cg;
                     uint32_t sv[32], dv[32], pp[16], gg[16];
                     // no row of this warp has a valid column among these 32: P = G = 0 without reading S / dP
                     if (__all_sync(0xffffffffu, hi < ch * 32 || lo >= ch * 32 + 31)) {
 #pragma unroll
                         for (int x = 0; x < 16; ++x) { pp[x] = 0u; gg[x] = 0u; }
-                        tmem_st16(lane_addr + buf * 128 + ch * 32, pp);
-                        tmem_st16(lane_addr + buf * 128 + 64 + ch * 32, gg);
-                        continue;
-                    }
+                    } else {
 #ifdef SA2_PROF
                     const long long seg_t0 = clock64();
 #endif
@@ -460,6 +412,7 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
 #ifdef SA2_PROF
                     seg_math += clock64() - seg_t1;
 #endif
+                    }
                     // P / G chunk over the first half of the columns of S / dP that this thread has just read (the
                     // other columns of the buffer may still be unread by the other compute group)
                     tmem_st16(lane_addr + buf * 128 + ch * 32, pp);
@@ -485,37 +438,6 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
 
 // ---------------------------------------------------------------- fold (warps 8-11): U, W -> dQ, dK2, dV2
 __device__ __forceinline__ void bq_fold_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-// Head dim 128: the fold thread of query row r forms row r of B_e = dO_i * v2_{i-e} for sweep e (the builder
-// group forms A_e); the whole row is fetched before the wait for the stage.
-template <int D>
-__device__ __forceinline__ bool bq_build_b(const BqParams &P, const BqGeom &g, int e, int r, uint8_t *sB, uint64_t *bars,
-                                           volatile int *abort_flag) {
-    const KernelParams &kp = P.kp;
-    const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
-    const int i = g.i0 + r;
-    const int kk = i + kp.off2 - g.e0 - e;
-    const bool ok = i < kp.n && kk >= 0;
-    const __nv_bfloat16 *dp = reinterpret_cast<const __nv_bfloat16 *>(kp.dout.p) + elem_off(kp.dout, b, ok ? i : 0, h);
-    const __nv_bfloat16 *vp = reinterpret_cast<const __nv_bfloat16 *>(kp.v2.p) + elem_off(kp.v2, b, ok ? kk : 0, hk);
-    uint4 dv[16], vv[16];
-#pragma unroll
-    for (int cc = 0; cc < 16; ++cc) {
-        dv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(dp + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-        vv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(vp + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-    }
-    if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
-#pragma unroll
-    for (int cc = 0; cc < 16; ++cc) {
-        uint4 bb;
-        bb.x = mul_bf16x2(dv[cc].x, vv[cc].x); bb.y = mul_bf16x2(dv[cc].y, vv[cc].y);
-        bb.z = mul_bf16x2(dv[cc].z, vv[cc].z); bb.w = mul_bf16x2(dv[cc].w, vv[cc].w);
-        *reinterpret_cast<uint4 *>(sB + (cc >> 3) * BqCfg<D>::BLK + sw128_offset(r, cc & 7)) = bb;
-    }
-    fence_proxy_async_smem();
-    mbar_arrive(&bars[BQ_AB_FULL]);
-    return true;
-}
 
 template <int D>
 __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc_k, float *acc_v, float *slab,
@@ -551,96 +473,100 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         }
     }
 
-    // row r of A_e and B_e for sweep e (head dim 64): the second-key rows are fetched before the wait for the stage
-    auto build = [&](int e) -> bool {
-        if constexpr (D <= 64) {
-            const int kk = i + kp.off2 - g.e0 - e;
-            const bool ok = row_ok && kk >= 0;
-            const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-            const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk);
-            uint4 kv[NC], vv[NC];
+    // A_e = q_i * k2_{i-e} and B_e = dO_i * v2_{i-e} of sweep e.  Up to head dim 64 a thread forms its own row, whose q and
+    // dO stay in its registers.  At head dim 128 sixteen lanes take a row, 16 bytes each, so that a load of the warp is
+    // whole rows: with a row per lane every load touched 32 cache lines, ~8000 cycles of L1 a sweep (10.3 -> 9.0 ms on
+    // b1 n16384 h16; at head dim 64, without the rows in registers, 1.8 -> 2.2 ms on b4 n4096 h8).  The products are
+    // formed before the wait for the stage, only the stores follow it.
+    constexpr int LPR = D / 8, RPI = 32 / LPR;            // lanes per row, rows per load
+    const int brow = (warp & 3) * 32 + lane / LPR, bcc = lane % LPR;
+    const int64_t b_q = elem_off(kp.q, b, 0, h) + bcc * 8, b_do = elem_off(kp.dout, b, 0, h) + bcc * 8;
+    const int64_t b_k2 = elem_off(kp.k2, b, 0, hk) + bcc * 8, b_v2 = elem_off(kp.v2, b, 0, hk) + bcc * 8;
+    auto build_row = [&](int e) -> bool {
+        const int kk = i + kp.off2 - g.e0 - e;
+        const bool ok = row_ok && kk >= 0;
+        const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
+        const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk);
+        uint4 kv[NC], vv[NC];
 #pragma unroll
-            for (int cc = 0; cc < NC; ++cc) {
-                kv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-                vv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(vp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-            }
-            // the products too are formed before the wait: only the stores follow it
-#pragma unroll
-            for (int cc = 0; cc < NC; ++cc) {
-                uint4 a = make_uint4(0u, 0u, 0u, 0u), bb = make_uint4(0u, 0u, 0u, 0u);
-                if (ok) {
-                    a.x = mul_bf16x2(qv[cc].x, kv[cc].x); a.y = mul_bf16x2(qv[cc].y, kv[cc].y);
-                    a.z = mul_bf16x2(qv[cc].z, kv[cc].z); a.w = mul_bf16x2(qv[cc].w, kv[cc].w);
-                    bb.x = mul_bf16x2(dv[cc].x, vv[cc].x); bb.y = mul_bf16x2(dv[cc].y, vv[cc].y);
-                    bb.z = mul_bf16x2(dv[cc].z, vv[cc].z); bb.w = mul_bf16x2(dv[cc].w, vv[cc].w);
-                }
-                kv[cc] = a;
-                vv[cc] = bb;
-            }
-            if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
-#ifdef SA2_PROF
-            const long long seg_t0 = clock64();
-#endif
-#pragma unroll
-            for (int cc = 0; cc < NC; ++cc) {
-                *reinterpret_cast<uint4 *>(sA + sw128_offset(r, cc)) = kv[cc];
-                *reinterpret_cast<uint4 *>(sB + sw128_offset(r, cc)) = vv[cc];
-            }
-            fence_proxy_async_smem();
-            mbar_arrive(&bars[BQ_AB_FULL]);
-#ifdef SA2_PROF
-            seg_build += clock64() - seg_t0;
-#endif
-            return true;
-        } else if constexpr (C::NCG == 2) {
-            // head dim 128 with two compute groups: this group forms A_e and B_e.  All four rows are fetched and
-            // multiplied before the wait (A_e, then B_e in two halves, to stay within the register budget).
-            const int kk = i + kp.off2 - g.e0 - e;
-            const bool ok = row_ok && kk >= 0;
-            const __nv_bfloat16 *qf = qrow - c0, *df = dorow - c0;
-            const __nv_bfloat16 *kp2 = k2 - c0 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-            const __nv_bfloat16 *vp2 = v2 - c0 + elem_off(kp.v2, b, ok ? kk : 0, hk);
-            uint4 a[16], bb[16];
-            {
-                uint4 x[16];
-#pragma unroll
-                for (int cc = 0; cc < 16; ++cc) {
-                    a[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(qf + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-                    x[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-                }
-#pragma unroll
-                for (int cc = 0; cc < 16; ++cc) {
-                    a[cc].x = mul_bf16x2(a[cc].x, x[cc].x); a[cc].y = mul_bf16x2(a[cc].y, x[cc].y);
-                    a[cc].z = mul_bf16x2(a[cc].z, x[cc].z); a[cc].w = mul_bf16x2(a[cc].w, x[cc].w);
-                }
-            }
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                uint4 x[8];
-#pragma unroll
-                for (int cc = 0; cc < 8; ++cc) {
-                    bb[hf * 8 + cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(df + (hf * 8 + cc) * 8)) : make_uint4(0u, 0u, 0u, 0u);
-                    x[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(vp2 + (hf * 8 + cc) * 8)) : make_uint4(0u, 0u, 0u, 0u);
-                }
-#pragma unroll
-                for (int cc = 0; cc < 8; ++cc) {
-                    uint4 &t = bb[hf * 8 + cc];
-                    t.x = mul_bf16x2(t.x, x[cc].x); t.y = mul_bf16x2(t.y, x[cc].y);
-                    t.z = mul_bf16x2(t.z, x[cc].z); t.w = mul_bf16x2(t.w, x[cc].w);
-                }
-            }
-            if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
-#pragma unroll
-            for (int cc = 0; cc < 16; ++cc) {
-                *reinterpret_cast<uint4 *>(sA + (cc >> 3) * C::BLK + sw128_offset(r, cc & 7)) = a[cc];
-                *reinterpret_cast<uint4 *>(sB + (cc >> 3) * C::BLK + sw128_offset(r, cc & 7)) = bb[cc];
-            }
-            fence_proxy_async_smem();
-            mbar_arrive(&bars[BQ_AB_FULL]);
-            return true;
-        } else {
-            return bq_build_b<D>(P, g, e, r, sB, bars, abort_flag);
+        for (int cc = 0; cc < NC; ++cc) {
+            kv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
+            vv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(vp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
         }
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) {
+            kv[cc] = make_uint4(mul_bf16x2(qv[cc].x, kv[cc].x), mul_bf16x2(qv[cc].y, kv[cc].y), mul_bf16x2(qv[cc].z, kv[cc].z), mul_bf16x2(qv[cc].w, kv[cc].w));
+            vv[cc] = make_uint4(mul_bf16x2(dv[cc].x, vv[cc].x), mul_bf16x2(dv[cc].y, vv[cc].y), mul_bf16x2(dv[cc].z, vv[cc].z), mul_bf16x2(dv[cc].w, vv[cc].w));
+            if (!ok) { kv[cc] = make_uint4(0u, 0u, 0u, 0u); vv[cc] = make_uint4(0u, 0u, 0u, 0u); }
+        }
+        if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
+#ifdef SA2_PROF
+        const long long seg_t0 = clock64();
+#endif
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) {
+            *reinterpret_cast<uint4 *>(sA + sw128_offset(r, cc)) = kv[cc];
+            *reinterpret_cast<uint4 *>(sB + sw128_offset(r, cc)) = vv[cc];
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(&bars[BQ_AB_FULL]);
+#ifdef SA2_PROF
+        seg_build += clock64() - seg_t0;
+#endif
+        return true;
+    };
+    auto build = [&](int e) -> bool {
+        if constexpr (D <= 64) return build_row(e);
+        uint4 pa[LPR], pb[LPR];
+        auto mul = [](const uint4 &x, const uint4 &y) {
+            return make_uint4(mul_bf16x2(x.x, y.x), mul_bf16x2(x.y, y.y), mul_bf16x2(x.z, y.z), mul_bf16x2(x.w, y.w));
+        };
+        auto fetch = [&](const TensorRef &t, int64_t base, int row) {
+            return __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(t.p) + base + (int64_t)row * t.sn));
+        };
+        constexpr int STEP = 2;                           // rows per lane that hold registers for a second operand
+#pragma unroll
+        for (int x0 = 0; x0 < LPR; x0 += STEP) {
+            uint4 y[STEP];
+#pragma unroll
+            for (int x = 0; x < STEP; ++x) {
+                const int ii = g.i0 + brow + (x0 + x) * RPI, kk = ii + kp.off2 - g.e0 - e;
+                const bool ok = ii < kp.n && kk >= 0;
+                pa[x0 + x] = ok ? fetch(kp.q, b_q, ii) : make_uint4(0u, 0u, 0u, 0u);
+                y[x] = ok ? fetch(kp.k2, b_k2, kk) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int x = 0; x < STEP; ++x) pa[x0 + x] = mul(pa[x0 + x], y[x]);
+        }
+#pragma unroll
+        for (int x0 = 0; x0 < LPR; x0 += STEP) {
+            uint4 y[STEP];
+#pragma unroll
+            for (int x = 0; x < STEP; ++x) {
+                const int ii = g.i0 + brow + (x0 + x) * RPI, kk = ii + kp.off2 - g.e0 - e;
+                const bool ok = ii < kp.n && kk >= 0;
+                pb[x0 + x] = ok ? fetch(kp.dout, b_do, ii) : make_uint4(0u, 0u, 0u, 0u);
+                y[x] = ok ? fetch(kp.v2, b_v2, kk) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int x = 0; x < STEP; ++x) pb[x0 + x] = mul(pb[x0 + x], y[x]);
+        }
+        if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
+#ifdef SA2_PROF
+        const long long seg_t0 = clock64();
+#endif
+#pragma unroll
+        for (int x = 0; x < LPR; ++x) {
+            const uint32_t o = (bcc >> 3) * C::BLK + sw128_offset(brow + x * RPI, bcc & 7);
+            *reinterpret_cast<uint4 *>(sA + o) = pa[x];
+            *reinterpret_cast<uint4 *>(sB + o) = pb[x];
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(&bars[BQ_AB_FULL]);
+#ifdef SA2_PROF
+        seg_build += clock64() - seg_t0;
+#endif
+        return true;
     };
 
     auto drain = [&](int v) -> bool {
@@ -876,8 +802,7 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
             // G_DONE and W_FULL one from each of the two second-product issuers
             const bool two = (x >= BQ_S_FULL && x < BQ_S_FULL + 3) || x == BQ_AB_EMPTY ||
                              (D <= 64 && ((x >= BQ_G_DONE && x < BQ_G_DONE + 3) || (x >= BQ_W_FULL && x < BQ_W_FULL + 2)));
-            // head dim 64: the fold group forms A_e and B_e; head dim 128: the builders A_e, the fold group B_e
-            mbar_init(&bars[x], x == BQ_AB_FULL ? (BqRegs<D>::BUILDERS ? 256u : 128u) : pfull ? 128u * C::NCG : many ? 128u : two ? 2u : 1u);
+            mbar_init(&bars[x], x == BQ_AB_FULL ? 128u : pfull ? 256u : many ? 128u : two ? 2u : 1u);
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -906,20 +831,13 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
             else if constexpr (D <= 64) err = bq_mma_second<D>(P, g, 1, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
             else err = bq_ring_producer<D>(P, g, &mapK, &mapV, sK, sV, bars, abort_flag);
         }
-    } else if (warp < 4 + 4 * C::NCG) {
+    } else if (warp < 12) {
         // one call site for both compute groups: they run the same instructions, which the instruction caches
         // of a scheduler then hold once
         reg_dealloc<BQ_REGS_COMPUTE>();
         err = bq_compute<D>(P, g, (warp >> 2) - 1, tmem, bars, abort_flag);
-    } else if (warp < 12) {
-        if constexpr (BqRegs<D>::BUILDERS) {
-            reg_alloc<BqRegs<D>::BUILD>();
-            if (g.total > 0) err = bq_builder<D>(P, g, sA, bars, abort_flag);
-        } else {
-            reg_dealloc<BQ_REGS_COMPUTE>();
-        }
     } else {
-        reg_alloc<BqRegs<D>::FOLD>();
+        reg_alloc<BQ_REGS_FOLD>();
         err = bq_fold<D>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
     }
     if (err) atomicOr(P.status, err);

@@ -104,7 +104,8 @@ struct FwdGeom {
     bool resident;    // every unit of the window has its own slot
 };
 
-__device__ __forceinline__ FwdGeom fwd_geom(const FwdParams &P) {
+template <class PT>
+__device__ __forceinline__ FwdGeom fwd_geom(const PT &P) {
     FwdGeom g;
     const KernelParams &kp = P.kp;
     g.ri_log2 = P.ri_log2;
@@ -631,6 +632,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
 // chunks), so the rule assumes four of them: at one element a tile may be twice as long as it could be, at
 // sixteen there may be twice as many tiles as needed.
 inline int fwd_ri_log2(const sa2_shape &s, int sms) {
+    const double unit = s.d == 128 ? 1.7 : 1.;          // head dim 128: twice the products, streamed
     int best = 6;
     double best_cost = 0.;
     for (int l = 6; l >= 3; --l) {
@@ -641,7 +643,7 @@ inline int fwd_ri_log2(const sa2_shape &s, int sms) {
         const int units = (keys + FWD_UNIT - 1) / FWD_UNIT;
         const int w2 = s.w2 < s.n + s.off2 ? s.w2 : s.n + s.off2;
         const int sweeps = (w2 + re - 1) / re;
-        const double both = sweeps * units * 650., one = ((sweeps + 1) / 2) * units * 1100.;
+        const double both = sweeps * units * 650. * unit, one = ((sweeps + 1) / 2) * units * 1100. * unit;
         const double waves = tiles > sms ? tiles / sms : 1.;
         const double cost = waves * (5500. + (both > one ? both : one));
         if (l == 6 || cost < 0.98 * best_cost) { best = l; best_cost = cost; }

@@ -1,11 +1,12 @@
 // Forward kernel on the 5th-generation tensor cores (tcgen05 + TMEM + TMA),
 // bf16 operands, fp32 accumulation, head dim 128.
 //
-// Same formulation as the head-dim-64 kernel (sa2_tc_fwd.cuh): a CTA owns 128
-// query rows of one (batch, query head); per offset e = i - k ("sweep") it forms
-// A_e[i,:] = q_i * k2_{i-e}, S = A_e K1^T per 64-key unit, P = exp2(c S - ref),
-// W_e += P V1, and at the end of the sweep the row owner adds v2_{i-e} * W_e to
-// its output registers.  Two softmax groups own the even and the odd sweeps.
+// Same formulation as the head-dim-64 kernel (sa2_tc_fwd.cuh): a tile is RI query rows times RE = 128 / RI second-key
+// offsets of one (batch, query head); per sweep it forms A[r,:] = q_i * k2_{i-e}, S = A K1^T per 64-key unit,
+// P = exp2(c S - ref), W += P V1, and at the end of the sweep the row owner adds v2_{i-e} * W to its output
+// registers.  Two softmax groups own the even and the odd sweeps; the RE partial outputs of a query row are merged
+// through shared memory.  (With 128 query rows per tile one new row behind a full window took 32 sweeps in turn:
+// b1 h8 w512/32 FWD128_DEC us.)
 //
 // What head dim 128 changes:
 //   * A K1/V1 window of 640 rows is 320 KB and does not fit in shared memory,
@@ -40,7 +41,7 @@
 //   12-15  softmax group 0 (even sweeps), 16-19 softmax group 1 (odd sweeps)
 //   20, 21 lane 0 is the TMA producer of the K1 ring / of the V1 ring; 22-23 idle
 #pragma once
-#include "sa2_tc_common.cuh"
+#include "sa2_tc_fwd.cuh"
 
 namespace sa2 {
 namespace tc {
@@ -49,7 +50,7 @@ namespace f128 {
 constexpr int THREADS = 768;
 // 768 threads start with 80 registers each; every warpgroup executes one setmaxnreg, and the budgets must add
 // up to at most 6 * 80 or the growing groups never return from theirs.
-constexpr int REGS_LAUNCH = 80, REGS_ISSUE = 56, REGS_OUT = 128, REGS_SOFTMAX = 72, REGS_PRODUCE = 24;
+constexpr int REGS_LAUNCH = 80, REGS_ISSUE = 40, REGS_OUT = 128, REGS_SOFTMAX = 80, REGS_PRODUCE = 24;
 static_assert(REGS_ISSUE + 2 * REGS_OUT + 2 * REGS_SOFTMAX + REGS_PRODUCE <= 6 * REGS_LAUNCH, "register pool must balance");
 static_assert(REGS_ISSUE <= REGS_LAUNCH && REGS_SOFTMAX <= REGS_LAUNCH && REGS_PRODUCE <= REGS_LAUNCH && REGS_OUT >= REGS_LAUNCH,
               "issuers, softmax groups and producers release registers, the output groups take them");
@@ -74,60 +75,59 @@ enum Bar {
     B_S_FULL = B_REF_FULL + 2,      // [4] group * 2 + buffer
     B_P_FULL = B_S_FULL + 4,        // [4]
     B_PV_DONE = B_P_FULL + 4,       // [4]
-    B_COUNT = B_PV_DONE + 4
+    B_WIN_FULL = B_PV_DONE + 4,     // second-value rows have landed
+    B_COUNT = B_WIN_FULL + 1
 };
 
 struct Params {
     KernelParams kp;
-    int nh;          // 64-row units per query tile: ceil((w1 + 127) / 64)
+    int ri_log2;     // query rows per tile
+    int nslots;      // (the rings' size: read by fwd_geom)
+    int win_boxes;   // 32-row boxes of staged second-value rows; 0: read from global memory
     float c;         // scale * log2(e)
     int pv_split;    // diagnostic: issue W += P V1 as two N = 64 products instead of one N = 128
     int *status;
 };
 
+constexpr int WIN_BOXES = 3;                      // most boxes of staged second-value rows
+constexpr uint32_t WIN_BLK = WIN_BOXES * 4096;    // one 64-channel block of them
 inline size_t smem_bytes() {
-    return 1024 + (size_t)2 * SLOTS * UNIT_BYTES + 2 * A_BYTES + FWD_STATS_FLOATS * 4 + B_COUNT * 8 + 64;
+    return 1024 + (size_t)2 * SLOTS * UNIT_BYTES + 2 * A_BYTES + 2 * WIN_BLK + FWD_STATS_FLOATS * 4 + B_COUNT * 8 + 64;
 }
-
-struct Geom {
-    int i0, i_last, hbase, h_first, nunits, nsweeps;
-    int nsw[2];       // sweeps of each softmax group
-};
-
-__device__ __forceinline__ Geom geom(const Params &P) {
-    Geom g;
-    g.i0 = blockIdx.x * TQ;
-    g.i_last = min(g.i0 + TQ - 1, P.kp.n - 1);
-    g.hbase = g.i0 + P.kp.off1 + TQ - UNIT * P.nh;        // unit x covers rows hbase + 64 x ... + 63
-    g.h_first = g.hbase >= 0 ? 0 : min(P.nh - 1, (-g.hbase) / UNIT);
-    g.nunits = P.nh - g.h_first;
-    g.nsweeps = min(P.kp.w2, g.i_last + P.kp.off2 + 1);
-    g.nsw[0] = (g.nsweeps + 1) / 2;
-    g.nsw[1] = g.nsweeps / 2;
-    return g;
+inline int win_boxes(int w2, int ri_log2) {
+    const int boxes = (w2 + (1 << ri_log2) - 1 + 31) / 32;
+    return boxes <= WIN_BOXES ? boxes : 0;
 }
+using Geom = FwdGeom;
 
 // ------------------------------------------------------------------ TMA producers (warps 2 and 3, one lane each)
 // Item x = (pair of sweeps x / nunits, unit x % nunits) goes to slot x % SLOTS; the walk is the one of
 // group 0, which has at least as many sweeps as group 1.
-__device__ __forceinline__ int producer(const Params &P, const Geom &g, const CUtensorMap *map, uint8_t *ring, int full0, int empty0,
+__device__ __forceinline__ int producer(const Params &P, const Geom &g, const CUtensorMap *map, const CUtensorMap *mapV2, uint8_t *ring, uint8_t *sWin, int full0, int empty0,
                                         uint64_t *bars, volatile int *abort_flag) {
     const int hk = blockIdx.y / P.kp.g, b = blockIdx.z;
     prefetch_tmap(map);
-    const int items = g.nsw[0] * g.nunits;
+    const bool stage = mapV2 && P.win_boxes > 0;
+    if (stage && elect_one()) {
+        mbar_arrive_expect_tx(&bars[B_WIN_FULL], 2 * P.win_boxes * 4096);
+        for (int bx = 0; bx < P.win_boxes; ++bx)
+            for (int cb = 0; cb < 2; ++cb) tma_load_4d(sWin + cb * WIN_BLK + bx * 4096, mapV2, &bars[B_WIN_FULL], cb * 64, hk, g.win0 + 32 * bx, b);
+    }
+    const int items = g.nsw[0] * g.upe;
     int w = 0;
     for (int x = 0; x < items; ++x) {
         const int slot = x % SLOTS;
         if (x >= SLOTS && !mbar_wait_warp(&bars[empty0 + slot], (x / SLOTS - 1) & 1, abort_flag, 32, 1)) return ERR_FWD_PRODUCER;
-        const int row = g.hbase + UNIT * (g.h_first + w);
+        const int row = g.jbase + UNIT * w;
         if (elect_one()) {
         mbar_arrive_expect_tx(&bars[full0 + slot], UNIT_BYTES);
         tma_load_4d(ring + slot * UNIT_BYTES, map, &bars[full0 + slot], 0, hk, row, b);
         tma_load_4d(ring + slot * UNIT_BYTES + BLK_BYTES, map, &bars[full0 + slot], 64, hk, row, b);
         }
-        if (++w == g.nunits) w = 0;
+        if (++w == g.upe) w = 0;
     }
     // every load must have landed before the CTA may exit, even if the consumers gave up
+    if (stage && !mbar_wait_warp(&bars[B_WIN_FULL], 0, abort_flag, 32)) return ERR_FWD_PRODUCER;
     for (int x = max(0, items - SLOTS); x < items; ++x)
         if (!mbar_wait_warp(&bars[full0 + x % SLOTS], (x / SLOTS) & 1, abort_flag, 32)) return ERR_FWD_PRODUCER;
     return 0;
@@ -143,7 +143,7 @@ __device__ __forceinline__ int issue_s(const Params &P, const Geom &g, int grp, 
     const uint64_t dA = smem_desc_sw128(smem_u32(sA) + grp * A_BYTES);
     const uint64_t dK = smem_desc_sw128(smem_u32(sK));
     const uint32_t tS = tmem + grp * 128;
-    const int nu = g.nunits;
+    const int nu = g.upe;
     const int n = g.nsw[grp] * nu;
     int w = 0, ks = 0;
     for (int u = 0; u < n; ++u) {
@@ -184,7 +184,7 @@ __device__ __forceinline__ int issue_pv(const Params &P, const Geom &g, int grp,
     constexpr uint32_t IDESC_PV64 = idesc_bf16(128, 64, false, true);
     const uint64_t dV = smem_desc_sw128(smem_u32(sV), 1024, BLK_BYTES);     // N = 128: channel blocks 8 KB apart
     const uint32_t tS = tmem + grp * 128, tW = tmem + 256 + grp * 128;
-    const int nu = g.nunits;
+    const int nu = g.upe;
     const int n = g.nsw[grp] * nu;
     int w = 0, ks = 0;
     for (int u = 0; u < n; ++u) {
@@ -228,33 +228,43 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
     const int r = (warp & 3) * 32 + lane;            // query row within the tile = TMEM lane
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t s_addr = lane_addr + grp * 128, w_addr = lane_addr + 256 + grp * 128;
-    const int i = g.i0 + r;
-    const bool row_ok = i < kp.n;
+    const int i = g.i0 + (r & (g.ri - 1)), e0 = r >> g.ri_log2;
+    const FwdWarpRows wr = fwd_warp_rows(kp, g);
     const float c = P.c;
     const int nsw = g.nsw[grp];
     float *ref_slot = stats + grp * 256 + r;          // + 128 * (parity of the group's sweep counter)
 
     float ref = -CUDART_INF_F, l = 0.f;
     int u = 0;
-    const int nu = g.nunits;
+    const int nu = g.upe;
     // The hand-over of a unit's P (wait for the TMEM stores, then arrive) is deferred until the first load of
     // the next unit has been issued, so that the store latency passes under that load.
     int pending = -1;
     {
         for (int ks = 0; ks < nsw; ++ks) {
-            const int e = 2 * ks + grp;
-            const bool sweep_ok = row_ok && (i + kp.off2 - e >= 0);
+            const int eb = g.re * (2 * ks + grp);
+            // every row of the warp pairs with a second key in this sweep / no row does
+            const bool all_ok = wr.imax < kp.n && eb + wr.emax < kp.w2 && wr.imin + kp.off2 - eb - wr.emax >= 0;
+            const bool none_ok = wr.imin >= kp.n || eb + wr.emin >= kp.w2 || wr.imax + kp.off2 - eb - wr.emin < 0;
+            const bool row_ok = i < kp.n && eb + e0 < kp.w2 && i + kp.off2 - eb - e0 >= 0;
+            const int full0 = all_ok ? wr.full0 : 1 << 30, some1 = none_ok ? -1 : wr.some1;
 #pragma unroll 1
             for (int w = 0; w < nu; ++w, ++u) {
                 const int sb = u & 1;
-                const int j0 = g.hbase + UNIT * (g.h_first + w);
+                const int j0 = g.jbase + UNIT * w;
                 // valid columns of this row: lo < col <= hi
-                const int d1 = i + kp.off1 - j0;
-                const int hi = sweep_ok ? min(d1, 63) : -1;
-                const int lo = max(d1 - kp.w1, -j0 - 1);
+                const int d1 = i + kp.off1 - j0, hi = row_ok ? d1 : -1, lo = max(d1 - kp.w1, -j0 - 1);
+                // exponentials of one 32-key chunk: all columns valid for every row of the warp, masked, or none
+                auto chunk = [&](const uint32_t (&s)[32], uint32_t (&pk)[16], int ch) -> float {
+                    const int x = 2 * w + ch;
+                    if (x >= full0 && x <= wr.full1) return fwd_probs32(s, pk, c, ref, true, 0, 0, 0);
+                    if (x >= wr.some0 && x <= some1) return fwd_probs32(s, pk, c, ref, false, ch * 32, lo, hi);
+#pragma unroll
+                    for (int z = 0; z < 16; ++z) pk[z] = 0u;
+                    return 0.f;
+                };
                 if (!warp_wait(&bars[B_S_FULL + grp * 2 + sb], (u >> 1) & 1, abort_flag, 1)) return ERR_FWD_SOFTMAX;
                 tc_fence_after();
-                const bool full = __all_sync(0xffffffffu, lo < 0 && hi >= 63);
                 const uint32_t buf = s_addr + sb * 64;
 
                 // the whole unit is read before any P is stored: P lies over the S columns
@@ -267,10 +277,10 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
                     pending = -1;
                 }
                 tmem_wait_ld();
-                float tile_sum = fwd_probs32(s, pk0, c, ref, full, 0, lo, hi);
+                float tile_sum = chunk(s, pk0, 0);
                 tmem_ld32(buf + 32, s);
                 tmem_wait_ld();
-                tile_sum += fwd_probs32(s, pk1, c, ref, full, 32, lo, hi);
+                tile_sum += chunk(s, pk1, 1);
                 const bool exceed = !(tile_sum <= 1.8446744e19f);       // above 2^64, inf or NaN
                 if (__any_sync(0xffffffffu, exceed)) {
                     // ---- slow path (whole warp): exact maximum of this unit, rescale, recompute
@@ -340,53 +350,44 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
 }
 
 // ------------------------------------------------------------------ output threads (warps 4-7: channels 0-63, 8-11: 64-127)
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-}
-
 __device__ __forceinline__ int output(const Params &P, const Geom &g, int cb, uint32_t tmem, float (&o)[64], float &ref_o,
-                                      uint8_t *sA, const float *stats, uint64_t *bars, volatile int *abort_flag) {
+                                      const uint8_t *sWin, uint8_t *sA, const float *stats, uint64_t *bars, volatile int *abort_flag) {
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
-    const int i = g.i0 + r;
-    const bool row_ok = i < kp.n;
-    const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p);
+    const int i = g.i0 + (r & (g.ri - 1)), e0 = r >> g.ri_log2;
+    const bool row_ok = i < kp.n, staged = P.win_boxes > 0;
+    const __nv_bfloat16 *q = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, 0, h);
+    const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p) + elem_off(kp.k2, b, 0, hk);
     const __nv_bfloat16 *v2 = reinterpret_cast<const __nv_bfloat16 *>(kp.v2.p);
-    const __nv_bfloat16 *qrow = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, row_ok ? i : 0, h) + cb * 64;
     const int T0 = g.nsw[0], T1 = g.nsw[1];
 
-    // This thread's half of row r of A_e = q_i * k2_{i-e}, e = 2 t + grp, into the group's A stage.  The
-    // loads of the first 32 channels are issued before the wait for the stage (`bar`, unless null), so
-    // that their latency passes while the tensor cores still read the previous A_e.
+    // A = q_i * k2_{i-e} of the group's sweep t: sixteen lanes take a row, 16 bytes each, so that a load of the warp
+    // is two whole rows (a row per lane touches 32 cache lines per load, ~4000 cycles of L1 per sweep); the first four
+    // rows of a lane are fetched before the wait for the stage (`bar`, unless null).
+    const int row0 = (warp - 4) * 16 + (lane >> 4), cc = lane & 15;
     auto build_a = [&](int grp, int t, uint64_t *bar, uint32_t parity) -> bool {
-        const int e = 2 * t + grp;
-        uint8_t *dst = sA + (size_t)grp * A_BYTES + (size_t)cb * ABLK_BYTES;
-        const int kk = i + kp.off2 - e;
-        const bool ok = row_ok && kk >= 0;
-        const __nv_bfloat16 *krow = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk) + cb * 64;
+        uint8_t *dst = sA + (size_t)grp * A_BYTES + (size_t)(cc >> 3) * ABLK_BYTES;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             uint4 qv[4], kv[4];
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                qv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(qrow + (half * 4 + cc) * 8)) : make_uint4(0u, 0u, 0u, 0u);
-                kv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(krow + (half * 4 + cc) * 8)) : make_uint4(0u, 0u, 0u, 0u);
+            for (int x = 0; x < 4; ++x) {
+                const int rr = row0 + 2 * (half * 4 + x), ii = g.i0 + (rr & (g.ri - 1)), e = g.re * (2 * t + grp) + (rr >> g.ri_log2);
+                const int kk = ii + kp.off2 - e;
+                const bool ok = ii < kp.n && e < kp.w2 && kk >= 0;
+                qv[x] = ok ? __ldg(reinterpret_cast<const uint4 *>(q + (int64_t)ii * kp.q.sn + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
+                kv[x] = ok ? __ldg(reinterpret_cast<const uint4 *>(k2 + (int64_t)kk * kp.k2.sn + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
             }
             if (half == 0 && bar && !warp_wait(bar, parity, abort_flag, 1)) return false;
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
+            for (int x = 0; x < 4; ++x) {
                 uint4 v;
-                v.x = mul_bf16x2(qv[cc].x, kv[cc].x); v.y = mul_bf16x2(qv[cc].y, kv[cc].y);
-                v.z = mul_bf16x2(qv[cc].z, kv[cc].z); v.w = mul_bf16x2(qv[cc].w, kv[cc].w);
-                *reinterpret_cast<uint4 *>(dst + sw128_offset(r, half * 4 + cc)) = v;
+                v.x = mul_bf16x2(qv[x].x, kv[x].x); v.y = mul_bf16x2(qv[x].y, kv[x].y);
+                v.z = mul_bf16x2(qv[x].z, kv[x].z); v.w = mul_bf16x2(qv[x].w, kv[x].w);
+                *reinterpret_cast<uint4 *>(dst + sw128_offset(row0 + 2 * (half * 4 + x), cc & 7)) = v;
             }
         }
         fence_proxy_async_smem();
@@ -397,12 +398,16 @@ __device__ __forceinline__ int output(const Params &P, const Geom &g, int cb, ui
     // o += v2_{i-e} * W (TMEM), with o held against the larger reference seen so far; the v2 row is
     // fetched before the waits
     auto drain = [&](int grp, int t) -> bool {
-        const int kk = i + kp.off2 - (2 * t + grp);
-        const bool row = row_ok && kk >= 0;
+        const int e = g.re * (2 * t + grp) + e0, kk = i + kp.off2 - e;
+        const bool row = row_ok && e < kp.w2 && kk >= 0;
         const __nv_bfloat16 *vp = v2 + elem_off(kp.v2, b, row ? kk : 0, hk) + cb * 64;
+        const uint8_t *wp = sWin + cb * WIN_BLK;
         uint4 raw[8];
 #pragma unroll
-        for (int cc = 0; cc < 8; ++cc) raw[cc] = row ? __ldg(reinterpret_cast<const uint4 *>(vp + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
+        for (int x = 0; x < 8; ++x) {
+            raw[x] = make_uint4(0u, 0u, 0u, 0u);
+            if (row) raw[x] = staged ? *reinterpret_cast<const uint4 *>(wp + sw128_offset(kk - g.win0, x)) : __ldg(reinterpret_cast<const uint4 *>(vp + x * 8));
+        }
         if (!warp_wait(&bars[B_REF_FULL + grp], t & 1, abort_flag, 2)) return false;
         const float ref_w = stats[grp * 256 + (t & 1) * 128 + r];
         if (!warp_wait(&bars[B_W_FULL + grp], t & 1, abort_flag, 3)) return false;
@@ -444,6 +449,7 @@ __device__ __forceinline__ int output(const Params &P, const Geom &g, int cb, ui
         return true;
     };
 
+    if (staged && !warp_wait(&bars[B_WIN_FULL], 0, abort_flag)) return ERR_FWD_OUTPUT;
     if (T0 > 0) build_a(0, 0, nullptr, 0);
     if (T1 > 0) build_a(1, 0, nullptr, 0);
     for (int t = 0; t < T0; ++t) {
@@ -457,21 +463,24 @@ __device__ __forceinline__ int output(const Params &P, const Geom &g, int cb, ui
 }
 
 __device__ __forceinline__ void rows_sync() { asm volatile("bar.sync 2, 512;" ::: "memory"); }
+__device__ __forceinline__ void out_sync() { asm volatile("bar.sync 3, 256;" ::: "memory"); }
 
 __global__ void __launch_bounds__(THREADS, 1)
-fwd128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const Params P) {
+fwd128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapV2,
+              const Params P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;                               // K1 ring
     uint8_t *sV = sK + SLOTS * UNIT_BYTES;            // V1 ring
     uint8_t *sA = sV + SLOTS * UNIT_BYTES;
-    float *stats = reinterpret_cast<float *>(sA + 2 * A_BYTES);
+    uint8_t *sWin = sA + 2 * A_BYTES;                 // staged second-value rows
+    float *stats = reinterpret_cast<float *>(sWin + 2 * WIN_BLK);
     uint64_t *bars = reinterpret_cast<uint64_t *>(stats + FWD_STATS_FLOATS);
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + B_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);       // warp-uniform, and known to be
-    const Geom g = geom(P);
+    const Geom g = fwd_geom(P);
     if (threadIdx.x == 0) {
         for (int x = 0; x < B_COUNT; ++x) {
             uint32_t count = 1;
@@ -507,8 +516,8 @@ fwd128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
         else err = issue_pv(P, g, 1, tmem, sV, bars, abort_flag);
     } else if (warp >= 20) {
         reg_dealloc<REGS_PRODUCE>();
-        if (warp == 20) err = producer(P, g, &mapK, sK, B_K_FULL, B_K_EMPTY, bars, abort_flag);
-        else if (warp == 21) err = producer(P, g, &mapV, sV, B_V_FULL, B_V_EMPTY, bars, abort_flag);
+        if (warp == 20) err = producer(P, g, &mapK, nullptr, sK, sWin, B_K_FULL, B_K_EMPTY, bars, abort_flag);
+        else if (warp == 21) err = producer(P, g, &mapV, &mapV2, sV, sWin, B_V_FULL, B_V_EMPTY, bars, abort_flag);
     } else if (warp >= 12) {
         reg_dealloc<REGS_SOFTMAX>();
         err = softmax(P, g, (warp - 12) >> 2, tmem, stats, bars, abort_flag);
@@ -521,35 +530,48 @@ fwd128_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
 #pragma unroll
         for (int x = 0; x < 64; ++x) o[x] = 0.f;
         float ref_o = -CUDART_INF_F;
-        err = output(P, g, cb, tmem, o, ref_o, sA, stats, bars, abort_flag);
+        err = output(P, g, cb, tmem, o, ref_o, sWin, sA, stats, bars, abort_flag);
         rows_sync();                                  // both groups' denominators are in shared memory
 
-        // merge: each denominator is expressed against its group's last reference, o against ref_o
+        if (err) *abort_flag = 1;
+        out_sync();
+        const bool bad = *abort_flag != 0;
+        // Merge of the RE partial results of every query row, over the K1 / V1 rings, which nothing reads any more: 128 rows
+        // of 132 floats, then two rows of statistics.  Each denominator is expressed against its group's last reference,
+        // o against ref_o.
+        constexpr int LD = 132;
         const KernelParams &kp = P.kp;
-        const int r = ((warp & 3) * 32) + (threadIdx.x & 31);
-        const int i = g.i0 + r;
-        const float l0 = stats[512 + r], l1 = stats[640 + r];
-        const float lref0 = stats[768 + r], lref1 = stats[896 + r];
-        const float rmax = fmaxf(lref0, lref1);
-        const float f0 = lref0 > -CUDART_INF_F ? ex2(lref0 - rmax) : 0.f;
-        const float f1 = lref1 > -CUDART_INF_F ? ex2(lref1 - rmax) : 0.f;
-        const float l = l0 * f0 + l1 * f1;
-        if (i < kp.n) {
-            // a CTA in which any wait ran out reports NaN instead of leaving its rows unwritten
-            const bool bad = err != 0 || *abort_flag != 0;
-            const float sc = bad ? CUDART_NAN_F : (ref_o > -CUDART_INF_F ? ex2(ref_o - rmax) / l : 0.f);
-            __nv_bfloat16 *op = reinterpret_cast<__nv_bfloat16 *>(kp.out.p) + elem_off(kp.out, blockIdx.z, i, blockIdx.y) + cb * 64;
+        float *buf = reinterpret_cast<float *>(sK), *sM = buf + 128 * LD, *sL = sM + 128;
+        const int r = ((warp & 3) * 32) + (threadIdx.x & 31), ii = r & (g.ri - 1), i = g.i0 + ii;
+        if (cb == 0) {
+            const float m0 = stats[768 + r], m1 = stats[896 + r], m = fmaxf(m0, m1);
+            const float f0 = m0 > -CUDART_INF_F ? ex2(m0 - m) : 0.f, f1 = m1 > -CUDART_INF_F ? ex2(m1 - m) : 0.f;
+            sM[r] = m;
+            sL[r] = stats[512 + r] * f0 + stats[640 + r] * f1;
+        }
+        out_sync();
+        float M = -CUDART_INF_F, L = 0.f;
+        for (int s = 0; s < g.re; ++s) M = fmaxf(M, sM[s * g.ri + ii]);
+        for (int s = 0; s < g.re; ++s) {
+            const float ms = sM[s * g.ri + ii];
+            L += ms > -CUDART_INF_F ? sL[s * g.ri + ii] * ex2(ms - M) : 0.f;
+        }
+        const float sc = bad ? CUDART_NAN_F : ref_o > -CUDART_INF_F ? ex2(ref_o - M) / L : 0.f;     // (a CTA in which a wait ran out reports NaN)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                uint4 v;
-                v.x = pack_bf16(o[u * 8 + 0] * sc, o[u * 8 + 1] * sc);
-                v.y = pack_bf16(o[u * 8 + 2] * sc, o[u * 8 + 3] * sc);
-                v.z = pack_bf16(o[u * 8 + 4] * sc, o[u * 8 + 5] * sc);
-                v.w = pack_bf16(o[u * 8 + 6] * sc, o[u * 8 + 7] * sc);
-                *reinterpret_cast<uint4 *>(op + u * 8) = v;
+        for (int x = 0; x < 64; x += 4)
+            *reinterpret_cast<float4 *>(buf + r * LD + cb * 64 + x) = make_float4(o[x] * sc, o[x + 1] * sc, o[x + 2] * sc, o[x + 3] * sc);
+        if (cb == 0 && r < g.ri && i < kp.n)
+            kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = bad ? CUDART_NAN_F : (M + lg2(L)) * 0.6931471805599453f;
+        out_sync();
+        for (int x = threadIdx.x - 128; x < g.ri * 32; x += 256) {
+            const int row = x >> 5, c = (x & 31) * 4;
+            if (g.i0 + row >= kp.n) break;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int s = 0; s < g.re; ++s) {
+                const float4 f = *reinterpret_cast<const float4 *>(buf + (s * g.ri + row) * LD + c);
+                v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
             }
-            if (cb == 0)
-                kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = bad ? CUDART_NAN_F : (rmax + lg2(l)) * 0.6931471805599453f;
+            store_vec<4>(kp.out.p, elem_off(kp.out, blockIdx.z, g.i0 + row, blockIdx.y) + c, true, v);
         }
     }
     if (err) atomicOr(P.status, err);
