@@ -7,7 +7,7 @@
 // walks over every (query head of the group, query tile I, offset e) that can
 // see its keys.  Per step the builder warps form
 //     A_e[i,:] = q_i * k2_{i-e}      B_e[i,:] = dO_i * v2_{i-e}      (bf16)
-// and the tensor cores compute, in two 64-column halves that ping-pong,
+// and the tensor cores compute, in units of 64 query columns,
 //     S^T  = K1 A_e^T       dP^T = V1 B_e^T          (rows j, columns i)
 // the compute warps (one thread per key row j) turn them into
 //     P^T = exp2(c S^T - lse2_i)      G^T = P^T * (dP^T - D_i)
@@ -21,28 +21,35 @@
 // of ones on the key side adds them with one more K=16 MMA, so that the accumulators already hold
 // S^T - lse2 / c and dP^T - D and the compute threads need no per-column loads.
 //
-// Warps (480 threads; warp 14 issues dP^T next to warp 1, which issues S^T): 0 TMA producer, then issuer of the second products (dV1, dK1);
-// 1 TMEM owner and issuer of the first products (S^T, dP^T); 2-5 compute group of
-// half 0; 6-9 compute group of half 1; 10-13 builders.  One thread issues about one
-// tcgen05.mma per 90 cycles, so the two products have an issuing thread each; dK1/dV1
-// are accumulated by one thread only, which keeps the summation order fixed.
-// TMEM columns: half h -> S^T [128h, +64), dP^T [128h+64, +64), P^T (bf16) [256+64h, +32),
-// G^T (bf16) [288+64h, +32); dK1 [384,448); dV1 [448,512).  P^T/G^T have their own
-// columns so that the next S^T/dP^T of a half can be issued as soon as the compute
-// group has read the current one.
+// Warps (640 threads, five aligned warpgroups with register hand-over): 0 TMA producer, then issuer of the second
+// products (dV1, dK1: one issuer, which keeps the summation order fixed); 1 TMEM owner and issuer of S^T; 2 issuer of
+// dP^T; 3 idle; 4-7 and 8-11 compute groups of the even and the odd units; 12-19 builders, two threads per query row.
+// TMEM columns: buffer x -> S^T [128x, +64), dP^T [128x+64, +64), three buffers in flight; P^T / G^T (bf16) overwrite the
+// first half of the S^T / dP^T columns they come from, so a buffer is busy until the second products of its unit are
+// done; dK1 [384,448); dV1 [448,512).
+//
+// Bound: the exponent passes of the two groups (512 MUFU cycles per unit and scheduler) next to ~740 cycles of products
+// and ~1700 cycles of shared-memory traffic per step of two units.  With a buffer per group, P^T / G^T in columns of
+// their own and four builder warps a group waited 1100 of 2800 cycles a step for its next S^T: the products of a unit
+// could start only when the group had finished the last (b4 n4096 h8 d64 w512/32: 1.59 -> 1.31 ms).
 //
 // The offsets may be split over several CTAs per key tile (consecutive ranges): a short sequence has few key tiles, and
 // with grouped-query heads each walks over every head of its group.  The splits write fp32 partials, which the
 // reduction of the dQ/dK2/dV2 kernel adds in order.  k1_split() picks the number.  (Splits as the CTAs of a cluster,
 // added through distributed shared memory, cost 20 to 35 % at large grids: a cluster waits for its SMs to be free
-// together.)  Measured: b1 n3001 h8/2 d64 w1024/16 0.78 -> SPLIT_LW ms, b2 n128 h4 d64 w64/32 58 -> SPLIT_ST us.
+// together.)  Measured: b1 n3001 h8/2 d64 w1024/16 0.78 -> 0.29 ms, b2 n128 h4 d64 w64/32 58 -> 16 us.
 #pragma once
 #include "sa2_tc_common.cuh"
 
 namespace sa2 {
 namespace tc {
 
-constexpr int BK1_THREADS = 480;
+constexpr int BK1_THREADS = 640;
+// 640 threads start with 96 registers each; every warpgroup executes one setmaxnreg, and the budgets must add up to at
+// most 5 * 96, or the growing groups never return from theirs.
+constexpr int BK1_REGS_LAUNCH = 96, BK1_REGS_ISSUE = 40, BK1_REGS_COMPUTE = 128, BK1_REGS_BUILD = 88;
+static_assert(BK1_REGS_ISSUE + 2 * BK1_REGS_COMPUTE + 2 * BK1_REGS_BUILD <= 5 * BK1_REGS_LAUNCH, "register pool must balance");
+constexpr int BK1_BUFS = 3;          // S^T / dP^T buffers in TMEM
 // A_e / B_e stages.  A stage is released only when the second products of its step have completed, i.e.
 // after build -> first products -> P^T/G^T pass -> second products; with two stages the builders (whose
 // 32 shared-memory accesses per step take ~1600 cycles next to the tensor cores' operand traffic) waited
@@ -53,13 +60,13 @@ enum Bk1Bar {
     BK1_KV_FULL = 0,
     BK1_AB_FULL = 1,     // [BK1_STAGES]
     BK1_AB_EMPTY = 4,    // [BK1_STAGES]
-    BK1_S_FULL = 7,      // [2] per half
-    BK1_P_FULL = 9,      // [2] per half
-    BK1_G_DONE = 11,     // [2] per half: second products of the step have completed
-    BK1_DONE = 13,
-    BK1_WIN_FREE = 14,   // the builders have finished reading the k2/v2 window of the previous query tile
-    BK1_WIN_FULL = 15,   // the window of the current query tile has landed
-    BK1_BAR_COUNT = 16
+    BK1_S_FULL = 7,      // [BK1_BUFS]
+    BK1_P_FULL = 10,     // [BK1_BUFS]
+    BK1_G_DONE = 13,     // [BK1_BUFS] second products of the unit have completed
+    BK1_DONE = 16,
+    BK1_WIN_FREE = 17,   // the builders have finished reading the k2/v2 window of the previous query tile
+    BK1_WIN_FULL = 18,   // the window of the current query tile has landed
+    BK1_BAR_COUNT = 19
 };
 
 enum { ERR_BK1_PRODUCER = 16, ERR_BK1_MMA = 32, ERR_BK1_COMPUTE = 64, ERR_BK1_BUILDER = 128 };
@@ -110,7 +117,7 @@ __device__ __forceinline__ Bk1Geom bk1_geom(const BwdParams &P) {
     return g;
 }
 
-// ---------------------------------------------------------------- builders (warps 10-13)
+// ---------------------------------------------------------------- builders (warps 12-19)
 // three bf16 terms whose sum is x to fp32 accuracy, packed with five zeros into one 16-byte chunk
 __device__ __forceinline__ uint4 split3_bf16(float x) {
     const __nv_bfloat16 h0 = __float2bfloat16_rn(x);
@@ -127,16 +134,16 @@ template <int D>
 __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g, const CUtensorMap *mapK2, const CUtensorMap *mapV2,
                                            uint8_t *sAB, uint8_t *sStat, uint8_t *sOnes, uint8_t *sWin,
                                            uint64_t *bars, volatile int *abort_flag) {
-    constexpr int NC = D / 8;              // 16-byte chunks of a row
+    constexpr int NC = D / 16;             // 16-byte chunks of half a row
     const KernelParams &kp = P.kp;
-    const int r = threadIdx.x - 320;       // row of the query tile
+    const int bt = threadIdx.x - 384, r = bt & 127, part = bt >> 7, c0 = part * NC;      // row of the query tile, its half
     const int hk = blockIdx.y, b = blockIdx.z;
     const __nv_bfloat16 *q = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p);
     const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p);
     const __nv_bfloat16 *dout = reinterpret_cast<const __nv_bfloat16 *>(kp.dout.p);
     const __nv_bfloat16 *v2 = reinterpret_cast<const __nv_bfloat16 *>(kp.v2.p);
     // the constant key-side tile: three ones per row (one per term of the split statistics)
-    {
+    if (part == 0) {
         uint4 one = make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u);
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc)
@@ -154,7 +161,7 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
         const bool win = P.epc <= 32;
         if (win) {
             if (tile_counter > 0) mbar_arrive(&bars[BK1_WIN_FREE]);
-            if (r == 0) {
+            if (bt == 0) {
                 if (tile_counter > 0 && !mbar_wait(&bars[BK1_WIN_FREE], (tile_counter - 1) & 1, abort_flag)) return ERR_BK1_BUILDER;
                 mbar_arrive_expect_tx(&bars[BK1_WIN_FULL], 2 * BK1_WIN_ROWS * 128);
                 const int row0 = g.i_lo + TQ * t + kp.off2 - g.e0 - 32;
@@ -168,18 +175,17 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
         uint4 qv[NC], dv[NC];
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc) { qv[cc] = make_uint4(0, 0, 0, 0); dv[cc] = make_uint4(0, 0, 0, 0); }
-        float lse2 = 0.f, dl = 0.f;
+        float stat = 0.f;                   // half 0: -lse2 / c, half 1: -D
         if (iv) {
-            const __nv_bfloat16 *qp = q + elem_off(kp.q, b, i, h);
-            const __nv_bfloat16 *dp = dout + elem_off(kp.dout, b, i, h);
+            const __nv_bfloat16 *qp = q + elem_off(kp.q, b, i, h) + c0 * 8;
+            const __nv_bfloat16 *dp = dout + elem_off(kp.dout, b, i, h) + c0 * 8;
 #pragma unroll
             for (int cc = 0; cc < NC; ++cc) {
                 qv[cc] = *reinterpret_cast<const uint4 *>(qp + cc * 8);
                 dv[cc] = *reinterpret_cast<const uint4 *>(dp + cc * 8);
             }
             const int64_t o = ((int64_t)b * kp.hq + h) * kp.n + i;
-            lse2 = kp.lse[o] * 1.4426950408889634f;
-            dl = kp.delta[o];
+            stat = part == 0 ? -kp.lse[o] * 1.4426950408889634f * inv_c : -kp.delta[o];
         }
         for (int e = 0; e < ne; ++e, ++s) {
             const int stage = s % BK1_STAGES;
@@ -189,35 +195,33 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
                 // such tiles hold the last four query tiles.  Step s - 3 has completed, and every tile has
                 // at least one step, so the slabs of four tiles ago are no longer read.
                 uint8_t *st = sStat + (size_t)((tile_counter >> 1) & 1) * TILE_BYTES;
-                const int c0 = (tile_counter & 1) * 4;
-                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0)) = split3_bf16(-lse2 * inv_c);
-                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 1)) = make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 2)) = split3_bf16(-dl);
-                *reinterpret_cast<uint4 *>(st + sw128_offset(r, c0 + 3)) = make_uint4(0u, 0u, 0u, 0u);
+                const int ch = (tile_counter & 1) * 4 + 2 * part;
+                *reinterpret_cast<uint4 *>(st + sw128_offset(r, ch)) = split3_bf16(stat);
+                *reinterpret_cast<uint4 *>(st + sw128_offset(r, ch + 1)) = make_uint4(0u, 0u, 0u, 0u);
             }
             uint8_t *dA = sAB + (size_t)stage * 2 * TILE_BYTES;
             uint8_t *dB = dA + TILE_BYTES;
             const int kk = i + kp.off2 - g.e0 - e;
             const bool ok = iv && kk >= 0;
-            const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-            const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk);
+            const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk) + c0 * 8;
+            const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk) + c0 * 8;
             const int wr = r + 32 - e;                       // row of the staged window
             const uint8_t *wk = sWin + wr * 128, *wv = wk + BK1_WIN_ROWS * 128;
 #pragma unroll
             for (int cc = 0; cc < NC; ++cc) {
                 uint4 a = make_uint4(0, 0, 0, 0), bb = make_uint4(0, 0, 0, 0);
                 if (ok) {
-                    const uint4 kv = win ? *reinterpret_cast<const uint4 *>(wk + ((cc ^ (wr & 7)) << 4))
+                    const uint4 kv = win ? *reinterpret_cast<const uint4 *>(wk + (((c0 + cc) ^ (wr & 7)) << 4))
                                          : *reinterpret_cast<const uint4 *>(kp2 + cc * 8);
-                    const uint4 vv = win ? *reinterpret_cast<const uint4 *>(wv + ((cc ^ (wr & 7)) << 4))
+                    const uint4 vv = win ? *reinterpret_cast<const uint4 *>(wv + (((c0 + cc) ^ (wr & 7)) << 4))
                                          : *reinterpret_cast<const uint4 *>(vp2 + cc * 8);
                     a.x = mul_bf16x2(qv[cc].x, kv.x); a.y = mul_bf16x2(qv[cc].y, kv.y);
                     a.z = mul_bf16x2(qv[cc].z, kv.z); a.w = mul_bf16x2(qv[cc].w, kv.w);
                     bb.x = mul_bf16x2(dv[cc].x, vv.x); bb.y = mul_bf16x2(dv[cc].y, vv.y);
                     bb.z = mul_bf16x2(dv[cc].z, vv.z); bb.w = mul_bf16x2(dv[cc].w, vv.w);
                 }
-                *reinterpret_cast<uint4 *>(dA + sw128_offset(r, cc)) = a;
-                *reinterpret_cast<uint4 *>(dB + sw128_offset(r, cc)) = bb;
+                *reinterpret_cast<uint4 *>(dA + sw128_offset(r, c0 + cc)) = a;
+                *reinterpret_cast<uint4 *>(dB + sw128_offset(r, c0 + cc)) = bb;
             }
             fence_proxy_async_smem();
             mbar_arrive(&bars[BK1_AB_FULL + stage]);
@@ -226,12 +230,8 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
     return 0;
 }
 
-// ---------------------------------------------------------------- issuer of S^T, dP^T (warp 1, one lane)
-// which = 0: S^T = K1 A_e^T - lse2 / c into columns [128 half, +64) (warp 1);
-// which = 1: dP^T = V1 B_e^T - D into columns [128 half + 64, +64) (warp 14).
-// The two products have an issuing thread each: the time from "the compute group has read the buffer" to
-// "the next S^T / dP^T are complete" is on the critical chain of every step, and one thread issues only
-// one tcgen05.mma per 60-100 cycles.
+// ---------------------------------------------------------------- issuers of S^T (warp 1) and dP^T (warp 2)
+// Unit u is half u & 1 of step u / 2 and uses buffer u % 3.  which = 0: S^T = K1 A_e^T - lse2 / c; 1: dP^T = V1 B_e^T - D.
 template <int D>
 __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Geom &g, int which, uint32_t tmem, uint8_t *sKV,
                                              uint8_t *sAB, uint8_t *sStat, uint8_t *sOnes, uint64_t *bars, volatile int *abort_flag) {
@@ -240,7 +240,7 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
     const uint64_t dAB = smem_desc_sw128(smem_u32(sAB + which * TILE_BYTES));
     const uint64_t dSt = smem_desc_sw128(smem_u32(sStat)), dOnes = smem_desc_sw128(smem_u32(sOnes));
     if (!mbar_wait_warp(&bars[BK1_KV_FULL], 0, abort_flag)) return ERR_BK1_MMA;
-    int s = 0, tile_counter = 0;
+    int s = 0, tile_counter = 0, buf = 0, use = 0;
     for (int x = g.x0; x < g.x1; ++x, ++tile_counter) {
         const int t = x % g.n_it;
         const int ne = bk1_sweeps(kp, g, t);
@@ -251,57 +251,56 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
             if (!mbar_wait_warp(&bars[BK1_AB_FULL + stage], (s / BK1_STAGES) & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                // the compute group must have read the previous step's S^T / dP^T of this half
-                if (s >= 1 && !mbar_wait_warp(&bars[BK1_P_FULL + half], (s - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
+                // the buffer holds P^T / G^T of its last unit until the second products of that unit are done
+                if (use >= 1 && !mbar_wait_warp(&bars[BK1_G_DONE + buf], (use - 1) & 1, abort_flag, 0, 2)) return ERR_BK1_MMA;
                 tc_fence_after();
                 const uint64_t a = dAB + (uint64_t)((stage * 2 * TILE_BYTES + half * 8192) >> 4);
                 const uint64_t st = stL0 + (uint64_t)((half * 8192) >> 4) + (uint64_t)(which * 2);
-                const uint32_t d = tmem + half * 128 + which * 64;
+                const uint32_t d = tmem + buf * 128 + which * 64;
                 if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k) mma_ss(d, dT + 2 * k, a + 2 * k, IDESC_F, k > 0 ? 1u : 0u);
                 mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
-                tc_commit(&bars[BK1_S_FULL + half]);
+                tc_commit(&bars[BK1_S_FULL + buf]);
                 }
+                if (++buf == BK1_BUFS) { buf = 0; ++use; }
             }
         }
     }
     return 0;
 }
 
-// ---------------------------------------------------------------- issuer of dV1, dK1 (warp 0, one lane)
+// ---------------------------------------------------------------- issuer of dV1, dK1 (warp 0)
 template <int D>
 __device__ __forceinline__ int bk1_mma_second(const Bk1Geom &g, uint32_t tmem, uint8_t *sAB, uint64_t *bars, volatile int *abort_flag) {
     constexpr uint32_t IDESC_G = idesc_bf16(128, D, false, true);    // B operand MN-major
     const uint64_t dAB = smem_desc_sw128(smem_u32(sAB));
+    int buf = 0, use = 0;
     for (int s = 0; s < g.total; ++s) {
         const int stage = s % BK1_STAGES;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            if (!mbar_wait_warp(&bars[BK1_P_FULL + half], s & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
+            if (!mbar_wait_warp(&bars[BK1_P_FULL + buf], use & 1, abort_flag, 0, 1)) return ERR_BK1_MMA;
             tc_fence_after();
             const uint64_t a = dAB + (uint64_t)((stage * 2 * TILE_BYTES + half * 8192) >> 4), bq = a + (TILE_BYTES >> 4);
-            const uint32_t t = tmem + 256 + half * 64;
+            const uint32_t tp = tmem + buf * 128, tg = tp + 64;
             const uint32_t first = (s > 0 || half > 0) ? 1u : 0u;
             if (elect_one()) {
-            mma_ts(tmem + 448, t, bq, IDESC_G, first);
-            mma_ts(tmem + 448, t + 8, bq + 128, IDESC_G, 1u);
-            mma_ts(tmem + 448, t + 16, bq + 256, IDESC_G, 1u);
-            mma_ts(tmem + 448, t + 24, bq + 384, IDESC_G, 1u);
-            mma_ts(tmem + 384, t + 32, a, IDESC_G, first);
-            mma_ts(tmem + 384, t + 40, a + 128, IDESC_G, 1u);
-            mma_ts(tmem + 384, t + 48, a + 256, IDESC_G, 1u);
-            mma_ts(tmem + 384, t + 56, a + 384, IDESC_G, 1u);
-            tc_commit(&bars[BK1_G_DONE + half]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma_ts(tmem + 448, tp + 8 * k, bq + 128 * k, IDESC_G, k > 0 ? 1u : first);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma_ts(tmem + 384, tg + 8 * k, a + 128 * k, IDESC_G, k > 0 ? 1u : first);
+            tc_commit(&bars[BK1_G_DONE + buf]);
             if (half == 1) tc_commit(&bars[BK1_AB_EMPTY + stage]);
             }
+            if (++buf == BK1_BUFS) { buf = 0; ++use; }
         }
     }
     if (elect_one()) tc_commit(&bars[BK1_DONE]);
     return 0;
 }
 
-// ---------------------------------------------------------------- compute (group h = half h: warps 2-5, 6-9)
+// ---------------------------------------------------------------- compute (group h: units of half h; warps 4-7, 8-11)
 template <int D>
 __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g, int half, uint32_t tmem,
                                            uint64_t *bars, volatile int *abort_flag) {
@@ -309,7 +308,6 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = (warp & 3) * 32 + lane;          // key row within the tile = TMEM lane
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t buf = lane_addr + half * 128, pg = lane_addr + 256 + half * 64;
     const int hk = blockIdx.y, b = blockIdx.z;
     const int j = g.j0 + r;
     const bool jv = j < kp.nk1;
@@ -317,20 +315,19 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
 
     // the walk over the steps; a wait that runs out ends it early, the rows are then reported as NaN below
     auto walk = [&]() -> int {
-        int s = 0;
+        int s = 0, u = half;
         for (int xt = g.x0; xt < g.x1; ++xt) {
             const int t = xt % g.n_it;
             const int it0 = g.i_lo + TQ * t;
             const int ne = bk1_sweeps(kp, g, t);
             const int base = j - kp.off1 - it0;                       // column of the diagonal i + off1 == j
             const int hi = (jv ? min(min(TQ - 1, base + kp.w1 - 1), g.i_hi - it0) : -1) - half * 64;
-            for (int e = 0; e < ne; ++e, ++s) {
+            for (int e = 0; e < ne; ++e, ++s, u += 2) {
+                const uint32_t buf = lane_addr + (u % BK1_BUFS) * 128;
                 const int lo = max(max(0, base), g.e0 + e - kp.off2 - it0) - half * 64;     // valid columns: lo <= col <= hi
-                if (!warp_wait(&bars[BK1_S_FULL + half], s & 1, abort_flag, 1)) return ERR_BK1_COMPUTE;
+                if (!warp_wait(&bars[BK1_S_FULL + u % BK1_BUFS], (u / BK1_BUFS) & 1, abort_flag, 1)) return ERR_BK1_COMPUTE;
                 tc_fence_after();
                 const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 63);
-                // P^T / G^T of the previous step must have been consumed before they are overwritten
-                if (s >= 1 && !warp_wait(&bars[BK1_G_DONE + half], (s - 1) & 1, abort_flag, 2)) return ERR_BK1_COMPUTE;
 #pragma unroll
                 for (int ch = 0; ch < 2; ++ch) {
                     uint32_t sv[32], dv[32], pk[16], gk[16];
@@ -362,12 +359,13 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
                             gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
                         }
                     }
-                    tmem_st16(pg + ch * 16, pk);
-                    tmem_st16(pg + 32 + ch * 16, gk);
+                    // over columns of S^T / dP^T that this thread has already read
+                    tmem_st16(buf + ch * 16, pk);
+                    tmem_st16(buf + 64 + ch * 16, gk);
                 }
                 tmem_wait_st();
                 tc_fence_before();
-                mbar_arrive(&bars[BK1_P_FULL + half]);
+                mbar_arrive(&bars[BK1_P_FULL + u % BK1_BUFS]);
             }
         }
         return 0;
@@ -429,10 +427,11 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);       // warp-uniform, and known to be
     if (threadIdx.x == 0) {
         for (int x = 0; x < BK1_BAR_COUNT; ++x) {
-            const bool many = (x >= BK1_AB_FULL && x < BK1_AB_FULL + BK1_STAGES) || (x >= BK1_P_FULL && x < BK1_P_FULL + 2) ||
-                              x == BK1_WIN_FREE;
-            // S_FULL collects one commit from each of the two first-product issuers
-            mbar_init(&bars[x], many ? 128u : (x >= BK1_S_FULL && x < BK1_S_FULL + 2) ? 2u : 1u);
+            uint32_t count = 1;
+            if ((x >= BK1_AB_FULL && x < BK1_AB_FULL + BK1_STAGES) || x == BK1_WIN_FREE) count = 256;     // every builder
+            else if (x >= BK1_P_FULL && x < BK1_P_FULL + BK1_BUFS) count = 128;
+            else if (x >= BK1_S_FULL && x < BK1_S_FULL + BK1_BUFS) count = 2;        // one commit from each first-product issuer
+            mbar_init(&bars[x], count);
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -452,28 +451,33 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
     const long long prof_t0 = clock64();
     sa2::sm100::prof_begin();
 #endif
-    if (warp == 0) {
-        if (g.total > 0) {
-            if (elect_one()) {
-                prefetch_tmap(&mapK);
-                prefetch_tmap(&mapV);
-                mbar_arrive_expect_tx(&bars[BK1_KV_FULL], 2 * TILE_BYTES);
-                tma_load_4d(sK, &mapK, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
-                tma_load_4d(sV, &mapV, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
+    if (warp < 4) {
+        reg_dealloc<BK1_REGS_ISSUE>();
+        if (warp == 0) {
+            if (g.total > 0) {
+                if (elect_one()) {
+                    prefetch_tmap(&mapK);
+                    prefetch_tmap(&mapV);
+                    mbar_arrive_expect_tx(&bars[BK1_KV_FULL], 2 * TILE_BYTES);
+                    tma_load_4d(sK, &mapK, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
+                    tma_load_4d(sV, &mapV, &bars[BK1_KV_FULL], 0, blockIdx.y, g.j0, blockIdx.z);
+                }
+                err = bk1_mma_second<D>(g, tmem, sAB, bars, abort_flag);
+                // the tile must have landed before the CTA may exit, even if every other role gave up
+                if (!mbar_wait_warp(&bars[BK1_KV_FULL], 0, abort_flag)) err |= ERR_BK1_PRODUCER;
+            } else if (elect_one()) {
+                tc_commit(&bars[BK1_DONE]);
             }
-            err = bk1_mma_second<D>(g, tmem, sAB, bars, abort_flag);
-            // the tile must have landed before the CTA may exit, even if every other role gave up
-            if (!mbar_wait_warp(&bars[BK1_KV_FULL], 0, abort_flag)) err |= ERR_BK1_PRODUCER;
-        } else if (elect_one()) {
-            tc_commit(&bars[BK1_DONE]);
+        } else if (warp == 1) {
+            if (g.total > 0) err = bk1_mma_first<D>(P.kp, g, 0, tmem, sK, sAB, sStat, sOnes, bars, abort_flag);
+        } else if (warp == 2) {
+            if (g.total > 0) err = bk1_mma_first<D>(P.kp, g, 1, tmem, sV, sAB, sStat, sOnes, bars, abort_flag);
         }
-    } else if (warp == 1) {
-        if (g.total > 0) err = bk1_mma_first<D>(P.kp, g, 0, tmem, sK, sAB, sStat, sOnes, bars, abort_flag);
-    } else if (warp == 14) {
-        if (g.total > 0) err = bk1_mma_first<D>(P.kp, g, 1, tmem, sV, sAB, sStat, sOnes, bars, abort_flag);
-    } else if (warp < 10) {
-        err = bk1_compute<D>(P, g, (warp - 2) >> 2, tmem, bars, abort_flag);
+    } else if (warp < 12) {
+        reg_alloc<BK1_REGS_COMPUTE>();
+        err = bk1_compute<D>(P, g, (warp - 4) >> 2, tmem, bars, abort_flag);
     } else {
+        reg_dealloc<BK1_REGS_BUILD>();
         err = bk1_builder<D>(P, g, &mapK2, &mapV2, sAB, sStat, sOnes, sWin, bars, abort_flag);
     }
     if (err) atomicOr(P.status, err);
