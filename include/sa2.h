@@ -239,12 +239,13 @@ size_t sa2_headnorm_partial_bytes(int64_t rows, int32_t channels);
  * channel: channels = d * (hq + 4 * hk), laid out as the fused projection is - hq query heads, then per key/value
  * head its two keys, then per key/value head its two values.  gain[0..4] = q, k, k', v, v', d entries each
  * (16-byte aligned); the backward writes their gradients, summed over rows and heads, to dgain[0..4] in gain_dtype.
- * `partial` as for sa2_headnorm_bwd with that many channels.  d must be 32, 64 or 128.
+ * `partial` as for sa2_headnorm_bwd with that many channels.  d must be 32, 64 or 128.  The forward also takes
+ * hq = 1, hk = 0 with d up to 512: an ordinary RMSNorm over the row with gain[0] in its own type.
  */
 typedef struct sa2_qkvnorm_args {
     const void *x, *dy;
     void *y;               /* forward: y; backward: dx */
-    float *rstd;           /* [rows][hq + 4 hk] */
+    float *rstd;           /* [rows][hq + 4 hk]: written by the forward unless null, read by the backward */
     const void *gain[5];
     void *dgain[5];        /* backward only */
     void *partial;         /* backward only */

@@ -376,15 +376,17 @@ int headnorm_dispatch(const sa2_headnorm_args *a, bool backward) {
 }
 
 int qkvnorm_fill(const sa2_qkvnorm_args *a, bool backward, sa2::headnorm::Params &P, GainGrads &grads) {
-    if (!a || !a->x || !a->y || a->rows <= 0 || a->hq <= 0 || a->hk <= 0) return SA2_ERR_INVALID;
-    if (a->d != 32 && a->d != 64 && a->d != 128) return SA2_ERR_UNSUPPORTED;
+    if (!a || !a->x || !a->y || a->rows <= 0 || a->hq <= 0 || a->hk < 0) return SA2_ERR_INVALID;
+    const bool whole_row = a->hk == 0 && a->hq == 1 && !backward;      // the module's prenorm / postnorm
+    if (a->hk == 0 && !whole_row) return SA2_ERR_INVALID;
+    if (a->d != 32 && a->d != 64 && a->d != 128 && !(whole_row && (a->d == 256 || a->d == 512))) return SA2_ERR_UNSUPPORTED;
     for (int dt : {a->x_dtype, a->y_dtype, a->gain_dtype})
         if (dt != SA2_F32 && dt != SA2_BF16) return SA2_ERR_UNSUPPORTED;
     const int64_t channels = (int64_t)a->d * (a->hq + 4LL * a->hk);
     if (channels > 1 << 20 || a->x_stride < channels) return SA2_ERR_INVALID;
     P = sa2::headnorm::Params{};
     grads = GainGrads{};
-    for (int v = 0; v < 5; ++v) {
+    for (int v = 0; v < (whole_row ? 1 : 5); ++v) {
         if (!a->gain[v] || !aligned16(a->gain[v])) return SA2_ERR_INVALID;
         P.gains.p[v] = a->gain[v];
         grads.p[v] = a->dgain[v];
@@ -406,9 +408,9 @@ int qkvnorm_dispatch(const sa2_qkvnorm_args *a, bool backward) {
     sa2::headnorm::Params P;
     GainGrads grads;
     if (int e = qkvnorm_fill(a, backward, P, grads)) return e;
-    if (!a->rstd || a->y_stride < P.channels) return SA2_ERR_INVALID;
+    if (a->y_stride < P.channels) return SA2_ERR_INVALID;
     if (backward) {
-        if (!a->dy || a->dy_stride < P.channels) return SA2_ERR_INVALID;
+        if (!a->rstd || !a->dy || a->dy_stride < P.channels) return SA2_ERR_INVALID;
         if (!a->partial || a->partial_bytes < sa2_headnorm_partial_bytes(a->rows, P.channels)) return SA2_ERR_WORKSPACE;
     }
     return headnorm_types(P, a->d, a->x_dtype, a->y_dtype, backward, nullptr, grads, reinterpret_cast<cudaStream_t>(a->stream));
@@ -455,7 +457,7 @@ int sa2_qkv_append(const sa2_qkvnorm_args *a, const sa2_append_set *sets, int32_
     sa2::headnorm::AppendParams A{};
     GainGrads grads;
     if (int e = qkvnorm_fill(a, false, A.norm, grads)) return e;
-    if (!sets || b <= 0 || n <= 0 || a->rows != (int64_t)b * n || a->x_dtype != a->y_dtype || !aligned16(a->y)) return SA2_ERR_INVALID;
+    if (!sets || a->hk == 0 || b <= 0 || n <= 0 || a->rows != (int64_t)b * n || a->x_dtype != a->y_dtype || !aligned16(a->y)) return SA2_ERR_INVALID;
     const int piece = a->x_dtype == SA2_BF16 ? 8 : 4;
     const int64_t segs = (A.norm.channels + 255) / 256, items = a->rows * segs;
     if (items > 1 << 28) return SA2_ERR_UNSUPPORTED;

@@ -136,9 +136,11 @@ struct Attn : torch::autograd::Function<Attn> {
         ctx->saved_data["scale"] = scale;
         ctx->saved_data["kernel"] = kernel;
         ctx->mark_non_differentiable({lse});
+        ctx->set_materialize_grads(false);      // no zeros for the gradient of lse
         return {out, lse};
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        if (!grads[0].defined()) return variable_list(9);
         const auto s = ctx->get_saved_variables();
         const c10::cuda::CUDAGuard guard(s[0].device());
         const Cfg c{ctx->saved_data["w1"].toInt(), ctx->saved_data["w2"].toInt(), ctx->saved_data["kernel"].toInt(), ctx->saved_data["scale"].toDouble()};
@@ -301,37 +303,90 @@ pybind11::object qkv_attn(const Tensor &proj, const std::vector<Tensor> &gain, i
     return pybind11::cast(QkvAttn::apply(proj, gain[0], gain[1], gain[2], gain[3], gain[4], hq, hk, d, eps, dt, w1, w2, kernel));
 }
 
-// Generation: (out [b][n][hq][d], [k, k', v, v'] with the new rows, cut to what later rows can see), or None.
-// cache: [k, k', v, v'] of the rows before; no gradients.
-pybind11::object qkv_attn_cached(const Tensor &proj, const std::vector<Tensor> &gain, const std::vector<Tensor> &cache, int64_t hq, int64_t hk,
-                                 int64_t d, double eps, int64_t w1, int64_t w2, int64_t kernel) {
-    const Heads h{hq, hk, d};
-    if (!projection_ok(proj, gain, h, proj.scalar_type()) || cache.size() != 4) return pybind11::none();
-    const int64_t b = proj.size(0), n = proj.size(1), piece = dtype_of(proj) == SA2_BF16 ? 8 : 4;
+bool cache_ok(const std::vector<Tensor> &cache, const Heads &h, int64_t b, at::ScalarType dt) {
+    if (cache.size() != 4) return false;
+    const int64_t piece = dt == at::kBFloat16 ? 8 : 4;
     for (const Tensor &t : cache)
-        if (!t.is_cuda() || t.dim() != 4 || t.scalar_type() != proj.scalar_type() || t.size(0) != b || t.size(2) != hk || t.size(3) != d || t.stride(3) != 1 ||
-            t.stride(0) % piece || t.stride(1) % piece || t.stride(2) % piece || !aligned(t)) return pybind11::none();
-    if (cache[0].size(1) != cache[2].size(1) || cache[1].size(1) != cache[3].size(1)) return pybind11::none();
-    const c10::cuda::CUDAGuard guard(proj.device());
-    const at::AutoDispatchBelowADInplaceOrView below;
+        if (!t.is_cuda() || t.dim() != 4 || t.scalar_type() != dt || t.size(0) != b || t.size(2) != h.hk || t.size(3) != h.d || t.stride(3) != 1 ||
+            t.stride(0) % piece || t.stride(1) % piece || t.stride(2) % piece || !aligned(t)) return false;
+    return cache[0].size(1) == cache[2].size(1) && cache[1].size(1) == cache[3].size(1);
+}
+
+// out [b][n][hq][d], and set = [k, k', v, v'] with the new rows behind the cached ones, cut to what later rows can see
+void attend_cached(const Tensor &proj, const std::vector<Tensor> &gain, const std::vector<Tensor> &cache, const Heads &h, double eps, int64_t w1,
+                   int64_t w2, int64_t kernel, Tensor &out, Tensor (&set)[4]) {
+    const int64_t b = proj.size(0), n = proj.size(1);
     const Tensor g5[5] = {gain[0], gain[1], gain[2], gain[3], gain[4]};
-    Tensor q = at::empty({b, n, hq, d}, proj.options()), set[4];
+    Tensor q = at::empty({b, n, h.hq, h.d}, proj.options()), lse;
     sa2_append_set as[4];
     for (int s = 0; s < 4; ++s) {
         const int64_t keep = cache[s].size(1);
-        set[s] = at::empty({b, keep + n, hk, d}, proj.options());
+        set[s] = at::empty({b, keep + n, h.hk, h.d}, proj.options());
         as[s] = sa2_append_set{cache[s].data_ptr(), strides(cache[s]), set[s].data_ptr(), (int32_t)keep};
     }
     sa2_qkvnorm_args a{};
     fill_norm(a, proj, g5, h, eps);
     a.y = q.data_ptr(); a.y_dtype = dtype_of(q);
     check(L.append(&a, as, (int32_t)b, (int32_t)n), "sa2_qkv_append");
-    Tensor out, lse;
-    run_forward(q, set[0], set[1], set[2], set[3], Cfg{w1, w2, kernel, 1. / std::sqrt((double)d)}, out, lse);
+    run_forward(q, set[0], set[1], set[2], set[3], Cfg{w1, w2, kernel, 1. / std::sqrt((double)h.d)}, out, lse);
     for (int s = 0; s < 4; ++s) {
         const int64_t rows = set[s].size(1), keep = std::min(rows, (s & 1 ? w2 : w1) - 1);
         if (keep < rows) set[s] = set[s].narrow(1, rows - keep, keep);
     }
+}
+
+// Generation: (out [b][n][hq][d], [k, k', v, v']), or None.  cache: [k, k', v, v'] of the rows before; no gradients.
+pybind11::object qkv_attn_cached(const Tensor &proj, const std::vector<Tensor> &gain, const std::vector<Tensor> &cache, int64_t hq, int64_t hk,
+                                 int64_t d, double eps, int64_t w1, int64_t w2, int64_t kernel) {
+    const Heads h{hq, hk, d};
+    if (!projection_ok(proj, gain, h, proj.scalar_type()) || !cache_ok(cache, h, proj.size(0), proj.scalar_type())) return pybind11::none();
+    const c10::cuda::CUDAGuard guard(proj.device());
+    const at::AutoDispatchBelowADInplaceOrView below;
+    Tensor out, set[4];
+    attend_cached(proj, gain, cache, h, eps, w1, w2, kernel, out, set);
+    return pybind11::make_tuple(out, set[0], set[1], set[2], set[3]);
+}
+
+bool row_norm_ok(const std::optional<Tensor> &w, const Tensor &x) {
+    return !w || (w->dim() == 1 && w->numel() == x.size(2) && w->is_cuda() && dtype_of(*w) >= 0 && w->stride(0) == 1 && aligned(*w));
+}
+// RMSNorm over the last dimension, the gain read in its own type; the row scale is not kept.  Widths that the kernel
+// does not take go where headnorm.py's RMSNorm sends them.
+Tensor row_norm(const Tensor &x, const Tensor &w, double eps) {
+    const int64_t d = w.numel();
+    if (d != 32 && d != 64 && d != 128 && d != 256 && d != 512) return at::rms_norm(x, {d}, w, eps);
+    const Tensor x2 = x.is_contiguous() ? x : x.contiguous();
+    Tensor y = at::empty(x2.sizes(), x2.options());
+    sa2_qkvnorm_args a{};
+    a.x = x2.data_ptr(); a.y = y.data_ptr(); a.gain[0] = w.data_ptr();
+    a.rows = x2.numel() / d; a.x_stride = a.y_stride = d; a.hq = 1; a.hk = 0; a.d = (int32_t)d;
+    a.x_dtype = a.y_dtype = dtype_of(x2); a.gain_dtype = dtype_of(w); a.eps = (float)eps;
+    a.stream = c10::cuda::getCurrentCUDAStream(x2.get_device()).stream();
+    check(L.qkv_fwd(&a), "sa2_qkvnorm_fwd");
+    return y;
+}
+
+// A whole generation step: (out [b][n][dim], [k, k', v, v']), or None.  norms: gain and eps of the prenorm and of
+// the postnorm, where there are any.  From Python, the module calls and autograd nodes around its five kernels
+// cost the host twice what the kernels of a small batch take.
+pybind11::object step(const Tensor &x, const std::optional<Tensor> &pre, double pre_eps, const Tensor &w_qkv, const std::vector<Tensor> &gain,
+                      const std::vector<Tensor> &cache, int64_t hq, int64_t hk, int64_t d, double eps, int64_t w1, int64_t w2, int64_t kernel,
+                      const Tensor &w_out, const std::optional<Tensor> &post, double post_eps) {
+    const Heads h{hq, hk, d};
+    if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || dtype_of(x) < 0 || !row_norm_ok(pre, x)) return pybind11::none();
+    for (const Tensor *w : {&w_qkv, &w_out})
+        if (!w->is_cuda() || w->dim() != 2 || w->scalar_type() != x.scalar_type()) return pybind11::none();
+    if (w_qkv.size(1) != x.size(2) || w_qkv.size(0) != h.channels() || w_out.size(1) != hq * d || w_out.size(0) != x.size(2) || !row_norm_ok(post, x))
+        return pybind11::none();
+    if (!cache_ok(cache, h, x.size(0), x.scalar_type())) return pybind11::none();
+    const c10::cuda::CUDAGuard guard(x.device());
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor proj = at::linear(pre ? row_norm(x, *pre, pre_eps) : x, w_qkv);
+    if (!projection_ok(proj, gain, h, x.scalar_type())) return pybind11::none();
+    Tensor out, set[4];
+    attend_cached(proj, gain, cache, h, eps, w1, w2, kernel, out, set);
+    out = at::linear(out.view({x.size(0), x.size(1), hq * d}), w_out);
+    if (post) out = row_norm(out, *post, post_eps);
     return pybind11::make_tuple(out, set[0], set[1], set[2], set[3]);
 }
 
@@ -343,4 +398,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("headnorm", &headnorm);
     m.def("qkv_attn", &qkv_attn);
     m.def("qkv_attn_cached", &qkv_attn_cached);
+    m.def("step", &step);
 }

@@ -17,6 +17,7 @@ from typing import Callable
 
 import torch
 from torch.nn import Identity, Linear, Module, ModuleList, RMSNorm
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _lib
 from .attention import divisible_by, exists, sliding_two_simplicial_attn
@@ -167,7 +168,7 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
         self.w1, self.w2 = w1, w2
 
     def _fused_call(self, proj):
-        """Arguments of the native calls that take the packed projection as a whole - norm and attention forward and
+        """(``proj``: the projection, or tokens of its device and dtype.)  Arguments of the native calls that take the packed projection as a whole - norm and attention forward and
         backward without splitting or concatenating it - or None where the general path is needed."""
         at = self.attend
         if not (self.fused_head_norm and self.qk_rmsnorm and proj.is_cuda and isinstance(at, partial)
@@ -195,6 +196,24 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
         gains, heads, dtype, windows = call
         return proj, _lib.ext().qkv_attn(proj, gains, *heads, dtype, *windows)
 
+    def _step(self, tokens, cache):
+        """A generation step as one native call, or None where a submodule is not the plain one this class made
+        (another type, a hook, a bias) or autocast is on: then the modules are called one by one."""
+        pre, post, qkv, comb = self.prenorm, self.postnorm, self.to_qkv, self.combine_heads
+        norms = (RowRMSNorm, Identity)
+        if type(pre) not in norms or type(post) not in norms or type(qkv) is not Linear or type(comb) is not Linear \
+                or qkv.bias is not None or comb.bias is not None or torch.is_autocast_enabled() or _has_any_global_hook():
+            return None
+        for m in (pre, post, qkv, comb):
+            if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+                return None
+        call = self._fused_call(tokens)
+        if call is None or call[3][:2] != (self.w1, self.w2):
+            return None
+        gains, heads, dtype, windows = call
+        args = [(None, 0.) if type(m) is Identity else (m.weight, m.eps if m.eps is not None else torch.finfo(dtype).eps) for m in (pre, post)]
+        return _lib.ext().step(tokens, *args[0], qkv.weight, gains, [*cache[0], *cache[1]], *heads, *windows, comb.weight, *args[1])
+
     def forward(self, tokens, cache=None, return_cache=False):
         """``cache`` (from an earlier call with ``return_cache=True``) holds the last ``w1 - 1`` rows of the
         first key/value set and the last ``w2 - 1`` rows of the second: all a later token can still see.
@@ -207,8 +226,13 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
                 return self._merge(out)
             queries, keys, values = self._split_heads(proj)
             return self._merge(self.attend(queries, keys, values))
+        generating = cache is not None and return_cache and not torch.is_grad_enabled()
+        if generating:
+            res = self._step(tokens, cache)
+            if res is not None:
+                return res[0], ((res[1], res[2]), (res[3], res[4]))
         proj = self.to_qkv(self.prenorm(tokens))
-        if cache is not None and return_cache and not torch.is_grad_enabled():
+        if generating:
             call = self._fused_call(proj)
             if call is not None and call[2] == proj.dtype and call[3][:2] == (self.w1, self.w2):
                 gains, heads, _, windows = call

@@ -73,6 +73,29 @@ def test_generation_equals_the_general_path(b, hq, hk, d, dtype, prompt):
                     assert a.shape == c.shape and (a - c).float().norm() <= 1e-2 * c.float().norm()
 
 
+@pytest.mark.parametrize("dim,pre,post,hook", [
+    (512, True, True, False),                  # the widest row of the norm kernel
+    (96, True, False, False),                  # a width it does not take
+    (64, False, False, False),
+    (64, True, False, True),                   # a hooked submodule has to be called
+])
+def test_generation_step_of_plain_and_hooked_modules(dim, pre, post, hook):
+    torch.manual_seed(0)
+    m = SlidingWindowTwoSimplicialMHA(dim=dim, dim_head=64, heads=4, key_value_heads=2, prenorm=pre, postnorm=post, w1=20, w2=4)
+    m = m.to("cuda", torch.bfloat16)
+    calls = []
+    if hook:
+        m.to_qkv.register_forward_hook(lambda *a: calls.append(1))
+    x = torch.randn(2, 30, dim, device="cuda").to(torch.bfloat16)
+    with torch.no_grad():
+        want = m(x)
+        _, cache = m(x[:, :25], return_cache=True)
+        calls.clear()
+        got, _ = m(x[:, 25:], cache=cache, return_cache=True)
+    assert bool(calls) == hook
+    assert (got - want[:, 25:]).float().norm() <= 1e-2 * want[:, 25:].float().norm()
+
+
 def test_other_attend_callables_still_run():
     m = _module(2, 2, 64, 16, 4, torch.float32)
     x = torch.randn(1, 30, 64, device="cuda")
