@@ -166,7 +166,7 @@ inline int bwd_q_launch(const BqParams &Q, const KernelParams &kp, const CUtenso
             !tmap::make_rows_map(&ringV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, 64))
             return SA2_ERR_CUDA;
     }
-    bwd_q_kernel<D><<<dim3(Q.nqt * Q.nsplit * BqCfg<D>::CH, kp.hq, kp.b), BQ_THREADS, smem, st>>>(ringK, ringV, Q);
+    bwd_q_kernel<D><<<dim3(Q.nqt * Q.nsplit * BqCfg<D>::CH, kp.hq, kp.b), BqCfg<D>::THREADS, smem, st>>>(ringK, ringV, Q);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 

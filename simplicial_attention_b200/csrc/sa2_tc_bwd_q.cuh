@@ -49,14 +49,18 @@
 namespace sa2 {
 namespace tc {
 
-constexpr int BQ_THREADS = 512;
-// Register hand-over between warpgroups.  Four warps per scheduler partition start with 128 registers a
-// thread; a group can only grow by what another has released, or its setmaxnreg never returns, so the
-// four budgets must add up to 4 * 128.
-constexpr int BQ_REGS_LAUNCH = 128, BQ_REGS_ISSUE = 40, BQ_REGS_COMPUTE = 120;
-// The fold group (232) holds dQ and, up to head dim 64, the q and dO rows, plus either the operands of the next sweep or
-// a k2 row and chunks of U and W.
+// Register hand-over between warpgroups.  A group can only grow by what another has released, or its setmaxnreg
+// never returns, so the budgets must add up to what the block was launched with.
+//   head dim 128: four groups of 128; the fold group takes 232 (dQ, and the operands of the next sweep or a k2 row
+//                 and chunks of U and W).
+//   up to 64:     five groups of 96 (640 threads): the U fold takes 152 (dQ and the q row, 96 registers, plus a k2
+//                 row or chunks of U), the W fold 112.
 template <int D> struct BqCfg {
+    static constexpr bool TWO_FOLDS = D <= 64;                   // U and W have a fold group each
+    static constexpr int THREADS = TWO_FOLDS ? 640 : 512;
+    static constexpr int REGS_LAUNCH = TWO_FOLDS ? 96 : 128, REGS_ISSUE = 40, REGS_COMPUTE = TWO_FOLDS ? 88 : 120;
+    static constexpr int REGS_FOLD = TWO_FOLDS ? 152 : 232, REGS_FOLD_W = TWO_FOLDS ? 112 : 0;
+    static_assert(REGS_ISSUE + 2 * REGS_COMPUTE + REGS_FOLD + REGS_FOLD_W == THREADS / 128 * REGS_LAUNCH, "register pool must balance");
     static constexpr int CH = D == 128 ? 2 : 1;                  // channel halves = CTAs per (query tile, split)
     static constexpr int CC = D < 64 ? D : 64;                   // channels this CTA produces
     static constexpr int KSTEPS = D / 16;                        // K = 16 steps of S and dP
@@ -71,8 +75,6 @@ template <int D> struct BqCfg {
     static constexpr int UWBUF = D <= 64 ? 1 : 2;                // U / W accumulator pairs in TMEM
     static constexpr uint32_t UW0 = NBUF * 128;                  // first TMEM column of U / W
 };
-constexpr int BQ_REGS_FOLD = 232;
-static_assert(BQ_REGS_ISSUE + 2 * BQ_REGS_COMPUTE + BQ_REGS_FOLD == 4 * BQ_REGS_LAUNCH, "register pool must balance");
 constexpr int BQ_MAX_TILES = 3;          // K1/V1 tiles of one split (head dim 64)
 // Shared accumulators of dK2 / dV2: in sweep e thread r adds to slab row r + epc - 1 - e (epc offsets per CTA), so 128 consecutive rows
 // are live at a time.
@@ -100,19 +102,21 @@ template <int D> struct BqAcc {
     }
 };
 
+// With a fold group each for U and W (head dims 32 and 64), entry 0 of a pair belongs to A_e, S, U and entry 1 to B_e,
+// dP, W, except S_FULL ... G_DONE; at head dim 128 A and B share entry 0, and U and W share the entry of their parity.
 enum BqBar {
     BQ_KV_FULL = 0,
-    BQ_AB_FULL = 1,
-    BQ_AB_EMPTY = 2,
-    BQ_S_FULL = 3,       // [3] per buffer
-    BQ_P_FULL = 6,       // [3]
-    BQ_G_DONE = 9,       // [3] the U / W products of the buffer's unit have completed
-    BQ_W_FULL = 12,      // [2] per U / W accumulator pair
-    BQ_W_EMPTY = 14,     // [2] the fold group holds U / W of the sweep in registers
-    BQ_KV_SLOT = 16,     // [3] head dim 128: the K1/V1 unit of the ring slot has landed
-    BQ_KV_FREE = 19,     // [3] head dim 128: the U / W products that read the slot have completed
-    BQ_FOLD_SYNC = 22,   // every fold thread has added its sweep into the shared accumulators
-    BQ_BAR_COUNT = 23
+    BQ_AB_FULL = 1,      // [2]
+    BQ_AB_EMPTY = 3,     // [2]
+    BQ_S_FULL = 5,       // [3] per buffer
+    BQ_P_FULL = 8,       // [3]
+    BQ_G_DONE = 11,      // [3] the U / W products of the buffer's unit have completed
+    BQ_W_FULL = 14,      // [2]
+    BQ_W_EMPTY = 16,     // [2] the fold group holds the accumulator of the sweep in registers
+    BQ_KV_SLOT = 18,     // [3] head dim 128: the K1/V1 unit of the ring slot has landed
+    BQ_KV_FREE = 21,     // [3] head dim 128: the U / W products that read the slot have completed
+    BQ_FOLD_SYNC = 24,   // [2] every fold thread has added its sweep into the shared accumulators
+    BQ_BAR_COUNT = 26
 };
 
 enum { ERR_BQ_PRODUCER = 256, ERR_BQ_MMA = 512, ERR_BQ_COMPUTE = 1024, ERR_BQ_BUILDER = 2048 };
@@ -199,10 +203,11 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
     if constexpr (D <= 64) {
         if (!mbar_wait_warp(&bars[BQ_KV_FULL], 0, abort_flag)) return ERR_BQ_MMA;
     }
+    const int ab = C::TWO_FOLDS ? which : 0;
     int u = 0, buf = 0, use = 0;                         // use = u / NBUF: how often the buffer has been used before
     int slot = 0, suse = 0;                              // head dim 128: ring slot u % NSLOT and u / NSLOT
     for (int e = 0; e < g.nsweeps; ++e) {
-        if (!mbar_wait_warp(&bars[BQ_AB_FULL], e & 1, abort_flag, 0, 1)) return ERR_BQ_MMA;
+        if (!mbar_wait_warp(&bars[BQ_AB_FULL + ab], e & 1, abort_flag, 0, 1)) return ERR_BQ_MMA;
         for (int w = 0; w < g.nunits; ++w, ++u) {
             // the buffer holds P / G of its previous unit until the U / W products of that unit are done
             if (use >= 1 && !mbar_wait_warp(&bars[BQ_G_DONE + buf], (use - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
@@ -231,7 +236,7 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
             if (++buf == C::NBUF) { buf = 0; ++use; }
             if (++slot == C::NSLOT) { slot = 0; ++suse; }
         }
-        if (elect_one()) tc_commit(&bars[BQ_AB_EMPTY]);
+        if (elect_one()) tc_commit(&bars[BQ_AB_EMPTY + ab]);
     }
     return 0;
 }
@@ -297,11 +302,12 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
     int u = 0, buf = 0, use = 0, slot = 0;
     for (int e = 0; e < g.nsweeps; ++e) {
         const int wb = e % C::UWBUF, wuse = e / C::UWBUF;
+        const int wbar = C::TWO_FOLDS ? part : wb;
         const uint32_t tu = tmem + C::UW0 + wb * 128, tw = tu + 64;
         for (int w = 0; w < g.nunits; ++w, ++u) {
             if (!mbar_wait_warp(&bars[BQ_P_FULL + buf], use & 1, abort_flag, 0, 1)) return ERR_BQ_MMA;
             // the fold group must have read the accumulators of the sweep that used them last
-            if (w == 0 && wuse >= 1 && !mbar_wait_warp(&bars[BQ_W_EMPTY + wb], (wuse - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
+            if (w == 0 && wuse >= 1 && !mbar_wait_warp(&bars[BQ_W_EMPTY + wbar], (wuse - 1) & 1, abort_flag, 0, 2)) return ERR_BQ_MMA;
             tc_fence_after();
             const uint64_t off = (uint64_t)((D <= 64 ? w * 8192 : slot * 2 * C::UBLK) >> 4);
             const uint64_t kt = dK + off, vt = dV + off;
@@ -327,12 +333,20 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
             if (++buf == C::NBUF) { buf = 0; ++use; }
             if (++slot == C::NSLOT) slot = 0;
         }
-        if (elect_one()) tc_commit(&bars[BQ_W_FULL + wb]);
+        if (elect_one()) tc_commit(&bars[BQ_W_FULL + wbar]);
     }
     return 0;
 }
 
 // ---------------------------------------------------------------- compute (warps 4-7; head dim 64: and 8-11): P and G
+// P and G = P (dP - D) of two columns, as packed bf16.  The kernel's issue slots count here (728 warp instructions a unit
+// and scheduler before the packed arithmetic of this and of the folds), so two columns share an instruction.
+__device__ __forceinline__ void pg_pair(float p0, float p1, uint32_t dp0, uint32_t dp1, uint64_t ndl2, uint32_t &pp, uint32_t &gg) {
+    float g0, g1;
+    f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(dp0, dp1), ndl2)), g0, g1);
+    pp = pack_bf16(p0, p1);
+    gg = pack_bf16(g0, g1);
+}
 // Head dim 64: group cg forms columns [32 cg, +32) of every unit, which halves the time between S / dP and P / G.
 template <int D>
 __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, int cg, uint32_t tmem, uint64_t *bars, volatile int *abort_flag) {
@@ -351,6 +365,7 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
         lse2 = kp.lse[o] * 1.4426950408889634f;
         dl = kp.delta[o];
     }
+    const uint64_t c2 = f2_pack(c, c), nlse2 = f2_pack(-lse2, -lse2), ndl2 = f2_pack(-dl, -dl);
 #ifdef SA2_PROF
     long long seg_ld = 0, seg_math = 0, seg_st = 0;       // cycles in TMEM loads, arithmetic, TMEM stores and hand-over
 #endif
@@ -389,24 +404,23 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                     if (full) {
 #pragma unroll
                         for (int x = 0; x < 32; x += 2) {
-                            const float p0 = ex2(fmaf(__uint_as_float(sv[x]), c, -lse2));
-                            const float p1 = ex2(fmaf(__uint_as_float(sv[x + 1]), c, -lse2));
-                            pp[x >> 1] = pack_bf16(p0, p1);
-                            gg[x >> 1] = pack_bf16(p0 * (__uint_as_float(dv[x]) - dl), p1 * (__uint_as_float(dv[x + 1]) - dl));
+                            float a0, a1;
+                            f2_unpack(f2_fma(f2_pack(sv[x], sv[x + 1]), c2, nlse2), a0, a1);
+                            pg_pair(ex2(a0), ex2(a1), dv[x], dv[x + 1], ndl2, pp[x >> 1], gg[x >> 1]);
                         }
                     } else {
-                        // valid columns are the integers in (lo, hi]: saturate(half + 1 - |col - mid|) is exactly 1
-                        // inside and 0 outside (FMA pipe instead of compares and selects on the ALU pipe); the
-                        // exponent is clamped so that a masked-out cell cannot give inf * 0
-                        const float mid = 0.5f * (float)(lo + 1 + hi) - (float)(ch * 32), hwp = 0.5f * (float)(hi - lo - 1) + 1.f;
+                        // valid columns are the integers in (lo, hi]: 2048 (half + 1/2 - |col - mid|) is at least 1024
+                        // inside and at most -1024 outside, so the minimum with it leaves the exponents of valid cells
+                        // alone and makes P exactly 0 elsewhere, whatever S is there (FMA pipe instead of compares and
+                        // selects on the ALU pipe; all values are exact)
+                        const float mid = 1024.f * (float)(lo + 1 + hi) - 2048.f * (float)(ch * 32), half = 1024.f * (float)(hi - lo);
 #pragma unroll
                         for (int x = 0; x < 32; x += 2) {
-                            const float v0 = __saturatef(hwp - fabsf((float)x - mid));
-                            const float v1 = __saturatef(hwp - fabsf((float)(x + 1) - mid));
-                            const float p0 = ex2(fminf(fmaf(__uint_as_float(sv[x]), c, -lse2), 100.f)) * v0;
-                            const float p1 = ex2(fminf(fmaf(__uint_as_float(sv[x + 1]), c, -lse2), 100.f)) * v1;
-                            pp[x >> 1] = pack_bf16(p0, p1);
-                            gg[x >> 1] = pack_bf16(p0 * (__uint_as_float(dv[x]) - dl), p1 * (__uint_as_float(dv[x + 1]) - dl));
+                            float a0, a1;
+                            f2_unpack(f2_fma(f2_pack(sv[x], sv[x + 1]), c2, nlse2), a0, a1);
+                            a0 = fminf(a0, half - fabsf(2048.f * x - mid));
+                            a1 = fminf(a1, half - fabsf(2048.f * (x + 1) - mid));
+                            pg_pair(ex2(a0), ex2(a1), dv[x], dv[x + 1], ndl2, pp[x >> 1], gg[x >> 1]);
                         }
                     }
 #ifdef SA2_PROF
@@ -436,8 +450,172 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
     return 0;
 }
 
-// ---------------------------------------------------------------- fold (warps 8-11): U, W -> dQ, dK2, dV2
-__device__ __forceinline__ void bq_fold_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// ---------------------------------------------------------------- fold: U, W -> dQ, dK2, dV2
+// (which: the fold group of U, or of both; 1: that of W)
+__device__ __forceinline__ void bq_fold_sync(int which) { asm volatile("bar.sync %0, 128;" ::"r"(1 + which) : "memory"); }
+
+// dQ of one row (NaN when a wait ran out, so that the failure is visible in the result): with one split per query tile
+// it is final and goes straight to the gradient, otherwise a partial for the reduction kernel
+template <int D, int N>
+__device__ __forceinline__ void bq_store_dq(const BqParams &P, const BqGeom &g, int i, const uint64_t (&dq2)[N], bool bad) {
+    const KernelParams &kp = P.kp;
+    const int h = blockIdx.y, b = blockIdx.z, c0 = g.chh * 64;
+    float dq[2 * N];
+#pragma unroll
+    for (int x = 0; x < N; ++x) f2_unpack(dq2[x], dq[2 * x], dq[2 * x + 1]);
+    if (P.nsplit == 1) {
+        const bool gbf16 = kp.grad_bf16 != 0;
+        const int64_t o = elem_off(kp.dq, b, i, h) + c0;
+#pragma unroll
+        for (int x = 0; x < 2 * N; x += 4) {
+            float v[4];
+#pragma unroll
+            for (int z = 0; z < 4; ++z) v[z] = bad ? CUDART_NAN_F : dq[x + z] * kp.scale;
+            store_vec<4>(kp.dq.p, o + x, gbf16, v);
+        }
+    } else {
+        float *dst = P.part_dq + ((((size_t)g.split * kp.b + b) * kp.n + i) * kp.hq + h) * D + c0;
+#pragma unroll
+        for (int x = 0; x < 2 * N; x += 4)
+            *reinterpret_cast<float4 *>(dst + x) = bad ? make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F)
+                                                       : make_float4(dq[x], dq[x + 1], dq[x + 2], dq[x + 3]);
+    }
+}
+
+__device__ __forceinline__ uint4 mul_bf16x8(const uint4 &x, const uint4 &y) {
+    return make_uint4(mul_bf16x2(x.x, y.x), mul_bf16x2(x.y, y.y), mul_bf16x2(x.z, y.z), mul_bf16x2(x.w, y.w));
+}
+
+// Head dims 32 and 64: WHICH = 0 forms A_e = q_i * k2_{i-e} and folds U_e into dQ_i (registers) and dK2_{i-e};
+// WHICH = 1 forms B_e = dO_i * v2_{i-e} and folds W_e into dV2_{i-e}.  One thread per query row; its q (dO) row stays
+// in its registers.  With one group for both, U / W of the next sweep waited ~1960 of 9400 cycles a sweep for the
+// accumulators to be read and S / dP ~1000 for their operands.
+template <int D, int WHICH>
+__device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc, uint8_t *sOp, uint64_t *bars,
+                                            volatile int *abort_flag) {
+    using C = BqCfg<D>;
+    const KernelParams &kp = P.kp;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = (warp & 3) * 32 + lane;             // query row within the tile = TMEM lane
+    const uint32_t cols = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::UW0 + WHICH * 64;
+    const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
+    const int i = g.i0 + r;
+    const bool row_ok = i < kp.n;
+    constexpr int NC = D / 8;                         // 16-byte chunks of a row
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const TensorRef &tx = WHICH ? kp.dout : kp.q, &ty = WHICH ? kp.v2 : kp.k2;
+    uint4 xr[NC];
+    {
+        const uint4 *px = reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(tx.p) + elem_off(tx, b, row_ok ? i : 0, h));
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) xr[cc] = row_ok ? __ldg(px + cc) : zero;
+    }
+    const __nv_bfloat16 *ybase = reinterpret_cast<const __nv_bfloat16 *>(ty.p) + elem_off(ty, b, 0, hk);
+    uint64_t dq[WHICH ? 2 : D / 2];                   // pairs of channels
+#pragma unroll
+    for (int x = 0; x < (WHICH ? 2 : D / 2); ++x) dq[x] = 0;
+#ifdef SA2_PROF
+    long long seg_build = 0, seg_drain = 0;           // cycles after the waits of a build and of a fold
+#endif
+    auto yrow = [&](int e, bool &ok) {
+        const int kk = i + kp.off2 - g.e0 - e;
+        ok = row_ok && kk >= 0;
+        return reinterpret_cast<const uint4 *>(ybase + (int64_t)(ok ? kk : 0) * ty.sn);
+    };
+    auto build = [&](int e) -> bool {
+        bool ok;
+        const uint4 *py = yrow(e, ok);
+        uint4 y[NC];
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) y[cc] = ok ? __ldg(py + cc) : zero;
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) y[cc] = ok ? mul_bf16x8(xr[cc], y[cc]) : zero;
+        if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY + WHICH], (e - 1) & 1, abort_flag, 3)) return false;
+#ifdef SA2_PROF
+        const long long seg_t0 = clock64();
+#endif
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) *reinterpret_cast<uint4 *>(sOp + sw128_offset(r, cc)) = y[cc];
+        fence_proxy_async_smem();
+        mbar_arrive(&bars[BQ_AB_FULL + WHICH]);
+#ifdef SA2_PROF
+        seg_build += clock64() - seg_t0;
+#endif
+        return true;
+    };
+    auto drain = [&](int e) -> bool {
+        bool ok;
+        const uint4 *py = yrow(e, ok);
+        // the k2 chunks of the next 16 channels are fetched ahead, the first ones before the wait
+        uint4 y0 = zero, y1 = zero;
+        if (WHICH == 0 && ok) { y0 = __ldg(py); y1 = __ldg(py + 1); }
+        if (!warp_wait(&bars[BQ_W_FULL + WHICH], e & 1, abort_flag, 1)) return false;
+        // A row of the shared accumulator is written by thread r in this sweep and by another thread in the
+        // last one: every fold thread must have finished that one first.
+        if (e >= 1 && !warp_wait(&bars[BQ_FOLD_SYNC + WHICH], (e - 1) & 1, abort_flag, 2)) return false;
+        tc_fence_after();
+#ifdef SA2_PROF
+        const long long seg_t0 = clock64();
+#endif
+        float *arow = acc + (size_t)(r + P.epc - 1 - e) * BQ_ACC_STRIDE;
+        constexpr int CH = 16;                        // channels per TMEM read
+#pragma unroll
+        for (int c = 0; c < D; c += CH) {
+            uint32_t t[CH];
+            tmem_ld16(cols + c, t);
+            tmem_wait_ld();
+            if (c + CH == D) {
+                // the rest is in registers: the tensor cores may overwrite the accumulator
+                tc_fence_before();
+                mbar_arrive(&bars[BQ_W_EMPTY + WHICH]);
+            }
+#pragma unroll
+            for (int o = 0; o < CH; o += 16) {
+                const uint4 yy[2] = {y0, y1};
+                if (WHICH == 0 && c + o + 16 < D && ok) { y0 = __ldg(py + (c + o) / 8 + 2); y1 = __ldg(py + (c + o) / 8 + 3); }
+                if (ok) {
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        const int ch = c + o + 8 * p;
+                        const uint32_t xw[4] = {xr[ch / 8].x, xr[ch / 8].y, xr[ch / 8].z, xr[ch / 8].w};
+                        const uint32_t yw[4] = {yy[p].x, yy[p].y, yy[p].z, yy[p].w};
+                        ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(arow + ch);
+                        ulonglong2 a[2] = {dst[0], dst[1]};
+                        unsigned long long *const acc2[4] = {&a[0].x, &a[0].y, &a[1].x, &a[1].y};
+#pragma unroll
+                        for (int z = 0; z < 4; ++z) {
+                            const uint64_t t2 = f2_pack(t[o + 8 * p + 2 * z], t[o + 8 * p + 2 * z + 1]);
+                            if constexpr (WHICH == 0) dq[ch / 2 + z] = f2_fma(t2, f2_from_bf16x2(yw[z]), dq[ch / 2 + z]);
+                            *acc2[z] = f2_fma(t2, f2_from_bf16x2(xw[z]), *acc2[z]);
+                        }
+                        dst[0] = a[0];
+                        dst[1] = a[1];
+                    }
+                }
+            }
+        }
+        mbar_arrive(&bars[BQ_FOLD_SYNC + WHICH]);
+#ifdef SA2_PROF
+        seg_drain += clock64() - seg_t0;
+#endif
+        return true;
+    };
+    const int nv = g.total > 0 ? g.nsweeps : 0;       // a split whose tiles all lie before the sequence start has no work
+    int err = 0;
+    if (nv > 0 && !build(0)) err = ERR_BQ_COMPUTE;
+    for (int e = 0; e < nv && err == 0; ++e) {
+        // the operands of the next sweep first: the tensor cores wait for them, U / W of this sweep arrive later
+        if ((e + 1 < nv && !build(e + 1)) || !drain(e)) err = ERR_BQ_COMPUTE;
+    }
+    SA2_PROF_ADD(4, seg_build);
+    SA2_PROF_ADD(5, seg_drain);
+    if constexpr (WHICH == 0) {
+        if (row_ok) bq_store_dq<D>(P, g, i, dq, err != 0 || *abort_flag != 0);
+    }
+    return err;
+}
+
+// Head dim 128: one group for both.
 
 template <int D>
 __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc_k, float *acc_v, float *slab,
@@ -452,9 +630,9 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     const int i = g.i0 + r;
     const bool row_ok = i < kp.n;
     constexpr int NC = C::CC / 8;                     // 16-byte chunks of the CTA's channels
-    float dq[C::CC];
+    uint64_t dq[C::CC / 2];                           // pairs of channels
 #pragma unroll
-    for (int x = 0; x < C::CC; ++x) dq[x] = 0.f;
+    for (int x = 0; x < C::CC / 2; ++x) dq[x] = 0;
     const __nv_bfloat16 *qrow = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, row_ok ? i : 0, h) + c0;
     const __nv_bfloat16 *dorow = reinterpret_cast<const __nv_bfloat16 *>(kp.dout.p) + elem_off(kp.dout, b, row_ok ? i : 0, h) + c0;
     const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p) + c0;
@@ -463,64 +641,16 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
 #ifdef SA2_PROF
     long long seg_build = 0, seg_drain = 0;           // cycles after the waits of a build and of a fold
 #endif
-    // head dim 64: the q and dO rows serve every A_e / B_e and every fold of this thread
-    uint4 qv[NC], dv[NC];
-    if constexpr (D <= 64) {
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-            qv[cc] = row_ok ? __ldg(reinterpret_cast<const uint4 *>(qrow + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-            dv[cc] = row_ok ? __ldg(reinterpret_cast<const uint4 *>(dorow + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-        }
-    }
-
-    // A_e = q_i * k2_{i-e} and B_e = dO_i * v2_{i-e} of sweep e.  Up to head dim 64 a thread forms its own row, whose q and
-    // dO stay in its registers.  At head dim 128 sixteen lanes take a row, 16 bytes each, so that a load of the warp is
-    // whole rows: with a row per lane every load touched 32 cache lines, ~8000 cycles of L1 a sweep (10.3 -> 9.0 ms on
+    // A_e = q_i * k2_{i-e} and B_e = dO_i * v2_{i-e} of sweep e.  Sixteen lanes take a row, 16 bytes each, so that a load
+    // of the warp is whole rows: with a row per lane every load touched 32 cache lines, ~8000 cycles of L1 a sweep (10.3 -> 9.0 ms on
     // b1 n16384 h16; at head dim 64, without the rows in registers, 1.8 -> 2.2 ms on b4 n4096 h8).  The products are
     // formed before the wait for the stage, only the stores follow it.
     constexpr int LPR = D / 8, RPI = 32 / LPR;            // lanes per row, rows per load
     const int brow = (warp & 3) * 32 + lane / LPR, bcc = lane % LPR;
     const int64_t b_q = elem_off(kp.q, b, 0, h) + bcc * 8, b_do = elem_off(kp.dout, b, 0, h) + bcc * 8;
     const int64_t b_k2 = elem_off(kp.k2, b, 0, hk) + bcc * 8, b_v2 = elem_off(kp.v2, b, 0, hk) + bcc * 8;
-    auto build_row = [&](int e) -> bool {
-        const int kk = i + kp.off2 - g.e0 - e;
-        const bool ok = row_ok && kk >= 0;
-        const __nv_bfloat16 *kp2 = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-        const __nv_bfloat16 *vp2 = v2 + elem_off(kp.v2, b, ok ? kk : 0, hk);
-        uint4 kv[NC], vv[NC];
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-            kv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(kp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-            vv[cc] = ok ? __ldg(reinterpret_cast<const uint4 *>(vp2 + cc * 8)) : make_uint4(0u, 0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-            kv[cc] = make_uint4(mul_bf16x2(qv[cc].x, kv[cc].x), mul_bf16x2(qv[cc].y, kv[cc].y), mul_bf16x2(qv[cc].z, kv[cc].z), mul_bf16x2(qv[cc].w, kv[cc].w));
-            vv[cc] = make_uint4(mul_bf16x2(dv[cc].x, vv[cc].x), mul_bf16x2(dv[cc].y, vv[cc].y), mul_bf16x2(dv[cc].z, vv[cc].z), mul_bf16x2(dv[cc].w, vv[cc].w));
-            if (!ok) { kv[cc] = make_uint4(0u, 0u, 0u, 0u); vv[cc] = make_uint4(0u, 0u, 0u, 0u); }
-        }
-        if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
-#ifdef SA2_PROF
-        const long long seg_t0 = clock64();
-#endif
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-            *reinterpret_cast<uint4 *>(sA + sw128_offset(r, cc)) = kv[cc];
-            *reinterpret_cast<uint4 *>(sB + sw128_offset(r, cc)) = vv[cc];
-        }
-        fence_proxy_async_smem();
-        mbar_arrive(&bars[BQ_AB_FULL]);
-#ifdef SA2_PROF
-        seg_build += clock64() - seg_t0;
-#endif
-        return true;
-    };
     auto build = [&](int e) -> bool {
-        if constexpr (D <= 64) return build_row(e);
         uint4 pa[LPR], pb[LPR];
-        auto mul = [](const uint4 &x, const uint4 &y) {
-            return make_uint4(mul_bf16x2(x.x, y.x), mul_bf16x2(x.y, y.y), mul_bf16x2(x.z, y.z), mul_bf16x2(x.w, y.w));
-        };
         auto fetch = [&](const TensorRef &t, int64_t base, int row) {
             return __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(t.p) + base + (int64_t)row * t.sn));
         };
@@ -536,7 +666,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
                 y[x] = ok ? fetch(kp.k2, b_k2, kk) : make_uint4(0u, 0u, 0u, 0u);
             }
 #pragma unroll
-            for (int x = 0; x < STEP; ++x) pa[x0 + x] = mul(pa[x0 + x], y[x]);
+            for (int x = 0; x < STEP; ++x) pa[x0 + x] = mul_bf16x8(pa[x0 + x], y[x]);
         }
 #pragma unroll
         for (int x0 = 0; x0 < LPR; x0 += STEP) {
@@ -549,7 +679,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
                 y[x] = ok ? fetch(kp.v2, b_v2, kk) : make_uint4(0u, 0u, 0u, 0u);
             }
 #pragma unroll
-            for (int x = 0; x < STEP; ++x) pb[x0 + x] = mul(pb[x0 + x], y[x]);
+            for (int x = 0; x < STEP; ++x) pb[x0 + x] = mul_bf16x8(pb[x0 + x], y[x]);
         }
         if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
 #ifdef SA2_PROF
@@ -588,76 +718,51 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         const long long seg_t0 = clock64();
 #endif
         const int arow = r + P.epc - 1 - e;           // slab row of this thread in this sweep
-        const bool fresh = BqAcc<D>::RING && (e == 0 || r == 0);      // ring: nothing has been added to the row yet
-        if (BqAcc<D>::RING && v >= 1 && warp == 12) {
+        const bool fresh = e == 0 || r == 0;          // nothing has been added to the row yet
+        if (v >= 1 && warp == 12) {
             // the top row of the last sweep is complete: it goes to the slab before thread 0 reuses its place
             const int trow = TQ - 1 + P.epc - e, arr = lane >> 4, c4 = (lane & 15) * 4;
             const float4 t = *reinterpret_cast<const float4 *>((arr ? acc_v : acc_k) + BqAcc<D>::off(trow, c4));
             *reinterpret_cast<float4 *>(slab + ((size_t)arr * (127 + P.epc) + trow) * D + c4) = t;
             __syncwarp();
         }
-        const bool add = ok || BqAcc<D>::RING;       // (a ring row is written even when this thread has nothing to add)
-        // eight channels of one accumulator row += x
-        auto rmw8 = [&](float *acc, int col, const float (&x)[8]) {
-            if constexpr (BqAcc<D>::RING) {
-                // both 16-byte pieces are read before either is written: the swizzled addresses hide from the
-                // compiler that they are distinct, and it would order the second read after the first write
-                float4 *p0 = reinterpret_cast<float4 *>(acc + BqAcc<D>::off(arow, col));
-                float4 *p1 = reinterpret_cast<float4 *>(acc + BqAcc<D>::off(arow, col + 4));
-                float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-                if (!fresh) { t0 = *p0; t1 = *p1; }
-                t0.x += x[0]; t0.y += x[1]; t0.z += x[2]; t0.w += x[3];
-                t1.x += x[4]; t1.y += x[5]; t1.z += x[6]; t1.w += x[7];
-                *p0 = t0;
-                *p1 = t1;
-            } else {
-                float4 *p = reinterpret_cast<float4 *>(acc + (size_t)arow * BQ_ACC_STRIDE + col);
-                float4 t0 = p[0], t1 = p[1];
-                t0.x += x[0]; t0.y += x[1]; t0.z += x[2]; t0.w += x[3];
-                t1.x += x[4]; t1.y += x[5]; t1.z += x[6]; t1.w += x[7];
-                p[0] = t0;
-                p[1] = t1;
+        // eight channels of one accumulator row += t * x (t: fp32 words, x: bf16; nothing where this thread has no row)
+        auto rmw8 = [&](float *acc, int col, const uint32_t *t, const uint4 &x) {
+            // both 16-byte pieces are read before either is written: the swizzled addresses hide from the
+            // compiler that they are distinct, and it would order the second read after the first write
+            ulonglong2 *p0 = reinterpret_cast<ulonglong2 *>(acc + BqAcc<D>::off(arow, col));
+            ulonglong2 *p1 = reinterpret_cast<ulonglong2 *>(acc + BqAcc<D>::off(arow, col + 4));
+            ulonglong2 t0 = {0, 0}, t1 = {0, 0};
+            if (!fresh) { t0 = *p0; t1 = *p1; }
+            if (ok) {
+                t0.x = f2_fma(f2_pack(t[0], t[1]), f2_from_bf16x2(x.x), t0.x);
+                t0.y = f2_fma(f2_pack(t[2], t[3]), f2_from_bf16x2(x.y), t0.y);
+                t1.x = f2_fma(f2_pack(t[4], t[5]), f2_from_bf16x2(x.z), t1.x);
+                t1.y = f2_fma(f2_pack(t[6], t[7]), f2_from_bf16x2(x.w), t1.y);
             }
+            *p0 = t0;
+            *p1 = t1;
         };
         // W first, then U, 32 channels at a time: only 32 registers of U / W are live at once, which keeps this
         // group within its budget without spills (the accumulator pair is released after the last read).
         {
             uint4 dr[NC];
 #pragma unroll
-            for (int c8 = 0; c8 < NC; ++c8) {
-                if constexpr (D <= 64) dr[c8] = dv[c8];
-                else dr[c8] = __ldg(reinterpret_cast<const uint4 *>(dorow + c8 * 8));
-            }
+            for (int c8 = 0; c8 < NC; ++c8) dr[c8] = __ldg(reinterpret_cast<const uint4 *>(dorow + c8 * 8));
 #pragma unroll
             for (int hf = 0; hf < C::CC / 32; ++hf) {
                 uint32_t w[32];
                 tmem_ld32(lane_addr + C::UW0 + wb * 128 + 64 + hf * 32, w);
                 tmem_wait_ld();
-                if (add) {
+                // (a row is written even when this thread has nothing to add)
 #pragma unroll
-                    for (int c4 = 0; c4 < 4; ++c4) {
-                        const int c8 = hf * 4 + c4;
-                        const uint32_t dw[4] = {dr[c8].x, dr[c8].y, dr[c8].z, dr[c8].w};
-                        float xv[8];
-#pragma unroll
-                        for (int z = 0; z < 4; ++z) {
-                            const __nv_bfloat162 d2 = *reinterpret_cast<const __nv_bfloat162 *>(&dw[z]);
-                            const int x = c4 * 8 + z * 2;
-                            xv[z * 2] = ok ? __uint_as_float(w[x]) * __low2float(d2) : 0.f;
-                            xv[z * 2 + 1] = ok ? __uint_as_float(w[x + 1]) * __high2float(d2) : 0.f;
-                        }
-                        rmw8(acc_v, c8 * 8, xv);
-                    }
-                }
+                for (int c4 = 0; c4 < 4; ++c4) rmw8(acc_v, (hf * 4 + c4) * 8, w + c4 * 8, dr[hf * 4 + c4]);
             }
         }
         {
             uint4 qr[NC];
 #pragma unroll
-            for (int c8 = 0; c8 < NC; ++c8) {
-                if constexpr (D <= 64) qr[c8] = qv[c8];
-                else qr[c8] = __ldg(reinterpret_cast<const uint4 *>(qrow + c8 * 8));
-            }
+            for (int c8 = 0; c8 < NC; ++c8) qr[c8] = __ldg(reinterpret_cast<const uint4 *>(qrow + c8 * 8));
 #pragma unroll
             for (int hf = 0; hf < C::CC / 32; ++hf) {
                 uint32_t u[32];
@@ -673,27 +778,14 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
                     tc_fence_before();
                     mbar_arrive(&bars[BQ_W_EMPTY + wb]);
                 }
-                if (add) {
 #pragma unroll
-                    for (int c4 = 0; c4 < 4; ++c4) {
-                        const int c8 = hf * 4 + c4;
-                        const uint4 kraw = k2r[c4];
-                        const uint32_t kw[4] = {kraw.x, kraw.y, kraw.z, kraw.w};
-                        const uint32_t qw[4] = {qr[c8].x, qr[c8].y, qr[c8].z, qr[c8].w};
-                        float xk[8];
+                for (int c4 = 0; c4 < 4; ++c4) {
+                    const int c8 = hf * 4 + c4;
+                    const uint32_t kw[4] = {k2r[c4].x, k2r[c4].y, k2r[c4].z, k2r[c4].w};       // zero without a row
 #pragma unroll
-                        for (int z = 0; z < 4; ++z) {
-                            const __nv_bfloat162 k2v = *reinterpret_cast<const __nv_bfloat162 *>(&kw[z]);
-                            const __nv_bfloat162 q2 = *reinterpret_cast<const __nv_bfloat162 *>(&qw[z]);
-                            const int x = c4 * 8 + z * 2;
-                            const float a0 = __uint_as_float(u[x]), a1 = __uint_as_float(u[x + 1]);
-                            dq[c8 * 8 + z * 2] = fmaf(a0, __low2float(k2v), dq[c8 * 8 + z * 2]);
-                            dq[c8 * 8 + z * 2 + 1] = fmaf(a1, __high2float(k2v), dq[c8 * 8 + z * 2 + 1]);
-                            xk[z * 2] = ok ? a0 * __low2float(q2) : 0.f;
-                            xk[z * 2 + 1] = ok ? a1 * __high2float(q2) : 0.f;
-                        }
-                        rmw8(acc_k, c8 * 8, xk);
-                    }
+                    for (int z = 0; z < 4; ++z)
+                        dq[c8 * 4 + z] = f2_fma(f2_pack(u[c4 * 8 + 2 * z], u[c4 * 8 + 2 * z + 1]), f2_from_bf16x2(kw[z]), dq[c8 * 4 + z]);
+                    rmw8(acc_k, c8 * 8, u + c4 * 8, qr[c8]);
                 }
             }
         }
@@ -715,48 +807,32 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
 
     SA2_PROF_ADD(4, seg_build);
     SA2_PROF_ADD(5, seg_drain);
-    // dQ of this row (NaN when a wait ran out, so that the failure is visible in the result): with one split per
-    // query tile it is final and goes straight to the gradient, otherwise a partial for the reduction kernel
-    if (row_ok) {
-        const bool bad = err != 0 || *abort_flag != 0;
-        if (P.nsplit == 1) {
-            const bool gbf16 = kp.grad_bf16 != 0;
-            const int64_t o = elem_off(kp.dq, b, i, h) + c0;
-#pragma unroll
-            for (int x = 0; x < C::CC; x += 4) {
-                float v[4];
-#pragma unroll
-                for (int z = 0; z < 4; ++z) v[z] = bad ? CUDART_NAN_F : dq[x + z] * kp.scale;
-                store_vec<4>(kp.dq.p, o + x, gbf16, v);
-            }
-        } else {
-            float *dst = P.part_dq + ((((size_t)g.split * kp.b + b) * kp.n + i) * kp.hq + h) * D + c0;
-#pragma unroll
-            for (int x = 0; x < C::CC; x += 4)
-                *reinterpret_cast<float4 *>(dst + x) = bad ? make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F)
-                                                           : make_float4(dq[x], dq[x + 1], dq[x + 2], dq[x + 3]);
-        }
-    }
+    if (row_ok) bq_store_dq<D>(P, g, i, dq, err != 0 || *abort_flag != 0);
     return err;
 }
 
-template <int D>
+// A fold group: WHICH = 0 U (head dim 128: both), 1 W.
+template <int D, int WHICH>
 __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc_k, float *acc_v, uint8_t *sA, uint8_t *sB,
                                        uint64_t *bars, volatile int *abort_flag) {
+    using C = BqCfg<D>;
     const KernelParams &kp = P.kp;
-    const int ft = threadIdx.x - 384;                 // 0..127 among the fold threads
+    const int ft = threadIdx.x & 127;
     const int h = blockIdx.y, b = blockIdx.z;
     const int slab_rows = 127 + P.epc;
     // this CTA's 64 channels of its slab (dK2 rows, then dV2 rows)
     float *slab = P.part_k2 + ((((size_t)b * kp.hq + h) * P.nqt + g.qt) * P.nsplit + g.split) * (size_t)(2 * slab_rows * D) + g.chh * 64;
-    if constexpr (!BqAcc<D>::RING) {
-        // zero the accumulators (acc_v follows acc_k); only this group touches them
-        for (int x = ft; x < 2 * slab_rows * BQ_ACC_STRIDE; x += 128) acc_k[x] = 0.f;
-        bq_fold_sync();
+    int err;
+    if constexpr (C::TWO_FOLDS) {
+        float *acc = WHICH ? acc_v : acc_k;
+        for (int x = ft; x < slab_rows * BQ_ACC_STRIDE; x += 128) acc[x] = 0.f;      // only this group touches it
+        bq_fold_sync(WHICH);
+        err = bq_fold_half<D, WHICH>(P, g, tmem, acc, WHICH ? sB : sA, bars, abort_flag);
+    } else {
+        err = bq_fold_body<D>(P, g, tmem, acc_k, acc_v, slab, sA, sB, bars, abort_flag);
     }
-    const int err = bq_fold_body<D>(P, g, tmem, acc_k, acc_v, slab, sA, sB, bars, abort_flag);
     // The barrier sits outside the body so that a warp that gave up on a wait still reaches it.
-    bq_fold_sync();
+    bq_fold_sync(WHICH);
     // Ring: rows above the live ones went to the slab when they were completed; the live rows follow now, and
     // the rows below them (second keys before the sequence start, when fewer than w2 sweeps ran) are zero.
     const int nv = g.total > 0 ? g.nsweeps : 0;
@@ -764,9 +840,9 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
     const int rows = BqAcc<D>::RING && nv > 0 ? live0 + BQ_ACC_RING : slab_rows;
     const bool held = !BqAcc<D>::RING || nv > 0;
     const bool bad = err != 0 || *abort_flag != 0;     // a CTA in which a wait ran out reports NaN
-    constexpr int C4 = BqCfg<D>::CC / 4;
-    for (int x = ft; x < 2 * rows * C4; x += 128) {
-        const int arr = x / (rows * C4), y = x - arr * rows * C4;
+    constexpr int C4 = C::CC / 4;
+    for (int x = ft; x < (C::TWO_FOLDS ? 1 : 2) * rows * C4; x += 128) {
+        const int arr = C::TWO_FOLDS ? WHICH : x / (rows * C4), y = C::TWO_FOLDS ? x : x - arr * rows * C4;
         const int row = y / C4, c4 = (y % C4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (held && row >= live0) v = *reinterpret_cast<const float4 *>((arr ? acc_v : acc_k) + BqAcc<D>::off(row, c4));
@@ -777,7 +853,7 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
 }
 
 template <int D>
-__global__ void __launch_bounds__(BQ_THREADS, 1)
+__global__ void __launch_bounds__(BqCfg<D>::THREADS, 1)
 bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const BqParams P) {
     using C = BqCfg<D>;
     extern __shared__ uint8_t smem_raw[];
@@ -797,12 +873,12 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     if (threadIdx.x == 0) {
         for (int x = 0; x < BQ_BAR_COUNT; ++x) {
             const bool pfull = x >= BQ_P_FULL && x < BQ_P_FULL + 3;          // every compute thread
-            const bool many = (x >= BQ_W_EMPTY && x < BQ_W_EMPTY + 2) || x == BQ_FOLD_SYNC;
-            // S_FULL and AB_EMPTY collect one commit from each of the two first-product issuers; head dim 64:
-            // G_DONE and W_FULL one from each of the two second-product issuers
-            const bool two = (x >= BQ_S_FULL && x < BQ_S_FULL + 3) || x == BQ_AB_EMPTY ||
-                             (D <= 64 && ((x >= BQ_G_DONE && x < BQ_G_DONE + 3) || (x >= BQ_W_FULL && x < BQ_W_FULL + 2)));
-            mbar_init(&bars[x], x == BQ_AB_FULL ? 128u : pfull ? 256u : many ? 128u : two ? 2u : 1u);
+            const bool fold = (x >= BQ_W_EMPTY && x < BQ_W_EMPTY + 2) || (x >= BQ_FOLD_SYNC && x < BQ_FOLD_SYNC + 2) ||
+                              (x >= BQ_AB_FULL && x < BQ_AB_FULL + 2);      // every thread of a fold group
+            // S_FULL collects a commit from each of the two first-product issuers, G_DONE (two folds) from each of
+            // the two second-product issuers; AB_EMPTY from both issuers where A and B share it
+            const bool two = (x >= BQ_S_FULL && x < BQ_S_FULL + 3) || (C::TWO_FOLDS ? x >= BQ_G_DONE && x < BQ_G_DONE + 3 : x == BQ_AB_EMPTY);
+            mbar_init(&bars[x], pfull ? 256u : fold ? 128u : two ? 2u : 1u);
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -823,7 +899,7 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     sa2::sm100::prof_begin();
 #endif
     if (warp < 4) {
-        reg_dealloc<BQ_REGS_ISSUE>();                 // one instruction for the whole warpgroup
+        reg_dealloc<C::REGS_ISSUE>();                 // one instruction for the whole warpgroup
         if (g.total > 0) {
             if (warp == 0) err = bq_mma_second<D>(P, g, D <= 64 ? 0 : 2, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
             else if (warp == 1) err = bq_mma_first<D>(g, 0, tmem, sK, sA, bars, abort_flag);
@@ -834,11 +910,14 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     } else if (warp < 12) {
         // one call site for both compute groups: they run the same instructions, which the instruction caches
         // of a scheduler then hold once
-        reg_dealloc<BQ_REGS_COMPUTE>();
+        reg_dealloc<C::REGS_COMPUTE>();
         err = bq_compute<D>(P, g, (warp >> 2) - 1, tmem, bars, abort_flag);
-    } else {
-        reg_alloc<BQ_REGS_FOLD>();
-        err = bq_fold<D>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
+    } else if (!C::TWO_FOLDS || warp < 16) {
+        reg_alloc<C::REGS_FOLD>();
+        err = bq_fold<D, 0>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
+    } else if constexpr (C::TWO_FOLDS) {
+        reg_alloc<C::REGS_FOLD_W>();
+        err = bq_fold<D, 1>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
