@@ -311,7 +311,7 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
     const int hk = blockIdx.y, b = blockIdx.z;
     const int j = g.j0 + r;
     const bool jv = j < kp.nk1;
-    const float c = P.c;
+    const uint64_t c2 = f2_pack(P.c, P.c);
 
     // the walk over the steps; a wait that runs out ends it early, the rows are then reported as NaN below
     auto walk = [&]() -> int {
@@ -335,28 +335,31 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
                     tmem_ld32(buf + 64 + ch * 32, dv);
                     tmem_wait_ld();
                     // the accumulators already hold S^T - lse2 / c and dP^T - D
+                    auto pair = [&](int x, float a0, float a1) {
+                        const float p0 = ex2(a0), p1 = ex2(a1);
+                        float g0, g1;
+                        f2_unpack(f2_mul(f2_pack(p0, p1), f2_pack(dv[x], dv[x + 1])), g0, g1);
+                        pk[x >> 1] = pack_bf16(p0, p1);
+                        gk[x >> 1] = pack_bf16(g0, g1);
+                    };
                     if (full) {
 #pragma unroll
                         for (int x = 0; x < 32; x += 2) {
-                            const float p0 = ex2(__uint_as_float(sv[x]) * c);
-                            const float p1 = ex2(__uint_as_float(sv[x + 1]) * c);
-                            pk[x >> 1] = pack_bf16(p0, p1);
-                            gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
+                            float a0, a1;
+                            f2_unpack(f2_mul(f2_pack(sv[x], sv[x + 1]), c2), a0, a1);
+                            pair(x, a0, a1);
                         }
                     } else {
-                        // valid columns are the integers in [lo, hi]: saturate(half + 1 - |col - mid|) is
-                        // exactly 1 inside and 0 outside (FMA pipe instead of compares and selects on the
-                        // ALU pipe); the exponent is clamped so that a masked-out cell cannot give inf * 0
-                        const float mid = 0.5f * (float)(lo + hi), hwp = 0.5f * (float)(hi - lo) + 1.f;
+                        // valid columns are the integers in [lo, hi]: 2048 (half + 1/2 - |col - mid|) is at least 1024
+                        // inside and at most -1024 outside, so the minimum with it leaves the exponents of valid cells
+                        // alone and makes P exactly 0 elsewhere, whatever S is there (FMA pipe instead of compares and
+                        // selects on the ALU pipe; all values are exact)
+                        const float mid = 1024.f * (float)(lo + hi) - 2048.f * (float)(ch * 32), half_w = 1024.f * (float)(hi - lo + 1);
 #pragma unroll
                         for (int x = 0; x < 32; x += 2) {
-                            const int col = ch * 32 + x;
-                            const float v0 = __saturatef(hwp - fabsf((float)col - mid));
-                            const float v1 = __saturatef(hwp - fabsf((float)(col + 1) - mid));
-                            const float p0 = ex2(fminf(__uint_as_float(sv[x]) * c, 100.f)) * v0;
-                            const float p1 = ex2(fminf(__uint_as_float(sv[x + 1]) * c, 100.f)) * v1;
-                            pk[x >> 1] = pack_bf16(p0, p1);
-                            gk[x >> 1] = pack_bf16(p0 * __uint_as_float(dv[x]), p1 * __uint_as_float(dv[x + 1]));
+                            float a0, a1;
+                            f2_unpack(f2_mul(f2_pack(sv[x], sv[x + 1]), c2), a0, a1);
+                            pair(x, fminf(a0, half_w - fabsf(2048.f * x - mid)), fminf(a1, half_w - fabsf(2048.f * (x + 1) - mid)));
                         }
                     }
                     // over columns of S^T / dP^T that this thread has already read
