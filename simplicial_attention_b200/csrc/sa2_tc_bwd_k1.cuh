@@ -31,7 +31,8 @@
 // Bound: the exponent passes of the two groups (512 MUFU cycles per unit and scheduler) next to ~740 cycles of products
 // and ~1700 cycles of shared-memory traffic per step of two units.  With a buffer per group, P^T / G^T in columns of
 // their own and four builder warps a group waited 1100 of 2800 cycles a step for its next S^T: the products of a unit
-// could start only when the group had finished the last (b4 n4096 h8 d64 w512/32: 1.59 -> 1.31 ms).
+// could start only when the group had finished the last (b4 n4096 h8 d64 w512/32: 1.59 -> 1.31 ms, and 1.27 with two
+// columns per instruction in the exponent pass).
 //
 // The offsets may be split over several CTAs per key tile (consecutive ranges): a short sequence has few key tiles, and
 // with grouped-query heads each walks over every head of its group.  The splits write fp32 partials, which the

@@ -1,6 +1,6 @@
 // Backward kernel for dQ, dK2, dV2 on tcgen05 tensor cores (bf16 operands,
-// fp32 accumulation in TMEM, head dim 64 or 128), plus the reduction of its
-// partials.
+// fp32 accumulation in TMEM, head dims 32, 64 and 128), plus the reduction of its
+// partials and of those of dK1 / dV1.
 //
 // A CTA owns 128 query rows i of one (batch, query head) and a subset ("split")
 // of the 128-row K1/V1 tiles of their window.  Because the backward recomputes
@@ -8,8 +8,8 @@
 // independent; each writes fp32 partials to scratch and a small second kernel
 // adds them in a fixed order (splits, then the query heads of a kv group), so
 // results are reproducible.
-// Head dim 64: a split keeps its (at most three) tiles resident in shared memory; a 5-tile window is
-// two splits.
+// Head dims 32 and 64: a split keeps its (at most three) tiles resident in shared memory; a 5-tile window is
+// two splits; the offsets may be split as well (bq_split).
 // Head dim 128: a CTA produces 64 of the 128 output channels (blockIdx.x also carries the channel
 // half): S and dP contract over all 128 channels, U and W use the 64-channel block of K1 / V1 as their
 // B operand, so the fold, its registers and the shared accumulators are those of head dim 64.  Shared
@@ -17,7 +17,7 @@
 // 64-row units stream through a three-slot TMA ring (32 KB per slot), once per sweep, from L2: a slot is
 // refilled when the U / W products of its unit are done, one unit ahead of the S / dP products that need it.
 //
-// Per offset e ("sweep") one warp group forms A_e = q_i * k2_{i-e} and B_e = dO_i * v2_{i-e}; per 64-key
+// Per offset e ("sweep") the fold groups form A_e = q_i * k2_{i-e} and B_e = dO_i * v2_{i-e}; per 64-key
 // unit the tensor cores compute
 //     S = A_e K1^T      dP = B_e V1^T                 (rows i, columns j)
 // the compute warps (one thread per query row and half of the unit's columns) form
@@ -30,19 +30,25 @@
 // Row i-e of the shared accumulators is touched by exactly one thread per
 // sweep, so the read-modify-write needs no atomics (see BqAcc for how the rows are kept).
 //
-// Warps (512 threads, four aligned warpgroups): 0 issuer of U (head dim 64: after loading the tiles; head dim 128:
-// of U and W); 1 TMEM owner and issuer of S; 2 issuer of dP; 3 issuer of W (head dim 128: TMA producer of the
-// ring); 4-7 and 8-11 two compute groups, each forming 32 of the 64 columns of every unit (P, G); 12-15 form A_e
-// and B_e of the next sweep, then fold U, W of the last one into dQ / dK2 / dV2 (head dim 64: the q and dO rows
-// stay in their registers for both).
-// Every thread starts with 128 registers; the issuer warpgroup keeps 40 (setmaxnreg), the compute groups 120
-// each and the fold group takes 232.
+// Warps: 0 issuer of U (up to head dim 64: after loading the tiles; head dim 128: of U and W); 1 TMEM owner and issuer of
+// S; 2 issuer of dP; 3 issuer of W (head dim 128: TMA producer of the ring); 4-7 and 8-11 two compute groups, each
+// forming 32 of the 64 columns of every unit (P, G).  Up to head dim 64 (640 threads) 12-15 form A_e of the next sweep
+// and fold U of the last one into dQ / dK2, 16-19 do the same with B_e, W and dV2; at head dim 128 (512 threads) 12-15 do
+// both (a second fold group and a third S / dP buffer there: 8.45 -> 9.2 ms on b1 n16384 h16 w512/32).
 // TMEM columns: S / dP buffer x -> S/P [128x, 128x+64), dP/G [128x+64, 128x+128); P and G (bf16, 16 columns per
 // 32 keys) overwrite the first half of the S and dP columns of the same keys - columns that the writing compute
 // group has itself read - so a buffer is busy from the issue of S / dP until the U / W products of its unit are
-// done.  Head dim 64 has three such buffers in flight (issue, compute and U / W of different units overlap) and
-// one U / W accumulator pair [384, 512), which the fold group reads into registers before the next sweep's
+// done.  Up to head dim 64 three such buffers are in flight (issue, compute and U / W of different units overlap) and
+// there is one U / W accumulator pair [384, 512), which the fold groups read into registers before the next sweep's
 // first product; head dim 128 has two buffers and U / W per sweep parity at [256 + 128p, +128).
+//
+// Bound, up to head dim 64: shared memory.  A unit's products fetch 512 cycles' worth of operands at 128 B/clk (S and dP:
+// N = 64, so A is read again for every unit), the folds and the operand rows a further ~400, and everything that
+// goes through shared memory - shuffles included - waits behind the tensor cores' fetches.  b4 n4096 h8 w512/32 takes
+// ~1350 cycles a unit: 1.97 -> 1.58 ms at head dim 64, 30 -> 1.27 ms at 32 (the fp32 kernels before).  Measured and not
+// kept: A_e and B_e in TMEM, double-buffered, which leaves two S / dP buffers (1.74 ms); k2 / v2 rows moved from lane to
+// lane by shuffles instead of a row per lane from memory (1.70 ms).  Head dim 128 (two buffers, S and dP formed in
+// both channel halves): 11.7 -> 8.5 ms on b1 n16384 h16; the chain S / dP -> P / G -> U / W of two buffers paces it.
 #pragma once
 #include "sa2_tc_bwd_k1.cuh"
 
@@ -53,13 +59,13 @@ namespace tc {
 // never returns, so the budgets must add up to what the block was launched with.
 //   head dim 128: four groups of 128; the fold group takes 232 (dQ, and the operands of the next sweep or a k2 row
 //                 and chunks of U and W).
-//   up to 64:     five groups of 96 (640 threads): the U fold takes 152 (dQ and the q row, 96 registers, plus a k2
-//                 row or chunks of U), the W fold 112.
+//   up to 64:     five groups of 96 (640 threads): the U fold takes 160 (dQ, q and k2 rows, 128 registers, and a
+//                 chunk of U), the W fold 104.
 template <int D> struct BqCfg {
     static constexpr bool TWO_FOLDS = D <= 64;                   // U and W have a fold group each
     static constexpr int THREADS = TWO_FOLDS ? 640 : 512;
     static constexpr int REGS_LAUNCH = TWO_FOLDS ? 96 : 128, REGS_ISSUE = 40, REGS_COMPUTE = TWO_FOLDS ? 88 : 120;
-    static constexpr int REGS_FOLD = TWO_FOLDS ? 152 : 232, REGS_FOLD_W = TWO_FOLDS ? 112 : 0;
+    static constexpr int REGS_FOLD = TWO_FOLDS ? 160 : 232, REGS_FOLD_W = TWO_FOLDS ? 104 : 0;
     static_assert(REGS_ISSUE + 2 * REGS_COMPUTE + REGS_FOLD + REGS_FOLD_W == THREADS / 128 * REGS_LAUNCH, "register pool must balance");
     static constexpr int CH = D == 128 ? 2 : 1;                  // channel halves = CTAs per (query tile, split)
     static constexpr int CC = D < 64 ? D : 64;                   // channels this CTA produces
@@ -546,9 +552,13 @@ __device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, 
     auto drain = [&](int e) -> bool {
         bool ok;
         const uint4 *py = yrow(e, ok);
-        // the k2 chunks of the next 16 channels are fetched ahead, the first ones before the wait
-        uint4 y0 = zero, y1 = zero;
-        if (WHICH == 0 && ok) { y0 = __ldg(py); y1 = __ldg(py + 1); }
+        // The k2 row is fetched before the wait: shared memory leaves 28 KB of L1, so it often comes from L2 (with the
+        // chunks fetched one step ahead of their use: 1.60 against 1.58 ms on b4 n4096 h8, head dim 64).
+        uint4 yd[WHICH ? 1 : NC];
+        if constexpr (WHICH == 0) {
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc) yd[cc] = ok ? __ldg(py + cc) : zero;
+        }
         if (!warp_wait(&bars[BQ_W_FULL + WHICH], e & 1, abort_flag, 1)) return false;
         // A row of the shared accumulator is written by thread r in this sweep and by another thread in the
         // last one: every fold thread must have finished that one first.
@@ -569,28 +579,23 @@ __device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, 
                 tc_fence_before();
                 mbar_arrive(&bars[BQ_W_EMPTY + WHICH]);
             }
+            if (ok) {
 #pragma unroll
-            for (int o = 0; o < CH; o += 16) {
-                const uint4 yy[2] = {y0, y1};
-                if (WHICH == 0 && c + o + 16 < D && ok) { y0 = __ldg(py + (c + o) / 8 + 2); y1 = __ldg(py + (c + o) / 8 + 3); }
-                if (ok) {
+                for (int p = 0; p < 2; ++p) {
+                    const int ch = c + 8 * p;
+                    const uint4 yy = yd[WHICH ? 0 : ch / 8];
+                    const uint32_t xw[4] = {xr[ch / 8].x, xr[ch / 8].y, xr[ch / 8].z, xr[ch / 8].w}, yw[4] = {yy.x, yy.y, yy.z, yy.w};
+                    ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(arow + ch);
+                    ulonglong2 a[2] = {dst[0], dst[1]};
+                    unsigned long long *const sum[4] = {&a[0].x, &a[0].y, &a[1].x, &a[1].y};
 #pragma unroll
-                    for (int p = 0; p < 2; ++p) {
-                        const int ch = c + o + 8 * p;
-                        const uint32_t xw[4] = {xr[ch / 8].x, xr[ch / 8].y, xr[ch / 8].z, xr[ch / 8].w};
-                        const uint32_t yw[4] = {yy[p].x, yy[p].y, yy[p].z, yy[p].w};
-                        ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(arow + ch);
-                        ulonglong2 a[2] = {dst[0], dst[1]};
-                        unsigned long long *const acc2[4] = {&a[0].x, &a[0].y, &a[1].x, &a[1].y};
-#pragma unroll
-                        for (int z = 0; z < 4; ++z) {
-                            const uint64_t t2 = f2_pack(t[o + 8 * p + 2 * z], t[o + 8 * p + 2 * z + 1]);
-                            if constexpr (WHICH == 0) dq[ch / 2 + z] = f2_fma(t2, f2_from_bf16x2(yw[z]), dq[ch / 2 + z]);
-                            *acc2[z] = f2_fma(t2, f2_from_bf16x2(xw[z]), *acc2[z]);
-                        }
-                        dst[0] = a[0];
-                        dst[1] = a[1];
+                    for (int z = 0; z < 4; ++z) {
+                        const uint64_t t2 = f2_pack(t[8 * p + 2 * z], t[8 * p + 2 * z + 1]);
+                        if constexpr (WHICH == 0) dq[ch / 2 + z] = f2_fma(t2, f2_from_bf16x2(yw[z]), dq[ch / 2 + z]);
+                        *sum[z] = f2_fma(t2, f2_from_bf16x2(xw[z]), *sum[z]);
                     }
+                    dst[0] = a[0];
+                    dst[1] = a[1];
                 }
             }
         }

@@ -3,7 +3,7 @@
 //
 // A tile is 128 (query row, second-key offset) pairs of one (batch, query head): RI query rows times
 // RE = 128 / RI offsets e = i - k, row r = s * RI + (i - i0) holding e = RE * t + s in "sweep" t.  Per sweep
-// the kernel forms A[r,:] = q_i * k2_{i-e} (bf16, written straight to TMEM), multiplies it against the
+// the kernel forms A[r,:] = q_i * k2_{i-e} (bf16, in shared memory), multiplies it against the
 // TMA-staged K1 window of the RI rows (S = A K1^T, 64 keys a unit), turns S into P = exp2(c*S - ref) in
 // registers, writes P to TMEM as bf16 and feeds it as the A operand of W += P V1 (V1 unit as an MN-major B
 // operand).  At the end of a sweep the row owner adds v2_{i-e} * W to its output registers; at the end of
@@ -27,16 +27,18 @@
 //
 // A unit is 64 keys.  TMEM columns of group g, from 256 g: S 2 x 64, P (bf16) 2 x 32, W 64.
 //
-// Bound: not the exponentials (512 MUFU cycles per scheduler and unit) but the chain of a group, P stored ->
-// P V1 -> S of the unit after the next -> its exponentials: without any arithmetic in the softmax groups a unit
-// still takes 950 cycles, with it 1000.  So a softmax warp has one barrier wait and one arrival per unit - the
-// issuing thread of a group alternates P V1 of unit u and S of unit u + 2, whose completion therefore also says
+// Bound: the two softmax groups, busy ~85 % of a unit's ~900 cycles (two warps a scheduler, 512 MUFU cycles a unit) and
+// mostly in phase with each other on the MUFU pipe.  A softmax warp has one barrier wait and one arrival per unit -
+// the issuing thread of a group alternates P V1 of unit u and S of unit u + 2, whose completion therefore also says
 // that the P columns are free - and which 32-column chunks need no mask, or are seen by nobody, is decided from
-// warp-uniform bounds without votes.  (Separate issuing threads for S and P V1, A in TMEM, 128-key units and a
-// second chunk in flight per warp were measured: 1.15 to 1.6 ms where this form takes 1.12.)
-// Measured: b4 n4096 h8 d64 w512/32 1.26 -> 1.12 ms (459 TFLOP/s), b2 n1024 0.178 -> 0.168 ms; what ran on the fp32
-// kernels before: b1 n3001 h8 d64 w1024/16 4.16 -> 0.23 ms, b4 n2048 h8 d32 w512/32 3.9 -> 0.48 ms; one new row
-// of b1 h8 behind a full window 0.19 -> 0.01 ms.
+// warp-uniform bounds without votes.
+// Measured: b4 n4096 h8 d64 w512/32 1.26 -> 0.96 ms (537 TFLOP/s), b2 n1024 0.178 -> 0.141 ms; what ran on the fp32
+// kernels before: b1 n3001 h8 d64 w1024/16 4.16 -> 0.20 ms, b4 n4096 h8 d32 w512/32 7.8 -> 0.89 ms; one new row
+// of b1 h8 behind a full window 0.19 -> 0.017 ms.
+// Measured and not kept, where this form takes 0.96 (or, earlier, 1.12) ms: A in TMEM with one P buffer (1.5 against 1.12),
+// 128-key units (1.4), S and P V1 from separate issuing threads (1.15), S(u + 2) before P V1(u) (1.19), ordering the
+// softmax groups against each other (1.04 against 0.96), A and W double-buffered (0.98), an output group that takes its
+// events as they come (1.01).
 //
 // Reference handling: probabilities are computed against a per-row reference
 // that only moves when it must, so the W accumulator in TMEM normally never

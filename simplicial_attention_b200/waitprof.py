@@ -22,19 +22,19 @@ PROF_LIB = os.path.join(PKG, "libsa2_prof.so")
 
 # what the slots 1..7 of a warp mean, per kernel and warp role (head dim 64 / 128 where they differ)
 SLOTS = {
-    "fwd": "d=64: issuers (warps 0-1) 1 A_e ready, 2 P ready, 3 W read by the output group; output group (4-7) 1 A_e stage "
-           "free, 2 reference ready, 3 W complete; softmax groups (8-15) 1 S ready.  d=128: issuers of S (0-1) 1 A_e ready, "
-           "2 K1 unit landed, 3 P V1 product of the buffer done; issuers of P V1 (2-3) 4 V1 unit landed, 5 P ready, 6 W read; "
-           "output group (4-11) 1 A_e stage free, 2 reference ready, 3 W complete; softmax groups (12-19) 1 S ready, 2 W read; "
-           "producers (20-21) 1 ring slot free",
-    "dk1_dv1": "issuer of dV1 / dK1 (0) 1 P^T/G^T ready; issuers of S^T / dP^T (1 and 14; d=128: 1 and 2) 1 A_e/B_e stage full, "
-               "2 the P^T/G^T pass of the half (d=128: its second products) done; compute groups 1 S^T/dP^T ready, 2 (d=64) second "
-               "products of the half done; builders (last four or eight warps) 1 k2/v2 window landed, 2 stage free",
+    "fwd": "d=64: issuers (warps 0-1) 1 A_e ready, 2 P ready, 3 W read by the output group; producers (2-3) 1 ring slot free; "
+           "output group (4-7) 1 A_e stage free, 2 reference ready, 3 W complete; softmax groups (8-15) 1 S ready.  d=128: issuers "
+           "of S (0-1) 1 A_e ready, 2 K1 unit landed, 3 P V1 product of the buffer done; issuers of P V1 (2-3) 4 V1 unit landed, 5 P "
+           "ready, 6 W read; output group (4-11) 1 A_e stage free, 2 reference ready, 3 W complete; softmax groups (12-19) 1 S "
+           "ready, 2 W read; producers (20-21) 1 ring slot free",
+    "dk1_dv1": "issuer of dV1 / dK1 (0) 1 P^T/G^T ready; issuers of S^T / dP^T (1 and 2) 1 A_e/B_e stage full, 2 the second products "
+               "of the buffer done; compute groups (4-11) 1 S^T/dP^T ready; builders (the last eight warps; d=128: the last four or "
+               "eight) 1 k2/v2 window landed, 2 stage free",
     "dq_dk2_dv2": "issuers of U / W (0, and 3 at d=64) 1 P/G ready, 2 U/W read by the fold group; issuers of S / dP (1, 2) "
                   "1 A_e/B_e ready, 2 buffer free, 3 K1/V1 unit landed (d=128), 4 cycles issuing products, 5 cycles in the commit; "
                   "producer (3 at d=128) 1 ring slot free; compute groups (4-11) 1 S/dP ready, 4 TMEM loads, 5 arithmetic, "
-                  "6 TMEM stores and hand-over; operand / fold group (12-15) 1 U/W complete, 2 the other fold threads, "
-                  "3 A_e/B_e stage free, 4 stores of A_e/B_e (d=64), 5 fold after its waits",
+                  "6 TMEM stores and hand-over; fold groups (12-15; d=64: of U, and 16-19 of W) 1 U/W complete, 2 the other fold "
+                  "threads, 3 A_e/B_e stage free, 4 stores of A_e/B_e, 5 fold after its waits",
 }
 
 
