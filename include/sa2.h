@@ -276,6 +276,13 @@ typedef struct sa2_append_set {
 
 int sa2_qkv_append(const sa2_qkvnorm_args *args, const sa2_append_set sets[4], int32_t b, int32_t n);
 
+/*
+ * Generation: y [rows][outs] = x [rows][k] W^T, W [outs][k], all bf16 and contiguous (16-byte aligned), fp32 sums: the
+ * module's two projections (simplicial_mha.py:93,135) for the few rows of a step.  rows <= 16, k a multiple of 32 and
+ * outs of 16; SA2_ERR_UNSUPPORTED otherwise.
+ */
+int sa2_rows_linear(const void *x, const void *w, void *y, int32_t rows, int32_t k, int32_t outs, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -5,6 +5,7 @@
 #include "sa2_simt.cuh"
 #include "sa2_tc.cuh"
 #include "sa2_headnorm.cuh"
+#include "sa2_rows_linear.cuh"
 #include <nvtx3/nvToolsExt.h>
 
 namespace sa2 {
@@ -473,6 +474,17 @@ int sa2_qkv_append(const sa2_qkvnorm_args *a, const sa2_append_set *sets, int32_
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
     return a->x_dtype == SA2_BF16 ? append_launch<__nv_bfloat16>(A, a->d, st) : append_launch<float>(A, a->d, st);
+}
+
+int sa2_rows_linear(const void *x, const void *w, void *y, int32_t rows, int32_t k, int32_t outs, void *stream) {
+    using namespace sa2::rows_linear;
+    sa2::nvtx::Range range("sa2_rows_linear");
+    if (!x || !w || !y || rows <= 0 || k <= 0 || outs <= 0 || !aligned16(x) || !aligned16(w) || !aligned16(y)) return SA2_ERR_INVALID;
+    if (rows > MAX_ROWS || k % 32 || outs % OUTS) return SA2_ERR_UNSUPPORTED;
+    auto run = rows <= 8 ? kernel<1> : kernel<2>;
+    run<<<outs / OUTS, WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const __nv_bfloat16 *>(x), reinterpret_cast<const __nv_bfloat16 *>(w), reinterpret_cast<__nv_bfloat16 *>(y), rows, k, outs);
+    return launch_status();
 }
 
 }  // extern "C"

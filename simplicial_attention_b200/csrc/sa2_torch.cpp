@@ -29,6 +29,7 @@ struct Lib {
     size_t (*partial_bytes)(int64_t, int32_t) = nullptr;
     int (*qkv_fwd)(const sa2_qkvnorm_args *) = nullptr;
     int (*qkv_bwd)(const sa2_qkvnorm_args *) = nullptr;
+    int (*linear)(const void *, const void *, void *, int32_t, int32_t, int32_t, void *) = nullptr;
     int (*append)(const sa2_qkvnorm_args *, const sa2_append_set *, int32_t, int32_t) = nullptr;
 } L;
 
@@ -36,7 +37,7 @@ void bind(const std::map<std::string, uintptr_t> &f) {
     auto set = [&](auto &slot, const char *name) { slot = reinterpret_cast<std::decay_t<decltype(slot)>>(f.at(name)); };
     set(L.fwd, "sa2_fwd"); set(L.bwd, "sa2_bwd"); set(L.workspace, "sa2_bwd_workspace_bytes");
     set(L.norm_fwd, "sa2_headnorm_fwd"); set(L.norm_bwd, "sa2_headnorm_bwd"); set(L.partial_bytes, "sa2_headnorm_partial_bytes");
-    set(L.qkv_fwd, "sa2_qkvnorm_fwd"); set(L.qkv_bwd, "sa2_qkvnorm_bwd"); set(L.append, "sa2_qkv_append");
+    set(L.qkv_fwd, "sa2_qkvnorm_fwd"); set(L.qkv_bwd, "sa2_qkvnorm_bwd"); set(L.append, "sa2_qkv_append"); set(L.linear, "sa2_rows_linear");
 }
 
 // raises _lib.Sa2Error, also from the autograd engine's threads
@@ -366,6 +367,17 @@ Tensor row_norm(const Tensor &x, const Tensor &w, double eps) {
     return y;
 }
 
+// x W^T over the last dimension: the kernel for few rows where it takes them (bf16, at most 16 rows), else the library
+Tensor step_linear(const Tensor &x, const Tensor &w) {
+    const int64_t rows = x.size(0) * x.size(1), k = w.size(1), outs = w.size(0);
+    if (rows > 16 || k % 32 || outs % 16 || x.scalar_type() != at::kBFloat16 || !x.is_contiguous() || !w.is_contiguous() || !aligned(x) || !aligned(w))
+        return at::linear(x, w);
+    Tensor y = at::empty({x.size(0), x.size(1), outs}, x.options());
+    check(L.linear(x.data_ptr(), w.data_ptr(), y.data_ptr(), (int32_t)rows, (int32_t)k, (int32_t)outs,
+                   c10::cuda::getCurrentCUDAStream(x.get_device()).stream()), "sa2_rows_linear");
+    return y;
+}
+
 // A whole generation step: (out [b][n][dim], [k, k', v, v']), or None.  norms: gain and eps of the prenorm and of
 // the postnorm, where there are any.  From Python, the module calls and autograd nodes around its five kernels
 // cost the host twice what the kernels of a small batch take.
@@ -381,11 +393,11 @@ pybind11::object step(const Tensor &x, const std::optional<Tensor> &pre, double 
     if (!cache_ok(cache, h, x.size(0), x.scalar_type())) return pybind11::none();
     const c10::cuda::CUDAGuard guard(x.device());
     const at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor proj = at::linear(pre ? row_norm(x, *pre, pre_eps) : x, w_qkv);
+    const Tensor proj = step_linear(pre ? row_norm(x, *pre, pre_eps) : x, w_qkv);
     if (!projection_ok(proj, gain, h, x.scalar_type())) return pybind11::none();
     Tensor out, set[4];
     attend_cached(proj, gain, cache, h, eps, w1, w2, kernel, out, set);
-    out = at::linear(out.view({x.size(0), x.size(1), hq * d}), w_out);
+    out = step_linear(out.view({x.size(0), x.size(1), hq * d}), w_out);
     if (post) out = row_norm(out, *post, post_eps);
     return pybind11::make_tuple(out, set[0], set[1], set[2], set[3]);
 }

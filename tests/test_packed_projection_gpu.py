@@ -1,11 +1,12 @@
 """The native calls on the packed projection (norm + attention in one autograd node; norm + cache append in one
 launch) against the general path of the same module, and the vectorised norm kernels at the edges of their warps."""
+import ctypes as C
 from functools import partial
 
 import pytest
 import torch
 
-from simplicial_attention_b200 import SlidingWindowTwoSimplicialMHA, sliding_two_simplicial_attn
+from simplicial_attention_b200 import SlidingWindowTwoSimplicialMHA, _lib, sliding_two_simplicial_attn
 from simplicial_attention_b200.headnorm import head_rmsnorm
 
 pytestmark = pytest.mark.gpu
@@ -94,6 +95,18 @@ def test_generation_step_of_plain_and_hooked_modules(dim, pre, post, hook):
         got, _ = m(x[:, 25:], cache=cache, return_cache=True)
     assert bool(calls) == hook
     assert (got - want[:, 25:]).float().norm() <= 1e-2 * want[:, 25:].float().norm()
+
+
+@pytest.mark.parametrize("rows,k,outs", [(1, 32, 16), (8, 64, 48), (9, 288, 64), (15, 512, 1536), (16, 2080, 128)])
+def test_projection_of_few_rows(rows, k, outs):
+    g = torch.Generator("cuda").manual_seed(rows)
+    x, w = (torch.randn(s, k, device="cuda", generator=g).to(torch.bfloat16) for s in (rows, outs))
+    y = torch.full((rows + 1, outs), 7., device="cuda", dtype=torch.bfloat16)
+    _lib.check(_lib.lib().sa2_rows_linear(*(C.c_void_p(t.data_ptr()) for t in (x, w, y)), rows, k, outs,
+                                          C.c_void_p(torch.cuda.current_stream().cuda_stream)), "sa2_rows_linear")
+    want = x.float() @ w.float().t()
+    assert (y[:rows].float() - want).abs().max() <= 1e-2 * want.abs().max()
+    assert (y[rows] == 7).all()
 
 
 def test_other_attend_callables_still_run():
