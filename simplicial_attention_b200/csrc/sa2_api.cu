@@ -41,6 +41,15 @@ int check_shape(const sa2_shape &s) {
     return SA2_OK;
 }
 
+// The shape as the kernels take it.  A row at key position i + off sees at most i + off + 1 <= n + off keys, so a longer
+// window selects the same pairs; every rule and loop below may then add tile sizes to w1 and w2 without overflow.
+sa2_shape clamped(sa2_shape s) {
+    const int64_t nk1 = (int64_t)s.n + s.off1, nk2 = (int64_t)s.n + s.off2;
+    if (s.w1 > nk1) s.w1 = (int32_t)nk1;
+    if (s.w2 > nk2) s.w2 = (int32_t)nk2;
+    return s;
+}
+
 void fill_common(KernelParams &p, const sa2_shape &s) {
     p.b = s.b; p.n = s.n; p.hq = s.hq; p.hk = s.hk; p.g = s.hq / s.hk;
     p.w1 = s.w1; p.w2 = s.w2; p.off1 = s.off1; p.off2 = s.off2;
@@ -81,8 +90,8 @@ int check_bwd_args(const sa2_bwd_args *a) {
     return SA2_OK;
 }
 
-void fill_bwd_params(KernelParams &p, const sa2_bwd_args *a, float *rowsum) {
-    fill_common(p, a->shape);
+void fill_bwd_params(KernelParams &p, const sa2_bwd_args *a, const sa2_shape &s, float *rowsum) {
+    fill_common(p, s);
     p.grad_bf16 = (a->grad_dtype == SA2_BF16);
     p.q = ref(a->q, a->sq); p.k1 = ref(a->k1, a->sk1); p.k2 = ref(a->k2, a->sk2);
     p.v1 = ref(a->v1, a->sv1); p.v2 = ref(a->v2, a->sv2);
@@ -164,19 +173,21 @@ const char *sa2_strerror(int status) {
     }
 }
 
-int sa2_kernel_launches(const sa2_shape *s, int backward) {
-    if (!s || check_shape(*s) != SA2_OK) return -1;
-    const bool tc_ok = backward ? sa2::tc::bwd_supported(*s) : sa2::tc::fwd_supported(*s);
-    if (s->kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
-    if (tc_ok && s->kernel != SA2_KERNEL_SIMT) return sa2::tc::launches(*s, backward != 0);
+int sa2_kernel_launches(const sa2_shape *shape, int backward) {
+    if (!shape || check_shape(*shape) != SA2_OK) return -1;
+    const sa2_shape s = clamped(*shape);
+    const bool tc_ok = backward ? sa2::tc::bwd_supported(s) : sa2::tc::fwd_supported(s);
+    if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT) return sa2::tc::launches(s, backward != 0);
     return backward ? 2 : 1;   // SIMT: row sums + all gradients
 }
 
-size_t sa2_bwd_workspace_bytes(const sa2_shape *s) {
-    if (!s || check_shape(*s) != SA2_OK) return 0;
-    size_t delta = (size_t)s->b * s->hq * s->n * sizeof(float);
+size_t sa2_bwd_workspace_bytes(const sa2_shape *shape) {
+    if (!shape || check_shape(*shape) != SA2_OK) return 0;
+    const sa2_shape s = clamped(*shape);
+    size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
     delta = (delta + 255) & ~(size_t)255;
-    return delta + sa2::tc::bwd_extra_workspace_bytes(*s);
+    return delta + sa2::tc::bwd_extra_workspace_bytes(s);
 }
 
 int sa2_fwd(const sa2_fwd_args *a) {
@@ -189,18 +200,19 @@ int sa2_fwd(const sa2_fwd_args *a) {
     const sa2_strides *ss[] = {&a->sq, &a->sk1, &a->sk2, &a->sv1, &a->sv2, &a->sout};
     for (const sa2_strides *s : ss) if (!strides_ok(*s)) return SA2_ERR_INVALID;
 
+    const sa2_shape s = clamped(a->shape);
     KernelParams p{};
-    fill_common(p, a->shape);
+    fill_common(p, s);
     p.q = ref(a->q, a->sq); p.k1 = ref(a->k1, a->sk1); p.k2 = ref(a->k2, a->sk2);
     p.v1 = ref(a->v1, a->sv1); p.v2 = ref(a->v2, a->sv2); p.out = ref(a->out, a->sout);
     p.lse = a->lse;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
 
-    const bool tc_ok = sa2::tc::fwd_supported(a->shape) && sa2::tc::fwd_addressable(p);
-    if (a->shape.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
-    if (tc_ok && a->shape.kernel != SA2_KERNEL_SIMT) return sa2::tc::fwd(p, a->shape, st);
+    const bool tc_ok = sa2::tc::fwd_supported(s) && sa2::tc::fwd_addressable(p);
+    if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT) return sa2::tc::fwd(p, s, st);
 
-    switch (a->shape.d) {
+    switch (s.d) {
         case 32: return simt_fwd<32>(p, st);
         case 64: return simt_fwd<64>(p, st);
         default: return simt_fwd<128>(p, st);
@@ -215,19 +227,20 @@ int sa2_bwd(const sa2_bwd_args *a) {
     if (!a->workspace || a->workspace_bytes < need || (reinterpret_cast<uintptr_t>(a->workspace) & 255u))
         return SA2_ERR_WORKSPACE;
 
+    const sa2_shape s = clamped(a->shape);
     KernelParams p{};
-    fill_bwd_params(p, a, reinterpret_cast<float *>(a->workspace));
+    fill_bwd_params(p, a, s, reinterpret_cast<float *>(a->workspace));
     cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
 
-    const bool tc_ok = sa2::tc::bwd_supported(a->shape) && sa2::tc::bwd_addressable(p);
-    if (a->shape.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
-    if (tc_ok && a->shape.kernel != SA2_KERNEL_SIMT) {
-        size_t delta = (size_t)a->shape.b * a->shape.hq * a->shape.n * sizeof(float);
+    const bool tc_ok = sa2::tc::bwd_supported(s) && sa2::tc::bwd_addressable(p);
+    if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT) {
+        size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
         delta = (delta + 255) & ~(size_t)255;
-        return sa2::tc::bwd(p, a->shape, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);
+        return sa2::tc::bwd(p, s, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);
     }
 
-    switch (a->shape.d) {
+    switch (s.d) {
         case 32: return simt_bwd<32>(p, st, a->phases);
         case 64: return simt_bwd<64>(p, st, a->phases);
         default: return simt_bwd<128>(p, st, a->phases);
@@ -279,10 +292,11 @@ int sa2_bwd_static_scratch(const sa2_bwd_args *a) {
     float *rowsum = static_rowsum_ptr();
     if (!rowsum) return SA2_ERR_CUDA;
 
+    const sa2_shape s = clamped(a->shape);
     KernelParams p{};
-    fill_bwd_params(p, a, rowsum);    // every entry the kernels read is rewritten first: nothing has to start at zero
+    fill_bwd_params(p, a, s, rowsum);    // every entry the kernels read is rewritten first: nothing has to start at zero
     cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
-    switch (a->shape.d) {
+    switch (s.d) {
         case 32: return simt_bwd<32>(p, st);
         case 64: return simt_bwd<64>(p, st);
         default: return simt_bwd<128>(p, st);
