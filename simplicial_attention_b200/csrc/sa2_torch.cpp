@@ -59,6 +59,12 @@ int dtype_of(const Tensor &t) {
 }
 bool aligned(const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
 
+// The kernels may read t's memory as it stands: t is on `where`, and no subclass stands between it and its values.  The
+// general paths run into torch's own errors, or its dispatch, for everything else.
+bool plain(const Tensor &t, c10::Device where) {
+    return t.device() == where && t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !t.key_set().has(c10::DispatchKey::Python);
+}
+
 // the tensor itself if the kernels can address it in place, else a contiguous copy
 Tensor usable(const Tensor &t) {
     const bool ok = t.stride(3) == 1 && t.stride(0) % 4 == 0 && t.stride(1) % 4 == 0 && t.stride(2) % 4 == 0 && aligned(t);
@@ -289,12 +295,17 @@ struct QkvAttn : torch::autograd::Function<QkvAttn> {
     }
 };
 
-bool projection_ok(const Tensor &proj, const std::vector<Tensor> &gain, const Heads &h, at::ScalarType dt) {
-    if (!proj.is_cuda() || proj.dim() != 3 || dtype_of(proj) < 0 || (dt != at::kFloat && dt != at::kBFloat16) || gain.size() != 5) return false;
-    if (proj.size(2) != h.channels() || proj.numel() == 0 || proj.stride(2) != 1 || proj.stride(0) != proj.size(1) * proj.stride(1)) return false;
+bool gains_ok(const std::vector<Tensor> &gain, const Heads &h, c10::Device where) {
+    if (gain.size() != 5) return false;
     for (const Tensor &g : gain)
-        if (!g.is_cuda() || g.scalar_type() != gain[0].scalar_type() || dtype_of(g) < 0 || g.dim() != 1 || g.size(0) != h.d || g.stride(0) != 1 || !aligned(g)) return false;
-    return h.d == 32 || h.d == 64 || h.d == 128;
+        if (!plain(g, where) || g.scalar_type() != gain[0].scalar_type() || dtype_of(g) < 0 || g.dim() != 1 || g.size(0) != h.d || g.stride(0) != 1 || !aligned(g))
+            return false;
+    return true;
+}
+bool projection_ok(const Tensor &proj, const std::vector<Tensor> &gain, const Heads &h, at::ScalarType dt) {
+    if (!plain(proj, proj.device()) || proj.dim() != 3 || dtype_of(proj) < 0 || (dt != at::kFloat && dt != at::kBFloat16)) return false;
+    if (proj.size(2) != h.channels() || proj.numel() == 0 || proj.stride(2) != 1 || proj.stride(0) != proj.size(1) * proj.stride(1)) return false;
+    return gains_ok(gain, h, proj.device()) && (h.d == 32 || h.d == 64 || h.d == 128);
 }
 
 // [b][n][hq][d], or None
@@ -304,11 +315,11 @@ pybind11::object qkv_attn(const Tensor &proj, const std::vector<Tensor> &gain, i
     return pybind11::cast(QkvAttn::apply(proj, gain[0], gain[1], gain[2], gain[3], gain[4], hq, hk, d, eps, dt, w1, w2, kernel));
 }
 
-bool cache_ok(const std::vector<Tensor> &cache, const Heads &h, int64_t b, at::ScalarType dt) {
+bool cache_ok(const std::vector<Tensor> &cache, const Heads &h, const Tensor &x) {
     if (cache.size() != 4) return false;
-    const int64_t piece = dt == at::kBFloat16 ? 8 : 4;
+    const int64_t piece = x.scalar_type() == at::kBFloat16 ? 8 : 4;
     for (const Tensor &t : cache)
-        if (!t.is_cuda() || t.dim() != 4 || t.scalar_type() != dt || t.size(0) != b || t.size(2) != h.hk || t.size(3) != h.d || t.stride(3) != 1 ||
+        if (!plain(t, x.device()) || t.dim() != 4 || t.scalar_type() != x.scalar_type() || t.size(0) != x.size(0) || t.size(2) != h.hk || t.size(3) != h.d || t.stride(3) != 1 ||
             t.stride(0) % piece || t.stride(1) % piece || t.stride(2) % piece || !aligned(t)) return false;
     return cache[0].size(1) == cache[2].size(1) && cache[1].size(1) == cache[3].size(1);
 }
@@ -340,7 +351,7 @@ void attend_cached(const Tensor &proj, const std::vector<Tensor> &gain, const st
 pybind11::object qkv_attn_cached(const Tensor &proj, const std::vector<Tensor> &gain, const std::vector<Tensor> &cache, int64_t hq, int64_t hk,
                                  int64_t d, double eps, int64_t w1, int64_t w2, int64_t kernel) {
     const Heads h{hq, hk, d};
-    if (!projection_ok(proj, gain, h, proj.scalar_type()) || !cache_ok(cache, h, proj.size(0), proj.scalar_type())) return pybind11::none();
+    if (!projection_ok(proj, gain, h, proj.scalar_type()) || !cache_ok(cache, h, proj)) return pybind11::none();
     const c10::cuda::CUDAGuard guard(proj.device());
     const at::AutoDispatchBelowADInplaceOrView below;
     Tensor out, set[4];
@@ -349,7 +360,7 @@ pybind11::object qkv_attn_cached(const Tensor &proj, const std::vector<Tensor> &
 }
 
 bool row_norm_ok(const std::optional<Tensor> &w, const Tensor &x) {
-    return !w || (w->dim() == 1 && w->numel() == x.size(2) && w->is_cuda() && dtype_of(*w) >= 0 && w->stride(0) == 1 && aligned(*w));
+    return !w || (w->dim() == 1 && w->numel() == x.size(2) && plain(*w, x.device()) && dtype_of(*w) >= 0 && w->stride(0) == 1 && aligned(*w));
 }
 // RMSNorm over the last dimension, the gain read in its own type; the row scale is not kept.  Widths that the kernel
 // does not take go where headnorm.py's RMSNorm sends them.
@@ -385,12 +396,12 @@ pybind11::object step(const Tensor &x, const std::optional<Tensor> &pre, double 
                       const std::vector<Tensor> &cache, int64_t hq, int64_t hk, int64_t d, double eps, int64_t w1, int64_t w2, int64_t kernel,
                       const Tensor &w_out, const std::optional<Tensor> &post, double post_eps) {
     const Heads h{hq, hk, d};
-    if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || dtype_of(x) < 0 || !row_norm_ok(pre, x)) return pybind11::none();
+    if (!plain(x, x.device()) || x.dim() != 3 || x.numel() == 0 || dtype_of(x) < 0 || !row_norm_ok(pre, x)) return pybind11::none();
     for (const Tensor *w : {&w_qkv, &w_out})
-        if (!w->is_cuda() || w->dim() != 2 || w->scalar_type() != x.scalar_type()) return pybind11::none();
+        if (!plain(*w, x.device()) || w->dim() != 2 || w->scalar_type() != x.scalar_type()) return pybind11::none();
     if (w_qkv.size(1) != x.size(2) || w_qkv.size(0) != h.channels() || w_out.size(1) != hq * d || w_out.size(0) != x.size(2) || !row_norm_ok(post, x))
         return pybind11::none();
-    if (!cache_ok(cache, h, x.size(0), x.scalar_type())) return pybind11::none();
+    if (!cache_ok(cache, h, x) || !gains_ok(gain, h, x.device())) return pybind11::none();
     const c10::cuda::CUDAGuard guard(x.device());
     const at::AutoDispatchBelowADInplaceOrView below;
     const Tensor proj = step_linear(pre ? row_norm(x, *pre, pre_eps) : x, w_qkv);

@@ -1,0 +1,62 @@
+"""The native host path takes plain tensors of one device; anything else goes to the general path, which raises torch's
+own errors or dispatches to the tensor's class.  Fake tensors stand for tensors of several GPUs and of a subclass, so
+this runs without one."""
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+import simplicial_attention_b200 as sa
+from simplicial_attention_b200 import _lib
+
+B, DIM, HQ, HK, D, W1, W2 = 2, 128, 2, 1, 64, 16, 8
+CHANNELS = D * (HQ + 4 * HK)
+
+
+def _fake(on_second=()):
+    """Arguments of a generation step; the tensors named in ``on_second`` sit on another GPU than the rest."""
+    shapes = {"x": (B, 1, DIM), "proj": (B, 1, CHANNELS), "pre": (DIM,), "w_qkv": (CHANNELS, DIM), "gain": (D,), "w_out": (DIM, HQ * D), "post": (DIM,),
+              "c1": (B, W1 - 1, HK, D), "c2": (B, W2 - 1, HK, D)}
+    with FakeTensorMode():
+        t = {k: torch.empty(s, dtype=torch.bfloat16, device=f"cuda:{int(k in on_second)}") for k, s in shapes.items()}
+    return t, [t["gain"]] * 5, [t["c1"], t["c2"], t["c1"], t["c2"]]
+
+
+@pytest.mark.parametrize("on_second", [(), ("w_qkv",), ("w_out",), ("gain",), ("c1",), ("pre",), ("post",)], ids=lambda s: "+".join(s) or "none")
+def test_generation_calls_decline(on_second):
+    t, gains, cache = _fake(on_second)
+    ext = _lib.ext()
+    assert ext.step(t["x"], t["pre"], 1e-6, t["w_qkv"], gains, cache, HQ, HK, D, 1e-6, W1, W2, 0, t["w_out"], t["post"], 1e-6) is None
+    assert ext.qkv_attn_cached(t["proj"], gains, cache, HQ, HK, D, 1e-6, W1, W2, 0) is None
+    assert ext.qkv_attn(t["proj"], gains, HQ, HK, D, 1e-6, torch.bfloat16, W1, W2, 0) is None
+
+
+class Wrapped(torch.Tensor):
+    """A weight whose values are elsewhere, as quantised weights are."""
+
+    @staticmethod
+    def __new__(cls, inner):
+        return torch.Tensor._make_wrapper_subclass(cls, inner.shape, dtype=inner.dtype, device=inner.device)
+
+    def __init__(self, inner):
+        self.inner = inner
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        un = lambda a: a.inner if isinstance(a, Wrapped) else a
+        res = func(*torch.utils._pytree.tree_map(un, args), **torch.utils._pytree.tree_map(un, kwargs or {}))
+        return cls(res) if func is torch.ops.aten.detach.default else res
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["to_qkv", "combine_heads", "q_norm"])
+def test_subclass_weights_are_dispatched(name):
+    torch.manual_seed(0)
+    m = sa.SlidingWindowTwoSimplicialMHA(dim=DIM, dim_head=D, heads=HQ, key_value_heads=HK, prenorm=True, w1=W1, w2=W2).cuda().bfloat16()
+    x = torch.randn(B, 20, DIM, device="cuda").bfloat16()
+    with torch.no_grad():
+        _, cache = m(x, return_cache=True)
+        want = m(x[:, :1], cache=cache, return_cache=True)[0]
+        layer = getattr(m, name)
+        layer.weight = torch.nn.Parameter(Wrapped(layer.weight.detach()), requires_grad=False)
+        got = m(x[:, :1], cache=cache, return_cache=True)[0]
+    assert (got.float() - want.float()).abs().max().item() <= 2e-2      # roundings of bf16 results of about 1
