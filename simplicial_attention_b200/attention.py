@@ -175,12 +175,15 @@ class SlidingTwoSimplicialAttention(Function):
     @staticmethod
     def apply(q, k1, k2, v1, v2, w1=512, w2=32, causal=True, scale=None, kernel="auto", return_lse=False):
         """Runs the node of the native host path, which does what ``forward`` and ``backward`` below do in Python
-        (a forward + backward pair cost the host 280 us there, more than the kernels of a short sequence)."""
+        (a forward + backward pair cost the host 280 us there, more than the kernels of a short sequence).  What the
+        native node declines - tracing, tensors under a transform or with a tangent, subclasses - goes through the
+        Python function, which torch knows how to record or to refuse."""
         assert causal, "only the causal sliding-window form is implemented (the reference's module always passes causal=True)"
         res = _lib.ext().attn(q, k1, k2, v1, v2, int(w1), int(w2), None if scale is None else float(scale), _lib.KERNELS[kernel], bool(return_lse))
         if res is None:
             _check_inputs(q, k1, k2, v1, v2)
-            raise ValueError("unsupported inputs")
+            return super(SlidingTwoSimplicialAttention, SlidingTwoSimplicialAttention).apply(
+                q, k1, k2, v1, v2, w1, w2, causal, scale, kernel, return_lse)
         return res
 
     @staticmethod

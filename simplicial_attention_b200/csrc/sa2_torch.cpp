@@ -4,12 +4,15 @@
 // blocks, as attention.py and headnorm.py do through ctypes.  In Python a forward + backward pair of the operator
 // cost the host 280 us and a generation step of the module 520 us, more than the kernels of short sequences take.
 //
-// Every function returns None when the tensors are not what the kernels take; the Python caller then runs its own
-// checks, which raise the documented exceptions, or its general path.
+// Every function returns None when the tensors are not what the kernels take, or when torch is recording or
+// transforming the computation; the Python caller then runs its own checks, which raise the documented exceptions, and
+// its general path.
 #include <torch/extension.h>
 #include <torch/csrc/Exceptions.h>
+#include <ATen/TracerMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include "sa2.h"
 
 namespace {
@@ -59,11 +62,16 @@ int dtype_of(const Tensor &t) {
 }
 bool aligned(const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
 
-// The kernels may read t's memory as it stands: t is on `where`, and no subclass stands between it and its values.  The
-// general paths run into torch's own errors, or its dispatch, for everything else.
+// The kernels may read t's memory as it stands: t is on `where`, and neither a subclass nor a functorch transform stands
+// between it and its values, nor does it carry a forward-mode tangent that a raw launch would drop.  The general paths
+// run into torch's own errors, or its dispatch, for everything else.
 bool plain(const Tensor &t, c10::Device where) {
-    return t.device() == where && t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !t.key_set().has(c10::DispatchKey::Python);
+    static const c10::DispatchKeySet wrappers({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
+    return t.device() == where && t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !t.key_set().has_any(wrappers) && !t._fw_grad(0).defined();
 }
+// torch.jit.trace is recording: it sees the allocations of the nodes below but not their launches, so that a replay
+// would return uninitialised memory
+bool tracing() { return at::tracer::impl::is_dispatch_enabled(); }
 
 // the tensor itself if the kernels can address it in place, else a contiguous copy
 Tensor usable(const Tensor &t) {
@@ -87,8 +95,9 @@ sa2_shape shape_of(const Tensor &q, const Tensor &k1, const Tensor &k2, const Cf
 }
 
 bool inputs_ok(const Tensor &q, const Tensor &k1, const Tensor &k2, const Tensor &v1, const Tensor &v2) {
+    if (tracing()) return false;
     for (const Tensor *t : {&q, &k1, &k2, &v1, &v2})
-        if (!t->is_cuda() || t->dim() != 4 || t->scalar_type() != q.scalar_type()) return false;
+        if (!plain(*t, q.device()) || t->dim() != 4 || t->scalar_type() != q.scalar_type()) return false;
     const auto n = q.size(1), d = q.size(3), hk = k1.size(2);
     if (dtype_of(q) < 0 || (d != 32 && d != 64 && d != 128) || hk <= 0 || q.size(2) % hk != 0) return false;
     if (k1.sizes() != v1.sizes() || k2.sizes() != v2.sizes()) return false;
@@ -213,8 +222,9 @@ struct HeadNorm : torch::autograd::Function<HeadNorm> {
         return {dx.view(ctx->saved_data["shape"].toIntVector()), dw.to((at::ScalarType)ctx->saved_data["wdtype"].toInt()), Tensor(), Tensor(), Tensor()};
     }
 };
-Tensor headnorm(const Tensor &x, const Tensor &weight, int64_t d, double eps, at::ScalarType out_dtype) {
-    return HeadNorm::apply(x, weight, d, eps, out_dtype);
+pybind11::object headnorm(const Tensor &x, const Tensor &weight, int64_t d, double eps, at::ScalarType out_dtype) {
+    if (tracing() || !plain(x, x.device()) || !plain(weight, x.device())) return pybind11::none();
+    return pybind11::cast(HeadNorm::apply(x, weight, d, eps, out_dtype));
 }
 
 // ------------------------------------------------------------------ the module: packed projection -> attention
@@ -303,7 +313,7 @@ bool gains_ok(const std::vector<Tensor> &gain, const Heads &h, c10::Device where
     return true;
 }
 bool projection_ok(const Tensor &proj, const std::vector<Tensor> &gain, const Heads &h, at::ScalarType dt) {
-    if (!plain(proj, proj.device()) || proj.dim() != 3 || dtype_of(proj) < 0 || (dt != at::kFloat && dt != at::kBFloat16)) return false;
+    if (tracing() || !plain(proj, proj.device()) || proj.dim() != 3 || dtype_of(proj) < 0 || (dt != at::kFloat && dt != at::kBFloat16)) return false;
     if (proj.size(2) != h.channels() || proj.numel() == 0 || proj.stride(2) != 1 || proj.stride(0) != proj.size(1) * proj.stride(1)) return false;
     return gains_ok(gain, h, proj.device()) && (h.d == 32 || h.d == 64 || h.d == 128);
 }
@@ -396,6 +406,8 @@ pybind11::object step(const Tensor &x, const std::optional<Tensor> &pre, double 
                       const std::vector<Tensor> &cache, int64_t hq, int64_t hk, int64_t d, double eps, int64_t w1, int64_t w2, int64_t kernel,
                       const Tensor &w_out, const std::optional<Tensor> &post, double post_eps) {
     const Heads h{hq, hk, d};
+    // (a dispatch mode wants to see the projections, which the kernel for few rows hides)
+    if (tracing() || c10::impl::TorchDispatchModeTLS::any_modes_set()) return pybind11::none();
     if (!plain(x, x.device()) || x.dim() != 3 || x.numel() == 0 || dtype_of(x) < 0 || !row_norm_ok(pre, x)) return pybind11::none();
     for (const Tensor *w : {&w_qkv, &w_out})
         if (!plain(*w, x.device()) || w->dim() != 2 || w->scalar_type() != x.scalar_type()) return pybind11::none();

@@ -22,7 +22,13 @@ def head_rmsnorm(x, weight, d, eps, out_dtype=None):
     entry per channel.  ``out_dtype`` defaults to ``x.dtype``."""
     out_dtype = x.dtype if out_dtype is None else out_dtype
     assert x.is_cuda and x.dtype in _DTYPES and out_dtype in _DTYPES
-    return _lib.ext().headnorm(x, weight, int(d), float(eps), out_dtype)
+    y = _lib.ext().headnorm(x, weight, int(d), float(eps), out_dtype)
+    if y is not None:
+        return y
+    # torch is recording or transforming the computation (the native call says when): the same arithmetic in its operators
+    heads = x.float().unflatten(-1, (-1, int(d)))
+    y = (heads * torch.rsqrt(heads.square().mean(-1, keepdim=True) + float(eps))).flatten(-2)
+    return (y * weight.float()).to(out_dtype)
 
 
 class RMSNorm(torch.nn.Module):

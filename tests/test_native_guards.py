@@ -60,3 +60,47 @@ def test_subclass_weights_are_dispatched(name):
         layer.weight = torch.nn.Parameter(Wrapped(layer.weight.detach()), requires_grad=False)
         got = m(x[:, :1], cache=cache, return_cache=True)[0]
     assert (got.float() - want.float()).abs().max().item() <= 2e-2      # roundings of bf16 results of about 1
+
+
+def _module():
+    torch.manual_seed(0)
+    m = sa.SlidingWindowTwoSimplicialMHA(dim=DIM, dim_head=D, heads=HQ, key_value_heads=HK, prenorm=True, postnorm=True, w1=W1, w2=W2)
+    return m.cuda().bfloat16().requires_grad_(False), torch.randn(B, 20, DIM, device="cuda").bfloat16()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["op", "module", "generation"])
+def test_traced_calls_compute(what):
+    """A trace replayed on other inputs gives their results (a trace of raw launches would return fresh, unwritten memory)."""
+    m, x = _module()
+    _, cache = m(x, return_cache=True)
+    if what == "op":
+        f = lambda q, k1, k2, v1, v2: sa.sliding_two_simplicial_attn(q, (k1, k2), (v1, v2), w1=W1, w2=W2)
+        first, other = ([torch.randn(1, 50, h, D, device="cuda").bfloat16() for h in (HQ, HK, HK, HK, HK)] for _ in range(2))
+    elif what == "module":
+        f, first, other = m, [x], [x.flip(1).contiguous()]
+    else:
+        f = lambda t, a, b, c, d: m(t, cache=((a, b), (c, d)), return_cache=True)[0]
+        first, other = ([x[:, i:i + 1].contiguous(), *cache[0], *cache[1]] for i in (0, 7))
+    with torch.no_grad():
+        traced = torch.jit.trace(f, tuple(first), check_trace=False)
+        got, want = traced(*other), f(*other)
+    assert (got.float() - want.float()).abs().max().item() <= 2 ** -5      # two roundings to bf16 of values below 4
+
+
+@pytest.mark.gpu
+def test_tangents_and_transforms_are_refused_not_dropped():
+    import torch.autograd.forward_ad as fa
+    m, x = _module()
+    _, cache = m(x, return_cache=True)
+    q, k1, k2, v1, v2 = (torch.randn(1, 50, h, D, device="cuda") for h in (HQ, HK, HK, HK, HK))
+    op = lambda t: sa.sliding_two_simplicial_attn(t, (k1, k2), (v1, v2), w1=W1, w2=W2)
+    with torch.no_grad(), fa.dual_level():
+        with pytest.raises(NotImplementedError):
+            m(fa.make_dual(x[:, :1].contiguous(), x[:, 1:2].contiguous()), cache=cache, return_cache=True)
+        with pytest.raises(NotImplementedError):
+            op(fa.make_dual(q, q))
+    with pytest.raises(RuntimeError):
+        torch.vmap(op)(q[None])
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: op(t).sum())(q)
