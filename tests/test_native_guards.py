@@ -104,3 +104,20 @@ def test_tangents_and_transforms_are_refused_not_dropped():
         torch.vmap(op)(q[None])
     with pytest.raises(RuntimeError):
         torch.func.grad(lambda t: op(t).sum())(q)
+
+
+@pytest.mark.gpu
+def test_undefined_output_gradient_gives_zeros():
+    """A consumer that returns no gradient leaves zeros on the operands, not None."""
+    class Drop(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, t):
+            return t.sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            return None
+
+    ins = [torch.randn(1, 50, h, D, device="cuda").requires_grad_() for h in (HQ, HK, HK, HK, HK)]
+    Drop.apply(sa.sliding_two_simplicial_attn(ins[0], ins[1:3], ins[3:5], w1=W1, w2=W2)).backward()
+    assert all(t.grad is not None and not t.grad.any() for t in ins)
