@@ -94,8 +94,8 @@ class HigherOrderAttention(Module):
     # One kernel normalises the whole fused projection instead of five RMSNorm modules plus casts
     # (CUDA tensors only; set to False to run the norms as separate torch modules, as the reference does).
     fused_head_norm = True
-    # The backward of that kernel keeps one fp32 partial row of the gain gradient per warp in shared
-    # memory (8 warps x channels x 4 bytes <= 200 KB); wider projections use the separate modules.
+    # Wider projections use the separate modules where there may be a backward, whose kernel spans a row with one CTA (25
+    # warps of 256 channels).  May be lowered, never raised.  Generation has no such limit.
     fused_head_norm_max_channels = 6400
 
     def _fused_norm(self, proj):
@@ -168,8 +168,9 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
         self.w1, self.w2 = w1, w2
 
     def _fused_call(self, proj):
-        """(``proj``: the projection, or tokens of its device and dtype.)  Arguments of the native calls that take the packed projection as a whole - norm and attention forward and
-        backward without splitting or concatenating it - or None where the general path is needed."""
+        """Arguments of the native calls that take the packed projection as a whole - norm and attention, forward and
+        backward, without splitting or concatenating it - or None where the general path is needed.  ``proj`` is the
+        projection, or tokens of its device and dtype."""
         at = self.attend
         if not (self.fused_head_norm and self.qk_rmsnorm and proj.is_cuda and isinstance(at, partial)
                 and at.func is sliding_two_simplicial_attn and not at.args
@@ -192,6 +193,8 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
         proj = self.to_qkv(self.prenorm(tokens))
         call = self._fused_call(proj)
         if call is None:
+            return proj, None
+        if proj.shape[-1] > self.fused_head_norm_max_channels:
             return proj, None
         gains, heads, dtype, windows = call
         return proj, _lib.ext().qkv_attn(proj, gains, *heads, dtype, *windows)

@@ -121,3 +121,14 @@ def test_undefined_output_gradient_gives_zeros():
     ins = [torch.randn(1, 50, h, D, device="cuda").requires_grad_() for h in (HQ, HK, HK, HK, HK)]
     Drop.apply(sa.sliding_two_simplicial_attn(ins[0], ins[1:3], ins[3:5], w1=W1, w2=W2)).backward()
     assert all(t.grad is not None and not t.grad.any() for t in ins)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit,modules_run", [(CHANNELS, False), (CHANNELS - 1, True)])
+def test_lowered_channel_limit_runs_the_norm_modules(limit, modules_run):
+    m, x = _module()
+    m.fused_head_norm_max_channels = limit
+    calls = []
+    m.q_norm.register_forward_hook(lambda *a: calls.append(1))
+    m(x)
+    assert bool(calls) == modules_run
