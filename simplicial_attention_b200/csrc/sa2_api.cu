@@ -382,6 +382,7 @@ int headnorm_dispatch(const sa2_headnorm_args *a, bool backward) {
     P.gains.table = a->weight;
     P.gains.al = aligned16(a->weight);
     P.partial = reinterpret_cast<float *>(a->partial);
+    P.partial_al = aligned16(a->partial);
     P.rows = a->rows; P.x_stride = a->x_stride; P.y_stride = a->y_stride; P.dy_stride = a->dy_stride;
     P.channels = a->channels; P.eps = a->eps;
     P.x_al = rows_aligned(a->x, a->x_stride, a->x_dtype);
@@ -411,6 +412,7 @@ int qkvnorm_fill(const sa2_qkvnorm_args *a, bool backward, sa2::headnorm::Params
     P.gains.hq = a->hq; P.gains.hk = a->hk;
     P.x = a->x; P.dy = a->dy; P.y = a->y; P.rstd = a->rstd;
     P.partial = reinterpret_cast<float *>(a->partial);
+    P.partial_al = aligned16(a->partial);
     P.rows = a->rows; P.x_stride = a->x_stride; P.y_stride = a->y_stride; P.dy_stride = a->dy_stride;
     P.channels = (int)channels; P.eps = a->eps;
     P.x_al = rows_aligned(a->x, a->x_stride, a->x_dtype);

@@ -99,6 +99,7 @@ struct Params {
     int channels;
     float eps;
     int x_al, y_al, dy_al;      // rows of x / y / dy start on 16-byte boundaries
+    int partial_al;             // so do those of partial (the caller's scratch has no alignment rule)
 };
 
 // sum over the lanes that share a head: D / 8 of them, all 32 for D >= 256
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(Seg<D>::CPL == 1 ? 1024 : 512) bwd_kernel(cons
 #pragma unroll
                 for (int z = 0; z < 8; ++z) dg[k][z] += t[z];
             }
-            store8<float>(P.partial + (size_t)blockIdx.x * P.channels + c0 + 256 * k, dg[k]);
+            store8u<float>(P.partial + (size_t)blockIdx.x * P.channels + c0 + 256 * k, P.partial_al, dg[k]);
         }
     }
 }

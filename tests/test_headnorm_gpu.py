@@ -100,3 +100,24 @@ def test_row_rmsnorm_module_matches_torch(dim):
     y.backward(dy.to(torch.bfloat16))
     assert xi.grad.dtype == torch.float32
     assert (y.float() - res[1][0]).abs().max().item() <= 2e-2 * res[1][0].abs().max().item()
+
+
+def test_scratch_needs_no_alignment():
+    """The gain gradient's scratch may start on any float (C ABI)."""
+    import ctypes as C
+    from simplicial_attention_b200 import _lib
+
+    lib, rows, channels = _lib.lib(), 700, 384
+    x, dy = (torch.randn(rows, channels, device="cuda") for _ in range(2))
+    gain, rstd = torch.ones(channels, device="cuda"), torch.ones(rows, channels // 64, device="cuda")
+    need = lib.sa2_headnorm_partial_bytes(rows, channels)
+    scratch = torch.empty(need // 4 + 4, device="cuda")
+    res = []
+    for shift in (0, 1):
+        dx, dw = torch.empty_like(x), torch.empty_like(gain)
+        args = _lib.HeadnormArgs(x.data_ptr(), dy.data_ptr(), gain.data_ptr(), dx.data_ptr(), rstd.data_ptr(), dw.data_ptr(),
+                                 scratch[shift:].data_ptr(), need, rows, channels, channels, channels, channels, 64, _lib.SA2_F32, _lib.SA2_F32,
+                                 1e-6, torch.cuda.current_stream().cuda_stream)
+        _lib.check(lib.sa2_headnorm_bwd(C.byref(args)), "sa2_headnorm_bwd")
+        res.append((dx, dw))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
