@@ -377,7 +377,18 @@ __device__ __forceinline__ void row_tile(const KernelParams &p, float *smem, int
 #pragma unroll
                             for (int jj = 0; jj < 4; ++jj) if (ok(ii, jj)) mx = fmaxf(mx, s[ii][jj]);
                             mx = half_warp_max(mx);
-                            if (!(mx > ref[ii])) continue;                 // (uniform over the half-warp that owns the row)
+                            // (both branches are uniform over the half-warp that owns the row)
+                            if (!(mx > ref[ii])) {
+                                // no reference yet, and none here: logits of -inf weigh nothing, and only NaN stays NaN
+                                if (ref[ii] > -CUDART_INF_F) continue;
+                                sum[ii] = 0.f;
+#pragma unroll
+                                for (int jj = 0; jj < 4; ++jj) {
+                                    pr[ii][jj] = ok(ii, jj) ? ex2f(s[ii][jj]) : 0.f;
+                                    sum[ii] += pr[ii][jj];
+                                }
+                                continue;
+                            }
                             const float f = ex2f(ref[ii] - mx);            // 0 on the first hit
                             ref[ii] = mx;
                             l_run[ii] *= f;
