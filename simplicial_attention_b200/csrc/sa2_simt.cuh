@@ -357,7 +357,9 @@ __device__ __forceinline__ void row_tile(const KernelParams &p, float *smem, int
                 auto ok = [&](int ii, int jj) { return full || (rvalid[ii] && (unsigned)(d0 + 16 * (ii - jj)) < (unsigned)p.w1); };
 
                 if (MODE == MODE_FWD) {
-                    // probabilities against a reference per row that moves only when they would grow beyond 2^64
+                    // Probabilities against a reference per row that moves only when four of them sum to more than 2^16: the
+                    // first tile's maximum mostly serves the whole row, and a sum of P v1 overflows no earlier than 2^22
+                    // (64 keys) from the end of the range.
                     float pr[4][4], sum[4];
                     bool exceed = false;
 #pragma unroll
@@ -368,7 +370,7 @@ __device__ __forceinline__ void row_tile(const KernelParams &p, float *smem, int
                             pr[ii][jj] = ok(ii, jj) ? ex2f(s[ii][jj] - ref[ii]) : 0.f;
                             sum[ii] += pr[ii][jj];
                         }
-                        exceed |= !(sum[ii] <= 1.8446744e19f);
+                        exceed |= !(sum[ii] <= 65536.f);
                     }
                     if (__any_sync(0xffffffffu, exceed)) {
 #pragma unroll

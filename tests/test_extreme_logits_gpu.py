@@ -38,3 +38,17 @@ def test_logits_of_minus_infinity_weigh_nothing_fp32(d):
     assert seen.sum() >= 150
     assert lse[:, :, seen].isfinite().all()
     assert (out[:, seen] - ref[:, seen]).abs().max().item() <= 1e-4 * ref[:, seen].abs().max().item()
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_rising_logits_with_large_values_fp32(d):
+    """Logits that climb by 60 over the window next to values of 1e22: the partial sums stay inside fp32."""
+    w1, w2 = 200, 3
+    q, k1, k2, v1, v2 = _operands(d, torch.float32)
+    q.fill_(1.)
+    k2.fill_(1.)
+    k1[:] = (torch.arange(200, device="cuda") * (0.3 * d ** -0.5)).view(1, -1, 1, 1)
+    v1 *= 1e22
+    out, lse = sa.sa2_forward(q, k1, k2, v1, v2, w1, w2)
+    ref = _reference(q, k1, k2, v1, v2, w1, w2)
+    assert (out - ref).abs().max().item() <= 1e-4 * ref.abs().max().item()
