@@ -210,7 +210,7 @@ int sa2_fwd(const sa2_fwd_args *a) {
 
     const bool tc_ok = sa2::tc::fwd_supported(s) && sa2::tc::fwd_addressable(p);
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
-    if (tc_ok && s.kernel != SA2_KERNEL_SIMT) return sa2::tc::fwd(p, s, st);
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT) return sa2::tc::fwd(p, s, sa2::tc::fwd_split(a->shape), st);
 
     switch (s.d) {
         case 32: return simt_fwd<32>(p, st);

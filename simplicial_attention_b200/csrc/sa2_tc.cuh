@@ -21,6 +21,12 @@ inline int tiles_per_query_tile(int w1) { return (w1 + TJ - 1 + TJ - 1) / TJ; } 
 
 // The tensor-core forward handles bf16 at every head dim and any window.
 inline bool fwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
+// Head dim 32, and head dim 64 with a first window of more than 513 rows (the caller's window, however short the sequence),
+// keep the products q * k2 and the probabilities to 16 bits and more, as a bf16 value and a bf16 rest each, so that only
+// the inputs and the result are rounded to 8 bits: callers of these shapes had fp32 arithmetic.  The products are exact
+// that way.  Relative error of the output against 64 bits 1.57e-3 to 1.67e-3, as with fp32 arithmetic (2.2e-3 to 3.2e-3 with
+// rounded operands); of the logsumexp 2e-6, absolute (3e-3 to 1.6e-2).
+inline bool fwd_split(const sa2_shape &s) { return s.d == 32 || (s.d == 64 && s.w1 > 513); }
 // So does the tensor-core backward.
 inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -117,13 +123,14 @@ inline int fwd128(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
-template <int D>
+template <int D, bool SPLIT>
 inline int fwd_launch(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
     FwdParams P;
     P.kp = kp;
     P.ri_log2 = fwd_ri_log2(s, SM_COUNT);
     P.win_boxes = fwd_win_boxes(s.w2, P.ri_log2);
-    P.nslots = fwd_slots(s.w1, P.ri_log2, P.win_boxes);
+    constexpr int A_TILES = 2 * FwdA<D, SPLIT>::TILES;
+    P.nslots = fwd_slots(s.w1, P.ri_log2, P.win_boxes, A_TILES);
     P.c = s.scale * 1.4426950408889634f;
     P.status = status_word();
     if (!P.status) return SA2_ERR_CUDA;
@@ -133,19 +140,19 @@ inline int fwd_launch(const KernelParams &kp, const sa2_shape &s, cudaStream_t s
         !tmap::make_rows_map(&mapK2, kp.k2.p, kp.b, kp.nk2, kp.hk, D, kp.k2.sb, kp.k2.sn, kp.k2.sh, 32) ||
         !tmap::make_rows_map(&mapV2, kp.v2.p, kp.b, kp.nk2, kp.hk, D, kp.v2.sb, kp.v2.sn, kp.v2.sh, 32))
         return SA2_ERR_CUDA;
-    const size_t smem = fwd_smem_bytes(P.nslots, P.win_boxes);
-    if (cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    const size_t smem = fwd_smem_bytes(P.nslots, P.win_boxes, A_TILES);
+    if (cudaFuncSetAttribute(fwd_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SA2_ERR_CUDA;
     const int ri = 1 << P.ri_log2;
-    fwd_kernel<D><<<dim3((kp.n + ri - 1) / ri, kp.hq, kp.b), FWD_THREADS, smem, st>>>(mapK, mapV, mapK2, mapV2, P);
+    fwd_kernel<D, SPLIT><<<dim3((kp.n + ri - 1) / ri, kp.hq, kp.b), FWD_THREADS, smem, st>>>(mapK, mapV, mapK2, mapV2, P);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
-inline int fwd(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {
+inline int fwd(const KernelParams &kp, const sa2_shape &s, bool split, cudaStream_t st) {
     if (!fwd_addressable(kp)) return SA2_ERR_INVALID;
     switch (s.d) {
-        case 32: return fwd_launch<32>(kp, s, st);
-        case 64: return fwd_launch<64>(kp, s, st);
+        case 32: return fwd_launch<32, true>(kp, s, st);
+        case 64: return split ? fwd_launch<64, true>(kp, s, st) : fwd_launch<64, false>(kp, s, st);
         default: return fwd128(kp, s, st);
     }
 }

@@ -31,6 +31,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t *>(&v);
 }
+// a * b - hi, hi = bf16(a * b): the product of two bf16 values has 16 bits, so the pair (hi, this) is exact
+__device__ __forceinline__ uint32_t mul_rest_bf16x2(uint32_t a, uint32_t b, uint32_t hi) {
+    __nv_bfloat162 r = __hfma2(*reinterpret_cast<__nv_bfloat162 *>(&a), *reinterpret_cast<__nv_bfloat162 *>(&b),
+                               __hneg2(*reinterpret_cast<__nv_bfloat162 *>(&hi)));
+    return *reinterpret_cast<uint32_t *>(&r);
+}
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162 *>(&a), *reinterpret_cast<__nv_bfloat162 *>(&b));
     return *reinterpret_cast<uint32_t *>(&r);
@@ -50,22 +56,30 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volati
 // [group][128] the reference it is expressed against
 constexpr int FWD_STATS_FLOATS = 2 * 2 * 128 + 2 * 128 + 2 * 128;
 
-// exp2(c * s - ref) for 32 logits of one row -> 16 packed bf16 pairs; returns their sum.
-// Columns outside (lo, hi] are masked (window / causality / sequence start).
-__device__ __forceinline__ float fwd_probs32(const uint32_t (&s)[32], uint32_t (&pk)[16], float c, float ref,
+// what two packed bf16 probabilities leave of the fp32 ones, as bf16: together they carry 16 bits
+__device__ __forceinline__ uint32_t pack_rest(float p0, float p1, uint32_t hi) {
+    return pack_bf16(p0 - __uint_as_float(hi << 16), p1 - __uint_as_float(hi & 0xffff0000u));
+}
+
+// exp2(c * s - ref) for 32 logits of one row -> 16 packed bf16 pairs, and the pairs of what the rounding left if SPLIT;
+// returns their sum.  Columns outside (lo, hi] are masked (window / causality / sequence start).
+template <bool SPLIT>
+__device__ __forceinline__ float fwd_probs32(const uint32_t (&s)[32], uint32_t (&pk)[16], uint32_t (&rest)[16], float c, float ref,
                                              bool full, int col0, int lo, int hi) {
+    float sum0 = 0.f, sum1 = 0.f;
+    auto put = [&](int x, float p0, float p1) {
+        sum0 += p0; sum1 += p1;
+        pk[x >> 1] = pack_bf16(p0, p1);
+        if constexpr (SPLIT) rest[x >> 1] = pack_rest(p0, p1, pk[x >> 1]);
+    };
     if (full) {
         const uint64_t c2 = f2_pack(c, c), nref2 = f2_pack(-ref, -ref);
-        float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
         for (int x = 0; x < 32; x += 2) {
             float a0, a1;
             f2_unpack(f2_fma(f2_pack(s[x], s[x + 1]), c2, nref2), a0, a1);
-            const float p0 = ex2(a0), p1 = ex2(a1);
-            sum0 += p0; sum1 += p1;
-            pk[x >> 1] = pack_bf16(p0, p1);
+            put(x, ex2(a0), ex2(a1));
         }
-        return sum0 + sum1;
     } else {
         // Valid columns are the integers in (lo, hi]: |col - mid| <= half, and an invalid column is at least
         // half + 1 away, so saturate(half + 1 - |col - mid|) is exactly 1 or 0: two FADDs and an FMUL on the
@@ -73,18 +87,15 @@ __device__ __forceinline__ float fwd_probs32(const uint32_t (&s)[32], uint32_t (
         // clamped so that a masked-out logit far above the reference cannot produce inf * 0; a clamped
         // valid logit still trips the slow path.
         const float mid = 0.5f * (float)(lo + 1 + hi), hwp = 0.5f * (float)(hi - lo - 1) + 1.f;
-        float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
         for (int x = 0; x < 32; x += 2) {
             const float v0 = __saturatef(hwp - fabsf((float)(col0 + x) - mid));
             const float v1 = __saturatef(hwp - fabsf((float)(col0 + x + 1) - mid));
-            const float p0 = ex2(fminf(fmaf(__uint_as_float(s[x]), c, -ref), 100.f)) * v0;
-            const float p1 = ex2(fminf(fmaf(__uint_as_float(s[x + 1]), c, -ref), 100.f)) * v1;
-            sum0 += p0; sum1 += p1;
-            pk[x >> 1] = pack_bf16(p0, p1);
+            put(x, ex2(fminf(fmaf(__uint_as_float(s[x]), c, -ref), 100.f)) * v0,
+                ex2(fminf(fmaf(__uint_as_float(s[x + 1]), c, -ref), 100.f)) * v1);
         }
-        return sum0 + sum1;
     }
+    return sum0 + sum1;
 }
 
 }  // namespace tc

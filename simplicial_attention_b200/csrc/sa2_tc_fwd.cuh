@@ -12,7 +12,7 @@
 //
 // Why pairs: the window of RI rows is w1 + RI - 1 keys, so a small RI wastes fewer masked columns (w1 = 512:
 // 576 columns at RI = 64, 640 at RI = 128), a short sequence is spread over more CTAs of fewer sweeps each,
-// and a single new token (generation) still fills the rows of its tile.  fwd_rows_per_tile() picks RI.
+// and a single new token (generation) still fills the rows of its tile.  fwd_ri_log2() picks RI.
 //
 // Warp roles (512 threads, four aligned warpgroups):
 //   warp 0, 1     issue the tcgen05.mma stream of group 0 / group 1 (warp 1 owns the TMEM allocation)
@@ -32,13 +32,18 @@
 // the issuing thread of a group alternates P V1 of unit u and S of unit u + 2, whose completion therefore also says
 // that the P columns are free - and which 32-column chunks need no mask, or are seen by nobody, is decided from
 // warp-uniform bounds without votes.
-// Measured: b4 n4096 h8 d64 w512/32 1.26 -> 0.96 ms (537 TFLOP/s), b2 n1024 0.178 -> 0.141 ms; what ran on the fp32
-// kernels before: b1 n3001 h8 d64 w1024/16 4.16 -> 0.20 ms, b4 n4096 h8 d32 w512/32 7.8 -> 0.89 ms; one new row
-// of b1 h8 behind a full window 0.19 -> 0.017 ms.
+// Measured: b4 n4096 h8 d64 w512/32 1.26 -> 0.96 ms (537 TFLOP/s), b2 n1024 0.178 -> 0.141 ms; one new row of b1 h8 behind a
+// full window 0.19 -> 0.017 ms.
 // Measured and not kept, where this form takes 0.96 (or, earlier, 1.12) ms: A in TMEM with one P buffer (1.5 against 1.12),
 // 128-key units (1.4), S and P V1 from separate issuing threads (1.15), S(u + 2) before P V1(u) (1.19), ordering the
 // softmax groups against each other (1.04 against 0.96), A and W double-buffered (0.98), an output group that takes its
 // events as they come (1.01).
+//
+// SPLIT (head dim 32, and head dim 64 with w1 > 513: see fwd_split): A and P are each a bf16 value and a bf16 rest, so S and
+// P V1 take two products per K step instead of one, with the rests of P over the S columns they come from.  The softmax
+// groups pack twice as many words, which is what the time goes to: b1 n3001 h8 d64 w1024/16 0.208 -> 0.269 ms,
+// b4 n4096 h8 d64 w1024/32 1.63 -> 2.27 ms, d32 w512/32 0.90 -> 1.12 ms against rounded operands; 4.15, 34 and 12.6 ms on the
+// fp32 kernels.
 //
 // Reference handling: probabilities are computed against a per-row reference
 // that only moves when it must, so the W accumulator in TMEM normally never
@@ -91,11 +96,19 @@ struct FwdParams {
 
 // at least 120 KB: one CTA per SM, so the 512-column TMEM allocation never waits for a co-resident CTA; at least
 // three slots: the merge of the row partials (128 rows of D + 4 floats) reuses them
-inline size_t fwd_smem_bytes(int nslots, int win_boxes) {
-    const size_t need = 1024 + (size_t)(nslots > 3 ? nslots : 3) * 2 * FWD_UNIT_BYTES + (size_t)win_boxes * 2 * 4096 + 2 * TILE_BYTES +
+inline size_t fwd_smem_bytes(int nslots, int win_boxes, int a_tiles) {
+    const size_t need = 1024 + (size_t)(nslots > 3 ? nslots : 3) * 2 * FWD_UNIT_BYTES + (size_t)win_boxes * 2 * 4096 + a_tiles * TILE_BYTES +
                         FWD_STATS_FLOATS * 4 + BAR_COUNT * 8 + 64;
     return need > 120 * 1024 ? need : 120 * 1024;
 }
+
+// The A rows of a group: one tile, of which head dim 32 uses half a row for the rounded products and, with SPLIT, the other
+// half for what the rounding left; head dim 64 puts that into a second tile.
+template <int D, bool SPLIT> struct FwdA {
+    static constexpr int TILES = SPLIT && D == 64 ? 2 : 1;             // per group
+    static constexpr uint32_t BYTES = TILES * TILE_BYTES;
+    static constexpr uint32_t REST = D == 64 ? TILE_BYTES : 64;        // bytes from an element to its rest
+};
 
 struct FwdGeom {
     int i0, i_last, ri, ri_log2, re;
@@ -172,13 +185,13 @@ __device__ __forceinline__ int fwd_producer(const FwdParams &P, const FwdGeom &g
 // so their MMA streams need no ordering between them.  P V1 of unit u goes before S of unit u + 2, whose
 // completion therefore covers it (and the sweep after the next needs its A rows by then, whose builder waits for
 // the W that P V1 completes).
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ int fwd_mma(const FwdParams &P, const FwdGeom &g, int grp, uint32_t tmem, uint8_t *sK, uint8_t *sV, uint8_t *sA,
                                        uint64_t *bars, volatile int *abort_flag) {
     constexpr uint32_t IDESC_S = idesc_bf16(128, FWD_UNIT, false, false);
     constexpr uint32_t IDESC_PV = idesc_bf16(128, 64, false, true);    // (head dim 32: the upper 32 channels are zeros)
     const uint64_t dK = smem_desc_sw128(smem_u32(sK)), dV = smem_desc_sw128(smem_u32(sV));
-    const uint64_t dA = smem_desc_sw128(smem_u32(sA) + grp * TILE_BYTES);
+    const uint64_t dA = smem_desc_sw128(smem_u32(sA) + grp * FwdA<D, SPLIT>::BYTES);
     const uint32_t tS = tmem + grp * 256, tP = tS + 128, tW = tS + 192;
     const int upe = g.upe, n = g.nsw[grp] * upe;
     FwdSlot ss, ps;
@@ -193,6 +206,10 @@ __device__ __forceinline__ int fwd_mma(const FwdParams &P, const FwdGeom &g, int
         if (elect_one()) {
 #pragma unroll
             for (int st = 0; st < D / 16; ++st) mma_ss(d, dA + st * 2, kt + st * 2, IDESC_S, st > 0 ? 1u : 0u);
+            if constexpr (SPLIT) {
+#pragma unroll
+                for (int st = 0; st < D / 16; ++st) mma_ss(d, dA + (FwdA<D, SPLIT>::REST >> 4) + st * 2, kt + st * 2, IDESC_S, 1u);
+            }
             tc_commit(&bars[BAR_S_FULL + grp * 2 + (u & 1)]);
             if (s_w == upe - 1) tc_commit(&bars[BAR_A_FREE + grp]);      // the A rows may be rebuilt
         }
@@ -211,13 +228,21 @@ __device__ __forceinline__ int fwd_mma(const FwdParams &P, const FwdGeom &g, int
         if (elect_one()) {
 #pragma unroll
             for (int st = 0; st < 4; ++st) mma_ts(tW, a + st * 8, vt + st * 128, IDESC_PV, (p_w > 0 || st > 0) ? 1u : 0u);
+            if constexpr (SPLIT) {          // the rests of P lie over the S they come from
+#pragma unroll
+                for (int st = 0; st < 4; ++st) mma_ts(tW, tS + (u & 1) * 64 + st * 8, vt + st * 128, IDESC_PV, 1u);
+            }
             tc_commit(&bars[BAR_PV_DONE + grp]);
             if (!g.resident) tc_commit(&bars[BAR_KV_FREE + ps.slot]);
             if (p_w == upe - 1) tc_commit(&bars[BAR_W_FULL + grp]);
         }
         ps.next(P, g, p_w);
         if (++p_w == upe) { p_w = 0; ++p_k; }
-        if (u + 2 < n && !issue_s(u + 2)) return ERR_FWD_MMA;
+        if (u + 2 < n) {
+            // S of unit u + 2 goes where the rests of P of unit u are; the softmax group has unit u + 1 to work on meanwhile
+            if (SPLIT && !mbar_wait_warp(&bars[BAR_PV_DONE + grp], u & 1, abort_flag, 0, 5)) return ERR_FWD_MMA;
+            if (!issue_s(u + 2)) return ERR_FWD_MMA;
+        }
     }
     // The ring follows group 0's walk.  With an odd number of sweeps group 1 has one sweep less: it lets the
     // units of that last sweep pass, so that every slot still collects two releases.
@@ -254,6 +279,13 @@ __device__ __forceinline__ FwdWarpRows fwd_warp_rows(const KernelParams &kp, con
     return w;
 }
 
+// where the rests of a chunk go: their own words, or (never written) the rounded ones
+template <bool SPLIT, int N> __device__ __forceinline__ uint32_t (&fwd_rest(uint32_t (&rest)[N], uint32_t (&pk)[16]))[16] {
+    if constexpr (SPLIT) return rest;
+    else return pk;
+}
+
+template <bool SPLIT>
 __device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g, int grp, uint32_t tmem, int d_w, float *stats,
                                            uint64_t *bars, volatile int *abort_flag) {
     const KernelParams &kp = P.kp;
@@ -286,19 +318,21 @@ __device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g,
             // valid columns of this row: lo < col <= hi
             const int d1 = i + kp.off1 - j0, hi = row_ok ? d1 : -1, lo = max(d1 - kp.w1, -j0 - 1);
             float sum = 0.f;
+            uint32_t rest[2][SPLIT ? 16 : 1];         // SPLIT: held until S need not be read again
 #pragma unroll
             for (int ch = 0; ch < 2; ++ch) {
                 uint32_t s[32], pk[16];
+                uint32_t (&pr)[16] = fwd_rest<SPLIT>(rest[ch], pk);
                 tmem_ld32(s_addr + ch * 32, s);
                 const int x = 2 * w + ch;            // 32-key chunk of the window
                 tmem_wait_ld(s);
                 if (x >= full0 && x <= wr.full1) {
-                    sum += fwd_probs32(s, pk, c, ref, true, 0, 0, 0);
+                    sum += fwd_probs32<SPLIT>(s, pk, pr, c, ref, true, 0, 0, 0);
                 } else if (x >= wr.some0 && x <= some1) {
-                    sum += fwd_probs32(s, pk, c, ref, false, ch * 32, lo, hi);
+                    sum += fwd_probs32<SPLIT>(s, pk, pr, c, ref, false, ch * 32, lo, hi);
                 } else {
 #pragma unroll
-                    for (int z = 0; z < 16; ++z) pk[z] = 0u;
+                    for (int z = 0; z < 16; ++z) { pk[z] = 0u; pr[z] = 0u; }
                 }
                 tmem_st16(p_addr + ch * 16, pk);
             }
@@ -340,14 +374,19 @@ __device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g,
                 }
                 tmem_wait_st();
                 sum = 0.f;
-#pragma unroll 1
+#pragma unroll (SPLIT ? 2 : 1)
                 for (int ch = 0; ch < 2; ++ch) {
                     uint32_t s[32], pk[16];
+                    uint32_t (&pr)[16] = fwd_rest<SPLIT>(rest[ch], pk);
                     tmem_ld32(s_addr + ch * 32, s);
                     tmem_wait_ld(s);
-                    sum += fwd_probs32(s, pk, c, ref, false, ch * 32, lo, hi);
+                    sum += fwd_probs32<SPLIT>(s, pk, pr, c, ref, false, ch * 32, lo, hi);
                     tmem_st16(p_addr + ch * 16, pk);
                 }
+            }
+            if constexpr (SPLIT) {
+                tmem_st16(s_addr, rest[0]);
+                tmem_st16(s_addr + 16, rest[1]);
             }
             l += sum;
             tmem_wait_st();
@@ -369,7 +408,7 @@ __device__ __forceinline__ int fwd_softmax(const FwdParams &P, const FwdGeom &g,
 // ------------------------------------------------------------------ output group (warps 4-7)
 // Thread r owns row r of the tile: it builds the row of every A and accumulates the row's output against the
 // larger of the references the two groups have reported (`ref_o`).
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ int fwd_output(const FwdParams &P, const FwdGeom &g, uint32_t tmem, uint64_t (&o)[D / 2], float &ref_o,
                                           const uint8_t *sWin, uint8_t *sA, const float *stats, uint64_t *bars, volatile int *abort_flag) {
     constexpr int NC = D / 8;                          // 16-byte chunks of a row
@@ -397,18 +436,27 @@ __device__ __forceinline__ int fwd_output(const FwdParams &P, const FwdGeom &g, 
         const bool ok = row_ok && e < kp.w2 && kk >= 0;
         const int wr = kk - g.win0;
         const __nv_bfloat16 *krow = k2 + elem_off(kp.k2, b, ok ? kk : 0, hk);
-        uint8_t *dst = sA + (size_t)grp * TILE_BYTES;
-        uint4 a[NC];
+        uint8_t *dst = sA + (size_t)grp * FwdA<D, SPLIT>::BYTES;
+        uint4 a[NC], rest[SPLIT ? NC : 1];
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc) {
             uint4 kv = make_uint4(0u, 0u, 0u, 0u);
             if (ok) kv = staged ? *reinterpret_cast<const uint4 *>(sWin + sw128_offset(wr, cc)) : __ldg(reinterpret_cast<const uint4 *>(krow + cc * 8));
             a[cc].x = mul_bf16x2(qv[cc].x, kv.x); a[cc].y = mul_bf16x2(qv[cc].y, kv.y);
             a[cc].z = mul_bf16x2(qv[cc].z, kv.z); a[cc].w = mul_bf16x2(qv[cc].w, kv.w);
+            if constexpr (SPLIT) {
+                rest[cc].x = mul_rest_bf16x2(qv[cc].x, kv.x, a[cc].x); rest[cc].y = mul_rest_bf16x2(qv[cc].y, kv.y, a[cc].y);
+                rest[cc].z = mul_rest_bf16x2(qv[cc].z, kv.z, a[cc].z); rest[cc].w = mul_rest_bf16x2(qv[cc].w, kv.w, a[cc].w);
+            }
         }
         if (bar && !warp_wait(bar, parity, abort_flag, 1)) return false;
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc) *reinterpret_cast<uint4 *>(dst + sw128_offset(r, cc)) = a[cc];
+        if constexpr (SPLIT) {
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc)
+                *reinterpret_cast<uint4 *>(dst + (D == 64 ? TILE_BYTES : 0) + sw128_offset(r, cc + (D == 64 ? 0 : 4))) = rest[cc];
+        }
         fence_proxy_async_smem();
         mbar_arrive(&bars[BAR_A_FULL + grp]);
         return true;
@@ -511,7 +559,7 @@ __device__ __forceinline__ void fwd_store(const FwdParams &P, const FwdGeom &g, 
     }
 }
 
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ void fwd_merge(const FwdParams &P, const FwdGeom &g, const uint64_t (&o)[D / 2], float ref_o,
                                           const float *stats, float *buf, bool bad) {
     constexpr int LD = D + 4;
@@ -539,8 +587,8 @@ __device__ __forceinline__ void fwd_merge(const FwdParams &P, const FwdGeom &g, 
         f2_unpack(o[2 * x + 1], v.z, v.w);
         *reinterpret_cast<float4 *>(buf + r * LD + 4 * x) = make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
     }
-    if (r < g.ri && i < kp.n)
-        kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = bad ? CUDART_NAN_F : (M + lg2(L)) * 0.6931471805599453f;
+    if (r < g.ri && i < kp.n)       // (lg2.approx would be off by 2e-6 at the denominators of a long window)
+        kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = bad ? CUDART_NAN_F : (M + (SPLIT ? log2f(L) : lg2(L))) * 0.6931471805599453f;
     fwd_out_sync();
     switch (g.re) {
         case 2: fwd_store<D, 2>(P, g, buf); break;
@@ -550,7 +598,7 @@ __device__ __forceinline__ void fwd_merge(const FwdParams &P, const FwdGeom &g, 
     }
 }
 
-template <int D>
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
            const __grid_constant__ CUtensorMap mapK2, const __grid_constant__ CUtensorMap mapV2, const FwdParams P) {
@@ -559,7 +607,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
     uint8_t *sK = smem;
     uint8_t *sV = sK + (size_t)max(P.nslots, 3) * FWD_UNIT_BYTES;
     uint8_t *sA = sV + (size_t)max(P.nslots, 3) * FWD_UNIT_BYTES;         // [2] one tile per group
-    uint8_t *sWin = sA + 2 * TILE_BYTES;
+    uint8_t *sWin = sA + 2 * FwdA<D, SPLIT>::BYTES;
     float *stats = reinterpret_cast<float *>(sWin + (size_t)P.win_boxes * 2 * 4096);
     uint64_t *bars = reinterpret_cast<uint64_t *>(stats + FWD_STATS_FLOATS);
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + BAR_COUNT);
@@ -593,13 +641,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
 #endif
     if (warp < 4) {
         reg_dealloc<FWD_REGS_ISSUE>();                // one instruction for the whole warpgroup
-        if (warp == 0) err = fwd_mma<D>(P, g, 0, tmem, sK, sV, sA, bars, abort_flag);
-        else if (warp == 1) err = fwd_mma<D>(P, g, 1, tmem, sK, sV, sA, bars, abort_flag);
+        if (warp == 0) err = fwd_mma<D, SPLIT>(P, g, 0, tmem, sK, sV, sA, bars, abort_flag);
+        else if (warp == 1) err = fwd_mma<D, SPLIT>(P, g, 1, tmem, sK, sV, sA, bars, abort_flag);
         else if (warp == 2) err = fwd_producer(P, g, &mapK, &mapK2, sK, sWin, bars, abort_flag);
         else err = fwd_producer(P, g, &mapV, &mapV2, sV, sWin + (size_t)P.win_boxes * 4096, bars, abort_flag);
     } else if (warp >= 8) {
         reg_dealloc<FWD_REGS_SOFTMAX>();
-        err = fwd_softmax(P, g, (warp - 8) >> 2, tmem, D, stats, bars, abort_flag);
+        err = fwd_softmax<SPLIT>(P, g, (warp - 8) >> 2, tmem, D, stats, bars, abort_flag);
         // the barrier sits outside fwd_softmax so that a group that gave up still reaches it
         fwd_rows_sync();
     } else {
@@ -608,10 +656,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUt
 #pragma unroll
         for (int x = 0; x < D / 2; ++x) o[x] = 0ull;
         float ref_o = -CUDART_INF_F;
-        err = fwd_output<D>(P, g, tmem, o, ref_o, sWin, sA, stats, bars, abort_flag);
+        err = fwd_output<D, SPLIT>(P, g, tmem, o, ref_o, sWin, sA, stats, bars, abort_flag);
         fwd_rows_sync();                              // both groups' denominators are in shared memory
         if (err) *abort_flag = 1;
-        fwd_merge<D>(P, g, o, ref_o, stats, reinterpret_cast<float *>(sK), err != 0 || *abort_flag != 0);
+        fwd_merge<D, SPLIT>(P, g, o, ref_o, stats, reinterpret_cast<float *>(sK), err != 0 || *abort_flag != 0);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
@@ -657,9 +705,9 @@ inline int fwd_win_boxes(int w2, int ri_log2) {
     return rows <= FWD_WIN_ROWS ? (rows + 31) / 32 : 0;
 }
 // slots for the widest window of a tile, or as many as fit beside everything else
-inline int fwd_slots(int w1, int ri_log2, int win_boxes) {
+inline int fwd_slots(int w1, int ri_log2, int win_boxes, int a_tiles) {
     const int units = (w1 + (1 << ri_log2) - 1 + FWD_UNIT - 1) / FWD_UNIT;
-    const size_t fixed = 1024 + (size_t)win_boxes * 8192 + 2 * TILE_BYTES + FWD_STATS_FLOATS * 4 + BAR_COUNT * 8 + 64;
+    const size_t fixed = 1024 + (size_t)win_boxes * 8192 + a_tiles * TILE_BYTES + FWD_STATS_FLOATS * 4 + BAR_COUNT * 8 + 64;
     const int room = (int)((232448 - fixed) / (2 * FWD_UNIT_BYTES)), most = room < FWD_MAX_SLOTS ? room : FWD_MAX_SLOTS;
     return units < most ? units : most;
 }

@@ -257,8 +257,8 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
                 // exponentials of one 32-key chunk: all columns valid for every row of the warp, masked, or none
                 auto chunk = [&](const uint32_t (&s)[32], uint32_t (&pk)[16], int ch) -> float {
                     const int x = 2 * w + ch;
-                    if (x >= full0 && x <= wr.full1) return fwd_probs32(s, pk, c, ref, true, 0, 0, 0);
-                    if (x >= wr.some0 && x <= some1) return fwd_probs32(s, pk, c, ref, false, ch * 32, lo, hi);
+                    if (x >= full0 && x <= wr.full1) return fwd_probs32<false>(s, pk, pk, c, ref, true, 0, 0, 0);
+                    if (x >= wr.some0 && x <= some1) return fwd_probs32<false>(s, pk, pk, c, ref, false, ch * 32, lo, hi);
 #pragma unroll
                     for (int z = 0; z < 16; ++z) pk[z] = 0u;
                     return 0.f;
@@ -318,10 +318,10 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
                     }
                     tmem_ld32(buf, s);
                     tmem_wait_ld();
-                    tile_sum = fwd_probs32(s, pk0, c, ref, false, 0, lo, hi);
+                    tile_sum = fwd_probs32<false>(s, pk0, pk0, c, ref, false, 0, lo, hi);
                     tmem_ld32(buf + 32, s);
                     tmem_wait_ld();
-                    tile_sum += fwd_probs32(s, pk1, c, ref, false, 32, lo, hi);
+                    tile_sum += fwd_probs32<false>(s, pk1, pk1, c, ref, false, 32, lo, hi);
                 }
                 l += tile_sum;
                 tmem_st16(buf, pk0);

@@ -1,0 +1,46 @@
+"""bf16 shapes whose arithmetic is that of fp32 (head dim 32, long first windows at head dim 64, long second windows):
+only the inputs and the results are rounded to bf16.  Against the oracle in 64 bits."""
+import pytest
+import torch
+
+import simplicial_attention_b200 as sa
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+FORWARD = [
+    # b, n, hq, hk, d, w1, w2
+    (1, 1, 1, 1, 32, 4, 2),
+    (2, 129, 4, 2, 32, 70, 5),        # odd number of sweeps, one row in the last tile
+    (1, 300, 2, 1, 32, 300, 33),      # window from global memory, grouped-query heads
+    (1, 200, 2, 2, 64, 514, 16),      # the shortest long window, longer than the sequence
+    (1, 1100, 1, 1, 64, 1024, 9),     # ring of units
+]
+
+
+@pytest.mark.parametrize("case", FORWARD, ids=lambda c: "b%d_n%d_hq%d_hk%d_d%d_w%d_%d" % c)
+def test_forward(case):
+    b, n, hq, hk, d, w1, w2 = case
+    ins = O.make_inputs(b, n, hq, hk, d, seed=n + w2, dtype=torch.bfloat16)
+    ref, ref_lse = O.two_simplicial_fwd(*[t.double() for t in ins[:5]], w1, w2)
+    out, lse = sa.sa2_forward(*[t.cuda() for t in ins[:5]], w1, w2)
+    assert sa.device_status() == 0
+    # sums of fp32 terms, exp2 to 2^-22 per logit: 1e-5 on logits of up to about 16
+    assert (lse.double().cpu() - ref_lse).abs().max().item() <= 1e-5
+    # half a unit of bf16, and 16-bit probabilities against values of about 4: 2^-17 * 4 * 4 / rms
+    over = (out.double().cpu() - ref).abs() - ref.abs() * 2 ** -8
+    assert over.max().item() <= 2e-4, over.max().item()
+
+
+def test_generation_row():
+    """One new row behind full windows."""
+    w1, w2 = 600, 20
+    ins = O.make_inputs(2, w1, 4, 2, 64, seed=3, dtype=torch.bfloat16)
+    ref, ref_lse = O.two_simplicial_fwd(*[t.double() for t in ins[:5]], w1, w2)
+    q, k1, k2, v1, v2 = [t.cuda() for t in ins[:5]]
+    s = w1 - 1
+    out, lse = sa.sa2_forward(q[:, s:], k1, k2[:, s - w2 + 1:], v1, v2[:, s - w2 + 1:], w1, w2)
+    assert sa.device_status() == 0
+    assert (lse.double().cpu() - ref_lse[:, :, s:]).abs().max().item() <= 1e-5
+    over = (out.double().cpu() - ref[:, s:]).abs() - ref[:, s:].abs() * 2 ** -8
+    assert over.max().item() <= 2e-4, over.max().item()
