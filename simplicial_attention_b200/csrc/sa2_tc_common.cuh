@@ -51,6 +51,9 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volati
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, SA2_WARP_WAIT_SLEEP, prof));
 }
 
+// The lowest reference a row takes: below every finite logit, above -inf, so that logits of -inf weigh 0 and not NaN.
+constexpr float LOWEST_REF = -3.4e38f;
+
 // per-row hand-over between a softmax thread and the output thread of its row:
 // [group][sweep parity][128] final reference of the sweep, then [group][128] denominator and
 // [group][128] the reference it is expressed against
@@ -81,18 +84,17 @@ __device__ __forceinline__ float fwd_probs32(const uint32_t (&s)[32], uint32_t (
             put(x, ex2(a0), ex2(a1));
         }
     } else {
-        // Valid columns are the integers in (lo, hi]: |col - mid| <= half, and an invalid column is at least
-        // half + 1 away, so saturate(half + 1 - |col - mid|) is exactly 1 or 0: two FADDs and an FMUL on the
-        // FMA pipe instead of two compares and a select on the (half as wide) ALU pipe.  The exponent is
-        // clamped so that a masked-out logit far above the reference cannot produce inf * 0; a clamped
-        // valid logit still trips the slow path.
-        const float mid = 0.5f * (float)(lo + 1 + hi), hwp = 0.5f * (float)(hi - lo - 1) + 1.f;
+        // Valid columns are the integers in (lo, hi]: 2048 (half + 1/2 - |col - mid|) is at least 1024 inside and at most
+        // -1024 outside, so the minimum with it leaves the exponents of valid cells alone and makes P exactly 0 elsewhere,
+        // whatever S is there (FMA pipe instead of compares and selects on the ALU pipe; all values are exact).  A valid
+        // NaN, or a logit far above the reference, gives inf and trips the slow path.
+        const float mid = 1024.f * (float)(lo + 1 + hi) - 2048.f * (float)col0, half = 1024.f * (float)(hi - lo);
+        const uint64_t c2 = f2_pack(c, c), nref2 = f2_pack(-ref, -ref);
 #pragma unroll
         for (int x = 0; x < 32; x += 2) {
-            const float v0 = __saturatef(hwp - fabsf((float)(col0 + x) - mid));
-            const float v1 = __saturatef(hwp - fabsf((float)(col0 + x + 1) - mid));
-            put(x, ex2(fminf(fmaf(__uint_as_float(s[x]), c, -ref), 100.f)) * v0,
-                ex2(fminf(fmaf(__uint_as_float(s[x + 1]), c, -ref), 100.f)) * v1);
+            float a0, a1;
+            f2_unpack(f2_fma(f2_pack(s[x], s[x + 1]), c2, nref2), a0, a1);
+            put(x, ex2(fminf(a0, half - fabsf(2048.f * x - mid))), ex2(fminf(a1, half - fabsf(2048.f * (x + 1) - mid))));
         }
     }
     return sum0 + sum1;

@@ -292,12 +292,12 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
 #pragma unroll
                         for (int x = 0; x < 32; ++x) {
                             const int col = ch * 32 + x;
-                            if (col > lo && col <= hi) mx = fmaxf(mx, __uint_as_float(s[x]));
+                            if (col > lo && col <= hi) mx = fmaxf(mx, __uint_as_float(s[x]) * c);
                         }
                     }
                     float f = 1.f;
                     if (exceed) {
-                        const float nref = mx * c;
+                        const float nref = fmaxf(mx, LOWEST_REF);
                         f = ex2(ref - nref);                       // 0 when ref was -inf
                         l *= f;
                         ref = nref;

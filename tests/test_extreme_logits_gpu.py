@@ -1,4 +1,4 @@
-"""Logits at the ends of their range: -inf beside finite ones."""
+"""Logits at the ends of their range: -inf and NaN beside finite ones, steep climbs, negative and zero scales."""
 import pytest
 import torch
 
@@ -52,3 +52,46 @@ def test_rising_logits_with_large_values_fp32(d):
     out, lse = sa.sa2_forward(q, k1, k2, v1, v2, w1, w2)
     ref = _reference(q, k1, k2, v1, v2, w1, w2)
     assert (out - ref).abs().max().item() <= 1e-4 * ref.abs().max().item()
+
+
+BF16 = [(32, 100), (64, 100), (64, 600), (128, 100)]
+
+
+@pytest.mark.parametrize("d,w1", BF16)
+def test_logits_of_minus_infinity_weigh_nothing_bf16(d, w1):
+    ins = _operands(d, torch.bfloat16)
+    for t in ins[:3]:
+        t.abs_()
+    ins[1][:, 60:155] = -3e38
+    out, lse = sa.sa2_forward(*ins, w1, 4)
+    ref = _reference(*ins, w1, 4)
+    assert sa.device_status() == 0
+    seen = ref.isfinite().all(-1).all(-1)[0]
+    assert seen.sum() >= 150 and lse[:, :, seen].isfinite().all()
+    assert (out[:, seen].double() - ref[:, seen]).norm() <= 1e-2 * ref[:, seen].norm()
+
+
+@pytest.mark.parametrize("d,w1", BF16)
+def test_nan_stays_where_it_is_seen_bf16(d, w1):
+    """A NaN key reaches the rows whose window holds it and no others."""
+    ins = _operands(d, torch.bfloat16)
+    ins[1][:, 70, 1] = float("nan")
+    out, lse = sa.sa2_forward(*ins, w1, 4)
+    assert sa.device_status() == 0
+    want = torch.zeros(200, dtype=torch.bool, device="cuda")
+    want[70:70 + w1] = True
+    assert out[0, :, 0].isfinite().all() and lse[0, 0].isfinite().all()
+    assert torch.equal(out[0, :, 1].isnan().all(-1), want) and torch.equal(out[0, :, 1].isnan().any(-1), want)
+
+
+@pytest.mark.parametrize("scale", [-0.125, -3.])
+@pytest.mark.parametrize("d,w1", BF16)
+def test_negative_scale_bf16(d, w1, scale):
+    """Rounded products put a logit off by at most |scale| * 2^-9 * sum_c |q k1 k2|, a sum of about d / 2 and below d here;
+    their root mean square, |scale| * 2^-9 * sqrt(d / 3) <= 0.04, bounds the output's relative error with room."""
+    ins = _operands(d, torch.bfloat16)
+    out, lse = sa.sa2_forward(*ins, w1, 4, scale=scale)
+    want, want_lse = sa.sa2_forward(*ins, w1, 4, scale=scale, kernel="simt")
+    assert sa.device_status() == 0
+    assert (lse - want_lse).abs().max().item() <= -scale * 2 ** -9 * d
+    assert (out.float() - want.float()).norm() <= (1e-2 if scale > -1 else 0.1) * want.float().norm()
