@@ -178,7 +178,7 @@ int sa2_kernel_launches(const sa2_shape *shape, int backward) {
     const sa2_shape s = clamped(*shape);
     const bool tc_ok = backward ? sa2::tc::bwd_supported(s) : sa2::tc::fwd_supported(s);
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
-    if (tc_ok && s.kernel != SA2_KERNEL_SIMT) return sa2::tc::launches(s, backward != 0);
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !(backward && !sa2::tc::bwd_scale_ok(s))) return sa2::tc::launches(s, backward != 0);
     return backward ? 2 : 1;   // SIMT: row sums + all gradients
 }
 
@@ -234,7 +234,7 @@ int sa2_bwd(const sa2_bwd_args *a) {
 
     const bool tc_ok = sa2::tc::bwd_supported(s) && sa2::tc::bwd_addressable(p);
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
-    if (tc_ok && s.kernel != SA2_KERNEL_SIMT) {
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT && sa2::tc::bwd_scale_ok(s)) {
         size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
         delta = (delta + 255) & ~(size_t)255;
         return sa2::tc::bwd(p, s, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);

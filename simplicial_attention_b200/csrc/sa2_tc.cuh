@@ -29,6 +29,8 @@ inline bool fwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 inline bool fwd_split(const sa2_shape &s) { return s.d == 32 || (s.d == 64 && s.w1 > 513); }
 // So does the tensor-core backward.
 inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
+// A scale of (nearly) zero goes to the fp32 kernels: dK1/dV1 folds lse / scale into its products.
+inline bool bwd_scale_ok(const sa2_shape &s) { return fabsf(s.scale) >= 1e-20f; }
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // CTAs sharing one query tile in the dQ/dK2/dV2 kernel: splits of the window (head dim 128 walks it in one CTA) times
 // splits of the offsets.  A CTA costs ~12000 cycles of set-up, loads, slab and its share of the reduction, a 64-key unit

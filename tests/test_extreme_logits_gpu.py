@@ -95,3 +95,14 @@ def test_negative_scale_bf16(d, w1, scale):
     assert sa.device_status() == 0
     assert (lse - want_lse).abs().max().item() <= -scale * 2 ** -9 * d
     assert (out.float() - want.float()).norm() <= (1e-2 if scale > -1 else 0.1) * want.float().norm()
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_zero_scale_bf16(d):
+    """Uniform weights: dq, dk1 and dk2 are zero, dv1 and dv2 are those of the fp32 kernels."""
+    ins = _operands(d, torch.bfloat16)
+    out, lse = sa.sa2_forward(*ins, 100, 4, scale=0.)
+    got, want = (sa.sa2_backward(*ins, out, lse, ins[0], 100, 4, scale=0., kernel=k) for k in ("auto", "simt"))
+    assert sa.device_status() == 0
+    for a, b in zip(got, want):
+        assert a.isfinite().all() and (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
