@@ -162,6 +162,7 @@ int sa2_bwd_static_scratch(const sa2_bwd_args *args);
  * Number of kernel launches sa2_fwd (backward == 0) or sa2_bwd (backward != 0)
  * issues for this shape, or -1 for a shape they would reject.  The reference
  * launches 1 forward and 4 backward kernels plus 5 memsets (:749,834,868,938,972,853-857).
+ * (The backward's number is that of gradients in the dtype of the operands.)
  */
 int sa2_kernel_launches(const sa2_shape *shape, int backward);
 

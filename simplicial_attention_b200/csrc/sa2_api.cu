@@ -234,7 +234,9 @@ int sa2_bwd(const sa2_bwd_args *a) {
 
     const bool tc_ok = sa2::tc::bwd_supported(s) && sa2::tc::bwd_addressable(p);
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
-    if (tc_ok && s.kernel != SA2_KERNEL_SIMT && sa2::tc::bwd_scale_ok(s)) {
+    // (fp32 gradients at head dim 32 show the last bits, which AUTO leaves to the fp32 kernels)
+    const bool exact = s.kernel == SA2_KERNEL_AUTO && s.d == 32 && a->grad_dtype == SA2_F32;
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !exact && sa2::tc::bwd_scale_ok(s)) {
         size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
         delta = (delta + 255) & ~(size_t)255;
         return sa2::tc::bwd(p, s, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);

@@ -27,7 +27,8 @@ inline bool fwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 // that way.  Relative error of the output against 64 bits 1.57e-3 to 1.67e-3, as with fp32 arithmetic (2.2e-3 to 3.2e-3 with
 // rounded operands); of the logsumexp 2e-6, absolute (3e-3 to 1.6e-2).
 inline bool fwd_split(const sa2_shape &s) { return s.d == 32 || (s.d == 64 && s.w1 > 513); }
-// So does the tensor-core backward.
+// So does the tensor-core backward.  Head dim 32 keeps A_e, B_e, P and G to 16 bits there (bwd_split); its gradients in bf16
+// are then off by what their own rounding costs, as with fp32 arithmetic.
 inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 // A scale of (nearly) zero goes to the fp32 kernels: dK1/dV1 folds lse / scale into its products.
 inline bool bwd_scale_ok(const sa2_shape &s) { return fabsf(s.scale) >= 1e-20f; }

@@ -3,9 +3,8 @@
 //
 // One CTA owns 128 rows j of K1/V1 of one (batch, kv head); the tile stays in
 // shared memory and dK1/dV1 for those rows accumulate in TMEM for the whole
-// kernel, so nothing is reduced across CTAs and there are no atomics.  The CTA
-// walks over every (query head of the group, query tile I, offset e) that can
-// see its keys.  Per step the builder warps form
+// kernel, without atomics.  The CTA walks over every (query head of the group,
+// query tile I, offset e) that can see its keys, or over its share of them.  Per step the builder warps form
 //     A_e[i,:] = q_i * k2_{i-e}      B_e[i,:] = dO_i * v2_{i-e}      (bf16)
 // and the tensor cores compute, in units of 64 query columns,
 //     S^T  = K1 A_e^T       dP^T = V1 B_e^T          (rows j, columns i)
@@ -25,7 +24,7 @@
 // products (dV1, dK1: one issuer, which keeps the summation order fixed); 1 TMEM owner and issuer of S^T; 2 issuer of
 // dP^T; 3 idle; 4-7 and 8-11 compute groups of the even and the odd units; 12-19 builders, two threads per query row.
 // TMEM columns: buffer x -> S^T [128x, +64), dP^T [128x+64, +64), three buffers in flight; P^T / G^T (bf16) overwrite the
-// first half of the S^T / dP^T columns they come from, so a buffer is busy until the second products of its unit are
+// first half of the S^T / dP^T columns they come from (at head dim 32, with their rests, all of them), so a buffer is busy until the second products of its unit are
 // done; dK1 [384,448); dV1 [448,512).
 //
 // Bound: the exponent passes of the two groups (512 MUFU cycles per unit and scheduler) next to ~740 cycles of products
@@ -131,6 +130,14 @@ __device__ __forceinline__ uint4 split3_bf16(float x) {
     return v;
 }
 
+// Head dim 32 leaves half of every 128-byte operand row free: the products q * k2 and dO * v2 are stored as a bf16 value
+// (channels 0-31) and its bf16 rest (channels 32-63), which together are exact, and P^T and G^T likewise over the columns of
+// S^T and dP^T.  The first products add the rests of A_e / B_e as two more K steps; the second ones take both halves of
+// the row as N = 64 columns, whose halves the store adds.  Gradients in bf16 are as far from 64 bits as those of the fp32
+// kernels (1.5e-3 to 4.3e-3; 2.9e-3 to 5.9e-3 with rounded operands).  b4 n4096 h8 w512/32: dK1/dV1 1.07 -> 1.64 ms against
+// rounded operands, dQ/dK2/dV2 1.33 -> 1.94; 19.7 and 40.0 on the fp32 kernels.
+template <int D> constexpr bool bwd_split = D == 32;
+
 template <int D>
 __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g, const CUtensorMap *mapK2, const CUtensorMap *mapV2,
                                            uint8_t *sAB, uint8_t *sStat, uint8_t *sOnes, uint8_t *sWin,
@@ -210,7 +217,7 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
             const uint8_t *wk = sWin + wr * 128, *wv = wk + BK1_WIN_ROWS * 128;
 #pragma unroll
             for (int cc = 0; cc < NC; ++cc) {
-                uint4 a = make_uint4(0, 0, 0, 0), bb = make_uint4(0, 0, 0, 0);
+                uint4 a = make_uint4(0, 0, 0, 0), bb = make_uint4(0, 0, 0, 0), ar = a, br = a;
                 if (ok) {
                     const uint4 kv = win ? *reinterpret_cast<const uint4 *>(wk + (((c0 + cc) ^ (wr & 7)) << 4))
                                          : *reinterpret_cast<const uint4 *>(kp2 + cc * 8);
@@ -220,9 +227,14 @@ __device__ __forceinline__ int bk1_builder(const BwdParams &P, const Bk1Geom &g,
                     a.z = mul_bf16x2(qv[cc].z, kv.z); a.w = mul_bf16x2(qv[cc].w, kv.w);
                     bb.x = mul_bf16x2(dv[cc].x, vv.x); bb.y = mul_bf16x2(dv[cc].y, vv.y);
                     bb.z = mul_bf16x2(dv[cc].z, vv.z); bb.w = mul_bf16x2(dv[cc].w, vv.w);
+                    if constexpr (bwd_split<D>) { ar = mul_rest_bf16x8(qv[cc], kv, a); br = mul_rest_bf16x8(dv[cc], vv, bb); }
                 }
                 *reinterpret_cast<uint4 *>(dA + sw128_offset(r, c0 + cc)) = a;
                 *reinterpret_cast<uint4 *>(dB + sw128_offset(r, c0 + cc)) = bb;
+                if constexpr (bwd_split<D>) {
+                    *reinterpret_cast<uint4 *>(dA + sw128_offset(r, 4 + c0 + cc)) = ar;
+                    *reinterpret_cast<uint4 *>(dB + sw128_offset(r, 4 + c0 + cc)) = br;
+                }
             }
             fence_proxy_async_smem();
             mbar_arrive(&bars[BK1_AB_FULL + stage]);
@@ -261,6 +273,10 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
                 if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k) mma_ss(d, dT + 2 * k, a + 2 * k, IDESC_F, k > 0 ? 1u : 0u);
+                if constexpr (bwd_split<D>) {
+#pragma unroll
+                    for (int k = 0; k < D / 16; ++k) mma_ss(d, dT + 2 * k, a + 4 + 2 * k, IDESC_F, 1u);
+                }
                 mma_ss(d, dOnes, st, IDESC_F, 1u);                // - lse2_i / c, or - D_i
                 tc_commit(&bars[BK1_S_FULL + buf]);
                 }
@@ -274,7 +290,10 @@ __device__ __forceinline__ int bk1_mma_first(const KernelParams &kp, const Bk1Ge
 // ---------------------------------------------------------------- issuer of dV1, dK1 (warp 0)
 template <int D>
 __device__ __forceinline__ int bk1_mma_second(const Bk1Geom &g, uint32_t tmem, uint8_t *sAB, uint64_t *bars, volatile int *abort_flag) {
-    constexpr uint32_t IDESC_G = idesc_bf16(128, D, false, true);    // B operand MN-major
+    constexpr bool SPLIT = bwd_split<D>;
+    constexpr uint32_t IDESC_G = idesc_bf16(128, SPLIT ? 2 * D : D, false, true);    // B operand MN-major
+    // P^T / G^T of keys [16 k, +16): side by side, or with their rests behind every 32 keys
+    auto cols = [](int k) { return SPLIT ? (k >> 1) * 32 + (k & 1) * 8 : 8 * k; };
     const uint64_t dAB = smem_desc_sw128(smem_u32(sAB));
     int buf = 0, use = 0;
     for (int s = 0; s < g.total; ++s) {
@@ -288,9 +307,15 @@ __device__ __forceinline__ int bk1_mma_second(const Bk1Geom &g, uint32_t tmem, u
             const uint32_t first = (s > 0 || half > 0) ? 1u : 0u;
             if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) mma_ts(tmem + 448, tp + 8 * k, bq + 128 * k, IDESC_G, k > 0 ? 1u : first);
+            for (int k = 0; k < 4; ++k) mma_ts(tmem + 448, tp + cols(k), bq + 128 * k, IDESC_G, k > 0 ? 1u : first);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) mma_ts(tmem + 384, tg + 8 * k, a + 128 * k, IDESC_G, k > 0 ? 1u : first);
+            for (int k = 0; k < 4; ++k) mma_ts(tmem + 384, tg + cols(k), a + 128 * k, IDESC_G, k > 0 ? 1u : first);
+            if constexpr (SPLIT) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma_ts(tmem + 448, tp + 16 + cols(k), bq + 128 * k, IDESC_G, 1u);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma_ts(tmem + 384, tg + 16 + cols(k), a + 128 * k, IDESC_G, 1u);
+            }
             tc_commit(&bars[BK1_G_DONE + buf]);
             if (half == 1) tc_commit(&bars[BK1_AB_EMPTY + stage]);
             }
@@ -331,7 +356,8 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
                 const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 63);
 #pragma unroll
                 for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t sv[32], dv[32], pk[16], gk[16];
+                    constexpr bool SPLIT = bwd_split<D>;
+                    uint32_t sv[32], dv[32], pk[16], gk[16], pr[SPLIT ? 16 : 1], gr[SPLIT ? 16 : 1];
                     tmem_ld32(buf + ch * 32, sv);
                     tmem_ld32(buf + 64 + ch * 32, dv);
                     tmem_wait_ld();
@@ -342,6 +368,10 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
                         f2_unpack(f2_mul(f2_pack(p0, p1), f2_pack(dv[x], dv[x + 1])), g0, g1);
                         pk[x >> 1] = pack_bf16(p0, p1);
                         gk[x >> 1] = pack_bf16(g0, g1);
+                        if constexpr (SPLIT) {
+                            pr[x >> 1] = pack_rest(p0, p1, pk[x >> 1]);
+                            gr[x >> 1] = pack_rest(g0, g1, gk[x >> 1]);
+                        }
                     };
                     if (full) {
 #pragma unroll
@@ -364,8 +394,15 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
                         }
                     }
                     // over columns of S^T / dP^T that this thread has already read
-                    tmem_st16(buf + ch * 16, pk);
-                    tmem_st16(buf + 64 + ch * 16, gk);
+                    if constexpr (SPLIT) {
+                        tmem_st16(buf + ch * 32, pk);
+                        tmem_st16(buf + ch * 32 + 16, pr);
+                        tmem_st16(buf + 64 + ch * 32, gk);
+                        tmem_st16(buf + 64 + ch * 32 + 16, gr);
+                    } else {
+                        tmem_st16(buf + ch * 16, pk);
+                        tmem_st16(buf + 64 + ch * 16, gk);
+                    }
                 }
                 tmem_wait_st();
                 tc_fence_before();
@@ -387,6 +424,13 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
         uint32_t w[32];
         tmem_ld32(lane_addr + 384 + half * 64 + hf * 32, w);
         tmem_wait_ld();
+        if constexpr (bwd_split<D>) {
+            uint32_t rest[32];
+            tmem_ld32(lane_addr + 384 + half * 64 + 32, rest);
+            tmem_wait_ld();
+#pragma unroll
+            for (int x = 0; x < 32; ++x) w[x] = __float_as_uint(__uint_as_float(w[x]) + __uint_as_float(rest[x]));
+        }
         if (P.ce > 1 && jv) {
             float *row = P.part + (((((size_t)(blockIdx.x % P.ce) * kp.b + b) * kp.nk1 + j) * kp.hk + hk) * 2 + half) * D + hf * 32;
 #pragma unroll

@@ -36,8 +36,8 @@
 // and fold U of the last one into dQ / dK2, 16-19 do the same with B_e, W and dV2; at head dim 128 (512 threads) 12-15 do
 // both (a second fold group and a third S / dP buffer there: 8.45 -> 9.2 ms on b1 n16384 h16 w512/32).
 // TMEM columns: S / dP buffer x -> S/P [128x, 128x+64), dP/G [128x+64, 128x+128); P and G (bf16, 16 columns per
-// 32 keys) overwrite the first half of the S and dP columns of the same keys - columns that the writing compute
-// group has itself read - so a buffer is busy from the issue of S / dP until the U / W products of its unit are
+// 32 keys; at head dim 32 their rests in the next 16) overwrite the S and dP columns of the same keys - columns that the
+// writing compute group has itself read - so a buffer is busy from the issue of S / dP until the U / W products of its unit are
 // done.  Up to head dim 64 three such buffers are in flight (issue, compute and U / W of different units overlap) and
 // there is one U / W accumulator pair [384, 512), which the fold groups read into registers before the next sweep's
 // first product; head dim 128 has two buffers and U / W per sweep parity at [256 + 128p, +128).
@@ -45,7 +45,8 @@
 // Bound, up to head dim 64: shared memory.  A unit's products fetch 512 cycles' worth of operands at 128 B/clk (S and dP:
 // N = 64, so A is read again for every unit), the folds and the operand rows a further ~400, and everything that
 // goes through shared memory - shuffles included - waits behind the tensor cores' fetches.  b4 n4096 h8 w512/32 takes
-// ~1350 cycles a unit: 1.97 -> 1.58 ms at head dim 64, 30 -> 1.27 ms at 32 (the fp32 kernels before).  Measured and not
+// ~1350 cycles a unit: 1.97 -> 1.58 ms at head dim 64, 40 -> 1.94 ms at 32 (the fp32 kernels before; 1.33 with A_e, B_e, P and
+// G rounded to bf16: see bwd_split).  Measured and not
 // kept: A_e and B_e in TMEM, double-buffered, which leaves two S / dP buffers (1.74 ms); k2 / v2 rows moved from lane to
 // lane by shuffles instead of a row per lane from memory (1.70 ms).  Head dim 128 (two buffers, S and dP formed in
 // both channel halves): 11.7 -> 8.5 ms on b1 n16384 h16; the chain S / dP -> P / G -> U / W of two buffers paces it.
@@ -228,6 +229,10 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
                 const uint64_t t = dT + (uint64_t)((w * 8192) >> 4);       // unit w: rows [64 w, +64) of the resident tiles
 #pragma unroll
                 for (int k = 0; k < C::KSTEPS; ++k) mma_ss(d, dA + 2 * k, t + 2 * k, IDESC_F, k > 0 ? 1u : 0u);
+                if constexpr (bwd_split<D>) {             // the rests of A_e / B_e: channels 32-63 of their rows
+#pragma unroll
+                    for (int k = 0; k < C::KSTEPS; ++k) mma_ss(d, dA + 4 + 2 * k, t + 2 * k, IDESC_F, 1u);
+                }
             } else {
                 const uint64_t t = dT + (uint64_t)((slot * 2 * C::UBLK) >> 4);
 #pragma unroll
@@ -326,12 +331,24 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
                 mma_ts(tu, a + 72, kt + 128, IDESC_G, 1u);
                 mma_ts(tu, a + 96, kt + 256, IDESC_G, 1u);
                 mma_ts(tu, a + 104, kt + 384, IDESC_G, 1u);
+                if constexpr (bwd_split<D>) {                       // the rests of G, behind it
+                    mma_ts(tu, a + 80, kt, IDESC_G, 1u);
+                    mma_ts(tu, a + 88, kt + 128, IDESC_G, 1u);
+                    mma_ts(tu, a + 112, kt + 256, IDESC_G, 1u);
+                    mma_ts(tu, a + 120, kt + 384, IDESC_G, 1u);
+                }
             }
             if (part != 0) {
                 mma_ts(tw, a, vt, IDESC_G, acc);                    // W += P V1
                 mma_ts(tw, a + 8, vt + 128, IDESC_G, 1u);
                 mma_ts(tw, a + 32, vt + 256, IDESC_G, 1u);
                 mma_ts(tw, a + 40, vt + 384, IDESC_G, 1u);
+                if constexpr (bwd_split<D>) {
+                    mma_ts(tw, a + 16, vt, IDESC_G, 1u);
+                    mma_ts(tw, a + 24, vt + 128, IDESC_G, 1u);
+                    mma_ts(tw, a + 48, vt + 256, IDESC_G, 1u);
+                    mma_ts(tw, a + 56, vt + 384, IDESC_G, 1u);
+                }
             }
             tc_commit(&bars[BQ_G_DONE + buf]);
             if constexpr (D == 128) tc_commit(&bars[BQ_KV_FREE + slot]);
@@ -347,11 +364,18 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
 // ---------------------------------------------------------------- compute (warps 4-7; head dim 64: and 8-11): P and G
 // P and G = P (dP - D) of two columns, as packed bf16.  The kernel's issue slots count here (728 warp instructions a unit
 // and scheduler before the packed arithmetic of this and of the folds), so two columns share an instruction.
-__device__ __forceinline__ void pg_pair(float p0, float p1, uint32_t dp0, uint32_t dp1, uint64_t ndl2, uint32_t &pp, uint32_t &gg) {
+// SPLIT: and what the rounding left of each.
+template <bool SPLIT>
+__device__ __forceinline__ void pg_pair(float p0, float p1, uint32_t dp0, uint32_t dp1, uint64_t ndl2, uint32_t &pp, uint32_t &gg, uint32_t &pr,
+                                        uint32_t &gr) {
     float g0, g1;
     f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(dp0, dp1), ndl2)), g0, g1);
     pp = pack_bf16(p0, p1);
     gg = pack_bf16(g0, g1);
+    if constexpr (SPLIT) {
+        pr = pack_rest(p0, p1, pp);
+        gr = pack_rest(g0, g1, gg);
+    }
 }
 // Head dim 64: group cg forms columns [32 cg, +32) of every unit, which halves the time between S / dP and P / G.
 template <int D>
@@ -391,11 +415,12 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                 const bool full = __all_sync(0xffffffffu, lo < 0 && hi >= 63);
                 {
                     const int ch = cg;
-                    uint32_t sv[32], dv[32], pp[16], gg[16];
+                    constexpr bool SPLIT = bwd_split<D>;
+                    uint32_t sv[32], dv[32], pp[16], gg[16], pr[SPLIT ? 16 : 1], gr[SPLIT ? 16 : 1];
                     // no row of this warp has a valid column among these 32: P = G = 0 without reading S / dP
                     if (__all_sync(0xffffffffu, hi < ch * 32 || lo >= ch * 32 + 31)) {
 #pragma unroll
-                        for (int x = 0; x < 16; ++x) { pp[x] = 0u; gg[x] = 0u; }
+                        for (int x = 0; x < 16; ++x) { pp[x] = 0u; gg[x] = 0u; pr[SPLIT ? x : 0] = 0u; gr[SPLIT ? x : 0] = 0u; }
                     } else {
 #ifdef SA2_PROF
                     const long long seg_t0 = clock64();
@@ -407,12 +432,15 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                     const long long seg_t1 = clock64();
                     seg_ld += seg_t1 - seg_t0;
 #endif
+                    auto pg = [&](int x, float a0, float a1) {
+                        pg_pair<SPLIT>(ex2(a0), ex2(a1), dv[x], dv[x + 1], ndl2, pp[x >> 1], gg[x >> 1], pr[SPLIT ? x >> 1 : 0], gr[SPLIT ? x >> 1 : 0]);
+                    };
                     if (full) {
 #pragma unroll
                         for (int x = 0; x < 32; x += 2) {
                             float a0, a1;
                             f2_unpack(f2_fma(f2_pack(sv[x], sv[x + 1]), c2, nlse2), a0, a1);
-                            pg_pair(ex2(a0), ex2(a1), dv[x], dv[x + 1], ndl2, pp[x >> 1], gg[x >> 1]);
+                            pg(x, a0, a1);
                         }
                     } else {
                         // valid columns are the integers in (lo, hi]: 2048 (half + 1/2 - |col - mid|) is at least 1024
@@ -426,7 +454,7 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                             f2_unpack(f2_fma(f2_pack(sv[x], sv[x + 1]), c2, nlse2), a0, a1);
                             a0 = fminf(a0, half - fabsf(2048.f * x - mid));
                             a1 = fminf(a1, half - fabsf(2048.f * (x + 1) - mid));
-                            pg_pair(ex2(a0), ex2(a1), dv[x], dv[x + 1], ndl2, pp[x >> 1], gg[x >> 1]);
+                            pg(x, a0, a1);
                         }
                     }
 #ifdef SA2_PROF
@@ -437,6 +465,10 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                     // other columns of the buffer may still be unread by the other compute group)
                     tmem_st16(lane_addr + buf * 128 + ch * 32, pp);
                     tmem_st16(lane_addr + buf * 128 + 64 + ch * 32, gg);
+                    if constexpr (SPLIT) {
+                        tmem_st16(lane_addr + buf * 128 + ch * 32 + 16, pr);
+                        tmem_st16(lane_addr + buf * 128 + 64 + ch * 32 + 16, gr);
+                    }
                 }
 #ifdef SA2_PROF
                 const long long seg_t2 = clock64();
@@ -531,17 +563,24 @@ __device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, 
     auto build = [&](int e) -> bool {
         bool ok;
         const uint4 *py = yrow(e, ok);
-        uint4 y[NC];
+        uint4 y[NC], rest[bwd_split<D> ? NC : 1];
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc) y[cc] = ok ? __ldg(py + cc) : zero;
 #pragma unroll
-        for (int cc = 0; cc < NC; ++cc) y[cc] = ok ? mul_bf16x8(xr[cc], y[cc]) : zero;
+        for (int cc = 0; cc < NC; ++cc) {
+            const uint4 hi = ok ? mul_bf16x8(xr[cc], y[cc]) : zero;
+            if constexpr (bwd_split<D>) rest[cc] = ok ? mul_rest_bf16x8(xr[cc], y[cc], hi) : zero;
+            y[cc] = hi;
+        }
         if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY + WHICH], (e - 1) & 1, abort_flag, 3)) return false;
 #ifdef SA2_PROF
         const long long seg_t0 = clock64();
 #endif
 #pragma unroll
-        for (int cc = 0; cc < NC; ++cc) *reinterpret_cast<uint4 *>(sOp + sw128_offset(r, cc)) = y[cc];
+        for (int cc = 0; cc < NC; ++cc) {
+            *reinterpret_cast<uint4 *>(sOp + sw128_offset(r, cc)) = y[cc];
+            if constexpr (bwd_split<D>) *reinterpret_cast<uint4 *>(sOp + sw128_offset(r, 4 + cc)) = rest[cc];
+        }
         fence_proxy_async_smem();
         mbar_arrive(&bars[BQ_AB_FULL + WHICH]);
 #ifdef SA2_PROF
@@ -641,7 +680,6 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     const __nv_bfloat16 *qrow = reinterpret_cast<const __nv_bfloat16 *>(kp.q.p) + elem_off(kp.q, b, row_ok ? i : 0, h) + c0;
     const __nv_bfloat16 *dorow = reinterpret_cast<const __nv_bfloat16 *>(kp.dout.p) + elem_off(kp.dout, b, row_ok ? i : 0, h) + c0;
     const __nv_bfloat16 *k2 = reinterpret_cast<const __nv_bfloat16 *>(kp.k2.p) + c0;
-    const __nv_bfloat16 *v2 = reinterpret_cast<const __nv_bfloat16 *>(kp.v2.p) + c0;
 
 #ifdef SA2_PROF
     long long seg_build = 0, seg_drain = 0;           // cycles after the waits of a build and of a fold

@@ -42,6 +42,10 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     return *reinterpret_cast<uint32_t *>(&r);
 }
 
+__device__ __forceinline__ uint4 mul_rest_bf16x8(const uint4 &a, const uint4 &b, const uint4 &hi) {
+    return make_uint4(mul_rest_bf16x2(a.x, b.x, hi.x), mul_rest_bf16x2(a.y, b.y, hi.y), mul_rest_bf16x2(a.z, b.z, hi.z), mul_rest_bf16x2(a.w, b.w, hi.w));
+}
+
 #ifndef SA2_WARP_WAIT_SLEEP
 #define SA2_WARP_WAIT_SLEEP 64
 #endif

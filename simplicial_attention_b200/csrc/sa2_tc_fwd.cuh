@@ -444,10 +444,7 @@ __device__ __forceinline__ int fwd_output(const FwdParams &P, const FwdGeom &g, 
             if (ok) kv = staged ? *reinterpret_cast<const uint4 *>(sWin + sw128_offset(wr, cc)) : __ldg(reinterpret_cast<const uint4 *>(krow + cc * 8));
             a[cc].x = mul_bf16x2(qv[cc].x, kv.x); a[cc].y = mul_bf16x2(qv[cc].y, kv.y);
             a[cc].z = mul_bf16x2(qv[cc].z, kv.z); a[cc].w = mul_bf16x2(qv[cc].w, kv.w);
-            if constexpr (SPLIT) {
-                rest[cc].x = mul_rest_bf16x2(qv[cc].x, kv.x, a[cc].x); rest[cc].y = mul_rest_bf16x2(qv[cc].y, kv.y, a[cc].y);
-                rest[cc].z = mul_rest_bf16x2(qv[cc].z, kv.z, a[cc].z); rest[cc].w = mul_rest_bf16x2(qv[cc].w, kv.w, a[cc].w);
-            }
+            if constexpr (SPLIT) rest[cc] = mul_rest_bf16x8(qv[cc], kv, a[cc]);
         }
         if (bar && !warp_wait(bar, parity, abort_flag, 1)) return false;
 #pragma unroll

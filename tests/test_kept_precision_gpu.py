@@ -44,3 +44,32 @@ def test_generation_row():
     assert (lse.double().cpu() - ref_lse[:, :, s:]).abs().max().item() <= 1e-5
     over = (out.double().cpu() - ref[:, s:]).abs() - ref[:, s:].abs() * 2 ** -8
     assert over.max().item() <= 2e-4, over.max().item()
+
+
+BACKWARD = [
+    # b, n, hq, hk, w1, w2
+    (1, 40, 1, 1, 40, 40),            # one tile, offset ranges that start past the first rows
+    (2, 129, 4, 2, 70, 5),            # one row in the last tile
+    (1, 300, 4, 1, 200, 33),          # four heads per key head, second-key rows from global memory
+    (1, 700, 2, 2, 512, 9),           # window splits
+]
+
+
+@pytest.mark.parametrize("case", BACKWARD, ids=lambda c: "b%d_n%d_hq%d_hk%d_w%d_%d" % c)
+def test_backward_head_dim_32(case):
+    """Gradients of bf16 operands in bf16, next to those of the fp32 kernels for the same saved output: both are off
+    from 64 bits by their rounding to bf16 and by that of the saved output, and by nothing else that shows."""
+    b, n, hq, hk, w1, w2 = case
+    ins = O.make_inputs(b, n, hq, hk, 32, seed=n + w2, dtype=torch.bfloat16)
+    ref = O.two_simplicial_fwd_bwd(*[t.double() for t in ins], w1, w2, dtype=torch.float64)
+    q, k1, k2, v1, v2, do = [t.cuda() for t in ins]
+    out, lse = sa.sa2_forward(q, k1, k2, v1, v2, w1, w2, kernel="simt")
+    got, base = (sa.sa2_backward(q, k1, k2, v1, v2, out, lse, do, w1, w2, kernel=k) for k in ("auto", "simt"))
+    fine, base_fine = (sa.sa2_backward(q, k1, k2, v1, v2, out, lse, do, w1, w2, kernel=k, grad_dtype=torch.float32) for k in ("tcgen05", "simt"))
+    assert sa.device_status() == 0
+    for i, name in enumerate(("dq", "dk1", "dk2", "dv1", "dv2")):
+        r = ref[name]
+        err = lambda x: ((x.double().cpu() - r).norm() / r.norm()).item()
+        assert err(got[i]) <= 1.01 * err(base[i]) + 2e-5, (name, err(got[i]), err(base[i]))
+        # 16-bit P and G in fp32 sums
+        assert (fine[i] - base_fine[i]).norm() <= 2e-5 * base_fine[i].norm(), name
