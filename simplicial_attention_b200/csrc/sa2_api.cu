@@ -178,7 +178,8 @@ int sa2_kernel_launches(const sa2_shape *shape, int backward) {
     const sa2_shape s = clamped(*shape);
     const bool tc_ok = backward ? sa2::tc::bwd_supported(s) : sa2::tc::fwd_supported(s);
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
-    if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !(backward && !sa2::tc::bwd_scale_ok(s))) return sa2::tc::launches(s, backward != 0);
+    if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !(backward && !sa2::tc::bwd_scale_ok(s)))
+        return sa2::tc::launches(s, backward != 0, shape->w2);
     return backward ? 2 : 1;   // SIMT: row sums + all gradients
 }
 
@@ -187,7 +188,7 @@ size_t sa2_bwd_workspace_bytes(const sa2_shape *shape) {
     const sa2_shape s = clamped(*shape);
     size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
     delta = (delta + 255) & ~(size_t)255;
-    return delta + sa2::tc::bwd_extra_workspace_bytes(s);
+    return delta + sa2::tc::bwd_extra_workspace_bytes(s, shape->w2);
 }
 
 int sa2_fwd(const sa2_fwd_args *a) {
@@ -239,7 +240,7 @@ int sa2_bwd(const sa2_bwd_args *a) {
     if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !exact && sa2::tc::bwd_scale_ok(s)) {
         size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
         delta = (delta + 255) & ~(size_t)255;
-        return sa2::tc::bwd(p, s, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);
+        return sa2::tc::bwd(p, s, a->shape.w2, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);
     }
 
     switch (s.d) {

@@ -27,8 +27,7 @@ inline bool fwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 // that way.  Relative error of the output against 64 bits 1.57e-3 to 1.67e-3, as with fp32 arithmetic (2.2e-3 to 3.2e-3 with
 // rounded operands); of the logsumexp 2e-6, absolute (3e-3 to 1.6e-2).
 inline bool fwd_split(const sa2_shape &s) { return s.d == 32 || (s.d == 64 && s.w1 > 513); }
-// So does the tensor-core backward.  Head dim 32 keeps A_e, B_e, P and G to 16 bits there (bwd_split); its gradients in bf16
-// are then off by what their own rounding costs, as with fp32 arithmetic.
+// So does the tensor-core backward (see bq_plan, and bwd_split for dK1 / dV1 at head dim 32).
 inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 // A scale of (nearly) zero goes to the fp32 kernels: dK1/dV1 folds lse / scale into its products.
 inline bool bwd_scale_ok(const sa2_shape &s) { return fabsf(s.scale) >= 1e-20f; }
@@ -37,14 +36,13 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // splits of the offsets.  A CTA costs ~12000 cycles of set-up, loads, slab and its share of the reduction, a 64-key unit
 // of a sweep ~1600 (3000 at head dim 128); at most as many offsets per CTA as its accumulators hold.
 struct BqSplit { int tsplit, esplit, epc; };
-inline BqSplit bq_split(const sa2_shape &s, int sms) {
+inline BqSplit bq_split(const sa2_shape &s, int max_tiles, int sms) {
     BqSplit r;
-    r.tsplit = s.d == 128 ? 1 : (tiles_per_query_tile(s.w1) + BQ_MAX_TILES - 1) / BQ_MAX_TILES;
     const int nt = tiles_per_query_tile(s.w1), have = (s.n + s.off1 + TJ - 1) / TJ;
+    r.tsplit = s.d == 128 ? 1 : (nt + max_tiles - 1) / max_tiles;
     const int tiles = (nt < have ? nt : have), per = (tiles + r.tsplit - 1) / r.tsplit;
     const int64_t ctas = (int64_t)((s.n + TQ - 1) / TQ) * s.hq * r.tsplit * (s.d == 128 ? 2 : 1);
-    const int w2 = s.w2 < s.n + s.off2 ? s.w2 : s.n + s.off2;
-    const int least = (w2 + BQ_MAX_EPC - 1) / BQ_MAX_EPC;
+    const int w2 = s.w2, least = (w2 + BQ_MAX_EPC - 1) / BQ_MAX_EPC;
     double best_cost = 0.;
     r.esplit = least;
     for (int es = least; es <= w2 && (es <= 16 || es == least); ++es) {
@@ -55,6 +53,38 @@ inline BqSplit bq_split(const sa2_shape &s, int sms) {
     r.esplit = (w2 + r.epc - 1) / r.epc;
     return r;
 }
+// How dQ, dK2 and dV2 are computed.  Up to 56 offsets (the caller's window, however short the sequence) head dims 64 and 128
+// round A_e, B_e, P and G to bf16.  Callers of head dim 32 and of longer second windows had fp32 arithmetic: those keep 16 bits
+// and more of each (BqCfg), and their gradients in bf16 are as far from 64 bits as those of the fp32 kernels.
+// A long window is many ranges of 56 offsets, whose partials grow with w1 * w2.  The batch then goes through the scratch
+// in rounds of at most BQ_ROUND_BYTES (one element at least); where one element needs more than BQ_MOST_BYTES, the fp32 kernels
+// do it without any (b1 n4096 h8 d64 w4096/4096 would take 36 GB).
+// Errors of dq, dk2, dv2 against 64 bits, n150...400: 1.9e-3 to 3.2e-3 as on the fp32 kernels, 2.3e-3 to 5.4e-3 with rounded
+// operands.  Times of dQ/dK2/dV2, fp32 kernels / rounded / this: b4 n1024 h8 d64 w512/64 38.6 / 0.77 / 1.36 ms; d128 b2 w512/60
+// 41.2 / 1.01 / 2.55 ms (K1 / V1 one unit at a time); b1 n190 h4 d64, full causal 11.0 / 0.058 / 0.112 ms.
+constexpr size_t BQ_ROUND_BYTES = (size_t)256 << 20, BQ_MOST_BYTES = (size_t)1 << 30;
+struct BqPlan {
+    bool tc, split;      // on the tensor cores; with rests
+    BqSplit sp;
+    int round;           // batch elements that share the scratch at a time
+};
+inline BqPlan bq_plan(const sa2_shape &s, int caller_w2, int sms) {
+    BqPlan p;
+    const bool longer = caller_w2 > BQ_MAX_EPC;
+    p.split = s.d == 32 || longer;
+    p.sp = bq_split(s, p.split && s.d == 64 ? BqCfg<64, true>::MAX_TILES : BqCfg<64, false>::MAX_TILES, sms);
+    p.round = s.b;
+    p.tc = true;
+    if (longer) {
+        sa2_shape one = s;
+        one.b = 1;
+        const int ns = p.sp.tsplit * p.sp.esplit;
+        const size_t bytes = bq_part_dq_bytes(one, ns) + bq_part_k2_bytes(one, ns, p.sp.epc);
+        p.tc = bytes <= BQ_MOST_BYTES;
+        if (bytes * s.b > BQ_ROUND_BYTES) p.round = bytes > BQ_ROUND_BYTES ? 1 : (int)(BQ_ROUND_BYTES / bytes);
+    }
+    return p;
+}
 // Diagnostic switch: SA2_MMA_N64=1 issues every head-dim-128 product over the channels as two N = 64
 // instructions instead of one N = 128 instruction.
 inline int n64_products() {
@@ -63,19 +93,31 @@ inline int n64_products() {
 }
 // scratch after the D vector: per-split partial dQ, the per-CTA dK2/dV2 slabs, partial dK1/dV1
 struct BwdScratch { size_t dq, k2, k1; };
-inline BwdScratch bwd_scratch(const sa2_shape &s) {
-    const BqSplit sp = bq_split(s, SM_COUNT);
+inline BwdScratch bwd_scratch(const sa2_shape &s, const BqPlan &q) {
     const K1Split k1 = k1_split(s, SM_COUNT);
-    const int ns = sp.tsplit * sp.esplit;
-    return BwdScratch{align256(bq_part_dq_bytes(s, ns)), align256(bq_part_k2_bytes(s, ns, sp.epc)), align256(k1_part_bytes(s, k1.si * k1.se))};
+    BwdScratch b{0, 0, align256(k1_part_bytes(s, k1.si * k1.se))};
+    if (q.tc) {
+        sa2_shape r = s;
+        r.b = q.round;
+        const int ns = q.sp.tsplit * q.sp.esplit;
+        b.dq = align256(bq_part_dq_bytes(r, ns));
+        b.k2 = align256(bq_part_k2_bytes(r, ns, q.sp.epc));
+    }
+    return b;
 }
-inline size_t bwd_extra_workspace_bytes(const sa2_shape &s) {
+inline size_t bwd_extra_workspace_bytes(const sa2_shape &s, int caller_w2) {
     if (!bwd_supported(s)) return 0;
-    const BwdScratch b = bwd_scratch(s);
+    const BwdScratch b = bwd_scratch(s, bq_plan(s, caller_w2, SM_COUNT));
     return b.dq + b.k2 + b.k1;
 }
-// forward: 1 kernel; backward: D = rowsum(O*dO), dK1/dV1, dQ/dK2/dV2 partials, their reduction
-inline int launches(const sa2_shape &, bool backward) { return backward ? 4 : 1; }
+// forward: 1 kernel; backward: D = rowsum(O*dO), dK1/dV1, then dQ/dK2/dV2 and the reduction of the partials, per round
+inline int launches(const sa2_shape &s, bool backward, int caller_w2) {
+    if (!backward) return 1;
+    const BqPlan q = bq_plan(s, caller_w2, SM_COUNT);
+    const K1Split k1 = k1_split(s, SM_COUNT);
+    const int rounds = (s.b + q.round - 1) / q.round, k1_reduce = k1.si * k1.se > 1;
+    return !q.tc ? 3 + k1_reduce : rounds == 1 ? 4 : 2 + 2 * rounds + k1_reduce;
+}
 
 inline bool tma_addressable(const TensorRef &t) {
     return (reinterpret_cast<uintptr_t>(t.p) & 15u) == 0 && t.sb % 8 == 0 && t.sn % 8 == 0 && t.sh % 8 == 0;
@@ -165,18 +207,19 @@ inline bool bwd_addressable(const KernelParams &kp) {
 }
 
 // dQ, dK2, dV2: query-tile-owned tcgen05 kernel
-template <int D>
-inline int bwd_q_launch(const BqParams &Q, const KernelParams &kp, const CUtensorMap &mapK, const CUtensorMap &mapV, cudaStream_t st) {
-    const size_t smem = bq_smem_bytes<D>(Q.epc);
-    if (cudaFuncSetAttribute(bwd_q_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+template <int D, bool SPLIT>
+inline int bwd_q_launch(const BqParams &Q, cudaStream_t st) {
+    using C = BqCfg<D, SPLIT>;
+    const KernelParams &kp = Q.kp;
+    const size_t smem = bq_smem_bytes<D, SPLIT>(Q.epc);
+    if (cudaFuncSetAttribute(bwd_q_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SA2_ERR_CUDA;
-    CUtensorMap ringK = mapK, ringV = mapV;
-    if (D == 128) {     // the streamed units are 64-row boxes
-        if (!tmap::make_rows_map(&ringK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, 64) ||
-            !tmap::make_rows_map(&ringV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, 64))
-            return SA2_ERR_CUDA;
-    }
-    bwd_q_kernel<D><<<dim3(Q.nqt * Q.nsplit * BqCfg<D>::CH, kp.hq, kp.b), BqCfg<D>::THREADS, smem, st>>>(ringK, ringV, Q);
+    CUtensorMap mapK, mapV;             // head dim 128 streams units of 64 rows
+    constexpr int ROWS = D == 128 ? 64 : TJ;
+    if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, ROWS) ||
+        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, ROWS))
+        return SA2_ERR_CUDA;
+    bwd_q_kernel<D, SPLIT><<<dim3(Q.nqt * Q.nsplit * C::CH, kp.hq, kp.b), C::THREADS, smem, st>>>(mapK, mapV, Q);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
@@ -216,28 +259,37 @@ inline int bwd_k1_launch(const KernelParams &kp, const sa2_shape &s, const CUten
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
+// batch elements [b0, b0 + nb) of a backward
+inline KernelParams batch_part(KernelParams kp, int b0, int nb) {
+    auto shift = [b0](TensorRef &t, int bytes) { t.p = reinterpret_cast<char *>(t.p) + b0 * t.sb * bytes; };
+    for (TensorRef *t : {&kp.q, &kp.k1, &kp.k2, &kp.v1, &kp.v2, &kp.out, &kp.dout}) shift(*t, kp.in_bf16 ? 2 : 4);
+    for (TensorRef *t : {&kp.dq, &kp.dk1, &kp.dk2, &kp.dv1, &kp.dv2}) shift(*t, kp.grad_bf16 ? 2 : 4);
+    kp.lse += (int64_t)b0 * kp.hq * kp.n;
+    kp.delta += (int64_t)b0 * kp.hq * kp.n;
+    kp.b = nb;
+    return kp;
+}
+
 template <int D>
-inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, void *extra, cudaStream_t st, int phases) {
+inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, int caller_w2, void *extra, cudaStream_t st, int phases) {
     const float c = s.scale * 1.4426950408889634f;
     int *status = status_word();
     if (!status) return SA2_ERR_CUDA;
     if (phases == 0) phases = SA2_BWD_ROWSUM | SA2_BWD_K1 | SA2_BWD_Q;
     // D_i = sum_c O_ic dO_ic
     if ((phases & SA2_BWD_ROWSUM) && !simt::launch_delta<D>(kp, st)) return SA2_ERR_CUDA;
-    // 128-row, 64-channel boxes of K1 / V1 (a head-dim-128 tile is two boxes)
-    CUtensorMap mapK, mapV;
-    if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, TJ) ||
-        !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, TJ))
-        return SA2_ERR_CUDA;
-    const BwdScratch room = bwd_scratch(s);
-    const BqSplit sp = bq_split(s, SM_COUNT);
+    BqPlan plan = bq_plan(s, caller_w2, SM_COUNT);
+    // fp32 gradients show the last bits, which AUTO leaves to the fp32 kernels
+    if (s.kernel == SA2_KERNEL_AUTO && !kp.grad_bf16 && caller_w2 > BQ_MAX_EPC) plan.tc = false;
+    const BwdScratch room = bwd_scratch(s, plan);
+    const K1Split k1 = k1_split(s, SM_COUNT);
     BqParams Q;
     Q.kp = kp;
     Q.c = c;
     Q.nt = tiles_per_query_tile(s.w1);
-    Q.tsplit = sp.tsplit;
-    Q.nsplit = sp.tsplit * sp.esplit;
-    Q.epc = sp.epc;
+    Q.tsplit = plan.sp.tsplit;
+    Q.nsplit = plan.sp.tsplit * plan.sp.esplit;
+    Q.epc = plan.sp.epc;
     Q.tiles_per_split = (Q.nt + Q.tsplit - 1) / Q.tsplit;
     Q.nqt = (kp.n + TQ - 1) / TQ;
     Q.part_dq = reinterpret_cast<float *>(extra);
@@ -245,23 +297,37 @@ inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, void *extra, c
     float *part_k1 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + room.dq + room.k2);
     Q.part_k1 = part_k1;
     Q.status = status;
-    const K1Split k1 = k1_split(s, SM_COUNT);
     Q.ce = k1.si * k1.se;
-    Q.reduce_q = (phases & SA2_BWD_Q) != 0;
-    Q.reduce_k1 = (phases & SA2_BWD_K1) && Q.ce > 1;
-    if (phases & SA2_BWD_K1)
+    const bool q_tc = (phases & SA2_BWD_Q) && plan.tc, k1_parts = (phases & SA2_BWD_K1) && Q.ce > 1;
+    if (phases & SA2_BWD_K1) {
+        CUtensorMap mapK, mapV;     // 128-row, 64-channel boxes of K1 / V1 (a head-dim-128 tile is two boxes)
+        if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, TJ) ||
+            !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, TJ))
+            return SA2_ERR_CUDA;
         if (int e = bwd_k1_launch<D>(kp, s, mapK, mapV, c, status, k1, part_k1, st)) return e;
-    if (phases & SA2_BWD_Q)
-        if (int e = bwd_q_launch<D>(Q, kp, mapK, mapV, st)) return e;
+    }
+    if ((phases & SA2_BWD_Q) && !plan.tc && !simt::launch_bwd<D>(kp, true, true, false, SM_COUNT, st)) return SA2_ERR_CUDA;
+    const bool one_round = plan.round >= kp.b;
+    for (int b0 = 0; q_tc && b0 < kp.b; b0 += plan.round) {
+        Q.kp = batch_part(kp, b0, kp.b - b0 < plan.round ? kp.b - b0 : plan.round);
+        if (int e = D == 32 || plan.split ? bwd_q_launch<D, true>(Q, st) : bwd_q_launch<D, D == 32>(Q, st)) return e;
+        Q.reduce_q = 1;
+        Q.reduce_k1 = one_round && k1_parts;
+        if (int e = bwd_reduce_launch<D>(Q, st)) return e;
+    }
+    if (!k1_parts || (q_tc && one_round)) return SA2_OK;
+    Q.kp = kp;
+    Q.reduce_q = 0;
+    Q.reduce_k1 = 1;
     return bwd_reduce_launch<D>(Q, st);
 }
 
-inline int bwd(const KernelParams &kp, const sa2_shape &s, void *extra, cudaStream_t st, int phases = 0) {
+inline int bwd(const KernelParams &kp, const sa2_shape &s, int caller_w2, void *extra, cudaStream_t st, int phases = 0) {
     if (!bwd_addressable(kp)) return SA2_ERR_INVALID;
     switch (s.d) {
-        case 32: return bwd_launch<32>(kp, s, extra, st, phases);
-        case 64: return bwd_launch<64>(kp, s, extra, st, phases);
-        default: return bwd_launch<128>(kp, s, extra, st, phases);
+        case 32: return bwd_launch<32>(kp, s, caller_w2, extra, st, phases);
+        case 64: return bwd_launch<64>(kp, s, caller_w2, extra, st, phases);
+        default: return bwd_launch<128>(kp, s, caller_w2, extra, st, phases);
     }
 }
 

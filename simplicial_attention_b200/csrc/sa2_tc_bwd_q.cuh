@@ -46,7 +46,7 @@
 // N = 64, so A is read again for every unit), the folds and the operand rows a further ~400, and everything that
 // goes through shared memory - shuffles included - waits behind the tensor cores' fetches.  b4 n4096 h8 w512/32 takes
 // ~1350 cycles a unit: 1.97 -> 1.58 ms at head dim 64, 40 -> 1.94 ms at 32 (the fp32 kernels before; 1.33 with A_e, B_e, P and
-// G rounded to bf16: see bwd_split).  Measured and not
+// G rounded to bf16: see bq_plan).  Measured and not
 // kept: A_e and B_e in TMEM, double-buffered, which leaves two S / dP buffers (1.74 ms); k2 / v2 rows moved from lane to
 // lane by shuffles instead of a row per lane from memory (1.70 ms).  Head dim 128 (two buffers, S and dP formed in
 // both channel halves): 11.7 -> 8.5 ms on b1 n16384 h16; the chain S / dP -> P / G -> U / W of two buffers paces it.
@@ -62,7 +62,7 @@ namespace tc {
 //                 and chunks of U and W).
 //   up to 64:     five groups of 96 (640 threads): the U fold takes 160 (dQ, q and k2 rows, 128 registers, and a
 //                 chunk of U), the W fold 104.
-template <int D> struct BqCfg {
+template <int D, bool SPLIT> struct BqCfg {
     static constexpr bool TWO_FOLDS = D <= 64;                   // U and W have a fold group each
     static constexpr int THREADS = TWO_FOLDS ? 640 : 512;
     static constexpr int REGS_LAUNCH = TWO_FOLDS ? 96 : 128, REGS_ISSUE = 40, REGS_COMPUTE = TWO_FOLDS ? 88 : 120;
@@ -72,17 +72,20 @@ template <int D> struct BqCfg {
     static constexpr int CC = D < 64 ? D : 64;                   // channels this CTA produces
     static constexpr int KSTEPS = D / 16;                        // K = 16 steps of S and dP
     static constexpr uint32_t BLK = TJ * 128;                    // A_e / B_e: one [128 rows][64 channels] swizzled block
-    static constexpr uint32_t TILE = CH * BLK;                   // A_e or B_e
+    // SPLIT: A_e, B_e, P and G are each a bf16 value and a bf16 rest.  The rests of A_e / B_e fill the free half of the rows
+    // at head dim 32 and take blocks of their own otherwise, for which K1 / V1 make room
+    static constexpr uint32_t REST = D == 32 ? 64 : CH * BLK;    // bytes from an element of A_e / B_e to its rest
+    static constexpr uint32_t TILE = CH * BLK * (SPLIT && D > 32 ? 2 : 1);        // A_e or B_e
+    static constexpr int MAX_TILES = SPLIT && D == 64 ? 2 : 3;   // K1/V1 tiles of a split (head dims 32, 64)
     // K1 / V1 in shared memory: head dim 64 keeps three 128-row tiles of 16 KB resident; head dim 128 has a
     // ring of three 64-row units, each two [64 rows][64 channels] blocks of 8 KB
-    static constexpr int NSLOT = 3;
-    static constexpr uint32_t KV_BYTES = D <= 64 ? 3 * BLK : NSLOT * 16384;
+    static constexpr int NSLOT = SPLIT && D == 128 ? 1 : 3;
+    static constexpr uint32_t KV_BYTES = D <= 64 ? MAX_TILES * BLK : NSLOT * 16384;
     static constexpr uint32_t UBLK = 8192;                       // one channel block of a 64-row unit (head dim 128)
     static constexpr int NBUF = D <= 64 ? 3 : 2;                 // S / dP (P / G) buffers in TMEM
     static constexpr int UWBUF = D <= 64 ? 1 : 2;                // U / W accumulator pairs in TMEM
     static constexpr uint32_t UW0 = NBUF * 128;                  // first TMEM column of U / W
 };
-constexpr int BQ_MAX_TILES = 3;          // K1/V1 tiles of one split (head dim 64)
 // Shared accumulators of dK2 / dV2: in sweep e thread r adds to slab row r + epc - 1 - e (epc offsets per CTA), so 128 consecutive rows
 // are live at a time.
 // Head dims 32 and 64 keep all 127 + epc rows, 68 floats apart (64 + 4: the row-per-thread accesses of a warp spread over
@@ -93,7 +96,7 @@ constexpr int BQ_MAX_TILES = 3;          // K1/V1 tiles of one split (head dim 6
 // floats; its sixteen 16-byte chunks are XOR-ed with the row number instead of padding.
 constexpr int BQ_ACC_RING = 128;
 constexpr int BQ_ACC_STRIDE = 68;
-constexpr int BQ_MAX_EPC = 56;           // offsets of a CTA: 127 + epc accumulator rows must fit (head dim 64)
+constexpr int BQ_MAX_EPC = 56;           // most offsets of a CTA: 127 + epc accumulator rows must fit (head dim 64)
 template <int D> struct BqAcc {
     static constexpr bool RING = D == 128;
     __host__ __device__ static int rows(int epc) { return RING ? BQ_ACC_RING : 127 + epc; }
@@ -145,8 +148,8 @@ struct BqParams {
     int ce, reduce_q, reduce_k1;
 };
 
-template <int D> inline size_t bq_smem_bytes(int epc) {
-    return 1024 + (size_t)2 * BqCfg<D>::KV_BYTES + 2 * BqCfg<D>::TILE +
+template <int D, bool SPLIT> inline size_t bq_smem_bytes(int epc) {
+    return 1024 + (size_t)2 * BqCfg<D, SPLIT>::KV_BYTES + 2 * BqCfg<D, SPLIT>::TILE +
            (size_t)2 * BqAcc<D>::rows(epc) * BqAcc<D>::row_floats() * sizeof(float) + 256;
 }
 // (a query tile with one split writes dQ itself and needs no partials)
@@ -169,8 +172,9 @@ template <int D>
 __device__ __forceinline__ BqGeom bq_geom(const BqParams &P) {
     BqGeom g;
     const KernelParams &kp = P.kp;
-    g.chh = blockIdx.x % BqCfg<D>::CH;
-    const int qs = blockIdx.x / BqCfg<D>::CH;
+    constexpr int CH = D == 128 ? 2 : 1;
+    g.chh = blockIdx.x % CH;
+    const int qs = blockIdx.x / CH;
     g.qt = qs / P.nsplit;
     g.split = qs % P.nsplit;
     g.i0 = g.qt * TQ;
@@ -201,10 +205,10 @@ __device__ __forceinline__ BqGeom bq_geom(const BqParams &P) {
 // One thread issues about one tcgen05.mma per 60-90 cycles, so the two product stages have an issuing
 // thread each; U / W are accumulated by one thread only, which keeps the summation order fixed.
 // which = 0: S = A_e K1^T into columns [128 buf, +64); which = 1: dP = B_e V1^T into [128 buf + 64, +64).
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t tmem, uint8_t *sKV, uint8_t *sAB,
                                             uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     constexpr uint32_t IDESC_F = idesc_bf16(128, 64, false, false);
     const uint64_t dT = smem_desc_sw128(smem_u32(sKV)), dA = smem_desc_sw128(smem_u32(sAB));
     if constexpr (D <= 64) {
@@ -229,16 +233,16 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
                 const uint64_t t = dT + (uint64_t)((w * 8192) >> 4);       // unit w: rows [64 w, +64) of the resident tiles
 #pragma unroll
                 for (int k = 0; k < C::KSTEPS; ++k) mma_ss(d, dA + 2 * k, t + 2 * k, IDESC_F, k > 0 ? 1u : 0u);
-                if constexpr (bwd_split<D>) {             // the rests of A_e / B_e: channels 32-63 of their rows
+                if constexpr (SPLIT) {
 #pragma unroll
-                    for (int k = 0; k < C::KSTEPS; ++k) mma_ss(d, dA + 4 + 2 * k, t + 2 * k, IDESC_F, 1u);
+                    for (int k = 0; k < C::KSTEPS; ++k) mma_ss(d, dA + (C::REST >> 4) + 2 * k, t + 2 * k, IDESC_F, 1u);
                 }
             } else {
                 const uint64_t t = dT + (uint64_t)((slot * 2 * C::UBLK) >> 4);
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
+                for (int k = 0; k < (SPLIT ? 16 : 8); ++k)
                     mma_ss(d, dA + (uint64_t)(((k >> 2) * C::BLK) >> 4) + (uint64_t)((k & 3) * 2),
-                           t + (uint64_t)(((k >> 2) * C::UBLK) >> 4) + (uint64_t)((k & 3) * 2), IDESC_F, k > 0 ? 1u : 0u);
+                           t + (uint64_t)(((k >> 2 & 1) * C::UBLK) >> 4) + (uint64_t)((k & 3) * 2), IDESC_F, k > 0 ? 1u : 0u);
             }
             SA2_PROF_LAP(4, seg);                         // issue of the products
             tc_commit(&bars[BQ_S_FULL + buf]);
@@ -253,10 +257,10 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
 }
 
 // ---------------------------------------------------------------- head dim 128: TMA producer of the K1/V1 ring (warp 3, one lane)
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_ring_producer(const BqParams &P, const BqGeom &g, const CUtensorMap *mapK, const CUtensorMap *mapV,
                                                 uint8_t *sK, uint8_t *sV, uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     const int hk = blockIdx.y / P.kp.g;
     prefetch_tmap(mapK);
     prefetch_tmap(mapV);
@@ -285,10 +289,10 @@ __device__ __forceinline__ int bq_ring_producer(const BqParams &P, const BqGeom 
 // ---------------------------------------------------------------- issuers of U, W (one lane each)
 // part 0 (warp 0; head dim 64: after loading the tiles): U += G K1; part 1 (warp 3): W += P V1; part 2 (head dim
 // 128, warp 0): both.  Each accumulator has one issuing thread, which keeps its summation order fixed.
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g, int part, const CUtensorMap *mapK, const CUtensorMap *mapV,
                                              uint32_t tmem, uint8_t *sK, uint8_t *sV, uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     constexpr uint32_t IDESC_G = idesc_bf16(128, C::CC, false, true);
     if constexpr (D <= 64) {
         if (part == 0) {
@@ -331,7 +335,7 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
                 mma_ts(tu, a + 72, kt + 128, IDESC_G, 1u);
                 mma_ts(tu, a + 96, kt + 256, IDESC_G, 1u);
                 mma_ts(tu, a + 104, kt + 384, IDESC_G, 1u);
-                if constexpr (bwd_split<D>) {                       // the rests of G, behind it
+                if constexpr (SPLIT) {                              // the rests of G, behind it
                     mma_ts(tu, a + 80, kt, IDESC_G, 1u);
                     mma_ts(tu, a + 88, kt + 128, IDESC_G, 1u);
                     mma_ts(tu, a + 112, kt + 256, IDESC_G, 1u);
@@ -343,7 +347,7 @@ __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g,
                 mma_ts(tw, a + 8, vt + 128, IDESC_G, 1u);
                 mma_ts(tw, a + 32, vt + 256, IDESC_G, 1u);
                 mma_ts(tw, a + 40, vt + 384, IDESC_G, 1u);
-                if constexpr (bwd_split<D>) {
+                if constexpr (SPLIT) {
                     mma_ts(tw, a + 16, vt, IDESC_G, 1u);
                     mma_ts(tw, a + 24, vt + 128, IDESC_G, 1u);
                     mma_ts(tw, a + 48, vt + 256, IDESC_G, 1u);
@@ -378,9 +382,9 @@ __device__ __forceinline__ void pg_pair(float p0, float p1, uint32_t dp0, uint32
     }
 }
 // Head dim 64: group cg forms columns [32 cg, +32) of every unit, which halves the time between S / dP and P / G.
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, int cg, uint32_t tmem, uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = (warp & 3) * 32 + lane;             // query row within the tile = TMEM lane
@@ -415,7 +419,6 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                 const bool full = __all_sync(0xffffffffu, lo < 0 && hi >= 63);
                 {
                     const int ch = cg;
-                    constexpr bool SPLIT = bwd_split<D>;
                     uint32_t sv[32], dv[32], pp[16], gg[16], pr[SPLIT ? 16 : 1], gr[SPLIT ? 16 : 1];
                     // no row of this warp has a valid column among these 32: P = G = 0 without reading S / dP
                     if (__all_sync(0xffffffffu, hi < ch * 32 || lo >= ch * 32 + 31)) {
@@ -528,10 +531,10 @@ __device__ __forceinline__ uint4 mul_bf16x8(const uint4 &x, const uint4 &y) {
 // WHICH = 1 forms B_e = dO_i * v2_{i-e} and folds W_e into dV2_{i-e}.  One thread per query row; its q (dO) row stays
 // in its registers.  With one group for both, U / W of the next sweep waited ~1960 of 9400 cycles a sweep for the
 // accumulators to be read and S / dP ~1000 for their operands.
-template <int D, int WHICH>
+template <int D, bool SPLIT, int WHICH>
 __device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc, uint8_t *sOp, uint64_t *bars,
                                             volatile int *abort_flag) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = (warp & 3) * 32 + lane;             // query row within the tile = TMEM lane
@@ -563,14 +566,12 @@ __device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, 
     auto build = [&](int e) -> bool {
         bool ok;
         const uint4 *py = yrow(e, ok);
-        uint4 y[NC], rest[bwd_split<D> ? NC : 1];
+        uint4 y[NC];
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc) y[cc] = ok ? __ldg(py + cc) : zero;
+        if constexpr (!SPLIT) {
 #pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-            const uint4 hi = ok ? mul_bf16x8(xr[cc], y[cc]) : zero;
-            if constexpr (bwd_split<D>) rest[cc] = ok ? mul_rest_bf16x8(xr[cc], y[cc], hi) : zero;
-            y[cc] = hi;
+            for (int cc = 0; cc < NC; ++cc) y[cc] = ok ? mul_bf16x8(xr[cc], y[cc]) : zero;
         }
         if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY + WHICH], (e - 1) & 1, abort_flag, 3)) return false;
 #ifdef SA2_PROF
@@ -578,8 +579,14 @@ __device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, 
 #endif
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc) {
-            *reinterpret_cast<uint4 *>(sOp + sw128_offset(r, cc)) = y[cc];
-            if constexpr (bwd_split<D>) *reinterpret_cast<uint4 *>(sOp + sw128_offset(r, 4 + cc)) = rest[cc];
+            uint8_t *dst = sOp + sw128_offset(r, cc);
+            if constexpr (SPLIT) {       // (formed here: a row of products and one of rests would not fit the registers)
+                const uint4 hi = ok ? mul_bf16x8(xr[cc], y[cc]) : zero;
+                *reinterpret_cast<uint4 *>(dst) = hi;
+                *reinterpret_cast<uint4 *>(D == 32 ? sOp + sw128_offset(r, 4 + cc) : dst + C::REST) = ok ? mul_rest_bf16x8(xr[cc], y[cc], hi) : zero;
+            } else {
+                *reinterpret_cast<uint4 *>(dst) = y[cc];
+            }
         }
         fence_proxy_async_smem();
         mbar_arrive(&bars[BQ_AB_FULL + WHICH]);
@@ -661,10 +668,10 @@ __device__ __forceinline__ int bq_fold_half(const BqParams &P, const BqGeom &g, 
 
 // Head dim 128: one group for both.
 
-template <int D>
+template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc_k, float *acc_v, float *slab,
                                             uint8_t *sA, uint8_t *sB, uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = (warp & 3) * 32 + lane;             // query row within the tile = TMEM lane
@@ -693,10 +700,39 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     const int64_t b_q = elem_off(kp.q, b, 0, h) + bcc * 8, b_do = elem_off(kp.dout, b, 0, h) + bcc * 8;
     const int64_t b_k2 = elem_off(kp.k2, b, 0, hk) + bcc * 8, b_v2 = elem_off(kp.v2, b, 0, hk) + bcc * 8;
     auto build = [&](int e) -> bool {
-        uint4 pa[LPR], pb[LPR];
         auto fetch = [&](const TensorRef &t, int64_t base, int row) {
             return __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(t.p) + base + (int64_t)row * t.sn));
         };
+        if constexpr (SPLIT) {
+            // products and rests of four rows at a time, behind the wait: there are no registers to hold them before it
+            if (e >= 1 && !warp_wait(&bars[BQ_AB_EMPTY], (e - 1) & 1, abort_flag, 3)) return false;
+#pragma unroll 1
+            for (int x0 = 0; x0 < LPR; x0 += 4) {
+                uint4 w[4][4];                            // q, k2, dO, v2 of each row
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int ii = g.i0 + brow + (x0 + x) * RPI, kk = ii + kp.off2 - g.e0 - e;
+                    const bool ok = ii < kp.n && kk >= 0;
+                    w[x][0] = ok ? fetch(kp.q, b_q, ii) : make_uint4(0u, 0u, 0u, 0u);
+                    w[x][1] = ok ? fetch(kp.k2, b_k2, kk) : make_uint4(0u, 0u, 0u, 0u);
+                    w[x][2] = ok ? fetch(kp.dout, b_do, ii) : make_uint4(0u, 0u, 0u, 0u);
+                    w[x][3] = ok ? fetch(kp.v2, b_v2, kk) : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const uint32_t o = (bcc >> 3) * C::BLK + sw128_offset(brow + (x0 + x) * RPI, bcc & 7);
+                    const uint4 a = mul_bf16x8(w[x][0], w[x][1]), b2 = mul_bf16x8(w[x][2], w[x][3]);
+                    *reinterpret_cast<uint4 *>(sA + o) = a;
+                    *reinterpret_cast<uint4 *>(sB + o) = b2;
+                    *reinterpret_cast<uint4 *>(sA + C::REST + o) = mul_rest_bf16x8(w[x][0], w[x][1], a);
+                    *reinterpret_cast<uint4 *>(sB + C::REST + o) = mul_rest_bf16x8(w[x][2], w[x][3], b2);
+                }
+            }
+            fence_proxy_async_smem();
+            mbar_arrive(&bars[BQ_AB_FULL]);
+            return true;
+        }
+        uint4 pa[LPR], pb[LPR];
         constexpr int STEP = 2;                           // rows per lane that hold registers for a second operand
 #pragma unroll
         for (int x0 = 0; x0 < LPR; x0 += STEP) {
@@ -855,10 +891,10 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
 }
 
 // A fold group: WHICH = 0 U (head dim 128: both), 1 W.
-template <int D, int WHICH>
+template <int D, bool SPLIT, int WHICH>
 __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc_k, float *acc_v, uint8_t *sA, uint8_t *sB,
                                        uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     const KernelParams &kp = P.kp;
     const int ft = threadIdx.x & 127;
     const int h = blockIdx.y, b = blockIdx.z;
@@ -870,9 +906,9 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
         float *acc = WHICH ? acc_v : acc_k;
         for (int x = ft; x < slab_rows * BQ_ACC_STRIDE; x += 128) acc[x] = 0.f;      // only this group touches it
         bq_fold_sync(WHICH);
-        err = bq_fold_half<D, WHICH>(P, g, tmem, acc, WHICH ? sB : sA, bars, abort_flag);
+        err = bq_fold_half<D, SPLIT, WHICH>(P, g, tmem, acc, WHICH ? sB : sA, bars, abort_flag);
     } else {
-        err = bq_fold_body<D>(P, g, tmem, acc_k, acc_v, slab, sA, sB, bars, abort_flag);
+        err = bq_fold_body<D, SPLIT>(P, g, tmem, acc_k, acc_v, slab, sA, sB, bars, abort_flag);
     }
     // The barrier sits outside the body so that a warp that gave up on a wait still reaches it.
     bq_fold_sync(WHICH);
@@ -895,10 +931,10 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
     return err;
 }
 
-template <int D>
-__global__ void __launch_bounds__(BqCfg<D>::THREADS, 1)
+template <int D, bool SPLIT>
+__global__ void __launch_bounds__(BqCfg<D, SPLIT>::THREADS, 1)
 bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const BqParams P) {
-    using C = BqCfg<D>;
+    using C = BqCfg<D, SPLIT>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;
@@ -944,23 +980,23 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     if (warp < 4) {
         reg_dealloc<C::REGS_ISSUE>();                 // one instruction for the whole warpgroup
         if (g.total > 0) {
-            if (warp == 0) err = bq_mma_second<D>(P, g, D <= 64 ? 0 : 2, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
-            else if (warp == 1) err = bq_mma_first<D>(g, 0, tmem, sK, sA, bars, abort_flag);
-            else if (warp == 2) err = bq_mma_first<D>(g, 1, tmem, sV, sB, bars, abort_flag);
-            else if constexpr (D <= 64) err = bq_mma_second<D>(P, g, 1, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
-            else err = bq_ring_producer<D>(P, g, &mapK, &mapV, sK, sV, bars, abort_flag);
+            if (warp == 0) err = bq_mma_second<D, SPLIT>(P, g, D <= 64 ? 0 : 2, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
+            else if (warp == 1) err = bq_mma_first<D, SPLIT>(g, 0, tmem, sK, sA, bars, abort_flag);
+            else if (warp == 2) err = bq_mma_first<D, SPLIT>(g, 1, tmem, sV, sB, bars, abort_flag);
+            else if constexpr (D <= 64) err = bq_mma_second<D, SPLIT>(P, g, 1, &mapK, &mapV, tmem, sK, sV, bars, abort_flag);
+            else err = bq_ring_producer<D, SPLIT>(P, g, &mapK, &mapV, sK, sV, bars, abort_flag);
         }
     } else if (warp < 12) {
         // one call site for both compute groups: they run the same instructions, which the instruction caches
         // of a scheduler then hold once
         reg_dealloc<C::REGS_COMPUTE>();
-        err = bq_compute<D>(P, g, (warp >> 2) - 1, tmem, bars, abort_flag);
+        err = bq_compute<D, SPLIT>(P, g, (warp >> 2) - 1, tmem, bars, abort_flag);
     } else if (!C::TWO_FOLDS || warp < 16) {
         reg_alloc<C::REGS_FOLD>();
-        err = bq_fold<D, 0>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
+        err = bq_fold<D, SPLIT, 0>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
     } else if constexpr (C::TWO_FOLDS) {
         reg_alloc<C::REGS_FOLD_W>();
-        err = bq_fold<D, 1>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
+        err = bq_fold<D, SPLIT, 1>(P, g, tmem, acc_k, acc_v, sA, sB, bars, abort_flag);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);

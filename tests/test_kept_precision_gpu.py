@@ -1,5 +1,7 @@
 """bf16 shapes whose arithmetic is that of fp32 (head dim 32, long first windows at head dim 64, long second windows):
 only the inputs and the results are rounded to bf16.  Against the oracle in 64 bits."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -73,3 +75,40 @@ def test_backward_head_dim_32(case):
         assert err(got[i]) <= 1.01 * err(base[i]) + 2e-5, (name, err(got[i]), err(base[i]))
         # 16-bit P and G in fp32 sums
         assert (fine[i] - base_fine[i]).norm() <= 2e-5 * base_fine[i].norm(), name
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("n,w1,w2", [(150, 150, 150), (90, 40, 57), (30, 20, 400), (400, 300, 60)])
+def test_long_second_window(n, w1, w2, d):
+    """dq, dk2 and dv2 are as far from 64 bits as those of the fp32 kernels, also where the sequence is shorter than the
+    window; in fp32 they are those of the fp32 kernels."""
+    ins = O.make_inputs(2, n, 2, 1, d, seed=n + d, dtype=torch.bfloat16)
+    ref = O.two_simplicial_fwd_bwd(*[t.double() for t in ins], w1, w2, dtype=torch.float64)
+    q, k1, k2, v1, v2, do = [t.cuda() for t in ins]
+    out, lse = sa.sa2_forward(q, k1, k2, v1, v2, w1, w2, kernel="simt")
+    got, base = (sa.sa2_backward(q, k1, k2, v1, v2, out, lse, do, w1, w2, kernel=k) for k in ("auto", "simt"))
+    fine, same, base_fine = (sa.sa2_backward(q, k1, k2, v1, v2, out, lse, do, w1, w2, kernel=k, grad_dtype=torch.float32)
+                             for k in ("tcgen05", "auto", "simt"))
+    assert sa.device_status() == 0
+    for i, name in ((0, "dq"), (2, "dk2"), (4, "dv2")):
+        err = lambda x: ((x.double().cpu() - ref[name]).norm() / ref[name].norm()).item()
+        assert err(got[i]) <= 1.01 * err(base[i]) + 2e-5, (name, err(got[i]), err(base[i]))
+        assert (fine[i] - base_fine[i]).norm() <= 2e-5 * base_fine[i].norm(), name       # 16-bit P and G in fp32 sums
+        assert torch.equal(same[i], base_fine[i])
+
+
+def test_long_second_window_in_rounds():
+    """More batch elements than the scratch takes at a time."""
+    b, n, w = 20, 300, 300
+    q, k1, k2, v1, v2, do = [t.cuda() for t in O.make_inputs(b, n, 4, 2, 64, seed=2, dtype=torch.bfloat16)]
+    out, lse = sa.sa2_forward(q, k1, k2, v1, v2, w, w)
+    call = sa.attention.BackwardCall(q, k1, k2, v1, v2, out, lse, do, w, w, grad_dtype=torch.float32, kernel="tcgen05")
+    shape = call.args.shape
+    assert sa._lib.lib().sa2_kernel_launches(C.byref(shape), 1) > 4
+    got, base = call.launch(), sa.sa2_backward(q, k1, k2, v1, v2, out, lse, do, w, w, grad_dtype=torch.float32, kernel="simt")
+    assert sa.device_status() == 0
+    for i in (0, 2, 4):
+        e = (got[i] - base[i]).flatten(1).norm(dim=1) / base[i].flatten(1).norm(dim=1)
+        assert e.max().item() <= 2e-5
+    for i in (1, 3):
+        assert (got[i] - base[i]).norm() <= 1e-2 * base[i].norm()

@@ -23,6 +23,16 @@ def test_scratch_is_that_of_the_sequence(w1, w2, d, off):
     assert need(w1, w2) == need(min(w1, 128 + off), min(w2, 128 + off))
 
 
+@pytest.mark.parametrize("b,n,w2", [(1, 4096, 4096), (1, 1024, 1024), (64, 1024, 64), (8, 190, 190)])
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_scratch_of_long_second_windows_is_bounded(b, n, w2, d):
+    """Row sums, the partials of dK1 / dV1 (at most 16 of each), and 1 GiB for the ranges of offsets; 256 MiB where a batch
+    is cut into rounds."""
+    rows, tensor = b * 8 * n * 4, b * n * 8 * d * 4
+    need = _lib.lib().sa2_bwd_workspace_bytes(C.byref(_shape(b=b, n=n, hq=8, hk=8, d=d, w1=n, w2=w2, dtype=1)))
+    assert need <= rows + 16 * 2 * tensor + ((256 if b > 1 else 1024) << 20) + 1024
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("d", [32, 64, 128])
