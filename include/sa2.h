@@ -131,6 +131,14 @@ int sa2_bwd(const sa2_bwd_args *args);
 size_t sa2_bwd_workspace_bytes(const sa2_shape *shape);
 
 /*
+ * The same for a part of a batch: how the work is split over CTAs, and with it the order of the sums, follows the size
+ * of the batch, so a caller that cuts one call of `whole_b` elements into calls of shape.b elements gets the
+ * whole call's bits by saying so (SA2_ERR_INVALID / 0 if whole_b < shape.b).  sa2_bwd is whole_b = shape.b.
+ */
+int sa2_bwd_part(const sa2_bwd_args *args, int32_t whole_b);
+size_t sa2_bwd_workspace_bytes_part(const sa2_shape *shape, int32_t whole_b);
+
+/*
  * Backward for callers that cannot supply scratch memory.  It has no
  * counterpart in the reference, which allocates whatever it needs from torch.
  *

@@ -19,7 +19,7 @@ BWD_ROWSUM, BWD_K1, BWD_Q = 1, 2, 4     # sa2_bwd_phase
 # symbols declared in include/sa2.h
 EXPORTS = ("sa2_fwd", "sa2_bwd", "sa2_bwd_workspace_bytes", "sa2_strerror", "sa2_version",
            "sa2_kernel_launches", "sa2_device_status", "sa2_check_device", "sa2_selftest_wait",
-           "sa2_bwd_static_scratch",
+           "sa2_bwd_static_scratch", "sa2_bwd_part", "sa2_bwd_workspace_bytes_part",
            "sa2_headnorm_fwd", "sa2_headnorm_bwd", "sa2_headnorm_partial_bytes",
            "sa2_qkvnorm_fwd", "sa2_qkvnorm_bwd", "sa2_qkv_append", "sa2_rows_linear")
 STATIC_SCRATCH_ROWS = 262144   # SA2_STATIC_SCRATCH_ROWS in include/sa2.h
@@ -100,6 +100,10 @@ def lib() -> C.CDLL:
         handle.sa2_fwd.restype = C.c_int
         handle.sa2_bwd.argtypes = [C.POINTER(BwdArgs)]
         handle.sa2_bwd.restype = C.c_int
+        handle.sa2_bwd_part.argtypes = [C.POINTER(BwdArgs), C.c_int32]
+        handle.sa2_bwd_part.restype = C.c_int
+        handle.sa2_bwd_workspace_bytes_part.argtypes = [C.POINTER(Shape), C.c_int32]
+        handle.sa2_bwd_workspace_bytes_part.restype = C.c_size_t
         handle.sa2_bwd_static_scratch.argtypes = [C.POINTER(BwdArgs)]
         handle.sa2_bwd_static_scratch.restype = C.c_int
         handle.sa2_bwd_workspace_bytes.argtypes = [C.POINTER(Shape)]

@@ -112,10 +112,11 @@ class BackwardCall:
     """A prepared ``sa2_bwd`` call: gradients and workspace are allocated once, ``launch(phases)``
     issues the kernels.  ``phases`` is 0 for the whole backward or an OR of ``_lib.BWD_ROWSUM``,
     ``_lib.BWD_K1`` (dK1, dV1), ``_lib.BWD_Q`` (dQ, dK2, dV2); the row sums must have been launched
-    (same stream, or otherwise ordered) before either of the other two."""
+    (same stream, or otherwise ordered) before either of the other two.  ``whole_batch``: the batch of the call that
+    this one is a part of, whose bits it then has (the batch decides how the work is split)."""
 
     def __init__(self, q, k1, k2, v1, v2, out, lse, dout, w1, w2, scale=None, kernel="auto", grad_dtype=None,
-                 grads=None):
+                 grads=None, whole_batch=None):
         _check_inputs(q, k1, k2, v1, v2)
         q, k1, k2, v1, v2, out, dout = (_usable(t) for t in (q, k1, k2, v1, v2, out, dout))
         if dout.dtype != q.dtype:
@@ -133,7 +134,8 @@ class BackwardCall:
         dq, dk1, dk2, dv1, dv2 = grads
         shape = _shape(q, k1, k2, w1, w2, scale, kernel)
         self.lib = _lib.lib()
-        ws_bytes = self.lib.sa2_bwd_workspace_bytes(C.byref(shape))
+        self.whole_batch = q.shape[0] if whole_batch is None else int(whole_batch)
+        ws_bytes = self.lib.sa2_bwd_workspace_bytes_part(C.byref(shape), self.whole_batch)
         ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=q.device)
         self.device = q.device
         self.grads = grads
@@ -155,16 +157,17 @@ class BackwardCall:
         self.args.phases = int(phases)
         self.args.stream = torch.cuda.current_stream(self.device).cuda_stream
         with torch.cuda.device(self.device):
-            _lib.check(self.lib.sa2_bwd(C.byref(self.args)), "sa2_bwd")
+            _lib.check(self.lib.sa2_bwd_part(C.byref(self.args), self.whole_batch), "sa2_bwd")
         return self.grads
 
 
-def sa2_backward(q, k1, k2, v1, v2, out, lse, dout, w1, w2, scale=None, kernel="auto", grad_dtype=None, grads=None):
+def sa2_backward(q, k1, k2, v1, v2, out, lse, dout, w1, w2, scale=None, kernel="auto", grad_dtype=None, grads=None,
+                 whole_batch=None):
     """Raw backward: returns ``(dq, dk1, dk2, dv1, dv2)`` in ``grad_dtype``
     (default: the input dtype).  Key/value gradients are already summed over
     each kv head's query group and cover the halo rows too.  ``grads`` may be
-    five preallocated tensors or strided views to write the results into."""
-    return BackwardCall(q, k1, k2, v1, v2, out, lse, dout, w1, w2, scale, kernel, grad_dtype, grads).launch(0)
+    five preallocated tensors or strided views to write the results into; ``whole_batch`` as for ``BackwardCall``."""
+    return BackwardCall(q, k1, k2, v1, v2, out, lse, dout, w1, w2, scale, kernel, grad_dtype, grads, whole_batch).launch(0)
 
 
 class SlidingTwoSimplicialAttention(Function):

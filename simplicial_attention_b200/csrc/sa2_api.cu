@@ -179,17 +179,19 @@ int sa2_kernel_launches(const sa2_shape *shape, int backward) {
     const bool tc_ok = backward ? sa2::tc::bwd_supported(s) : sa2::tc::fwd_supported(s);
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
     if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !(backward && !sa2::tc::bwd_scale_ok(s)))
-        return sa2::tc::launches(s, backward != 0, shape->w2);
+        return sa2::tc::launches(s, backward != 0, {shape->w2, shape->b});
     return backward ? 2 : 1;   // SIMT: row sums + all gradients
 }
 
-size_t sa2_bwd_workspace_bytes(const sa2_shape *shape) {
-    if (!shape || check_shape(*shape) != SA2_OK) return 0;
+size_t sa2_bwd_workspace_bytes_part(const sa2_shape *shape, int32_t whole_b) {
+    if (!shape || check_shape(*shape) != SA2_OK || whole_b < shape->b) return 0;
     const sa2_shape s = clamped(*shape);
     size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
     delta = (delta + 255) & ~(size_t)255;
-    return delta + sa2::tc::bwd_extra_workspace_bytes(s, shape->w2);
+    return delta + sa2::tc::bwd_extra_workspace_bytes(s, {shape->w2, whole_b});
 }
+
+size_t sa2_bwd_workspace_bytes(const sa2_shape *shape) { return shape ? sa2_bwd_workspace_bytes_part(shape, shape->b) : 0; }
 
 int sa2_fwd(const sa2_fwd_args *a) {
     sa2::nvtx::Range range("sa2_fwd");
@@ -220,11 +222,14 @@ int sa2_fwd(const sa2_fwd_args *a) {
     }
 }
 
-int sa2_bwd(const sa2_bwd_args *a) {
+int sa2_bwd(const sa2_bwd_args *a) { return sa2_bwd_part(a, a ? a->shape.b : 0); }
+
+int sa2_bwd_part(const sa2_bwd_args *a, int32_t whole_b) {
     sa2::nvtx::Range range("sa2_bwd");
     if (int e = check_bwd_args(a)) return e;
+    if (whole_b < a->shape.b) return SA2_ERR_INVALID;
     if (a->phases < 0 || a->phases > (SA2_BWD_ROWSUM | SA2_BWD_K1 | SA2_BWD_Q)) return SA2_ERR_INVALID;
-    const size_t need = sa2_bwd_workspace_bytes(&a->shape);
+    const size_t need = sa2_bwd_workspace_bytes_part(&a->shape, whole_b);
     if (!a->workspace || a->workspace_bytes < need || (reinterpret_cast<uintptr_t>(a->workspace) & 255u))
         return SA2_ERR_WORKSPACE;
 
@@ -240,7 +245,7 @@ int sa2_bwd(const sa2_bwd_args *a) {
     if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !exact && sa2::tc::bwd_scale_ok(s)) {
         size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
         delta = (delta + 255) & ~(size_t)255;
-        return sa2::tc::bwd(p, s, a->shape.w2, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);
+        return sa2::tc::bwd(p, s, {a->shape.w2, whole_b}, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);
     }
 
     switch (s.d) {

@@ -36,7 +36,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // splits of the offsets.  A CTA costs ~12000 cycles of set-up, loads, slab and its share of the reduction, a 64-key unit
 // of a sweep ~1600 (3000 at head dim 128); at most as many offsets per CTA as its accumulators hold.
 struct BqSplit { int tsplit, esplit, epc; };
-inline BqSplit bq_split(const sa2_shape &s, int max_tiles, int sms) {
+inline BqSplit bq_split(const sa2_shape &s, const BwdCaller &call, int max_tiles, int sms) {
     BqSplit r;
     const int nt = tiles_per_query_tile(s.w1), have = (s.n + s.off1 + TJ - 1) / TJ;
     r.tsplit = s.d == 128 ? 1 : (nt + max_tiles - 1) / max_tiles;
@@ -46,8 +46,8 @@ inline BqSplit bq_split(const sa2_shape &s, int max_tiles, int sms) {
     double best_cost = 0.;
     r.esplit = least;
     for (int es = least; es <= w2 && (es <= 16 || es == least); ++es) {
-        const double cost = split_cost(ctas * es, 12000. + (w2 + es - 1) / es * (per * 2. * (s.d == 128 ? 3000. : 1600.)), sms);
-        if (best_cost == 0. || cost < 0.94 * best_cost) { r.esplit = es; best_cost = cost; }
+        const double cost = split_cost(ctas * es, 12000. + (w2 + es - 1) / es * (per * 2. * (s.d == 128 ? 3000. : 1600.)), call.batch, sms);
+        if (best_cost == 0. || cost < SPLIT_GAIN * best_cost) { r.esplit = es; best_cost = cost; }
     }
     r.epc = (w2 + r.esplit - 1) / r.esplit;
     r.esplit = (w2 + r.epc - 1) / r.epc;
@@ -68,11 +68,11 @@ struct BqPlan {
     BqSplit sp;
     int round;           // batch elements that share the scratch at a time
 };
-inline BqPlan bq_plan(const sa2_shape &s, int caller_w2, int sms) {
+inline BqPlan bq_plan(const sa2_shape &s, const BwdCaller &call, int sms) {
     BqPlan p;
-    const bool longer = caller_w2 > BQ_MAX_EPC;
+    const bool longer = call.w2 > BQ_MAX_EPC;
     p.split = s.d == 32 || longer;
-    p.sp = bq_split(s, p.split && s.d == 64 ? BqCfg<64, true>::MAX_TILES : BqCfg<64, false>::MAX_TILES, sms);
+    p.sp = bq_split(s, call, p.split && s.d == 64 ? BqCfg<64, true>::MAX_TILES : BqCfg<64, false>::MAX_TILES, sms);
     p.round = s.b;
     p.tc = true;
     if (longer) {
@@ -93,8 +93,8 @@ inline int n64_products() {
 }
 // scratch after the D vector: per-split partial dQ, the per-CTA dK2/dV2 slabs, partial dK1/dV1
 struct BwdScratch { size_t dq, k2, k1; };
-inline BwdScratch bwd_scratch(const sa2_shape &s, const BqPlan &q) {
-    const K1Split k1 = k1_split(s, SM_COUNT);
+inline BwdScratch bwd_scratch(const sa2_shape &s, const BwdCaller &call, const BqPlan &q) {
+    const K1Split k1 = k1_split(s, call, SM_COUNT);
     BwdScratch b{0, 0, align256(k1_part_bytes(s, k1.si * k1.se))};
     if (q.tc) {
         sa2_shape r = s;
@@ -105,16 +105,16 @@ inline BwdScratch bwd_scratch(const sa2_shape &s, const BqPlan &q) {
     }
     return b;
 }
-inline size_t bwd_extra_workspace_bytes(const sa2_shape &s, int caller_w2) {
+inline size_t bwd_extra_workspace_bytes(const sa2_shape &s, const BwdCaller &call) {
     if (!bwd_supported(s)) return 0;
-    const BwdScratch b = bwd_scratch(s, bq_plan(s, caller_w2, SM_COUNT));
+    const BwdScratch b = bwd_scratch(s, call, bq_plan(s, call, SM_COUNT));
     return b.dq + b.k2 + b.k1;
 }
 // forward: 1 kernel; backward: D = rowsum(O*dO), dK1/dV1, then dQ/dK2/dV2 and the reduction of the partials, per round
-inline int launches(const sa2_shape &s, bool backward, int caller_w2) {
+inline int launches(const sa2_shape &s, bool backward, const BwdCaller &call) {
     if (!backward) return 1;
-    const BqPlan q = bq_plan(s, caller_w2, SM_COUNT);
-    const K1Split k1 = k1_split(s, SM_COUNT);
+    const BqPlan q = bq_plan(s, call, SM_COUNT);
+    const K1Split k1 = k1_split(s, call, SM_COUNT);
     const int rounds = (s.b + q.round - 1) / q.round, k1_reduce = k1.si * k1.se > 1;
     return !q.tc ? 3 + k1_reduce : rounds == 1 ? 4 : 2 + 2 * rounds + k1_reduce;
 }
@@ -271,18 +271,18 @@ inline KernelParams batch_part(KernelParams kp, int b0, int nb) {
 }
 
 template <int D>
-inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, int caller_w2, void *extra, cudaStream_t st, int phases) {
+inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, const BwdCaller &call, void *extra, cudaStream_t st, int phases) {
     const float c = s.scale * 1.4426950408889634f;
     int *status = status_word();
     if (!status) return SA2_ERR_CUDA;
     if (phases == 0) phases = SA2_BWD_ROWSUM | SA2_BWD_K1 | SA2_BWD_Q;
     // D_i = sum_c O_ic dO_ic
     if ((phases & SA2_BWD_ROWSUM) && !simt::launch_delta<D>(kp, st)) return SA2_ERR_CUDA;
-    BqPlan plan = bq_plan(s, caller_w2, SM_COUNT);
+    BqPlan plan = bq_plan(s, call, SM_COUNT);
     // fp32 gradients show the last bits, which AUTO leaves to the fp32 kernels
-    if (s.kernel == SA2_KERNEL_AUTO && !kp.grad_bf16 && caller_w2 > BQ_MAX_EPC) plan.tc = false;
-    const BwdScratch room = bwd_scratch(s, plan);
-    const K1Split k1 = k1_split(s, SM_COUNT);
+    if (s.kernel == SA2_KERNEL_AUTO && !kp.grad_bf16 && call.w2 > BQ_MAX_EPC) plan.tc = false;
+    const BwdScratch room = bwd_scratch(s, call, plan);
+    const K1Split k1 = k1_split(s, call, SM_COUNT);
     BqParams Q;
     Q.kp = kp;
     Q.c = c;
@@ -322,12 +322,12 @@ inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, int caller_w2,
     return bwd_reduce_launch<D>(Q, st);
 }
 
-inline int bwd(const KernelParams &kp, const sa2_shape &s, int caller_w2, void *extra, cudaStream_t st, int phases = 0) {
+inline int bwd(const KernelParams &kp, const sa2_shape &s, const BwdCaller &call, void *extra, cudaStream_t st, int phases = 0) {
     if (!bwd_addressable(kp)) return SA2_ERR_INVALID;
     switch (s.d) {
-        case 32: return bwd_launch<32>(kp, s, caller_w2, extra, st, phases);
-        case 64: return bwd_launch<64>(kp, s, caller_w2, extra, st, phases);
-        default: return bwd_launch<128>(kp, s, caller_w2, extra, st, phases);
+        case 32: return bwd_launch<32>(kp, s, call, extra, st, phases);
+        case 64: return bwd_launch<64>(kp, s, call, extra, st, phases);
+        default: return bwd_launch<128>(kp, s, call, extra, st, phases);
     }
 }
 

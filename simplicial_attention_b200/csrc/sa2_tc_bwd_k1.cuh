@@ -541,17 +541,23 @@ bwd_k1_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------ host side
-// The weight of splitting work into `ctas` CTAs per batch element of `one` cycles each: whole waves of one CTA per SM.  A
-// result must not depend, to the last bit, on what else rides in the call, so the rules weigh one batch element (where
-// splitting fills the chip) and eight (where it costs set-up).
-inline double split_cost(int64_t ctas, double one, int sms) {
-    return (double)((ctas + sms - 1) / sms) * one * ((double)((ctas * 8 + sms - 1) / sms) * one);
-}
+// What the split rules look at besides the (clamped) shape.
+struct BwdCaller {
+    int w2;        // the caller's second window, however short the sequence
+    int batch;     // batch elements of the whole call: a part of it (sa2_bwd_part) is cut as the whole is, for the same bits
+};
+// Cycles of `batch` times `ctas` CTAs of `one` cycles each: whole waves of one CTA per SM.
+// A rule for one and for eight elements at once, which needed no batch, cost many short sequences dear: with eight ranges
+// of offsets in both kernels b128 n128 h8 d64 w512/32 took 2506 us and 2.0 GiB of scratch, 988 us and 80 MiB with one.
+// A split must promise 8 %: at 7 % b2 n4096 h8 d64 w512/32 (3.5 waves of CTAs into 6.9 shorter ones) got 5 % slower.
+constexpr double SPLIT_GAIN = 0.92;
+inline double split_cost(int64_t ctas, double one, int batch, int sms) { return (double)((ctas * batch + sms - 1) / sms) * one; }
 // CTAs per key tile: splits of the (query head, query tile) pairs first, then of the offsets.  A CTA costs ~8000 cycles
 // of set-up, loads and store, a pair ~4000 (its rows and second-key window), a step of 128 query rows and one offset
-// ~2600 (twice that at head dim 128), measured on a B200.
+// ~2600 (twice that at head dim 128), measured on a B200; twice as much again with more than 32 offsets, whose second keys
+// do not fit the staged window (b5 n1500 hq16 hk2 d128 w700/40 with 40 offsets per CTA 5441 us, with 5 of them 2815).
 struct K1Split { int si, se, epc; };
-inline K1Split k1_split(const sa2_shape &s, int sms) {
+inline K1Split k1_split(const sa2_shape &s, const BwdCaller &call, int sms) {
     const int nk1 = s.n + s.off1, rows = s.w1 + TJ - 1 < s.n ? s.w1 + TJ - 1 : s.n;
     const int64_t tiles = (int64_t)((nk1 + TJ - 1) / TJ) * s.hk;
     const int pairs = (s.hq / s.hk) * ((rows + TQ - 1) / TQ), w2 = s.w2 < s.n + s.off2 ? s.w2 : s.n + s.off2;
@@ -561,8 +567,8 @@ inline K1Split k1_split(const sa2_shape &s, int sms) {
     for (int se = 1; se <= 16 && se <= w2; ++se)
         for (int si = 1; si * se <= 16 && si <= pairs; ++si) {
             const int epc = (w2 + se - 1) / se;
-            const double cost = split_cost(tiles * si * se, 8000. + (pairs + si - 1) / si * (4000. + epc * step), sms);
-            if (best_cost == 0. || cost < 0.94 * best_cost) { best = K1Split{si, (w2 + epc - 1) / epc, epc}; best_cost = cost; }
+            const double cost = split_cost(tiles * si * se, 8000. + (pairs + si - 1) / si * (4000. + epc * (epc > 32 ? 2. : 1.) * step), call.batch, sms);
+            if (best_cost == 0. || cost < SPLIT_GAIN * best_cost) { best = K1Split{si, (w2 + epc - 1) / epc, epc}; best_cost = cost; }
         }
     return best;
 }

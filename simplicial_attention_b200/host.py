@@ -138,7 +138,7 @@ class HostPipeline:
                     self.s_run.wait_event(self.copied[slot])      # the last results of this slot are on the host
                 out, lse = sa2_forward(q, k1, k2, v1, v2, self.w1, self.w2, kernel=self.kernel, out=res[0])
                 grads = sa2_backward(q, k1, k2, v1, v2, out, lse, dout, self.w1, self.w2, kernel=self.kernel,
-                                     grad_dtype=res[1].dtype, grads=res[1:])
+                                     grad_dtype=res[1].dtype, grads=res[1:], whole_batch=b)
                 done = torch.cuda.Event()
                 done.record(self.s_run)
                 self.free[slot] = done
