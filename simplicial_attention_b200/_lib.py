@@ -147,7 +147,7 @@ def ext():
         import torch  # noqa: F401  (its libraries must be loaded first)
 
         from . import build
-        path = build.build_ext()
+        path = build.build_ext(force=bool(os.environ.get("SA2_REBUILD")))
         spec = importlib.util.spec_from_file_location("_sa2_torch", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)

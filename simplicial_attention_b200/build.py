@@ -2,7 +2,7 @@
 
     python -m simplicial_attention_b200.build [--force] [--verbose]
 
-Produces ``simplicial_attention_b200/libsa2.so`` (C ABI in ``include/sa2.h``) and ``_sa2_torch.so`` (the argument
+Produces ``simplicial_attention_b200/libsa2.so`` (C ABI in ``include/sa2.h``) and ``_sa2_torch.<versions>.so`` (the argument
 blocks, allocations and autograd nodes of the Python entry points in C++, against torch's headers).
 nvcc cross-compiles without a GPU, so this also serves as the build check.
 """
@@ -17,7 +17,6 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libsa2.so")
-EXT = os.path.join(PKG, "_sa2_torch.so")
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -47,18 +46,30 @@ def is_stale() -> bool:
     return any(os.path.getmtime(f) > t for f in _inputs())
 
 
+def ext_path() -> str:
+    """The extension is C++ against the headers of one Python and one torch: their versions are part of its name, so that
+    another torch in the same tree builds its own instead of loading this one's."""
+    import sysconfig
+
+    import torch
+    tag = f"{sysconfig.get_config_var('SOABI')}-torch{torch.__version__}-cxx11abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
+    return os.path.join(PKG, f"_sa2_torch.{tag.replace('+', '_')}.so")
+
+
 def ext_is_stale() -> bool:
-    if not os.path.exists(EXT):
+    path = ext_path()
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(EXT)
+    t = os.path.getmtime(path)
     return any(os.path.getmtime(f) > t for f in (os.path.join(CSRC, "sa2_torch.cpp"), os.path.join(ROOT, "include", "sa2.h"),
                                                  os.path.abspath(__file__)))
 
 
 def build_ext(force: bool = False) -> str:
-    """Compile _sa2_torch.so if it is missing or older than its sources (host code only, so g++)."""
+    """Compile the extension if it is missing or older than its sources (host code only, so g++)."""
+    path = ext_path()
     if not force and not ext_is_stale():
-        return EXT
+        return path
     import sysconfig
 
     import torch
@@ -66,7 +77,7 @@ def build_ext(force: bool = False) -> str:
     lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     includes = [os.path.join(ROOT, "include"), *cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    tmp = EXT + f".{os.getpid()}.tmp"
+    tmp = path + f".{os.getpid()}.tmp"
     cmd = [
         shutil.which("g++") or "g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-DTORCH_EXTENSION_NAME=_sa2_torch", "-DTORCH_API_INCLUDE_EXTENSION_H",
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[x for d in includes for x in ("-isystem", d)],
@@ -76,8 +87,8 @@ def build_ext(force: bool = False) -> str:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
-    os.replace(tmp, EXT)
-    return EXT
+    os.replace(tmp, path)
+    return path
 
 
 def build(force: bool = False, verbose: bool = False, out: str = LIB, defines: tuple[str, ...] = ()) -> str:
