@@ -12,6 +12,28 @@ from simplicial_attention_b200.headnorm import head_rmsnorm
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture
+def native(monkeypatch):
+    """Names of the native module calls that answered (a None sends the module to its general path)."""
+    real, answered = _lib.ext(), []
+
+    class Counted:
+        def __getattr__(self, name):
+            f = getattr(real, name)
+            if name not in ("qkv_attn", "qkv_attn_cached", "step"):
+                return f
+
+            def call(*args):
+                res = f(*args)
+                if res is not None:
+                    answered.append(name)
+                return res
+            return call
+
+    monkeypatch.setattr(_lib, "ext", lambda: Counted())
+    return answered
+
+
 def _module(hq, hk, d, w1, w2, dtype, seed=0):
     torch.manual_seed(seed)
     m = SlidingWindowTwoSimplicialMHA(dim=64, dim_head=d, heads=hq, key_value_heads=hk, prenorm=True, w1=w1, w2=w2).to("cuda", dtype)
@@ -35,7 +57,7 @@ def _general(m):
     (3, 1, 128, 40, torch.bfloat16, False),
     (8, 4, 64, 130, torch.float32, True),
 ])
-def test_training_pass_equals_the_general_path(hq, hk, d, n, dtype, autocast):
+def test_training_pass_equals_the_general_path(native, hq, hk, d, n, dtype, autocast):
     res = []
     for general in (False, True):
         m = _module(hq, hk, d, 24, 5, dtype)
@@ -44,6 +66,7 @@ def test_training_pass_equals_the_general_path(hq, hk, d, n, dtype, autocast):
         x = torch.randn(2, n, 64, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).to(dtype).requires_grad_()
         with torch.autocast("cuda", dtype=torch.bfloat16, enabled=autocast):
             out = m(x)
+        assert native == ["qkv_attn"]           # the first module's call, and none of the second's
         out.backward(torch.randn(out.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(2)).to(out.dtype))
         res.append([out.detach(), x.grad] + [p.grad for p in m.parameters()])
     tol = 1e-5 if dtype == torch.float32 and not autocast else 1e-2
@@ -57,7 +80,7 @@ def test_training_pass_equals_the_general_path(hq, hk, d, n, dtype, autocast):
     (3, 4, 2, 32, torch.bfloat16, 40),
     (2, 2, 1, 128, torch.float32, 17),
 ])
-def test_generation_equals_the_general_path(b, hq, hk, d, dtype, prompt):
+def test_generation_equals_the_general_path(native, b, hq, hk, d, dtype, prompt):
     w1, w2 = 20, 4
     fast, slow = _module(hq, hk, d, w1, w2, dtype), _general(_module(hq, hk, d, w1, w2, dtype))
     x = torch.randn(b, prompt + 6, 64, device="cuda").to(dtype)
@@ -72,6 +95,7 @@ def test_generation_equals_the_general_path(b, hq, hk, d, dtype, prompt):
             for s, t in zip(*states):
                 for a, c in zip(s, t):
                     assert a.shape == c.shape and (a - c).float().norm() <= 1e-2 * c.float().norm()
+    assert native == ["step"] * 4
 
 
 @pytest.mark.parametrize("dim,pre,post,hook", [
@@ -80,7 +104,7 @@ def test_generation_equals_the_general_path(b, hq, hk, d, dtype, prompt):
     (64, False, False, False),
     (64, True, False, True),                   # a hooked submodule has to be called
 ])
-def test_generation_step_of_plain_and_hooked_modules(dim, pre, post, hook):
+def test_generation_step_of_plain_and_hooked_modules(native, dim, pre, post, hook):
     torch.manual_seed(0)
     m = SlidingWindowTwoSimplicialMHA(dim=dim, dim_head=64, heads=4, key_value_heads=2, prenorm=pre, postnorm=post, w1=20, w2=4)
     m = m.to("cuda", torch.bfloat16)
@@ -92,8 +116,9 @@ def test_generation_step_of_plain_and_hooked_modules(dim, pre, post, hook):
         want = m(x)
         _, cache = m(x[:, :25], return_cache=True)
         calls.clear()
+        native.clear()
         got, _ = m(x[:, 25:], cache=cache, return_cache=True)
-    assert bool(calls) == hook
+    assert bool(calls) == hook and native == ["qkv_attn_cached" if hook else "step"]
     assert (got - want[:, 25:]).float().norm() <= 1e-2 * want[:, 25:].float().norm()
 
 
@@ -109,12 +134,15 @@ def test_projection_of_few_rows(rows, k, outs):
     assert (y[rows] == 7).all()
 
 
-def test_other_attend_callables_still_run():
+def test_other_attend_callables_still_run(native):
     m = _module(2, 2, 64, 16, 4, torch.float32)
     x = torch.randn(1, 30, 64, device="cuda")
     ref = m(x)
     m.attend = partial(sliding_two_simplicial_attn, w1=16, w2=4, kernel="simt")
     assert torch.allclose(m(x), ref, atol=1e-5)
+    assert native == ["qkv_attn"] * 2
+    m.attend = lambda q, k, v: sliding_two_simplicial_attn(q, k, v, w1=16, w2=4)
+    assert torch.allclose(m(x), ref, atol=1e-5) and native == ["qkv_attn"] * 2
     with pytest.raises(KeyError):
         m.attend = partial(sliding_two_simplicial_attn, w1=16, w2=4, kernel="other")
         m(x)
