@@ -230,7 +230,7 @@ __device__ __forceinline__ int builder(const Params &P, const Geom &g, const CUt
     return 0;
 }
 
-// ---------------------------------------------------------------- issuers of S^T (warp 1) and dP^T (warp 2), one lane each
+// ---------------------------------------------------------------- issuers of S^T (warp 1) and dP^T (warp 2)
 // Step s uses stage s % 3 and TMEM half s % 2.
 __device__ __forceinline__ int mma_first(const KernelParams &kp, const Geom &g, int which, uint32_t tmem, uint8_t *sKV,
                                          uint8_t *sAB, uint8_t *sConst, uint64_t *bars, volatile int *abort_flag) {
@@ -268,7 +268,7 @@ __device__ __forceinline__ int mma_first(const KernelParams &kp, const Geom &g, 
     return 0;
 }
 
-// ---------------------------------------------------------------- issuer of dV1, dK1 (warp 0, one lane)
+// ---------------------------------------------------------------- issuer of dV1, dK1 (warp 0)
 __device__ __forceinline__ int mma_second(const Params &P, const Geom &g, uint32_t tmem, uint8_t *sAB, uint64_t *bars,
                                           volatile int *abort_flag) {
     constexpr uint32_t IDESC_G = idesc_bf16(128, 128, false, true);     // B operand MN-major, N = 128

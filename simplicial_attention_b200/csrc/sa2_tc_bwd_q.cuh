@@ -17,6 +17,9 @@
 // 64-row units stream through a three-slot TMA ring (32 KB per slot), once per sweep, from L2: a slot is
 // refilled when the U / W products of its unit are done, one unit ahead of the S / dP products that need it.
 //
+// SPLIT (head dim 32, and second windows above 56 rows: see bq_plan) keeps A_e, B_e, P and G as a bf16 value and a bf16 rest
+// each, with twice the products; the rests cost a K1/V1 tile at head dim 64 and two of the three ring slots at 128.
+//
 // Per offset e ("sweep") the fold groups form A_e = q_i * k2_{i-e} and B_e = dO_i * v2_{i-e}; per 64-key
 // unit the tensor cores compute
 //     S = A_e K1^T      dP = B_e V1^T                 (rows i, columns j)
@@ -200,10 +203,10 @@ __device__ __forceinline__ BqGeom bq_geom(const BqParams &P) {
     return g;
 }
 
-// ---------------------------------------------------------------- issuers of S (warp 1) and dP (warp 2), one lane each
+// ---------------------------------------------------------------- issuers of S (warp 1) and dP (warp 2)
 // Unit u (numbered over the whole kernel) is unit u % nunits of sweep u / nunits and uses TMEM buffer u % NBUF.
-// One thread issues about one tcgen05.mma per 60-90 cycles, so the two product stages have an issuing
-// thread each; U / W are accumulated by one thread only, which keeps the summation order fixed.
+// A warp issues about one tcgen05.mma per 45-90 cycles, so the two product stages have an issuing warp
+// each; U / W are accumulated by one warp only, which keeps the summation order fixed.
 // which = 0: S = A_e K1^T into columns [128 buf, +64); which = 1: dP = B_e V1^T into [128 buf + 64, +64).
 template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t tmem, uint8_t *sKV, uint8_t *sAB,
@@ -256,7 +259,7 @@ __device__ __forceinline__ int bq_mma_first(const BqGeom &g, int which, uint32_t
     return 0;
 }
 
-// ---------------------------------------------------------------- head dim 128: TMA producer of the K1/V1 ring (warp 3, one lane)
+// ---------------------------------------------------------------- head dim 128: TMA producer of the K1/V1 ring (warp 3)
 template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_ring_producer(const BqParams &P, const BqGeom &g, const CUtensorMap *mapK, const CUtensorMap *mapV,
                                                 uint8_t *sK, uint8_t *sV, uint64_t *bars, volatile int *abort_flag) {
@@ -286,9 +289,9 @@ __device__ __forceinline__ int bq_ring_producer(const BqParams &P, const BqGeom 
     return 0;
 }
 
-// ---------------------------------------------------------------- issuers of U, W (one lane each)
+// ---------------------------------------------------------------- issuers of U, W
 // part 0 (warp 0; head dim 64: after loading the tiles): U += G K1; part 1 (warp 3): W += P V1; part 2 (head dim
-// 128, warp 0): both.  Each accumulator has one issuing thread, which keeps its summation order fixed.
+// 128, warp 0): both.  Each accumulator has one issuing warp, which keeps its summation order fixed.
 template <int D, bool SPLIT>
 __device__ __forceinline__ int bq_mma_second(const BqParams &P, const BqGeom &g, int part, const CUtensorMap *mapK, const CUtensorMap *mapV,
                                              uint32_t tmem, uint8_t *sK, uint8_t *sV, uint64_t *bars, volatile int *abort_flag) {

@@ -12,7 +12,8 @@
 //
 // Why pairs: the window of RI rows is w1 + RI - 1 keys, so a small RI wastes fewer masked columns (w1 = 512:
 // 576 columns at RI = 64, 640 at RI = 128), a short sequence is spread over more CTAs of fewer sweeps each,
-// and a single new token (generation) still fills the rows of its tile.  fwd_ri_log2() picks RI.
+// and a single new token (generation) takes 16 offsets of its window at a time: 16 live rows of a tile of RI = 8, the
+// smallest.  fwd_ri_log2() picks RI.
 //
 // Warp roles (512 threads, four aligned warpgroups):
 //   warp 0, 1     issue the tcgen05.mma stream of group 0 / group 1 (warp 1 owns the TMEM allocation)

@@ -32,14 +32,14 @@
 //     folded in.
 //
 // Warps (768 threads, six aligned warpgroups):
-//   0, 1   lane 0 issues the S products of group 0 / group 1 (warp 1 owns the TMEM allocation)
-//   2, 3   lane 0 issues the P V1 products of group 0 / group 1.  A thread issues one tcgen05
+//   0, 1   issue the S products of group 0 / group 1 (warp 1 owns the TMEM allocation)
+//   2, 3   issue the P V1 products of group 0 / group 1.  A warp issues one tcgen05
 //          instruction per 60-130 cycles and a unit takes 12 products and 6 commits, so with one
 //          issuing thread per group the issue itself (~3900 cycles per unit) paced the kernel.
 //   4-7    output threads of channel block 0, one per query row
 //   8-11   output threads of channel block 1
 //   12-15  softmax group 0 (even sweeps), 16-19 softmax group 1 (odd sweeps)
-//   20, 21 lane 0 is the TMA producer of the K1 ring / of the V1 ring; 22-23 idle
+//   20, 21 TMA producers of the K1 ring / of the V1 ring; 22-23 idle
 #pragma once
 #include "sa2_tc_fwd.cuh"
 
@@ -100,7 +100,7 @@ inline int win_boxes(int w2, int ri_log2) {
 }
 using Geom = FwdGeom;
 
-// ------------------------------------------------------------------ TMA producers (warps 2 and 3, one lane each)
+// ------------------------------------------------------------------ TMA producers (warps 20 and 21)
 // Item x = (pair of sweeps x / nunits, unit x % nunits) goes to slot x % SLOTS; the walk is the one of
 // group 0, which has at least as many sweeps as group 1.
 __device__ __forceinline__ int producer(const Params &P, const Geom &g, const CUtensorMap *map, const CUtensorMap *mapV2, uint8_t *ring, uint8_t *sWin, int full0, int empty0,
@@ -133,7 +133,7 @@ __device__ __forceinline__ int producer(const Params &P, const Geom &g, const CU
     return 0;
 }
 
-// ------------------------------------------------------------------ MMA issuers (two lanes per group)
+// ------------------------------------------------------------------ MMA issuers (two warps per group)
 // Group g's units: unit r is unit r % nunits of the group's (r / nunits)-th sweep, e = 2 (r / nunits) + g,
 // in ring slot r % SLOTS.  Buffer r & 1 of the group holds S, then P, of unit r.  The S products and the
 // P V1 products of a group are issued by two threads; everything that orders them goes through barriers.

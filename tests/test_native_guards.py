@@ -132,3 +132,18 @@ def test_lowered_channel_limit_runs_the_norm_modules(limit, modules_run):
     m.q_norm.register_forward_hook(lambda *a: calls.append(1))
     m(x)
     assert bool(calls) == modules_run
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_python_function_equals_the_native_node(dtype):
+    """The autograd function behind the calls that the native node declines: same bits, forward and backward."""
+    cls = sa.SlidingTwoSimplicialAttention
+    ins = [torch.randn(2, 70, h, D, device="cuda").to(dtype).requires_grad_() for h in (HQ, HK, HK, HK, HK)]
+    dout = torch.randn(2, 70, HQ, D, device="cuda").to(dtype)
+    res = []
+    for apply in (cls.apply, super(cls, cls).apply):
+        out, lse = apply(*ins, W1, W2, True, None, "auto", True)
+        assert not lse.requires_grad
+        res.append([out, lse, *torch.autograd.grad(out, ins, dout)])
+    assert all(torch.equal(a, b) for a, b in zip(*res))
