@@ -41,6 +41,14 @@ def _usable(t: Tensor) -> Tensor:
     return t if ok else t.contiguous()
 
 
+def _usable_kv(t: Tensor) -> Tensor:
+    """The same for keys and values, which the bf16 kernels load with TMA: it cannot repeat a dimension, so an expanded
+    tensor is copied."""
+    if t.dtype == torch.bfloat16 and any(s == 0 and n > 1 for s, n in zip(t.stride(), t.shape)):
+        return t.contiguous()
+    return _usable(t)
+
+
 def _strides(t: Tensor) -> _lib.Strides:
     return _lib.Strides(t.stride(0), t.stride(1), t.stride(2))
 
@@ -88,7 +96,7 @@ def sa2_forward(q, k1, k2, v1, v2, w1, w2, scale=None, kernel="auto", out=None):
     preallocated tensor or strided view to write the result into.
     """
     _check_inputs(q, k1, k2, v1, v2)
-    q, k1, k2, v1, v2 = (_usable(t) for t in (q, k1, k2, v1, v2))
+    q, k1, k2, v1, v2 = _usable(q), *(_usable_kv(t) for t in (k1, k2, v1, v2))
     b, n, hq, d = q.shape
     scale = d ** -0.5 if scale is None else scale
     if out is None:
@@ -118,7 +126,8 @@ class BackwardCall:
     def __init__(self, q, k1, k2, v1, v2, out, lse, dout, w1, w2, scale=None, kernel="auto", grad_dtype=None,
                  grads=None, whole_batch=None):
         _check_inputs(q, k1, k2, v1, v2)
-        q, k1, k2, v1, v2, out, dout = (_usable(t) for t in (q, k1, k2, v1, v2, out, dout))
+        q, out, dout = (_usable(t) for t in (q, out, dout))
+        k1, k2, v1, v2 = (_usable_kv(t) for t in (k1, k2, v1, v2))
         if dout.dtype != q.dtype:
             dout = dout.to(q.dtype)
         lse = lse.contiguous()

@@ -139,10 +139,14 @@ inline int *status_word() {
     return ptrs[dev];
 }
 
+// keys and values, which TMA loads: a tensor map cannot repeat a dimension (stride 0, an expanded tensor)
+inline bool kv_addressable(const TensorRef &t, const KernelParams &kp, int rows) {
+    return tma_addressable(t) && (t.sb != 0 || kp.b == 1) && (t.sn != 0 || rows == 1) && (t.sh != 0 || kp.hk == 1);
+}
 // 16-byte vector access and TMA need 16-byte aligned bases and strides that are multiples of 8 elements
 inline bool fwd_addressable(const KernelParams &kp) {
-    return tma_addressable(kp.k1) && tma_addressable(kp.v1) && tma_addressable(kp.q) && tma_addressable(kp.k2) &&
-           tma_addressable(kp.v2) && tma_addressable(kp.out);
+    return kv_addressable(kp.k1, kp, kp.nk1) && kv_addressable(kp.v1, kp, kp.nk1) && kv_addressable(kp.k2, kp, kp.nk2) &&
+           kv_addressable(kp.v2, kp, kp.nk2) && tma_addressable(kp.q) && tma_addressable(kp.out);
 }
 
 inline int fwd128(const KernelParams &kp, const sa2_shape &s, cudaStream_t st) {

@@ -78,6 +78,13 @@ Tensor usable(const Tensor &t) {
     const bool ok = t.stride(3) == 1 && t.stride(0) % 4 == 0 && t.stride(1) % 4 == 0 && t.stride(2) % 4 == 0 && aligned(t);
     return ok ? t : t.contiguous();
 }
+// keys and values, which the bf16 kernels load with TMA: it cannot repeat a dimension (an expanded tensor)
+Tensor usable_kv(const Tensor &t) {
+    if (t.scalar_type() == at::kBFloat16)
+        for (int x = 0; x < 3; ++x)
+            if (t.stride(x) == 0 && t.size(x) > 1) return t.contiguous();
+    return usable(t);
+}
 sa2_strides strides(const Tensor &t) { return sa2_strides{t.stride(0), t.stride(1), t.stride(2)}; }
 
 struct Cfg {
@@ -145,7 +152,7 @@ struct Attn : torch::autograd::Function<Attn> {
         const c10::cuda::CUDAGuard guard(q.device());
         const Cfg c{w1, w2, kernel, scale};
         Tensor out, lse;
-        run_forward(usable(q), usable(k1), usable(k2), usable(v1), usable(v2), c, out, lse);
+        run_forward(usable(q), usable_kv(k1), usable_kv(k2), usable_kv(v1), usable_kv(v2), c, out, lse);
         ctx->save_for_backward({q, k1, k2, v1, v2, out, lse});
         ctx->saved_data["w1"] = w1;
         ctx->saved_data["w2"] = w2;
@@ -163,7 +170,7 @@ struct Attn : torch::autograd::Function<Attn> {
         if (dout.scalar_type() != s[0].scalar_type()) dout = dout.to(s[0].scalar_type());
         Tensor g[5];
         for (int x = 0; x < 5; ++x) g[x] = at::empty(s[x].sizes(), s[x].options());
-        run_backward(usable(s[0]), usable(s[1]), usable(s[2]), usable(s[3]), usable(s[4]), s[5], s[6], dout, c, g);
+        run_backward(usable(s[0]), usable_kv(s[1]), usable_kv(s[2]), usable_kv(s[3]), usable_kv(s[4]), s[5], s[6], dout, c, g);
         return {g[0], g[1], g[2], g[3], g[4], Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
