@@ -49,3 +49,17 @@ def test_strides_of_zero_at_the_abi(form):
                             *(_strides(t) for t in (q, k1, k2, v1, v2, out)), torch.cuda.current_stream().cuda_stream)
         assert _lib.lib().sa2_fwd(C.byref(args)) == status
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("d,w1,w2", [(32, 100, 9), (64, 100, 9), (64, 600, 70), (128, 100, 9)])
+def test_head_first_memory(d, w1, w2):
+    """Operands and output gradient stored (b, h, n, d): strides in another order, read in place."""
+    q, kv, dout = _operands("batch", d, torch.bfloat16)
+    plain = [t.contiguous() for t in (q, *kv, dout)]
+    turned = [t.transpose(1, 2).contiguous().transpose(1, 2) for t in plain]
+    res = []
+    for q, k1, k2, v1, v2, do in (plain, turned):
+        out, lse = sa.sa2_forward(q, k1, k2, v1, v2, w1, w2)
+        res.append([out, lse, *sa.sa2_backward(q, k1, k2, v1, v2, out, lse, do, w1, w2)])
+    assert sa.device_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(*res))
