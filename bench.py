@@ -323,8 +323,7 @@ def run_c4(args):
 
 def load_traffic():
     """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the tensor-core kernels, taken
-    from the ncu captures summarised under profiles/ and scaled to a full launch where the capture was a
-    smaller case.  Keyed by "<workload>:<kernel>"."""
+    from the ncu captures of the same workload summarised under profiles/.  Keyed by "<workload>:<kernel>"."""
     path = os.path.join(ROOT, "profiles", "dram_traffic.json")
     try:
         with open(path) as f:

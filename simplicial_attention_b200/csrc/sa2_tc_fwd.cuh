@@ -33,7 +33,7 @@
 // the issuing thread of a group alternates P V1 of unit u and S of unit u + 2, whose completion therefore also says
 // that the P columns are free - and which 32-column chunks need no mask, or are seen by nobody, is decided from
 // warp-uniform bounds without votes.
-// Measured: b4 n4096 h8 d64 w512/32 1.26 -> 0.96 ms (537 TFLOP/s), b2 n1024 0.178 -> 0.141 ms; one new row of b1 h8 behind a
+// Measured: b4 n4096 h8 d64 w512/32 1.26 -> 0.95 ms (543 TFLOP/s), b2 n1024 0.179 -> 0.139 ms; one new row of b1 h8 behind a
 // full window 0.19 -> 0.017 ms.
 // Measured and not kept, where this form takes 0.96 (or, earlier, 1.12) ms: A in TMEM with one P buffer (1.5 against 1.12),
 // 128-key units (1.4), S and P V1 from separate issuing threads (1.15), S(u + 2) before P V1(u) (1.19), ordering the
@@ -42,9 +42,8 @@
 //
 // SPLIT (head dim 32, and head dim 64 with w1 > 513: see fwd_split): A and P are each a bf16 value and a bf16 rest, so S and
 // P V1 take two products per K step instead of one, with the rests of P over the S columns they come from.  The softmax
-// groups pack twice as many words, which is what the time goes to: b1 n3001 h8 d64 w1024/16 0.208 -> 0.269 ms,
-// b4 n4096 h8 d64 w1024/32 1.63 -> 2.27 ms, d32 w512/32 0.90 -> 1.12 ms against rounded operands; 4.15, 34 and 12.6 ms on the
-// fp32 kernels.
+// groups pack twice as many words, which is what the time goes to: b1 n3001 h8 d64 w1024/16 0.207 -> 0.250 ms, b4 n4096 h8 d32
+// w512/32 0.90 -> 1.08 ms against rounded operands; 4.15 and 12.6 ms on the fp32 kernels.
 //
 // Reference handling: probabilities are computed against a per-row reference
 // that only moves when it must, so the W accumulator in TMEM normally never
