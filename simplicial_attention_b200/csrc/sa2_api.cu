@@ -4,6 +4,7 @@
 #include "sa2_common.cuh"
 #include "sa2_simt.cuh"
 #include "sa2_tc.cuh"
+#include "sa2_f32.cuh"
 #include "sa2_headnorm.cuh"
 #include "sa2_rows_linear.cuh"
 #include <nvtx3/nvToolsExt.h>
@@ -180,6 +181,7 @@ int sa2_kernel_launches(const sa2_shape *shape, int backward) {
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
     if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !(backward && !sa2::tc::bwd_scale_ok(s)))
         return sa2::tc::launches(s, backward != 0, {shape->w2, shape->b});
+    if (sa2::f32::supported(s) && backward) return sa2::f32::bwd_launches(s, shape->b, sa2::tc::SM_COUNT);
     return backward ? 2 : 1;   // SIMT: row sums + all gradients
 }
 
@@ -188,6 +190,7 @@ size_t sa2_bwd_workspace_bytes_part(const sa2_shape *shape, int32_t whole_b) {
     const sa2_shape s = clamped(*shape);
     size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
     delta = (delta + 255) & ~(size_t)255;
+    if (sa2::f32::supported(s)) return delta + sa2::f32::bwd_workspace_bytes(s, whole_b, sa2::tc::SM_COUNT);
     return delta + sa2::tc::bwd_extra_workspace_bytes(s, {shape->w2, whole_b});
 }
 
@@ -214,6 +217,12 @@ int sa2_fwd(const sa2_fwd_args *a) {
     const bool tc_ok = sa2::tc::fwd_supported(s) && sa2::tc::fwd_addressable(p);
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
     if (tc_ok && s.kernel != SA2_KERNEL_SIMT) return sa2::tc::fwd(p, s, sa2::tc::fwd_split(a->shape), st);
+
+    if (sa2::f32::supported(s)) {
+        int *status = sa2::tc::status_word();
+        if (!status) return SA2_ERR_CUDA;
+        return s.d == 32 ? sa2::f32::fwd<32>(p, status, sa2::tc::SM_COUNT, st) : sa2::f32::fwd<64>(p, status, sa2::tc::SM_COUNT, st);
+    }
 
     switch (s.d) {
         case 32: return simt_fwd<32>(p, st);
@@ -242,10 +251,18 @@ int sa2_bwd_part(const sa2_bwd_args *a, int32_t whole_b) {
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return SA2_ERR_UNSUPPORTED;
     // (fp32 gradients at head dim 32 show the last bits, which AUTO leaves to the fp32 kernels)
     const bool exact = s.kernel == SA2_KERNEL_AUTO && s.d == 32 && a->grad_dtype == SA2_F32;
+    size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
+    delta = (delta + 255) & ~(size_t)255;
     if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !exact && sa2::tc::bwd_scale_ok(s)) {
-        size_t delta = (size_t)s.b * s.hq * s.n * sizeof(float);
-        delta = (delta + 255) & ~(size_t)255;
         return sa2::tc::bwd(p, s, {a->shape.w2, whole_b}, reinterpret_cast<char *>(a->workspace) + delta, st, a->phases);
+    }
+
+    if (sa2::f32::supported(s)) {
+        const sa2::f32::Plan plan = sa2::f32::plan(s, whole_b, sa2::tc::SM_COUNT);
+        int *status = sa2::tc::status_word();
+        if (!status) return SA2_ERR_CUDA;
+        char *extra = reinterpret_cast<char *>(a->workspace) + delta;
+        if (plan.tc) return s.d == 32 ? sa2::f32::bwd<32>(p, plan, extra, status, st, a->phases) : sa2::f32::bwd<64>(p, plan, extra, status, st, a->phases);
     }
 
     switch (s.d) {

@@ -1,0 +1,112 @@
+// Host side of the fp32 kernels on the tensor cores: which calls they take, splits, scratch, launches.
+#pragma once
+#include "sa2.h"
+#include "sa2_f32_fwd.cuh"
+#include "sa2_f32_bwd.cuh"
+#include "sa2_simt.cuh"
+
+namespace sa2 {
+namespace f32 {
+
+// fp32 tensors at head dims 32 and 64, any window, any strides the ABI takes.  (Head dim 128: the three terms of A_e, B_e and of
+// a unit of K1 and V1 do not fit the shared memory of an SM.)
+inline bool supported(const sa2_shape &s) { return s.kernel == SA2_KERNEL_AUTO && s.dtype == SA2_F32 && s.d <= 64; }
+
+template <int D> inline int fwd(const KernelParams &kp, int *status, int sms, cudaStream_t st) {
+    const int tiles = (kp.n + ROWS - 1) / ROWS, ce = simt::cluster_size((int64_t)tiles * kp.hq, kp.w2, 2, sms);
+    return simt::launch_clusters(fwd_kernel<D>, dim3(tiles * ce, kp.hq, kp.b), FWD_THREADS, fwd_smem_bytes<D>(), ce, st, kp, status) ? SA2_OK : SA2_ERR_CUDA;
+}
+
+// Splits of a tile's work over CTAs: the query heads of its group (MODE_K1: pairs of one and a query unit) and the offsets.
+// A unit takes ~4500 cycles, a CTA ~10000 of set-up and its results, a sweep of MODE_K2 ~2500 for its operands and its fold.
+// Partials are written and read again at ~2000 bytes a cycle.  `rows` and `slab_rows`: rows of D floats a CTA leaves.
+struct Split { int hs, es, epc; };
+inline Split split(int64_t ctas, int heads, int w2, double per_offset, double bytes, int batch, int sms) {
+    Split best{1, 1, w2};
+    double best_cost = 0.;
+    for (int hs = 1; hs <= heads && hs <= 16; ++hs)
+        for (int es = 1; es <= w2 && hs * es <= 64; ++es) {
+            const int epc = (w2 + es - 1) / es;
+            if ((w2 + epc - 1) / epc != es) continue;
+            const double one = 10000. + (double)((heads + hs - 1) / hs) * epc * per_offset;
+            const double cost = tc::split_cost(ctas * hs * es, one, batch, sms) + (hs * es > 1 ? 3000. + bytes * hs * es * batch / 2000. : 0.);
+            if (best_cost == 0. || cost < tc::SPLIT_GAIN * best_cost) { best = Split{hs, es, epc}; best_cost = cost; }
+        }
+    return best;
+}
+inline Split split_k2(const sa2_shape &s, int batch, int sms) {
+    const int64_t tiles = (int64_t)((s.n + s.off2 + ROWS - 1) / ROWS) * s.hk;
+    const int keys = s.w1 + ROWS - 1 < s.n + s.off1 ? s.w1 + ROWS - 1 : s.n + s.off1;
+    return split(tiles, s.hq / s.hk, s.w2, 2500. + (keys + UNIT - 1) / UNIT * 4500., (double)tiles * ROWS * s.d * 12, batch, sms);
+}
+inline Split split_k1(const sa2_shape &s, int batch, int sms) {
+    const int64_t tiles = (int64_t)((s.n + s.off1 + ROWS - 1) / ROWS) * s.hk;
+    const int rows = s.w1 + ROWS - 1 < s.n ? s.w1 + ROWS - 1 : s.n;
+    return split(tiles, s.hq / s.hk * ((rows + UNIT - 1) / UNIT), s.w2, 4500., (double)tiles * ROWS * s.d * 8, batch, sms);
+}
+
+// Scratch after the D vector, for `round` batch elements at a time: an element that alone needs more than MOST runs on the scalar
+// kernels, which need none (long second windows: the dQ slabs grow with n * w2).
+constexpr size_t ROUND_BYTES = (size_t)256 << 20, MOST_BYTES = (size_t)1 << 30;
+struct Plan {
+    bool tc;
+    Split k1, k2;
+    int tiles, round;
+    size_t slab, part2, part1;
+};
+inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+inline Plan plan(const sa2_shape &s, int whole_batch, int sms) {
+    Plan p;
+    p.k1 = split_k1(s, whole_batch, sms);
+    p.k2 = split_k2(s, whole_batch, sms);
+    p.tiles = (s.n + s.off2 + ROWS - 1) / ROWS;
+    const size_t row = (size_t)s.d * sizeof(float), n1 = p.k1.hs * p.k1.es, n2 = p.k2.hs * p.k2.es;
+    const size_t slab = (size_t)s.hq * p.tiles * p.k2.es * (ROWS - 1 + p.k2.epc) * row;
+    const size_t part2 = n2 > 1 ? n2 * (s.n + s.off2) * s.hk * 2 * row : 0, part1 = n1 > 1 ? n1 * (s.n + s.off1) * s.hk * 2 * row : 0;
+    const size_t one = slab + part2 + part1;
+    p.tc = one <= MOST_BYTES;
+    p.round = one * s.b <= ROUND_BYTES ? s.b : one > ROUND_BYTES ? 1 : (int)(ROUND_BYTES / one);
+    p.slab = align256(slab * p.round);
+    p.part2 = align256(part2 * p.round);
+    p.part1 = align256(part1 * p.round);
+    return p;
+}
+inline size_t bwd_workspace_bytes(const sa2_shape &s, int whole_batch, int sms) {
+    const Plan p = plan(s, whole_batch, sms);
+    return p.tc ? p.slab + p.part2 + p.part1 : 0;
+}
+inline int bwd_launches(const sa2_shape &s, int whole_batch, int sms) {
+    const Plan p = plan(s, whole_batch, sms);
+    return p.tc ? 1 + 3 * ((s.b + p.round - 1) / p.round) : 2;
+}
+
+template <int D, int MODE> inline int bwd_launch(const BwdParams &P, int rows, cudaStream_t st) {
+    if (cudaFuncSetAttribute(bwd_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem_bytes<D, MODE>()) != cudaSuccess)
+        return SA2_ERR_CUDA;
+    bwd_kernel<D, MODE><<<dim3((rows + ROWS - 1) / ROWS * P.nsplit, P.kp.hk, P.kp.b), BWD_THREADS, bwd_smem_bytes<D, MODE>(), st>>>(P);
+    return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
+}
+template <int D> inline int bwd(const KernelParams &all, const Plan &p, char *extra, int *status, cudaStream_t st, int phases) {
+    if (phases == 0) phases = SA2_BWD_ROWSUM | SA2_BWD_K1 | SA2_BWD_Q;
+    if ((phases & SA2_BWD_ROWSUM) && !simt::launch_delta<D>(all, st)) return SA2_ERR_CUDA;
+    const bool k1 = phases & SA2_BWD_K1, k2 = phases & SA2_BWD_Q;
+    for (int b0 = 0; (k1 || k2) && b0 < all.b; b0 += p.round) {
+        const KernelParams kp = tc::batch_part(all, b0, all.b - b0 < p.round ? all.b - b0 : p.round);
+        float *slab = reinterpret_cast<float *>(extra), *part2 = reinterpret_cast<float *>(extra + p.slab);
+        float *part1 = reinterpret_cast<float *>(extra + p.slab + p.part2);
+        const int n1 = p.k1.hs * p.k1.es, n2 = p.k2.hs * p.k2.es;
+        if (k1)
+            if (int e = bwd_launch<D, MODE_K1>({kp, n1, p.k1.hs, p.k1.epc, 0, part1, nullptr, status}, kp.nk1, st)) return e;
+        if (k2)
+            if (int e = bwd_launch<D, MODE_K2>({kp, n2, p.k2.hs, p.k2.epc, p.tiles, part2, slab, status}, kp.nk2, st)) return e;
+        const ReduceParams R{kp, slab, part2, part1, p.tiles, p.k2.es, p.k2.epc, k2 && n2 > 1 ? n2 : 0, k1 && n1 > 1 ? n1 : 0, k2};
+        const int64_t rows = (k2 ? (int64_t)kp.n * kp.hq : 0) + (R.k2_splits ? (int64_t)kp.nk2 * kp.hk : 0) + (R.k1_splits ? (int64_t)kp.nk1 * kp.hk : 0);
+        if (rows == 0) continue;
+        reduce_kernel<D><<<(unsigned)((rows * kp.b * (D / 4) + 255) / 256), 256, 0, st>>>(R);
+        if (cudaGetLastError() != cudaSuccess) return SA2_ERR_CUDA;
+    }
+    return SA2_OK;
+}
+
+}  // namespace f32
+}  // namespace sa2

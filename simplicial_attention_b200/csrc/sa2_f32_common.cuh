@@ -1,0 +1,194 @@
+// fp32 tensors on the bf16 tensor cores: what the kernels of sa2_f32_fwd.cuh and sa2_f32_bwd.cuh share.
+//
+// Every fp32 operand x is three bf16 values, h = bf16(x), m = bf16(x - h), l = x - h - m, which carry all 24 bits of it, and a
+// product of two operands is the six products of their terms that are not below 2^-24 of it: h h, h m, m h, m m, h l, l h,
+// the small ones first.  The tensor cores truncate as they accumulate, so no accumulator lives longer than one unit of 64
+// keys (four K steps of the large product): the sums over a window, over the offsets and over the heads are fp32 additions
+// in registers.  Errors against 64 bits, norm of the difference over norm of the result, scalar fp32 kernels of sa2_simt.cuh
+// against these: b1 n1000 d64 w512/32 out 2.8e-7 -> 1.5e-7, dq 5.9e-7 -> 4.0e-7, dk1 1.7e-6 -> 4.3e-7, dv1 1.5e-6 -> 3.3e-7, dk2
+// 5.9e-7 -> 4.0e-7, dv2 3.7e-7 -> 2.6e-7, lse 5.0e-8 -> 4.9e-8; b1 n128 h2 d32, full causal, dk1 7.1e-7 -> 3.9e-7.
+//
+// Operands are made by the kernels from plain fp32 rows (any 16-byte aligned strides): no tensor maps and no scratch.
+#pragma once
+#include "sa2_tc_common.cuh"
+
+namespace sa2 {
+namespace f32 {
+
+using namespace sa2::sm100;
+using sa2::tc::ex2;
+using sa2::tc::pack_bf16;
+using sa2::tc::warp_wait;
+
+constexpr int ROWS = 128;         // rows of a tile: TMEM lanes
+constexpr int UNIT = 64;          // columns of a logit tile
+constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+// What a logit loses to the truncations of its large products, half a unit in the last place each and about one in all, is given
+// back where the reference or the logsumexp is subtracted.
+constexpr float REGAIN = 1.f + 1.1920929e-7f;
+// error bits of the device status word
+enum { ERR_FWD = 1 << 17, ERR_BWD = 1 << 18 };
+
+// The three terms of an operand tile in shared memory, rows of 128 bytes with the 128-byte swizzle: a tile per term, or at
+// head dim 32 h and m side by side and l in a second tile.
+template <int D> struct Planes {
+    static constexpr int TILES = D == 32 ? 2 : 3;
+    __host__ __device__ static constexpr uint32_t bytes(int rows) { return (uint32_t)(TILES * rows * 128); }
+    __host__ __device__ static constexpr uint32_t at(int rows, int term) {
+        return D == 32 ? (uint32_t)((term >> 1) * rows * 128 + (term & 1) * 64) : (uint32_t)(term * rows * 128);
+    }
+};
+
+// two values -> their three terms, packed
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l) {
+    const uint64_t minus = f2_pack(-1.f, -1.f);
+    h = pack_bf16(x0, x1);
+    const uint64_t r = f2_fma(f2_from_bf16x2(h), minus, f2_pack(x0, x1));
+    float a, b;
+    f2_unpack(r, a, b);
+    m = pack_bf16(a, b);
+    f2_unpack(f2_fma(f2_from_bf16x2(m), minus, r), a, b);
+    l = pack_bf16(a, b);
+}
+
+// eight channels (chunk `chunk`) of row r of an operand tile of `rows` rows
+template <int D>
+__device__ __forceinline__ void put8(uint8_t *tile, int rows, int r, int chunk, const float (&x)[8]) {
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int z = 0; z < 4; ++z) split2(x[2 * z], x[2 * z + 1], h[z], m[z], l[z]);
+    const uint32_t o = sw128_offset(r, chunk);
+    *reinterpret_cast<uint4 *>(tile + o) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(tile + (D == 32 ? sw128_offset(r, chunk + 4) : rows * 128 + o)) = make_uint4(m[0], m[1], m[2], m[3]);
+    *reinterpret_cast<uint4 *>(tile + (D == 32 ? rows * 128 : 2 * rows * 128) + o) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+__device__ __forceinline__ void load8(float (&x)[8], const float *p, bool ok) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (ok) {
+        a = __ldg(reinterpret_cast<const float4 *>(p));
+        b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+    }
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+__device__ __forceinline__ const float *row_ptr(const TensorRef &t, int b, int n, int h) {
+    return reinterpret_cast<const float *>(t.p) + elem_off(t, b, n, h);
+}
+
+// The six products of two operands, the smallest first: terms (l h) (h l) (m m) (m h) (h m) (h h)
+__host__ __device__ constexpr int term_a(int t) { return t == 0 ? 2 : t == 2 || t == 3 ? 1 : 0; }
+__host__ __device__ constexpr int term_b(int t) { return t == 1 ? 2 : t == 2 || t == 4 ? 1 : 0; }
+
+// d[128 x 64] = A B^T over the D channels: A [128 rows], B [64 rows], both K-major in shared memory
+template <int D>
+__device__ __forceinline__ void issue_nt(uint32_t d, uint64_t a, uint64_t b) {
+    constexpr uint32_t IDESC = idesc_bf16(128, 64, false, false);
+#pragma unroll
+    for (int t = 0; t < 6; ++t)
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k)
+            mma_ss(d, a + (Planes<D>::at(ROWS, term_a(t)) >> 4) + 2 * k, b + (Planes<D>::at(UNIT, term_b(t)) >> 4) + 2 * k, IDESC, t + k > 0);
+}
+// TMEM column of term `term` of the 16 keys [16 k, +16) within a region of 96 columns (see put_terms)
+__host__ __device__ constexpr uint32_t term_col(int term, int k) { return (uint32_t)((k >> 1) * 48 + term * 16 + (k & 1) * 8); }
+// d[128 x D] = P B over 64 keys: P [128 x 64] in TMEM, B [64 rows] in shared memory.  Head dim 32: the products with h and m
+// of B, which share its rows, land in columns [0, 32) and [32, 64), whose sum is the result.
+template <int D>
+__device__ __forceinline__ void issue_pv(uint32_t d, uint32_t p, uint64_t b) {
+    constexpr uint32_t N64 = idesc_bf16(128, 64, false, true), N32 = idesc_bf16(128, 32, false, true);
+    if constexpr (D == 32) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_ts(d, p + term_col(1, k), b + 128 * k, N64, k > 0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_ts(d, p + term_col(2, k), b + 128 * k, N32, 1u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_ts(d, p + term_col(0, k), b + (UNIT * 128 >> 4) + 128 * k, N32, 1u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_ts(d, p + term_col(0, k), b + 128 * k, N64, 1u);
+    } else {
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                mma_ts(d, p + term_col(term_a(t), k), b + (Planes<D>::at(UNIT, term_b(t)) >> 4) + 128 * k, N64, t + k > 0);
+    }
+}
+// A region of 96 columns holds a logit tile in [32, 96); the terms of its columns [32 ch, +32) go to [48 ch, +48), over
+// columns that have been read when the chunks are taken in order.
+__device__ __forceinline__ void put_terms(uint32_t region, int ch, const uint32_t (&x)[32]) {
+    uint32_t h[16], m[16], l[16];
+#pragma unroll
+    for (int z = 0; z < 16; ++z) split2(__uint_as_float(x[2 * z]), __uint_as_float(x[2 * z + 1]), h[z], m[z], l[z]);
+    tmem_st16(region + ch * 48, h);
+    tmem_st16(region + ch * 48 + 16, m);
+    tmem_st16(region + ch * 48 + 32, l);
+}
+// the values of columns [32 ch, +32), from their terms (exact)
+__device__ __forceinline__ void get_terms(uint32_t region, int ch, uint32_t (&x)[32]) {
+    uint32_t h[16], m[16], l[16];
+    tmem_ld16(region + ch * 48, h);
+    tmem_ld16(region + ch * 48 + 16, m);
+    tmem_ld16(region + ch * 48 + 32, l);
+    tmem_wait_ld();
+#pragma unroll
+    for (int z = 0; z < 16; ++z) {
+        float a, b;
+        f2_unpack(f2_add(f2_add(f2_from_bf16x2(l[z]), f2_from_bf16x2(m[z])), f2_from_bf16x2(h[z])), a, b);
+        x[2 * z] = __float_as_uint(a);
+        x[2 * z + 1] = __float_as_uint(b);
+    }
+}
+// sum[] += the D columns of an accumulator (pairs of channels)
+template <int D>
+__device__ __forceinline__ void add_acc(uint32_t cols, uint64_t (&sum)[D / 2]) {
+#pragma unroll
+    for (int c = 0; c < 64; c += 32) {
+        uint32_t t[32];
+        tmem_ld32(cols + c, t);
+        tmem_wait_ld(t);
+#pragma unroll
+        for (int z = 0; z < 16; ++z) {
+            uint64_t &s = sum[(D == 32 ? 0 : c / 2) + z];
+            s = f2_add(s, f2_pack(t[2 * z], t[2 * z + 1]));
+        }
+    }
+}
+
+// valid columns [lo, hi] of a logit row as the unsigned test x - lo <= len; none if hi < lo
+__device__ __forceinline__ void column_range(int &lo, int hi, uint32_t &len) {
+    if (hi < lo) { lo = 64; hi = 64; }
+    len = (uint32_t)(hi - lo);
+}
+
+// Terms of infinite values, and products that leave the range on one side only, make a NaN of a logit (times log2 e) that is
+// none: the NaN among the columns `ask` of s[] are formed again, in scalar fp32 from the rows themselves.  operands(z, q, k2,
+// k1) names those of column z, finish(z, logit) the value that takes its place.
+template <int D, typename Operands, typename Finish>
+__device__ __forceinline__ void scalar_logits(uint32_t (&s)[32], uint32_t ask, float mul, Operands operands, Finish finish) {
+#pragma unroll
+    for (int z = 0; z < 32; ++z)
+        if (__uint_as_float(s[z]) == __uint_as_float(s[z])) ask &= ~(1u << z);
+    while (ask) {
+        const int z = __ffs(ask) - 1;
+        const float *q, *k2, *k1;
+        operands(z, q, k2, k1);
+        float v = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < D; ++c) v = fmaf(mul * q[c] * k2[c], k1[c], v);
+        v = finish(z, v);
+#pragma unroll
+        for (int y = 0; y < 32; ++y) if (y == z) s[y] = __float_as_uint(v);
+        ask &= ask - 1;
+    }
+}
+// bits of the columns [c0, c0 + 32) that lie in [lo, lo + len]
+__device__ __forceinline__ uint32_t column_mask(int c0, int lo, uint32_t len) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int z = 0; z < 32; ++z) m |= (uint32_t)(c0 + z - lo) <= len ? 1u << z : 0u;
+    return m;
+}
+
+}  // namespace f32
+}  // namespace sa2
