@@ -292,6 +292,21 @@ int sa2_qkv_append(const sa2_qkvnorm_args *args, const sa2_append_set sets[4], i
  */
 int sa2_rows_linear(const void *x, const void *w, void *y, int32_t rows, int32_t k, int32_t outs, void *stream);
 
+/*
+ * The same for up to 64 rows, with an RMSNorm of the rows of x on their way in (gain [k], fp32 or bf16, 16-byte aligned) unless
+ * gain is null: the module's prenorm and its projection (simplicial_mha.py:93,112) in one launch.
+ */
+int sa2_norm_linear(const void *x, const void *gain, int32_t gain_dtype, float eps, const void *w, void *y, int32_t rows, int32_t k, int32_t outs,
+                    void *stream);
+
+/*
+ * Generation, one new token for each of b sequences (bf16, d 64 or 128, w2 <= 64; SA2_ERR_UNSUPPORTED otherwise): sa2_qkv_append and
+ * the attention of the new rows in one launch.  args as there (rows = b; y and rstd are not used); sets[s].dst is
+ * [b][min(keep + 1, w - 1)][hk][d], w = w1 for k and v and w2 for k' and v': the last of the cached rows and the new one that a later
+ * token sees.  out [b][hq][d].
+ */
+int sa2_step_attn(const sa2_qkvnorm_args *args, const sa2_append_set sets[4], void *out, int32_t b, int32_t w1, int32_t w2, float scale);
+
 #ifdef __cplusplus
 }
 #endif

@@ -21,7 +21,8 @@ EXPORTS = ("sa2_fwd", "sa2_bwd", "sa2_bwd_workspace_bytes", "sa2_strerror", "sa2
            "sa2_kernel_launches", "sa2_device_status", "sa2_check_device", "sa2_selftest_wait",
            "sa2_bwd_static_scratch", "sa2_bwd_part", "sa2_bwd_workspace_bytes_part",
            "sa2_headnorm_fwd", "sa2_headnorm_bwd", "sa2_headnorm_partial_bytes",
-           "sa2_qkvnorm_fwd", "sa2_qkvnorm_bwd", "sa2_qkv_append", "sa2_rows_linear")
+           "sa2_qkvnorm_fwd", "sa2_qkvnorm_bwd", "sa2_qkv_append", "sa2_rows_linear",
+           "sa2_norm_linear", "sa2_step_attn")
 STATIC_SCRATCH_ROWS = 262144   # SA2_STATIC_SCRATCH_ROWS in include/sa2.h
 SELFTEST_WAIT_BIT = 0x10000    # SA2_SELFTEST_WAIT_BIT
 SA2_ERR_DEVICE = 5

@@ -7,7 +7,9 @@
 #include "sa2_f32.cuh"
 #include "sa2_headnorm.cuh"
 #include "sa2_rows_linear.cuh"
+#include "sa2_step.cuh"
 #include <nvtx3/nvToolsExt.h>
+#include <type_traits>
 
 namespace sa2 {
 namespace nvtx {
@@ -469,6 +471,21 @@ int append_launch(const sa2::headnorm::AppendParams &A, int d, cudaStream_t st) 
     return launch_status();
 }
 
+int rows_linear_run(const void *x, const void *gain, int gain_dtype, float eps, const void *w, void *y, int rows, int k, int outs, void *stream) {
+    using namespace sa2::rows_linear;
+    if (!x || !w || !y || rows <= 0 || k <= 0 || outs <= 0 || !aligned16(x) || !aligned16(w) || !aligned16(y) || (gain && !aligned16(gain))) return SA2_ERR_INVALID;
+    if (rows > MAX_NORM_ROWS || k % 32 || outs % OUTS) return SA2_ERR_UNSUPPORTED;
+    auto pick = [&](auto normed) {
+        constexpr bool N = decltype(normed)::value;
+        return rows <= 8 ? kernel<1, N> : rows <= 16 ? kernel<2, N> : rows <= 32 ? kernel<4, N> : kernel<8, N>;
+    };
+    auto run = gain ? pick(std::true_type{}) : pick(std::false_type{});
+    run<<<outs / OUTS, WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const __nv_bfloat16 *>(x), reinterpret_cast<const __nv_bfloat16 *>(w), reinterpret_cast<__nv_bfloat16 *>(y), rows, k, outs,
+        Norm{gain, gain_dtype == SA2_BF16, eps});
+    return launch_status();
+}
+
 }  // namespace
 
 extern "C" {
@@ -518,14 +535,46 @@ int sa2_qkv_append(const sa2_qkvnorm_args *a, const sa2_append_set *sets, int32_
 }
 
 int sa2_rows_linear(const void *x, const void *w, void *y, int32_t rows, int32_t k, int32_t outs, void *stream) {
-    using namespace sa2::rows_linear;
     sa2::nvtx::Range range("sa2_rows_linear");
-    if (!x || !w || !y || rows <= 0 || k <= 0 || outs <= 0 || !aligned16(x) || !aligned16(w) || !aligned16(y)) return SA2_ERR_INVALID;
-    if (rows > MAX_ROWS || k % 32 || outs % OUTS) return SA2_ERR_UNSUPPORTED;
-    auto run = rows <= 8 ? kernel<1> : kernel<2>;
-    run<<<outs / OUTS, WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const __nv_bfloat16 *>(x), reinterpret_cast<const __nv_bfloat16 *>(w), reinterpret_cast<__nv_bfloat16 *>(y), rows, k, outs);
-    return launch_status();
+    if (rows > sa2::rows_linear::MAX_ROWS) return x && w && y && k > 0 && outs > 0 ? SA2_ERR_UNSUPPORTED : SA2_ERR_INVALID;
+    return rows_linear_run(x, nullptr, 0, 0.f, w, y, rows, k, outs, stream);
+}
+
+int sa2_norm_linear(const void *x, const void *gain, int32_t gain_dtype, float eps, const void *w, void *y, int32_t rows, int32_t k, int32_t outs, void *stream) {
+    sa2::nvtx::Range range("sa2_norm_linear");
+    if (gain && gain_dtype != SA2_F32 && gain_dtype != SA2_BF16) return SA2_ERR_UNSUPPORTED;
+    return rows_linear_run(x, gain, gain_dtype, eps, w, y, rows, k, outs, stream);
+}
+
+int sa2_step_attn(const sa2_qkvnorm_args *a, const sa2_append_set *sets, void *out, int32_t b, int32_t w1, int32_t w2, float scale) {
+    sa2::nvtx::Range range("sa2_step_attn");
+    if (!a || !a->x || !sets || !out || !aligned16(out) || b <= 0 || a->rows != b || a->hq <= 0 || a->hk <= 0 || a->hq % a->hk || w1 <= 0 || w2 <= 0)
+        return SA2_ERR_INVALID;
+    if ((a->d != 64 && a->d != 128) || a->x_dtype != SA2_BF16 || (a->gain_dtype != SA2_F32 && a->gain_dtype != SA2_BF16) || w2 > sa2::step::MAX_W2)
+        return SA2_ERR_UNSUPPORTED;
+    if (a->x_stride < (int64_t)a->d * (a->hq + 4LL * a->hk) || !rows_aligned(a->x, a->x_stride, SA2_BF16)) return SA2_ERR_INVALID;
+    sa2::step::Params P{};
+    for (int v = 0; v < 5; ++v) {
+        if (!a->gain[v] || !aligned16(a->gain[v])) return SA2_ERR_INVALID;
+        P.gains.p[v] = a->gain[v];
+    }
+    P.gains.bf16 = a->gain_dtype == SA2_BF16;
+    P.gains.hq = a->hq; P.gains.hk = a->hk;
+    P.proj = reinterpret_cast<const __nv_bfloat16 *>(a->x);
+    P.stride = a->x_stride; P.eps = a->eps; P.c = scale * 1.4426950408889634f;
+    for (int s = 0; s < 4; ++s) {
+        const sa2_append_set &t = sets[s];
+        const int w = s & 1 ? w2 : w1, rows = t.keep + 1 < w ? t.keep + 1 : w - 1;
+        if (t.keep < 0 || t.keep != sets[s & 1].keep || (rows > 0 && (!t.dst || !aligned16(t.dst)))) return SA2_ERR_INVALID;
+        if (t.keep > 0 && (!t.cache || !aligned16(t.cache) || t.strides.batch % 8 || t.strides.seq % 8 || t.strides.head % 8)) return SA2_ERR_INVALID;
+        P.set[s] = sa2::step::Set{reinterpret_cast<const __nv_bfloat16 *>(t.cache), t.strides.batch, t.strides.seq, t.strides.head,
+                                  reinterpret_cast<__nv_bfloat16 *>(t.dst), t.keep, rows};
+    }
+    P.out = reinterpret_cast<__nv_bfloat16 *>(out);
+    P.hq = a->hq; P.hk = a->hk; P.g = a->hq / a->hk; P.w1 = w1; P.w2 = w2;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
+    const int rc = a->d == 64 ? sa2::step::launch<64>(P, b, sa2::tc::SM_COUNT, st) : sa2::step::launch<128>(P, b, sa2::tc::SM_COUNT, st);
+    return rc < 0 ? SA2_ERR_UNSUPPORTED : rc == 0 ? SA2_OK : SA2_ERR_CUDA;
 }
 
 }  // extern "C"

@@ -32,15 +32,17 @@ struct Lib {
     size_t (*partial_bytes)(int64_t, int32_t) = nullptr;
     int (*qkv_fwd)(const sa2_qkvnorm_args *) = nullptr;
     int (*qkv_bwd)(const sa2_qkvnorm_args *) = nullptr;
-    int (*linear)(const void *, const void *, void *, int32_t, int32_t, int32_t, void *) = nullptr;
     int (*append)(const sa2_qkvnorm_args *, const sa2_append_set *, int32_t, int32_t) = nullptr;
+    int (*norm_linear)(const void *, const void *, int32_t, float, const void *, void *, int32_t, int32_t, int32_t, void *) = nullptr;
+    int (*step_attn)(const sa2_qkvnorm_args *, const sa2_append_set *, void *, int32_t, int32_t, int32_t, float) = nullptr;
 } L;
 
 void bind(const std::map<std::string, uintptr_t> &f) {
     auto set = [&](auto &slot, const char *name) { slot = reinterpret_cast<std::decay_t<decltype(slot)>>(f.at(name)); };
     set(L.fwd, "sa2_fwd"); set(L.bwd, "sa2_bwd"); set(L.workspace, "sa2_bwd_workspace_bytes");
     set(L.norm_fwd, "sa2_headnorm_fwd"); set(L.norm_bwd, "sa2_headnorm_bwd"); set(L.partial_bytes, "sa2_headnorm_partial_bytes");
-    set(L.qkv_fwd, "sa2_qkvnorm_fwd"); set(L.qkv_bwd, "sa2_qkvnorm_bwd"); set(L.append, "sa2_qkv_append"); set(L.linear, "sa2_rows_linear");
+    set(L.qkv_fwd, "sa2_qkvnorm_fwd"); set(L.qkv_bwd, "sa2_qkvnorm_bwd"); set(L.append, "sa2_qkv_append");
+    set(L.norm_linear, "sa2_norm_linear"); set(L.step_attn, "sa2_step_attn");
 }
 
 // raises _lib.Sa2Error, also from the autograd engine's threads
@@ -363,6 +365,27 @@ void attend_cached(const Tensor &proj, const std::vector<Tensor> &gain, const st
     }
 }
 
+// One new row per sequence: the same in one launch, with set = [k, k', v, v'] cut to what later rows can see as it is made.
+// False where sa2_step_attn does not take the shape.
+bool attend_one(const Tensor &proj, const std::vector<Tensor> &gain, const std::vector<Tensor> &cache, const Heads &h, double eps, int64_t w1,
+                int64_t w2, Tensor &out, Tensor (&set)[4]) {
+    const int64_t b = proj.size(0);
+    const Tensor g5[5] = {gain[0], gain[1], gain[2], gain[3], gain[4]};
+    sa2_append_set as[4];
+    for (int s = 0; s < 4; ++s) {
+        const int64_t keep = cache[s].size(1);
+        set[s] = at::empty({b, std::min(keep + 1, (s & 1 ? w2 : w1) - 1), h.hk, h.d}, proj.options());
+        as[s] = sa2_append_set{cache[s].data_ptr(), strides(cache[s]), set[s].data_ptr(), (int32_t)keep};
+    }
+    sa2_qkvnorm_args a{};
+    fill_norm(a, proj, g5, h, eps);
+    out = at::empty({b, 1, h.hq, h.d}, proj.options());
+    const int rc = L.step_attn(&a, as, out.data_ptr(), (int32_t)b, (int32_t)w1, (int32_t)w2, (float)(1. / std::sqrt((double)h.d)));
+    if (rc == SA2_ERR_UNSUPPORTED) return false;
+    check(rc, "sa2_step_attn");
+    return true;
+}
+
 // Generation: (out [b][n][hq][d], [k, k', v, v']), or None.  cache: [k, k', v, v'] of the rows before; no gradients.
 pybind11::object qkv_attn_cached(const Tensor &proj, const std::vector<Tensor> &gain, const std::vector<Tensor> &cache, int64_t hq, int64_t hk,
                                  int64_t d, double eps, int64_t w1, int64_t w2, int64_t kernel) {
@@ -394,15 +417,24 @@ Tensor row_norm(const Tensor &x, const Tensor &w, double eps) {
     return y;
 }
 
-// x W^T over the last dimension: the kernel for few rows where it takes them (bf16, at most 16 rows), else the library
-Tensor step_linear(const Tensor &x, const Tensor &w) {
+// Does the kernel for few rows take x W^T?  Up to 16 rows always, up to 64 with a small W: there a microsecond or two more on the
+// device than the library's kernel outweigh neither the 8 us its call costs the host more nor the norm's own launch.
+bool few_rows(const Tensor &x, const Tensor &w) {
     const int64_t rows = x.size(0) * x.size(1), k = w.size(1), outs = w.size(0);
-    if (rows > 16 || k % 32 || outs % 16 || x.scalar_type() != at::kBFloat16 || !x.is_contiguous() || !w.is_contiguous() || !aligned(x) || !aligned(w))
-        return at::linear(x, w);
-    Tensor y = at::empty({x.size(0), x.size(1), outs}, x.options());
-    check(L.linear(x.data_ptr(), w.data_ptr(), y.data_ptr(), (int32_t)rows, (int32_t)k, (int32_t)outs,
-                   c10::cuda::getCurrentCUDAStream(x.get_device()).stream()), "sa2_rows_linear");
+    return rows <= (k * outs <= 1 << 20 ? 64 : 16) && k % 32 == 0 && outs % 16 == 0 && x.scalar_type() == at::kBFloat16 && x.is_contiguous() &&
+           w.is_contiguous() && aligned(x) && aligned(w);
+}
+// x W^T over the last dimension, and the same behind an RMSNorm
+Tensor few_rows_linear(const Tensor &x, const Tensor *gain, double eps, const Tensor &w) {
+    Tensor y = at::empty({x.size(0), x.size(1), w.size(0)}, x.options());
+    check(L.norm_linear(x.data_ptr(), gain ? gain->data_ptr() : nullptr, gain ? dtype_of(*gain) : SA2_F32, (float)eps, w.data_ptr(), y.data_ptr(),
+                        (int32_t)(x.size(0) * x.size(1)), (int32_t)w.size(1), (int32_t)w.size(0),
+                        c10::cuda::getCurrentCUDAStream(x.get_device()).stream()), "sa2_norm_linear");
     return y;
+}
+Tensor step_linear(const Tensor &x, const Tensor &w) { return few_rows(x, w) ? few_rows_linear(x, nullptr, 0., w) : at::linear(x, w); }
+Tensor step_norm_linear(const Tensor &x, const Tensor &gain, double eps, const Tensor &w) {
+    return few_rows(x, w) ? few_rows_linear(x, &gain, eps, w) : at::linear(row_norm(x, gain, eps), w);
 }
 
 // A whole generation step: (out [b][n][dim], [k, k', v, v']), or None.  norms: gain and eps of the prenorm and of
@@ -422,10 +454,11 @@ pybind11::object step(const Tensor &x, const std::optional<Tensor> &pre, double 
     if (!cache_ok(cache, h, x) || !gains_ok(gain, h, x.device())) return pybind11::none();
     const c10::cuda::CUDAGuard guard(x.device());
     const at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor proj = step_linear(pre ? row_norm(x, *pre, pre_eps) : x, w_qkv);
+    const Tensor proj = pre ? step_norm_linear(x, *pre, pre_eps, w_qkv) : step_linear(x, w_qkv);
     if (!projection_ok(proj, gain, h, x.scalar_type())) return pybind11::none();
     Tensor out, set[4];
-    attend_cached(proj, gain, cache, h, eps, w1, w2, kernel, out, set);
+    const bool one = x.size(1) == 1 && x.scalar_type() == at::kBFloat16 && (d == 64 || d == 128) && w2 <= 64 && kernel == SA2_KERNEL_AUTO;
+    if (!one || !attend_one(proj, gain, cache, h, eps, w1, w2, out, set)) attend_cached(proj, gain, cache, h, eps, w1, w2, kernel, out, set);
     out = step_linear(out.view({x.size(0), x.size(1), hq * d}), w_out);
     if (post) out = row_norm(out, *post, post_eps);
     return pybind11::make_tuple(out, set[0], set[1], set[2], set[3]);
