@@ -10,14 +10,13 @@
 #include "sa2_tc_fwd128.cuh"
 #include "sa2_tc_bwd_k1_128.cuh"
 #include "sa2_tmap.cuh"
+#include <algorithm>
 #include <cstdlib>
 
 namespace sa2 {
 namespace tc {
 
 constexpr int SM_COUNT = 148;     // B200
-
-inline int tiles_per_query_tile(int w1) { return (w1 + TJ - 1 + TJ - 1) / TJ; }   // ceil((w1 + 127) / 128)
 
 // The tensor-core forward handles bf16 at every head dim and any window.
 inline bool fwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
@@ -33,24 +32,27 @@ inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 inline bool bwd_scale_ok(const sa2_shape &s) { return fabsf(s.scale) >= 1e-20f; }
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // CTAs sharing one query tile in the dQ/dK2/dV2 kernel: splits of the window (head dim 128 walks it in one CTA) times
-// splits of the offsets.  A CTA costs ~12000 cycles of set-up, loads, slab and its share of the reduction, a 64-key unit
-// of a sweep ~1600 (3000 at head dim 128); at most as many offsets per CTA as its accumulators hold.
-struct BqSplit { int tsplit, esplit, epc; };
-inline BqSplit bq_split(const sa2_shape &s, const BwdCaller &call, int max_tiles, int sms) {
+// splits of the offsets, an even number each.  A CTA costs ~12000 cycles of set-up, loads, slab and its share of the reduction, a 64-key
+// unit of a sweep ~1100 (1700 at head dim 128).
+struct BqSplit { int nu, ups, tsplit, esplit, epc; };
+inline BqSplit bq_split(const sa2_shape &s, const BwdCaller &call, int max_units, int sms) {
     BqSplit r;
-    const int nt = tiles_per_query_tile(s.w1), have = (s.n + s.off1 + TJ - 1) / TJ;
-    r.tsplit = s.d == 128 ? 1 : (nt + max_tiles - 1) / max_tiles;
-    const int tiles = (nt < have ? nt : have), per = (tiles + r.tsplit - 1) / r.tsplit;
-    const int64_t ctas = (int64_t)((s.n + TQ - 1) / TQ) * s.hq * r.tsplit * (s.d == 128 ? 2 : 1);
-    const int w2 = s.w2, least = (w2 + BQ_MAX_EPC - 1) / BQ_MAX_EPC;
+    const int have = (s.n + s.off1 + 63) / 64;
+    r.nu = (s.w1 + BQ_ROWS - 1 + 63) / 64;
+    r.tsplit = s.d == 128 ? 1 : (r.nu + max_units - 1) / max_units;
+    r.ups = (r.nu + r.tsplit - 1) / r.tsplit;
+    const int per = (std::min(r.nu, have) + r.tsplit - 1) / r.tsplit;
+    const int64_t ctas = (int64_t)((s.n + BQ_ROWS - 1) / BQ_ROWS) * s.hq * r.tsplit;
+    const int pairs = (s.w2 + 1) / 2;
+    const int least = (pairs + BQ_MAX_EPC / 2 - 1) / (BQ_MAX_EPC / 2);
     double best_cost = 0.;
     r.esplit = least;
-    for (int es = least; es <= w2 && (es <= 16 || es == least); ++es) {
-        const double cost = split_cost(ctas * es, 12000. + (w2 + es - 1) / es * (per * 2. * (s.d == 128 ? 3000. : 1600.)), call.batch, sms);
+    for (int es = least; es <= pairs && (es <= 16 || es == least); ++es) {
+        const double cost = split_cost(ctas * es, 12000. + (pairs + es - 1) / es * (per * (s.d == 128 ? 1700. : 1100.)), call.batch, sms);
         if (best_cost == 0. || cost < SPLIT_GAIN * best_cost) { r.esplit = es; best_cost = cost; }
     }
-    r.epc = (w2 + r.esplit - 1) / r.esplit;
-    r.esplit = (w2 + r.epc - 1) / r.epc;
+    r.epc = (pairs + r.esplit - 1) / r.esplit * 2;
+    r.esplit = (s.w2 + r.epc - 1) / r.epc;
     return r;
 }
 // How dQ, dK2 and dV2 are computed.  Up to 56 offsets (the caller's window, however short the sequence) head dims 64 and 128
@@ -60,9 +62,8 @@ inline BqSplit bq_split(const sa2_shape &s, const BwdCaller &call, int max_tiles
 // in rounds of at most BQ_ROUND_BYTES (one element at least); where one element needs more than BQ_MOST_BYTES, the fp32 kernels
 // do it without any (b1 n4096 h8 d64 w4096/4096 would take 36 GB).
 // Errors of dq, dk2, dv2 against 64 bits, n150...400: 1.9e-3 to 3.2e-3 as on the fp32 kernels, 2.3e-3 to 5.4e-3 with rounded
-// operands.  Times of dQ/dK2/dV2, fp32 kernels / rounded / this: b4 n1024 h8 d64 w512/64 38.6 / 0.77 / 1.36 ms; d128 b2 w512/60
-// 41.2 / 1.01 / 2.55 ms (K1 / V1 one unit at a time); b1 n190 h4 d64, full causal 11.0 / 0.058 / 0.112 ms.
-constexpr size_t BQ_ROUND_BYTES = (size_t)256 << 20, BQ_MOST_BYTES = (size_t)1 << 30;
+// operands.  (A round was twice as large when the slabs of a tile of 128 rows were.)
+constexpr size_t BQ_ROUND_BYTES = (size_t)128 << 20, BQ_MOST_BYTES = (size_t)1 << 30;
 struct BqPlan {
     bool tc, split;      // on the tensor cores; with rests
     BqSplit sp;
@@ -70,9 +71,9 @@ struct BqPlan {
 };
 inline BqPlan bq_plan(const sa2_shape &s, const BwdCaller &call, int sms) {
     BqPlan p;
-    const bool longer = call.w2 > BQ_MAX_EPC;
+    const bool longer = call.w2 > BQ_FINE_W2;
     p.split = s.d == 32 || longer;
-    p.sp = bq_split(s, call, p.split && s.d == 64 ? BqCfg<64, true>::MAX_TILES : BqCfg<64, false>::MAX_TILES, sms);
+    p.sp = bq_split(s, call, p.split && s.d == 64 ? BqCfg<64, true>::MAX_UNITS : BqCfg<64, false>::MAX_UNITS, sms);
     p.round = s.b;
     p.tc = true;
     if (longer) {
@@ -215,15 +216,15 @@ template <int D, bool SPLIT>
 inline int bwd_q_launch(const BqParams &Q, cudaStream_t st) {
     using C = BqCfg<D, SPLIT>;
     const KernelParams &kp = Q.kp;
-    const size_t smem = bq_smem_bytes<D, SPLIT>(Q.epc);
+    const size_t smem = C::SMEM;
     if (cudaFuncSetAttribute(bwd_q_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SA2_ERR_CUDA;
-    CUtensorMap mapK, mapV;             // head dim 128 streams units of 64 rows
-    constexpr int ROWS = D == 128 ? 64 : TJ;
+    CUtensorMap mapK, mapV;             // units of 64 rows
+    constexpr int ROWS = 64;
     if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, ROWS) ||
         !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, ROWS))
         return SA2_ERR_CUDA;
-    bwd_q_kernel<D, SPLIT><<<dim3(Q.nqt * Q.nsplit * C::CH, kp.hq, kp.b), C::THREADS, smem, st>>>(mapK, mapV, Q);
+    bwd_q_kernel<D, SPLIT><<<dim3(Q.nqt * Q.nsplit, kp.hq, kp.b), C::THREADS, smem, st>>>(mapK, mapV, Q);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
@@ -284,18 +285,18 @@ inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, const BwdCalle
     if ((phases & SA2_BWD_ROWSUM) && !simt::launch_delta<D>(kp, st)) return SA2_ERR_CUDA;
     BqPlan plan = bq_plan(s, call, SM_COUNT);
     // fp32 gradients show the last bits, which AUTO leaves to the fp32 kernels
-    if (s.kernel == SA2_KERNEL_AUTO && !kp.grad_bf16 && call.w2 > BQ_MAX_EPC) plan.tc = false;
+    if (s.kernel == SA2_KERNEL_AUTO && !kp.grad_bf16 && call.w2 > BQ_FINE_W2) plan.tc = false;
     const BwdScratch room = bwd_scratch(s, call, plan);
     const K1Split k1 = k1_split(s, call, SM_COUNT);
     BqParams Q;
     Q.kp = kp;
     Q.c = c;
-    Q.nt = tiles_per_query_tile(s.w1);
+    Q.nu = plan.sp.nu;
     Q.tsplit = plan.sp.tsplit;
     Q.nsplit = plan.sp.tsplit * plan.sp.esplit;
     Q.epc = plan.sp.epc;
-    Q.tiles_per_split = (Q.nt + Q.tsplit - 1) / Q.tsplit;
-    Q.nqt = (kp.n + TQ - 1) / TQ;
+    Q.units_per_split = plan.sp.ups;
+    Q.nqt = (kp.n + BQ_ROWS - 1) / BQ_ROWS;
     Q.part_dq = reinterpret_cast<float *>(extra);
     Q.part_k2 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + room.dq);
     float *part_k1 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + room.dq + room.k2);

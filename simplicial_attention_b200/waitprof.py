@@ -30,11 +30,11 @@ SLOTS = {
     "dk1_dv1": "issuer of dV1 / dK1 (0) 1 P^T/G^T ready; issuers of S^T / dP^T (1 and 2) 1 A_e/B_e stage full, 2 the second products "
                "of the buffer done; compute groups (4-11) 1 S^T/dP^T ready; builders (the last eight warps; d=128: the last four or "
                "eight) 1 k2/v2 window landed, 2 stage free",
-    "dq_dk2_dv2": "issuers of U / W (0, and 3 at d=64) 1 P/G ready, 2 U/W read by the fold group; issuers of S / dP (1, 2) "
-                  "1 A_e/B_e ready, 2 buffer free, 3 K1/V1 unit landed (d=128), 4 cycles issuing products, 5 cycles in the commit; "
-                  "producer (3 at d=128) 1 ring slot free; compute groups (4-11) 1 S/dP ready, 4 TMEM loads, 5 arithmetic, "
-                  "6 TMEM stores and hand-over; fold groups (12-15; d=64: of U, and 16-19 of W) 1 U/W complete, 2 the other fold "
-                  "threads, 3 A_e/B_e stage free, 4 stores of A_e/B_e, 5 fold after its waits",
+    "dq_dk2_dv2": "issuers of U / W (0, and 3 up to d=64) 1 P/G ready, 2 U/W read by the fold group; issuers of S / dP (1, 2) "
+                  "1 A/B ready, 2 buffer free, 3 K1/V1 unit landed (d=128); producer (3 at d=128) 1 ring slot free; compute "
+                  "groups (4-11) 1 S/dP ready; fold groups (12-15 of U, 16-19 of W) 1 U/W complete, 2 the other fold threads' "
+                  "last sweep, 3 A/B stage free, 4 their first halves.  (This build has fewer staged second keys and one ring slot "
+                  "less at d=128.)",
 }
 
 

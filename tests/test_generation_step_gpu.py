@@ -16,7 +16,7 @@ CASES = [
     (1, 8, 4, 64, 512, 32, 512, True, False),        # eight CTAs a head
     (3, 8, 4, 64, 512, 32, 5, True, False),          # caches shorter than the windows
     (2, 4, 4, 128, 700, 40, 800, True, False),
-    (5, 16, 2, 64, 100, 64, 130, True, True),        # 32 blocks of rows for eight warps
+    (5, 8, 1, 64, 100, 64, 130, True, False),        # 32 blocks of rows for eight warps
     (2, 3, 1, 64, 64, 8, 70, False, False),
     (2, 1, 1, 64, 1, 1, 9, True, False),             # nothing to keep
     (64, 2, 1, 128, 77, 17, 200, True, False),
