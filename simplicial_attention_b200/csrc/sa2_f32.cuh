@@ -4,6 +4,8 @@
 #include "sa2_f32_fwd.cuh"
 #include "sa2_f32_bwd.cuh"
 #include "sa2_simt.cuh"
+#include <algorithm>
+#include <atomic>
 
 namespace sa2 {
 namespace f32 {
@@ -12,8 +14,34 @@ namespace f32 {
 // a unit of K1 and V1 do not fit the shared memory of an SM.)
 inline bool supported(const sa2_shape &s) { return s.kernel == SA2_KERNEL_AUTO && s.dtype == SA2_F32 && s.d <= 64; }
 
+// Clusters of sixteen CTAs are the device's choice (at one CTA per SM they take most of a GPC): asked for once per device.
+template <int D> inline bool sixteen_fit() {
+    static std::atomic<int> known[64];             // 0: not asked yet, 1: no, 2: yes
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int k = known[dev].load(std::memory_order_relaxed);
+    if (k == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 16; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(16); cfg.blockDim = dim3(FWD_THREADS); cfg.dynamicSmemBytes = fwd_smem_bytes<D>();
+        cfg.attrs = &attr; cfg.numAttrs = 1;
+        int n = 0;
+        const bool ok = cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem_bytes<D>()) == cudaSuccess &&
+                        cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, fwd_kernel<D>, &cfg) == cudaSuccess && n >= 2;
+        if (!ok) (void)cudaGetLastError();
+        k = ok ? 2 : 1;
+        known[dev].store(k, std::memory_order_relaxed);
+    }
+    return k == 2;
+}
+// CTAs of a row tile (see simt::cluster_size); sixteen where eight leave most of the chip idle and each still has two pairs of offsets.
 template <int D> inline int fwd(const KernelParams &kp, int *status, int sms, cudaStream_t st) {
-    const int tiles = (kp.n + ROWS - 1) / ROWS, ce = simt::cluster_size((int64_t)tiles * kp.hq, kp.w2, 2, sms);
+    const int tiles = (kp.n + ROWS - 1) / ROWS;
+    int ce = simt::cluster_size((int64_t)tiles * kp.hq, kp.w2, 2, sms);
+    if (ce == 8 && (int64_t)tiles * kp.hq * 32 <= sms && kp.w2 >= 64 && sixteen_fit<D>()) ce = 16;
     return simt::launch_clusters(fwd_kernel<D>, dim3(tiles * ce, kp.hq, kp.b), FWD_THREADS, fwd_smem_bytes<D>(), ce, st, kp, status) ? SA2_OK : SA2_ERR_CUDA;
 }
 
@@ -83,7 +111,7 @@ inline int bwd_launches(const sa2_shape &s, int whole_batch, int sms) {
 template <int D, int MODE> inline int bwd_launch(const BwdParams &P, int rows, cudaStream_t st) {
     if (cudaFuncSetAttribute(bwd_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem_bytes<D, MODE>()) != cudaSuccess)
         return SA2_ERR_CUDA;
-    bwd_kernel<D, MODE><<<dim3((rows + ROWS - 1) / ROWS * P.nsplit, P.kp.hk, P.kp.b), BWD_THREADS, bwd_smem_bytes<D, MODE>(), st>>>(P);
+    bwd_kernel<D, MODE><<<dim3((rows + ROWS - 1) / ROWS * P.nsplit, P.kp.hk, P.kp.b), BwdCfg<MODE>::THREADS, bwd_smem_bytes<D, MODE>(), st>>>(P);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 template <int D> inline int bwd(const KernelParams &all, const Plan &p, char *extra, int *status, cudaStream_t st, int phases) {
@@ -102,7 +130,10 @@ template <int D> inline int bwd(const KernelParams &all, const Plan &p, char *ex
         const ReduceParams R{kp, slab, part2, part1, p.tiles, p.k2.es, p.k2.epc, k2 && n2 > 1 ? n2 : 0, k1 && n1 > 1 ? n1 : 0, k2};
         const int64_t rows = (k2 ? (int64_t)kp.n * kp.hq : 0) + (R.k2_splits ? (int64_t)kp.nk2 * kp.hk : 0) + (R.k1_splits ? (int64_t)kp.nk1 * kp.hk : 0);
         if (rows == 0) continue;
-        reduce_kernel<D><<<(unsigned)((rows * kp.b * (D / 4) + 255) / 256), 256, 0, st>>>(R);
+        const int most = std::max(std::max(R.dq ? p.k2.es : 0, R.k2_splits), R.k1_splits);
+        const int64_t threads = rows * kp.b * (D / 4);
+        if (most >= 8) reduce_kernel<D, 8><<<(unsigned)((threads * 8 + 255) / 256), 256, 0, st>>>(R);
+        else reduce_kernel<D, 1><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(R);
         if (cudaGetLastError() != cudaSuccess) return SA2_ERR_CUDA;
     }
     return SA2_OK;

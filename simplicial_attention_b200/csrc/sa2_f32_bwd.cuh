@@ -11,12 +11,13 @@
 // of the group and need no atomics.  dQ rows move by one row a sweep: a ring of 128 rows in shared memory, whose finished row
 // goes to a slab of 127 + epc rows in scratch; the reduction adds the slabs of the tiles and offset ranges in order.
 //
-// Warps (512 threads): 0 / 3 issuers of U / W, 1 / 2 of S / dP; 4-7 form P and G; 8-11 build A_e (K1) and sum U, 12-15 build
-// B_e (V1) and sum W.  TMEM: buffer x: S, then the terms of P [192 x, +96), dP and G [192 x + 96, +96); U [384, +64), W [448, +64).
+// Warps (512 threads, 640 in MODE_K2): 0 / 3 issuers of U / W, 1 / 2 of S / dP; then one or two groups of four that form P and G, four
+// that build A_e (K1) and sum U, four that build B_e (V1) and sum W.  TMEM: buffer x: S, then the terms of P [192 x, +96), dP and G
+// [192 x + 96, +96); U [384, +64), W [448, +64).
 //
 // Bound: a unit's 96 products fetch 384 KB from shared memory, ~3100 cycles; the chain operands -> S / dP -> P / G -> U / W of two
-// units in flight takes ~6100 cycles a unit.  b1 n1024 h8 d64 w512/32: 5.5 ms on the scalar kernels -> 0.53 (MODE_K1) + 0.63 ms;
-// forward + backward 7.5 -> 1.5 ms, b1 n128 h2 d32 full causal 0.30 -> 0.14 ms.
+// units in flight takes ~6000 cycles a unit.  b1 n1024 h8 d64 w512/32: 5.5 ms on the scalar kernels -> 0.53 (MODE_K1) + 0.60 ms;
+// forward + backward 7.5 -> 1.45 ms, b1 n128 h2 d32 full causal 0.30 -> 0.11 ms.
 #pragma once
 #include "sa2_f32_common.cuh"
 #include "sa2_tc_bwd_k1.cuh"
@@ -25,9 +26,14 @@ namespace sa2 {
 namespace f32 {
 
 enum { MODE_K1 = 0, MODE_K2 = 1 };
-constexpr int BWD_THREADS = 512;
-constexpr int BWD_REGS_LAUNCH = 128, BWD_REGS_ISSUE = 40, BWD_REGS_COMPUTE = 152, BWD_REGS_SUM = 160;
-static_assert(BWD_REGS_ISSUE + BWD_REGS_COMPUTE + 2 * BWD_REGS_SUM == 4 * BWD_REGS_LAUNCH, "register pool must balance");
+// Compute groups: two in MODE_K2, 32 columns of a unit each (0.63 -> 0.60 ms on b1 n1024 h8 d64 w512/32), one in MODE_K1 (0.53; 0.63
+// with two, whose registers the sums and the rows of q would have to give).
+template <int MODE> struct BwdCfg {
+    static constexpr int GROUPS = MODE == MODE_K1 ? 1 : 2, THREADS = 384 + 128 * GROUPS;
+    static constexpr int REGS_LAUNCH = GROUPS == 2 ? 96 : 128, REGS_ISSUE = GROUPS == 2 ? 32 : 40, REGS_COMPUTE = GROUPS == 2 ? 80 : 152;
+    static constexpr int REGS_SUM = GROUPS == 2 ? 144 : 160;
+    static_assert(REGS_ISSUE + GROUPS * REGS_COMPUTE + 2 * REGS_SUM == THREADS / 128 * REGS_LAUNCH, "register pool must balance");
+};
 
 enum BwdBar {
     B_M_FULL = 0,      // [2] row-side operand of S / dP
@@ -137,7 +143,7 @@ __device__ __forceinline__ int bwd_first(const BwdParams &P, int which, uint32_t
         if (u >= 2 && !mbar_wait_warp(&bars[B_DONE + 2 * (1 - which) + buf], ((u >> 1) - 1) & 1, abort_flag, 0, 3)) return ERR_BWD;
         tc_fence_after();
         if (elect_one()) {
-            issue_nt<D>(tmem + 192 * buf + 96 * which + 32, dM, dN + buf * (Planes<D>::bytes(UNIT) >> 4));
+            issue_nt<D>(tmem + 192 * buf + 96 * which + LOGITS, dM, dN + buf * (Planes<D>::bytes(UNIT) >> 4));
             tc_commit(&bars[B_S_FULL + buf]);
             if (MODE == MODE_K2 && wk.last()) tc_commit(&bars[B_M_EMPTY + which]);
         }
@@ -162,9 +168,9 @@ __device__ __forceinline__ int bwd_second(const BwdParams &P, int which, uint32_
     return 0;
 }
 
-// P and G of every unit (warps 4-7, a thread per row)
+// P and G of every unit, a thread per row; group cg of the compute groups
 template <int D, int MODE>
-__device__ __forceinline__ int bwd_compute(const BwdParams &P, uint32_t tmem, const float2 *stats, uint64_t *bars, volatile int *abort_flag) {
+__device__ __forceinline__ int bwd_compute(const BwdParams &P, int cg, uint32_t tmem, const float2 *stats, uint64_t *bars, volatile int *abort_flag) {
     const KernelParams &kp = P.kp;
     const int r = threadIdx.x & 127, hk = blockIdx.y, b = blockIdx.z;
     const uint32_t lanes = tmem + ((uint32_t)(r & 96) << 16);
@@ -195,31 +201,33 @@ __device__ __forceinline__ int bwd_compute(const BwdParams &P, uint32_t tmem, co
         column_range(lo, hi, len);
         if (!warp_wait(&bars[B_S_FULL + buf], (u >> 1) & 1, abort_flag, 1)) return ERR_BWD;
         tc_fence_after();
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            const int c0 = ch * 32;
+        // sixteen columns at a time, either half from the outside in (put_terms)
+#pragma unroll 2
+        for (int y = 0; y < 4 / BwdCfg<MODE>::GROUPS; ++y) {
+            const int half = BwdCfg<MODE>::GROUPS == 2 ? cg : y >> 1, k = half ? 3 - (y & 1) : y & 1;
+            const int c0 = 16 * k;
             const uint32_t rp = lanes + 192 * buf, rg = rp + 96;
-            uint32_t s[32], g[32];
-            if (__all_sync(0xffffffffu, lo > c0 + 31 || (int)(lo + len) < c0)) {       // nothing valid for this warp
+            uint32_t s[16], g[16];
+            if (__all_sync(0xffffffffu, lo > c0 + 15 || (int)(lo + len) < c0)) {       // nothing valid for this warp
 #pragma unroll
-                for (int z = 0; z < 32; ++z) { s[z] = 0u; g[z] = 0u; }
+                for (int z = 0; z < 16; ++z) { s[z] = 0u; g[z] = 0u; }
             } else {
-                tmem_ld32(rp + 32 + c0, s);
-                tmem_ld32(rg + 32 + c0, g);
+                tmem_ld16(rp + LOGITS + c0, s);
+                tmem_ld16(rg + LOGITS + c0, g);
                 tmem_wait_ld(s);
                 tmem_wait_ld(g);
-                const bool full = __all_sync(0xffffffffu, lo <= c0 && (int)(lo + len) >= c0 + 31);
+                const bool full = __all_sync(0xffffffffu, lo <= c0 && (int)(lo + len) >= c0 + 15);
                 auto exponent = [&](int z, float v) { return fmaf(v, REGAIN, -(MODE == MODE_K2 ? lse2 : st[c0 + z].x)); };
                 float seen = 0.f;
 #pragma unroll
-                for (int z = 0; z < 32; ++z) {
+                for (int z = 0; z < 16; ++z) {
                     float a = exponent(z, __uint_as_float(s[z]));
                     if (!full && (uint32_t)(c0 + z - lo) > len) a = -CUDART_INF_F;
                     seen += a;
                     s[z] = __float_as_uint(a);
                 }
                 if (seen != seen)                    // (masked columns are -inf, not NaN)
-                    scalar_logits<D>(s, 0xffffffffu, mul,
+                    scalar_logits<D>(s, 0xffffu, mul,
                                      [&](int z, const float *&pq, const float *&pk2, const float *&pk1) {
                                          const int i = MODE == MODE_K2 ? row - kp.off2 + wk.e : wk.c0 + c0 + z;
                                          pq = row_ptr(kp.q, b, i, wk.head());
@@ -228,7 +236,7 @@ __device__ __forceinline__ int bwd_compute(const BwdParams &P, uint32_t tmem, co
                                      },
                                      exponent);
 #pragma unroll
-                for (int z = 0; z < 32; z += 2) {
+                for (int z = 0; z < 16; z += 2) {
                     const float p0 = ex2(__uint_as_float(s[z])), p1 = ex2(__uint_as_float(s[z + 1]));
                     const float d0 = MODE == MODE_K2 ? dl : st[c0 + z].y, d1 = MODE == MODE_K2 ? dl : st[c0 + z + 1].y;
                     float g0, g1;
@@ -237,8 +245,8 @@ __device__ __forceinline__ int bwd_compute(const BwdParams &P, uint32_t tmem, co
                     g[z] = __float_as_uint(g0); g[z + 1] = __float_as_uint(g1);
                 }
             }
-            put_terms(rp, ch, s);
-            put_terms(rg, ch, g);
+            put_terms(rp, k, s);
+            put_terms(rg, k, g);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -247,7 +255,7 @@ __device__ __forceinline__ int bwd_compute(const BwdParams &P, uint32_t tmem, co
     return 0;
 }
 
-// Operands and sums of one side (warps 8-11: which = 0, A_e, K1 and U; 12-15: which = 1, B_e, V1 and W).  Unit u of the
+// Operands and sums of one side (which = 0: A_e, K1 and U; 1: B_e, V1 and W).  Unit u of the
 // operands is made when unit u - 2 is done and its product has been added up: both take the same slot.
 template <int D, int MODE>
 __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t tmem, uint8_t *sM, uint8_t *sN, float2 *stats, float *ring,
@@ -268,6 +276,7 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
     Walk<MODE> nxt(P), cur(P);
     const int row = nxt.r0 + t;                        // the row whose sums this thread keeps
     int sweeps = 0, folds = 0, err = 0;
+    float held[MODE == MODE_K1 ? TASKS : 1][8];
     if (MODE == MODE_K1 && !nxt.done()) {
 #pragma unroll 1
         for (int x = 0; x < ROWS / RPP; ++x) {
@@ -324,27 +333,26 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
     for (int u = 0;; ++u) {
         const bool more = !nxt.done();
         const int slot = u & 1;
-        // the unit's rows, fetched before the wait
+        // the unit's rows, fetched before the wait (MODE_K1: the rows of q or dO once for all offsets)
+        constexpr int EARLY = MODE == MODE_K2 && BwdCfg<MODE>::GROUPS == 2 ? TASKS / 2 : TASKS;
         float x[TASKS][8];
         float2 stat = make_float2(0.f, 0.f);
+        auto key_row = [&](int z) {
+            const int j = nxt.c0 + q0 + z * RPP;
+            load8(x[z], row_ptr(tk, b, j < kp.nk1 ? j : 0, hk) + c * 8, j < kp.nk1);
+        };
         if (more) {
             if constexpr (MODE == MODE_K2) {
 #pragma unroll
-                for (int z = 0; z < TASKS; ++z) {
-                    const int j = nxt.c0 + q0 + z * RPP;
-                    load8(x[z], row_ptr(tk, b, j < kp.nk1 ? j : 0, hk) + c * 8, j < kp.nk1);
-                }
+                for (int z = 0; z < EARLY; ++z) key_row(z);
             } else {
                 const int h = nxt.head();
 #pragma unroll
                 for (int z = 0; z < TASKS; ++z) {
                     const int i = nxt.c0 + q0 + z * RPP, k = i + kp.off2 - nxt.e;
+                    if (nxt.first()) load8(held[z], row_ptr(tx, b, i <= nxt.i_hi ? i : 0, h) + c * 8, i <= nxt.i_hi);
                     const bool ok = i <= nxt.i_hi && k >= 0;
-                    float y[8];
-                    load8(x[z], row_ptr(tx, b, ok ? i : 0, h) + c * 8, ok);
-                    load8(y, row_ptr(ty, b, ok ? k : 0, hk) + c * 8, ok);
-#pragma unroll
-                    for (int w = 0; w < 8; ++w) x[z][w] = mul * x[z][w] * y[w];
+                    load8(x[z], row_ptr(ty, b, ok ? k : 0, hk) + c * 8, ok);
                 }
                 const int i = nxt.c0 + t;
                 if (which == 0 && t < UNIT && i <= nxt.i_hi) {
@@ -365,7 +373,16 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
         if (more) {
             uint8_t *d = dN + slot * Planes<D>::bytes(UNIT);
 #pragma unroll
-            for (int z = 0; z < TASKS; ++z) put8<D>(d, UNIT, q0 + z * RPP, c, x[z]);
+            for (int z = 0; z < TASKS; ++z) {
+                if constexpr (MODE == MODE_K1) {
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) x[z][w] = mul * held[MODE == MODE_K1 ? z : 0][w] * x[z][w];
+                } else if (z == EARLY) {
+#pragma unroll
+                    for (int y = EARLY; y < TASKS; ++y) key_row(y);
+                }
+                put8<D>(d, UNIT, q0 + z * RPP, c, x[z]);
+            }
             if (MODE == MODE_K1 && which == 0 && t < UNIT) stats[slot * UNIT + t] = stat;
             fence_proxy_async_smem();
             mbar_arrive(&bars[B_N_FULL + 2 * which + slot]);
@@ -427,7 +444,8 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
 }
 
 template <int D, int MODE>
-__global__ void __launch_bounds__(BWD_THREADS, 1) bwd_kernel(const BwdParams P) {
+__global__ void __launch_bounds__(BwdCfg<MODE>::THREADS, 1) bwd_kernel(const BwdParams P) {
+    using C = BwdCfg<MODE>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = align_smem(smem_raw);
     uint8_t *sM = smem;                                           // [2]: A_e, B_e or K1, V1
@@ -442,7 +460,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) bwd_kernel(const BwdParams P) 
         for (int x = 0; x < B_BAR_COUNT; ++x) {
             const bool one = (x >= B_M_EMPTY && x < B_M_EMPTY + 2) || (x >= B_DONE && x < B_DONE + 4);
             const bool two = x == B_S_FULL || x == B_S_FULL + 1;
-            mbar_init(&bars[x], one ? 1u : two ? 2u : 128u);
+            const bool compute = x == B_P_FULL || x == B_P_FULL + 1;
+            mbar_init(&bars[x], one ? 1u : two ? 2u : compute ? 128u * C::GROUPS : 128u);
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -461,15 +480,16 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) bwd_kernel(const BwdParams P) 
     sa2::sm100::prof_begin();
 #endif
     if (warp < 4) {
-        reg_dealloc<BWD_REGS_ISSUE>();
+        reg_dealloc<C::REGS_ISSUE>();
         if (warp == 1 || warp == 2) err = bwd_first<D, MODE>(P, warp - 1, tmem, sM, sN, bars, abort_flag);
         else err = bwd_second<D, MODE>(P, warp == 3, tmem, sN, bars, abort_flag);
-    } else if (warp < 8) {
-        reg_alloc<BWD_REGS_COMPUTE>();
-        err = bwd_compute<D, MODE>(P, tmem, reinterpret_cast<const float2 *>(extra), bars, abort_flag);
+    } else if (warp < 4 + 4 * C::GROUPS) {
+        if constexpr (C::REGS_COMPUTE > C::REGS_LAUNCH) reg_alloc<C::REGS_COMPUTE>();
+        else reg_dealloc<C::REGS_COMPUTE>();
+        err = bwd_compute<D, MODE>(P, (warp >> 2) - 1, tmem, reinterpret_cast<const float2 *>(extra), bars, abort_flag);
     } else {
-        reg_alloc<BWD_REGS_SUM>();
-        err = bwd_side<D, MODE>(P, warp >= 12, tmem, sM, sN, reinterpret_cast<float2 *>(extra), reinterpret_cast<float *>(extra), bars, abort_flag);
+        reg_alloc<C::REGS_SUM>();
+        err = bwd_side<D, MODE>(P, warp >= 8 + 4 * C::GROUPS, tmem, sM, sN, reinterpret_cast<float2 *>(extra), reinterpret_cast<float *>(extra), bars, abort_flag);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
@@ -494,23 +514,37 @@ struct ReduceParams {
     int k2_splits, k1_splits;     // 0: nothing to add up
     int dq;                       // dQ is asked for
 };
-template <int D>
+// G threads take the offset ranges or splits of a piece by turns, and their sums are added in order: where splits are many, the rows
+// are few (b1 n128 h2 d32 full causal, 64 ranges: 26 -> 6 us with eight).
+template <int D, int G>
 __global__ void __launch_bounds__(256) reduce_kernel(const ReduceParams R) {
     const KernelParams &kp = R.kp;
-    constexpr int TPR = D / 4;
-    int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    const int c = (int)(idx % TPR) * 4;
-    idx /= TPR;
+    constexpr int TPR = D / 4, RPB = 256 / (TPR * G);        // threads of a row, rows of a block
+    __shared__ float4 sums[G > 1 ? 2 : 1][G > 1 ? 256 : 1];
+    const int c = (int)(threadIdx.x % TPR) * 4, g = (int)threadIdx.x / TPR % G;
+    int64_t idx = (int64_t)blockIdx.x * RPB + threadIdx.x / (TPR * G);
     const bool gbf16 = kp.grad_bf16 != 0;
     const int64_t nq = R.dq ? (int64_t)kp.b * kp.n * kp.hq : 0;
-    if (idx < nq) {
+    const int64_t n2 = R.k2_splits ? (int64_t)kp.b * kp.nk2 * kp.hk : 0, n1 = R.k1_splits ? (int64_t)kp.b * kp.nk1 * kp.hk : 0;
+    float v[2][4] = {};
+    auto add = [](float (&a)[4], const float4 &x) { a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w; };
+    // the first of the G threads of a piece has the sum
+    auto gather = [&](int y) {
+        if constexpr (G > 1) {
+            sums[y][threadIdx.x] = make_float4(v[y][0], v[y][1], v[y][2], v[y][3]);
+            __syncthreads();
+            if (g == 0)
+                for (int x = 1; x < G; ++x) add(v[y], sums[y][threadIdx.x + x * TPR]);
+        }
+    };
+    const bool is_q = idx < nq, is_2 = !is_q && idx < nq + n2, is_1 = !is_q && !is_2 && idx < nq + n2 + n1;
+    if (is_q) {
         const int h = (int)(idx % kp.hq), i = (int)(idx / kp.hq % kp.n), b = (int)(idx / ((int64_t)kp.hq * kp.n));
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
         const int rows = ROWS - 1 + R.epc;
         const float *slab = R.slab + ((size_t)b * kp.hq + h) * R.tiles * R.esplit * rows * D + c;
         // (unrolled for the loads in flight; the order of the sum is that of the loop)
 #pragma unroll 4
-        for (int es = 0; es < R.esplit; ++es) {
+        for (int es = g; es < R.esplit; es += G) {
             const int e0 = es * R.epc, e1 = min(kp.w2, e0 + R.epc);
             // second keys i + off2 - e of the range, from the last tile that holds one to the first
             const int k_hi = i + kp.off2 - e0, k_lo = max(0, i + kp.off2 - e1 + 1), last = k_hi < 0 ? -1 : k_hi / ROWS, first = k_lo / ROWS;
@@ -520,37 +554,35 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceParams R) {
             float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
             if (last >= first) x = row(last);
             if (last > first) y = row(last - 1);
-            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-            v[0] += y.x; v[1] += y.y; v[2] += y.z; v[3] += y.w;
-            for (int tile = last - 2; tile >= first; --tile) {
-                x = row(tile);
-                v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-            }
+            add(v[0], x);
+            add(v[0], y);
+            for (int tile = last - 2; tile >= first; --tile) add(v[0], row(tile));
         }
+    } else if (is_2 || is_1) {
+        idx -= is_2 ? nq : nq + n2;
+        const int64_t all = is_2 ? n2 : n1;
+        const int splits = is_2 ? R.k2_splits : R.k1_splits;
+        const float *part = is_2 ? R.part_k2 : R.part_k1;
+#pragma unroll 4
+        for (int s = g; s < splits; s += G) {
+            const float *src = part + ((s * all + idx) * 2) * D + c;
+            add(v[0], *reinterpret_cast<const float4 *>(src));
+            add(v[1], *reinterpret_cast<const float4 *>(src + D));
+        }
+    }
+    gather(0);
+    gather(1);
+    if (g != 0 || !(is_q || is_2 || is_1)) return;
+    if (is_q) {
+        const int h = (int)(idx % kp.hq), i = (int)(idx / kp.hq % kp.n), b = (int)(idx / ((int64_t)kp.hq * kp.n));
 #pragma unroll
-        for (int z = 0; z < 4; ++z) v[z] *= kp.scale;
-        store_vec<4>(kp.dq.p, elem_off(kp.dq, b, i, h) + c, gbf16, v);
+        for (int z = 0; z < 4; ++z) v[0][z] *= kp.scale;
+        store_vec<4>(kp.dq.p, elem_off(kp.dq, b, i, h) + c, gbf16, v[0]);
         return;
     }
-    idx -= nq;
-    const int64_t n2 = R.k2_splits ? (int64_t)kp.b * kp.nk2 * kp.hk : 0, n1 = R.k1_splits ? (int64_t)kp.b * kp.nk1 * kp.hk : 0;
-    const bool first = idx >= n2;
-    if (first) idx -= n2;
-    if (first && idx >= n1) return;
-    const int rows = first ? kp.nk1 : kp.nk2, splits = first ? R.k1_splits : R.k2_splits;
-    const float *part = first ? R.part_k1 : R.part_k2;
-    const int64_t all = (int64_t)kp.b * rows * kp.hk;
+    const int rows = is_2 ? kp.nk2 : kp.nk1;
     const int hk = (int)(idx % kp.hk), row = (int)(idx / kp.hk % rows), b = (int)(idx / ((int64_t)kp.hk * rows));
-    float v[2][4] = {};
-#pragma unroll 4
-    for (int s = 0; s < splits; ++s) {
-#pragma unroll
-        for (int y = 0; y < 2; ++y) {
-            const float4 x = *reinterpret_cast<const float4 *>(part + ((s * all + idx) * 2 + y) * D + c);
-            v[y][0] += x.x; v[y][1] += x.y; v[y][2] += x.z; v[y][3] += x.w;
-        }
-    }
-    const TensorRef &dk = first ? kp.dk1 : kp.dk2, &dv = first ? kp.dv1 : kp.dv2;
+    const TensorRef &dk = is_2 ? kp.dk2 : kp.dk1, &dv = is_2 ? kp.dv2 : kp.dv1;
     store_vec<4>(dk.p, elem_off(dk, b, row, hk) + c, gbf16, v[0]);
     store_vec<4>(dv.p, elem_off(dv, b, row, hk) + c, gbf16, v[1]);
 }

@@ -5,8 +5,8 @@
 // the small ones first.  The tensor cores truncate as they accumulate, so no accumulator lives longer than one unit of 64
 // keys (four K steps of the large product): the sums over a window, over the offsets and over the heads are fp32 additions
 // in registers.  Errors against 64 bits, norm of the difference over norm of the result, scalar fp32 kernels of sa2_simt.cuh
-// against these: b1 n1000 d64 w512/32 out 2.8e-7 -> 1.5e-7, dq 5.9e-7 -> 4.0e-7, dk1 1.7e-6 -> 4.3e-7, dv1 1.5e-6 -> 3.3e-7, dk2
-// 5.9e-7 -> 4.0e-7, dv2 3.7e-7 -> 2.6e-7, lse 5.0e-8 -> 4.9e-8; b1 n128 h2 d32, full causal, dk1 7.1e-7 -> 3.9e-7.
+// against these: b1 n1000 d64 w512/32 out 2.8e-7 -> 1.2e-7, dq 5.9e-7 -> 3.9e-7, dk1 1.7e-6 -> 4.2e-7, dv1 1.5e-6 -> 3.1e-7, dk2
+// 5.9e-7 -> 4.0e-7, dv2 3.7e-7 -> 2.7e-7, lse 5.0e-8 -> 4.9e-8; b1 n128 h2 d32, full causal, dk1 7.1e-7 -> 3.5e-7.
 //
 // Operands are made by the kernels from plain fp32 rows (any 16-byte aligned strides): no tensor maps and no scratch.
 #pragma once
@@ -90,8 +90,8 @@ __device__ __forceinline__ void issue_nt(uint32_t d, uint64_t a, uint64_t b) {
         for (int k = 0; k < D / 16; ++k)
             mma_ss(d, a + (Planes<D>::at(ROWS, term_a(t)) >> 4) + 2 * k, b + (Planes<D>::at(UNIT, term_b(t)) >> 4) + 2 * k, IDESC, t + k > 0);
 }
-// TMEM column of term `term` of the 16 keys [16 k, +16) within a region of 96 columns (see put_terms)
-__host__ __device__ constexpr uint32_t term_col(int term, int k) { return (uint32_t)((k >> 1) * 48 + term * 16 + (k & 1) * 8); }
+// TMEM column of term `term` of the 16 keys [16 k, +16) within a region of 96 columns
+__host__ __device__ constexpr uint32_t term_col(int term, int k) { return (uint32_t)(k * 24 + term * 8); }
 // d[128 x D] = P B over 64 keys: P [128 x 64] in TMEM, B [64 rows] in shared memory.  Head dim 32: the products with h and m
 // of B, which share its rows, land in columns [0, 32) and [32, 64), whose sum is the result.
 template <int D>
@@ -114,27 +114,28 @@ __device__ __forceinline__ void issue_pv(uint32_t d, uint32_t p, uint64_t b) {
                 mma_ts(d, p + term_col(term_a(t), k), b + (Planes<D>::at(UNIT, term_b(t)) >> 4) + 128 * k, N64, t + k > 0);
     }
 }
-// A region of 96 columns holds a logit tile in [32, 96); the terms of its columns [32 ch, +32) go to [48 ch, +48), over
-// columns that have been read when the chunks are taken in order.
-__device__ __forceinline__ void put_terms(uint32_t region, int ch, const uint32_t (&x)[32]) {
-    uint32_t h[16], m[16], l[16];
+// A region of 96 columns holds a logit tile in [16, 80).  The terms of its columns [16 k, +16) go to [24 k, +24): over columns that
+// have been read if those of either half are taken from the outside in, k = 0, 1 and k = 3, 2.
+constexpr uint32_t LOGITS = 16;
+__device__ __forceinline__ void put_terms(uint32_t region, int k, const uint32_t (&x)[16]) {
+    uint32_t h[8], m[8], l[8];
 #pragma unroll
-    for (int z = 0; z < 16; ++z) split2(__uint_as_float(x[2 * z]), __uint_as_float(x[2 * z + 1]), h[z], m[z], l[z]);
-    tmem_st16(region + ch * 48, h);
-    tmem_st16(region + ch * 48 + 16, m);
-    tmem_st16(region + ch * 48 + 32, l);
+    for (int z = 0; z < 8; ++z) split2(__uint_as_float(x[2 * z]), __uint_as_float(x[2 * z + 1]), h[z], m[z], l[z]);
+    tmem_st8(region + 24 * k, h);
+    tmem_st8(region + 24 * k + 8, m);
+    tmem_st8(region + 24 * k + 16, l);
 }
-// the values of columns [32 ch, +32), from their terms (exact)
-__device__ __forceinline__ void get_terms(uint32_t region, int ch, uint32_t (&x)[32]) {
-    uint32_t h[16], m[16], l[16];
-    tmem_ld16(region + ch * 48, h);
-    tmem_ld16(region + ch * 48 + 16, m);
-    tmem_ld16(region + ch * 48 + 32, l);
-    tmem_wait_ld();
+// the values of columns [16 k, +16), from their terms (exact)
+__device__ __forceinline__ void get_terms(uint32_t region, int k, uint32_t (&x)[16]) {
+    uint32_t w[16], l[16];         // (the load of l takes eight columns more than its own)
+    tmem_ld16(region + 24 * k, w);
+    tmem_ld16(region + 24 * k + 8, l);
+    tmem_wait_ld(w);
+    tmem_wait_ld(l);
 #pragma unroll
-    for (int z = 0; z < 16; ++z) {
+    for (int z = 0; z < 8; ++z) {
         float a, b;
-        f2_unpack(f2_add(f2_add(f2_from_bf16x2(l[z]), f2_from_bf16x2(m[z])), f2_from_bf16x2(h[z])), a, b);
+        f2_unpack(f2_add(f2_add(f2_from_bf16x2(l[8 + z]), f2_from_bf16x2(w[8 + z])), f2_from_bf16x2(w[z])), a, b);
         x[2 * z] = __float_as_uint(a);
         x[2 * z + 1] = __float_as_uint(b);
     }
@@ -165,9 +166,9 @@ __device__ __forceinline__ void column_range(int &lo, int hi, uint32_t &len) {
 // none: the NaN among the columns `ask` of s[] are formed again, in scalar fp32 from the rows themselves.  operands(z, q, k2,
 // k1) names those of column z, finish(z, logit) the value that takes its place.
 template <int D, typename Operands, typename Finish>
-__device__ __forceinline__ void scalar_logits(uint32_t (&s)[32], uint32_t ask, float mul, Operands operands, Finish finish) {
+__device__ __forceinline__ void scalar_logits(uint32_t (&s)[16], uint32_t ask, float mul, Operands operands, Finish finish) {
 #pragma unroll
-    for (int z = 0; z < 32; ++z)
+    for (int z = 0; z < 16; ++z)
         if (__uint_as_float(s[z]) == __uint_as_float(s[z])) ask &= ~(1u << z);
     while (ask) {
         const int z = __ffs(ask) - 1;
@@ -178,15 +179,15 @@ __device__ __forceinline__ void scalar_logits(uint32_t (&s)[32], uint32_t ask, f
         for (int c = 0; c < D; ++c) v = fmaf(mul * q[c] * k2[c], k1[c], v);
         v = finish(z, v);
 #pragma unroll
-        for (int y = 0; y < 32; ++y) if (y == z) s[y] = __float_as_uint(v);
+        for (int y = 0; y < 16; ++y) if (y == z) s[y] = __float_as_uint(v);
         ask &= ask - 1;
     }
 }
-// bits of the columns [c0, c0 + 32) that lie in [lo, lo + len]
+// bits of the columns [c0, c0 + 16) that lie in [lo, lo + len]
 __device__ __forceinline__ uint32_t column_mask(int c0, int lo, uint32_t len) {
     uint32_t m = 0;
 #pragma unroll
-    for (int z = 0; z < 32; ++z) m |= (uint32_t)(c0 + z - lo) <= len ? 1u << z : 0u;
+    for (int z = 0; z < 16; ++z) m |= (uint32_t)(c0 + z - lo) <= len ? 1u << z : 0u;
     return m;
 }
 

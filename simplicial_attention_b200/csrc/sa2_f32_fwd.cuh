@@ -10,11 +10,12 @@
 //
 // Warps (512 threads): 0 and 1 issuers of the groups' products; 4-7 and 8-11 softmax groups; 12-15 builders of A_e and of the
 // terms of K1 / V1 units (two slots).  An issuer's products complete in order, so one barrier says both that S of unit u is
-// there and that W of unit u - 1 is.  TMEM: group x at 160 x: terms of P over S in 96 columns, W in 64.
+// there and that W of unit u - 1 is.  TMEM: group x at 160 x: terms of P over S in 96 columns, W in 64; the rows'
+// partial outputs at 320 + 64 x, touched once a sweep.
 //
-// Bound: the chain S -> P -> P V1 of a group, ~3600 cycles of a softmax warp and as many of products a unit, of which two groups
-// overlap; the products alone would take ~1900 (24 of each kind, an operand fetch of 6 KB each for S).  b1 n1024 h8 d64 w512/32
-// 2.0 ms on the scalar kernels -> 0.36 ms.
+// Bound: the chain S -> P -> P V1 of a group: ~3600 cycles of a softmax warp a unit, then ~2200 of products (24 of each kind), during
+// which the other group has the exponentials.  b1 n1024 h8 d64 w512/32 2.0 ms on the scalar kernels -> 0.29 ms; 0.37 without the
+// turns (F_TURN), with or without the output in registers.
 #pragma once
 #include "sa2_f32_common.cuh"
 #include <cooperative_groups.h>
@@ -23,7 +24,7 @@ namespace sa2 {
 namespace f32 {
 
 constexpr int FWD_THREADS = 512;
-constexpr int FWD_REGS_LAUNCH = 128, FWD_REGS_ISSUE = 40, FWD_REGS_SOFTMAX = 200, FWD_REGS_BUILD = 72;
+constexpr int FWD_REGS_LAUNCH = 128, FWD_REGS_ISSUE = 40, FWD_REGS_SOFTMAX = 168, FWD_REGS_BUILD = 136;
 static_assert(FWD_REGS_ISSUE + 2 * FWD_REGS_SOFTMAX + FWD_REGS_BUILD == 4 * FWD_REGS_LAUNCH, "register pool must balance");
 
 enum FwdBar {
@@ -33,7 +34,8 @@ enum FwdBar {
     F_KV_EMPTY = 6,    // [2]
     F_S_FULL = 8,      // [2] per group: S of unit u and W of unit u - 1
     F_P_FULL = 10,     // [2]
-    F_BAR_COUNT = 12
+    F_TURN = 12,       // [2] the other group's products of the unit have been issued
+    F_BAR_COUNT = 14
 };
 
 template <int D> inline size_t fwd_smem_bytes() {
@@ -67,7 +69,7 @@ __device__ __forceinline__ FwdGeom fwd_geom(const KernelParams &kp) {
 template <int D>
 __device__ __forceinline__ int fwd_issue(const FwdGeom &g, int x, uint32_t tmem, const uint8_t *sA, const uint8_t *sK, const uint8_t *sV,
                                          uint64_t *bars, volatile int *abort_flag) {
-    const uint32_t s = tmem + x * 160 + 32, p = tmem + x * 160, w = tmem + x * 160 + 96;
+    const uint32_t s = tmem + x * 160 + LOGITS, p = tmem + x * 160, w = tmem + x * 160 + 96;
     const uint64_t dA = smem_desc_sw128(smem_u32(sA) + x * Planes<D>::bytes(ROWS));
     const uint64_t dK = smem_desc_sw128(smem_u32(sK)), dV = smem_desc_sw128(smem_u32(sV));
     constexpr uint32_t SLOT = Planes<D>::bytes(UNIT) >> 4;
@@ -75,21 +77,21 @@ __device__ __forceinline__ int fwd_issue(const FwdGeom &g, int x, uint32_t tmem,
     int u = 0;
     for (int pp = 0; pp < g.npairs; ++pp) {
         for (int k = 0; k < g.nunits; ++k, ++u) {
-            if (u > 0) {
-                if (!mbar_wait_warp(&bars[F_P_FULL + x], (u - 1) & 1, abort_flag, 0, 1)) return ERR_FWD;
-                tc_fence_after();
-                if (elect_one()) {
+            if (u > 0 && !mbar_wait_warp(&bars[F_P_FULL + x], (u - 1) & 1, abort_flag, 0, 1)) return ERR_FWD;
+            if (k == 0 && !mbar_wait_warp(&bars[F_A_FULL + x], pp & 1, abort_flag, 0, 2)) return ERR_FWD;
+            if (!mbar_wait_warp(&bars[F_KV_FULL + (u & 1)], (u >> 1) & 1, abort_flag, 0, 3)) return ERR_FWD;
+            // The groups take turns: left to themselves they fall into step, both on the tensor cores and then both on their exponentials.
+            if ((x == 1 || u > 0) && !mbar_wait_warp(&bars[F_TURN + x], (x == 1 ? u : u - 1) & 1, abort_flag, 0, 4)) return ERR_FWD;
+            tc_fence_after();
+            if (elect_one()) {
+                if (u > 0) {
                     issue_pv<D>(w, p, dV + ((u - 1) & 1) * SLOT);
                     tc_commit(&bars[F_KV_EMPTY + ((u - 1) & 1)]);
                 }
-            }
-            if (k == 0 && !mbar_wait_warp(&bars[F_A_FULL + x], pp & 1, abort_flag, 0, 2)) return ERR_FWD;
-            if (!mbar_wait_warp(&bars[F_KV_FULL + (u & 1)], (u >> 1) & 1, abort_flag, 0, 3)) return ERR_FWD;
-            tc_fence_after();
-            if (elect_one()) {
                 issue_nt<D>(s, dA, dK + (u & 1) * SLOT);
                 tc_commit(&bars[F_S_FULL + x]);
                 if (k == g.nunits - 1) tc_commit(&bars[F_A_EMPTY + x]);
+                mbar_arrive(&bars[F_TURN + 1 - x]);
             }
         }
     }
@@ -117,21 +119,21 @@ __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &
         for (int w = 0; w < g.nunits; ++w, ++u) {
             const int j0 = g.j_lo + UNIT * w, slot = u & 1;
             uint8_t *dk = sK + slot * Planes<D>::bytes(UNIT), *dv = sV + slot * Planes<D>::bytes(UNIT);
+            {
+                constexpr int N = UNIT / RPP;
+                float k[N][8], v[N][8];
 #pragma unroll
-            for (int x = 0; x < UNIT / RPP; x += 2) {
-                float k[2][8], v[2][8];
-#pragma unroll
-                for (int y = 0; y < 2; ++y) {
-                    const int j = j0 + r0 + (x + y) * RPP;
+                for (int y = 0; y < N; ++y) {
+                    const int j = j0 + r0 + y * RPP;
                     const bool ok = j < kp.nk1;
                     load8(k[y], row_ptr(kp.k1, b, ok ? j : 0, hk) + c * 8, ok);
                     load8(v[y], row_ptr(kp.v1, b, ok ? j : 0, hk) + c * 8, ok);
                 }
-                if (x == 0 && u >= 2 && !warp_wait(&bars[F_KV_EMPTY + slot], ((u >> 1) - 1) & 1, abort_flag, 1)) return ERR_FWD;
+                if (u >= 2 && !warp_wait(&bars[F_KV_EMPTY + slot], ((u >> 1) - 1) & 1, abort_flag, 1)) return ERR_FWD;
 #pragma unroll
-                for (int y = 0; y < 2; ++y) {
-                    put8<D>(dk, UNIT, r0 + (x + y) * RPP, c, k[y]);
-                    put8<D>(dv, UNIT, r0 + (x + y) * RPP, c, v[y]);
+                for (int y = 0; y < N; ++y) {
+                    put8<D>(dk, UNIT, r0 + y * RPP, c, k[y]);
+                    put8<D>(dv, UNIT, r0 + y * RPP, c, v[y]);
                 }
             }
             fence_proxy_async_smem();
@@ -142,10 +144,10 @@ __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &
                 const int e = 2 * (g.pair0 + pp * g.dpair) + x;
                 uint8_t *da = sA + x * Planes<D>::bytes(ROWS);
 #pragma unroll 1
-                for (int y0 = 0; y0 < ROWS / RPP; y0 += 2) {
-                    float q[2][8], k2[2][8];
+                for (int y0 = 0; y0 < ROWS / RPP; y0 += 4) {
+                    float q[4][8], k2[4][8];
 #pragma unroll
-                    for (int y = 0; y < 2; ++y) {
+                    for (int y = 0; y < 4; ++y) {
                         const int i = g.i0 + r0 + (y0 + y) * RPP, k = i + kp.off2 - e;
                         const bool ok = i < kp.n && k >= 0 && e < kp.w2;
                         load8(q[y], row_ptr(kp.q, b, ok ? i : 0, h) + c * 8, ok);
@@ -153,7 +155,7 @@ __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &
                     }
                     if (y0 == 0 && pp > 0 && !warp_wait(&bars[F_A_EMPTY + x], (pp - 1) & 1, abort_flag, 2)) return ERR_FWD;
 #pragma unroll
-                    for (int y = 0; y < 2; ++y) {
+                    for (int y = 0; y < 4; ++y) {
 #pragma unroll
                         for (int z = 0; z < 8; ++z) q[y][z] = mul * q[y][z] * k2[y][z];
                         put8<D>(da, ROWS, r0 + (y0 + y) * RPP, c, q[y]);
@@ -167,9 +169,10 @@ __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &
     return 0;
 }
 
-// Softmax group x.  Leaves the row's partial output in o[] against the reference `ref`, with the denominator l.
+// Softmax group x.  Leaves the row's partial output in TMEM (columns o) against the reference `ref`, with the denominator l; returns
+// whether there is one through `any`.
 template <int D>
-__device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom &g, int x, uint32_t tmem, uint64_t (&o)[D / 2], float &ref, float &l,
+__device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom &g, int x, uint32_t tmem, uint32_t o, bool &any, float &ref, float &l,
                                            uint64_t *bars, volatile int *abort_flag) {
     const int r = threadIdx.x & 127;
     const uint32_t region = tmem + ((uint32_t)(r & 96) << 16) + x * 160;
@@ -179,7 +182,8 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
     const float mul = kp.scale * LOG2E;
     uint64_t ws[D / 2];
 #pragma unroll
-    for (int z = 0; z < D / 2; ++z) { o[z] = 0; ws[z] = 0; }
+    for (int z = 0; z < D / 2; ++z) ws[z] = 0;
+    any = false;
     ref = -CUDART_INF_F;
     l = 0.f;
     // W of the unit before: to the sum of its sweep, and at the end of the sweep to the row
@@ -187,15 +191,33 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
         add_acc<D>(region + 96, ws);
         if (!last) return;
         const int k = i + kp.off2 - e;
-        if (row_ok && e < kp.w2 && k >= 0) {
-            const float4 *v2 = reinterpret_cast<const float4 *>(row_ptr(kp.v2, b, k, hk));
+        const bool ok = row_ok && e < kp.w2 && k >= 0;
+        const float4 *v2 = reinterpret_cast<const float4 *>(row_ptr(kp.v2, b, ok ? k : 0, hk));
 #pragma unroll
-            for (int z = 0; z < D / 4; ++z) {
-                const float4 v = __ldg(v2 + z);
-                o[2 * z] = f2_fma(ws[2 * z], f2_pack(v.x, v.y), o[2 * z]);
-                o[2 * z + 1] = f2_fma(ws[2 * z + 1], f2_pack(v.z, v.w), o[2 * z + 1]);
+        for (int c = 0; c < D; c += 32) {
+            uint32_t t[32];
+            if (any) {
+                tmem_ld32(o + c, t);
+                tmem_wait_ld(t);
+            } else {
+#pragma unroll
+                for (int z = 0; z < 32; ++z) t[z] = 0u;
             }
+            if (ok) {
+#pragma unroll
+                for (int z = 0; z < 8; ++z) {
+                    const float4 v = __ldg(v2 + c / 4 + z);
+                    float a[4];
+                    f2_unpack(f2_fma(ws[c / 2 + 2 * z], f2_pack(v.x, v.y), f2_pack(t[4 * z], t[4 * z + 1])), a[0], a[1]);
+                    f2_unpack(f2_fma(ws[c / 2 + 2 * z + 1], f2_pack(v.z, v.w), f2_pack(t[4 * z + 2], t[4 * z + 3])), a[2], a[3]);
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) t[4 * z + y] = __float_as_uint(a[y]);
+                }
+            }
+            tmem_st32(o + c, t);
         }
+        tmem_wait_st();
+        any = true;
 #pragma unroll
         for (int z = 0; z < D / 2; ++z) ws[z] = 0;
     };
@@ -212,39 +234,40 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
             if (!warp_wait(&bars[F_S_FULL + x], u & 1, abort_flag, 1)) return ERR_FWD;
             tc_fence_after();
             if (u > 0) collect(w == 0, e - 2 * g.dpair);
+            // sixteen columns at a time, either half from the outside in (put_terms)
 #pragma unroll
-            for (int ch = 0; ch < 2; ++ch) {
-                uint32_t s[32];
-                // P of the 32 columns against the reference; their sum
+            for (int y = 0; y < 4; ++y) {
+                const int kk = y < 2 ? y : 5 - y, c0 = 16 * kk;
+                uint32_t s[16];
+                // P of the columns against the reference; their sum
                 auto probs = [&](bool full) -> float {
                     float s0 = 0.f, s1 = 0.f;
                     const uint64_t nref = f2_pack(-ref, -ref), regain = f2_pack(REGAIN, REGAIN);
 #pragma unroll
-                    for (int z = 0; z < 32; z += 2) {
+                    for (int z = 0; z < 16; z += 2) {
                         float a0, a1;
                         f2_unpack(f2_fma(f2_pack(s[z], s[z + 1]), regain, nref), a0, a1);
                         float p0 = ex2(a0), p1 = ex2(a1);
                         if (!full) {
-                            p0 = (uint32_t)(ch * 32 + z - lo) <= len ? p0 : 0.f;
-                            p1 = (uint32_t)(ch * 32 + z + 1 - lo) <= len ? p1 : 0.f;
+                            p0 = (uint32_t)(c0 + z - lo) <= len ? p0 : 0.f;
+                            p1 = (uint32_t)(c0 + z + 1 - lo) <= len ? p1 : 0.f;
                         }
                         s0 += p0; s1 += p1;
                         s[z] = __float_as_uint(p0); s[z + 1] = __float_as_uint(p1);
                     }
                     return s0 + s1;
                 };
-                const int c0 = ch * 32;
-                if (__all_sync(0xffffffffu, lo > c0 + 31 || (int)(lo + len) < c0)) {       // nothing valid for this warp
+                if (__all_sync(0xffffffffu, lo > c0 + 15 || (int)(lo + len) < c0)) {       // nothing valid for this warp
 #pragma unroll
-                    for (int z = 0; z < 32; ++z) s[z] = 0u;
+                    for (int z = 0; z < 16; ++z) s[z] = 0u;
                 } else {
-                    tmem_ld32(region + 32 + c0, s);
+                    tmem_ld16(region + LOGITS + c0, s);
                     tmem_wait_ld(s);
-                    const bool full = __all_sync(0xffffffffu, lo <= c0 && (int)(lo + len) >= c0 + 31);
+                    const bool full = __all_sync(0xffffffffu, lo <= c0 && (int)(lo + len) >= c0 + 15);
                     float sum = full ? probs(true) : probs(false);
                     if (__any_sync(0xffffffffu, !(sum <= 65536.f))) {
                         // a reference moves (always at a row's first keys), or a logit is NaN or +inf
-                        tmem_ld32(region + 32 + c0, s);
+                        tmem_ld16(region + LOGITS + c0, s);
                         tmem_wait_ld(s);
                         scalar_logits<D>(s, column_mask(c0, lo, len), mul,
                                          [&](int z, const float *&pq, const float *&pk2, const float *&pk1) {
@@ -255,25 +278,40 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
                                          [](int, float v) { return v; });
                         float mx = -CUDART_INF_F;
 #pragma unroll
-                        for (int z = 0; z < 32; ++z)
+                        for (int z = 0; z < 16; ++z)
                             if ((uint32_t)(c0 + z - lo) <= len) mx = fmaxf(mx, __uint_as_float(s[z]));
                         float f = 1.f;
                         if (!(sum <= 65536.f) && mx > ref) {
                             f = ex2(ref - mx);                             // 0 on the first hit
-                            const uint64_t f2 = f2_pack(f, f);
                             ref = mx;
                             l *= f;
+                            const uint64_t f2 = f2_pack(f, f);
 #pragma unroll
-                            for (int z = 0; z < D / 2; ++z) { o[z] = f2_mul(o[z], f2); ws[z] = f2_mul(ws[z], f2); }
+                            for (int z = 0; z < D / 2; ++z) ws[z] = f2_mul(ws[z], f2);
                         }
-                        if (ch == 1 && __any_sync(0xffffffffu, f != 1.f)) {
-                            // the unit's first 32 columns were formed against the old one
+                        if (__any_sync(0xffffffffu, f != 1.f)) {
+                            // what was formed against the old one: the output, and this unit's columns so far
                             tmem_wait_st();
-                            uint32_t first[32];
-                            get_terms(region, 0, first);
+                            if (any)
+#pragma unroll 1
+                                for (int c = 0; c < D; c += 32) {
+                                    uint32_t t[32];
+                                    tmem_ld32(o + c, t);
+                                    tmem_wait_ld(t);
 #pragma unroll
-                            for (int z = 0; z < 32; ++z) first[z] = __float_as_uint(__uint_as_float(first[z]) * f);
-                            put_terms(region, 0, first);
+                                    for (int z = 0; z < 32; ++z) t[z] = __float_as_uint(__uint_as_float(t[z]) * f);
+                                    tmem_st32(o + c, t);
+                                }
+#pragma unroll 1
+                            for (int before = 0; before < y; ++before) {
+                                const int kb = before < 2 ? before : 5 - before;
+                                uint32_t t[16];
+                                get_terms(region, kb, t);
+#pragma unroll
+                                for (int z = 0; z < 16; ++z) t[z] = __float_as_uint(__uint_as_float(t[z]) * f);
+                                put_terms(region, kb, t);
+                            }
+                            tmem_wait_st();
                         }
                         // (no reference yet, and none here: logits of -inf weigh nothing, and only NaN stays NaN)
                         const float keep = ref;
@@ -283,7 +321,7 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
                     }
                     l += sum;
                 }
-                put_terms(region, ch, s);
+                put_terms(region, kk, s);
             }
             tmem_wait_st();
             tc_fence_before();
@@ -313,7 +351,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     if (threadIdx.x == 0) {
         for (int x = 0; x < F_BAR_COUNT; ++x) {
-            const bool one = x == F_A_EMPTY || x == F_A_EMPTY + 1 || x == F_S_FULL || x == F_S_FULL + 1;
+            const bool one = x == F_A_EMPTY || x == F_A_EMPTY + 1 || x == F_S_FULL || x == F_S_FULL + 1 || x >= F_TURN;
             const bool two = x == F_KV_EMPTY || x == F_KV_EMPTY + 1;
             mbar_init(&bars[x], one ? 1u : two ? 2u : 128u);
         }
@@ -346,24 +384,30 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
     } else if (warp < 12) {
         reg_alloc<FWD_REGS_SOFTMAX>();
         const int x = (warp >> 2) - 1, r = threadIdx.x & 127;
-        uint64_t o[D / 2];
+        const uint32_t o = tmem + ((uint32_t)(r & 96) << 16) + 320 + 64 * x;
         float ref, l;
-        err = fwd_softmax<D>(kp, g, x, tmem, o, ref, l, bars, abort_flag);
+        bool any;
+        err = fwd_softmax<D>(kp, g, x, tmem, o, any, ref, l, bars, abort_flag);
         const bool bad = __any_sync(0xffffffffu, err != 0) || *abort_flag != 0;
         tc_fence_before();
         __syncthreads();                  // no product reads the operands any more
         float *row = part + (x * ROWS + r) * LD;
 #pragma unroll
-        for (int z = 0; z < D / 4; ++z) {
-            float4 v;
-            f2_unpack(o[2 * z], v.x, v.y);
-            f2_unpack(o[2 * z + 1], v.z, v.w);
-            *reinterpret_cast<float4 *>(row + 4 * z) = bad ? make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F) : v;
+        for (int c = 0; c < D; c += 32) {
+            uint32_t t[32];
+            tmem_ld32(o + c, t);
+            tmem_wait_ld(t);
+#pragma unroll
+            for (int z = 0; z < 32; z += 4)
+                *reinterpret_cast<float4 *>(row + c + z) =
+                    bad ? make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F)
+                        : !any ? make_float4(0.f, 0.f, 0.f, 0.f)
+                               : make_float4(__uint_as_float(t[z]), __uint_as_float(t[z + 1]), __uint_as_float(t[z + 2]), __uint_as_float(t[z + 3]));
         }
         stats[(x * 2) * ROWS + r] = bad ? 0.f : ref;
         stats[(x * 2 + 1) * ROWS + r] = bad ? CUDART_NAN_F : l;
     } else {
-        reg_dealloc<FWD_REGS_BUILD>();
+        reg_alloc<FWD_REGS_BUILD>();
         err = fwd_build<D>(kp, g, sA, sK, sV, bars, abort_flag);
         tc_fence_before();
         __syncthreads();
