@@ -44,19 +44,20 @@
 // W [448, 512); head dim 128 has two buffers, U [256, 384) and W [384, 512).  The fold groups read U / W into registers before the
 // next sweep's first product.
 //
-// Bound, up to head dim 64: the compute groups, busy ~1080 of ~1250 cycles a unit (512 of them MUFU cycles of two warps a scheduler;
+// Bound, up to head dim 64: the compute groups, busy ~1080 of ~1280 cycles a unit (512 of them MUFU cycles of two warps a scheduler;
 // the wait accounting shows them waiting 10 to 15 % of the time, every other role half of it).  Everything that goes through shared
-// memory waits behind the tensor cores' operand fetches (300 cycles and more an access), so the folds read U and W into registers
-// at once, which frees the accumulators, and add at their leisure; the second keys come from a staged copy.  At head dim 128 the fold
-// of U has no registers for that: its ~18000 cycles a sweep (half a row per lane from L2) hold up the next sweep's U / W.
+// memory waits behind the tensor cores' operand fetches (300 cycles and more an access), so a fold reads half a row of U or W at a
+// time, loads what two pieces of it need before it adds and stores, and has its second keys in a staged copy; windows of few units
+// are bound by the folds, ~6000 cycles a sweep.  At head dim 128 the fold of U has no registers for half a row: its ~18000 cycles a
+// sweep (operands from L2, half a row per lane) hold up the next sweep's U / W.
 // Measured, this kernel and its reduction, against tiles of 128 rows and one offset with the window in two splits (head dim 64) or two
-// CTAs of 64 channels each that formed S and dP twice (head dim 128): b4 n4096 h8 d64 w512/32 1.62 -> 1.35 ms, b16 n1024 1.45 -> 1.24
-// (layer), b1 n3001 h8/2 w1024/16 0.28 -> 0.28, b1 n16384 h16 d128 w512/32 8.7 -> 7.6 ms.
-// Measured and not kept, head dim 64 where this form takes 1.30 (without the reduction): U and W read as they are folded 1.82 (U / W of
-// the next sweep wait), compute groups on alternate units 1.35, 32 columns at a time with 88 registers 1.41, the next sixteen
-// columns fetched ahead 1.69 (spills), the mask applied to every unit 1.37; head dim 128, 7.6: a ring of two slots with q and dO
-// staged in its place 8.6, one slot 10.5, eight channels at a time with operands fetched one to four ahead 7.9 to 8.2, both operands
-// built by the W fold 7.8.
+// CTAs of 64 channels each that formed S and dP twice (head dim 128): b4 n4096 h8 d64 w512/32 1.64 -> 1.38 ms, b1 n3001 h8 w1024/16
+// 320 -> 288 us, b4 n1966 h4 w105/26 211 -> 207, b1 n300 h4 w300/32 56 -> 44, b1 n16384 h16 d128 w512/32 8.74 -> 7.61 ms.
+// Measured and not kept (head dim 64, C = b4 n4096 above, S = b4 n1966): a row of U or W read at once, which frees the accumulators
+// sooner and leaves no registers to load ahead, C 1.35 but S 229 us; U and W read sixteen channels at a time, C 1.87; compute groups on
+// alternate units, C 1.40; 32 columns at a time with 88 registers, C 1.46; the next sixteen columns fetched ahead, C 1.74 (spills); the
+// mask applied to every unit, C 1.42.  Head dim 128: a ring of two slots with q and dO staged in its place 8.8 ms, one slot 10.5,
+// eight channels at a time with operands fetched one to four ahead 7.9 to 8.2, both operands built by the W fold 7.8.
 #pragma once
 #include "sa2_tc_bwd_k1.cuh"
 
@@ -78,7 +79,7 @@ constexpr int BQ_MAX_EPC = 56;
 
 // Register hand-over between warpgroups.  A group can only grow by what another has released, or its setmaxnreg
 // never returns, so the budgets must add up to what the block was launched with: five groups of 96 (640 threads).  Up to head dim
-// 64 the U fold takes 160 (dQ, q and k2 rows, 128 registers, and a chunk of U), the W fold 104; at head dim 128 the U fold 184 (dQ,
+// 64 the U fold takes 176 (dQ, the q row and half a row of U, 128 registers, and what two pieces need), the W fold 112; at head dim 128 the U fold 184 (dQ,
 // 128 registers, and chunks of the rest), the W fold 96.
 template <int D, bool SPLIT> struct BqCfg {
     static constexpr int THREADS = 640;
@@ -570,25 +571,18 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         auto ychunk = [&](int cc) { return ok ? __ldg(py + (cc ^ (rot / 8))) : zero; };
         if (!warp_wait(&bars[BQ_W_FULL + WHICH], t & 1, abort_flag, 1)) return false;
         tc_fence_after();
-        // Up to head dim 64 U and W are read at once, so that the tensor cores may soon overwrite them; the additions to
-        // shared memory, which wait behind the tensor cores' fetches, then have a sweep's time.
+        // Up to head dim 64 half a row of U or W is read at a time, head dim 128 reads sixteen channels.
         constexpr int H = D / 2;
-        uint32_t held[2][HELD ? H : 1];
-        auto read = [&](int half) {
-            uint32_t (&to)[HELD ? H : 1] = held[half];
-            if constexpr (D == 64) tmem_ld32(cols + ((half * H) ^ rot), to);
-            else if constexpr (D == 32) tmem_ld16(cols + ((half * H) ^ rot), to);
-        };
-        auto release = [&]() {
+        uint32_t part[HELD ? H : 16];
+        auto read = [&](int c) {
+            if constexpr (D == 64) tmem_ld32(cols + (c ^ rot), part);
+            else tmem_ld16(cols + (c ^ rot), part);
             tmem_wait_ld();
+        };
+        auto release = [&]() {            // the rest is in registers: the tensor cores may overwrite the accumulator
             tc_fence_before();
             mbar_arrive(&bars[BQ_W_EMPTY + WHICH]);
         };
-        if constexpr (HELD) {
-            read(0);
-            read(1);
-            release();
-        }
         // every row of the ring belonged to other threads in the last sweep
         if (t >= 1 && !warp_wait(&bars[BQ_FOLD_SYNC + WHICH], (t - 1) & 1, abort_flag, 2)) return false;
         const bool sole = r == BQ_ROWS - 1 || r == BQ_ROWS;           // the first row of the sweep and the last have one writer
@@ -597,7 +591,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         ulonglong2 *gone = reinterpret_cast<ulonglong2 *>(slab + (size_t)slab_row * D);
         // GROUP pieces of eight channels at a time: all their loads first, since every access to shared memory waits behind the
         // tensor cores' fetches (300 cycles and more)
-        constexpr int GROUP = HELD ? 1 : 2;
+        constexpr int GROUP = 2;
 #pragma unroll
         for (int c0 = 0; c0 < NC; c0 += GROUP) {
             const bool second = c0 >= NC / 2;
@@ -624,11 +618,9 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
                 a[g][0] = a[g][1] = make_ulonglong2(0, 0);
                 if (!fresh) { a[g][0] = *place_of(g, 0); a[g][1] = *place_of(g, 1); }
             }
-            uint32_t stream[HELD ? 1 : 16];
-            if constexpr (!HELD) {
-                tmem_ld16(cols + ((c0 * 8) ^ rot), stream);
-                tmem_wait_ld();
-                if (c0 + GROUP == NC) release();
+            if (!HELD || c0 % (NC / 2) == 0) {
+                read(c0 * 8);
+                if (HELD ? c0 == NC / 2 : c0 + GROUP == NC) release();
             }
 #pragma unroll
             for (int g = 0; g < GROUP; ++g) {
@@ -638,11 +630,8 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
                 if (ok) {
 #pragma unroll
                     for (int z = 0; z < 4; ++z) {
-                        const int q = (cc * 8) % H + 2 * z;
-                        uint32_t u0, u1;
-                        if constexpr (HELD) { u0 = held[second ? 1 : 0][HELD ? q : 0]; u1 = held[second ? 1 : 0][HELD ? q + 1 : 0]; }
-                        else { u0 = stream[HELD ? 0 : 8 * g + 2 * z]; u1 = stream[HELD ? 0 : 8 * g + 2 * z + 1]; }
-                        const uint64_t t2 = f2_pack(u0, u1);
+                        const int q = (HELD ? cc * 8 % H : 8 * g) + 2 * z;
+                        const uint64_t t2 = f2_pack(part[q], part[q + 1]);
                         if constexpr (WHICH == 0) dq[cc * 4 + z] = f2_fma(t2, f2_from_bf16x2(yw[z]), dq[cc * 4 + z]);
                         *sum[z] = f2_fma(t2, f2_from_bf16x2(xw[z]), *sum[z]);
                     }
