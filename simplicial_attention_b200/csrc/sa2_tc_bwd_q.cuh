@@ -53,6 +53,9 @@
 // Measured, this kernel and its reduction, against tiles of 128 rows and one offset with the window in two splits (head dim 64) or two
 // CTAs of 64 channels each that formed S and dP twice (head dim 128): b4 n4096 h8 d64 w512/32 1.64 -> 1.38 ms, b1 n3001 h8 w1024/16
 // 320 -> 288 us, b4 n1966 h4 w105/26 211 -> 207, b1 n300 h4 w300/32 56 -> 44, b1 n16384 h16 d128 w512/32 8.74 -> 7.61 ms.
+// SPLIT: b4 n3000 h8 d32 w512/32 1.39 -> 1.10 ms, d64 w512/64 4.49 -> 4.19, d128 w512/64 16.7 -> 10.3 (both chunks of a group's columns read
+// before either is written, as it was at first, does not fit 80 registers: 2.12, 5.59 and 12.2).  Slower than the tiles of 128 rows: few
+// units and few offsets, b4 n3000 h8 d64 w64/9 231 -> 254 us, w76/10 252 -> 267, where set-up is a fifth of a CTA.
 // Measured and not kept (head dim 64, C = b4 n4096 above, S = b4 n1966): a row of U or W read at once, which frees the accumulators
 // sooner and leaves no registers to load ahead, C 1.35 but S 229 us; U and W read sixteen channels at a time, C 1.87; compute groups on
 // alternate units, C 1.40; 32 columns at a time with 88 registers, C 1.46; the next sixteen columns fetched ahead, C 1.74 (spills); the
@@ -85,6 +88,7 @@ template <int D, bool SPLIT> struct BqCfg {
     static constexpr int THREADS = 640;
     static constexpr int REGS_LAUNCH = 96, REGS_ISSUE = D <= 64 ? 32 : 40, REGS_COMPUTE = 80;
     static constexpr int REGS_FOLD = D <= 64 ? 176 : 184, REGS_FOLD_W = D <= 64 ? 112 : 96;
+    static_assert(REGS_COMPUTE <= REGS_LAUNCH, "the compute groups release registers");
     static_assert(REGS_ISSUE + 2 * REGS_COMPUTE + REGS_FOLD + REGS_FOLD_W == THREADS / 128 * REGS_LAUNCH, "register pool must balance");
     static constexpr int CB = D == 128 ? 2 : 1;                  // 64-channel blocks of a row
     static constexpr int KSTEPS = D / 16;                        // K = 16 steps of S and dP
@@ -372,20 +376,23 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
         if (!warp_wait(&bars[BQ_S_FULL + buf], use & 1, abort_flag, 1)) return ERR_BQ_COMPUTE;
         tc_fence_after();
         const bool full = __all_sync(0xffffffffu, lo < 0 && hi >= 63);
-        // sixteen columns at a time; SPLIT reads all before it writes: the rests go over columns of the second chunk
-        uint32_t sv[SPLIT ? 2 : 1][16], dv[SPLIT ? 2 : 1][16];
-        auto load = [&](int x) {
-            tmem_ld16(s_addr + c0 + 16 * x, sv[SPLIT ? x : 0]);
-            tmem_ld16(d_addr + c0 + 16 * x, dv[SPLIT ? x : 0]);
-        };
-        if constexpr (SPLIT) { load(0); load(1); }
+        // sixteen columns at a time.  P / G go over the first half of the group's columns of S / dP (the other group's columns of the
+        // buffer may still be unread), the rests over the second half once that has been read
+        uint32_t pr[2][8], gr[2][8];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             const int col = c0 + 16 * x;
-            uint32_t (&s)[16] = sv[SPLIT ? x : 0], (&d)[16] = dv[SPLIT ? x : 0], pp[8], gg[8], pr[8], gr[8];
-            if constexpr (!SPLIT) load(x);
+            uint32_t s[16], d[16], pp[8], gg[8];
+            tmem_ld16(s_addr + col, s);
+            tmem_ld16(d_addr + col, d);
             tmem_wait_ld(s);
             tmem_wait_ld(d);
+            if constexpr (SPLIT) {
+                if (x == 1) {
+                    tmem_st8(s_addr + c0 + 16, pr[0]);
+                    tmem_st8(d_addr + c0 + 16, gr[0]);
+                }
+            }
             auto pass = [&](bool masked) {
                 const float m = mid - 2048.f * (float)col;
 #pragma unroll
@@ -396,21 +403,21 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
                         a0 = fminf(a0, half - fabsf(2048.f * z - m));
                         a1 = fminf(a1, half - fabsf(2048.f * (z + 1) - m));
                     }
-                    pg_pair<SPLIT>(ex2(a0), ex2(a1), d[z], d[z + 1], ndl2, pp[z >> 1], gg[z >> 1], pr[SPLIT ? z >> 1 : 0], gr[SPLIT ? z >> 1 : 0]);
+                    pg_pair<SPLIT>(ex2(a0), ex2(a1), d[z], d[z + 1], ndl2, pp[z >> 1], gg[z >> 1], pr[x][z >> 1], gr[x][z >> 1]);
                 }
             };
             if (full) pass(false);
             else if (__all_sync(0xffffffffu, hi < col || lo >= col + 15)) {        // no row of this warp has a valid column here
 #pragma unroll
-                for (int z = 0; z < 8; ++z) pp[z] = gg[z] = pr[z] = gr[z] = 0u;
+                for (int z = 0; z < 8; ++z) pp[z] = gg[z] = pr[x][z] = gr[x][z] = 0u;
             } else pass(true);
-            // P / G over the first half of the group's columns of S / dP (the other group's columns of the buffer may still be
-            // unread), the rests over the second half
             tmem_st8(s_addr + c0 + 8 * x, pp);
             tmem_st8(d_addr + c0 + 8 * x, gg);
             if constexpr (SPLIT) {
-                tmem_st8(s_addr + c0 + 16 + 8 * x, pr);
-                tmem_st8(d_addr + c0 + 16 + 8 * x, gr);
+                if (x == 1) {
+                    tmem_st8(s_addr + c0 + 24, pr[1]);
+                    tmem_st8(d_addr + c0 + 24, gr[1]);
+                }
             }
         }
         tmem_wait_st();
@@ -767,7 +774,7 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     } else if (warp < 12) {
         // one call site for both compute groups: they run the same instructions, which the instruction caches
         // of a scheduler then hold once (with two copies: 3.5 ms against 2.3)
-        reg_dealloc<C::REGS_COMPUTE>();
+        if constexpr (C::REGS_COMPUTE < C::REGS_LAUNCH) reg_dealloc<C::REGS_COMPUTE>();
         err = bq_compute<D, SPLIT>(P, g, (warp >> 2) - 1, tmem, bars, abort_flag);
     } else if (warp < 16) {
         reg_alloc<C::REGS_FOLD>();
