@@ -28,6 +28,16 @@ def default(v, d):
     return v if exists(v) else d
 
 
+def _child(module, name):
+    """``module.name`` for a submodule or parameter, from the module's own tables where it is there: torch's attribute lookup
+    costs a generation step of one sequence, which the host bounds, a third of a microsecond each."""
+    d = module.__dict__
+    found = d["_modules"].get(name)
+    if found is None:
+        found = d["_parameters"].get(name)
+    return getattr(module, name) if found is None else found
+
+
 class HigherOrderAttention(Module):
     """Projection / head-split / norm shell with a pluggable ``attend``
     callable ``attend(queries, keys, values[, causal=True]) -> out``
@@ -177,15 +187,16 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
                 and at.keywords.keys() <= {"w1", "w2", "causal", "kernel"} and at.keywords.get("causal", True)):
             return None
         autocast = torch.is_autocast_enabled()
-        norms = (self.q_norm, *self.k_norms, *self.v_norms)
-        eps = self.q_norm.eps
-        if any(n.eps != eps for n in norms):
-            return None
+        norms = [_child(self, "q_norm"), *_child(self, "k_norms")._modules.values(), *_child(self, "v_norms")._modules.values()]
+        eps = norms[0].eps
+        for n in norms:
+            if n.eps != eps:
+                return None
         # the modules leave eps unset: the machine epsilon of the dtype they compute in (fp32 under autocast)
         if eps is None:
             eps = torch.finfo(torch.float32 if autocast else proj.dtype).eps
         dtype = torch.get_autocast_dtype("cuda") if autocast else proj.dtype
-        return ([n.weight for n in norms], (self.heads, self.key_value_heads, self.dim_head, eps), dtype,
+        return ([_child(n, "weight") for n in norms], (self.heads, self.key_value_heads, self.dim_head, eps), dtype,
                 (at.keywords.get("w1", 512), at.keywords.get("w2", 32), _lib.KERNELS[at.keywords.get("kernel", "auto")]))
 
     def _attend_packed(self, tokens):
@@ -202,10 +213,10 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
     def _step(self, tokens, cache):
         """A generation step as one native call, or None where a submodule is not the plain one this class made
         (another type, a hook, a bias) or autocast is on: then the modules are called one by one."""
-        pre, post, qkv, comb = self.prenorm, self.postnorm, self.to_qkv, self.combine_heads
+        pre, post, qkv, comb = [_child(self, name) for name in ("prenorm", "postnorm", "to_qkv", "combine_heads")]
         norms = (RowRMSNorm, Identity)
         if type(pre) not in norms or type(post) not in norms or type(qkv) is not Linear or type(comb) is not Linear \
-                or qkv.bias is not None or comb.bias is not None or torch.is_autocast_enabled() or _has_any_global_hook():
+                or qkv._parameters.get("bias", qkv) is not None or comb._parameters.get("bias", comb) is not None or torch.is_autocast_enabled() or _has_any_global_hook():
             return None
         for m in (pre, post, qkv, comb):
             if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
@@ -214,8 +225,8 @@ class SlidingWindowTwoSimplicialMHA(HigherOrderAttention):
         if call is None or call[3][:2] != (self.w1, self.w2):
             return None
         gains, heads, dtype, windows = call
-        args = [(None, 0.) if type(m) is Identity else (m.weight, m.eps if m.eps is not None else torch.finfo(dtype).eps) for m in (pre, post)]
-        return _lib.ext().step(tokens, *args[0], qkv.weight, gains, [*cache[0], *cache[1]], *heads, *windows, comb.weight, *args[1])
+        args = [(None, 0.) if type(m) is Identity else (_child(m, "weight"), m.eps if m.eps is not None else torch.finfo(dtype).eps) for m in (pre, post)]
+        return _lib.ext().step(tokens, *args[0], _child(qkv, "weight"), gains, [*cache[0], *cache[1]], *heads, *windows, _child(comb, "weight"), *args[1])
 
     def forward(self, tokens, cache=None, return_cache=False):
         """``cache`` (from an earlier call with ``return_cache=True``) holds the last ``w1 - 1`` rows of the
