@@ -46,8 +46,8 @@ typedef enum sa2_status {
 
 typedef enum sa2_dtype { SA2_F32 = 0, SA2_BF16 = 1 } sa2_dtype;
 
-/* Which implementation runs.  AUTO picks the tcgen05 tensor-core path when the
- * problem fits it (bf16, supported head dim) and the fp32 SIMT path otherwise. */
+/* Which implementation runs.  AUTO picks a tcgen05 tensor-core path when the problem fits it (bf16; fp32 of head
+ * dims 32 and 64, each operand as three bf16 terms) and the scalar fp32 path otherwise. */
 typedef enum sa2_kernel { SA2_KERNEL_AUTO = 0, SA2_KERNEL_SIMT = 1, SA2_KERNEL_TCGEN05 = 2 } sa2_kernel;
 
 /* element strides of one [batch][seq][head][channel] tensor */

@@ -4,7 +4,8 @@
 // fp32, every product and sum is fp32, and nothing is rounded to bf16 on the
 // way.  They handle every head dim in {32, 64, 128}, any sequence length, any
 // window and grouped-query heads, and they are the kernels the tensor-core
-// path is checked against on the device.
+// path is checked against on the device.  fp32 tensors of head dims 32 and 64 come here only by request, without
+// scratch, or where their backward needs more of it than is allowed; sa2_f32.cuh has them otherwise.
 //
 // Formulation ("k'-offset"): for an offset e = i - k in [0, w2) every query
 // row i is paired with ONE second key k2[i-e].  A_e[i,:] = scale*q_i*k2_{i-e}

@@ -54,8 +54,9 @@
 // CTAs of 64 channels each that formed S and dP twice (head dim 128): b4 n4096 h8 d64 w512/32 1.64 -> 1.38 ms, b1 n3001 h8 w1024/16
 // 320 -> 288 us, b4 n1966 h4 w105/26 211 -> 207, b1 n300 h4 w300/32 56 -> 44, b1 n16384 h16 d128 w512/32 8.74 -> 7.61 ms.
 // SPLIT: b4 n3000 h8 d32 w512/32 1.39 -> 1.10 ms, d64 w512/64 4.49 -> 4.19, d128 w512/64 16.7 -> 10.3 (both chunks of a group's columns read
-// before either is written, as it was at first, does not fit 80 registers: 2.12, 5.59 and 12.2).  Slower than the tiles of 128 rows: few
-// units and few offsets, b4 n3000 h8 d64 w64/9 231 -> 254 us, w76/10 252 -> 267, where set-up is a fifth of a CTA.
+// before either is written, as it was at first, does not fit 80 registers: 2.12, 5.59 and 12.2).  Slower than the tiles of 128 rows: windows
+// of one to three units up to head dim 64, b16 n128 h8 94 -> 113 us, b4 n3000 h8 d64 w64/9 231 -> 254 us, w76/10 252 -> 267: a sweep
+// takes what its fold takes, and the fold of two offsets has a barrier more.
 // Measured and not kept (head dim 64, C = b4 n4096 above, S = b4 n1966): a row of U or W read at once, which frees the accumulators
 // sooner and leaves no registers to load ahead, C 1.35 but S 229 us; U and W read sixteen channels at a time, C 1.87; compute groups on
 // alternate units, C 1.40; 32 columns at a time with 88 registers, C 1.46; the next sixteen columns fetched ahead, C 1.74 (spills); the
