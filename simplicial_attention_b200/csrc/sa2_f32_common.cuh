@@ -24,7 +24,8 @@ constexpr int ROWS = 128;         // rows of a tile: TMEM lanes
 constexpr int UNIT = 64;          // columns of a logit tile
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 // What a logit loses to the truncations of its large products, half a unit in the last place each and about one in all, is given
-// back where the reference or the logsumexp is subtracted.
+// back in the logsumexp, and where the backward subtracts that.  Not where a row's reference is subtracted: the largest logit has
+// weight 1 whatever its size, and what a difference of 150 at most loses is below its own last place.
 constexpr float REGAIN = 1.f + 1.1920929e-7f;
 // error bits of the device status word
 enum { ERR_FWD = 1 << 17, ERR_BWD = 1 << 18 };

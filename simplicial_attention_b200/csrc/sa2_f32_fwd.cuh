@@ -242,11 +242,11 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
                 // P of the columns against the reference; their sum
                 auto probs = [&](bool full) -> float {
                     float s0 = 0.f, s1 = 0.f;
-                    const uint64_t nref = f2_pack(-ref, -ref), regain = f2_pack(REGAIN, REGAIN);
+                    const uint64_t nref = f2_pack(-ref, -ref);
 #pragma unroll
                     for (int z = 0; z < 16; z += 2) {
                         float a0, a1;
-                        f2_unpack(f2_fma(f2_pack(s[z], s[z + 1]), regain, nref), a0, a1);
+                        f2_unpack(f2_add(f2_pack(s[z], s[z + 1]), nref), a0, a1);
                         float p0 = ex2(a0), p1 = ex2(a1);
                         if (!full) {
                             p0 = (uint32_t)(c0 + z - lo) <= len ? p0 : 0.f;
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
 #pragma unroll
         for (int z = 0; z < 4; ++z) v[z] *= inv;
         store_vec<4>(kp.out.p, elem_off(kp.out, blockIdx.z, i, blockIdx.y) + c, false, v);
-        if (c == 0) kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = M * LN2 + __logf(L);
+        if (c == 0) kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = M * REGAIN * LN2 + __logf(L);
     }
     cl.sync();               // no CTA leaves while its shared memory is read
     if (warp == 0) {

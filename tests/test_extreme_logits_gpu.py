@@ -54,6 +54,23 @@ def test_rising_logits_with_large_values_fp32(d):
     assert (out - ref).abs().max().item() <= 1e-4 * ref.abs().max().item()
 
 
+@pytest.mark.parametrize("sign", [1., -1.])
+@pytest.mark.parametrize("size", [300., 700., 3000.])
+@pytest.mark.parametrize("d", [32, 64])
+def test_large_finite_logits_fp32(d, size, sign):
+    """Logits of 1e8 to 1e11, all of one sign: a row is its largest logit's value, far ahead of what either kernel's logits are off by
+    (a few units in the last place), so that the weights are 0 and 1 and a result is v1 * v2 to the last bits."""
+    ins = _operands(d, torch.float32)
+    for t in ins[:3]:
+        t.abs_().mul_(size)
+    out, lse = sa.sa2_forward(*ins, 100, 4, scale=sign * d ** -0.5)
+    want, want_lse = sa.sa2_forward(*ins, 100, 4, scale=sign * d ** -0.5, kernel="simt")
+    assert sa.device_status() == 0
+    assert want.isfinite().all() and out.isfinite().all() and lse.isfinite().all()
+    assert (out - want).norm() <= 2 ** -20 * want.norm()
+    assert (lse - want_lse).norm() <= 2 ** -20 * want_lse.norm()
+
+
 BF16 = [(32, 100), (64, 100), (64, 600), (128, 100)]
 
 
