@@ -155,7 +155,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // D[tmem] (+)= A[smem] * B[smem]
@@ -230,10 +229,14 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
     "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), \
     "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
 // Wait for the TMEM loads in flight, tied to the registers of one of them: nothing that uses `r` can be moved
-// above the wait, so a load may be issued well before its values are needed.
+// above the wait, so a load may be issued well before its values are needed.  (There is no form without registers: arithmetic on
+// them is not ordered by a memory clobber.)
 __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" : SA2_R32(r) :: "memory");
 }
+
+// ... and the registers of another load that the same wait is for
+__device__ __forceinline__ void tmem_waited(uint32_t (&r)[32]) { asm volatile("" : SA2_R32(r)); }
 
 __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"

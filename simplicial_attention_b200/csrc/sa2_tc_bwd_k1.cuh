@@ -360,7 +360,8 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
                     uint32_t sv[32], dv[32], pk[16], gk[16], pr[SPLIT ? 16 : 1], gr[SPLIT ? 16 : 1];
                     tmem_ld32(buf + ch * 32, sv);
                     tmem_ld32(buf + 64 + ch * 32, dv);
-                    tmem_wait_ld();
+                    tmem_wait_ld(sv);
+                    tmem_waited(dv);
                     // the accumulators already hold S^T - lse2 / c and dP^T - D
                     auto pair = [&](int x, float a0, float a1) {
                         const float p0 = ex2(a0), p1 = ex2(a1);
@@ -423,11 +424,11 @@ __device__ __forceinline__ int bk1_compute(const BwdParams &P, const Bk1Geom &g,
     for (int hf = 0; hf < D / 32; ++hf) {
         uint32_t w[32];
         tmem_ld32(lane_addr + 384 + half * 64 + hf * 32, w);
-        tmem_wait_ld();
+        tmem_wait_ld(w);
         if constexpr (bwd_split<D>) {
             uint32_t rest[32];
             tmem_ld32(lane_addr + 384 + half * 64 + 32, rest);
-            tmem_wait_ld();
+            tmem_wait_ld(rest);
 #pragma unroll
             for (int x = 0; x < 32; ++x) w[x] = __float_as_uint(__uint_as_float(w[x]) + __uint_as_float(rest[x]));
         }

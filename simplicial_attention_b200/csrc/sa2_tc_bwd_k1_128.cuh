@@ -340,7 +340,8 @@ __device__ __forceinline__ int compute(const Params &P, const Geom &g, int half,
                     uint32_t sv[32], dv[32], pk[16], gk[16];
                     tmem_ld32(buf + ch * 32, sv);
                     tmem_ld32(buf + 64 + ch * 32, dv);
-                    tmem_wait_ld();
+                    tmem_wait_ld(sv);
+                    tmem_waited(dv);
                     // the accumulators already hold S^T - lse2 / c and dP^T - D
                     auto pair = [&](int x, float a0, float a1) {
                         const float p0 = ex2(a0), p1 = ex2(a1);
@@ -392,7 +393,7 @@ __device__ __forceinline__ int compute(const Params &P, const Geom &g, int half,
     for (int q4 = 0; q4 < 4; ++q4) {
         uint32_t w[32];
         tmem_ld32(lane_addr + 256 + half * 128 + q4 * 32, w);
-        tmem_wait_ld();
+        tmem_wait_ld(w);
         if (P.ce > 1 && jv) {
             float *row = P.part + (((((size_t)(blockIdx.x % P.ce) * kp.b + b) * kp.nk1 + j) * kp.hk + hk) * 2 + half) * 128 + q4 * 32;
 #pragma unroll

@@ -585,7 +585,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         auto read = [&](int c) {
             if constexpr (D == 64) tmem_ld32(cols + (c ^ rot), part);
             else tmem_ld16(cols + (c ^ rot), part);
-            tmem_wait_ld();
+            tmem_wait_ld(part);
         };
         auto release = [&]() {            // the rest is in registers: the tensor cores may overwrite the accumulator
             tc_fence_before();

@@ -276,10 +276,10 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
                     mbar_arrive(&bars[B_P_FULL + grp * 2 + pending]);
                     pending = -1;
                 }
-                tmem_wait_ld();
+                tmem_wait_ld(s);
                 float tile_sum = chunk(s, pk0, 0);
                 tmem_ld32(buf + 32, s);
-                tmem_wait_ld();
+                tmem_wait_ld(s);
                 tile_sum += chunk(s, pk1, 1);
                 const bool exceed = !(tile_sum <= 1.8446744e19f);       // above 2^64, inf or NaN
                 if (__any_sync(0xffffffffu, exceed)) {
@@ -288,7 +288,7 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
 #pragma unroll 1
                     for (int ch = 0; ch < 2; ++ch) {
                         tmem_ld32(buf + ch * 32, s);
-                        tmem_wait_ld();
+                        tmem_wait_ld(s);
 #pragma unroll
                         for (int x = 0; x < 32; ++x) {
                             const int col = ch * 32 + x;
@@ -310,17 +310,17 @@ __device__ __forceinline__ int softmax(const Params &P, const Geom &g, int grp, 
 #pragma unroll 1
                         for (int q4 = 0; q4 < 4; ++q4) {
                             tmem_ld32(w_addr + q4 * 32, s);
-                            tmem_wait_ld();
+                            tmem_wait_ld(s);
 #pragma unroll
                             for (int x = 0; x < 32; ++x) s[x] = __float_as_uint(__uint_as_float(s[x]) * f);
                             tmem_st32(w_addr + q4 * 32, s);
                         }
                     }
                     tmem_ld32(buf, s);
-                    tmem_wait_ld();
+                    tmem_wait_ld(s);
                     tile_sum = fwd_probs32<false>(s, pk0, pk0, c, ref, false, 0, lo, hi);
                     tmem_ld32(buf + 32, s);
-                    tmem_wait_ld();
+                    tmem_wait_ld(s);
                     tile_sum += fwd_probs32<false>(s, pk1, pk1, c, ref, false, 32, lo, hi);
                 }
                 l += tile_sum;
@@ -428,7 +428,7 @@ __device__ __forceinline__ int output(const Params &P, const Geom &g, int cb, ui
         for (int q4 = 0; q4 < 4; ++q4) {
             uint32_t w[16];
             tmem_ld16(lane_addr + 256 + grp * 128 + cb * 64 + q4 * 16, w);
-            tmem_wait_ld();
+            tmem_wait_ld(w);
             if (ok) {
 #pragma unroll
                 for (int u8 = 0; u8 < 2; ++u8) {
