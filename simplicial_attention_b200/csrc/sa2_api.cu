@@ -183,7 +183,7 @@ int sa2_kernel_launches(const sa2_shape *shape, int backward) {
     if (s.kernel == SA2_KERNEL_TCGEN05 && !tc_ok) return -1;
     if (tc_ok && s.kernel != SA2_KERNEL_SIMT && !(backward && !sa2::tc::bwd_scale_ok(s)))
         return sa2::tc::launches(s, backward != 0, {shape->w2, shape->b});
-    if (sa2::f32::supported(s) && backward) return sa2::f32::bwd_launches(s, shape->b, sa2::tc::SM_COUNT);
+    if (sa2::f32::supported(s)) return backward ? sa2::f32::bwd_launches(s, shape->b, sa2::tc::SM_COUNT) : 2;
     return backward ? 2 : 1;   // SIMT: row sums + all gradients
 }
 
@@ -264,7 +264,8 @@ int sa2_bwd_part(const sa2_bwd_args *a, int32_t whole_b) {
         int *status = sa2::tc::status_word();
         if (!status) return SA2_ERR_CUDA;
         char *extra = reinterpret_cast<char *>(a->workspace) + delta;
-        if (plan.tc) return s.d == 32 ? sa2::f32::bwd<32>(p, plan, extra, status, st, a->phases) : sa2::f32::bwd<64>(p, plan, extra, status, st, a->phases);
+        if (plan.tc) return s.d == 32 ? sa2::f32::bwd<32>(p, plan, extra, status, sa2::tc::SM_COUNT, st, a->phases)
+                                    : sa2::f32::bwd<64>(p, plan, extra, status, sa2::tc::SM_COUNT, st, a->phases);
     }
 
     switch (s.d) {

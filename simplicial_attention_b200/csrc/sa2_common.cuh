@@ -26,6 +26,19 @@ struct KernelParams {
     float scale;
 };
 
+// A logsumexp that stands for "not computed": rows that a kernel leaves to the scalar one behind it (a NaN that arithmetic does not
+// return)
+constexpr uint32_t LSE_REDO = 0x7fc5a2e1u;
+
+// What A_e = mul * q * k2 carries: scale * log2(e).  The tensor-core kernels of fp32 tensors (and the scalar ones behind them) put one
+// unit in the last place on top, about what a logit loses to the truncations of its large products.
+__device__ __forceinline__ float logit_factor(float scale, bool truncated) {
+    const float mul = scale * 1.4426950408889634f;
+    return truncated ? fmaf(mul, 1.1920929e-7f, mul) : mul;
+}
+// ... and what a sum of G A_e has to be multiplied with
+__device__ __forceinline__ float logit_unfactor(float scale, float mul) { return mul == 0.f ? 0.6931471805599453f : scale / mul; }
+
 __device__ __forceinline__ int64_t elem_off(const TensorRef &t, int b, int n, int h) {
     return (int64_t)b * t.sb + (int64_t)n * t.sn + (int64_t)h * t.sh;
 }

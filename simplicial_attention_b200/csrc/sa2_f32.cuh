@@ -42,7 +42,8 @@ template <int D> inline int fwd(const KernelParams &kp, int *status, int sms, cu
     const int tiles = (kp.n + ROWS - 1) / ROWS;
     int ce = simt::cluster_size((int64_t)tiles * kp.hq, kp.w2, 2, sms);
     if (ce == 8 && (int64_t)tiles * kp.hq * 32 <= sms && kp.w2 >= 64 && sixteen_fit<D>()) ce = 16;
-    return simt::launch_clusters(fwd_kernel<D>, dim3(tiles * ce, kp.hq, kp.b), FWD_THREADS, fwd_smem_bytes<D>(), ce, st, kp, status) ? SA2_OK : SA2_ERR_CUDA;
+    return simt::launch_clusters(fwd_kernel<D>, dim3(tiles * ce, kp.hq, kp.b), FWD_THREADS, fwd_smem_bytes<D>(), ce, st, kp, status) &&
+                   simt::launch_fwd<D>(kp, sms, st, true) ? SA2_OK : SA2_ERR_CUDA;
 }
 
 // Splits of a tile's work over CTAs: the query heads of its group (MODE_K1: pairs of one and a query unit) and the offsets.
@@ -80,7 +81,7 @@ struct Plan {
     bool tc;
     Split k1, k2;
     int tiles, round;
-    size_t slab, part2, part1;
+    size_t redo, slab, part2, part1;
 };
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 inline Plan plan(const sa2_shape &s, int whole_batch, int sms) {
@@ -94,6 +95,7 @@ inline Plan plan(const sa2_shape &s, int whole_batch, int sms) {
     const size_t one = slab + part2 + part1;
     p.tc = one <= MOST_BYTES;
     p.round = one * s.b <= ROUND_BYTES ? s.b : one > ROUND_BYTES ? 1 : (int)(ROUND_BYTES / one);
+    p.redo = align256((size_t)2 * s.b * sizeof(int));
     p.slab = align256(slab * p.round);
     p.part2 = align256(part2 * p.round);
     p.part1 = align256(part1 * p.round);
@@ -101,11 +103,11 @@ inline Plan plan(const sa2_shape &s, int whole_batch, int sms) {
 }
 inline size_t bwd_workspace_bytes(const sa2_shape &s, int whole_batch, int sms) {
     const Plan p = plan(s, whole_batch, sms);
-    return p.tc ? p.slab + p.part2 + p.part1 : 0;
+    return p.tc ? p.redo + p.slab + p.part2 + p.part1 : 0;
 }
 inline int bwd_launches(const sa2_shape &s, int whole_batch, int sms) {
     const Plan p = plan(s, whole_batch, sms);
-    return p.tc ? 1 + 3 * ((s.b + p.round - 1) / p.round) : 2;
+    return p.tc ? 2 + 3 * ((s.b + p.round - 1) / p.round) : 2;
 }
 
 template <int D, int MODE> inline int bwd_launch(const BwdParams &P, int rows, cudaStream_t st) {
@@ -114,9 +116,11 @@ template <int D, int MODE> inline int bwd_launch(const BwdParams &P, int rows, c
     bwd_kernel<D, MODE><<<dim3((rows + ROWS - 1) / ROWS * P.nsplit, P.kp.hk, P.kp.b), BwdCfg<MODE>::THREADS, bwd_smem_bytes<D, MODE>(), st>>>(P);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
-template <int D> inline int bwd(const KernelParams &all, const Plan &p, char *extra, int *status, cudaStream_t st, int phases) {
+template <int D> inline int bwd(const KernelParams &all, const Plan &p, char *extra, int *status, int sms, cudaStream_t st, int phases) {
     if (phases == 0) phases = SA2_BWD_ROWSUM | SA2_BWD_K1 | SA2_BWD_Q;
-    if ((phases & SA2_BWD_ROWSUM) && !simt::launch_delta<D>(all, st)) return SA2_ERR_CUDA;
+    int *redo = reinterpret_cast<int *>(extra);
+    if ((phases & SA2_BWD_ROWSUM) && !simt::launch_delta<D>(all, st, redo)) return SA2_ERR_CUDA;
+    extra += p.redo;
     const bool k1 = phases & SA2_BWD_K1, k2 = phases & SA2_BWD_Q;
     for (int b0 = 0; (k1 || k2) && b0 < all.b; b0 += p.round) {
         const KernelParams kp = tc::batch_part(all, b0, all.b - b0 < p.round ? all.b - b0 : p.round);
@@ -124,9 +128,9 @@ template <int D> inline int bwd(const KernelParams &all, const Plan &p, char *ex
         float *part1 = reinterpret_cast<float *>(extra + p.slab + p.part2);
         const int n1 = p.k1.hs * p.k1.es, n2 = p.k2.hs * p.k2.es;
         if (k1)
-            if (int e = bwd_launch<D, MODE_K1>({kp, n1, p.k1.hs, p.k1.epc, 0, part1, nullptr, status}, kp.nk1, st)) return e;
+            if (int e = bwd_launch<D, MODE_K1>({kp, n1, p.k1.hs, p.k1.epc, 0, part1, nullptr, redo + b0, status}, kp.nk1, st)) return e;
         if (k2)
-            if (int e = bwd_launch<D, MODE_K2>({kp, n2, p.k2.hs, p.k2.epc, p.tiles, part2, slab, status}, kp.nk2, st)) return e;
+            if (int e = bwd_launch<D, MODE_K2>({kp, n2, p.k2.hs, p.k2.epc, p.tiles, part2, slab, redo + all.b + b0, status}, kp.nk2, st)) return e;
         const ReduceParams R{kp, slab, part2, part1, p.tiles, p.k2.es, p.k2.epc, k2 && n2 > 1 ? n2 : 0, k1 && n1 > 1 ? n1 : 0, k2};
         const int64_t rows = (k2 ? (int64_t)kp.n * kp.hq : 0) + (R.k2_splits ? (int64_t)kp.nk2 * kp.hk : 0) + (R.k1_splits ? (int64_t)kp.nk1 * kp.hk : 0);
         if (rows == 0) continue;
@@ -136,6 +140,7 @@ template <int D> inline int bwd(const KernelParams &all, const Plan &p, char *ex
         else reduce_kernel<D, 1><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(R);
         if (cudaGetLastError() != cudaSuccess) return SA2_ERR_CUDA;
     }
+    if ((k1 || k2) && !simt::launch_bwd<D>(all, k2, k2, k1, sms, st, redo)) return SA2_ERR_CUDA;
     return SA2_OK;
 }
 

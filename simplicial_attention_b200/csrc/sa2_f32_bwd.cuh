@@ -55,6 +55,7 @@ struct BwdParams {
     int tiles;         // MODE_K2: tiles of a head
     float *part;       // partial dK, dV [nsplit][b][rows][hk][2][d], if nsplit > 1
     float *slab;       // MODE_K2: dQ [b][hq][tiles][offset splits][127 + epc][d]
+    int *redo;         // [b]: set where the scalar kernels have to do the mode's gradients
     int *status;
 };
 
@@ -143,7 +144,7 @@ __device__ __forceinline__ int bwd_first(const BwdParams &P, int which, uint32_t
         if (u >= 2 && !mbar_wait_warp(&bars[B_DONE + 2 * (1 - which) + buf], ((u >> 1) - 1) & 1, abort_flag, 0, 3)) return ERR_BWD;
         tc_fence_after();
         if (elect_one()) {
-            issue_nt<D>(tmem + 192 * buf + 96 * which + LOGITS, dM, dN + buf * (Planes<D>::bytes(UNIT) >> 4));
+            issue_nt<D, MODE == MODE_K1>(tmem + 192 * buf + 96 * which + LOGITS, dM, dN + buf * (Planes<D>::bytes(UNIT) >> 4));
             tc_commit(&bars[B_S_FULL + buf]);
             if (MODE == MODE_K2 && wk.last()) tc_commit(&bars[B_M_EMPTY + which]);
         }
@@ -172,9 +173,8 @@ __device__ __forceinline__ int bwd_second(const BwdParams &P, int which, uint32_
 template <int D, int MODE>
 __device__ __forceinline__ int bwd_compute(const BwdParams &P, int cg, uint32_t tmem, const float2 *stats, uint64_t *bars, volatile int *abort_flag) {
     const KernelParams &kp = P.kp;
-    const int r = threadIdx.x & 127, hk = blockIdx.y, b = blockIdx.z;
+    const int r = threadIdx.x & 127, b = blockIdx.z;
     const uint32_t lanes = tmem + ((uint32_t)(r & 96) << 16);
-    const float mul = kp.scale * LOG2E;
     float lse2 = 0.f, dl = 0.f;
     int u = 0;
     for (Walk<MODE> wk(P); !wk.done(); wk.next(), ++u) {
@@ -217,24 +217,11 @@ __device__ __forceinline__ int bwd_compute(const BwdParams &P, int cg, uint32_t 
                 tmem_wait_ld(s);
                 tmem_wait_ld(g);
                 const bool full = __all_sync(0xffffffffu, lo <= c0 && (int)(lo + len) >= c0 + 15);
-                auto exponent = [&](int z, float v) { return fmaf(v, REGAIN, -(MODE == MODE_K2 ? lse2 : st[c0 + z].x)); };
-                float seen = 0.f;
 #pragma unroll
                 for (int z = 0; z < 16; ++z) {
-                    float a = exponent(z, __uint_as_float(s[z]));
-                    if (!full && (uint32_t)(c0 + z - lo) > len) a = -CUDART_INF_F;
-                    seen += a;
-                    s[z] = __float_as_uint(a);
+                    const float a = __uint_as_float(s[z]) - (MODE == MODE_K2 ? lse2 : st[c0 + z].x);
+                    s[z] = __float_as_uint(!full && (uint32_t)(c0 + z - lo) > len ? -CUDART_INF_F : a);
                 }
-                if (seen != seen)                    // (masked columns are -inf, not NaN)
-                    scalar_logits<D>(s, 0xffffu, mul,
-                                     [&](int z, const float *&pq, const float *&pk2, const float *&pk1) {
-                                         const int i = MODE == MODE_K2 ? row - kp.off2 + wk.e : wk.c0 + c0 + z;
-                                         pq = row_ptr(kp.q, b, i, wk.head());
-                                         pk2 = row_ptr(kp.k2, b, i + kp.off2 - wk.e, hk);
-                                         pk1 = row_ptr(kp.k1, b, MODE == MODE_K2 ? wk.c0 + c0 + z : row, hk);
-                                     },
-                                     exponent);
 #pragma unroll
                 for (int z = 0; z < 16; z += 2) {
                     const float p0 = ex2(__uint_as_float(s[z])), p1 = ex2(__uint_as_float(s[z + 1]));
@@ -259,14 +246,14 @@ __device__ __forceinline__ int bwd_compute(const BwdParams &P, int cg, uint32_t 
 // operands is made when unit u - 2 is done and its product has been added up: both take the same slot.
 template <int D, int MODE>
 __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t tmem, uint8_t *sM, uint8_t *sN, float2 *stats, float *ring,
-                                        uint64_t *bars, volatile int *abort_flag) {
+                                        uint64_t *bars, volatile int *abort_flag, uint32_t *most) {
     constexpr int CPR = D / 8, RPP = 128 / CPR;        // chunks of a row, rows 128 threads cover at a time
     constexpr int TASKS = UNIT / RPP;
     const KernelParams &kp = P.kp;
     const int t = threadIdx.x & 127, c = t % CPR, q0 = t / CPR;
     const int hk = blockIdx.y, b = blockIdx.z;
     const uint32_t cols = tmem + ((uint32_t)(t & 96) << 16) + 384 + 64 * which;
-    const float mul = which ? 1.f : kp.scale * LOG2E;
+    const float mul = which ? 1.f : logit_factor(kp.scale, true);
     const TensorRef &tx = which ? kp.dout : kp.q, &ty = which ? kp.v2 : kp.k2, &tk = which ? kp.v1 : kp.k1;
     uint8_t *dM = sM + which * Planes<D>::bytes(ROWS), *dN = sN + which * 2 * Planes<D>::bytes(UNIT);
     uint64_t acc[D / 2], sum[MODE == MODE_K2 ? D / 2 : 1];
@@ -276,6 +263,7 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
     Walk<MODE> nxt(P), cur(P);
     const int row = nxt.r0 + t;                        // the row whose sums this thread keeps
     int sweeps = 0, folds = 0, err = 0;
+    float most_m = 0.f, most_n = 0.f;
     float held[MODE == MODE_K1 ? TASKS : 1][8];
     if (MODE == MODE_K1 && !nxt.done()) {
 #pragma unroll 1
@@ -283,7 +271,7 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
             const int rr = q0 + x * RPP, j = nxt.r0 + rr;
             float k[8];
             load8(k, row_ptr(tk, b, j < kp.nk1 ? j : 0, hk) + c * 8, j < kp.nk1);
-            put8<D>(dM, ROWS, rr, c, k);
+            put8<D>(dM, ROWS, rr, c, k, most_m);
         }
         fence_proxy_async_smem();
         mbar_arrive(&bars[B_M_FULL + which]);
@@ -381,7 +369,7 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
 #pragma unroll
                     for (int y = EARLY; y < TASKS; ++y) key_row(y);
                 }
-                put8<D>(d, UNIT, q0 + z * RPP, c, x[z]);
+                put8<D>(d, UNIT, q0 + z * RPP, c, x[z], most_n);
             }
             if (MODE == MODE_K1 && which == 0 && t < UNIT) stats[slot * UNIT + t] = stat;
             fence_proxy_async_smem();
@@ -399,7 +387,7 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
                     load8(y, row_ptr(ty, b, ok ? k : 0, hk) + c * 8, ok);
 #pragma unroll
                     for (int w = 0; w < 8; ++w) a[w] = mul * a[w] * y[w];
-                    put8<D>(dM, ROWS, rr, c, a);
+                    put8<D>(dM, ROWS, rr, c, a, most_m);
                 }
                 fence_proxy_async_smem();
                 mbar_arrive(&bars[B_M_FULL + which]);
@@ -412,13 +400,15 @@ __device__ __forceinline__ int bwd_side(const BwdParams &P, int which, uint32_t 
         }
     }
 
+    put_most(&most[which], most_m);
+    put_most(&most[2 + which], most_n);
     // the row's sums: final, or a partial for the reduction
     const bool bad = __any_sync(0xffffffffu, err != 0) || *abort_flag != 0;
     const int rows = MODE == MODE_K1 ? kp.nk1 : kp.nk2;
     if (row < rows) {
         const TensorRef &dst = MODE == MODE_K1 ? (which ? kp.dv1 : kp.dk1) : (which ? kp.dv2 : kp.dk2);
         // (A_e carries scale * log2(e); U does not carry the scale)
-        const float fac = which ? 1.f : MODE == MODE_K1 ? LN2 : kp.scale;
+        const float fac = which ? 1.f : MODE == MODE_K1 ? logit_unfactor(kp.scale, mul) : kp.scale;
         float *part = P.part + (((((size_t)(blockIdx.x % P.nsplit) * kp.b + b) * rows + row) * kp.hk + hk) * 2 + which) * D;
         const int64_t off = elem_off(dst, b, row, hk);
 #pragma unroll
@@ -454,6 +444,7 @@ __global__ void __launch_bounds__(BwdCfg<MODE>::THREADS, 1) bwd_kernel(const Bwd
     uint64_t *bars = reinterpret_cast<uint64_t *>(extra + (MODE == MODE_K2 ? ROWS * D * 4 : 2 * UNIT * 8));
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + B_BAR_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
+    uint32_t *most = tmem_holder + 2;            // [4] largest magnitudes of A_e and B_e (or K1 and V1), and of the operands on the other side
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     if (threadIdx.x == 0) {
@@ -464,6 +455,7 @@ __global__ void __launch_bounds__(BwdCfg<MODE>::THREADS, 1) bwd_kernel(const Bwd
             mbar_init(&bars[x], one ? 1u : two ? 2u : compute ? 128u * C::GROUPS : 128u);
         }
         *abort_flag = 0;
+        for (int x = 0; x < 4; ++x) most[x] = 0u;
         fence_barrier_init();
     }
     if (warp == 1) {
@@ -489,13 +481,17 @@ __global__ void __launch_bounds__(BwdCfg<MODE>::THREADS, 1) bwd_kernel(const Bwd
         err = bwd_compute<D, MODE>(P, (warp >> 2) - 1, tmem, reinterpret_cast<const float2 *>(extra), bars, abort_flag);
     } else {
         reg_alloc<C::REGS_SUM>();
-        err = bwd_side<D, MODE>(P, warp >= 8 + 4 * C::GROUPS, tmem, sM, sN, reinterpret_cast<float2 *>(extra), reinterpret_cast<float *>(extra), bars, abort_flag);
+        err = bwd_side<D, MODE>(P, warp >= 8 + 4 * C::GROUPS, tmem, sM, sN, reinterpret_cast<float2 *>(extra), reinterpret_cast<float *>(extra), bars, abort_flag,
+                                most);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
     SA2_PROF_END();
     tc_fence_before();
     __syncthreads();
+    // (dP is the product of most[1] and most[3], G is of its size)
+    if (threadIdx.x < 5 && out_of_range(threadIdx.x < 4 ? __uint_as_float(most[threadIdx.x]) : fminf(1.f, __uint_as_float(most[1])) * __uint_as_float(most[3])))
+        P.redo[blockIdx.z] = 1;
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);

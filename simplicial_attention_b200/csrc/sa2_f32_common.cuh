@@ -9,6 +9,12 @@
 // 5.9e-7 -> 4.0e-7, dv2 3.7e-7 -> 2.7e-7, lse 5.0e-8 -> 4.9e-8; b1 n128 h2 d32, full causal, dk1 7.1e-7 -> 3.5e-7.
 //
 // Operands are made by the kernels from plain fp32 rows (any 16-byte aligned strides): no tensor maps and no scratch.
+//
+// Three bf16 terms are not every fp32 value: from 3.39e38 the first one is infinite (and the second a NaN, as those of infinities
+// are), below 2^-109 the last ones leave bf16's range.  Where an operand's largest entry in a CTA is not in [2^-80, 2^60), or an output
+// is not finite, the scalar kernels, launched behind these, do the work again: the forward's row tile by row tile (LSE_REDO), the backward's
+// batch element by batch element (a flag in the workspace).  Otherwise they return at once (2 to 3 us each).  The maxima ride with the
+// splitting of the operands, four instructions to its forty; a check of every entry for itself cost 5 to 11 % of a kernel.
 #pragma once
 #include "sa2_tc_common.cuh"
 
@@ -23,10 +29,6 @@ using sa2::tc::warp_wait;
 constexpr int ROWS = 128;         // rows of a tile: TMEM lanes
 constexpr int UNIT = 64;          // columns of a logit tile
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
-// What a logit loses to the truncations of its large products, half a unit in the last place each and about one in all, is given
-// back in the logsumexp, and where the backward subtracts that.  Not where a row's reference is subtracted: the largest logit has
-// weight 1 whatever its size, and what a difference of 150 at most loses is below its own last place.
-constexpr float REGAIN = 1.f + 1.1920929e-7f;
 // error bits of the device status word
 enum { ERR_FWD = 1 << 17, ERR_BWD = 1 << 18 };
 
@@ -52,9 +54,24 @@ __device__ __forceinline__ void split2(float x0, float x1, uint32_t &h, uint32_t
     l = pack_bf16(a, b);
 }
 
-// eight channels (chunk `chunk`) of row r of an operand tile of `rows` rows
+// the largest magnitude among `most` and eight values, NaN if there is one
+__device__ __forceinline__ float most_of(float most, const float (&x)[8]) {
+#pragma unroll
+    for (int z = 0; z < 8; z += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(x[z]), "f"(x[z + 1]));
+    return most;
+}
+// is it one that three terms do not represent?  (0: nothing but zeros)
+__device__ __forceinline__ bool out_of_range(float most) { return !(most < 1.1529215e18f) || (most > 0.f && most < 8.2718061e-25f); }
+// from the threads of a warp to a word of shared memory that starts at 0 (bits of magnitudes are ordered, a NaN comes last)
+__device__ __forceinline__ void put_most(uint32_t *word, float most) {
+    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
+    if ((threadIdx.x & 31) == 0) atomicMax(word, m);
+}
+
+// eight channels (chunk `chunk`) of row r of an operand tile of `rows` rows; `most` is the operand's largest magnitude so far
 template <int D>
-__device__ __forceinline__ void put8(uint8_t *tile, int rows, int r, int chunk, const float (&x)[8]) {
+__device__ __forceinline__ void put8(uint8_t *tile, int rows, int r, int chunk, const float (&x)[8], float &most) {
+    most = most_of(most, x);
     uint32_t h[4], m[4], l[4];
 #pragma unroll
     for (int z = 0; z < 4; ++z) split2(x[2 * z], x[2 * z + 1], h[z], m[z], l[z]);
@@ -81,15 +98,17 @@ __device__ __forceinline__ const float *row_ptr(const TensorRef &t, int b, int n
 __host__ __device__ constexpr int term_a(int t) { return t == 0 ? 2 : t == 2 || t == 3 ? 1 : 0; }
 __host__ __device__ constexpr int term_b(int t) { return t == 1 ? 2 : t == 2 || t == 4 ? 1 : 0; }
 
-// d[128 x 64] = A B^T over the D channels: A [128 rows], B [64 rows], both K-major in shared memory
-template <int D>
+// d[128 x 64] = A B^T over the D channels: A [128 rows], B [64 rows], both K-major in shared memory.  SWAP: the products in the order of
+// B A^T, for a transposed tile of the same bits (which large logits need: their logsumexp is subtracted).
+template <int D, bool SWAP = false>
 __device__ __forceinline__ void issue_nt(uint32_t d, uint64_t a, uint64_t b) {
     constexpr uint32_t IDESC = idesc_bf16(128, 64, false, false);
 #pragma unroll
     for (int t = 0; t < 6; ++t)
 #pragma unroll
         for (int k = 0; k < D / 16; ++k)
-            mma_ss(d, a + (Planes<D>::at(ROWS, term_a(t)) >> 4) + 2 * k, b + (Planes<D>::at(UNIT, term_b(t)) >> 4) + 2 * k, IDESC, t + k > 0);
+            mma_ss(d, a + (Planes<D>::at(ROWS, SWAP ? term_b(t) : term_a(t)) >> 4) + 2 * k,
+                   b + (Planes<D>::at(UNIT, SWAP ? term_a(t) : term_b(t)) >> 4) + 2 * k, IDESC, t + k > 0);
 }
 // TMEM column of term `term` of the 16 keys [16 k, +16) within a region of 96 columns
 __host__ __device__ constexpr uint32_t term_col(int term, int k) { return (uint32_t)(k * 24 + term * 8); }
@@ -161,35 +180,6 @@ __device__ __forceinline__ void add_acc(uint32_t cols, uint64_t (&sum)[D / 2]) {
 __device__ __forceinline__ void column_range(int &lo, int hi, uint32_t &len) {
     if (hi < lo) { lo = 64; hi = 64; }
     len = (uint32_t)(hi - lo);
-}
-
-// Terms of infinite values, and products that leave the range on one side only, make a NaN of a logit (times log2 e) that is
-// none: the NaN among the columns `ask` of s[] are formed again, in scalar fp32 from the rows themselves.  operands(z, q, k2,
-// k1) names those of column z, finish(z, logit) the value that takes its place.
-template <int D, typename Operands, typename Finish>
-__device__ __forceinline__ void scalar_logits(uint32_t (&s)[16], uint32_t ask, float mul, Operands operands, Finish finish) {
-#pragma unroll
-    for (int z = 0; z < 16; ++z)
-        if (__uint_as_float(s[z]) == __uint_as_float(s[z])) ask &= ~(1u << z);
-    while (ask) {
-        const int z = __ffs(ask) - 1;
-        const float *q, *k2, *k1;
-        operands(z, q, k2, k1);
-        float v = 0.f;
-#pragma unroll 1
-        for (int c = 0; c < D; ++c) v = fmaf(mul * q[c] * k2[c], k1[c], v);
-        v = finish(z, v);
-#pragma unroll
-        for (int y = 0; y < 16; ++y) if (y == z) s[y] = __float_as_uint(v);
-        ask &= ask - 1;
-    }
-}
-// bits of the columns [c0, c0 + 16) that lie in [lo, lo + len]
-__device__ __forceinline__ uint32_t column_mask(int c0, int lo, uint32_t len) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int z = 0; z < 16; ++z) m |= (uint32_t)(c0 + z - lo) <= len ? 1u << z : 0u;
-    return m;
 }
 
 }  // namespace f32

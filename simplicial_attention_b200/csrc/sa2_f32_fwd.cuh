@@ -109,11 +109,12 @@ __device__ __forceinline__ int fwd_issue(const FwdGeom &g, int x, uint32_t tmem,
 // builders: K1 / V1 units, and A_e of both groups at the start of a pair of sweeps
 template <int D>
 __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &g, uint8_t *sA, uint8_t *sK, uint8_t *sV, uint64_t *bars,
-                                         volatile int *abort_flag) {
+                                         volatile int *abort_flag, uint32_t *most) {
     constexpr int CPR = D / 8, RPP = 128 / CPR;          // chunks of a row, rows the builders cover at a time
     const int t = threadIdx.x & 127, c = t % CPR, r0 = t / CPR;
     const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
-    const float mul = kp.scale * LOG2E;
+    const float mul = logit_factor(kp.scale, true);
+    float most_a = 0.f, most_k = 0.f, most_v = 0.f;
     int u = 0;
     for (int pp = 0; pp < g.npairs; ++pp) {
         for (int w = 0; w < g.nunits; ++w, ++u) {
@@ -132,8 +133,8 @@ __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &
                 if (u >= 2 && !warp_wait(&bars[F_KV_EMPTY + slot], ((u >> 1) - 1) & 1, abort_flag, 1)) return ERR_FWD;
 #pragma unroll
                 for (int y = 0; y < N; ++y) {
-                    put8<D>(dk, UNIT, r0 + y * RPP, c, k[y]);
-                    put8<D>(dv, UNIT, r0 + y * RPP, c, v[y]);
+                    put8<D>(dk, UNIT, r0 + y * RPP, c, k[y], most_k);
+                    put8<D>(dv, UNIT, r0 + y * RPP, c, v[y], most_v);
                 }
             }
             fence_proxy_async_smem();
@@ -158,7 +159,7 @@ __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &
                     for (int y = 0; y < 4; ++y) {
 #pragma unroll
                         for (int z = 0; z < 8; ++z) q[y][z] = mul * q[y][z] * k2[y][z];
-                        put8<D>(da, ROWS, r0 + (y0 + y) * RPP, c, q[y]);
+                        put8<D>(da, ROWS, r0 + (y0 + y) * RPP, c, q[y], most_a);
                     }
                 }
                 fence_proxy_async_smem();
@@ -166,6 +167,9 @@ __device__ __forceinline__ int fwd_build(const KernelParams &kp, const FwdGeom &
             }
         }
     }
+    put_most(&most[0], most_a);
+    put_most(&most[1], most_k);
+    put_most(&most[2], most_v);
     return 0;
 }
 
@@ -179,7 +183,6 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
     const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
     const int i = g.i0 + r;
     const bool row_ok = i < kp.n;
-    const float mul = kp.scale * LOG2E;
     uint64_t ws[D / 2];
 #pragma unroll
     for (int z = 0; z < D / 2; ++z) ws[z] = 0;
@@ -266,16 +269,9 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
                     const bool full = __all_sync(0xffffffffu, lo <= c0 && (int)(lo + len) >= c0 + 15);
                     float sum = full ? probs(true) : probs(false);
                     if (__any_sync(0xffffffffu, !(sum <= 65536.f))) {
-                        // a reference moves (always at a row's first keys), or a logit is NaN or +inf
+                        // a reference moves (always at a row's first keys)
                         tmem_ld16(region + LOGITS + c0, s);
                         tmem_wait_ld(s);
-                        scalar_logits<D>(s, column_mask(c0, lo, len), mul,
-                                         [&](int z, const float *&pq, const float *&pk2, const float *&pk1) {
-                                             pq = row_ptr(kp.q, b, i, h);
-                                             pk2 = row_ptr(kp.k2, b, k, hk);
-                                             pk1 = row_ptr(kp.k1, b, j0 + c0 + z, hk);
-                                         },
-                                         [](int, float v) { return v; });
                         float mx = -CUDART_INF_F;
 #pragma unroll
                         for (int z = 0; z < 16; ++z)
@@ -313,11 +309,7 @@ __device__ __forceinline__ int fwd_softmax(const KernelParams &kp, const FwdGeom
                             }
                             tmem_wait_st();
                         }
-                        // (no reference yet, and none here: logits of -inf weigh nothing, and only NaN stays NaN)
-                        const float keep = ref;
-                        if (!(ref > -CUDART_INF_F)) ref = 0.f;
                         sum = probs(false);
-                        ref = keep;
                     }
                     l += sum;
                 }
@@ -347,6 +339,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
     uint64_t *bars = reinterpret_cast<uint64_t *>(sV + 2 * Planes<D>::bytes(UNIT));
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + F_BAR_COUNT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
+    uint32_t *most = tmem_holder + 2;                             // [3] largest magnitudes of A_e, K1, V1
+    int *redo = reinterpret_cast<int *>(tmem_holder + 5);         // the tile is left to the scalar kernel
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     if (threadIdx.x == 0) {
@@ -356,6 +350,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
             mbar_init(&bars[x], one ? 1u : two ? 2u : 128u);
         }
         *abort_flag = 0;
+        *redo = 0;
+        most[0] = most[1] = most[2] = 0u;
         fence_barrier_init();
     }
     if (warp == 0) {
@@ -392,11 +388,14 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
         tc_fence_before();
         __syncthreads();                  // no product reads the operands any more
         float *row = part + (x * ROWS + r) * LD;
+        float top = fabsf(l);
 #pragma unroll
         for (int c = 0; c < D; c += 32) {
             uint32_t t[32];
             tmem_ld32(o + c, t);
             tmem_wait_ld(t);
+#pragma unroll
+            for (int z = 0; z < 32; z += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(top) : "f"(__uint_as_float(t[z])), "f"(__uint_as_float(t[z + 1])));
 #pragma unroll
             for (int z = 0; z < 32; z += 4)
                 *reinterpret_cast<float4 *>(row + c + z) =
@@ -404,13 +403,15 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
                         : !any ? make_float4(0.f, 0.f, 0.f, 0.f)
                                : make_float4(__uint_as_float(t[z]), __uint_as_float(t[z + 1]), __uint_as_float(t[z + 2]), __uint_as_float(t[z + 3]));
         }
+        if (any && !bad && !(top <= CUDART_MAX_NORMAL_F)) *redo = 1;
         stats[(x * 2) * ROWS + r] = bad ? 0.f : ref;
         stats[(x * 2 + 1) * ROWS + r] = bad ? CUDART_NAN_F : l;
     } else {
         reg_alloc<FWD_REGS_BUILD>();
-        err = fwd_build<D>(kp, g, sA, sK, sV, bars, abort_flag);
+        err = fwd_build<D>(kp, g, sA, sK, sV, bars, abort_flag, most);
         tc_fence_before();
         __syncthreads();
+        if ((threadIdx.x & 127) < 3 && out_of_range(__uint_as_float(most[threadIdx.x & 127]))) *redo = 1;
     }
     if (err) atomicOr(status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
@@ -421,11 +422,18 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
     for (int idx = threadIdx.x; idx < rows * (D / 4); idx += FWD_THREADS) {
         const int r = (int)cl.block_rank() * rows + idx / (D / 4), c = (idx % (D / 4)) * 4, i = g.i0 + r;
         if (i >= kp.n) continue;
+        float *lse = kp.lse + ((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i;
+        bool again = false;
+        for (int q = 0; q < ce; ++q) again |= *cl.map_shared_rank(redo, q) != 0;
+        if (again) {
+            if (c == 0) *lse = __uint_as_float(LSE_REDO);
+            continue;
+        }
         float M = -CUDART_INF_F, L = 0.f, v[4] = {0.f, 0.f, 0.f, 0.f};
         for (int q = 0; q < 2 * ce; ++q) M = fmaxf(M, cl.map_shared_rank(stats, q >> 1)[(q & 1) * 2 * ROWS + r]);
         for (int q = 0; q < 2 * ce; ++q) {
             const float *st = cl.map_shared_rank(stats, q >> 1) + (q & 1) * 2 * ROWS;
-            // (a group without a reference has at most NaN to say)
+            // (a group without a reference says nothing, or NaN where a wait ran out)
             if (!(st[r] > -CUDART_INF_F) && st[ROWS + r] == 0.f) continue;
             const float f = st[r] > -CUDART_INF_F ? ex2(st[r] - M) : 1.f;
             const float4 p = *reinterpret_cast<const float4 *>(cl.map_shared_rank(part, q >> 1) + ((q & 1) * ROWS + r) * LD + c);
@@ -436,7 +444,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) fwd_kernel(const KernelParams 
 #pragma unroll
         for (int z = 0; z < 4; ++z) v[z] *= inv;
         store_vec<4>(kp.out.p, elem_off(kp.out, blockIdx.z, i, blockIdx.y) + c, false, v);
-        if (c == 0) kp.lse[((int64_t)blockIdx.z * kp.hq + blockIdx.y) * kp.n + i] = M * REGAIN * LN2 + __logf(L);
+        if (c == 0) *lse = M * LN2 + __logf(L);
     }
     cl.sync();               // no CTA leaves while its shared memory is read
     if (warp == 0) {

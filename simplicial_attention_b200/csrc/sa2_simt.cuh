@@ -236,7 +236,7 @@ __device__ __forceinline__ void cluster_rank(int &ce, int &rank) {
 // Row-owned tiles: forward, dQ, or dK2/dV2.  `tile`: row tile, `h_in`: query head (forward, dQ) or key/value head.
 // ---------------------------------------------------------------------------
 template <int D, int MODE>
-__device__ __forceinline__ void row_tile(const KernelParams &p, float *smem, int tile, int h_in, int bi) {
+__device__ __forceinline__ void row_tile(const KernelParams &p, float *smem, int tile, int h_in, int bi, bool redo) {
     namespace cg = cooperative_groups;
     using C = Cfg<D>;
     constexpr int CPT = C::CPT, VEC = C::VEC, NV = C::NV, TF = C::TF;
@@ -297,7 +297,7 @@ __device__ __forceinline__ void row_tile(const KernelParams &p, float *smem, int
             fill_tile<D>(KV + TF, p.v1, bi, hk_i, j_lo, p.nk1, bf16);
             cp_commit();
             if (any) {
-                build_prod_tile<D>(As, p.q, h, p.k2, hk_i, bi, i_base, p.n, k_base, p.nk2, p.scale * LOG2E, bf16);
+                build_prod_tile<D>(As, p.q, h, p.k2, hk_i, bi, i_base, p.n, k_base, p.nk2, logit_factor(p.scale, redo), bf16);
                 if (BWD) build_prod_tile<D>(Bs, p.dout, h, p.v2, hk_i, bi, i_base, p.n, k_base, p.nk2, 1.f, bf16);
             }
             bool rvalid[4];
@@ -511,7 +511,7 @@ __device__ __forceinline__ void row_tile(const KernelParams &p, float *smem, int
 // First-key-owned tiles: dK1, dV1.  Works on transposed tiles S^T[j][i] so that the accumulators are row-owned.
 // ---------------------------------------------------------------------------
 template <int D>
-__device__ __forceinline__ void k1_tile(const KernelParams &p, float *smem, int tile, int hk_i, int bi) {
+__device__ __forceinline__ void k1_tile(const KernelParams &p, float *smem, int tile, int hk_i, int bi, bool redo) {
     namespace cg = cooperative_groups;
     using C = Cfg<D>;
     constexpr int CPT = C::CPT, TF = C::TF;
@@ -559,7 +559,7 @@ __device__ __forceinline__ void k1_tile(const KernelParams &p, float *smem, int 
                 const int k_base = i0 + p.off2 - e;
                 if (it_hi + p.off2 - e < 0) break;   // no valid second key for any row, nor for larger e
                 group_sync(grp);
-                build_prod_tile<D>(As, p.q, h, p.k2, hk_i, bi, i0, it_hi + 1, k_base, p.nk2, p.scale * LOG2E, bf16);
+                build_prod_tile<D>(As, p.q, h, p.k2, hk_i, bi, i0, it_hi + 1, k_base, p.nk2, logit_factor(p.scale, redo), bf16);
                 build_prod_tile<D>(Bs, p.dout, h, p.v2, hk_i, bi, i0, it_hi + 1, k_base, p.nk2, 1.f, bf16);
                 group_sync(grp);
                 float st[4][4];
@@ -597,39 +597,44 @@ __device__ __forceinline__ void k1_tile(const KernelParams &p, float *smem, int 
     put_acc<D>(smem + grp * 2 * TF + TF, dv, ty, tx);
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
-    reduce_store<D>(smem, 2, p.dk1, bi, hk_i, j0, p.nk1, LN2, gbf16);       // A carries scale * log2(e)
+    reduce_store<D>(smem, 2, p.dk1, bi, hk_i, j0, p.nk1, redo ? logit_unfactor(p.scale, logit_factor(p.scale, true)) : LN2, gbf16);
     reduce_store<D>(smem + TF, 2, p.dv1, bi, hk_i, j0, p.nk1, 1.f, gbf16);
     cl.sync();
 }
 
-// grid: clusters of CTAs along x; forward (tile, query head, batch)
+// grid: clusters of CTAs along x; forward (tile, query head, batch).  redo: only the tiles whose rows hold LSE_REDO.
 template <int D>
-__global__ void __launch_bounds__(Cfg<D>::THREADS) fwd_kernel(const KernelParams p) {
+__global__ void __launch_bounds__(Cfg<D>::THREADS) fwd_kernel(const KernelParams p, const bool redo) {
     extern __shared__ __align__(16) float smem[];
     const int ce = (int)cooperative_groups::this_cluster().num_blocks();
-    row_tile<D, MODE_FWD>(p, smem, blockIdx.x / ce, blockIdx.y, blockIdx.z);
+    if (redo && __float_as_uint(p.lse[((int64_t)blockIdx.z * p.hq + blockIdx.y) * p.n + blockIdx.x / ce * TILE]) != LSE_REDO) return;
+    row_tile<D, MODE_FWD>(p, smem, blockIdx.x / ce, blockIdx.y, blockIdx.z, redo);
 }
 
 // All three gradients: x / cluster size counts the row tiles of dQ, then of dK2/dV2, then of dK1/dV1 (nq, nk2t, nk1t
-// of them, already multiplied by their heads), y is the batch.
+// of them, already multiplied by their heads), y is the batch.  redo: only the batch elements that it holds a non-zero for, one array
+// for dK1/dV1 and one behind it for the others.
 struct BwdTiles { int q, k2, k1; };
 template <int D>
-__global__ void __launch_bounds__(Cfg<D>::THREADS) bwd_kernel(const KernelParams p, const BwdTiles n) {
+__global__ void __launch_bounds__(Cfg<D>::THREADS) bwd_kernel(const KernelParams p, const BwdTiles n, const int *redo) {
     extern __shared__ __align__(16) float smem[];
     const int ce = (int)cooperative_groups::this_cluster().num_blocks();
     int x = blockIdx.x / ce;
+    if (redo && !redo[(x >= n.k2 && x < n.k2 + n.k1 ? 0 : p.b) + blockIdx.y]) return;
     // the longest tiles first
-    if (x < n.k2) { row_tile<D, MODE_BWD_K2>(p, smem, x / p.hk, x % p.hk, blockIdx.y); return; }
+    if (x < n.k2) { row_tile<D, MODE_BWD_K2>(p, smem, x / p.hk, x % p.hk, blockIdx.y, redo != nullptr); return; }
     x -= n.k2;
-    if (x < n.k1) { k1_tile<D>(p, smem, x / p.hk, x % p.hk, blockIdx.y); return; }
+    if (x < n.k1) { k1_tile<D>(p, smem, x / p.hk, x % p.hk, blockIdx.y, redo != nullptr); return; }
     x -= n.k1;
-    row_tile<D, MODE_BWD_Q>(p, smem, x / p.hq, x % p.hq, blockIdx.y);
+    row_tile<D, MODE_BWD_Q>(p, smem, x / p.hq, x % p.hq, blockIdx.y, redo != nullptr);
 }
 
-// D_i = sum_c O_ic dO_ic: D / 8 lanes per (b, i, h) row, eight channels each
+// D_i = sum_c O_ic dO_ic: D / 8 lanes per (b, i, h) row, eight channels each.  redo (or null): [2][b] flags to clear.
 template <int D>
-__global__ void __launch_bounds__(256) delta_kernel(const KernelParams p) {
+__global__ void __launch_bounds__(256) delta_kernel(const KernelParams p, int *redo) {
     constexpr int LPR = D / 8;
+    static_assert(LPR >= 2, "a thread at least for each flag");
+    if (redo && (int64_t)blockIdx.x * 256 + threadIdx.x < 2LL * p.b) redo[blockIdx.x * 256 + threadIdx.x] = 0;
     const int64_t rows = (int64_t)p.b * p.n * p.hq;
     const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / LPR;
     const int c = (threadIdx.x % LPR) * 8;
@@ -676,25 +681,25 @@ inline bool launch_clusters(K kernel, dim3 grid, int threads, size_t smem, int c
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
 }
 
-template <int D> inline bool launch_delta(const KernelParams &p, cudaStream_t st) {
+template <int D> inline bool launch_delta(const KernelParams &p, cudaStream_t st, int *redo = nullptr) {
     const int64_t threads = (int64_t)p.b * p.n * p.hq * (D / 8);
-    delta_kernel<D><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(p);
+    delta_kernel<D><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(p, redo);
     return cudaGetLastError() == cudaSuccess;
 }
-template <int D> inline bool launch_fwd(const KernelParams &p, int sms, cudaStream_t st) {
+template <int D> inline bool launch_fwd(const KernelParams &p, int sms, cudaStream_t st, bool redo = false) {
     using C = Cfg<D>;
     const int tiles = (p.n + TILE - 1) / TILE, ce = cluster_size((int64_t)tiles * p.hq, p.w2, C::NG, sms);
-    return launch_clusters(fwd_kernel<D>, dim3(tiles * ce, p.hq, p.b), C::THREADS, C::smem(false), ce, st, p);
+    return launch_clusters(fwd_kernel<D>, dim3(tiles * ce, p.hq, p.b), C::THREADS, C::smem(false), ce, st, p, redo);
 }
 // dq / dk2, dv2 / dk1, dv1, those asked for, in one launch
-template <int D> inline bool launch_bwd(const KernelParams &p, bool q, bool k2, bool k1, int sms, cudaStream_t st) {
+template <int D> inline bool launch_bwd(const KernelParams &p, bool q, bool k2, bool k1, int sms, cudaStream_t st, const int *redo = nullptr) {
     using C = Cfg<D>;
     auto tiles = [](int rows) { return (rows + TILE - 1) / TILE; };
     const BwdTiles n{q ? tiles(p.n) * p.hq : 0, k2 ? tiles(p.nk2) * p.hk : 0, k1 ? tiles(p.nk1) * p.hk : 0};
     // (from the whole backward's tiles, so that a part launched alone gives the same bits)
     const int64_t all = (int64_t)tiles(p.n) * p.hq + (int64_t)(tiles(p.nk2) + tiles(p.nk1)) * p.hk;
     const int ce = cluster_size(all, p.w2, C::NG, sms);
-    return launch_clusters(bwd_kernel<D>, dim3((unsigned)(n.q + n.k2 + n.k1) * ce, p.b), C::THREADS, C::smem(true), ce, st, p, n);
+    return launch_clusters(bwd_kernel<D>, dim3((unsigned)(n.q + n.k2 + n.k1) * ce, p.b), C::THREADS, C::smem(true), ce, st, p, n, redo);
 }
 
 }  // namespace simt

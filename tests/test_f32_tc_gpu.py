@@ -84,6 +84,69 @@ def test_infinite_keys_weigh_nothing(d):
     assert (out[rows] - want[rows]).norm() <= 2 * REL * want[rows].norm()
 
 
+def _same(x, want):
+    """The same NaN and infinities, and finite values within the error of either kernel."""
+    assert torch.equal(x.isnan(), want.isnan())
+    assert torch.equal(x.isinf(), want.isinf()) and torch.equal(x[x.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    assert (x[fine].double() - want[fine].double()).norm() <= 2 * REL * want[fine].double().norm()
+
+
+INF = float("inf")
+ONE = [(t, v) for t in range(6) for v in (INF, -INF, float("nan"), 3.395e38, 1e-39)]
+
+
+@pytest.mark.parametrize("d", [32, 64])
+@pytest.mark.parametrize("which,value", ONE, ids=lambda x: str(x))
+def test_values_that_three_terms_are_not(which, value, d):
+    """One entry that is not finite, rounds to an infinite bf16 or is below its range: outputs and gradients are those of the scalar
+    kernels, also in the rows and heads that do not see it, and the other batch element's do not move."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    ins = [torch.randn(2, 300, 2, d, device="cuda", generator=g) for _ in range(6)]
+    plain = sa.sa2_forward(*ins[:5], 64, 9)
+    before = (*plain, *sa.sa2_backward(*ins[:5], *plain, ins[5], 64, 9))
+    ins[which][1, 70, 1, 5] = value
+    res = []
+    for kernel in ("auto", "simt"):
+        out, lse = sa.sa2_forward(*ins[:5], 64, 9, kernel=kernel)
+        res.append((out, lse, *sa.sa2_backward(*ins[:5], out, lse, ins[5], 64, 9, kernel=kernel)))
+    assert sa.device_status() == 0
+    # (a logit of 1e38 is known to 1e31: the backward, which subtracts its logsumexp, has no answer to compare)
+    compared = 2 if which < 3 and value == 3.395e38 else 7
+    for x, want, was in list(zip(*res, before))[:compared]:
+        _same(x, want)
+        assert torch.equal(x[0], was[0])
+
+
+@pytest.mark.parametrize("factors", [(1, 1, 1, 1e-36, 1, 1), (1, 1, 1, 1, 1, 1e-36), (1e-18, 1e36, 1e-18, 1, 1, 1), (1e-20, 1, 1e-15, 1, 1, 1),
+                                     (1, 1, 1, 1e30, 1, 1), (1, 1, 1, 1, 1, 1e30)], ids=str)
+def test_tiny_and_large_operands_keep_their_bits(factors):
+    """Operands whose second and third terms would leave bf16's range, and sums that would leave fp32's."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    ins = [f * torch.randn(1, 200, 2, 64, device="cuda", generator=g) for f in factors]
+    res = []
+    for kernel in ("auto", "simt"):
+        out, lse = sa.sa2_forward(*ins[:5], 100, 4, kernel=kernel)
+        res.append((out, lse, *sa.sa2_backward(*ins[:5], out, lse, ins[5], 100, 4, kernel=kernel)))
+    assert sa.device_status() == 0
+    for x, want in zip(*res):
+        _same(x, want)
+
+
+def test_parts_of_a_backward_do_odd_values_too():
+    """The row sums clear the marks, either part of the backward does what it has marked."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    ins = [torch.randn(2, 200, 2, 64, device="cuda", generator=g) for _ in range(6)]
+    ins[4][1, 50, 0, 3] = INF
+    out, lse = sa.sa2_forward(*ins[:5], 100, 4)
+    whole = sa.sa2_backward(*ins[:5], out, lse, ins[5], 100, 4)
+    call = sa.BackwardCall(*ins[:5], out, lse, ins[5], 100, 4)
+    for phase in (_lib.BWD_ROWSUM, _lib.BWD_K1, _lib.BWD_Q):
+        call.launch(phase)
+    for x, want in zip(call.grads, whole):
+        assert torch.equal(x.nan_to_num(7.), want.nan_to_num(7.)) and torch.equal(x.isnan(), want.isnan())
+
+
 def test_scratch_rounds():
     """A batch whose scratch passes the limit of a round goes through it in several; an element alone does in one."""
     b, n = 16, 700
