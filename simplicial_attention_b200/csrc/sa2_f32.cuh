@@ -46,37 +46,49 @@ template <int D> inline int fwd(const KernelParams &kp, int *status, int sms, cu
                    simt::launch_fwd<D>(kp, sms, st, true) ? SA2_OK : SA2_ERR_CUDA;
 }
 
+// Scratch after the D vector, for `round` batch elements at a time: an element that alone needs more than MOST runs on the scalar
+// kernels, which need none (long second windows: the dQ slabs grow with n * w2).
+constexpr size_t ROUND_BYTES = (size_t)256 << 20, MOST_BYTES = (size_t)1 << 30;
+
 // Splits of a tile's work over CTAs: the query heads of its group (MODE_K1: pairs of one and a query unit) and the offsets.
 // A unit takes ~4500 cycles, a CTA ~10000 of set-up and its results, a sweep of MODE_K2 ~2500 for its operands and its fold.
-// Partials are written and read again at ~2000 bytes a cycle.  `rows` and `slab_rows`: rows of D floats a CTA leaves.
+// Scratch is written and read again at ~2000 bytes a cycle: `part`, the bytes of one partial result, for every split (none if there is
+// one), and MODE_K2's dQ slabs of 127 + epc rows, `row` bytes over all tiles and query heads, for every range of offsets.
+// Splits whose scratch does not fit `room` are not looked at, except none: ranges of one or two offsets cost the slab of a whole tile each,
+// and with groups of query heads that is most of the traffic.  (By the cost alone b1 n14406 hq16 hk2 d64 w507/31 took 31 ranges and 1.75 GB.)
 struct Split { int hs, es, epc; };
-inline Split split(int64_t ctas, int heads, int w2, double per_offset, double bytes, int batch, int sms) {
+inline size_t split_bytes(const Split &s, size_t part, size_t row) {
+    return (s.hs * s.es > 1 ? s.hs * s.es * part : 0) + s.es * (size_t)(ROWS - 1 + s.epc) * row;
+}
+inline Split split(int64_t ctas, int heads, int w2, double per_offset, size_t part, size_t row, size_t room, int batch, int sms) {
     Split best{1, 1, w2};
     double best_cost = 0.;
     for (int hs = 1; hs <= heads && hs <= 16; ++hs)
         for (int es = 1; es <= w2 && hs * es <= 64; ++es) {
-            const int epc = (w2 + es - 1) / es;
-            if ((w2 + epc - 1) / epc != es) continue;
-            const double one = 10000. + (double)((heads + hs - 1) / hs) * epc * per_offset;
-            const double cost = tc::split_cost(ctas * hs * es, one, batch, sms) + (hs * es > 1 ? 3000. + bytes * hs * es * batch / 2000. : 0.);
-            if (best_cost == 0. || cost < tc::SPLIT_GAIN * best_cost) { best = Split{hs, es, epc}; best_cost = cost; }
+            const Split s{hs, es, (w2 + es - 1) / es};
+            if ((w2 + s.epc - 1) / s.epc != es) continue;
+            const size_t bytes = split_bytes(s, part, row);
+            if (bytes > room && hs * es > 1) continue;
+            const double one = 10000. + (double)((heads + hs - 1) / hs) * s.epc * per_offset;
+            const double cost = tc::split_cost(ctas * hs * es, one, batch, sms) + (hs * es > 1 ? 3000. : 0.) + (double)bytes * batch / 2000.;
+            if (best_cost == 0. || cost < tc::SPLIT_GAIN * best_cost) { best = s; best_cost = cost; }
         }
     return best;
 }
+inline int k2_tiles(const sa2_shape &s) { return (s.n + s.off2 + ROWS - 1) / ROWS; }
+inline size_t part_bytes(const sa2_shape &s, int64_t rows) { return (size_t)rows * s.hk * 2 * s.d * sizeof(float); }
+inline size_t slab_row_bytes(const sa2_shape &s) { return (size_t)s.hq * k2_tiles(s) * s.d * sizeof(float); }
 inline Split split_k2(const sa2_shape &s, int batch, int sms) {
-    const int64_t tiles = (int64_t)((s.n + s.off2 + ROWS - 1) / ROWS) * s.hk;
     const int keys = s.w1 + ROWS - 1 < s.n + s.off1 ? s.w1 + ROWS - 1 : s.n + s.off1;
-    return split(tiles, s.hq / s.hk, s.w2, 2500. + (keys + UNIT - 1) / UNIT * 4500., (double)tiles * ROWS * s.d * 12, batch, sms);
+    return split((int64_t)k2_tiles(s) * s.hk, s.hq / s.hk, s.w2, 2500. + (keys + UNIT - 1) / UNIT * 4500., part_bytes(s, (int64_t)k2_tiles(s) * ROWS),
+                 slab_row_bytes(s), ROUND_BYTES, batch, sms);
 }
-inline Split split_k1(const sa2_shape &s, int batch, int sms) {
+inline Split split_k1(const sa2_shape &s, size_t room, int batch, int sms) {
     const int64_t tiles = (int64_t)((s.n + s.off1 + ROWS - 1) / ROWS) * s.hk;
     const int rows = s.w1 + ROWS - 1 < s.n ? s.w1 + ROWS - 1 : s.n;
-    return split(tiles, s.hq / s.hk * ((rows + UNIT - 1) / UNIT), s.w2, 4500., (double)tiles * ROWS * s.d * 8, batch, sms);
+    return split(tiles, s.hq / s.hk * ((rows + UNIT - 1) / UNIT), s.w2, 4500., part_bytes(s, tiles / s.hk * ROWS), 0, room, batch, sms);
 }
 
-// Scratch after the D vector, for `round` batch elements at a time: an element that alone needs more than MOST runs on the scalar
-// kernels, which need none (long second windows: the dQ slabs grow with n * w2).
-constexpr size_t ROUND_BYTES = (size_t)256 << 20, MOST_BYTES = (size_t)1 << 30;
 struct Plan {
     bool tc;
     Split k1, k2;
@@ -86,13 +98,11 @@ struct Plan {
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 inline Plan plan(const sa2_shape &s, int whole_batch, int sms) {
     Plan p;
-    p.k1 = split_k1(s, whole_batch, sms);
     p.k2 = split_k2(s, whole_batch, sms);
-    p.tiles = (s.n + s.off2 + ROWS - 1) / ROWS;
-    const size_t row = (size_t)s.d * sizeof(float), n1 = p.k1.hs * p.k1.es, n2 = p.k2.hs * p.k2.es;
-    const size_t slab = (size_t)s.hq * p.tiles * p.k2.es * (ROWS - 1 + p.k2.epc) * row;
-    const size_t part2 = n2 > 1 ? n2 * (s.n + s.off2) * s.hk * 2 * row : 0, part1 = n1 > 1 ? n1 * (s.n + s.off1) * s.hk * 2 * row : 0;
-    const size_t one = slab + part2 + part1;
+    const size_t slab = split_bytes(p.k2, 0, slab_row_bytes(s)), part2 = split_bytes(p.k2, part_bytes(s, s.n + s.off2), 0);
+    p.k1 = split_k1(s, slab + part2 < ROUND_BYTES ? ROUND_BYTES - slab - part2 : 0, whole_batch, sms);
+    p.tiles = k2_tiles(s);
+    const size_t part1 = split_bytes(p.k1, part_bytes(s, s.n + s.off1), 0), one = slab + part2 + part1;
     p.tc = one <= MOST_BYTES;
     p.round = one * s.b <= ROUND_BYTES ? s.b : one > ROUND_BYTES ? 1 : (int)(ROUND_BYTES / one);
     p.redo = align256((size_t)2 * s.b * sizeof(int));
