@@ -32,26 +32,42 @@ inline bool bwd_supported(const sa2_shape &s) { return s.dtype == SA2_BF16; }
 inline bool bwd_scale_ok(const sa2_shape &s) { return fabsf(s.scale) >= 1e-20f; }
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // CTAs sharing one query tile in the dQ/dK2/dV2 kernel: splits of the window (head dim 128 walks it in one CTA) times
-// splits of the offsets, an even number each.  A CTA costs ~12000 cycles of set-up, loads, slab and its share of the reduction, a 64-key
-// unit of a sweep ~1100 (1700 at head dim 128).
-struct BqSplit { int nu, ups, tsplit, esplit, epc; };
-inline BqSplit bq_split(const sa2_shape &s, const BwdCaller &call, int max_units, int sms) {
+// splits of the offsets (an even number each with pairs).  Head dim 128: a CTA costs ~12000 cycles of set-up, loads, slab and its share of
+// the reduction, a 64-key unit of a sweep ~1700.  Up to head dim 64, fitted to b4 n3000 h8 with first windows of 64 to 512 rows and to b64 of
+// 64 to 512 rows: set-up of a CTA, a sweep and its units, and the least a sweep takes.  Over these 78 shapes the tile that the model
+// picks takes at most 3.4 % longer than the better one; pairs take up to 27 % longer in short windows, 128 rows up to 70 % in long ones.
+struct BqCost { double setup, sweep, unit, least; };
+inline BqCost bq_cost(int d, bool split, bool pair) {
+    if (d == 32) return pair ? BqCost{11000., 2750., 980., 5000.} : BqCost{13400., 2320., 1010., 0.};
+    if (split) return pair ? BqCost{13500., 5000., 1130., 7000.} : BqCost{19500., 3900., 1250., 0.};
+    return pair ? BqCost{13500., 3572., 745., 5300.} : BqCost{19500., 2900., 790., 0.};
+}
+struct BqSplit { bool pair; int nu, ups, tsplit, esplit, epc; double cost; };
+inline BqSplit bq_split(const sa2_shape &s, const BwdCaller &call, bool split, bool pair, int sms) {
     BqSplit r;
-    const int have = (s.n + s.off1 + 63) / 64;
-    r.nu = (s.w1 + BQ_ROWS - 1 + 63) / 64;
+    r.pair = pair;
+    const int rows = bq_rows(pair), step = bq_step(pair), have = (s.n + s.off1 + 63) / 64;
+    const int max_units = split && s.d == 64 ? (pair ? BqCfg<64, true, true>::MAX_UNITS : BqCfg<64, true, false>::MAX_UNITS)
+                                             : (pair ? BqCfg<64, false, true>::MAX_UNITS : BqCfg<64, false, false>::MAX_UNITS);
+    r.nu = (s.w1 + rows - 1 + 63) / 64;
     r.tsplit = s.d == 128 ? 1 : (r.nu + max_units - 1) / max_units;
     r.ups = (r.nu + r.tsplit - 1) / r.tsplit;
     const int per = (std::min(r.nu, have) + r.tsplit - 1) / r.tsplit;
-    const int64_t ctas = (int64_t)((s.n + BQ_ROWS - 1) / BQ_ROWS) * s.hq * r.tsplit;
-    const int pairs = (s.w2 + 1) / 2;
-    const int least = (pairs + BQ_MAX_EPC / 2 - 1) / (BQ_MAX_EPC / 2);
-    double best_cost = 0.;
+    const int64_t ctas = (int64_t)((s.n + rows - 1) / rows) * s.hq * r.tsplit;
+    const int sweeps = (s.w2 + step - 1) / step, most = BQ_MAX_EPC / step, least = (sweeps + most - 1) / most;
+    // What a sweep costs: half of the columns in partly masked units come for nothing (warps without a valid column skip them).
+    const double rows_all = s.n, ramp = std::min(std::max(s.w1 - s.off1, 0), s.n);
+    const double seen = (ramp * (2. * s.off1 + ramp + 1.) / 2. + (rows_all - ramp) * s.w1) / rows_all;           // keys of a row, on average
+    const double units = (seen / 64. + rows / 128. * (1. - ramp / (2. * rows_all))) / r.tsplit;
+    const BqCost c = bq_cost(s.d, split, pair);
+    const double sweep = s.d == 128 ? per * 1700. : std::max(c.least, c.sweep + units * c.unit), setup = s.d == 128 ? 12000. : c.setup;
+    r.cost = 0.;
     r.esplit = least;
-    for (int es = least; es <= pairs && (es <= 16 || es == least); ++es) {
-        const double cost = split_cost(ctas * es, 12000. + (pairs + es - 1) / es * (per * (s.d == 128 ? 1700. : 1100.)), call.batch, sms);
-        if (best_cost == 0. || cost < SPLIT_GAIN * best_cost) { r.esplit = es; best_cost = cost; }
+    for (int es = least; es <= sweeps && (es <= 16 || es == least); ++es) {
+        const double cost = split_cost(ctas * es, setup + (sweeps + es - 1) / es * sweep, call.batch, sms);
+        if (r.cost == 0. || cost < SPLIT_GAIN * r.cost) { r.esplit = es; r.cost = cost; }
     }
-    r.epc = (pairs + r.esplit - 1) / r.esplit * 2;
+    r.epc = (sweeps + r.esplit - 1) / r.esplit * step;
     r.esplit = (s.w2 + r.epc - 1) / r.epc;
     return r;
 }
@@ -73,14 +89,18 @@ inline BqPlan bq_plan(const sa2_shape &s, const BwdCaller &call, int sms) {
     BqPlan p;
     const bool longer = call.w2 > BQ_FINE_W2;
     p.split = s.d == 32 || longer;
-    p.sp = bq_split(s, call, p.split && s.d == 64 ? BqCfg<64, true>::MAX_UNITS : BqCfg<64, false>::MAX_UNITS, sms);
+    p.sp = bq_split(s, call, p.split, true, sms);
+    if (s.d <= 64) {
+        const BqSplit rows = bq_split(s, call, p.split, false, sms);
+        if (rows.cost < p.sp.cost) p.sp = rows;
+    }
     p.round = s.b;
     p.tc = true;
     if (longer) {
         sa2_shape one = s;
         one.b = 1;
         const int ns = p.sp.tsplit * p.sp.esplit;
-        const size_t bytes = bq_part_dq_bytes(one, ns) + bq_part_k2_bytes(one, ns, p.sp.epc);
+        const size_t bytes = bq_part_dq_bytes(one, ns) + bq_part_k2_bytes(one, bq_rows(p.sp.pair), ns, p.sp.epc);
         p.tc = bytes <= BQ_MOST_BYTES;
         if (bytes * s.b > BQ_ROUND_BYTES) p.round = bytes > BQ_ROUND_BYTES ? 1 : (int)(BQ_ROUND_BYTES / bytes);
     }
@@ -102,7 +122,7 @@ inline BwdScratch bwd_scratch(const sa2_shape &s, const BwdCaller &call, const B
         r.b = q.round;
         const int ns = q.sp.tsplit * q.sp.esplit;
         b.dq = align256(bq_part_dq_bytes(r, ns));
-        b.k2 = align256(bq_part_k2_bytes(r, ns, q.sp.epc));
+        b.k2 = align256(bq_part_k2_bytes(r, bq_rows(q.sp.pair), ns, q.sp.epc));
     }
     return b;
 }
@@ -212,30 +232,32 @@ inline bool bwd_addressable(const KernelParams &kp) {
 }
 
 // dQ, dK2, dV2: query-tile-owned tcgen05 kernel
-template <int D, bool SPLIT>
+template <int D, bool SPLIT, bool PAIR>
 inline int bwd_q_launch(const BqParams &Q, cudaStream_t st) {
-    using C = BqCfg<D, SPLIT>;
+    using C = BqCfg<D, SPLIT, PAIR>;
     const KernelParams &kp = Q.kp;
     const size_t smem = C::SMEM;
-    if (cudaFuncSetAttribute(bwd_q_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(bwd_q_kernel<D, SPLIT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SA2_ERR_CUDA;
     CUtensorMap mapK, mapV;             // units of 64 rows
     constexpr int ROWS = 64;
     if (!tmap::make_rows_map(&mapK, kp.k1.p, kp.b, kp.nk1, kp.hk, D, kp.k1.sb, kp.k1.sn, kp.k1.sh, ROWS) ||
         !tmap::make_rows_map(&mapV, kp.v1.p, kp.b, kp.nk1, kp.hk, D, kp.v1.sb, kp.v1.sn, kp.v1.sh, ROWS))
         return SA2_ERR_CUDA;
-    bwd_q_kernel<D, SPLIT><<<dim3(Q.nqt * Q.nsplit, kp.hq, kp.b), C::THREADS, smem, st>>>(mapK, mapV, Q);
+    bwd_q_kernel<D, SPLIT, PAIR><<<dim3(Q.nqt * Q.nsplit, kp.hq, kp.b), C::THREADS, smem, st>>>(mapK, mapV, Q);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
 // deterministic reduction of the partials
 template <int D>
-inline int bwd_reduce_launch(const BqParams &Q, cudaStream_t st) {
+inline int bwd_reduce_launch(const BqParams &Q, bool pair, cudaStream_t st) {
     const KernelParams &kp = Q.kp;
     const int64_t rows = (Q.reduce_q ? (Q.nsplit == 1 ? 0 : (int64_t)kp.b * kp.n * kp.hq) + (int64_t)kp.b * kp.nk2 * kp.hk : 0) +
                          (Q.reduce_k1 ? (int64_t)kp.b * kp.nk1 * kp.hk : 0);
     if (rows == 0) return SA2_OK;
-    bwd_q_reduce_kernel<D><<<(unsigned)((rows * (D / 4) + 255) / 256), 256, 0, st>>>(Q);
+    const unsigned blocks = (unsigned)((rows * (D / 4) + 255) / 256);
+    if (D == 128 || pair) bwd_q_reduce_kernel<D, true><<<blocks, 256, 0, st>>>(Q);
+    else bwd_q_reduce_kernel<D, D == 128><<<blocks, 256, 0, st>>>(Q);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 
@@ -296,7 +318,7 @@ inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, const BwdCalle
     Q.nsplit = plan.sp.tsplit * plan.sp.esplit;
     Q.epc = plan.sp.epc;
     Q.units_per_split = plan.sp.ups;
-    Q.nqt = (kp.n + BQ_ROWS - 1) / BQ_ROWS;
+    Q.nqt = (kp.n + bq_rows(plan.sp.pair) - 1) / bq_rows(plan.sp.pair);
     Q.part_dq = reinterpret_cast<float *>(extra);
     Q.part_k2 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + room.dq);
     float *part_k1 = reinterpret_cast<float *>(reinterpret_cast<char *>(extra) + room.dq + room.k2);
@@ -315,16 +337,19 @@ inline int bwd_launch(const KernelParams &kp, const sa2_shape &s, const BwdCalle
     const bool one_round = plan.round >= kp.b;
     for (int b0 = 0; q_tc && b0 < kp.b; b0 += plan.round) {
         Q.kp = batch_part(kp, b0, kp.b - b0 < plan.round ? kp.b - b0 : plan.round);
-        if (int e = D == 32 || plan.split ? bwd_q_launch<D, true>(Q, st) : bwd_q_launch<D, D == 32>(Q, st)) return e;
+        const bool pair = D == 128 || plan.sp.pair;       // (tiles of 128 rows are not built for head dim 128)
+        if (int e = D == 32 || plan.split ? (pair ? bwd_q_launch<D, true, true>(Q, st) : bwd_q_launch<D, true, D == 128>(Q, st))
+                                          : (pair ? bwd_q_launch<D, D == 32, true>(Q, st) : bwd_q_launch<D, D == 32, D == 128>(Q, st)))
+            return e;
         Q.reduce_q = 1;
         Q.reduce_k1 = one_round && k1_parts;
-        if (int e = bwd_reduce_launch<D>(Q, st)) return e;
+        if (int e = bwd_reduce_launch<D>(Q, plan.sp.pair, st)) return e;
     }
     if (!k1_parts || (q_tc && one_round)) return SA2_OK;
     Q.kp = kp;
     Q.reduce_q = 0;
     Q.reduce_k1 = 1;
-    return bwd_reduce_launch<D>(Q, st);
+    return bwd_reduce_launch<D>(Q, plan.sp.pair, st);
 }
 
 inline int bwd(const KernelParams &kp, const sa2_shape &s, const BwdCaller &call, void *extra, cudaStream_t st, int phases = 0) {

@@ -2,21 +2,23 @@
 // fp32 accumulation in TMEM, head dims 32, 64 and 128), plus the reduction of its
 // partials and of those of dK1 / dV1.
 //
-// A tile is 128 (query row, offset) pairs of one (batch, query head): 64 query rows i times two consecutive offsets
-// e = i - k; rows 0-63 have the even offset of a "sweep", rows 64-127 the odd one.  A CTA owns the 64 query rows and a
+// A tile is 128 (query row, offset) pairs of one (batch, query head), e = i - k being the offset.  PAIR: 64 query rows i times two
+// consecutive offsets; rows 0-63 have the even offset of a "sweep", rows 64-127 the odd one.  Otherwise 128 query rows and one offset
+// a sweep (head dims 32 and 64; bq_plan chooses).  A CTA owns the query rows and a
 // subset ("split") of their K1/V1 units and offsets.  Because the backward recomputes probabilities from the saved
 // logsumexp, the splits of one query tile are independent; each writes fp32 partials to scratch and a small second kernel
 // adds them in a fixed order (splits, then the query heads of a kv group), so results are reproducible.
-// Head dims 32 and 64: a split keeps its (at most nine) 64-key units resident in shared memory; a window of up to 513 keys is
-// one split.  Head dim 128: the units stream through a three-slot TMA ring (32 KB per slot), once per sweep, from L2: a slot is
+// Head dims 32 and 64: a split keeps its 64-key units (at most nine, or six beside 128 rows) resident in shared memory; with pairs a
+// window of up to 513 keys is one split.  Head dim 128: the units stream through a three-slot TMA ring (32 KB per slot), once per sweep, from L2: a slot is
 // refilled when the U / W products of its unit are done.  The offsets may be split as well (bq_split).
 //
-// Why pairs: the window of 64 rows is w1 + 63 keys where that of 128 rows is w1 + 127 (9 units against 10 at w1 = 512), it
+// Why pairs: in long windows the window of 64 rows is w1 + 63 keys where that of 128 rows is w1 + 127 (9 units against 10 at w1 = 512), it
 // fits the shared memory of one CTA, so that dQ needs no partials, and a sweep's operands and its fold are shared by 9 units
-// where a window in two splits shared them by 4 and 6.
+// where a window in two splits shared them by 4 and 6.  Why not always: a sweep takes at least what its fold takes, ~5300 cycles with
+// pairs (their fold has a hand-over in the middle) against ~2900 and ~790 for each unit with 128 rows.
 //
 // SPLIT (head dim 32, and second windows above 56 rows: see bq_plan) keeps A_e, B_e, P and G as a bf16 value and a bf16 rest
-// each, with twice the products; the rests cost two units at head dim 64 and two of the three ring slots at 128.
+// each, with twice the products; the rests cost two units at head dim 64 (of nine or six) and two of the three ring slots at 128.
 //
 // Per sweep the fold groups form A[r] = q_i * k2_{i-e} and B[r] = dO_i * v2_{i-e}; per 64-key
 // unit the tensor cores compute
@@ -28,10 +30,10 @@
 // At the end of a sweep the row owners fold U, W into
 //     dQ_i += U * k2_{i-e}                             (registers; the two rows of a query are added at the end)
 //     dK2_{i-e} += U * q_i,  dV2_{i-e} += W * dO_i     (fp32 rows in shared memory)
-// Both rows (i, e) and (i + 1, e + 1) add to row i - e of the shared accumulators: the even rows of the sweep do their first half
-// of the channels while the odd rows do the second one, a barrier, and then the other halves, so that each value has one writer
-// at a time and a fixed order.  65 rows are live in a sweep and the next one starts two rows further down: the accumulators are
-// a ring of 65 rows, and whoever adds to a row last writes it to the slab in global memory instead.
+// With pairs both rows (i, e) and (i + 1, e + 1) add to row i - e of the shared accumulators: the even rows of the sweep do their first
+// half of the channels while the odd rows do the second one, a barrier, and then the other halves, so that each value has one writer
+// at a time and a fixed order.  65 rows are live in a sweep and the next one starts two rows further down (without pairs 128, and one):
+// the accumulators are a ring of as many rows, and whoever adds to a row last writes it to the slab in global memory instead.
 //
 // Warps (640 threads): 0 issuer of U (after loading the units; head dim 128: of U and W); 1 TMEM owner and issuer of
 // S; 2 issuer of dP; 3 issuer of W (head dim 128: TMA producer of the ring); 4-7 and 8-11 two compute groups, each
@@ -51,12 +53,13 @@
 // are bound by the folds, ~6000 cycles a sweep.  At head dim 128 the fold of U has no registers for half a row: its ~18000 cycles a
 // sweep (operands from L2, half a row per lane) hold up the next sweep's U / W.
 // Measured, this kernel and its reduction, against tiles of 128 rows and one offset with the window in two splits (head dim 64) or two
-// CTAs of 64 channels each that formed S and dP twice (head dim 128): b4 n4096 h8 d64 w512/32 1.64 -> 1.38 ms, b1 n3001 h8 w1024/16
-// 320 -> 288 us, b4 n1966 h4 w105/26 211 -> 207, b1 n300 h4 w300/32 56 -> 44, b1 n16384 h16 d128 w512/32 8.74 -> 7.61 ms.
-// SPLIT: b4 n3000 h8 d32 w512/32 1.39 -> 1.10 ms, d64 w512/64 4.49 -> 4.19, d128 w512/64 16.7 -> 10.3 (both chunks of a group's columns read
-// before either is written, as it was at first, does not fit 80 registers: 2.12, 5.59 and 12.2).  Slower than the tiles of 128 rows: windows
-// of one to three units up to head dim 64, b16 n128 h8 94 -> 113 us, b4 n3000 h8 d64 w64/9 231 -> 254 us, w76/10 252 -> 267: a sweep
-// takes what its fold takes, and the fold of two offsets has a barrier more.
+// CTAs of 64 channels each that formed S and dP twice (head dim 128): b4 n4096 h8 d64 w512/32 1.66 -> 1.40 ms, b1 n3001 h8 w1024/16
+// 293 -> 285 us, b4 n1966 h4 w105/26 188 -> 182, b1 n300 h4 w300/32 38 -> 27, b1 n16384 h16 d128 w512/32 8.74 -> 7.4 ms.
+// SPLIT: b4 n3000 h8 d32 w512/32 1.42 -> 1.13 ms, d64 w512/64 4.53 -> 4.24, d128 w512/64 16.7 -> 10.4 (both chunks of a group's columns read
+// before either is written, as it was at first, does not fit 80 registers: 2.12, 5.59 and 12.2).
+// Tiles of 128 rows, this kernel's (in brackets: an earlier one's, with all accumulator rows and no staged second keys) against pairs: b128
+// n128 h8 d64 w512/32 583 (644) / 802 us, b16 n128 h8 89 (100) / 113, b4 n3000 h8 d64 w64/9 217 (231) / 254, w76/10 247 (253) / 267,
+// b64 n256 hq8 hk4 725 (755) / 869, b128 n128 h8 d32 530 (543) / 675.
 // Measured and not kept (head dim 64, C = b4 n4096 above, S = b4 n1966): a row of U or W read at once, which frees the accumulators
 // sooner and leaves no registers to load ahead, C 1.35 but S 229 us; U and W read sixteen channels at a time, C 1.87; compute groups on
 // alternate units, C 1.40; 32 columns at a time with 88 registers, C 1.46; the next sixteen columns fetched ahead, C 1.74 (spills); the
@@ -68,8 +71,8 @@
 namespace sa2 {
 namespace tc {
 
-constexpr int BQ_ROWS = 64;      // query rows of a tile
-constexpr int BQ_RING = 65;      // rows of the shared accumulators
+__host__ __device__ constexpr int bq_rows(bool pair) { return pair ? 64 : 128; }      // query rows of a tile
+__host__ __device__ constexpr int bq_step(bool pair) { return pair ? 2 : 1; }         // offsets of a sweep
 constexpr int BQ_FINE_W2 = 56;   // second windows above this keep fp32 accuracy (bq_plan)
 // Most offsets of a CTA: the second keys they pair with are staged in shared memory up to head dim 64.  (The wait accounting wants
 // some of it, and a ring slot of head dim 128.)
@@ -85,8 +88,9 @@ constexpr int BQ_MAX_EPC = 56;
 // never returns, so the budgets must add up to what the block was launched with: five groups of 96 (640 threads).  Up to head dim
 // 64 the U fold takes 176 (dQ, the q row and half a row of U, 128 registers, and what two pieces need), the W fold 112; at head dim 128 the U fold 184 (dQ,
 // 128 registers, and chunks of the rest), the W fold 96.
-template <int D, bool SPLIT> struct BqCfg {
+template <int D, bool SPLIT, bool PAIR = true> struct BqCfg {
     static constexpr int THREADS = 640;
+    static constexpr int ROWS = bq_rows(PAIR), STEP = bq_step(PAIR), RING = PAIR ? 65 : 128;        // RING: rows of the shared accumulators
     static constexpr int REGS_LAUNCH = 96, REGS_ISSUE = D <= 64 ? 32 : 40, REGS_COMPUTE = 80;
     static constexpr int REGS_FOLD = D <= 64 ? 176 : 184, REGS_FOLD_W = D <= 64 ? 112 : 96;
     static_assert(REGS_COMPUTE <= REGS_LAUNCH, "the compute groups release registers");
@@ -99,7 +103,7 @@ template <int D, bool SPLIT> struct BqCfg {
     static constexpr uint32_t REST = D == 32 ? 64 : CB * BLK;    // bytes from an element of A / B to its rest
     static constexpr uint32_t TILE = CB * BLK * (SPLIT && D > 32 ? 2 : 1);        // A or B
     static constexpr uint32_t UBLK = 8192;                       // one channel block of a 64-row unit of K1 / V1
-    static constexpr int MAX_UNITS = SPLIT && D == 64 ? 7 : 9;   // resident units of a split (head dims 32, 64)
+    static constexpr int MAX_UNITS = SPLIT && D == 64 ? (PAIR ? 7 : 4) : (PAIR ? 9 : 6);   // resident units of a split (head dims 32, 64)
     static constexpr int NSLOT = SPLIT ? 1 : BQ_ACCOUNTED ? 2 : 3;                  // ring slots (head dim 128)
     static constexpr uint32_t KV_BYTES = D <= 64 ? MAX_UNITS * UBLK : NSLOT * 2 * UBLK;
     static constexpr int NBUF = D <= 64 ? 3 : 2;                 // S / dP (P / G) buffers in TMEM
@@ -108,11 +112,11 @@ template <int D, bool SPLIT> struct BqCfg {
     // and the offsets inside a row are compile-time constants; head dim 128 has no room for the padding and XORs the
     // 16-byte chunk with the row instead.
     static constexpr int ACC_STRIDE = D == 128 ? 128 : D + 4;
-    static constexpr uint32_t ACC_BYTES = BQ_RING * ACC_STRIDE * 4;
+    static constexpr uint32_t ACC_BYTES = RING * ACC_STRIDE * 4;
     // Up to head dim 64 the second keys of the tile, which the U fold reads a row per lane: that costs the L1 32 cycles an
     // instruction from global memory and four from here.
     static constexpr bool STAGE_Y = D <= 64;
-    static constexpr uint32_t STAGE_BYTES = STAGE_Y ? (BQ_ROWS - 1 + BQ_MAX_EPC) * 128 : 0;
+    static constexpr uint32_t STAGE_BYTES = STAGE_Y ? (ROWS - 1 + BQ_MAX_EPC) * 128 : 0;
     static constexpr size_t SMEM = 1024 + 2 * (size_t)KV_BYTES + 2 * TILE + 2 * ACC_BYTES + STAGE_BYTES + 256;
     static_assert(SMEM <= 227 * 1024, "shared memory of an SM");
 };
@@ -143,10 +147,10 @@ struct BqParams {
     int nsplit;         // CTAs sharing one query tile: tsplit x (offset splits)
     int tsplit;         // splits of the K1/V1 window
     int units_per_split;
-    int epc;            // second-key offsets of a CTA, an even number: split s takes [epc * (s / tsplit), +epc)
+    int epc;            // second-key offsets of a CTA, a multiple of those of a sweep: split s takes [epc * (s / tsplit), +epc)
     int nqt;            // query tiles
     float *part_dq;     // [nsplit][b][n][hq][d]
-    float *part_k2;     // [b][hq][nqt][nsplit][2][63 + epc][d]   (dK2 slab, then dV2 slab)
+    float *part_k2;     // [b][hq][nqt][nsplit][2][rows of a tile - 1 + epc][d]   (dK2 slab, then dV2 slab)
     int *status;
     // what the reduction adds up: dQ and dK2/dV2, and the dK1/dV1 partials of ce CTAs per key tile
     const float *part_k1;
@@ -155,33 +159,35 @@ struct BqParams {
 
 // (a query tile with one split writes dQ itself and needs no partials)
 inline size_t bq_part_dq_bytes(const sa2_shape &s, int nsplit) { return nsplit == 1 ? 0 : (size_t)nsplit * s.b * s.n * s.hq * s.d * sizeof(float); }
-inline size_t bq_part_k2_bytes(const sa2_shape &s, int nsplit, int epc) {
-    const size_t nqt = (s.n + BQ_ROWS - 1) / BQ_ROWS;
-    return (size_t)s.b * s.hq * nqt * nsplit * 2 * (BQ_ROWS - 1 + epc) * s.d * sizeof(float);
+inline size_t bq_part_k2_bytes(const sa2_shape &s, int rows, int nsplit, int epc) {
+    const size_t nqt = (s.n + rows - 1) / rows;
+    return (size_t)s.b * s.hq * nqt * nsplit * 2 * (rows - 1 + epc) * s.d * sizeof(float);
 }
 
 struct BqGeom {
     int qt, split;               // query tile and split of this CTA
     int i0;
-    int e0, e1;                  // its offsets; sweep t: e0 + 2 t and the one behind it
+    int e0, e1;                  // its offsets; sweep t: e0 + 2 t and the one behind it (or e0 + t)
     int nsweeps;
     int ubase;                   // first-key row of the CTA's unit 0; unit x covers rows ubase + 64 x ... + 63
     int nunits;                  // 64-key units the CTA visits in every sweep
     int total;                   // nunits * nsweeps
 };
 
+template <bool PAIR>
 __device__ __forceinline__ BqGeom bq_geom(const BqParams &P, int qt, int split) {
     BqGeom g;
     const KernelParams &kp = P.kp;
     g.qt = qt;
     g.split = split;
-    g.i0 = qt * BQ_ROWS;
-    const int i_last = min(g.i0 + BQ_ROWS - 1, kp.n - 1);
+    constexpr int ROWS = bq_rows(PAIR), STEP = bq_step(PAIR);
+    g.i0 = qt * ROWS;
+    const int i_last = min(g.i0 + ROWS - 1, kp.n - 1);
     g.e0 = (split / P.tsplit) * P.epc;
     g.e1 = min(min(kp.w2, g.e0 + P.epc), i_last + kp.off2 + 1);
-    g.nsweeps = max(0, (g.e1 - g.e0 + 1) / 2);
+    g.nsweeps = max(0, (g.e1 - g.e0 + STEP - 1) / STEP);
     const int ts = split % P.tsplit;
-    const int base = g.i0 + kp.off1 + BQ_ROWS - 64 * P.nu;       // unit x of the window covers rows base + 64 x ...
+    const int base = g.i0 + kp.off1 + ROWS - 64 * P.nu;       // unit x of the window covers rows base + 64 x ...
     const int first = base >= 0 ? 0 : min(P.nu - 1, (-base) / 64);
     const int begin = max(first, ts * P.units_per_split), end = min(P.nu, (ts + 1) * P.units_per_split);
     g.ubase = base + 64 * begin;
@@ -341,14 +347,14 @@ __device__ __forceinline__ void pg_pair(float p0, float p1, uint32_t dp0, uint32
     }
 }
 // Group cg forms columns [32 cg, +32) of every unit, which halves the time between S / dP and P / G.
-template <int D, bool SPLIT>
+template <int D, bool SPLIT, bool PAIR>
 __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, int cg, uint32_t tmem, uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D, SPLIT>;
+    using C = BqCfg<D, SPLIT, PAIR>;
     const KernelParams &kp = P.kp;
     const int r = threadIdx.x & 127;                  // row of the tile = TMEM lane
     const uint32_t lane_addr = tmem + ((uint32_t)(r & 96) << 16);
     const int h = blockIdx.y, b = blockIdx.z;
-    const int i = g.i0 + (r & (BQ_ROWS - 1));
+    const int i = g.i0 + (r & (C::ROWS - 1));
     const bool row_ok = i < kp.n;
     const float c = P.c;
     float lse2 = 0.f, dl = 0.f;
@@ -359,9 +365,9 @@ __device__ __forceinline__ int bq_compute(const BqParams &P, const BqGeom &g, in
     }
     const uint64_t c2 = f2_pack(c, c), nlse2 = f2_pack(-lse2, -lse2), ndl2 = f2_pack(-dl, -dl);
     const int c0 = 32 * cg;                           // the group's first column
-    int e = g.e0 + (r >> 6), w = 0;
+    int e = g.e0 + (PAIR ? r >> 6 : 0), w = 0;
     for (int u = 0; u < g.total; ++u, ++w) {
-        if (w == g.nunits) { w = 0; e += 2; }
+        if (w == g.nunits) { w = 0; e += C::STEP; }
         const bool sweep_ok = row_ok && e < g.e1 && i + kp.off2 - e >= 0;
         const int buf = u % C::NBUF, use = u / C::NBUF;
         const int j0 = g.ubase + 64 * w;
@@ -441,17 +447,18 @@ __device__ __forceinline__ uint4 mul_bf16x8(const uint4 &x, const uint4 &y) {
 // an odd row is channel x ^ (D / 2) of the tensors.
 // Up to head dim 64 the row of q (dO) stays in registers.  At head dim 128 an operand row is fetched by sixteen lanes, 16 bytes each, so
 // that a load of the warp is whole rows: with a row per lane every load touched 32 cache lines, ~8000 cycles of L1 a sweep.
-template <int D, bool SPLIT, int WHICH>
+template <int D, bool SPLIT, bool PAIR, int WHICH>
 __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc, uint8_t *sOp, uint8_t *sStage, float *slab, uint64_t (&dq)[D / 2],
                                             uint64_t *bars, volatile int *abort_flag) {
-    using C = BqCfg<D, SPLIT>;
+    using C = BqCfg<D, SPLIT, PAIR>;
+    constexpr int ROWS = C::ROWS, STEP = C::STEP;
     const KernelParams &kp = P.kp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = threadIdx.x & 127, odd = __shfl_sync(0xffffffffu, r >> 6, 0);     // row of the tile = TMEM lane
+    const int r = threadIdx.x & 127, odd = PAIR ? __shfl_sync(0xffffffffu, r >> 6, 0) : 0;     // row of the tile = TMEM lane
     const int rot = odd ? D / 2 : 0;
     const uint32_t cols = tmem + ((uint32_t)(r & 96) << 16) + (WHICH ? C::W0 : C::U0);
     const int h = blockIdx.y, b = blockIdx.z, hk = h / kp.g;
-    const int ir = r & (BQ_ROWS - 1), i = g.i0 + ir;
+    const int ir = r & (ROWS - 1), i = g.i0 + ir;
     const bool row_ok = i < kp.n;
     constexpr int NC = D / 8;                         // 16-byte chunks of a row
     constexpr bool HELD = D <= 64;                    // the row of q (dO) stays in registers
@@ -470,18 +477,18 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     }
     constexpr bool STAGE_Y = C::STAGE_Y && WHICH == 0;
     const int top_row = ir + P.epc - 1 - odd;         // row of the slab, and of the staged second keys, in sweep 0
-    if constexpr (STAGE_Y) {
+    auto stage = [&]() {
         const int k0 = g.i0 + kp.off2 - g.e0 - (P.epc - 1);
-        for (int x = r; x < (BQ_ROWS - 1 + P.epc) * NC; x += 128) {
+        for (int x = r; x < (ROWS - 1 + P.epc) * NC; x += 128) {
             const int row = x / NC, cc = x % NC, k = k0 + row;
             *reinterpret_cast<uint4 *>(sStage + sw128_offset(row, cc)) =
                 k >= 0 && k < kp.nk2 ? __ldg(reinterpret_cast<const uint4 *>(ybase + (int64_t)k * ty.sn) + cc) : zero;
         }
         bq_fold_sync(WHICH);
-    }
-    auto ystaged = [&](int t, int cc) { return *reinterpret_cast<const uint4 *>(sStage + sw128_offset(top_row - 2 * t, cc)); };
+    };
+    auto ystaged = [&](int t, int cc) { return *reinterpret_cast<const uint4 *>(sStage + sw128_offset(top_row - STEP * t, cc)); };
     auto yrow = [&](int t, bool &ok) {
-        const int e = g.e0 + 2 * t + odd, kk = i + kp.off2 - e;
+        const int e = g.e0 + STEP * t + odd, kk = i + kp.off2 - e;
         ok = row_ok && e < g.e1 && kk >= 0;
         return reinterpret_cast<const uint4 *>(ybase + (int64_t)(ok ? kk : 0) * ty.sn);
     };
@@ -491,7 +498,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         uint4 y[NC];
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc) {
-            if constexpr (STAGE_Y) y[cc] = ystaged(t, cc ^ (rot / 8));
+            if (STAGE_Y && t > 0) y[cc] = ystaged(t, cc ^ (rot / 8));
             else y[cc] = ok ? __ldg(py + (cc ^ (rot / 8))) : zero;
         }
         if constexpr (!SPLIT) {
@@ -516,13 +523,13 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     constexpr int LPR = D / 8, RPI = 32 / LPR, LOADS = 32 / RPI;            // lanes per row, rows per load, loads of a warp
     const int brow = (warp & 3) * 32 + lane / LPR, bcc = lane % LPR;
     auto build_rows = [&](int t) -> bool {
-        const int e = g.e0 + 2 * t + odd;
+        const int e = g.e0 + STEP * t + odd;
         const __nv_bfloat16 *bx = reinterpret_cast<const __nv_bfloat16 *>(tx.p) + elem_off(tx, b, 0, h) + bcc * 8, *by = ybase + bcc * 8;
         // loads [x0, x0 + m): operands of a row and, with SPLIT, what their product is not
         auto rows = [&](int x0, int m, uint4 *p, uint4 *rest) {
 #pragma unroll
             for (int x = 0; x < m; ++x) {
-                const int ii = g.i0 + ((brow + (x0 + x) * RPI) & (BQ_ROWS - 1)), kk = ii + kp.off2 - e;
+                const int ii = g.i0 + ((brow + (x0 + x) * RPI) & (ROWS - 1)), kk = ii + kp.off2 - e;
                 const bool ok = ii < kp.n && e < g.e1 && kk >= 0;
                 p[x] = ok ? __ldg(reinterpret_cast<const uint4 *>(bx + (int64_t)ii * tx.sn)) : zero;
                 rest[x] = ok ? __ldg(reinterpret_cast<const uint4 *>(by + (int64_t)kk * ty.sn)) : zero;
@@ -571,7 +578,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         return true;
     };
 
-    int slab_row = top_row, place = slab_row % BQ_RING;     // row of the slab and of the ring, of the next sweep
+    int slab_row = top_row, place = slab_row % C::RING;     // row of the slab and of the ring, of the next sweep
     auto drain = [&](int t) -> bool {
         bool ok;
         const uint4 *py = yrow(t, ok);
@@ -593,7 +600,7 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
         };
         // every row of the ring belonged to other threads in the last sweep
         if (t >= 1 && !warp_wait(&bars[BQ_FOLD_SYNC + WHICH], (t - 1) & 1, abort_flag, 2)) return false;
-        const bool sole = r == BQ_ROWS - 1 || r == BQ_ROWS;           // the first row of the sweep and the last have one writer
+        const bool sole = r == 63 || r == 64;           // (pairs) the first row of the sweep and the last have one writer
         const bool end = t == g.nsweeps - 1;
         float *row = acc + place * C::ACC_STRIDE;
         ulonglong2 *gone = reinterpret_cast<ulonglong2 *>(slab + (size_t)slab_row * D);
@@ -603,13 +610,13 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
 #pragma unroll
         for (int c0 = 0; c0 < NC; c0 += GROUP) {
             const bool second = c0 >= NC / 2;
-            if (c0 == NC / 2) {
+            if (PAIR && c0 == NC / 2) {
                 mbar_arrive(&bars[BQ_FOLD_MID + WHICH]);
                 if (!warp_wait(&bars[BQ_FOLD_MID + WHICH], t & 1, abort_flag, 4)) return false;
             }
             // nothing has been added to the row (here: to these channels) yet / nothing will be after this
-            const bool fresh = second ? r == BQ_ROWS || (t == 0 && r == BQ_ROWS - 1) : t == 0 || r == 0 || r == BQ_ROWS || r == BQ_ROWS + 1;
-            const bool out = second ? end || r == BQ_ROWS - 2 || r == BQ_ROWS - 1 || r == 127 : r == BQ_ROWS - 1 || (end && sole);
+            const bool fresh = !PAIR ? t == 0 || r == 0 : second ? r == 64 || (t == 0 && r == 63) : t == 0 || r == 0 || r == 64 || r == 65;
+            const bool out = !PAIR ? end || r == 127 : second ? end || r == 62 || r == 63 || r == 127 : r == 63 || (end && sole);
             uint4 xx[GROUP], yy[GROUP];
             ulonglong2 a[GROUP][2];
             auto place_of = [&](int g, int half) {          // first 16-byte piece of the eight floats, and the one behind it
@@ -654,13 +661,16 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
             }
         }
         mbar_arrive(&bars[BQ_FOLD_SYNC + WHICH]);
-        slab_row -= 2;
-        place -= 2;
-        if (place < 0) place += BQ_RING;
+        slab_row -= STEP;
+        place -= STEP;
+        if (place < 0) place += C::RING;
         return true;
     };
     const int nv = g.total > 0 ? g.nsweeps : 0;       // a split whose units all lie before the sequence start has no work
+    // (the first operands come from global memory: the tensor cores wait for them, and not for the staged copy)
     if (nv > 0 && !build(0)) return ERR_BQ_COMPUTE;
+    if constexpr (STAGE_Y)
+        if (nv > 0) stage();
     for (int t = 0; t < nv; ++t) {
         // the operands of the next sweep first: the tensor cores wait for them, U / W of this sweep arrive later
         if ((t + 1 < nv && !build(t + 1)) || !drain(t)) return ERR_BQ_COMPUTE;
@@ -668,24 +678,25 @@ __device__ __forceinline__ int bq_fold_body(const BqParams &P, const BqGeom &g, 
     return 0;
 }
 
-template <int D, bool SPLIT, int WHICH>
+template <int D, bool SPLIT, bool PAIR, int WHICH>
 __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint32_t tmem, float *acc, uint8_t *sOp, uint8_t *sStage, uint64_t *bars,
                                        volatile int *abort_flag) {
     const KernelParams &kp = P.kp;
-    const int r = threadIdx.x & 127, ir = r & (BQ_ROWS - 1), i = g.i0 + ir, rot = r >> 6 ? D / 2 : 0;
+    constexpr int ROWS = bq_rows(PAIR);
+    const int r = threadIdx.x & 127, ir = r & (ROWS - 1), i = g.i0 + ir, rot = PAIR && r >> 6 ? D / 2 : 0;
     const int h = blockIdx.y, b = blockIdx.z;
-    const int slab_rows = BQ_ROWS - 1 + P.epc;
+    const int slab_rows = ROWS - 1 + P.epc;
     float *slab = P.part_k2 + (((((size_t)b * kp.hq + h) * P.nqt + g.qt) * P.nsplit + g.split) * 2 + WHICH) * (size_t)(slab_rows * D);
     uint64_t dq[WHICH ? 1 : D / 2];
     int err;
-    if constexpr (WHICH == 0) err = bq_fold_body<D, SPLIT, 0>(P, g, tmem, acc, sOp, sStage, slab, dq, bars, abort_flag);
+    if constexpr (WHICH == 0) err = bq_fold_body<D, SPLIT, PAIR, 0>(P, g, tmem, acc, sOp, sStage, slab, dq, bars, abort_flag);
     else {
         uint64_t none[D / 2];
-        err = bq_fold_body<D, SPLIT, 1>(P, g, tmem, acc, sOp, sStage, slab, none, bars, abort_flag);
+        err = bq_fold_body<D, SPLIT, PAIR, 1>(P, g, tmem, acc, sOp, sStage, slab, none, bars, abort_flag);
     }
     const bool bad = err != 0 || *abort_flag != 0;     // a CTA in which a wait ran out reports NaN
     if constexpr (WHICH == 0) {
-        // The rows of the odd offsets hand their share of dQ over in shared memory: every product that reads A is done.
+        // Pairs: the rows of the odd offsets hand their share of dQ over in shared memory: every product that reads A is done.
         float *buf = reinterpret_cast<float *>(sOp) + ir * D;
         auto piece = [&](int x) { return buf + 4 * (x ^ (ir & (D / 4 - 1))); };
         if (rot) {
@@ -694,14 +705,14 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
                 *reinterpret_cast<ulonglong2 *>(piece(x ^ (D / 8))) = make_ulonglong2(dq[2 * x], dq[2 * x + 1]);
         }
         // (reached by a warp that gave up as well)
-        bq_fold_sync(0);
+        if constexpr (PAIR) bq_fold_sync(0);
         if (!rot && i < kp.n) {
             // with one split per query tile dQ is final and goes straight to the gradient, otherwise a partial for the reduction
             float *dst = P.nsplit == 1 ? nullptr : P.part_dq + ((((size_t)g.split * kp.b + b) * kp.n + i) * kp.hq + h) * D;
             const int64_t o = elem_off(kp.dq, b, i, h);
 #pragma unroll
             for (int x = 0; x < D / 4; ++x) {
-                const float4 y = *reinterpret_cast<const float4 *>(piece(x));
+                const float4 y = PAIR ? *reinterpret_cast<const float4 *>(piece(x)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 float v[4];
                 f2_unpack(dq[2 * x], v[0], v[1]);
                 f2_unpack(dq[2 * x + 1], v[2], v[3]);
@@ -718,10 +729,10 @@ __device__ __forceinline__ int bq_fold(const BqParams &P, const BqGeom &g, uint3
     return err;
 }
 
-template <int D, bool SPLIT>
-__global__ void __launch_bounds__(BqCfg<D, SPLIT>::THREADS, 1)
+template <int D, bool SPLIT, bool PAIR>
+__global__ void __launch_bounds__(BqCfg<D, SPLIT, PAIR>::THREADS, 1)
 bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const BqParams P) {
-    using C = BqCfg<D, SPLIT>;
+    using C = BqCfg<D, SPLIT, PAIR>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = align_smem(smem_raw);
     uint8_t *sK = smem;
@@ -756,7 +767,7 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_holder;
-    const BqGeom g = bq_geom(P, blockIdx.x / P.nsplit, blockIdx.x % P.nsplit);
+    const BqGeom g = bq_geom<PAIR>(P, blockIdx.x / P.nsplit, blockIdx.x % P.nsplit);
 
     int err = 0;
 #ifdef SA2_PROF
@@ -776,13 +787,13 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
         // one call site for both compute groups: they run the same instructions, which the instruction caches
         // of a scheduler then hold once (with two copies: 3.5 ms against 2.3)
         if constexpr (C::REGS_COMPUTE < C::REGS_LAUNCH) reg_dealloc<C::REGS_COMPUTE>();
-        err = bq_compute<D, SPLIT>(P, g, (warp >> 2) - 1, tmem, bars, abort_flag);
+        err = bq_compute<D, SPLIT, PAIR>(P, g, (warp >> 2) - 1, tmem, bars, abort_flag);
     } else if (warp < 16) {
         reg_alloc<C::REGS_FOLD>();
-        err = bq_fold<D, SPLIT, 0>(P, g, tmem, acc_k, sA, sStage, bars, abort_flag);
+        err = bq_fold<D, SPLIT, PAIR, 0>(P, g, tmem, acc_k, sA, sStage, bars, abort_flag);
     } else {
         if constexpr (C::REGS_FOLD_W > C::REGS_LAUNCH) reg_alloc<C::REGS_FOLD_W>();
-        err = bq_fold<D, SPLIT, 1>(P, g, tmem, acc_v, sB, sStage, bars, abort_flag);
+        err = bq_fold<D, SPLIT, PAIR, 1>(P, g, tmem, acc_v, sB, sStage, bars, abort_flag);
     }
     if (err) atomicOr(P.status, err);
     SA2_PROF_ADD(0, clock64() - prof_t0);
@@ -803,14 +814,15 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
 //   dv2[b,k,hk] =         same over slab_v
 //   dk1[b,j,hk] = scale * sum_{split of the key tile} part_k1[...], dv1 the same (two or more splits only)
 // Row k (position k - off2 in query coordinates) lies in the slab of query tile
-// T and the split of offsets [e0, e0 + epc) at slab row k - off2 - 64 T + e0 + epc - 1, for the
-// tiles where that index falls inside [0, 63 + epc) and among the rows of the sweeps that the CTA ran.
+// T of R rows and the split of offsets [e0, e0 + epc) at slab row k - off2 - R T + e0 + epc - 1, for the
+// tiles where that index falls inside [0, R - 1 + epc) and among the rows of the sweeps that the CTA ran.
 // ---------------------------------------------------------------------------
-template <int D>
+template <int D, bool PAIR>
 __global__ void bwd_q_reduce_kernel(const BqParams P) {
     constexpr int TPR = D / 4;                          // threads per row
+    constexpr int ROWS = bq_rows(PAIR);
     const KernelParams &kp = P.kp;
-    const int acc_rows = BQ_ROWS - 1 + P.epc;
+    const int acc_rows = ROWS - 1 + P.epc;
     const int64_t nq = !P.reduce_q || P.nsplit == 1 ? 0 : (int64_t)kp.b * kp.n * kp.hq * TPR;      // one split: dQ is already in place
     const int64_t nk = !P.reduce_q ? 0 : (int64_t)kp.b * kp.nk2 * kp.hk * TPR;
     const int64_t nk1 = !P.reduce_k1 ? 0 : (int64_t)kp.b * kp.nk1 * kp.hk * TPR;
@@ -842,13 +854,18 @@ __global__ void bwd_q_reduce_kernel(const BqParams P) {
         for (int hh = 0; hh < kp.g; ++hh) {
             const int h = hk * kp.g + hh;
             for (int s = 0; s < P.nsplit; ++s) {
-                // tiles T with 0 <= pos - 64 T + top < acc_rows
-                const int top = (s / P.tsplit) * P.epc + P.epc - 1;
-                const int t_hi = min(P.nqt - 1, pos + top >= 0 ? (pos + top) / BQ_ROWS : -1);
-                for (int T = pos + top < acc_rows ? 0 : (pos + top - acc_rows) / BQ_ROWS + 1; T <= t_hi; ++T) {
-                    const int row = pos - BQ_ROWS * T + top;
-                    const BqGeom g = bq_geom(P, T, s);
-                    if (g.nunits == 0 || row < P.epc - 2 * g.nsweeps) continue;
+                // tiles T with 0 <= pos - ROWS T + top < acc_rows
+                const int e0 = (s / P.tsplit) * P.epc, top = e0 + P.epc - 1;
+                const int low = P.epc - (min(kp.w2 - e0, P.epc) + bq_step(PAIR) - 1) / bq_step(PAIR) * bq_step(PAIR);      // first row there is
+                const int t_hi = min(P.nqt - 1, pos + top >= 0 ? (pos + top) / ROWS : -1);
+                for (int T = pos + top < acc_rows ? 0 : (pos + top - acc_rows) / ROWS + 1; T <= t_hi; ++T) {
+                    const int row = pos - ROWS * T + top;
+                    // (a tile that sees no start of the sequence has run all the split's sweeps, over units)
+                    if (row < low) continue;
+                    if (ROWS * T + kp.off2 < kp.w2 - 1 || ROWS * (T + 1) + kp.off1 < 64 * P.nu) {
+                        const BqGeom g = bq_geom<PAIR>(P, T, s);
+                        if (g.nunits == 0 || row < P.epc - bq_step(PAIR) * g.nsweeps) continue;
+                    }
                     const float *slab = P.part_k2 + ((((size_t)b * kp.hq + h) * P.nqt + T) * P.nsplit + s) * (size_t)(2 * acc_rows * D);
                     const float4 vk = *reinterpret_cast<const float4 *>(slab + (size_t)row * D + c4);
                     const float4 vv = *reinterpret_cast<const float4 *>(slab + (size_t)(acc_rows + row) * D + c4);

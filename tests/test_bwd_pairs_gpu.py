@@ -1,7 +1,8 @@
-"""dQ, dK2 and dV2 on tiles of 64 query rows times two offsets: lengths around a tile, odd numbers of offsets, a window of one unit
+"""dQ, dK2 and dV2 on tiles of 64 query rows times two offsets, or 128 times one: lengths around a tile, odd numbers of offsets, a window of one unit
 more than a CTA holds, ranges of offsets, halos.  Against the fp32 kernels on the same bf16 tensors."""
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 import simplicial_attention_b200 as sa
 
@@ -25,8 +26,34 @@ CASES = [
 ]
 
 
+# shapes that run on tiles of 128 rows and one offset
+ROWS = [
+    (40, 128, 8, 2, 64, 512, 5, 0),
+    (32, 100, 8, 8, 32, 100, 3, 0),
+    (12, 450, 8, 4, 64, 200, 1, 0),       # one sweep
+    (6, 700, 8, 2, 64, 64, 7, 0),
+    (20, 128, 8, 2, 64, 128, 63, 0),      # two ranges of offsets, with rests
+    (18, 200, 8, 4, 64, 60, 11, 70),      # halo rows in front
+    (18, 200, 8, 4, 32, 60, 11, 70),
+]
+
+
+@pytest.mark.parametrize("case", ROWS, ids=lambda c: "b%d_n%d_hq%d_hk%d_d%d_w%d_%d_off%d" % c)
+def test_short_windows_take_tiles_of_128_rows(case):
+    names = []
+
+    def look(call):
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            call()
+            torch.cuda.synchronize()
+        names.extend(e.key for e in p.key_averages())
+
+    test_matches_the_fp32_kernels(case, look)
+    assert any("bwd_q_kernel<" in k and "false>" in k for k in names), names
+
+
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "b%d_n%d_hq%d_hk%d_d%d_w%d_%d_off%d" % c)
-def test_matches_the_fp32_kernels(case):
+def test_matches_the_fp32_kernels(case, look=None):
     b, n, hq, hk, d, w1, w2, off = case
     g = torch.Generator(device="cuda").manual_seed(n + d)
     rand = lambda rows, h: torch.randn(b, rows, h, d, device="cuda", generator=g).to(torch.bfloat16)
@@ -34,6 +61,8 @@ def test_matches_the_fp32_kernels(case):
     out, lse = sa.sa2_forward(q, *keys, w1, w2)
     got, again = (sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="tcgen05") for _ in range(2))
     want = sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="simt")
+    if look:
+        look(lambda: sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="tcgen05"))
     assert sa.device_status() == 0
     for x, (a, r, w) in enumerate(zip(got, again, want)):
         assert torch.equal(a, r)
