@@ -1,10 +1,13 @@
 """The one-token kernel of generation (norms, cache hand-over and attention in one launch) and the projections of up to 64 rows:
-remainders of keys, offsets and heads, short and over-long caches, and the shapes that go elsewhere.  Against the same module
-called module by module."""
+remainders of keys, offsets and heads, and short caches against the same module called module by module; over-long and strided caches,
+and the shapes that the kernel takes or leaves, at its C entry against 64 bits."""
+import ctypes as C
+
 import pytest
 import torch
 
 import simplicial_attention_b200 as sa
+from simplicial_attention_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 # Results are bf16 (2^-9 each) behind two projections of bf16 operands whose rounded inputs may differ by one unit in the last place
@@ -61,3 +64,90 @@ def test_nan_key_reaches_its_head_only():
         cache[0][0][1, 30, 0, 5] = float("nan")
         out, _ = m(torch.randn(2, 1, 256, device="cuda", dtype=torch.bfloat16), cache=cache, return_cache=True)
     assert out[0].isfinite().all() and out[1].isnan().all()
+
+
+class _NormArgs(C.Structure):
+    _fields_ = [("x", C.c_void_p), ("dy", C.c_void_p), ("y", C.c_void_p), ("rstd", C.c_void_p), ("gain", C.c_void_p * 5), ("dgain", C.c_void_p * 5),
+                ("partial", C.c_void_p), ("partial_bytes", C.c_size_t), ("rows", C.c_int64), ("x_stride", C.c_int64), ("y_stride", C.c_int64),
+                ("dy_stride", C.c_int64), ("hq", C.c_int32), ("hk", C.c_int32), ("d", C.c_int32), ("x_dtype", C.c_int32), ("y_dtype", C.c_int32),
+                ("gain_dtype", C.c_int32), ("eps", C.c_float), ("stream", C.c_void_p)]
+
+
+class _Set(C.Structure):
+    _fields_ = [("cache", C.c_void_p), ("strides", _lib.Strides), ("dst", C.c_void_p), ("keep", C.c_int32)]
+
+
+def _step_attn(proj, gains, caches, hq, hk, d, w1, w2):
+    """(status, out, new caches) of sa2_step_attn; caches [k, k', v, v'], each [b][keep][hk][d]."""
+    b = proj.shape[0]
+    a = _NormArgs(x=proj.data_ptr(), rows=b, x_stride=proj.stride(0), hq=hq, hk=hk, d=d, x_dtype=_lib.SA2_BF16, y_dtype=_lib.SA2_BF16,
+                  gain_dtype=_lib.SA2_BF16, eps=1e-6, stream=torch.cuda.current_stream().cuda_stream)
+    for v in range(5):
+        a.gain[v] = gains[v].data_ptr()
+    sets, new = (_Set * 4)(), []
+    for s, c in enumerate(caches):
+        keep = c.shape[1]
+        new.append(torch.empty(b, min(keep + 1, (w2 if s & 1 else w1) - 1), hk, d, device="cuda", dtype=torch.bfloat16))
+        sets[s] = _Set(c.data_ptr(), _lib.Strides(*c.stride()[:3]), new[s].data_ptr(), keep)
+    out = torch.empty(b, hq, d, device="cuda", dtype=torch.bfloat16)
+    fn = _lib.lib().sa2_step_attn
+    fn.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_float]
+    return fn(C.byref(a), sets, out.data_ptr(), b, w1, w2, d ** -0.5), out, new
+
+
+def _step_inputs(b, hq, hk, d, keep1, keep2):
+    g = torch.Generator(device="cuda").manual_seed(hq + keep1)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    proj, gains = rand(b, d * (hq + 4 * hk)), [(1 + 0.2 * rand(d)).to(torch.bfloat16) for _ in range(5)]
+    # every cache a window of a wider tensor: other rows, heads and channels around it
+    caches = [rand(b, keep + 3, 2 * hk, d + 8)[:, 2:2 + keep, 1:1 + hk, 8:] for keep in (keep1, keep2, keep1, keep2)]
+    return proj, gains, caches
+
+
+def _step_reference(proj, gains, caches, hq, hk, d, w1, w2):
+    """Rows as the kernel rounds them, then 64 bits: (out, the five kinds of new rows)."""
+    b = proj.shape[0]
+    x = proj.float().view(b, hq + 4 * hk, d)
+    x = x * (x.square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    kv = x[:, hq:].view(b, 2, hk, 2, d)
+    rows = [x[:, :hq], kv[:, 0, :, 0], kv[:, 0, :, 1], kv[:, 1, :, 0], kv[:, 1, :, 1]]
+    q, *new = [(r * g.float()).to(torch.bfloat16) for r, g in zip(rows, gains)]
+    k1, k2, v1, v2 = [torch.cat((c, n[:, None]), 1)[:, -w:].double().repeat_interleave(hq // hk, 2)
+                      for c, n, w in zip(caches, new, (w1, w2, w1, w2))]
+    s = torch.einsum("bhc,bjhc,bkhc->bhjk", q.double(), k1, k2) * d ** -0.5
+    p = s.flatten(-2).softmax(-1).view_as(s)
+    return torch.einsum("bhjk,bjhc,bkhc->bhc", p, v1, v2), new
+
+
+ENTRY = [
+    # b, hq, hk, d, w1, w2, keep1, keep2
+    (2, 4, 2, 64, 64, 8, 90, 30),           # caches longer than the windows
+    (1, 8, 1, 64, 300, 17, 411, 16),
+    (3, 2, 2, 128, 70, 64, 69, 100),
+    (2, 3, 3, 64, 40, 33, 12, 40),          # the first one shorter, the second one longer
+    (1, 1, 1, 64, 1, 1, 5, 5),
+    (2, 2, 1, 128, 513, 32, 600, 3),
+]
+
+
+@pytest.mark.parametrize("case", ENTRY, ids=lambda c: "b%d_hq%d_hk%d_d%d_w%d_%d_keep%d_%d" % c)
+def test_entry_takes_long_and_strided_caches(case):
+    b, hq, hk, d, w1, w2, keep1, keep2 = case
+    proj, gains, caches = _step_inputs(b, hq, hk, d, keep1, keep2)
+    status, out, new = _step_attn(proj, gains, caches, hq, hk, d, w1, w2)
+    assert status == _lib.SA2_OK
+    want, rows = _step_reference(proj, gains, caches, hq, hk, d, w1, w2)
+    # only operands and result are rounded; a row's norm may differ by one unit in its last place (2^-8) in a few entries
+    assert (out.double() - want).norm() <= 2 ** -7 * want.norm()
+    for n, c, r, w in zip(new, caches, rows, (w1, w2, w1, w2)):
+        whole = torch.cat((c, r[:, None]), 1)[:, max(0, c.shape[1] + 2 - w):]
+        assert n.shape == whole.shape
+        if n.shape[1]:
+            assert torch.equal(n[:, :-1], whole[:, :-1])
+            assert ((n[:, -1].float() - whole[:, -1].float()).abs() <= 2 ** -7 * whole[:, -1].float().abs()).all()
+
+
+def test_entry_leaves_what_it_does_not_take():
+    for d, w2 in ((64, 65), (32, 8)):
+        proj, gains, caches = _step_inputs(1, 2, 1, d, 20, 20)
+        assert _step_attn(proj, gains, caches, 2, 1, d, 30, w2)[0] == 2        # SA2_ERR_UNSUPPORTED
