@@ -80,8 +80,57 @@ __host__ __device__ __forceinline__ Items items(int g, int w2) {
     return t;
 }
 
+// Second values that are infinite or 2^64 and more: a W of some of the keys times one of them can be infinite of either sign where the W of
+// all keys has one.  So the first CTA of a head, alone, forms W over all keys before it multiplies, against the maximum m and denominator l
+// that the cluster found: a warp per offset, a product at a time (0.2 ms at windows 512/32).
 template <int D>
-__global__ void __launch_bounds__(THREADS, PER_SM<D>) kernel(const Params P) {
+__device__ __noinline__ void whole_rows(const Params &P, const __nv_bfloat16 *sNew, const __nv_bfloat16 *sK2, const __nv_bfloat16 *sV2, float *scratch,
+                                        int head, float m, float l) {
+    constexpr int CH = D / 32;                           // channels of a lane
+    const Set &S1 = P.set[0], &T1 = P.set[2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, hk = blockIdx.y, b = blockIdx.z;
+    const int n1 = min(P.w1, S1.keep + 1), n2 = min(P.w2, P.set[1].keep + 1);
+    auto at = [&](const __nv_bfloat16 *s, int row, int c) { return __bfloat162float(s[sw<D>(row, c >> 3) + (c & 7)]); };
+    float acc[CH];
+#pragma unroll
+    for (int z = 0; z < CH; ++z) acc[z] = 0.f;
+    for (int r = warp; r < n2; r += WARPS) {
+        float a[CH], w[CH];
+#pragma unroll
+        for (int z = 0; z < CH; ++z) {
+            const int c = lane * CH + z;
+            a[z] = __bfloat162float(sNew[head * D + c]) * at(sK2, r, c);
+            w[z] = 0.f;
+        }
+        for (int j = S1.keep + 1 - n1; j <= S1.keep; ++j) {
+            const bool fresh = j == S1.keep;
+            const __nv_bfloat16 *k = fresh ? sNew + P.g * D : S1.cache + b * S1.sb + (int64_t)j * S1.sn + hk * S1.sh;
+            const __nv_bfloat16 *v = fresh ? sNew + (P.g + 2) * D : T1.cache + b * T1.sb + (int64_t)j * T1.sn + hk * T1.sh;
+            float s = 0.f;
+#pragma unroll
+            for (int z = 0; z < CH; ++z) s = fmaf(a[z], __bfloat162float(k[lane * CH + z]), s);
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const float p = tc::ex2(s * P.c - m);
+#pragma unroll
+            for (int z = 0; z < CH; ++z) w[z] = fmaf(p, __bfloat162float(v[lane * CH + z]), w[z]);
+        }
+#pragma unroll
+        for (int z = 0; z < CH; ++z) acc[z] = fmaf(w[z] / l, at(sV2, r, lane * CH + z), acc[z]);
+    }
+#pragma unroll
+    for (int z = 0; z < CH; ++z) scratch[warp * D + lane * CH + z] = acc[z];
+    __syncthreads();
+    for (int c = threadIdx.x; c < D; c += THREADS) {
+        float o = 0.f;
+        for (int w = 0; w < WARPS; ++w) o += scratch[w * D + c];
+        P.out[((int64_t)b * P.hq + hk * P.g + head) * D + c] = __float2bfloat16_rn(o);
+    }
+    __syncthreads();
+}
+
+template <int D>
+__global__ void __launch_bounds__(THREADS, PER_SM<D>) kernel(const __grid_constant__ Params P) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -144,6 +193,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM<D>) kernel(const Params P) {
     }
     for (int x = threadIdx.x; x < it.blocks * it.parts * (D + 2); x += THREADS) part[x] = x % (D + 2) == D ? tc::LOWEST_REF : 0.f;
 
+    bool whole = false;                                  // see whole_rows
     for (int j0 = j_begin; j0 < j_end; j0 += PIECE<D>) {
         const int count = min(PIECE<D>, j_end - j0);
         if (j0 > j_begin) {
@@ -162,13 +212,21 @@ __global__ void __launch_bounds__(THREADS, PER_SM<D>) kernel(const Params P) {
             if (j0 + count == S1.keep + 1) { put(sK, count - 1, 0); put(sV, count - 1, 2); }
             if (j0 == j_begin) { put(sK2, n2 - 1, 1); put(sV2, n2 - 1, 3); }
         }
+        uint32_t most = 0u;                              // of the exponents of the second values
+        if (j0 == j_begin)
+            for (int x = threadIdx.x; x < n2 * CPR; x += THREADS) {
+                const int r = x / CPR, c = x % CPR;
+                const uint4 u = *reinterpret_cast<const uint4 *>(r == n2 - 1 ? sNew + (P.g + 3) * D + c * 8 : sV2 + sw<D>(r, c));
+                most = __vmaxu2(most, __vmaxu2(__vmaxu2(u.x & 0x7f807f80u, u.y & 0x7f807f80u), __vmaxu2(u.z & 0x7f807f80u, u.w & 0x7f807f80u)));
+            }
+        whole |= (most & 0xffffu) >= (191u << 7) || most >> 16 >= (191u << 7);
         const int padded = min(PIECE<D>, (count + 31) & ~31);
         for (int x = threadIdx.x; x < (padded - count) * CPR; x += THREADS) {
             const int o = sw<D>(count + x / CPR, x % CPR);
             *reinterpret_cast<uint4 *>(sK + o) = make_uint4(0u, 0u, 0u, 0u);
             *reinterpret_cast<uint4 *>(sV + o) = make_uint4(0u, 0u, 0u, 0u);
         }
-        __syncthreads();
+        whole = __syncthreads_or(whole);
         keep(S1, sK, j0, j0, j0 + count);
         keep(T1, sV, j0, j0, j0 + count);
         if (split == 0 && j0 == j_begin) {
@@ -318,9 +376,10 @@ __global__ void __launch_bounds__(THREADS, PER_SM<D>) kernel(const Params P) {
         if (c == 0) { own[head * (D + 2) + D] = m; own[head * (D + 2) + D + 1] = l; }
     }
     cl.sync();
-    for (int x = split * THREADS + threadIdx.x; x < P.g * D; x += P.splits * THREADS) {
-        const int head = x / D, c = x % D;
-        float m = tc::LOWEST_REF, l = 0.f, o = 0.f;
+    auto merged = [&](int head, int c, float &m, float &l) {
+        float o = 0.f;
+        m = tc::LOWEST_REF;
+        l = 0.f;
         for (int r = 0; r < P.splits; ++r) m = fmaxf(m, cl.map_shared_rank(own, r)[head * (D + 2) + D]);
         for (int r = 0; r < P.splits; ++r) {
             const float *src = cl.map_shared_rank(own, r) + head * (D + 2);
@@ -328,6 +387,17 @@ __global__ void __launch_bounds__(THREADS, PER_SM<D>) kernel(const Params P) {
             o = fmaf(src[c], f, o);
             l = fmaf(src[D + 1], f, l);
         }
+        return o;
+    };
+    float m, l;
+    if (whole) {
+        for (int head = 0; split == 0 && head < P.g; ++head) {
+            merged(head, 0, m, l);
+            whole_rows<D>(P, sNew, sK2, sV2, reinterpret_cast<float *>(sK), head, m, l);
+        }
+    } else for (int x = split * THREADS + threadIdx.x; x < P.g * D; x += P.splits * THREADS) {
+        const int head = x / D, c = x % D;
+        const float o = merged(head, c, m, l);
         P.out[((int64_t)b * P.hq + hk * P.g + head) * D + c] = __float2bfloat16_rn(o / l);
     }
     cl.sync();               // no CTA leaves while its shared memory is read

@@ -1,6 +1,6 @@
 """The one-token kernel of generation (norms, cache hand-over and attention in one launch) and the projections of up to 64 rows:
 remainders of keys, offsets and heads, and short caches against the same module called module by module; over-long and strided caches,
-and the shapes that the kernel takes or leaves, at its C entry against 64 bits."""
+and the shapes that the kernel takes or leaves, at its C entry against 64 bits; second values that are not finite."""
 import ctypes as C
 
 import pytest
@@ -151,3 +151,21 @@ def test_entry_leaves_what_it_does_not_take():
     for d, w2 in ((64, 65), (32, 8)):
         proj, gains, caches = _step_inputs(1, 2, 1, d, 20, 20)
         assert _step_attn(proj, gains, caches, 2, 1, d, 30, w2)[0] == 2        # SA2_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("d,w1,w2", [(64, 100, 9), (128, 100, 16), (64, 700, 33)])
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), 3e38, float("nan")])
+@pytest.mark.parametrize("row", [0, 3, -1])
+def test_second_values_that_are_not_finite(d, w1, w2, value, row):
+    """Infinite second values reach the outputs of their channel as infinities of the sign that the sum over all keys has."""
+    b, hq, hk = 2, 4, 2
+    proj, gains, caches = _step_inputs(b, hq, hk, d, w1 + 20, w2 - 1)
+    caches[3][1, row, 0, 5] = value
+    status, out, _ = _step_attn(proj, gains, caches, hq, hk, d, w1, w2)
+    want = _step_reference(proj, gains, caches, hq, hk, d, w1, w2)[0].to(torch.bfloat16)
+    assert status == _lib.SA2_OK
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf()) and torch.equal(out[out.isinf()], want[want.isinf()])
+    rest = want.isfinite() & (want.abs() < 1e30)
+    assert (out[rest].double() - want[rest].double()).norm() <= 2 ** -7 * want[rest].double().norm()
+    big = want.isfinite() & ~rest
+    assert ((out[big].double() - want[big].double()).abs() <= 2 ** -4 * want[big].double().abs()).all()
