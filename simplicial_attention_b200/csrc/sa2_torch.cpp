@@ -417,8 +417,12 @@ Tensor row_norm(const Tensor &x, const Tensor &w, double eps) {
     return y;
 }
 
-// Does the kernel for few rows take x W^T?  Up to 16 rows always, up to 64 with a small W: there a microsecond or two more on the
-// device than the library's kernel outweigh neither the 8 us its call costs the host more nor the norm's own launch.
+// Does the kernel for few rows take x W^T?  Up to 16 rows always: it is the faster one on the device too.  Up to 64 with a W of at most
+// 2^20 entries: on the device it takes longer there (with the norm, 512 -> 1536: 4.9 us at 32 rows and 7.5 at 64, against 3.0 and the norm's
+// own 2.0), but its two calls cost the host 16 to 20 us less.  Whole steps back to back, with the library's kernel / with this one (in
+// brackets the same as a graph, which the host does not bound): W of 0.75 and 0.25 M entries, 17 rows 48 / 30 us (16.6 / 16.9), 32 rows 48 /
+// 30 (17.2 / 18.4), 64 rows 47 / 31 (17.5 / 24.5).  Above the line the gap closes and turns: 1.25 and 0.25 M, 64 rows 48 / 43 (25.6 / 37.8);
+// 5 and 1 M, 64 rows 52 / 82 (44 / 75); 20 and 4 M, 17 rows 54 / 69 (35 / 63).
 bool few_rows(const Tensor &x, const Tensor &w) {
     const int64_t rows = x.size(0) * x.size(1), k = w.size(1), outs = w.size(0);
     return rows <= (k * outs <= 1 << 20 ? 64 : 16) && k % 32 == 0 && outs % 16 == 0 && x.scalar_type() == at::kBFloat16 && x.is_contiguous() &&
