@@ -13,7 +13,9 @@
 // Three bf16 terms are not every fp32 value: from 3.39e38 the first one is infinite (and the second a NaN, as those of infinities
 // are), below 2^-109 the last ones leave bf16's range.  Where an operand's largest entry in a CTA is not in [2^-80, 2^60), or an output
 // is not finite, the scalar kernels, launched behind these, do the work again: the forward's row tile by row tile (LSE_REDO), the backward's
-// batch element by batch element (a flag in the workspace).  Otherwise they return at once (2 to 3 us each).  The maxima ride with the
+// batch element by batch element (a flag in the workspace).  Otherwise they return at once, and since
+// their blocks may take their places while the kernel before ends, a pass is 2 us longer forward and 3 both ways (4 and 6 without that; b1
+// n128 h2 d32).  The maxima ride with the
 // splitting of the operands, four instructions to its forty; a check of every entry for itself cost 5 to 11 % of a kernel.
 #pragma once
 #include "sa2_tc_common.cuh"

@@ -607,6 +607,7 @@ template <int D>
 __global__ void __launch_bounds__(Cfg<D>::THREADS) fwd_kernel(const KernelParams p, const bool redo) {
     extern __shared__ __align__(16) float smem[];
     const int ce = (int)cooperative_groups::this_cluster().num_blocks();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (redo && __float_as_uint(p.lse[((int64_t)blockIdx.z * p.hq + blockIdx.y) * p.n + blockIdx.x / ce * TILE]) != LSE_REDO) return;
     row_tile<D, MODE_FWD>(p, smem, blockIdx.x / ce, blockIdx.y, blockIdx.z, redo);
 }
@@ -620,6 +621,7 @@ __global__ void __launch_bounds__(Cfg<D>::THREADS) bwd_kernel(const KernelParams
     extern __shared__ __align__(16) float smem[];
     const int ce = (int)cooperative_groups::this_cluster().num_blocks();
     int x = blockIdx.x / ce;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (redo && !redo[(x >= n.k2 && x < n.k2 + n.k1 ? 0 : p.b) + blockIdx.y]) return;
     // the longest tiles first
     if (x < n.k2) { row_tile<D, MODE_BWD_K2>(p, smem, x / p.hk, x % p.hk, blockIdx.y, redo != nullptr); return; }
@@ -669,16 +671,23 @@ inline int cluster_size(int64_t tiles_per_element, int w2, int groups, int sms) 
     return ce;
 }
 
+// early: the kernel begins with griddepcontrol.wait, so its blocks may take their places while the kernel before it ends
 template <typename K, typename... Args>
-inline bool launch_clusters(K kernel, dim3 grid, int threads, size_t smem, int ce, cudaStream_t st, const Args &...args) {
+inline bool launch_clusters_at(bool early, K kernel, dim3 grid, int threads, size_t smem, int ce, cudaStream_t st, const Args &...args) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = ce; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ce; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
+    cfg.attrs = attr; cfg.numAttrs = early ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+template <typename K, typename... Args>
+inline bool launch_clusters(K kernel, dim3 grid, int threads, size_t smem, int ce, cudaStream_t st, const Args &...args) {
+    return launch_clusters_at(false, kernel, grid, threads, smem, ce, st, args...);
 }
 
 template <int D> inline bool launch_delta(const KernelParams &p, cudaStream_t st, int *redo = nullptr) {
@@ -689,7 +698,7 @@ template <int D> inline bool launch_delta(const KernelParams &p, cudaStream_t st
 template <int D> inline bool launch_fwd(const KernelParams &p, int sms, cudaStream_t st, bool redo = false) {
     using C = Cfg<D>;
     const int tiles = (p.n + TILE - 1) / TILE, ce = cluster_size((int64_t)tiles * p.hq, p.w2, C::NG, sms);
-    return launch_clusters(fwd_kernel<D>, dim3(tiles * ce, p.hq, p.b), C::THREADS, C::smem(false), ce, st, p, redo);
+    return launch_clusters_at(redo, fwd_kernel<D>, dim3(tiles * ce, p.hq, p.b), C::THREADS, C::smem(false), ce, st, p, redo);
 }
 // dq / dk2, dv2 / dk1, dv1, those asked for, in one launch
 template <int D> inline bool launch_bwd(const KernelParams &p, bool q, bool k2, bool k1, int sms, cudaStream_t st, const int *redo = nullptr) {
@@ -699,7 +708,7 @@ template <int D> inline bool launch_bwd(const KernelParams &p, bool q, bool k2, 
     // (from the whole backward's tiles, so that a part launched alone gives the same bits)
     const int64_t all = (int64_t)tiles(p.n) * p.hq + (int64_t)(tiles(p.nk2) + tiles(p.nk1)) * p.hk;
     const int ce = cluster_size(all, p.w2, C::NG, sms);
-    return launch_clusters(bwd_kernel<D>, dim3((unsigned)(n.q + n.k2 + n.k1) * ce, p.b), C::THREADS, C::smem(true), ce, st, p, n, redo);
+    return launch_clusters_at(redo != nullptr, bwd_kernel<D>, dim3((unsigned)(n.q + n.k2 + n.k1) * ce, p.b), C::THREADS, C::smem(true), ce, st, p, n, redo);
 }
 
 }  // namespace simt
