@@ -72,7 +72,7 @@ typedef struct sa2_shape {
 
 /*
  * Parts of the backward that sa2_bwd_args.phases can select (0 runs all of them).  ROWSUM writes
- * D_i = sum_c O_ic dO_ic into the workspace; K1 (dK1, dV1) and Q (dQ, dK2, dV2) read it and are
+ * D_i = sum_c O_ic dO_ic into the workspace (and clears the marks kept there); K1 (dK1, dV1) and Q (dQ, dK2, dV2) read it and are
  * independent of each other, so a caller may time them apart or run them on different streams
  * after ROWSUM has been ordered before both.
  */

@@ -16,8 +16,8 @@
 // [192 x + 96, +96); U [384, +64), W [448, +64).
 //
 // Bound: a unit's 96 products fetch 384 KB from shared memory, ~3100 cycles; the chain operands -> S / dP -> P / G -> U / W of two
-// units in flight takes ~6000 cycles a unit.  b1 n1024 h8 d64 w512/32: 5.5 ms on the scalar kernels -> 0.53 (MODE_K1) + 0.60 ms;
-// forward + backward 7.5 -> 1.45 ms, b1 n128 h2 d32 full causal 0.30 -> 0.11 ms.
+// units in flight takes ~6000 cycles a unit.  b1 n1024 h8 d64 w512/32: 5.5 ms on the scalar kernels -> 0.54 (MODE_K1) + 0.60 ms;
+// forward + backward 7.5 -> 1.45 ms, b1 n128 h2 d32 full causal 0.30 -> 0.10 ms.
 #pragma once
 #include "sa2_f32_common.cuh"
 #include "sa2_tc_bwd_k1.cuh"

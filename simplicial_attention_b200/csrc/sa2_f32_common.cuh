@@ -5,8 +5,8 @@
 // the small ones first.  The tensor cores truncate as they accumulate, so no accumulator lives longer than one unit of 64
 // keys (four K steps of the large product): the sums over a window, over the offsets and over the heads are fp32 additions
 // in registers.  Errors against 64 bits, norm of the difference over norm of the result, scalar fp32 kernels of sa2_simt.cuh
-// against these: b1 n1000 d64 w512/32 out 2.8e-7 -> 1.2e-7, dq 5.9e-7 -> 3.9e-7, dk1 1.7e-6 -> 4.2e-7, dv1 1.5e-6 -> 3.1e-7, dk2
-// 5.9e-7 -> 4.0e-7, dv2 3.7e-7 -> 2.7e-7, lse 5.0e-8 -> 4.9e-8; b1 n128 h2 d32, full causal, dk1 7.1e-7 -> 3.5e-7.
+// against these: b1 n1000 d64 w512/32 out 2.8e-7 -> 1.3e-7, dq 5.9e-7 -> 4.1e-7, dk1 1.7e-6 -> 4.4e-7, dv1 1.5e-6 -> 3.0e-7, dk2
+// 5.9e-7 -> 4.1e-7, dv2 3.7e-7 -> 2.6e-7, lse 5.0e-8 -> 5.0e-8; b1 n128 h2 d32, full causal, dk1 7.1e-7 -> 3.7e-7.
 //
 // Operands are made by the kernels from plain fp32 rows (any 16-byte aligned strides): no tensor maps and no scratch.
 //

@@ -256,8 +256,9 @@ inline int bwd_reduce_launch(const BqParams &Q, bool pair, cudaStream_t st) {
                          (Q.reduce_k1 ? (int64_t)kp.b * kp.nk1 * kp.hk : 0);
     if (rows == 0) return SA2_OK;
     const unsigned blocks = (unsigned)((rows * (D / 4) + 255) / 256);
-    if (D == 128 || pair) bwd_q_reduce_kernel<D, true><<<blocks, 256, 0, st>>>(Q);
-    else bwd_q_reduce_kernel<D, D == 128><<<blocks, 256, 0, st>>>(Q);
+    const bool grouped = kp.g > 1 && Q.nsplit == 1;
+    if (D == 128 || pair) (grouped ? bwd_q_reduce_kernel<D, true, true> : bwd_q_reduce_kernel<D, true, false>)<<<blocks, 256, 0, st>>>(Q);
+    else (grouped ? bwd_q_reduce_kernel<D, D == 128, true> : bwd_q_reduce_kernel<D, D == 128, false>)<<<blocks, 256, 0, st>>>(Q);
     return cudaGetLastError() == cudaSuccess ? SA2_OK : SA2_ERR_CUDA;
 }
 

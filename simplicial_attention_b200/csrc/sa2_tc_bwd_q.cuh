@@ -817,8 +817,10 @@ bwd_q_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ C
 // T of R rows and the split of offsets [e0, e0 + epc) at slab row k - off2 - R T + e0 + epc - 1, for the
 // tiles where that index falls inside [0, R - 1 + epc) and among the rows of the sweeps that the CTA ran.
 // ---------------------------------------------------------------------------
-template <int D, bool PAIR>
-__global__ void bwd_q_reduce_kernel(const BqParams P) {
+// GROUPED: more than one query head a key/value head and one split, four heads' loads at a time (with one head their registers would only
+// cost blocks).  b2 n495 hq16 hk2 d32 w214/10 16.7 us with a head after the other -> 4.7.
+template <int D, bool PAIR, bool GROUPED>
+__global__ void __launch_bounds__(256) bwd_q_reduce_kernel(const BqParams P) {
     constexpr int TPR = D / 4;                          // threads per row
     constexpr int ROWS = bq_rows(PAIR);
     const KernelParams &kp = P.kp;
@@ -851,28 +853,54 @@ __global__ void bwd_q_reduce_kernel(const BqParams P) {
         const int b = (int)(rest / kp.nk2);
         float ak[4] = {0.f, 0.f, 0.f, 0.f}, av[4] = {0.f, 0.f, 0.f, 0.f};
         const int pos = k - kp.off2;                    // in query coordinates (may be negative for halo rows)
-        for (int hh = 0; hh < kp.g; ++hh) {
-            const int h = hk * kp.g + hh;
-            for (int s = 0; s < P.nsplit; ++s) {
-                // tiles T with 0 <= pos - ROWS T + top < acc_rows
-                const int e0 = (s / P.tsplit) * P.epc, top = e0 + P.epc - 1;
-                const int low = P.epc - (min(kp.w2 - e0, P.epc) + bq_step(PAIR) - 1) / bq_step(PAIR) * bq_step(PAIR);      // first row there is
-                const int t_hi = min(P.nqt - 1, pos + top >= 0 ? (pos + top) / ROWS : -1);
-                for (int T = pos + top < acc_rows ? 0 : (pos + top - acc_rows) / ROWS + 1; T <= t_hi; ++T) {
-                    const int row = pos - ROWS * T + top;
-                    // (a tile that sees no start of the sequence has run all the split's sweeps, over units)
-                    if (row < low) continue;
-                    if (ROWS * T + kp.off2 < kp.w2 - 1 || ROWS * (T + 1) + kp.off1 < 64 * P.nu) {
-                        const BqGeom g = bq_geom<PAIR>(P, T, s);
-                        if (g.nunits == 0 || row < P.epc - bq_step(PAIR) * g.nsweeps) continue;
-                    }
-                    const float *slab = P.part_k2 + ((((size_t)b * kp.hq + h) * P.nqt + T) * P.nsplit + s) * (size_t)(2 * acc_rows * D);
-                    const float4 vk = *reinterpret_cast<const float4 *>(slab + (size_t)row * D + c4);
-                    const float4 vv = *reinterpret_cast<const float4 *>(slab + (size_t)(acc_rows + row) * D + c4);
-                    ak[0] += vk.x; ak[1] += vk.y; ak[2] += vk.z; ak[3] += vk.w;
-                    av[0] += vv.x; av[1] += vv.y; av[2] += vv.z; av[3] += vv.w;
+        // The slab rows of split s that hold row k: at most two tiles T with 0 <= pos - ROWS T + top < acc_rows, T1 and the one before it
+        static_assert(ROWS - 1 + BQ_MAX_EPC <= 2 * ROWS, "two tiles at most");
+        int T1, row[2];
+        bool ok[2];
+        auto find = [&](int s) {
+            const int e0 = (s / P.tsplit) * P.epc, top = e0 + P.epc - 1;
+            const int low = P.epc - (min(kp.w2 - e0, P.epc) + bq_step(PAIR) - 1) / bq_step(PAIR) * bq_step(PAIR);      // first row there is
+            T1 = min(P.nqt - 1, pos + top >= 0 ? (pos + top) / ROWS : -1);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int T = T1 - 1 + x;
+                row[x] = pos - ROWS * T + top;
+                ok[x] = T >= 0 && row[x] >= low && row[x] < acc_rows;
+                // (a tile that sees no start of the sequence has run all the split's sweeps, over units)
+                if (ok[x] && (ROWS * T + kp.off2 < kp.w2 - 1 || ROWS * (T + 1) + kp.off1 < 64 * P.nu)) {
+                    const BqGeom g = bq_geom<PAIR>(P, T, s);
+                    ok[x] = g.nunits > 0 && row[x] >= P.epc - bq_step(PAIR) * g.nsweeps;
                 }
             }
+        };
+        // all loads of a head before its sums: where they are not there a zero is added
+        auto add = [&](int h, int s) {
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 vk[2], vv[2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const float *slab = P.part_k2 + ((((size_t)b * kp.hq + h) * P.nqt + (T1 - 1 + x)) * P.nsplit + s) * (size_t)(2 * acc_rows * D) + c4;
+                vk[x] = ok[x] ? *reinterpret_cast<const float4 *>(slab + (size_t)row[x] * D) : zero;
+                vv[x] = ok[x] ? *reinterpret_cast<const float4 *>(slab + (size_t)(acc_rows + row[x]) * D) : zero;
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                ak[0] += vk[x].x; ak[1] += vk[x].y; ak[2] += vk[x].z; ak[3] += vk[x].w;
+                av[0] += vv[x].x; av[1] += vv[x].y; av[2] += vv[x].z; av[3] += vv[x].w;
+            }
+        };
+        if constexpr (GROUPED) {
+            find(0);
+#pragma unroll 4
+            for (int hh = 0; hh < kp.g; ++hh) add(hk * kp.g + hh, 0);
+        } else {
+#pragma unroll 1
+            for (int hh = 0; hh < kp.g; ++hh)
+#pragma unroll 1
+                for (int s = 0; s < P.nsplit; ++s) {
+                    find(s);
+                    add(hk * kp.g + hh, s);
+                }
         }
 #pragma unroll
         for (int z = 0; z < 4; ++z) ak[z] *= kp.scale;
