@@ -1,5 +1,5 @@
-"""dQ, dK2 and dV2 on tiles of 64 query rows times two offsets, or 128 times one: lengths around a tile, odd numbers of offsets, a window of one unit
-more than a CTA holds, ranges of offsets, halos.  Against the fp32 kernels on the same bf16 tensors."""
+"""dQ, dK2 and dV2 on tiles of 64 query rows times two offsets, and of 128 rows and one: lengths around a tile, odd numbers of
+offsets, a window of one unit more than a CTA holds, ranges of offsets, halos.  Against the fp32 kernels on the same bf16 tensors."""
 import pytest
 import torch
 from torch.profiler import ProfilerActivity, profile
@@ -26,6 +26,21 @@ CASES = [
 ]
 
 
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "b%d_n%d_hq%d_hk%d_d%d_w%d_%d_off%d" % c)
+def test_matches_the_fp32_kernels(case):
+    b, n, hq, hk, d, w1, w2, off = case
+    g = torch.Generator(device="cuda").manual_seed(n + d)
+    rand = lambda rows, h: torch.randn(b, rows, h, d, device="cuda", generator=g).to(torch.bfloat16)
+    q, do, keys = rand(n, hq), rand(n, hq), [rand(n + off, hk) for _ in range(4)]
+    out, lse = sa.sa2_forward(q, *keys, w1, w2)
+    got, again = (sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="tcgen05") for _ in range(2))
+    want = sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="simt")
+    assert sa.device_status() == 0
+    for x, (a, r, w) in enumerate(zip(got, again, want)):
+        assert torch.equal(a, r)
+        assert (a - w).norm() <= REL * w.norm(), (x, ((a - w).norm() / w.norm()).item())
+
+
 # shapes that run on tiles of 128 rows and one offset
 ROWS = [
     (40, 128, 8, 2, 64, 512, 5, 0),
@@ -40,30 +55,12 @@ ROWS = [
 
 @pytest.mark.parametrize("case", ROWS, ids=lambda c: "b%d_n%d_hq%d_hk%d_d%d_w%d_%d_off%d" % c)
 def test_short_windows_take_tiles_of_128_rows(case):
-    names = []
-
-    def look(call):
-        with profile(activities=[ProfilerActivity.CUDA]) as p:
-            call()
-            torch.cuda.synchronize()
-        names.extend(e.key for e in p.key_averages())
-
-    test_matches_the_fp32_kernels(case, look)
-    assert any("bwd_q_kernel<" in k and "false>" in k for k in names), names
-
-
-@pytest.mark.parametrize("case", CASES, ids=lambda c: "b%d_n%d_hq%d_hk%d_d%d_w%d_%d_off%d" % c)
-def test_matches_the_fp32_kernels(case, look=None):
+    test_matches_the_fp32_kernels(case)
     b, n, hq, hk, d, w1, w2, off = case
-    g = torch.Generator(device="cuda").manual_seed(n + d)
-    rand = lambda rows, h: torch.randn(b, rows, h, d, device="cuda", generator=g).to(torch.bfloat16)
-    q, do, keys = rand(n, hq), rand(n, hq), [rand(n + off, hk) for _ in range(4)]
+    q, *keys = [torch.randn(b, rows, h, d, device="cuda", dtype=torch.bfloat16) for rows, h in ((n, hq),) + ((n + off, hk),) * 4]
     out, lse = sa.sa2_forward(q, *keys, w1, w2)
-    got, again = (sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="tcgen05") for _ in range(2))
-    want = sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="simt")
-    if look:
-        look(lambda: sa.sa2_backward(q, *keys, out, lse, do, w1, w2, grad_dtype=torch.float32, kernel="tcgen05"))
-    assert sa.device_status() == 0
-    for x, (a, r, w) in enumerate(zip(got, again, want)):
-        assert torch.equal(a, r)
-        assert (a - w).norm() <= REL * w.norm(), (x, ((a - w).norm() / w.norm()).item())
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        sa.sa2_backward(q, *keys, out, lse, q, w1, w2)
+        torch.cuda.synchronize()
+    names = [e.key for e in p.key_averages()]
+    assert any("bwd_q_kernel<" in k and "false>" in k for k in names), names
